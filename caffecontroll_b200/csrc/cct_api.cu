@@ -318,7 +318,7 @@ int cct_conv_plan_create(cct_ctx* ctx, const cct_conv_desc* desc, cct_conv_plan*
   p->G = G;
   p->algo = algo;
   if (algo == CCT_ALGO_UMMA_3XTF32) {
-    const int rc2 = umma_plan_create(ctx, G, &p->umma);
+    const int rc2 = umma_plan_create(ctx, G, desc->algo == CCT_ALGO_UMMA_3XTF32, &p->umma);
     if (rc2 != CCT_OK) {
       delete p;
       return rc2;

@@ -99,7 +99,9 @@ int simt_conv_backward(cct_ctx* ctx, const ConvGeom& G, const float* X, const fl
 
 // ---- tcgen05 3xTF32 path (conv_umma.cu) ----
 struct UmmaPlan;  // opaque: tables, packed weights, split-K scratch
-int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out);
+// `tensor_only`: every pass on the tensor cores, however small the layer (CCT_ALGO_UMMA_3XTF32 by name); otherwise small
+// layers take the fp32 kernels of conv_small.cuh.
+int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan** out);
 void umma_plan_destroy(cct_ctx* ctx, UmmaPlan* p);
 size_t umma_plan_workspace_bytes(const UmmaPlan* p);
 bool umma_supported(const ConvGeom& G);

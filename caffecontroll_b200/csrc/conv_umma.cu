@@ -148,7 +148,12 @@ struct GatherParams {
   int out_pitch, out_plane;
   long long out_batch_stride;
   int out_group_channels, out_tile_channels;  // output channels per real group / per channel tile
-  int n, n_pad, k_pad;     // real / padded accumulator columns per virtual group, padded reduction length
+  int n, n_pad, k_pad;     // real / padded accumulator columns per virtual group, padded reduction length of one tile
+  int cols_per_channel;    // accumulator columns per output channel: 1, or the block of pixels of the data gradient
+  // Split reduction (forward, data gradient): a tile covers k_pad of the reduction, `splits` tiles share an accumulator's
+  // place and write raw sums to `partial` [split][vg][n_pad][pix_pad], which gather_reduce_kernel adds in order.
+  int splits, pix_pad;
+  float* partial;
   int n_pix_tiles, total_tiles;
   int a_stages, b_stages, acc_bufs;
   int tmem_cols;           // tensor-memory columns this CTA allocates: 512, or 256 when two CTAs share an SM
@@ -175,10 +180,11 @@ struct TileId {
 __device__ __forceinline__ TileId decode_tile(const GatherParams& P, int t, int kblocks) {
   TileId id;
   if (!P.wg) {
-    id.vg = t / P.n_pix_tiles;
-    id.ptile = t - id.vg * P.n_pix_tiles;
-    id.kb0 = 0;
-    id.split = 0;
+    const int r = t / P.n_pix_tiles, vgroups = P.total_tiles / (P.n_pix_tiles * P.splits);
+    id.ptile = t - r * P.n_pix_tiles;
+    id.split = P.splits == 1 ? 0 : r / vgroups;
+    id.vg = r - id.split * vgroups;
+    id.kb0 = id.split * kblocks;
   } else {
     const int r = t / P.wg_mtiles;
     id.ptile = t - r * P.wg_mtiles;
@@ -261,6 +267,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     const float* in_px = P.in;
     uint32_t mask = 0;                   // forward / data gradient: which taps are in bounds for this lane's pixel
     const MaskTap* pix_tab = P.taps;     // weight gradient: this tile's slice of the per-pixel table
+    const MaskTap* tile_taps = s_taps;   // forward / data gradient: this tile's part of the tap table
     auto setup_tile = [&](int tile_local) {
       const int t = blockIdx.x + tile_local * gridDim.x;
       const TileId id = decode_tile(P, t, kblocks);
@@ -280,6 +287,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         pix_tab = P.taps + (size_t)id.kb0 * kBlockK;
         return;
       }
+      tile_taps = s_taps + id.kb0 * kBlockK;
       const int pix = id.ptile * kTileM + row;
       mask = 0;  // which tap rows (bits 0-14) and tap columns (bits 16-30) fall inside the plane
       if (pix < P.n_pix) {
@@ -323,7 +331,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         }
         return;
       }
-      const MaskTap* tp = s_taps + kb * kBlockK;
+      const MaskTap* tp = tile_taps + kb * kBlockK;
 #pragma unroll
       for (int e = 0; e < kBlockK; ++e) {
         const MaskTap tap = tp[e];
@@ -479,6 +487,31 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         continue;
       }
       const int pix = ptile * kTileM + row;
+      if (P.splits > 1) {
+        // raw sums, lanes along the pixels
+        mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
+        tc_fence_after();
+        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.acc_cols);
+        float* op = P.partial + (size_t)(id.split * (P.total_tiles / (P.n_pix_tiles * P.splits)) + vg) * P.n_pad * P.pix_pad + pix;
+        for (int c = 0; c < P.n_pad / 16; ++c) {
+          float v[16];
+          tmem_ld16(acc + (uint32_t)(c * 16), v);
+          if (P.dual) {
+            float w[16];
+            tmem_ld16(acc + (uint32_t)(P.n_pad + c * 16), w);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] += w[j];
+          }
+          if (!failed) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) op[(size_t)(c * 16 + j) * P.pix_pad] = v[j];
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
+        continue;
+      }
       int b = 0, qy = 0, qx = 0;
       if (pix < P.n_pix) {
         const int per_img = P.q_h * P.q_w;
@@ -492,6 +525,8 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       float* op = P.out + (long long)b * P.out_batch_stride + (long long)ch0 * P.out_plane +
                   (long long)oy0 * P.out_pitch + ox0;
       const float* bias = s_bias + (P.n_bias ? ch0 : 0);  // zero padded: readable for every column of the tile
+      // the last channel tile of a group may hold fewer channels than the others
+      const int n_live = min(P.n, (P.out_group_channels - ntile * P.out_tile_channels) * P.cols_per_channel);
       mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
       tc_fence_after();
       const uint32_t live = (pix < P.n_pix && !failed) ? 1u : 0u;
@@ -525,7 +560,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
             const int col = c * 16 + h * 8 + j;
             const uint32_t in_y = (unsigned)(oy0 + ce[j].cy) < (unsigned)P.out_lim ? 1u : 0u;
             const uint32_t in_x = (unsigned)(ox0 + ce[j].cx) < (unsigned)P.out_lim ? 1u : 0u;
-            const uint32_t ok = live & (col < P.n ? 1u : 0u) & (unchecked | (in_y & in_x));
+            const uint32_t ok = live & (col < n_live ? 1u : 0u) & (unchecked | (in_y & in_x));
             float y = v[h * 8 + j] + bv[j];
             y = P.relu ? fmaxf(y, 0.f) : y;
             stg_if(op + ce[j].off, y, ok);
@@ -540,6 +575,46 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, (uint32_t)P.tmem_cols);
+}
+
+// Adds the split sums of gather_conv_kernel in split order, then does what its epilogue does: bias, ReLU, the scatter of
+// the data gradient.  Lanes along the pixels (both sides coalesced), a thread owns COLS columns of its pixel: eight where
+// there are plenty of pixels (one decode of the pixel for eight columns: CaffeNet conv5 at batch 32, 11 MB of L2-resident
+// sums, 14 -> 6 us against one column per thread), one where there are few and the splits' loads have to be in flight
+// together (conv3 of one image, 12 splits: 8 -> 4 us against eight).
+template <int COLS>
+__global__ void __launch_bounds__(128) gather_reduce_kernel(const __grid_constant__ GatherParams P, int col_tiles) {
+  pdl_wait();
+  const int pix = blockIdx.x * 128 + threadIdx.x;
+  const int vg = blockIdx.y / col_tiles, col0 = (blockIdx.y - vg * col_tiles) * COLS, vgroups = gridDim.y / col_tiles;
+  const int grp = vg / P.tiles_per_group, ntile = vg - grp * P.tiles_per_group;
+  const int live = min(COLS, min(P.n, (P.out_group_channels - ntile * P.out_tile_channels) * P.cols_per_channel) - col0);
+  if (pix >= P.n_pix || live <= 0) return;
+  const float* src = P.partial + ((size_t)vg * P.n_pad + col0) * P.pix_pad + pix;
+  const size_t stride = (size_t)vgroups * P.n_pad * P.pix_pad;
+  float y[COLS];
+#pragma unroll
+  for (int c = 0; c < COLS; ++c) y[c] = 0.f;
+#pragma unroll(COLS == 1 ? 8 : 2)
+  for (int s = 0; s < P.splits; ++s, src += stride)
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) y[c] += c < live ? __ldg(src + (size_t)c * P.pix_pad) : 0.f;
+  const int per_img = P.q_h * P.q_w;
+  const int b = pix / per_img, r = pix - b * per_img;
+  const int qy = r / P.q_w, qx = r - qy * P.q_w;
+  const int oy0 = qy * P.oy_mul + P.oy_add, ox0 = qx * P.ox_mul + P.ox_add;
+  const int ch0 = grp * P.out_group_channels + ntile * P.out_tile_channels;
+  float* op = P.out + (long long)b * P.out_batch_stride + (long long)ch0 * P.out_plane + (long long)oy0 * P.out_pitch + ox0;
+#pragma unroll
+  for (int c = 0; c < COLS; ++c) {
+    if (c < live) {
+      const ColEnt ce = P.cols[col0 + c];
+      float v = y[c];
+      if (P.bias) v += __ldg(P.bias + ch0 + col0 + c);  // the forward pass: one column per channel
+      if (P.relu) v = fmaxf(v, 0.f);
+      if (!P.check_out || ((unsigned)(oy0 + ce.cy) < (unsigned)P.out_lim && (unsigned)(ox0 + ce.cx) < (unsigned)P.out_lim)) op[ce.off] = v;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------- weight-gradient kernel
@@ -719,7 +794,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
       constexpr int kDyRows = kNPad / kWgDyWarps;
       const float* dyg = P.dy + (long long)(grp * P.dy_group_channels + ntile * P.n_real + w8) * P.mm;
       const int dy_step = kWgDyWarps * P.mm;  // elements between consecutive channel rows of this warp
-      const int b_live = P.n_real > w8 ? (P.n_real - w8 + kWgDyWarps - 1) / kWgDyWarps : 0;  // real rows
+      const int n_live = min(P.n_real, P.dy_group_channels - ntile * P.n_real);  // the last tile of a group may be shorter
+      const int b_live = n_live > w8 ? (n_live - w8 + kWgDyWarps - 1) / kWgDyWarps : 0;  // real rows
       uint8_t* lane_ptr = base_ptr + SUBS * 2 * kATile + w8 * 128 + ((((lane >> 2) ^ (w8 & 7)) << 4) + (lane & 3) * 4);
       float vb[kDyRows];
       auto load_rows = [&]() {
@@ -935,7 +1011,8 @@ __global__ void __launch_bounds__(kTsThreads, 1) wgrad_ts_kernel(const __grid_co
       // ---- dY: channels 32q .. 32q+31 of the tile; tensor-memory lanes of the same numbers
       const int q = warp - kTsTapWarps;
       const float* dyg = P.dy + (long long)(grp * P.dy_group_channels + ntile * P.n_real + q * 32) * P.mm;
-      const int live = min(32, max(0, P.n_real - q * 32));  // real channels of this quadrant
+      const int n_live = min(P.n_real, P.dy_group_channels - ntile * P.n_real);  // the last tile of a group may be shorter
+      const int live = min(32, max(0, n_live - q * 32));  // real channels of this quadrant
       float* turn = reinterpret_cast<float*>(base_ptr + kTsTurnOff) + q * (32 * 33);
       const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + kACol0;
       float vb[32];
@@ -1039,6 +1116,10 @@ WgradKernel wgrad_pick(int subs, int n_pad) {
   return subs == 2 ? wgrad_pick_nb<2>(n_pad / 16) : wgrad_pick_nb<1>(n_pad / 16);
 }
 
+}  // namespace
+#include "conv_small.cuh"
+namespace {
+
 // dW[o][kk] and db[o] from the split partial sums, added in split order (deterministic).  One block per 32 x 32
 // tile of (kk, channel): the partial sums are read along the channels (their fastest index), the tile is turned in
 // shared memory, and dW is written along kk (its fastest index) - both sides coalesced, no division per element.
@@ -1052,6 +1133,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
   const int kk0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
   const int ch0 = (vg / tiles_per_group) * og + (vg % tiles_per_group) * n_real;
+  n_real = min(n_real, og - (vg % tiles_per_group) * n_real);  // the last channel tile of a group may be shorter
   const size_t split_stride = (size_t)vgroups * rows_pad * n_pad;
   const int last = db ? k_real : k_real - 1;  // the bias row exists only where the kernel produced it
 #pragma unroll
@@ -1077,40 +1159,40 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
   }
 }
 
-// The same reduction for small outputs, where 32 x 32 tiles would leave most SMs idle: one block per row (channel
-// tile, kk) of the partial sums; 32 channels x 8 interleaved slices of the splits per pass, the eight slice sums
-// added in a fixed order - the result does not depend on the grid, and a thread's chain is splits / 8 long.
-__global__ void __launch_bounds__(256) wgrad_reduce_rows_kernel(const float* __restrict__ partial, float* __restrict__ dW,
-                                                                float* __restrict__ db, int splits, int vgroups,
-                                                                int tiles_per_group, int rows_pad, int n_real,
-                                                                int n_pad, int k_real, int og, int accumulate) {
+// The same reduction for small outputs, where 32 x 32 tiles would leave most SMs idle: a block owns 32 consecutive
+// elements of the partial sums' (row, channel) plane and SLICES interleaved slices of the splits, the slice sums added in a
+// fixed order - the result does not depend on the grid, and a thread's chain is splits / SLICES long.  dW is written
+// without coalescing (a few ten thousand elements).
+template <int SLICES>
+__global__ void __launch_bounds__(32 * SLICES) wgrad_reduce_flat_kernel(const float* __restrict__ partial,
+                                                                        float* __restrict__ dW, float* __restrict__ db,
+                                                                        int splits, int vgroups, int tiles_per_group,
+                                                                        int rows_pad, int n_real, int n_pad, int k_real,
+                                                                        int og, int accumulate) {
   pdl_wait();
-  __shared__ float part[8][33];
+  __shared__ float part[SLICES][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int rows = vgroups * (k_real + 1);
+  const int vg = blockIdx.y, e = blockIdx.x * 32 + tx;  // e = kk * n_pad + channel
   const size_t split_stride = (size_t)vgroups * rows_pad * n_pad;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    const int vg = r / (k_real + 1), kk = r - vg * (k_real + 1);
-    if (kk == k_real && !db) continue;  // no bias row in the partial sums (uniform over the block)
-    const int ch0 = (vg / tiles_per_group) * og + (vg % tiles_per_group) * n_real;
-    for (int j0 = 0; j0 < n_real; j0 += 32) {
-      const int j = j0 + tx;
-      float acc = 0.f;
-      if (j < n_real) {
-        const float* src = partial + ((size_t)vg * rows_pad + kk) * n_pad + j;
-#pragma unroll 4
-        for (int s = ty; s < splits; s += 8) acc += src[(size_t)s * split_stride];
-      }
-      __syncthreads();  // the previous pass has been read
-      part[ty][tx] = acc;
-      __syncthreads();
-      if (ty == 0 && j < n_real) {
-        float t = part[0][tx];
+  const bool in = e < (k_real + 1) * n_pad;
+  float acc = 0.f;
+  if (in) {
+    const float* src = partial + (size_t)vg * rows_pad * n_pad + e;
+#pragma unroll 8
+    for (int s = ty; s < splits; s += SLICES) acc += src[(size_t)s * split_stride];
+  }
+  part[ty][tx] = acc;
+  __syncthreads();
+  if (ty == 0 && in) {
+    const int kk = e / n_pad, j = e - kk * n_pad, first = (vg % tiles_per_group) * n_real;
+    // the last channel tile of a group may be shorter; the bias row exists only where the kernel produced it
+    if (j < min(n_real, og - first) && (kk < k_real || db)) {
+      float t = part[0][tx];
 #pragma unroll
-        for (int y = 1; y < 8; ++y) t += part[y][tx];
-        float* dst = kk < k_real ? dW + (size_t)(ch0 + j) * k_real + kk : db + ch0 + j;
-        *dst = accumulate ? *dst + t : t;
-      }
+      for (int y = 1; y < SLICES; ++y) t += part[y][tx];
+      const int ch = (vg / tiles_per_group) * og + first + j;
+      float* dst = kk < k_real ? dW + (size_t)ch * k_real + kk : db + ch;
+      *dst = accumulate ? *dst + t : t;
     }
   }
 }
@@ -1181,92 +1263,130 @@ __global__ void bias_grad_kernel(const float* __restrict__ plane_sums, float* __
 }
 
 // ------------------------------------------------------------------------------------------ weight packing
+// A block writes one row of the packed operand (blockIdx.y = (vg, j)), four consecutive reduction indices per thread and
+// step: one decode per four elements and 16-byte stores (a flat grid-stride loop spent most of its time dividing: CaffeNet
+// conv3's 0.9 M weights 8.0 / 11.6 us for the two operands, bound by neither memory nor launch).
+constexpr int kPackThreads = 128;
+
+__device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, const float* v) {
+  float h[4], l[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) split_tf32(v[e], h[e], l[e]);
+  *reinterpret_cast<float4*>(hi + at) = make_float4(h[0], h[1], h[2], h[3]);
+  *reinterpret_cast<float4*>(lo + at) = make_float4(l[0], l[1], l[2], l[3]);
+}
+
 // Forward B operand: [2 (hi, lo)][vg][n_pad][k_pad] <- W[o][Dg*k*k], zero padded.
-__global__ void pack_fwd_kernel(const float* __restrict__ W, float* __restrict__ hi, float* __restrict__ lo, int vgroups,
-                                int tiles_per_group, int og, int n_real, int n_pad, int k_real, int k_pad) {
+__global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __restrict__ W, float* __restrict__ hi,
+                                                                float* __restrict__ lo, int tiles_per_group, int og,
+                                                                int n_real, int n_pad, int k_real, int k_pad) {
   pdl_wait();
-  const size_t total = (size_t)vgroups * n_pad * k_pad;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int kk = (int)(t % k_pad);
-    const int j = (int)((t / k_pad) % n_pad);
-    const int vg = (int)(t / ((size_t)k_pad * n_pad));
-    float v = 0.f;
-    if (j < n_real && kk < k_real) {
-      const int ch = (vg / tiles_per_group) * og + (vg % tiles_per_group) * n_real + j;
-      v = W[(size_t)ch * k_real + kk];
-    }
-    float h, l;
-    split_tf32(v, h, l);
-    hi[t] = h;
-    lo[t] = l;
+  const int vg = blockIdx.y / n_pad, j = blockIdx.y - vg * n_pad;
+  const int ch = (vg % tiles_per_group) * n_real + j;  // inside the group
+  const bool live = j < n_real && ch < og;
+  const float* src = W + (size_t)((vg / tiles_per_group) * og + ch) * k_real;
+  const size_t row = (size_t)blockIdx.y * k_pad;
+  for (int kk = (blockIdx.x * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.x * kPackThreads * 4) {
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = (live && kk + e < k_real) ? __ldg(src + kk + e) : 0.f;
+    store_split4(hi, lo, row + kk, v);
   }
 }
 
 // Data-gradient B operand: [2][vg][n_pad][k_pad]; row j = (d, py, px) of channel tile nt of group g (py, px: position
 // inside an s x s block of input pixels), column kk = (oc, jy, jx) <- W[g*og + oc][d][py + jy*s][px + jx*s], zero where
 // the tap index exceeds the kernel.
-__global__ void pack_dgrad_kernel(const float* __restrict__ W, float* __restrict__ hi, float* __restrict__ lo,
-                                  int vgroups, int tiles_per_group, int og, int Dg, int k, int s, int taps, int d_tile,
-                                  int n_real, int n_pad, int k_real, int k_pad) {
+__global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* __restrict__ W, float* __restrict__ hi,
+                                                                  float* __restrict__ lo, int tiles_per_group, int og,
+                                                                  int Dg, int k, int s, int taps, int d_tile, int n_real,
+                                                                  int n_pad, int k_real, int k_pad) {
   pdl_wait();
-  const size_t total = (size_t)vgroups * n_pad * k_pad;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int kk = (int)(t % k_pad);
-    const int j = (int)((t / k_pad) % n_pad);
-    const int vg = (int)(t / ((size_t)k_pad * n_pad));
-    float v = 0.f;
-    if (j < n_real && kk < k_real) {
-      const int grp = vg / tiles_per_group;
-      const int d = (vg % tiles_per_group) * d_tile + j / (s * s);
-      const int py = (j / s) % s, px = j % s;
-      const int jx = kk % taps, jy = (kk / taps) % taps, oc = kk / (taps * taps);
+  const int vg = blockIdx.y / n_pad, j = blockIdx.y - vg * n_pad;
+  const int grp = vg / tiles_per_group, d = (vg - grp * tiles_per_group) * d_tile + j / (s * s);
+  const int py = (j / s) % s, px = j % s;
+  const bool live = j < n_real && d < Dg;
+  const float* src = W + ((size_t)grp * og * Dg + d) * k * k;
+  const size_t row = (size_t)blockIdx.y * k_pad;
+  for (int kk = (blockIdx.x * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.x * kPackThreads * 4) {
+    int oc = kk / (taps * taps), jy = (kk - oc * taps * taps) / taps, jx = kk % taps;
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
       const int kr = py + jy * s, kc = px + jx * s;
-      if (kr < k && kc < k) v = W[(((size_t)(grp * og + oc)) * Dg + d) * k * k + kr * k + kc];
+      v[e] = (live && kk + e < k_real && kr < k && kc < k) ? __ldg(src + (size_t)oc * Dg * k * k + kr * k + kc) : 0.f;
+      if (++jx == taps) {
+        jx = 0;
+        if (++jy == taps) { jy = 0; ++oc; }
+      }
     }
-    float h, l;
-    split_tf32(v, h, l);
-    hi[t] = h;
-    lo[t] = l;
+    store_split4(hi, lo, row + kk, v);
   }
 }
 
 int round_up(int v, int a) { return (v + a - 1) / a * a; }
 
-// Smallest number of equal channel tiles such that a tile spans at most `limit` accumulator columns.
+// Fewest channel tiles of at most 256 accumulator columns each (0: one channel alone is wider).
 int channel_tiles(int channels, int cols_per_channel) {
-  for (int t = 1; t <= channels; ++t)
-    if (channels % t == 0 && (channels / t) * cols_per_channel <= 256) return t;
-  return 0;
+  return cols_per_channel > 256 ? 0 : (channels + 256 / cols_per_channel - 1) / (256 / cols_per_channel);
 }
 
-// Channel tiles of the data gradient.  The widest accumulator is not always the fastest: work units (pixel tile x
-// channel tile) are spread over the resident CTAs in whole rounds, and accumulators of at most 128 columns run as two
-// CTAs per SM, whose last, half-empty round costs about half a round.  Estimated cycles = rounds x k-blocks x cycles per
-// k-block (MMA issue: 75 cycles each; MMA execution: half a cycle per column, shared by the SM's CTAs; gather: about
-// 2 500 cycles per k-block and producer set), for the widest tiling and for the next narrower ones down to 64 columns.
-int dgrad_channel_tiles(int sm_count, int channels, int cols_per_channel, long long pixel_tiles, int groups, int kblocks) {
+// Weight slots (hi and lo tile each) of a gather problem in shared memory: up to four.
+int gather_slots(int n_pad, int taps_smem, int n_bias, int ptab, size_t limit) {
+  int b = 4;
+  while (b > 1 && gather_smem(n_pad, taps_smem, b, n_bias, ptab).total + 1024 > limit) --b;
+  return b;
+}
+// Accumulators of at most 128 columns leave room for two CTAs per SM: 256 columns each (accumulator + two A slots) and half
+// the shared memory (the SM holds 228 KB, 1 KB of it reserved per resident CTA).  Three weight slots per CTA, or two when
+// the accumulator is the full 128 columns (each MMA then lasts long enough to cover the refill: CaffeNet conv5 forward
+// 0.189 -> 0.153 ms).
+bool two_ctas_per_sm(int n_pad, int taps_smem, int n_bias, int ptab, int* slots) {
+  const int acc_cols = n_pad <= 64 ? 2 * n_pad : n_pad;
+  *slots = gather_slots(n_pad, taps_smem, n_bias, ptab, 113 * 1024);
+  return acc_cols <= 128 && (*slots >= 3 || (*slots == 2 && acc_cols == 128));
+}
+
+// Channel tiles and splits of the reduction for the forward pass and the data gradient, by an estimate of the kernel's
+// time in microseconds.  A work unit is (pixel tile, channel tile, split); units are spread over the resident CTAs in whole
+// rounds.  Per k-block a CTA takes what its MMAs take (75 cycles to issue one, half a cycle per column to run it), or what
+// its producers take to gather (measured: 0.62 us alone on an SM with two producer sets, 0.8 us when two CTAs share one,
+// 0.35 us with four sets); a unit adds an epilogue that grows with its columns (64 columns 1.3 us, 192 columns 2.8 us), a
+// split reduction one more kernel and the traffic of the sums.  So: a last round that is nearly empty (CaffeNet conv3 at
+// batch 256: 2 x 338 units on 148 CTAs are five rounds, 3 x 338 half-width ones on 296 are 3.4) asks for narrower tiles, a
+// layer of few pixels (43 tiles at batch 32, 2 at batch 1) for narrower tiles and splits.  A candidate has to win by 3 %.
+struct GatherTiling {
+  int tiles = 0, splits = 1, kps = 0;
+};
+GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, int channels, int cols_per_channel, int kblocks,
+                                  int n_bias) {
+  GatherTiling best;
+  double best_us = 0.0;
   const int t0 = channel_tiles(channels, cols_per_channel);
-  if (t0 == 0) return 0;
-  int best_t = t0;
-  double best = 0.0;
-  for (int t = t0; t <= channels; ++t) {
-    if (channels % t) continue;
-    const int n_pad = round_up((channels / t) * cols_per_channel, 16);
-    if (t > t0 && n_pad < 64) break;
-    const bool dual = n_pad <= 64, two_per_sm = (dual ? 2 * n_pad : n_pad) <= 128;
+  for (int t = t0; t > 0 && t <= channels; ++t) {
+    const int n_pad = round_up((channels + t - 1) / t * cols_per_channel, 16);
+    if (t > t0 && n_pad < 32) break;
+    if ((channels + t - 1) / t * (t - 1) >= channels) continue;  // the last tile would be empty
+    int slots_unused;
+    const bool two = two_ctas_per_sm(n_pad, kblocks * kBlockK, n_bias, 0, &slots_unused), dual = n_pad <= 64;
     const int mmas = dual ? 8 : 12;
-    const double exec = mmas * (dual ? n_pad : n_pad / 2.0);
-    const double per_kb = two_per_sm ? std::max({mmas * 75.0, 2.0 * exec, 2500.0 / 2}) : std::max({mmas * 75.0, exec, 2500.0 / 4});
-    const long long units = pixel_tiles * groups * t, slots = (long long)sm_count * (two_per_sm ? 2 : 1);
-    const long long tail = units % slots;
-    const double rounds = (double)(units / slots) + (tail == 0 ? 0.0 : (two_per_sm && 2 * tail <= slots) ? 0.55 : 1.0);
-    const double cost = rounds * kblocks * per_kb;
-    if (t == t0 || cost < 0.97 * best) {  // a narrower tiling gathers every pixel once more: it has to win clearly
-      best = cost;
-      best_t = t;
+    const double mhz = 1600.0, exec = mmas * (dual ? n_pad : n_pad / 2.0) / mhz, issue = mmas * 75 / mhz;  // clock under load
+    const double alone = std::max({exec, issue, two ? 0.62 : 0.35}), shared = two ? std::max({2 * exec, issue, 0.8}) : alone;
+    const double epilogue = 0.5 + 0.012 * n_pad;
+    for (int s = 1; s <= std::max(1, std::min(32, kblocks / 2)); ++s) {
+      const int kps = (kblocks + s - 1) / s;
+      if ((kblocks + kps - 1) / kps != s) continue;
+      const long long units = pixel_tiles * groups * t * s, slots = (long long)sms * (two ? 2 : 1), tail = units % slots;
+      double us = (double)(units / slots) * (kps * shared + 0.4 * epilogue) +
+                  (tail ? kps * (two && tail > sms ? shared : alone) + epilogue : 0.6 * epilogue) + 4.0;
+      if (s > 1) us += 2.3 + units * 128.0 * n_pad * 8.0 / 4e6;
+      if (!best.tiles || us < 0.97 * best_us) {
+        best_us = us;
+        best = GatherTiling{t, s, kps};
+      }
     }
   }
-  return best_t;
+  return best;
 }
 
 }  // namespace
@@ -1285,15 +1405,22 @@ struct GatherProblem {
   int taps_smem = -1;             // tap-table entries staged in shared memory (-1: k_pad)
   size_t map_k = 0;               // extent of the packed operand along the reduction (0: k_pad)
   size_t smem = 0;
+  int splits = 1, split_k = 0;    // splits of the reduction and the length of one (a multiple of 32; k_pad without splits)
+  float* partial = nullptr;       // split sums
+  size_t pix_pad = 0;
+  int small_ct = 0;               // > 0: small_conv_kernel with this many channels per block instead of gather_conv_kernel
 };
 
 struct UmmaPlan {
   ConvGeom G;
   GatherProblem fwd, dgr;
   int dgr_taps = 0, dgr_q = 0, dgr_q0 = 0;  // taps per axis; super-pixels per axis and the first one that holds a pixel
-  // weight gradient
+  // weight gradient: channel tiles per group, channels per tile (the last one may be shorter), padded to 16
+  int wt_tiles = 1, wt_n = 0;
   int w_mtiles, w_subs, w_stages, w_mgroups, w_splits, w_kblocks_total, w_kblocks_per_split, w_npad;
   size_t w_smem = 0;
+  bool w_small = false;             // weight gradient by small_wgrad_kernel
+  int ws_rows = 0, ws_cols = 0, ws_pix = 0;  // its row tiles, channel tiles and pixels per split
   bool w_ts = false;  // weight gradient by wgrad_ts_kernel (dY through tensor memory) instead of wgrad_kernel
   MaskTap* w_taps = nullptr;
   float* w_partial = nullptr;
@@ -1339,7 +1466,7 @@ int set_smem(cct_ctx* ctx, K kernel, size_t bytes) {
   return CCT_OK;
 }
 
-// Split reduction: tiles when they fill the machine, rows otherwise (both add in split order).
+// Split reduction: tiles when they fill the machine, the flat form otherwise (both add in a fixed order).
 void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* db, int splits, int vgroups,
                          int tiles_per_group, int rows_pad, int n_real, int n_pad, int k_real, int og,
                          int accumulate = 0) {
@@ -1347,46 +1474,60 @@ void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* d
   if ((int)(tiles.x * tiles.y * tiles.z) >= ctx->sm_count)
     launch_pdl(wgrad_reduce_kernel, dim3(tiles), dim3(256), 0, ctx->stream, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad,
                                                        n_real, n_pad, k_real, og, accumulate);
-  else
-    launch_pdl(wgrad_reduce_rows_kernel, dim3(std::max(1, std::min(vgroups * (k_real + 1), ctx->sm_count * 8))), dim3(256), 0, ctx->stream, 
-        partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate);
+  else {
+    const dim3 grid(((k_real + 1) * n_pad + 31) / 32, vgroups);
+    auto go = [&](auto kernel, int slices) {
+      launch_pdl(kernel, grid, dim3(32 * slices), 0, ctx->stream, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real,
+                 n_pad, k_real, og, accumulate);
+    };
+    if (splits < 16) go(wgrad_reduce_flat_kernel<4>, 4);
+    else if (splits < 64 || grid.x * grid.y > 2u * ctx->sm_count) go(wgrad_reduce_flat_kernel<8>, 8);
+    else go(wgrad_reduce_flat_kernel<32>, 32);
+  }
 }
 
-int pack_grid(cct_ctx* ctx, size_t total) {
-  size_t b = (total + 255) / 256;
-  return (int)std::min<size_t>(std::max<size_t>(b, 1), (size_t)ctx->sm_count * 8);
+dim3 pack_grid(int rows, int k_pad) { return dim3((k_pad / 4 + kPackThreads - 1) / kPackThreads, rows); }
+
+// Where the fp32 kernels of conv_small.cuh are the faster ones (measured, kernels alone, tensor cores -> fp32): forward of
+// 37 MFLOP (LeNet conv1, batch 64) 9.7 -> 5.0 us, 58 MFLOP (64 channels, 14 x 14, 3 x 3) 13.7 -> 6.8, 148 MFLOP 17 -> 12,
+// 231 MFLOP 14.8 -> 15.4; windows of 7 and 11 (too many window columns for the register pipeline) 94 MFLOP 10.1 -> 10.4,
+// 211 MFLOP 14.3 -> 23.  Weight gradient: 58 MFLOP 26 -> 9 us, 205 MFLOP 17.7 -> 19.  Flops count a multiply-add as two and
+// the idle channels and rows of the blocks with the others.
+constexpr double kSmallConvFlops = 1.5e8, kSmallWideFlops = 8e7, kSmallWgradFlops = 1.7e8;
+
+// Channels per block of small_conv_kernel for one pass (0: the tensor-core kernel).
+int use_small_conv(int k, int s, long long out_pixels, int groups, int ci, int co) {
+  const int ct = small_conv_ct(co);
+  if (!small_conv_pick(k, s, ct) || small_conv_smem(k, ct, ci, 0) > 48 * 1024) return 0;
+  const double flops = 2.0 * out_pixels * groups * ((co + ct - 1) / ct * ct) * ci * k * k;
+  return flops <= (k >= 7 ? kSmallWideFlops : kSmallConvFlops) ? ct : 0;
+}
+bool use_small_wgrad(long long pixels, int vgroups, int n, int k_real) {
+  const double flops = 2.0 * pixels * vgroups * ((n + kSwTile - 1) / kSwTile * kSwTile) * ((k_real + kSwTile) / kSwTile * kSwTile);
+  return flops <= kSmallWgradFlops;
 }
 
 // Tensor-memory and shared-memory budget of a gather problem, packed-weight buffer and its tensor map.
 int finish_problem(cct_ctx* ctx, UmmaPlan* p, GatherProblem& gp, int vgroups, int n_bias) {
   // Tensor memory (512 columns) = accumulator buffers + A stages of 64 columns.  Narrow problems run "dual" (see the
   // MMA loop): their accumulator is 2*n_pad wide.  Two accumulator buffers let the epilogue overlap the next tile.
-  const int taps_smem = gp.taps_smem < 0 ? gp.k_pad : gp.taps_smem;
+  const int taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k : gp.taps_smem;
   const size_t map_k = gp.map_k ? gp.map_k : (size_t)gp.k_pad;
   gp.dual = gp.n_pad <= 64;  // 2 MMAs of width <= 128 instead of 3 narrow ones; wider ones gain nothing
   gp.acc_cols = gp.dual ? 2 * gp.n_pad : gp.n_pad;
   if (2 * gp.acc_cols + 4 * 64 <= 512) { gp.acc_bufs = 2; gp.a_stages = 4; }
-  else if (2 * gp.acc_cols + 2 * 64 <= 512 && gp.k_pad / kBlockK <= 16) { gp.acc_bufs = 2; gp.a_stages = 2; }  // short K: the epilogue matters more
+  else if (2 * gp.acc_cols + 2 * 64 <= 512 && (gp.split_k ? gp.split_k : gp.k_pad) / kBlockK <= 16) { gp.acc_bufs = 2; gp.a_stages = 2; }  // short K: the epilogue matters more
   else { gp.acc_bufs = 1; gp.a_stages = std::min(4, (512 - gp.acc_cols) / 64); }
-  // Weight slots (hi and lo tile each) in shared memory: up to four, independent of the number of A slots.
   const int ptab = gp.taps_smem == 0 ? 16 : 0;  // weight-gradient mode: per-warp table slices (sized for 16 warps)
-  auto slots_that_fit = [&](size_t limit) {
-    int b = 4;
-    while (b > 1 && gather_smem(gp.n_pad, taps_smem, b, n_bias, ptab).total + 1024 > limit) --b;
-    return b;
-  };
-  gp.b_stages = slots_that_fit(kSmemLimit);
-  // Accumulators of at most 128 columns leave room for two CTAs per SM: 256 columns each (accumulator + two A
-  // slots) and half the shared memory (the SM holds 228 KB, 1 KB of it reserved per resident CTA).  Three weight slots
-  // per CTA, or two when the accumulator is the full 128 columns (each MMA then lasts long enough to cover the refill:
-  // CaffeNet conv5 forward 0.189 -> 0.153 ms).
-  const int b_two = slots_that_fit(113 * 1024);
-  if (gp.acc_cols <= 128 && (b_two >= 3 || (b_two == 2 && gp.acc_cols == 128))) {
+  gp.b_stages = gather_slots(gp.n_pad, taps_smem, n_bias, ptab, kSmemLimit);
+  int b_two;
+  if (two_ctas_per_sm(gp.n_pad, taps_smem, n_bias, ptab, &b_two)) {
     gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = 2; gp.b_stages = b_two;
   }
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
   gp.w_half = (size_t)vgroups * gp.n_pad * map_k;
   int rc = dev_alloc(ctx, p, &gp.w, 2 * gp.w_half);
+  if (rc == CCT_OK && gp.splits > 1) rc = dev_alloc(ctx, p, &gp.partial, (size_t)gp.splits * vgroups * gp.n_pad * gp.pix_pad);
   if (rc != CCT_OK) return rc;
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) {
@@ -1409,7 +1550,7 @@ int finish_problem(cct_ctx* ctx, UmmaPlan* p, GatherProblem& gp, int vgroups, in
 
 }  // namespace
 
-int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out) {
+int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan** out) {
   UmmaPlan* p = new UmmaPlan();
   p->G = G;
   int rc = CCT_OK;
@@ -1417,13 +1558,16 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out) {
   // ---- forward: accumulator columns = output channels of a tile, reduction = (d, kr, kc)
   {
     GatherProblem& f = p->fwd;
-    f.tiles = channel_tiles(G.og, 1);
-    f.ch_tile = f.n = G.og / f.tiles;
-    f.n_pad = round_up(f.n, 16);
     f.k_real = G.Dg * kk;
     f.k_pad = round_up(f.k_real, kBlockK);
-    std::vector<MaskTap> t(f.k_pad);
-    for (int i = 0; i < f.k_pad; ++i) {
+    const long long pixel_tiles = ((long long)G.B * G.m * G.m + kTileM - 1) / kTileM;
+    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, G.bias ? G.o : 0);
+    f.tiles = tl.tiles;
+    f.ch_tile = f.n = (G.og + f.tiles - 1) / f.tiles;
+    f.n_pad = round_up(f.n, 16);
+    f.splits = tl.splits; f.split_k = tl.kps * kBlockK; f.pix_pad = (size_t)pixel_tiles * kTileM;
+    std::vector<MaskTap> t((size_t)f.splits * f.split_k);  // padding entries behind the last split's real ones
+    for (int i = 0; i < (int)t.size(); ++i) {
       if (i < f.k_real) {
         const int d = i / kk, kr = (i / G.k) % G.k, kc = i % G.k;
         t[i] = MaskTap{d * G.n * G.n + kr * G.n + kc, (1u << kr) | (1u << (16 + kc))};
@@ -1435,7 +1579,8 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out) {
     for (int j = 0; j < f.n_pad; ++j) c[j] = ColEnt{j * G.m * G.m, 0, 0};
     rc = upload(ctx, p, &f.taps, t);
     if (rc == CCT_OK) rc = upload(ctx, p, &f.cols, c);
-    if (rc == CCT_OK) rc = finish_problem(ctx, p, f, G.g * f.tiles, G.bias ? G.o : 0);
+    if (!tensor_only) f.small_ct = use_small_conv(G.k, G.s, (long long)G.B * G.m * G.m, G.g, G.Dg, G.og);
+    if (rc == CCT_OK && !f.small_ct) rc = finish_problem(ctx, p, f, G.g * f.tiles, G.bias ? G.o : 0);
   }
   // ---- data gradient as a stride-1 gather over dY: one "super pixel" = an s x s block of input pixels; accumulator
   //      columns = (d, py, px), reduction = (oc, jy, jx) with jy, jx < ceil(k/s); depth-to-space in the epilogue.
@@ -1445,19 +1590,18 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out) {
     p->dgr_taps = (G.k + G.s - 1) / G.s;
     p->dgr_q0 = G.p / G.s;
     p->dgr_q = (G.n - 1 + G.p) / G.s + 1 - p->dgr_q0;
-    {
-      const int J0 = (G.k + G.s - 1) / G.s, q0 = G.p / G.s, q = (G.n - 1 + G.p) / G.s + 1 - q0;
-      d.tiles = dgrad_channel_tiles(ctx->planning_sms(), G.Dg, ss, ((long long)G.B * q * q + kTileM - 1) / kTileM, G.g,
-                                    (G.og * J0 * J0 + kBlockK - 1) / kBlockK);
-    }
-    d.ch_tile = G.Dg / d.tiles;
-    d.n = d.ch_tile * ss;
-    d.n_pad = round_up(d.n, 16);
     const int J = p->dgr_taps;
     d.k_real = G.og * J * J;
     d.k_pad = round_up(d.k_real, kBlockK);
-    std::vector<MaskTap> t(d.k_pad);
-    for (int i = 0; i < d.k_pad; ++i) {
+    const long long pixel_tiles = ((long long)G.B * p->dgr_q * p->dgr_q + kTileM - 1) / kTileM;
+    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.Dg, ss, d.k_pad / kBlockK, 0);
+    d.tiles = tl.tiles;
+    d.ch_tile = (G.Dg + d.tiles - 1) / d.tiles;
+    d.n = d.ch_tile * ss;
+    d.n_pad = round_up(d.n, 16);
+    d.splits = tl.splits; d.split_k = tl.kps * kBlockK; d.pix_pad = (size_t)pixel_tiles * kTileM;
+    std::vector<MaskTap> t((size_t)d.splits * d.split_k);
+    for (int i = 0; i < (int)t.size(); ++i) {
       if (i < d.k_real) {
         const int jx = i % J, jy = (i / J) % J, oc = i / (J * J);
         t[i] = MaskTap{oc * G.m * G.m - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
@@ -1472,12 +1616,16 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out) {
     }
     rc = upload(ctx, p, &d.taps, t);
     if (rc == CCT_OK) rc = upload(ctx, p, &d.cols, c);
-    if (rc == CCT_OK) rc = finish_problem(ctx, p, d, G.g * d.tiles, 0);
+    if (!tensor_only && G.s == 1) d.small_ct = use_small_conv(G.k, 1, (long long)G.B * G.n * G.n, G.g, G.og, G.Dg);
+    if (rc == CCT_OK && !d.small_ct) rc = finish_problem(ctx, p, d, G.g * d.tiles, 0);
   }
   // ---- weight gradient: rows = (d, kr, kc) plus the all-ones row, columns = output channels of a tile
   if (rc == CCT_OK) {
-    const GatherProblem& f = p->fwd;
-    p->w_npad = f.n_pad;
+    GatherProblem f;  // the widest channel tiles, whatever the forward pass takes
+    f.k_real = p->fwd.k_real;
+    f.tiles = p->wt_tiles = channel_tiles(G.og, 1);
+    f.n = p->wt_n = (G.og + f.tiles - 1) / f.tiles;
+    f.n_pad = p->w_npad = round_up(f.n, 16);
     p->w_mtiles = (f.k_real + 1 + kTileM - 1) / kTileM;
     std::vector<MaskTap> t((size_t)p->w_mtiles * kTileM);
     for (size_t i = 0; i < t.size(); ++i) {
@@ -1516,30 +1664,41 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out) {
       splits = std::max(1, waves * ctx->sm_count / out_tiles);
       if ((p->w_kblocks_total + splits - 1) / splits <= kMaxChainKblocks) break;
     }
-    splits = std::min(splits, std::max(1, p->w_kblocks_total / 8));  // at least 8 k-blocks per CTA
+    splits = std::min(splits, std::max(1, p->w_kblocks_total / 3));  // at least 3 k-blocks per CTA
     p->w_kblocks_per_split = (p->w_kblocks_total + splits - 1) / splits;
     p->w_splits = (p->w_kblocks_total + p->w_kblocks_per_split - 1) / p->w_kblocks_per_split;
-    if (rc == CCT_OK)
+    p->w_small = !tensor_only && use_small_wgrad(n_pix, G.g * f.tiles, f.n, f.k_real);
+    if (p->w_small) {
+      // About one block per SM (two where a block keeps at least two chunks of pixels).
+      p->ws_rows = (f.k_real + 1 + kSwTile - 1) / kSwTile;
+      p->ws_cols = (f.n + kSwTile - 1) / kSwTile;
+      const int tiles = p->ws_rows * p->ws_cols * G.g * f.tiles;
+      const int want = std::max(1, ctx->sm_count * 2 / tiles);
+      p->ws_pix = std::max(kSwPix, round_up((n_pix + want - 1) / want, kSwPix));
+      p->w_splits = (n_pix + p->ws_pix - 1) / p->ws_pix;
+      if (rc == CCT_OK)
+        rc = dev_alloc(ctx, p, &p->w_partial, (size_t)p->w_splits * G.g * f.tiles * p->ws_rows * kSwTile * p->ws_cols * kSwTile);
+    } else if (rc == CCT_OK)
       rc = dev_alloc(ctx, p, &p->w_partial, (size_t)p->w_splits * G.g * f.tiles * p->w_mtiles * kTileM * f.n_pad);
   }
   // ---- weight gradient through the gather kernel (the default): tiles = splits x channel tiles x M-tiles
   // It needs one extra pass over dY (split into hi / lo, 12 bytes moved per element), which pays when every dY
   // element takes part in many multiply-adds: measured faster from CaffeNet conv2 (1200 lowered rows) upwards,
   // slower for AlexNet conv1 (363 rows), so short lowered matrices keep the shared-memory kernel above.
-  if (rc == CCT_OK && p->fwd.k_real >= 512) {
-    const GatherProblem& f = p->fwd;
+  if (rc == CCT_OK && p->fwd.k_real >= 512 && !p->w_small) {
     GatherProblem& w = p->wgp;
+    struct { int tiles, n, n_pad, k_real; } f = {p->wt_tiles, p->wt_n, p->w_npad, p->fwd.k_real};
     const int n_pix = G.B * G.m * G.m;
     const int kb_total = (n_pix + kBlockK - 1) / kBlockK;
     const int vgroups = G.g * f.tiles;
-    w.tiles = f.tiles; w.ch_tile = f.ch_tile; w.n = f.n; w.n_pad = f.n_pad;
+    w.tiles = f.tiles; w.ch_tile = f.n; w.n = f.n; w.n_pad = f.n_pad;
     w.k_real = n_pix;
     p->wg_mtiles = (f.k_real + kTileM - 1) / kTileM;  // no all-ones row here: the bias gradient comes from the dY pass
     const int base_tiles = vgroups * p->wg_mtiles;
     // Splits of the pixel range: all work units (base tiles x splits) cost the same, so the kernel's time is
     // (rounds of units over the resident CTAs) x (k-blocks per unit) - pick the split count that minimises it, plus the
     // traffic of the partial sums it creates (written once, read once by the reduction).  Chains stay bounded
-    // (kMaxChainKblocks) and units no shorter than 16 k-blocks.  A last round that fills at most half of the slots of
+    // (kMaxChainKblocks); a unit's set-up and epilogue cost about five k-blocks.  A last round that fills at most half of the slots of
     // the two-CTAs-per-SM shape costs about half a round: its CTAs have their SM's tensor pipe to themselves.
     {
       const bool two_per_sm = f.n_pad <= 128;  // the shape finish_problem() will pick for this accumulator width
@@ -1550,12 +1709,12 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out) {
       const int s_min = std::max(1, (kb_total + kMaxChainKblocks - 1) / kMaxChainKblocks);
       for (int s = s_min; s <= std::max(s_min, 8 * slots / base_tiles + 1); ++s) {
         const int kps = (kb_total + s - 1) / s;
-        if (kps < 16 && best_kps) break;
+        if (kps < 4 && best_kps) break;
         const int units = base_tiles * ((kb_total + kps - 1) / kps);
         const int tail = units % slots;
         const double rounds = units / slots + (tail == 0 ? 0.0 : (two_per_sm && 2 * tail <= slots) ? 0.55 : 1.0);
         const double reduce = 1.5 * units * (double)kTileM * f.n_pad * 8.0 / 6.5e6 / us_per_kblock;
-        const double cost = rounds * kps + reduce;
+        const double cost = rounds * (kps + 5) + reduce;
         if (!best_kps || cost < best - 1e-9) { best = cost; best_kps = kps; }
       }
       p->wg_kps = best_kps;
@@ -1597,7 +1756,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out) {
   }
   if (rc == CCT_OK) rc = set_smem(ctx, gather_conv_kernel<4>, kSmemLimit);
   if (rc == CCT_OK) rc = set_smem(ctx, gather_conv_kernel<2>, 113 * 1024);
-  if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->fwd.n_pad), kSmemLimit);
+  if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad), kSmemLimit);
   if (rc == CCT_OK && p->w_ts) rc = set_smem(ctx, wgrad_ts_kernel, kSmemLimit);
   if (rc != CCT_OK) {
     umma_plan_destroy(ctx, p);
@@ -1609,7 +1768,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, UmmaPlan** out) {
 
 void umma_plan_destroy(cct_ctx* ctx, UmmaPlan* p) {
   if (!p) return;
-  for (GatherProblem* gp : {&p->fwd, &p->dgr, &p->wgp}) { cudaFree(gp->taps); cudaFree(gp->cols); cudaFree(gp->w); }
+  for (GatherProblem* gp : {&p->fwd, &p->dgr, &p->wgp}) { cudaFree(gp->taps); cudaFree(gp->cols); cudaFree(gp->w); cudaFree(gp->partial); }
   cudaFree(p->wg_pix); cudaFree(p->wg_plane_sums);
   cudaFree(p->w_taps); cudaFree(p->w_partial);
   delete p;
@@ -1623,10 +1782,12 @@ void fill_common(GatherParams& P, const GatherProblem& gp, cct_ctx* ctx, int vgr
   P.taps = gp.taps; P.cols = gp.cols;
   P.tiles_per_group = gp.tiles;
   P.out_tile_channels = gp.ch_tile;
-  P.n = gp.n; P.n_pad = gp.n_pad; P.k_pad = gp.k_pad;
-  P.taps_smem = gp.taps_smem < 0 ? gp.k_pad : gp.taps_smem;
+  P.n = gp.n; P.n_pad = gp.n_pad; P.k_pad = gp.split_k ? gp.split_k : gp.k_pad;
+  P.cols_per_channel = gp.n / gp.ch_tile;
+  P.splits = gp.splits; P.partial = gp.partial; P.pix_pad = (int)gp.pix_pad;
+  P.taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k : gp.taps_smem;
   P.n_pix_tiles = (P.n_pix + kTileM - 1) / kTileM;
-  P.total_tiles = P.n_pix_tiles * vgroups;
+  P.total_tiles = P.n_pix_tiles * vgroups * gp.splits;
   P.a_stages = gp.a_stages; P.b_stages = gp.b_stages; P.acc_bufs = gp.acc_bufs;
   P.dual = gp.dual; P.acc_cols = gp.acc_cols; P.tmem_cols = gp.tmem_cols;
   P.n_bias = P.bias ? n_bias : 0;
@@ -1634,7 +1795,25 @@ void fill_common(GatherParams& P, const GatherProblem& gp, cct_ctx* ctx, int vgr
   P.status = ctx->status_dev;
 }
 
-// Persistent grid: one CTA per SM (4 producer sets) or two (2 sets).
+void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct) {
+  const int jr = small_rows(k);
+  P.row_groups = (P.n_out + jr - 1) / jr;
+  P.positions = P.batch * P.row_groups * P.n_out;
+  // Narrower channel tiles and more warps on the input channels until the SMs have about sixteen warps each.
+  const long long lots = (P.positions + 31) / 32, want = 16ll * ctx->launch_sms();
+  if (ct == 8 && lots * P.groups * ((P.co + 7) / 8) * std::min(16, std::max(1, P.ci / 2)) < want) ct = 4;
+  P.col_tiles = (P.co + ct - 1) / ct;
+  int warps = 4;
+  P.share = P.ci >= 4 && lots * P.groups * P.col_tiles < want;
+  while (P.share && warps < 16 && P.ci >= 4 * warps && lots * P.groups * P.col_tiles * warps < want &&
+         small_conv_smem(k, ct, P.ci, 2 * warps) <= 48 * 1024)
+    warps *= 2;
+  const int per_block = P.share ? 32 : 32 * warps;
+  launch_pdl(small_conv_pick(k, s, ct), dim3((P.positions + per_block - 1) / per_block, P.groups * P.col_tiles), dim3(32 * warps),
+             small_conv_smem(k, ct, P.ci, P.share ? warps : 0), ctx->stream, P);
+}
+
+// Persistent grid: one CTA per SM (4 producer sets) or two (2 sets); then the reduction over the splits, if any.
 void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp) {
   if (gp.sets == 2) {
     const int grid = std::min(P.total_tiles, 2 * ctx->launch_sms());
@@ -1642,6 +1821,12 @@ void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp)
   } else {
     const int grid = std::min(P.total_tiles, ctx->launch_sms());
     launch_pdl(gather_conv_kernel<4>, dim3(grid), dim3(gather_threads(4)), gp.smem, ctx->stream, P, gp.map);
+  }
+  if (P.splits > 1) {
+    const int vgroups = P.total_tiles / (P.n_pix_tiles * P.splits), cols = P.n_pix_tiles * vgroups * P.n > 32 * ctx->sm_count ? 8 : 1;
+    const int col_tiles = (P.n + cols - 1) / cols;
+    launch_pdl(cols == 8 ? gather_reduce_kernel<8> : gather_reduce_kernel<1>, dim3((P.n_pix + 127) / 128, vgroups * col_tiles), dim3(128),
+               0, ctx->stream, P, col_tiles);
   }
 }
 
@@ -1654,10 +1839,18 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
   GatherProblem& f = p->fwd;
   const int vgroups = G.g * f.tiles;
   const int B = batch > 0 ? batch : G.B;  // a leading slice of the batch (host-buffer calls pipeline over slices)
+  if (f.small_ct) {
+    SmallConv P{X, W, G.bias ? bias : nullptr, Y, B, G.n, G.m, G.p, G.Dg, G.og, G.g, 0, relu};
+    t->begin(0, ctx->stream);
+    launch_small_conv(ctx, P, G.k, G.s, f.small_ct);
+    t->end(0, ctx->stream);
+    CCT_CHECK_LAUNCH(ctx);
+    return CCT_OK;
+  }
   if (repack) {
     t->begin(4, ctx->stream);
-    launch_pdl(pack_fwd_kernel, dim3(pack_grid(ctx, f.w_half)), dim3(256), 0, ctx->stream, W, f.w, f.w + f.w_half, vgroups, f.tiles, G.og,
-                                                                     f.n, f.n_pad, f.k_real, f.k_pad);
+    launch_pdl(pack_fwd_kernel, pack_grid(vgroups * f.n_pad, f.k_pad), dim3(kPackThreads), 0, ctx->stream, W, f.w,
+               f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad);
     t->end(4, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   }
@@ -1696,12 +1889,12 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   const ConvGeom& G = p->G;
   if (p->wg_gather) {
-    const GatherProblem& f = p->fwd;
+    struct { int tiles, n, n_pad, k_real; } f = {p->wt_tiles, p->wt_n, p->w_npad, p->fwd.k_real};
     GatherProblem& w = p->wgp;
     const int vgroups = G.g * f.tiles, mm = G.m * G.m;
     t->begin(1, ctx->stream);
     launch_pdl(split_dy_kernel, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, 
-        dY, w.w, w.w + w.w_half, G.bias ? p->wg_plane_sums : nullptr, G.B * G.o, G.o, mm, G.og, f.ch_tile, f.tiles,
+        dY, w.w, w.w + w.w_half, G.bias ? p->wg_plane_sums : nullptr, G.B * G.o, G.o, mm, G.og, f.n, f.tiles,
         f.n_pad, w.map_k);
     CCT_CHECK_LAUNCH(ctx);
     GatherParams P{};
@@ -1724,7 +1917,7 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     t->end(2, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   } else {
-    const GatherProblem& f = p->fwd;
+    struct { int tiles, n, n_pad, k_real; } f = {p->wt_tiles, p->wt_n, p->w_npad, p->fwd.k_real};
     WgradParams P{};
     P.x = X; P.dy = dY; P.partial = p->w_partial; P.taps = p->w_taps;
     P.n_pix = G.B * G.m * G.m; P.m = G.m; P.mm = G.m * G.m; P.n = G.n; P.s = G.s; P.p = G.p; P.k = G.k;
@@ -1740,16 +1933,22 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     P.status = ctx->status_dev;
     const int vgroups = G.g * f.tiles;
     dim3 grid(p->w_mgroups, p->w_splits, vgroups);
+    int rows_pad = p->w_mtiles * kTileM;
     t->begin(1, ctx->stream);
-    if (p->w_ts)
+    if (p->w_small) {
+      P.n_pad = p->ws_cols * kSwTile;
+      rows_pad = p->ws_rows * kSwTile;
+      launch_pdl(small_wgrad_kernel, dim3(p->ws_rows * p->ws_cols * vgroups, p->w_splits), dim3(kSwThreads), 0, ctx->stream, P,
+                 rows_pad, p->ws_rows, p->ws_cols, p->ws_pix);
+    } else if (p->w_ts)
       launch_pdl(wgrad_ts_kernel, dim3(grid), dim3(kTsThreads), p->w_smem, ctx->stream, P);
     else
       launch_pdl(wgrad_pick(p->w_subs, f.n_pad), dim3(grid), dim3(kWgThreads), p->w_smem, ctx->stream, P);
     t->end(1, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
     t->begin(2, ctx->stream);
-    launch_wgrad_reduce(ctx, p->w_partial, dW, G.bias ? db : nullptr, p->w_splits, vgroups, f.tiles,
-                        p->w_mtiles * kTileM, f.n, f.n_pad, f.k_real, G.og);
+    launch_wgrad_reduce(ctx, p->w_partial, dW, G.bias ? db : nullptr, p->w_splits, vgroups, f.tiles, rows_pad, f.n, P.n_pad,
+                        f.k_real, G.og);
     t->end(2, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   }
@@ -1766,10 +1965,16 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
     GatherProblem& d = p->dgr;
     const int vgroups = G.g * d.tiles;
     t->begin(3, ctx->stream);
+    if (d.small_ct) {
+      SmallConv P{dY, W, nullptr, dX, B, G.m, G.n, G.k - 1 - G.p, G.og, G.Dg, G.g, 1, 0};
+      launch_small_conv(ctx, P, G.k, 1, d.small_ct);
+      t->end(3, ctx->stream);
+      CCT_CHECK_LAUNCH(ctx);
+      return CCT_OK;
+    }
     if (repack) {
-      launch_pdl(pack_dgrad_kernel, dim3(pack_grid(ctx, d.w_half)), dim3(256), 0, ctx->stream, W, d.w, d.w + d.w_half, vgroups, d.tiles, G.og,
-                                                                         G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n,
-                                                                         d.n_pad, d.k_real, d.k_pad);
+      launch_pdl(pack_dgrad_kernel, pack_grid(vgroups * d.n_pad, d.k_pad), dim3(kPackThreads), 0, ctx->stream, W, d.w,
+                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad);
       CCT_CHECK_LAUNCH(ctx);
     }
     GatherParams P{};
@@ -1855,7 +2060,7 @@ extern "C" int cct_conv_weight_grad_noalloc(cct_ctx* ctx, const cct_conv_desc* d
 
   // Same tiling rules as the plan-based path.
   const int tiles = channel_tiles(G.og, 1);
-  const int n_real = G.og / tiles, n_pad = round_up(n_real, 16);
+  const int n_real = (G.og + tiles - 1) / tiles, n_pad = round_up(n_real, 16);
   const int k_real = G.Dg * G.k * G.k;
   const int m_tiles = (k_real + 1 + kTileM - 1) / kTileM;
   int subs = 1;
