@@ -1431,6 +1431,7 @@ struct UmmaPlan {
   MaskTap* wg_pix = nullptr;       // per pixel: offset of the tap origin, taps out of bounds (padded to splits * kps * 32)
   float* wg_plane_sums = nullptr;  // [batch][channel] sums of dY for the bias gradient
   int wg_splits = 1, wg_kps = 1, wg_mtiles = 1;
+  void* memory = nullptr;          // everything above that lives on the device (PlanMemory)
   size_t bytes = 0;
 };
 
@@ -1445,20 +1446,36 @@ bool umma_supported(const ConvGeom& G) {
 
 namespace {
 
-template <class T>
-int dev_alloc(cct_ctx* ctx, UmmaPlan* p, T** ptr, size_t count) {
-  CCT_CUDA(ctx, cudaMalloc((void**)ptr, std::max<size_t>(count, 1) * sizeof(T)));
-  p->bytes += count * sizeof(T);
-  return CCT_OK;
-}
-
-template <class T>
-int upload(cct_ctx* ctx, UmmaPlan* p, T** dst, const std::vector<T>& host) {
-  int rc = dev_alloc(ctx, p, dst, host.size());
-  if (rc != CCT_OK) return rc;
-  CCT_CUDA(ctx, cudaMemcpy(*dst, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice));
-  return CCT_OK;
-}
+// The plan's device memory: everything a plan owns is one allocation (an allocation and its release cost some eighty
+// microseconds each, a plan has up to eleven buffers), laid out first and obtained at the end.
+struct PlanMemory {
+  struct Part { void** slot; size_t off; bool table; };
+  std::vector<Part> parts;
+  std::vector<unsigned char> tables;  // contents of the tables, in their layout
+  size_t room_bytes = 0;
+  static size_t aligned(size_t v) { return (v + 255) & ~(size_t)255; }
+  template <class T>
+  void table(T** slot, const std::vector<T>& host) {
+    const size_t at = tables.size();
+    tables.resize(aligned(at + host.size() * sizeof(T)));
+    std::copy_n(reinterpret_cast<const unsigned char*>(host.data()), host.size() * sizeof(T), tables.data() + at);
+    parts.push_back({(void**)slot, at, true});
+  }
+  template <class T>
+  void room(T** slot, size_t count) {
+    parts.push_back({(void**)slot, room_bytes, false});
+    room_bytes = aligned(room_bytes + count * sizeof(T));
+  }
+  int obtain(cct_ctx* ctx, void** memory, size_t* bytes) {
+    unsigned char* base = nullptr;
+    CCT_CUDA(ctx, cudaMalloc((void**)&base, tables.size() + room_bytes));
+    *memory = base;
+    *bytes = tables.size() + room_bytes;
+    CCT_CUDA(ctx, cudaMemcpy(base, tables.data(), tables.size(), cudaMemcpyHostToDevice));
+    for (const Part& p : parts) *p.slot = base + (p.table ? 0 : tables.size()) + p.off;
+    return CCT_OK;
+  }
+};
 
 template <class K>
 int set_smem(cct_ctx* ctx, K kernel, size_t bytes) {
@@ -1507,8 +1524,8 @@ bool use_small_wgrad(long long pixels, int vgroups, int n, int k_real) {
   return flops <= kSmallWgradFlops;
 }
 
-// Tensor-memory and shared-memory budget of a gather problem, packed-weight buffer and its tensor map.
-int finish_problem(cct_ctx* ctx, UmmaPlan* p, GatherProblem& gp, int vgroups, int n_bias) {
+// Tensor-memory and shared-memory budget of a gather problem, room for its packed operand.
+void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias) {
   // Tensor memory (512 columns) = accumulator buffers + A stages of 64 columns.  Narrow problems run "dual" (see the
   // MMA loop): their accumulator is 2*n_pad wide.  Two accumulator buffers let the epilogue overlap the next tile.
   const int taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k : gp.taps_smem;
@@ -1526,9 +1543,12 @@ int finish_problem(cct_ctx* ctx, UmmaPlan* p, GatherProblem& gp, int vgroups, in
   }
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
   gp.w_half = (size_t)vgroups * gp.n_pad * map_k;
-  int rc = dev_alloc(ctx, p, &gp.w, 2 * gp.w_half);
-  if (rc == CCT_OK && gp.splits > 1) rc = dev_alloc(ctx, p, &gp.partial, (size_t)gp.splits * vgroups * gp.n_pad * gp.pix_pad);
-  if (rc != CCT_OK) return rc;
+  mem.room(&gp.w, 2 * gp.w_half);
+}
+
+// The tensor map of a gather problem's packed operand.
+int encode_problem(cct_ctx* ctx, GatherProblem& gp, int vgroups) {
+  const size_t map_k = gp.map_k ? gp.map_k : (size_t)gp.k_pad;
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) {
     ctx->last_error = "cuTensorMapEncodeTiled is not available from this driver";
@@ -1553,7 +1573,8 @@ int finish_problem(cct_ctx* ctx, UmmaPlan* p, GatherProblem& gp, int vgroups, in
 int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan** out) {
   UmmaPlan* p = new UmmaPlan();
   p->G = G;
-  int rc = CCT_OK;
+  PlanMemory mem;
+  size_t sums = 0;  // floats of the split sums: one buffer for all passes, none needs its sums after its own reduction
   const int kk = G.k * G.k;
   // ---- forward: accumulator columns = output channels of a tile, reduction = (d, kr, kc)
   {
@@ -1577,14 +1598,17 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     }
     std::vector<ColEnt> c(f.n_pad);
     for (int j = 0; j < f.n_pad; ++j) c[j] = ColEnt{j * G.m * G.m, 0, 0};
-    rc = upload(ctx, p, &f.taps, t);
-    if (rc == CCT_OK) rc = upload(ctx, p, &f.cols, c);
     if (!tensor_only) f.small_ct = use_small_conv(G.k, G.s, (long long)G.B * G.m * G.m, G.g, G.Dg, G.og);
-    if (rc == CCT_OK && !f.small_ct) rc = finish_problem(ctx, p, f, G.g * f.tiles, G.bias ? G.o : 0);
+    if (!f.small_ct) {
+      mem.table(&f.taps, t);
+      mem.table(&f.cols, c);
+      finish_problem(mem, f, G.g * f.tiles, G.bias ? G.o : 0);
+      if (f.splits > 1) sums = std::max(sums, (size_t)f.splits * G.g * f.tiles * f.n_pad * f.pix_pad);
+    }
   }
   // ---- data gradient as a stride-1 gather over dY: one "super pixel" = an s x s block of input pixels; accumulator
   //      columns = (d, py, px), reduction = (oc, jy, jx) with jy, jx < ceil(k/s); depth-to-space in the epilogue.
-  if (rc == CCT_OK) {
+  {
     GatherProblem& d = p->dgr;
     const int ss = G.s * G.s;
     p->dgr_taps = (G.k + G.s - 1) / G.s;
@@ -1614,31 +1638,22 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       const int dl = j / ss, py = (j / G.s) % G.s, px = j % G.s;
       c[j] = ColEnt{dl * G.n * G.n + py * G.n + px, (short)py, (short)px};
     }
-    rc = upload(ctx, p, &d.taps, t);
-    if (rc == CCT_OK) rc = upload(ctx, p, &d.cols, c);
     if (!tensor_only && G.s == 1) d.small_ct = use_small_conv(G.k, 1, (long long)G.B * G.n * G.n, G.g, G.og, G.Dg);
-    if (rc == CCT_OK && !d.small_ct) rc = finish_problem(ctx, p, d, G.g * d.tiles, 0);
+    if (!d.small_ct) {
+      mem.table(&d.taps, t);
+      mem.table(&d.cols, c);
+      finish_problem(mem, d, G.g * d.tiles, 0);
+      if (d.splits > 1) sums = std::max(sums, (size_t)d.splits * G.g * d.tiles * d.n_pad * d.pix_pad);
+    }
   }
   // ---- weight gradient: rows = (d, kr, kc) plus the all-ones row, columns = output channels of a tile
-  if (rc == CCT_OK) {
+  {
     GatherProblem f;  // the widest channel tiles, whatever the forward pass takes
     f.k_real = p->fwd.k_real;
     f.tiles = p->wt_tiles = channel_tiles(G.og, 1);
     f.n = p->wt_n = (G.og + f.tiles - 1) / f.tiles;
     f.n_pad = p->w_npad = round_up(f.n, 16);
     p->w_mtiles = (f.k_real + 1 + kTileM - 1) / kTileM;
-    std::vector<MaskTap> t((size_t)p->w_mtiles * kTileM);
-    for (size_t i = 0; i < t.size(); ++i) {
-      if ((int)i < f.k_real) {
-        const int d = (int)i / kk, kr = ((int)i / G.k) % G.k, kc = (int)i % G.k;
-        t[i] = MaskTap{d * G.n * G.n + kr * G.n + kc, kWgValidBit | (1u << kr) | (1u << (16 + kc))};
-      } else if ((int)i == f.k_real) {
-        t[i] = MaskTap{0, kWgOnesBits};
-      } else {
-        t[i] = MaskTap{0, kWgPadBit};
-      }
-    }
-    rc = upload(ctx, p, &p->w_taps, t);
     // M-tiles per CTA: as many as leave room for two stages in shared memory (and whose accumulators fit in tensor
     // memory); the dY tile of a k-block is staged once for all of them.
     int subs = 1;
@@ -1676,16 +1691,31 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       const int want = std::max(1, ctx->sm_count * 2 / tiles);
       p->ws_pix = std::max(kSwPix, round_up((n_pix + want - 1) / want, kSwPix));
       p->w_splits = (n_pix + p->ws_pix - 1) / p->ws_pix;
-      if (rc == CCT_OK)
-        rc = dev_alloc(ctx, p, &p->w_partial, (size_t)p->w_splits * G.g * f.tiles * p->ws_rows * kSwTile * p->ws_cols * kSwTile);
-    } else if (rc == CCT_OK)
-      rc = dev_alloc(ctx, p, &p->w_partial, (size_t)p->w_splits * G.g * f.tiles * p->w_mtiles * kTileM * f.n_pad);
+      sums = std::max(sums, (size_t)p->w_splits * G.g * f.tiles * p->ws_rows * kSwTile * p->ws_cols * kSwTile);
+    }
+    p->wg_gather = !p->w_small && f.k_real >= 512;  // see below
+    if (!p->w_small && !p->wg_gather)
+      sums = std::max(sums, (size_t)p->w_splits * G.g * f.tiles * p->w_mtiles * kTileM * f.n_pad);
+    if (!p->wg_gather) {
+      std::vector<MaskTap> t((size_t)p->w_mtiles * kTileM);
+      for (size_t i = 0; i < t.size(); ++i) {
+        if ((int)i < f.k_real) {
+          const int d = (int)i / kk, kr = ((int)i / G.k) % G.k, kc = (int)i % G.k;
+          t[i] = MaskTap{d * G.n * G.n + kr * G.n + kc, kWgValidBit | (1u << kr) | (1u << (16 + kc))};
+        } else if ((int)i == f.k_real) {
+          t[i] = MaskTap{0, kWgOnesBits};
+        } else {
+          t[i] = MaskTap{0, kWgPadBit};
+        }
+      }
+      mem.table(&p->w_taps, t);
+    }
   }
   // ---- weight gradient through the gather kernel (the default): tiles = splits x channel tiles x M-tiles
   // It needs one extra pass over dY (split into hi / lo, 12 bytes moved per element), which pays when every dY
   // element takes part in many multiply-adds: measured faster from CaffeNet conv2 (1200 lowered rows) upwards,
   // slower for AlexNet conv1 (363 rows), so short lowered matrices keep the shared-memory kernel above.
-  if (rc == CCT_OK && p->fwd.k_real >= 512 && !p->w_small) {
+  if (p->wg_gather) {
     GatherProblem& w = p->wgp;
     struct { int tiles, n, n_pad, k_real; } f = {p->wt_tiles, p->wt_n, p->w_npad, p->fwd.k_real};
     const int n_pix = G.B * G.m * G.m;
@@ -1723,36 +1753,35 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     w.k_pad = p->wg_kps * kBlockK;
     w.taps_smem = 0;
     w.map_k = (size_t)kb_total * kBlockK;
-    std::vector<MaskTap> t((size_t)p->wg_splits * p->wg_kps * kBlockK);
-    for (size_t i = 0; i < t.size(); ++i) {
-      if ((long long)i < n_pix) {
-        const int b = (int)(i / (G.m * G.m)), r = (int)(i % (G.m * G.m));
-        const int iy0 = (r / G.m) * G.s - G.p, ix0 = (r % G.m) * G.s - G.p;
-        uint32_t valid = 0;
-        for (int a = 0; a < G.k; ++a) {
-          if (iy0 + a >= 0 && iy0 + a < G.n) valid |= 1u << a;
-          if (ix0 + a >= 0 && ix0 + a < G.n) valid |= 1u << (16 + a);
-        }
-        const long long off = (long long)b * G.D * G.n * G.n + (long long)iy0 * G.n + ix0;
-        t[i] = MaskTap{(int)off, ~valid};
-      } else {
-        t[i] = MaskTap{0, 0xffffffffu};
+    // Per-pixel table: where the pixel's window starts, and which of its rows and columns lie outside the plane.
+    std::vector<uint32_t> outside(G.m);  // the same for rows and columns: bit a = window row a of output row r is outside
+    for (int r = 0; r < G.m; ++r)
+      for (int a = 0; a < kMaxTapsPerAxis; ++a)
+        if (a >= G.k || r * G.s - G.p + a < 0 || r * G.s - G.p + a >= G.n) outside[r] |= 1u << a;
+    std::vector<MaskTap> t((size_t)p->wg_splits * p->wg_kps * kBlockK, MaskTap{0, 0xffffffffu});
+    size_t i = 0;
+    for (int b = 0; b < G.B; ++b)
+      for (int r = 0; r < G.m; ++r) {
+        const int row = (int)((long long)b * G.D * G.n * G.n) + (r * G.s - G.p) * G.n - G.p;
+        for (int q = 0; q < G.m; ++q, ++i) t[i] = MaskTap{row + q * G.s, outside[r] | (outside[q] << 16) | 0x80008000u};
       }
-    }
-    rc = upload(ctx, p, &p->wg_pix, t);
-    if (rc == CCT_OK) rc = finish_problem(ctx, p, w, vgroups, 0);
-    if (rc == CCT_OK && cudaMemsetAsync(w.w, 0, 2 * w.w_half * sizeof(float), ctx->stream) != cudaSuccess) {  // padded channel rows stay zero
+    mem.table(&p->wg_pix, t);
+    finish_problem(mem, w, vgroups, 0);
+    if (G.bias) mem.room(&p->wg_plane_sums, (size_t)G.B * G.o);
+    sums = std::max(sums, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
+  }
+  float* sum_memory = nullptr;
+  mem.room(&sum_memory, sums);
+  int rc = mem.obtain(ctx, &p->memory, &p->bytes);
+  p->fwd.partial = p->dgr.partial = p->w_partial = sum_memory;
+  if (rc == CCT_OK && p->fwd.w) rc = encode_problem(ctx, p->fwd, G.g * p->fwd.tiles);
+  if (rc == CCT_OK && p->dgr.w) rc = encode_problem(ctx, p->dgr, G.g * p->dgr.tiles);
+  if (rc == CCT_OK && p->wg_gather) {
+    rc = encode_problem(ctx, p->wgp, G.g * p->wt_tiles);
+    if (rc == CCT_OK && cudaMemsetAsync(p->wgp.w, 0, 2 * p->wgp.w_half * sizeof(float), ctx->stream) != cudaSuccess) {  // padded channel rows stay zero
       ctx->last_error = "cudaMemsetAsync of the pre-split dY buffer failed";
       rc = CCT_ERR_CUDA;
     }
-    if (rc == CCT_OK && G.bias) rc = dev_alloc(ctx, p, &p->wg_plane_sums, (size_t)G.B * G.o);
-    if (rc == CCT_OK) {
-      cudaFree(p->w_partial);  // sized for the other kernel's split count
-      p->bytes -= (size_t)p->w_splits * vgroups * p->w_mtiles * kTileM * f.n_pad * sizeof(float);
-      p->w_partial = nullptr;
-      rc = dev_alloc(ctx, p, &p->w_partial, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
-    }
-    p->wg_gather = rc == CCT_OK;
   }
   if (rc == CCT_OK) rc = set_smem(ctx, gather_conv_kernel<4>, kSmemLimit);
   if (rc == CCT_OK) rc = set_smem(ctx, gather_conv_kernel<2>, 113 * 1024);
@@ -1768,9 +1797,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
 
 void umma_plan_destroy(cct_ctx* ctx, UmmaPlan* p) {
   if (!p) return;
-  for (GatherProblem* gp : {&p->fwd, &p->dgr, &p->wgp}) { cudaFree(gp->taps); cudaFree(gp->cols); cudaFree(gp->w); cudaFree(gp->partial); }
-  cudaFree(p->wg_pix); cudaFree(p->wg_plane_sums);
-  cudaFree(p->w_taps); cudaFree(p->w_partial);
+  cudaFree(p->memory);
   delete p;
 }
 
