@@ -221,8 +221,8 @@ class ConvolutionBridge:
 class FullyConnectedBridge:
     """The reference's FullyConnectedBridge (src/bridges/FullyConnectedBridge_impl.hxx:171-235, 257-330): Y = X W^T + b
     over the flattened input, weight layout [o][d][r][c].  Runs on the fully connected plan of the C ABI (tensor-core
-    GEMMs that read X, W and dY in place); layers whose feature counts are not multiples of 4, and
-    algo=ALGO_SIMT_FP32, run as a 1x1 convolution over the input viewed as D*R*C channels of one pixel instead.
+    GEMMs that read X, W and dY in place); algo=ALGO_SIMT_FP32 runs as a 1x1 convolution over the input viewed as D*R*C
+    channels of one pixel instead.
     The output layer is B x num_output x 1 x 1.
 
     Fusion switches (the bridges around the layer in CaffeNet): fuse_relu clamps the output at 0; dropout_mask /
@@ -247,9 +247,7 @@ class FullyConnectedBridge:
         self.dropout_mask, self.dropout_scale = None, 1.0
         self.input_dropout_mask, self.input_dropout_scale = None, 1.0
         self.plan, self._conv = None, None
-        use_plan = algo == capi.ALGO_UMMA_3XTF32 or (algo == capi.ALGO_AUTO and self.in_features % 4 == 0 and
-                                                      self.oD % 4 == 0)
-        if use_plan:
+        if algo != capi.ALGO_SIMT_FP32:
             plan = C.c_void_p()
             capi.check(self.lib.cct_fc_plan_create(self.ctx.h, self.iB, self.in_features, self.oD, int(bias_term),
                                                    C.byref(plan)), "cct_fc_plan_create", self.ctx.h)

@@ -29,33 +29,38 @@ namespace {
 
 constexpr int kFcEpiWarps = 4, kFcTmaWarp = 4, kFcMmaWarp = 5, kFcXformWarp0 = 6, kFcXformWarps = 8;
 constexpr int kFcThreads = (kFcXformWarp0 + kFcXformWarps) * 32;  // 448
-constexpr int kFcMaxStages = 4;
-constexpr int kFcMaxChainKblocks = 96;  // k-blocks of 32 per partial sum: the tensor core's fp32 accumulate truncates
+constexpr int kFcRing = 4;                    // deepest ring of any kind; the lo and done barriers are a ring of four
+constexpr int kFcMaxChainKblocks = 96;        // k-blocks of 32 per partial sum: the tensor core's fp32 accumulate truncates
 constexpr uint32_t kFcATile = kTileM * 128u;  // bytes of one 128 x 32 fp32 tile
+constexpr uint32_t kFcStoreTile = 32u * 16u * 4u;  // 16 columns x 32 lanes on their way out
 
 struct FcGemmParams {
-  float* out;               // out[split * split_stride + n * ld_out + m]
-  long long ld_out, split_stride;
   int M, N;                 // extents of the output (m fastest in memory)
   int n_pad;                // accumulator columns per tile: N rounded up (a multiple of 32 for MN-major B)
+  int dual, acc_cols;       // dual: B's lo tile sits right behind the raw one and one MMA of width 2 * n_pad covers both
   int m_tiles, n_tiles, splits, kblocks_total, kblocks_per_split;
   int a_mn, b_mn;           // 1: the operand is MN-major (row index contiguous in memory)
-  int a_tmem;               // 1: the A operand is split into tensor memory (hi and lo), the MMAs read it from there
-  int stages, acc_bufs;
+  int raw_slots, lo_slots, a_slots, acc_bufs, store_bufs;
   int tmem_cols;            // tensor-memory columns the CTA allocates: 512, or 256 when two CTAs share an SM
+  float* direct;            // non-null: plain stores to direct[n * ld_direct + m] (an output no tensor map describes)
+  long long ld_direct;
   int* status;
 };
 
+// Raw ring (A tile and B tile as TMA delivers them; for `dual` B's lo tile behind them), lo ring (B's lo tiles), the tiles
+// on their way out, barriers.
 struct FcSmem {
-  uint32_t b_tile_bytes, b_off, stage_bytes, bars_off, total;
+  uint32_t b_tile_bytes, raw_bytes, lo_off, lo_stride, store_off, bars_off, total;
 };
-__host__ __device__ inline FcSmem fc_smem(int n_pad, int stages, int a_tmem) {
+__host__ __device__ inline FcSmem fc_smem(int n_pad, int dual, int raw_slots, int lo_slots, int store_bufs) {
   FcSmem L;
   L.b_tile_bytes = (uint32_t)n_pad * 128u;
-  L.b_off = (a_tmem ? 1u : 2u) * kFcATile;            // A raw, (A lo unless A's halves live in tensor memory,)
-  L.stage_bytes = L.b_off + 2u * L.b_tile_bytes;      // B raw, B lo
-  L.bars_off = (uint32_t)stages * L.stage_bytes;
-  L.total = L.bars_off + 8u * (3 * kFcMaxStages + 4) + 16u;
+  L.raw_bytes = kFcATile + (dual ? 2u : 1u) * L.b_tile_bytes;
+  L.lo_off = dual ? kFcATile + L.b_tile_bytes : (uint32_t)raw_slots * L.raw_bytes;
+  L.lo_stride = dual ? L.raw_bytes : L.b_tile_bytes;
+  L.store_off = (uint32_t)raw_slots * L.raw_bytes + (dual ? 0u : (uint32_t)lo_slots * L.b_tile_bytes);
+  L.bars_off = L.store_off + (uint32_t)(kFcEpiWarps * store_bufs) * kFcStoreTile;
+  L.total = L.bars_off + 8u * (3 * kFcRing + 4) + 16u;
   return L;
 }
 
@@ -67,25 +72,41 @@ __device__ __forceinline__ uint64_t make_desc_mn(uint32_t smem_addr) {
          (1ull << 46) | (1ull << 61);
 }
 
+__device__ __forceinline__ void fc_store_3d(const void* tmap, uint32_t src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(tmap), "r"(x), "r"(y), "r"(z),
+               "r"(src)
+               : "memory");
+}
+
+// What bounds it: at batch 256 the tensor pipe (12 MMAs of N / 2 cycles per k-block), at small batches the stream of W (or,
+// for the weight gradient, of dW) - so the same roles in two shapes.
+//   N > 128 columns: one CTA per SM, the whole batch in one accumulator, so that a weight tile is split into tensor memory
+//   once (two CTAs with half the batch each split it twice and waited for it: 61 % of the tensor pipe, now see below).
+//   N <= 128: two CTAs per SM, 256 tensor-memory columns each.
+// K-block i (running index) uses raw slot i % raw_slots, lo slot i % lo_slots, tensor-memory slot i % a_slots; the raw slot,
+// which is also the hi operand, is held for TMA + transform + MMA, the other two only from transform to MMA, so the raw ring
+// is the deeper one.  raw[slot] completes when the TMA bytes have landed, lo[i % 4] when the transform warps are through,
+// done[i % 4] when the block's MMAs have finished, which frees all three slots (nobody waits more than four blocks back).
+// The epilogue turns sixteen accumulator columns at a time into a 16 x 32 tile in shared memory (one conflict-free store per
+// column) that a TMA store takes out, clipping it at the edges: per-lane global stores with their addresses and bounds cost
+// about ten instructions each and made the weight gradient of small batches instruction-bound (fc6, batch 32: 70 us, 2.1 TB/s).
 __global__ void __launch_bounds__(kFcThreads, 2)
     fc_gemm_kernel(const __grid_constant__ FcGemmParams P, const __grid_constant__ CUtensorMap a_map,
-                   const __grid_constant__ CUtensorMap b_map) {
+                   const __grid_constant__ CUtensorMap b_map, const __grid_constant__ CUtensorMap out_map) {
   pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const FcSmem L = fc_smem(P.n_pad, P.stages, P.a_tmem);
+  const FcSmem L = fc_smem(P.n_pad, P.dual, P.raw_slots, P.lo_slots, P.store_bufs);
   const uint32_t bars = base + L.bars_off;
-  // raw[s]: the stage's TMA bytes have landed; lo[s]: the transform warps have written the lo tiles; empty[s]: the
-  // stage's MMAs have finished (tcgen05.commit), the TMA thread may refill it.
-  const uint32_t raw_bar = bars, lo_bar = raw_bar + 8u * kFcMaxStages, empty_bar = lo_bar + 8u * kFcMaxStages,
-                 acc_full = empty_bar + 8u * kFcMaxStages, acc_empty = acc_full + 16u, tmem_slot = acc_empty + 16u;
+  const uint32_t raw_bar = bars, lo_bar = raw_bar + 8u * kFcRing, done_bar = lo_bar + 8u * kFcRing,
+                 acc_full = done_bar + 8u * kFcRing, acc_empty = acc_full + 16u, tmem_slot = acc_empty + 16u;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int s = 0; s < kFcMaxStages; ++s) {
+    for (int s = 0; s < kFcRing; ++s) {
       mbar_init(raw_bar + 8u * s, 1);
       mbar_init(lo_bar + 8u * s, kFcXformWarps);
-      mbar_init(empty_bar + 8u * s, 1);
+      mbar_init(done_bar + 8u * s, 1);
     }
     for (int b = 0; b < 2; ++b) { mbar_init(acc_full + 8u * b, 1); mbar_init(acc_empty + 8u * b, kFcEpiWarps); }
     fence_mbar_init();
@@ -96,7 +117,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-  const uint32_t a_col0 = (uint32_t)(P.acc_bufs * P.n_pad);  // A stages (64 columns each) behind the accumulators
+  const uint32_t a_col0 = (uint32_t)(P.acc_bufs * P.acc_cols);  // A slots (64 columns: 32 hi + 32 lo) behind the accumulators
   const int total_tiles = P.m_tiles * P.n_tiles * P.splits;
   bool failed = false;
   // tile t -> (split, n-tile, m-tile), m-tile fastest; k-blocks [kb0, kb1)
@@ -108,18 +129,23 @@ __global__ void __launch_bounds__(kFcThreads, 2)
     kb0 = split * P.kblocks_per_split;
     kb1 = min(P.kblocks_total, kb0 + P.kblocks_per_split);
   };
+  // the MMAs of the k-block `back` blocks before block i have finished
+  auto wait_done = [&](int i, int back, int code) {
+    const int j = i - back;
+    if (j >= 0) mbar_wait<false>(done_bar + 8u * (j & 3), (uint32_t)(j >> 2) & 1u, failed, P.status, code);
+  };
 
   if (warp == kFcTmaWarp) {
     if (lane == 0) {
       Ring ring;
+      int i = 0;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
         int mt, nt, split, kb0, kb1;
         tile_of(t, mt, nt, split, kb0, kb1);
-        for (int kb = kb0; kb < kb1; ++kb, ring.advance(P.stages)) {
-          const int s = ring.idx;
-          if (ring.use > 0) mbar_wait<false>(empty_bar + 8u * s, (uint32_t)(ring.use - 1) & 1u, failed, P.status, 0x1100);
-          const uint32_t st = base + (uint32_t)s * L.stage_bytes, a_raw = st, b_raw = st + L.b_off;
-          const uint32_t bar = raw_bar + 8u * s;
+        for (int kb = kb0; kb < kb1; ++kb, ++i, ring.advance(P.raw_slots)) {
+          wait_done(i, P.raw_slots, 0x1100);
+          const uint32_t a_raw = base + (uint32_t)ring.idx * L.raw_bytes, b_raw = a_raw + kFcATile;
+          const uint32_t bar = raw_bar + 8u * ring.idx;
           mbar_expect_tx(bar, kFcATile + L.b_tile_bytes);
           if (P.a_mn) {
 #pragma unroll
@@ -138,187 +164,222 @@ __global__ void __launch_bounds__(kFcThreads, 2)
     }
   } else if (warp == kFcMmaWarp) {
     if (lane == 0) {
-      const uint32_t idesc = make_idesc(P.n_pad) | (P.a_mn ? 1u << 15 : 0u) | (P.b_mn ? 1u << 16 : 0u);
-      const uint32_t idesc_ts = make_idesc(P.n_pad) | (P.b_mn ? 1u << 16 : 0u);  // A from tensor memory: lanes x K
-      Ring ring;
-      int tile_iter = 0;
+      const uint32_t idesc = make_idesc(P.acc_cols) | (P.b_mn ? 1u << 16 : 0u);  // A from tensor memory: lanes x K
+      Ring raw, lo, ta;
+      int i = 0, tile_iter = 0;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_iter) {
         int mt, nt, split, kb0, kb1;
         tile_of(t, mt, nt, split, kb0, kb1);
         const int buf = tile_iter & (P.acc_bufs - 1), use = tile_iter >> (P.acc_bufs - 1);
         if (use > 0) mbar_wait<false>(acc_empty + 8u * buf, (uint32_t)(use - 1) & 1u, failed, P.status, 0x1200);
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * P.n_pad);
-        for (int kb = kb0; kb < kb1; ++kb, ring.advance(P.stages)) {
-          const int s = ring.idx;
-          mbar_wait<false>(raw_bar + 8u * s, (uint32_t)ring.use & 1u, failed, P.status, 0x1300);
-          mbar_wait<false>(lo_bar + 8u * s, (uint32_t)ring.use & 1u, failed, P.status, 0x1400);
+        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * P.acc_cols);
+        for (int kb = kb0; kb < kb1; ++kb, ++i) {
+          mbar_wait<false>(raw_bar + 8u * raw.idx, (uint32_t)raw.use & 1u, failed, P.status, 0x1300);
+          mbar_wait<false>(lo_bar + 8u * (i & 3), (uint32_t)(i >> 2) & 1u, failed, P.status, 0x1400);
           tc_fence_after();
-          const uint32_t st = base + (uint32_t)s * L.stage_bytes;
-          const uint32_t a_raw = st, a_lo = st + kFcATile, b_raw = st + L.b_off, b_lo = b_raw + L.b_tile_bytes;
-          if (P.a_tmem) {
-            const uint32_t t_hi = tmem_base + a_col0 + (uint32_t)(s * 64), t_lo = t_hi + 32u;
-#pragma unroll
-            for (int j = 0; j < kBlockK / 8; ++j) {
-              const uint64_t bh = P.b_mn ? make_desc_mn(b_raw + j * 1024u) : make_desc(b_raw) + (uint64_t)(j * 2);
-              const uint64_t bl = P.b_mn ? make_desc_mn(b_lo + j * 1024u) : make_desc(b_lo) + (uint64_t)(j * 2);
-              umma_tf32_ts(d_tmem, t_lo + (uint32_t)(j * 8), bh, idesc_ts, (kb == kb0 && j == 0) ? 0u : 1u);
-              umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bl, idesc_ts, 1u);
-              umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bh, idesc_ts, 1u);
-            }
-            umma_commit(empty_bar + 8u * s);
-            continue;
-          }
+          const uint32_t b_raw = base + (uint32_t)raw.idx * L.raw_bytes + kFcATile;
+          const uint32_t b_lo = base + L.lo_off + (uint32_t)lo.idx * L.lo_stride;
+          const uint32_t t_hi = tmem_base + a_col0 + (uint32_t)(ta.idx * 64), t_lo = t_hi + 32u;
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
             // K-major: 8 reduction indices = 32 bytes along the swizzled row; MN-major: 8 rows of 128 bytes
-            const uint64_t ah = P.a_mn ? make_desc_mn(a_raw + j * 1024u) : make_desc(a_raw) + (uint64_t)(j * 2);
-            const uint64_t al = P.a_mn ? make_desc_mn(a_lo + j * 1024u) : make_desc(a_lo) + (uint64_t)(j * 2);
             const uint64_t bh = P.b_mn ? make_desc_mn(b_raw + j * 1024u) : make_desc(b_raw) + (uint64_t)(j * 2);
-            const uint64_t bl = P.b_mn ? make_desc_mn(b_lo + j * 1024u) : make_desc(b_lo) + (uint64_t)(j * 2);
-            umma_tf32_ss(d_tmem, al, bh, idesc, (kb == kb0 && j == 0) ? 0u : 1u);
-            umma_tf32_ss(d_tmem, ah, bl, idesc, 1u);
-            umma_tf32_ss(d_tmem, ah, bh, idesc, 1u);
+            const uint32_t first = (kb == kb0 && j == 0) ? 0u : 1u;
+            umma_tf32_ts(d_tmem, t_lo + (uint32_t)(j * 8), bh, idesc, first);
+            if (!P.dual) {
+              const uint64_t bl = P.b_mn ? make_desc_mn(b_lo + j * 1024u) : make_desc(b_lo) + (uint64_t)(j * 2);
+              umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bl, idesc, 1u);
+            }
+            umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bh, idesc, 1u);
           }
-          umma_commit(empty_bar + 8u * s);
+          umma_commit(done_bar + 8u * (i & 3));
+          raw.advance(P.raw_slots);
+          lo.advance(P.lo_slots);
+          ta.advance(P.a_slots);
         }
         umma_commit(acc_full + 8u * buf);
       }
     }
   } else if (warp >= kFcXformWarp0) {
-    // ---- lo = x - (x with the low 13 mantissa bits cleared), element-wise over the stage's two raw tiles
+    // ---- A: hi and lo into tensor memory; B: lo = x - (x with the low 13 mantissa bits cleared), element-wise
     const int xt = tid - kFcXformWarp0 * 32;
     constexpr int kXThreads = kFcXformWarps * 32;
-    const int a_vec = kFcATile / 16, b_vec = (int)(L.b_tile_bytes / 16);
-    Ring ring;
+    const int b_vec = (int)(L.b_tile_bytes / 16);
+    const int q = warp & 3, half = (warp - kFcXformWarp0) >> 2;
+    const int m = q * 32 + lane;  // row of the tile = tensor-memory lane; this thread takes half of the k-block's 32 indices
+    const int back = min(P.lo_slots, P.a_slots);
+    Ring raw, lo, ta;
+    int i = 0;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
       int mt, nt, split, kb0, kb1;
       tile_of(t, mt, nt, split, kb0, kb1);
-      for (int kb = kb0; kb < kb1; ++kb, ring.advance(P.stages)) {
-        const int s = ring.idx;
-        mbar_wait(raw_bar + 8u * s, (uint32_t)ring.use & 1u, failed, P.status, 0x1500);
-        uint8_t* st = base_ptr + (size_t)s * L.stage_bytes;
-        if (P.a_tmem) {
-          // The stage's tensor-memory columns are free: the TMA thread refilled the stage only after the MMAs that read
-          // them had completed (empty barrier), and this thread has just seen that refill land.
-          tc_fence_after();
-          // A: thread = (row m of the tile = tensor-memory lane, half of the k-block's 32 reduction indices).  Its 16
-          // values come out of the swizzled tile the TMA wrote; hi and lo go to the stage's 64 tensor-memory columns.
-          const int q = warp & 3, half = (warp - kFcXformWarp0) >> 2;
-          const int m = q * 32 + lane;
-          float x[16];
-          if (P.a_mn) {
-            // 32 x 32 boxes, row = reduction index (128 bytes), 32-byte chunks XORed with the row index mod 4
-            const uint8_t* box = st + (size_t)(m >> 5) * 4096u;
+      for (int kb = kb0; kb < kb1; ++kb, ++i) {
+        mbar_wait(raw_bar + 8u * raw.idx, (uint32_t)raw.use & 1u, failed, P.status, 0x1500);
+        if (i >= back) mbar_wait(done_bar + 8u * ((i - back) & 3), (uint32_t)((i - back) >> 2) & 1u, failed, P.status, 0x1510);
+        tc_fence_after();
+        const uint8_t* st = base_ptr + (size_t)raw.idx * L.raw_bytes;
+        float x[16];
+        if (P.a_mn) {
+          // 32 x 32 boxes, row = reduction index (128 bytes), 32-byte chunks XORed with the row index mod 4
+          const uint8_t* box = st + (size_t)(m >> 5) * 4096u;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const uint32_t k = (uint32_t)(half * 16 + i);
-              const uint32_t off = k * 128u + (uint32_t)(m & 31) * 4u;
-              x[i] = *reinterpret_cast<const float*>(box + (off ^ ((k & 3u) << 5)));
-            }
-          } else {
-            // rows of 128 bytes, 16-byte chunks XORed with the row index mod 8
-            const uint8_t* rowp = st + (size_t)m * 128u;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const uint32_t c = (uint32_t)(half * 4 + i);
-              const float4 v4 = *reinterpret_cast<const float4*>(rowp + ((c ^ (uint32_t)(m & 7)) << 4));
-              x[4 * i] = v4.x; x[4 * i + 1] = v4.y; x[4 * i + 2] = v4.z; x[4 * i + 3] = v4.w;
-            }
+          for (int e = 0; e < 16; ++e) {
+            const uint32_t k = (uint32_t)(half * 16 + e);
+            const uint32_t off = k * 128u + (uint32_t)(m & 31) * 4u;
+            x[e] = *reinterpret_cast<const float*>(box + (off ^ ((k & 3u) << 5)));
           }
-          const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + a_col0 + (uint32_t)(s * 64 + half * 16);
+        } else {
+          // rows of 128 bytes, 16-byte chunks XORed with the row index mod 8
+          const uint8_t* rowp = st + (size_t)m * 128u;
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            uint32_t hi[8], lo[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) split_tf32_trunc(x[c * 8 + e], hi[e], lo[e]);
-            tmem_st8(taddr + (uint32_t)(c * 8), hi);
-            tmem_st8(taddr + 32u + (uint32_t)(c * 8), lo);
+          for (int e = 0; e < 4; ++e) {
+            const uint32_t c = (uint32_t)(half * 4 + e);
+            const float4 v4 = *reinterpret_cast<const float4*>(rowp + ((c ^ (uint32_t)(m & 7)) << 4));
+            x[4 * e] = v4.x; x[4 * e + 1] = v4.y; x[4 * e + 2] = v4.z; x[4 * e + 3] = v4.w;
           }
         }
-        for (int i = P.a_tmem ? a_vec + xt : xt; i < a_vec + b_vec; i += kXThreads) {
-          const bool in_a = i < a_vec;
-          uint8_t* src = in_a ? st + (size_t)i * 16 : st + L.b_off + (size_t)(i - a_vec) * 16;
-          const float4 x = *reinterpret_cast<const float4*>(src);
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + a_col0 + (uint32_t)(ta.idx * 64 + half * 16);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t hi[8], l8[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) split_tf32_trunc(x[c * 8 + e], hi[e], l8[e]);
+          tmem_st8(taddr + (uint32_t)(c * 8), hi);
+          tmem_st8(taddr + 32u + (uint32_t)(c * 8), l8);
+        }
+        const float4* b_raw = reinterpret_cast<const float4*>(st + kFcATile);
+        float4* b_lo = reinterpret_cast<float4*>(base_ptr + L.lo_off + (size_t)lo.idx * L.lo_stride);
+#pragma unroll 4
+        for (int v = xt; v < b_vec; v += kXThreads) {
+          const float4 r = b_raw[v];
           float4 l;
-          l.x = x.x - __uint_as_float(__float_as_uint(x.x) & 0xFFFFE000u);
-          l.y = x.y - __uint_as_float(__float_as_uint(x.y) & 0xFFFFE000u);
-          l.z = x.z - __uint_as_float(__float_as_uint(x.z) & 0xFFFFE000u);
-          l.w = x.w - __uint_as_float(__float_as_uint(x.w) & 0xFFFFE000u);
-          *reinterpret_cast<float4*>(src + (in_a ? kFcATile : L.b_tile_bytes)) = l;
+          l.x = r.x - __uint_as_float(__float_as_uint(r.x) & 0xFFFFE000u);
+          l.y = r.y - __uint_as_float(__float_as_uint(r.y) & 0xFFFFE000u);
+          l.z = r.z - __uint_as_float(__float_as_uint(r.z) & 0xFFFFE000u);
+          l.w = r.w - __uint_as_float(__float_as_uint(r.w) & 0xFFFFE000u);
+          b_lo[v] = l;
         }
         fence_proxy_async_smem();
-        if (P.a_tmem) {
-          tmem_wait_st();
-          tc_fence_before();
-        }
+        tmem_wait_st();
+        tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(lo_bar + 8u * s);
+        if (lane == 0) mbar_arrive(lo_bar + 8u * (i & 3));
+        raw.advance(P.raw_slots);
+        lo.advance(P.lo_slots);
+        ta.advance(P.a_slots);
       }
     }
   } else {
     // ---- epilogue: lane = m (contiguous in the output), one column = one n
     const int quarter = warp;  // warps 0-3 own tensor-memory lanes 32 * warp ...
-    int tile_iter = 0;
+    uint8_t* out_ptr = base_ptr + L.store_off + (size_t)(warp * P.store_bufs) * kFcStoreTile;
+    const uint32_t out_smem = base + L.store_off + (uint32_t)(warp * P.store_bufs) * kFcStoreTile;
+    int tile_iter = 0, stores = 0;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_iter) {
       int mt, nt, split, kb0, kb1;
       tile_of(t, mt, nt, split, kb0, kb1);
       const int buf = tile_iter & (P.acc_bufs - 1), use = tile_iter >> (P.acc_bufs - 1);
       mbar_wait(acc_full + 8u * buf, (uint32_t)use & 1u, failed, P.status, 0x1600);
       tc_fence_after();
-      const int m = mt * kTileM + quarter * 32 + lane;
-      const int n0 = nt * P.n_pad;
-      float* op = P.out + (long long)split * P.split_stride + (long long)n0 * P.ld_out + m;
-      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.n_pad);
-      const uint32_t live = (m < P.M && !failed) ? 1u : 0u;
-      for (int c = 0; c < P.n_pad / 16; ++c) {
+      const int m0 = mt * kTileM + quarter * 32, n0 = nt * P.n_pad;
+      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.acc_cols);
+      const int chunks = min(P.n_pad, P.N - n0 + 15) / 16;  // columns behind N are never looked at
+      for (int c = 0; c < chunks; ++c) {
         float v[16];
         tmem_ld16(acc + (uint32_t)(c * 16), v);
+        if (P.dual) {
+          float w[16];
+          tmem_ld16(acc + (uint32_t)(P.n_pad + c * 16), w);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int n = n0 + c * 16 + j;
-          if (live && n < P.N) op[(long long)(c * 16 + j) * P.ld_out] = v[j];
+          for (int j = 0; j < 16; ++j) v[j] += w[j];
+        }
+        if (failed || m0 >= P.M) continue;
+        if (P.direct) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (m0 + lane < P.M && n0 + c * 16 + j < P.N) P.direct[(long long)(n0 + c * 16 + j) * P.ld_direct + m0 + lane] = v[j];
+          continue;
+        }
+        const uint32_t slot = P.store_bufs == 2 ? (uint32_t)(stores++ & 1) * kFcStoreTile : 0u;
+        if (lane == 0) {  // the store that read this tile last has done so
+          if (P.store_bufs == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) *reinterpret_cast<float*>(out_ptr + slot + j * 128 + lane * 4) = v[j];
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          fc_store_3d(&out_map, out_smem + slot, m0, n0 + c * 16, split);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, (uint32_t)P.tmem_cols);
 }
 
-// Y[b][o] = act(bias[o] + sum over splits of partial[s][b][o]), act = optional ReLU then optional dropout
-// (DropoutBridge forward: x * mask * scale, src/bridges/DropoutBridge_impl.hxx:71-74).  Splits are added in order.
-__global__ void fc_reduce_fwd_kernel(const float* __restrict__ partial, int splits, size_t split_stride,
-                                     const float* __restrict__ bias, float* __restrict__ Y, size_t total, int O, int relu,
-                                     const uint32_t* __restrict__ drop_mask, float drop_scale) {
+// Sums the splits of a contraction in split order and applies what surrounds it, VEC columns of a row per thread.
+//   forward        Y[b][o] = act(bias[o] + sum), act = optional ReLU then optional dropout (DropoutBridge forward:
+//                  x * mask * scale, src/bridges/DropoutBridge_impl.hxx:71-74)
+//   data gradient  dX[b][k] = sum x mask * scale (DropoutBridge::backward) x [X > 0] (the ReLU bridge in front,
+//                  src/kernels/relu.hxx:35-43)
+struct FcReduceParams {
+  const float* partial;      // [splits][rows][pitch]
+  float* out;                // [rows][cols]
+  const float* bias;         // forward
+  const float* X;            // data gradient: the ReLU mask's source, or null
+  const uint32_t* drop_mask;
+  float drop_scale;
+  int rows, cols, pitch, splits, relu;
+};
+template <int VEC>
+__global__ void __launch_bounds__(256) fc_reduce_kernel(const __grid_constant__ FcReduceParams P) {
   pdl_wait();
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    float acc = 0.f;
-    for (int s = 0; s < splits; ++s) acc += partial[(size_t)s * split_stride + i];
-    if (bias) acc += bias[i % O];
-    if (relu) acc = fmaxf(acc, 0.f);
-    if (drop_mask) acc = acc * (float)(drop_mask[i] != 0u) * drop_scale;
-    Y[i] = acc;
+  const int per_row = (P.cols + VEC - 1) / VEC;
+  const int t = blockIdx.x * 256 + threadIdx.x;
+  if (t >= P.rows * per_row) return;
+  const int row = t / per_row, col = (t - row * per_row) * VEC;
+  const float* src = P.partial + (size_t)row * P.pitch + col;
+  const size_t stride = (size_t)P.rows * P.pitch;
+  float acc[VEC];
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < P.splits; ++s, src += stride) {
+    if (VEC == 4) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(src));
+      acc[0] += v.x; acc[VEC > 1 ? 1 : 0] += v.y; acc[VEC > 2 ? 2 : 0] += v.z; acc[VEC > 3 ? 3 : 0] += v.w;
+    } else {
+      acc[0] += __ldg(src);
+    }
   }
+  const size_t at = (size_t)row * P.cols + col;
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) {
+    if (P.bias) acc[e] += __ldg(P.bias + col + e);
+    if (P.relu) acc[e] = fmaxf(acc[e], 0.f);
+    if (P.drop_mask) acc[e] = acc[e] * (float)(P.drop_mask[at + e] != 0u) * P.drop_scale;
+    if (P.X) acc[e] = acc[e] * (P.X[at + e] > 0.f ? 1.f : 0.f);
+  }
+  if (VEC == 4) *reinterpret_cast<float4*>(P.out + at) = make_float4(acc[0], acc[VEC > 1 ? 1 : 0], acc[VEC > 2 ? 2 : 0], acc[VEC > 3 ? 3 : 0]);
+  else P.out[at] = acc[0];
 }
 
-// dX[b][k] = (sum over splits) x [X > 0] (the ReLU bridge in front, src/kernels/relu.hxx:35-43) x mask * scale (the
-// dropout bridge in front, DropoutBridge::backward).
-__global__ void fc_reduce_dgrad_kernel(const float* __restrict__ partial, int splits, size_t split_stride,
-                                       float* __restrict__ dX, size_t total, const float* __restrict__ X, int in_relu,
-                                       const uint32_t* __restrict__ drop_mask, float drop_scale) {
+// A row-major matrix whose rows are no multiple of 16 bytes, copied into rows that are (the tensor maps' pitch rule).
+__global__ void __launch_bounds__(256) fc_pad_kernel(const float* __restrict__ src, float* __restrict__ dst, int rows, int cols, int pitch) {
   pdl_wait();
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    float acc = 0.f;
-    for (int s = 0; s < splits; ++s) acc += partial[(size_t)s * split_stride + i];
-    if (drop_mask) acc = acc * (float)(drop_mask[i] != 0u) * drop_scale;
-    if (in_relu) acc = acc * (X[i] > 0.f ? 1.f : 0.f);
-    dX[i] = acc;
-  }
+  for (int r = blockIdx.y; r < rows; r += gridDim.y)
+    for (int c = blockIdx.x * 256 + threadIdx.x; c < pitch; c += gridDim.x * 256)
+      dst[(size_t)r * pitch + c] = c < cols ? __ldg(src + (size_t)r * cols + c) : 0.f;
 }
 
 // db[o] = sum_b dY[b][o] (FullyConnectedBridge_impl.hxx:298: backward_bias_fc).  A block of 32 x 8 threads owns 32
@@ -353,22 +414,16 @@ __global__ void __launch_bounds__(256) fc_bias_grad_kernel(const float* __restri
 
 int fc_round_up(int v, int a) { return (v + a - 1) / a * a; }
 
-// rows x cols fp32 matrix, cols contiguous.  K-major use: box = 32 cols (reduction) x box_rows, 128-byte swizzle.
-// MN-major use: box = 32 cols (the operand's row index) x 32 rows (reduction), 128-byte swizzle with 32-byte atoms.
-int fc_make_map(cct_ctx* ctx, CUtensorMap* map, const float* ptr, size_t rows, size_t cols, int box_rows, bool mn_major) {
+int fc_encode(cct_ctx* ctx, CUtensorMap* map, const float* ptr, int rank, const cuuint64_t* dim, const cuuint64_t* stride,
+              const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) {
     ctx->last_error = "cuTensorMapEncodeTiled is not available from this driver";
     return CCT_ERR_CUDA;
   }
-  const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t gstride[1] = {(cuuint64_t)cols * sizeof(float)};
-  const cuuint32_t box[2] = {32u, (cuuint32_t)(mn_major ? 32 : box_rows)};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(ptr), gdim, gstride, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank, const_cast<float*>(ptr), dim, stride, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     ctx->last_error = "cuTensorMapEncodeTiled (fully connected operand) failed with code " + std::to_string((int)r);
     return CCT_ERR_CUDA;
@@ -376,57 +431,169 @@ int fc_make_map(cct_ctx* ctx, CUtensorMap* map, const float* ptr, size_t rows, s
   return CCT_OK;
 }
 
+// A tensor map and the address it was made for: a training loop passes the same buffers every time.
+struct FcMap {
+  CUtensorMap map;
+  const float* ptr = nullptr;
+};
+
+// rows x cols fp32 matrix, cols contiguous, rows `pitch` floats apart.  K-major use: box = 32 cols (reduction) x box_rows,
+// 128-byte swizzle.  MN-major use: box = 32 cols (the operand's row index) x 32 rows (reduction), 128-byte swizzle with
+// 32-byte atoms.
+int fc_operand_map(cct_ctx* ctx, FcMap* m, const float* ptr, size_t rows, size_t cols, size_t pitch, int box_rows, bool mn_major) {
+  if (m->ptr == ptr) return CCT_OK;
+  const cuuint64_t dim[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, stride[1] = {(cuuint64_t)pitch * sizeof(float)};
+  const cuuint32_t box[2] = {32u, (cuuint32_t)(mn_major ? 32 : box_rows)};
+  const int rc = fc_encode(ctx, &m->map, ptr, 2, dim, stride, box, mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B);
+  m->ptr = rc == CCT_OK ? ptr : nullptr;
+  return rc;
+}
+
+// An output of the contraction: [splits][N][pitch], stored in tiles of 16 rows x 32 columns.
+int fc_output_map(cct_ctx* ctx, FcMap* m, const float* ptr, size_t M, size_t N, size_t splits, size_t pitch) {
+  if (m->ptr == ptr) return CCT_OK;
+  const cuuint64_t dim[3] = {(cuuint64_t)M, (cuuint64_t)N, (cuuint64_t)splits},
+                   stride[2] = {(cuuint64_t)pitch * sizeof(float), (cuuint64_t)(N * pitch) * sizeof(float)};
+  const cuuint32_t box[3] = {32u, 16u, 1u};
+  const int rc = fc_encode(ctx, &m->map, ptr, 3, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+  m->ptr = rc == CCT_OK ? ptr : nullptr;
+  return rc;
+}
+
+// Tile shape, rings and splits of one contraction.
+struct FcShape {
+  FcGemmParams P{};
+  bool pair = false;  // two CTAs per SM
+  size_t smem = 0;
+};
+
+// Rings that fit: the raw ring first (it holds a slot for TMA + transform + MMA), then the second tile on its way out.
+bool fc_fit_rings(FcShape& s) {
+  FcGemmParams& P = s.P;
+  const size_t budget = s.pair ? 113 * 1024 : kSmemLimit;
+  P.tmem_cols = s.pair ? 256 : 512;
+  P.a_slots = std::min(kFcRing, (P.tmem_cols - P.acc_bufs * P.acc_cols) / 64);
+  for (int raw = kFcRing; raw >= 2; --raw)
+    for (int st = 2; st >= 1; --st) {
+      const int lo = P.dual ? raw : 2;
+      const size_t need = fc_smem(P.n_pad, P.dual, raw, lo, st).total + 1024;
+      if (need <= budget) {
+        P.raw_slots = raw; P.lo_slots = lo; P.store_bufs = st;
+        s.smem = need;
+        return P.a_slots >= 2;
+      }
+    }
+  return false;
+}
+
+// Forward pass and data gradient: M = the layer's output (input) features, N = batch.  The splits of the reduction are
+// chosen by the rounds of (tile, split) units over the resident CTAs: a k-block takes its 12 (dual: 8) MMAs, at least 75
+// cycles to issue each, and two CTAs on an SM share the tensor pipe; a unit adds set-up and epilogue, a split the traffic of
+// one more partial sum.
+FcShape fc_batch_shape(int sms, int M, int N, int R) {
+  FcShape s;
+  FcGemmParams& P = s.P;
+  P.M = M; P.N = N;
+  P.m_tiles = (M + kTileM - 1) / kTileM;
+  P.n_tiles = (N + 255) / 256;
+  P.n_pad = fc_round_up((N + P.n_tiles - 1) / P.n_tiles, 16);
+  P.dual = P.n_pad <= 64;
+  P.acc_cols = P.dual ? 2 * P.n_pad : P.n_pad;
+  P.acc_bufs = 1;
+  s.pair = P.n_pad <= 128;
+  P.kblocks_total = (R + kBlockK - 1) / kBlockK;
+  const double mmas = P.dual ? 8 : 12, exec = mmas * P.acc_cols / 2.0, alone = std::max(exec, mmas * 75) / 1750.0,
+               shared = std::max(2 * exec, mmas * 75) / 1750.0;
+  const long long slots = (long long)sms * (s.pair ? 2 : 1);
+  double best = 0.0;
+  for (int n = 1; n <= std::max(1, P.kblocks_total / 2); ++n) {
+    const int kps = (P.kblocks_total + n - 1) / n;
+    if ((P.kblocks_total + kps - 1) / kps != n || kps > kFcMaxChainKblocks) continue;
+    const long long units = (long long)P.m_tiles * P.n_tiles * n, tail = units % slots;
+    const double unit = 1.5 + 0.006 * P.n_pad;
+    const double us = (units / slots) * (kps * (s.pair ? shared : alone) + unit) +
+                      (tail ? kps * (s.pair && tail > sms ? shared : alone) + unit : 0.0) + (double)n * M * N * 8.0 / 4e6;
+    if (best == 0.0 || us < best) {
+      best = us;
+      P.splits = n;
+      P.kblocks_per_split = kps;
+    }
+  }
+  return s;
+}
+
+// Weight gradient: M = input features, N = output features, reduction over the batch (short): two accumulators, so that
+// one is written out while the next is formed.  Widest tiles that do not cost a round.
+FcShape fc_weight_shape(int sms, int K, int O, int B) {
+  FcShape best;
+  double best_us = 0.0;
+  for (int n = 192; n >= 32; n -= 32) {
+    if (n > 32 && n >= fc_round_up(O, 32) + 32) continue;
+    FcShape s;
+    FcGemmParams& P = s.P;
+    P.M = K; P.N = O;
+    P.m_tiles = (K + kTileM - 1) / kTileM;
+    P.n_pad = n; P.acc_cols = n; P.acc_bufs = 2;
+    P.n_tiles = (O + n - 1) / n;
+    P.splits = 1;
+    P.kblocks_total = P.kblocks_per_split = (B + kBlockK - 1) / kBlockK;
+    P.a_mn = P.b_mn = 1;
+    const long long rounds = ((long long)P.m_tiles * P.n_tiles + sms - 1) / sms;
+    const double mma = P.kblocks_total * 12.0 * std::max(75.0, n / 2.0) / 1750.0, out = 0.2 + 0.006 * n;
+    const double us = rounds * std::max(mma, out) + mma + out;
+    if (!best.P.n_pad || us < 0.98 * best_us) {
+      best = s;
+      best_us = us;
+    }
+  }
+  return best;
+}
+
 }  // namespace
 
 struct cct_fc_plan {
   cct_ctx* ctx = nullptr;
   int B = 0, K = 0, O = 0, bias = 0;
+  int K4 = 0, O4 = 0;        // row pitches: multiples of four floats
+  FcShape fwd, dgr, wgr;
   float* partial = nullptr;  // split partial sums of the forward pass and of the data gradient
-  size_t partial_elems = 0, bytes = 0;
-  int f_splits = 1, f_kps = 1, d_splits = 1, d_kps = 1;
+  float *Xp = nullptr, *Wp = nullptr, *dYp = nullptr;  // copies with padded rows, where K or O is no multiple of four
+  size_t bytes = 0;
+  FcMap w_fwd, x_fwd, w_dgr, dy_dgr, x_wgr, dy_wgr, out_fwd, out_dgr, out_wgr;
   PhaseTimer timer;
 };
 
 namespace {
 
-// Splits of a reduction of `kblocks` k-blocks over `tiles` output tiles: about one CTA per SM, chains bounded.
-void fc_pick_splits(int slots, int tiles, int kblocks, int* splits, int* kps) {
-  int s = std::max(1, slots / std::max(1, tiles));
-  s = std::max(s, (kblocks + kFcMaxChainKblocks - 1) / kFcMaxChainKblocks);
-  s = std::min(s, std::max(1, kblocks / 4));
-  *kps = (kblocks + s - 1) / s;
-  *splits = (kblocks + *kps - 1) / *kps;
-}
-
-// Accumulator width of the forward pass and the data gradient (N = batch): at most 128 columns, so that two CTAs fit on
-// an SM (256 tensor-memory columns and half the shared memory each) - two pipelines of TMA, transform and MMA issue per
-// SM hide each other's latencies, which one CTA with two 96 KB stages cannot.
-int fc_batch_tile(int batch) { return fc_round_up(std::min(batch, 128), 16); }
-
-int fc_launch(cct_ctx* ctx, FcGemmParams& P, const CUtensorMap& a_map, const CUtensorMap& b_map) {
-  const bool pair = P.a_tmem && P.n_pad <= 128;  // two CTAs per SM
-  const uint32_t stage = fc_smem(P.n_pad, 1, P.a_tmem).stage_bytes;
-  const uint32_t budget = pair ? 113u * 1024u : (uint32_t)kSmemLimit;
-  P.stages = std::min(kFcMaxStages, (int)((budget - 2048) / stage));
-  if (P.stages < 2) {
-    ctx->last_error = "fully connected tile does not fit in shared memory twice";
-    return CCT_ERR_UNSUPPORTED;
-  }
-  // Tensor memory = accumulator buffers (+ 64 columns per stage for an A operand kept there).
-  P.tmem_cols = pair ? 256 : 512;
-  if (P.a_tmem) P.stages = std::min(P.stages, (P.tmem_cols - P.n_pad) / 64);
-  const int a_cols = P.a_tmem ? P.stages * 64 : 0;
-  P.acc_bufs = 2 * P.n_pad + a_cols <= P.tmem_cols ? 2 : 1;
-  const size_t smem = fc_smem(P.n_pad, P.stages, P.a_tmem).total + 1024;
+int fc_launch(cct_ctx* ctx, const FcShape& s, const FcMap& a, const FcMap& b, const FcMap& out, float* direct = nullptr,
+              long long ld_direct = 0) {
+  FcGemmParams P = s.P;
+  P.direct = direct; P.ld_direct = ld_direct;
   P.status = ctx->status_dev;
   const int tiles = P.m_tiles * P.n_tiles * P.splits;
-  launch_pdl(fc_gemm_kernel, dim3(std::min(tiles, (pair ? 2 : 1) * ctx->launch_sms())), dim3(kFcThreads), smem, ctx->stream, P, a_map, b_map);
+  launch_pdl(fc_gemm_kernel, dim3(std::min(tiles, (s.pair ? 2 : 1) * ctx->launch_sms())), dim3(kFcThreads), s.smem, ctx->stream, P,
+             a.map, b.map, out.map);
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
 
-int fc_ew_grid(cct_ctx* ctx, size_t total) {
-  return (int)std::max<size_t>(1, std::min<size_t>((total + 255) / 256, (size_t)ctx->sm_count * 8));
+bool fc_aligned(std::initializer_list<const void*> ptrs) {
+  for (const void* p : ptrs)
+    if (reinterpret_cast<uintptr_t>(p) & 15u) return false;
+  return true;
+}
+
+int fc_reduce(cct_ctx* ctx, const FcReduceParams& R) {
+  const bool vec = R.cols % 4 == 0 && fc_aligned({R.partial, R.out});
+  const long long threads = (long long)R.rows * (vec ? R.cols / 4 : R.cols);
+  launch_pdl(vec ? fc_reduce_kernel<4> : fc_reduce_kernel<1>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, ctx->stream, R);
+  CCT_CHECK_LAUNCH(ctx);
+  return CCT_OK;
+}
+
+void fc_pad(cct_ctx* ctx, const float* src, float* dst, int rows, int cols, int pitch) {
+  launch_pdl(fc_pad_kernel, dim3(std::min((pitch + 255) / 256, 8), std::min(rows, 8 * ctx->sm_count)), dim3(256), 0, ctx->stream, src, dst,
+             rows, cols, pitch);
 }
 
 }  // namespace
@@ -437,28 +604,40 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   if (!ctx || !out) return CCT_ERR_INVALID;
   *out = nullptr;
   if (batch <= 0 || in_features <= 0 || out_features <= 0) return CCT_ERR_INVALID;
-  // TMA needs row pitches that are multiples of 16 bytes; the weight gradient reads X and dY with the batch as the
-  // reduction, in boxes of 32 columns.
-  if (in_features % 4 || out_features % 4) {
-    ctx->last_error = "fully connected layers need in_features and out_features that are multiples of 4";
+  if ((double)batch * std::max(in_features, out_features) > 2147483647.0 || (double)in_features * out_features > 4e9) {
+    ctx->last_error = "fully connected layer too large";
     return CCT_ERR_UNSUPPORTED;
   }
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   cct_fc_plan* p = new (std::nothrow) cct_fc_plan();
   if (!p) return CCT_ERR_NOMEM;
   p->ctx = ctx; p->B = batch; p->K = in_features; p->O = out_features; p->bias = bias_term != 0;
-  const int n_tiles = (batch + fc_batch_tile(batch) - 1) / fc_batch_tile(batch);
-  fc_pick_splits(2 * ctx->sm_count, ((out_features + kTileM - 1) / kTileM) * n_tiles, (in_features + kBlockK - 1) / kBlockK,
-                 &p->f_splits, &p->f_kps);
-  fc_pick_splits(2 * ctx->sm_count, ((in_features + kTileM - 1) / kTileM) * n_tiles, (out_features + kBlockK - 1) / kBlockK,
-                 &p->d_splits, &p->d_kps);
-  p->partial_elems = std::max((size_t)p->f_splits * batch * out_features, (size_t)p->d_splits * batch * in_features);
-  if (cudaMalloc((void**)&p->partial, p->partial_elems * sizeof(float)) != cudaSuccess) {
-    ctx->last_error = "cudaMalloc of the fully connected layer's split partial sums failed";
+  p->K4 = fc_round_up(in_features, 4); p->O4 = fc_round_up(out_features, 4);
+  p->fwd = fc_batch_shape(ctx->sm_count, out_features, batch, in_features);
+  p->dgr = fc_batch_shape(ctx->sm_count, in_features, batch, out_features);
+  p->dgr.P.a_mn = 1;
+  p->wgr = fc_weight_shape(ctx->sm_count, in_features, out_features, batch);
+  if (!fc_fit_rings(p->fwd) || !fc_fit_rings(p->dgr) || !fc_fit_rings(p->wgr)) {
+    ctx->last_error = "fully connected tile does not fit in shared memory twice";
+    delete p;
+    return CCT_ERR_UNSUPPORTED;
+  }
+  // One allocation: split sums, then the padded copies that are needed.
+  const size_t sums = std::max((size_t)p->fwd.P.splits * batch * p->O4, (size_t)p->dgr.P.splits * batch * p->K4);
+  const bool pad_k = p->K4 != p->K, pad_o = p->O4 != p->O;
+  auto room = [](size_t n) { return (n + 63) & ~(size_t)63; };
+  const size_t x = pad_k ? room((size_t)batch * p->K4) : 0, w = pad_k ? room((size_t)out_features * p->K4) : 0,
+               dy = pad_o ? room((size_t)batch * p->O4) : 0;
+  p->bytes = (room(sums) + x + w + dy) * sizeof(float);
+  if (cudaMalloc((void**)&p->partial, p->bytes) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->last_error = "cudaMalloc of the fully connected layer's scratch failed";
     delete p;
     return CCT_ERR_NOMEM;
   }
-  p->bytes = p->partial_elems * sizeof(float);
+  float* at = p->partial + room(sums);
+  if (pad_k) { p->Xp = at; p->Wp = at + x; }
+  if (pad_o) p->dYp = at + x + w;
   const cudaError_t e = cudaFuncSetAttribute(fc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   if (e != cudaSuccess) {
     ctx->last_error = std::string("cudaFuncSetAttribute(fc_gemm_kernel): ") + cudaGetErrorString(e);
@@ -493,28 +672,23 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
   cct_ctx* ctx = plan->ctx;
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
-  const int B = plan->B, K = plan->K, O = plan->O;
-  FcGemmParams P{};
-  P.M = O; P.N = B;
-  P.n_pad = fc_batch_tile(B);
-  P.m_tiles = (O + kTileM - 1) / kTileM; P.n_tiles = (B + P.n_pad - 1) / P.n_pad;
-  P.kblocks_total = (K + kBlockK - 1) / kBlockK; P.splits = plan->f_splits; P.kblocks_per_split = plan->f_kps;
-  P.a_mn = 0; P.b_mn = 0; P.a_tmem = 1;
-  P.out = plan->partial; P.ld_out = O; P.split_stride = (long long)B * O;
-  CUtensorMap a_map, b_map;
-  int rc = fc_make_map(ctx, &a_map, W, O, K, kTileM, false);
-  if (rc == CCT_OK) rc = fc_make_map(ctx, &b_map, X, B, K, P.n_pad, false);
-  if (rc != CCT_OK) return rc;
+  const int B = plan->B, K = plan->K, O = plan->O, K4 = plan->K4, O4 = plan->O4;
   plan->timer.begin(0, ctx->stream);
-  rc = fc_launch(ctx, P, a_map, b_map);
-  if (rc != CCT_OK) return rc;
-  const size_t total = (size_t)B * O;
-  launch_pdl(fc_reduce_fwd_kernel, dim3(fc_ew_grid(ctx, total)), dim3(256), 0, ctx->stream, plan->partial, P.splits, (size_t)P.split_stride,
-                                                                      plan->bias ? bias : nullptr, Y, total, O, relu,
-                                                                      drop_mask, drop_scale);
+  if (plan->Wp) {
+    fc_pad(ctx, X, plan->Xp, B, K, K4);
+    fc_pad(ctx, W, plan->Wp, O, K, K4);
+    X = plan->Xp;
+    W = plan->Wp;
+  }
+  int rc = fc_operand_map(ctx, &plan->w_fwd, W, O, K, K4, kTileM, false);
+  if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->x_fwd, X, B, K, K4, plan->fwd.P.n_pad, false);
+  if (rc == CCT_OK) rc = fc_output_map(ctx, &plan->out_fwd, plan->partial, O, B, plan->fwd.P.splits, O4);
+  if (rc == CCT_OK) rc = fc_launch(ctx, plan->fwd, plan->w_fwd, plan->x_fwd, plan->out_fwd);
+  if (rc == CCT_OK)
+    rc = fc_reduce(ctx, FcReduceParams{plan->partial, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4,
+                                       plan->fwd.P.splits, relu});
   plan->timer.end(0, ctx->stream);
-  CCT_CHECK_LAUNCH(ctx);
-  return CCT_OK;
+  return rc;
 }
 
 int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const float* dY, float* dX, float* dW, float* db,
@@ -523,51 +697,36 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   cct_ctx* ctx = plan->ctx;
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
-  const int B = plan->B, K = plan->K, O = plan->O;
-  int rc;
+  const int B = plan->B, K = plan->K, O = plan->O, K4 = plan->K4, O4 = plan->O4;
+  const float *Xm = X, *dYm = dY;
   // ---- weight gradient: out = dW[o][k] (m = k, n = o), reduction over the batch; both operands MN-major
-  {
-    FcGemmParams P{};
-    P.M = K; P.N = O;
-    P.n_pad = fc_round_up(std::min(O, 256), 32);
-    P.m_tiles = (K + kTileM - 1) / kTileM; P.n_tiles = (O + P.n_pad - 1) / P.n_pad;
-    P.kblocks_total = (B + kBlockK - 1) / kBlockK; P.splits = 1; P.kblocks_per_split = P.kblocks_total;
-    P.a_mn = 1; P.b_mn = 1;
-    P.out = dW; P.ld_out = K; P.split_stride = 0;
-    CUtensorMap a_map, b_map;
-    rc = fc_make_map(ctx, &a_map, X, B, K, 32, true);
-    if (rc == CCT_OK) rc = fc_make_map(ctx, &b_map, dY, B, O, 32, true);
-    if (rc != CCT_OK) return rc;
-    plan->timer.begin(1, ctx->stream);
-    rc = fc_launch(ctx, P, a_map, b_map);
-    if (rc != CCT_OK) return rc;
-    if (plan->bias) launch_pdl(fc_bias_grad_kernel, dim3((O + 31) / 32), dim3(256), 0, ctx->stream, dY, db, B, O);
-    plan->timer.end(1, ctx->stream);
-    CCT_CHECK_LAUNCH(ctx);
-  }
+  plan->timer.begin(1, ctx->stream);
+  if (plan->Xp) { fc_pad(ctx, X, plan->Xp, B, K, K4); Xm = plan->Xp; }
+  if (plan->dYp) { fc_pad(ctx, dY, plan->dYp, B, O, O4); dYm = plan->dYp; }
+  const bool direct = K4 != K || !fc_aligned({dW});  // an output no tensor map describes
+  int rc = fc_operand_map(ctx, &plan->x_wgr, Xm, B, K, K4, 32, true);
+  if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_wgr, dYm, B, O, O4, 32, true);
+  if (rc == CCT_OK && !direct) rc = fc_output_map(ctx, &plan->out_wgr, dW, K, O, 1, K);
+  if (rc == CCT_OK)
+    rc = fc_launch(ctx, plan->wgr, plan->x_wgr, plan->dy_wgr, direct ? plan->x_wgr : plan->out_wgr, direct ? dW : nullptr, K);
+  if (rc != CCT_OK) return rc;
+  if (plan->bias) launch_pdl(fc_bias_grad_kernel, dim3((O + 31) / 32), dim3(256), 0, ctx->stream, dY, db, B, O);
+  plan->timer.end(1, ctx->stream);
+  CCT_CHECK_LAUNCH(ctx);
   // ---- data gradient: out = dX[b][k] (m = k, n = b), reduction over o; A = W read MN-major, B = dY K-major
   if (dX) {
-    FcGemmParams P{};
-    P.M = K; P.N = B;
-    P.n_pad = fc_batch_tile(B);
-    P.m_tiles = (K + kTileM - 1) / kTileM; P.n_tiles = (B + P.n_pad - 1) / P.n_pad;
-    P.kblocks_total = (O + kBlockK - 1) / kBlockK; P.splits = plan->d_splits; P.kblocks_per_split = plan->d_kps;
-    P.a_mn = 1; P.b_mn = 0; P.a_tmem = 1;
-    P.out = plan->partial; P.ld_out = K; P.split_stride = (long long)B * K;
-    CUtensorMap a_map, b_map;
-    rc = fc_make_map(ctx, &a_map, W, O, K, 32, true);
-    if (rc == CCT_OK) rc = fc_make_map(ctx, &b_map, dY, B, O, P.n_pad, false);
-    if (rc != CCT_OK) return rc;
     plan->timer.begin(3, ctx->stream);
-    rc = fc_launch(ctx, P, a_map, b_map);
-    if (rc != CCT_OK) return rc;
-    const size_t total = (size_t)B * K;
-    launch_pdl(fc_reduce_dgrad_kernel, dim3(fc_ew_grid(ctx, total)), dim3(256), 0, ctx->stream, plan->partial, P.splits, (size_t)P.split_stride,
-                                                                          dX, total, X, in_relu, in_drop_mask, in_drop_scale);
+    if (plan->Wp) { fc_pad(ctx, W, plan->Wp, O, K, K4); W = plan->Wp; }
+    rc = fc_operand_map(ctx, &plan->w_dgr, W, O, K, K4, 32, true);
+    if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_dgr, dYm, B, O, O4, plan->dgr.P.n_pad, false);
+    if (rc == CCT_OK) rc = fc_output_map(ctx, &plan->out_dgr, plan->partial, K, B, plan->dgr.P.splits, K4);
+    if (rc == CCT_OK) rc = fc_launch(ctx, plan->dgr, plan->w_dgr, plan->dy_dgr, plan->out_dgr);
+    if (rc == CCT_OK)
+      rc = fc_reduce(ctx, FcReduceParams{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4,
+                                         plan->dgr.P.splits, 0});
     plan->timer.end(3, ctx->stream);
-    CCT_CHECK_LAUNCH(ctx);
   }
-  return CCT_OK;
+  return rc;
 }
 
 int cct_fc_plan_enable_timing(cct_fc_plan* plan, int enable) {

@@ -196,8 +196,8 @@ int cct_conv_plan_last_timings(cct_conv_plan* plan, float ms[5]);
  *      (src/bridges/FullyConnectedBridge_impl.hxx:171-235, 257-330) and the driver calls they make (sgemm_new,
  *      backward_bias_fc: src/sched/DeviceDriver_GPU.cu:1142-1160).  X is [batch][in_features] (a cube of any R x C x D
  *      with R*C*D = in_features, flattened as the reference does), W is [out_features][in_features], Y is
- *      [batch][out_features].  in_features and out_features must be multiples of 4.  The three contractions run as
- *      3xTF32 on the tensor cores with the operands read in place by TMA (nothing is transposed or packed). ---- */
+ *      [batch][out_features].  The three contractions run as 3xTF32 on the tensor cores with the operands read in place by
+ *      TMA (nothing is transposed or packed); feature counts that are no multiples of 4 take copies with padded rows first. ---- */
 typedef struct cct_fc_plan cct_fc_plan;
 int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_features, int bias_term, cct_fc_plan** out);
 int cct_fc_plan_destroy(cct_fc_plan* plan);
