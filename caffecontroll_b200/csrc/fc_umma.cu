@@ -32,7 +32,7 @@ constexpr int kFcThreads = (kFcXformWarp0 + kFcXformWarps) * 32;  // 448
 constexpr int kFcRing = 4;                    // deepest ring of any kind; the lo and done barriers are a ring of four
 constexpr int kFcMaxChainKblocks = 96;        // k-blocks of 32 per partial sum: the tensor core's fp32 accumulate truncates
 constexpr uint32_t kFcATile = kTileM * 128u;  // bytes of one 128 x 32 fp32 tile
-constexpr uint32_t kFcStoreTile = 32u * 16u * 4u;  // 16 columns x 32 lanes on their way out
+constexpr uint32_t kFcStoreTile = 32u * 32u * 4u;  // 32 columns x 32 lanes on their way out
 
 struct FcGemmParams {
   int M, N;                 // extents of the output (m fastest in memory)
@@ -50,7 +50,7 @@ struct FcGemmParams {
 // Raw ring (A tile and B tile as TMA delivers them; for `dual` B's lo tile behind them), lo ring (B's lo tiles), the tiles
 // on their way out, barriers.
 struct FcSmem {
-  uint32_t b_tile_bytes, raw_bytes, lo_off, lo_stride, store_off, bars_off, total;
+  uint32_t b_tile_bytes, raw_bytes, lo_off, lo_stride, store_off, total;
 };
 __host__ __device__ inline FcSmem fc_smem(int n_pad, int dual, int raw_slots, int lo_slots, int store_bufs) {
   FcSmem L;
@@ -59,8 +59,7 @@ __host__ __device__ inline FcSmem fc_smem(int n_pad, int dual, int raw_slots, in
   L.lo_off = dual ? kFcATile + L.b_tile_bytes : (uint32_t)raw_slots * L.raw_bytes;
   L.lo_stride = dual ? L.raw_bytes : L.b_tile_bytes;
   L.store_off = (uint32_t)raw_slots * L.raw_bytes + (dual ? 0u : (uint32_t)lo_slots * L.b_tile_bytes);
-  L.bars_off = L.store_off + (uint32_t)(kFcEpiWarps * store_bufs) * kFcStoreTile;
-  L.total = L.bars_off + 8u * (3 * kFcRing + 4) + 16u;
+  L.total = L.store_off + (uint32_t)(kFcEpiWarps * store_bufs) * kFcStoreTile;  // the barriers go where the 1 KB of alignment slack leaves room
   return L;
 }
 
@@ -87,8 +86,8 @@ __device__ __forceinline__ void fc_store_3d(const void* tmap, uint32_t src, int 
 // which is also the hi operand, is held for TMA + transform + MMA, the other two only from transform to MMA, so the raw ring
 // is the deeper one.  raw[slot] completes when the TMA bytes have landed, lo[i % 4] when the transform warps are through,
 // done[i % 4] when the block's MMAs have finished, which frees all three slots (nobody waits more than four blocks back).
-// The epilogue turns sixteen accumulator columns at a time into a 16 x 32 tile in shared memory (one conflict-free store per
-// column) that a TMA store takes out, clipping it at the edges: per-lane global stores with their addresses and bounds cost
+// The epilogue turns 32 accumulator columns at a time into a 32 x 32 tile in shared memory (one conflict-free store per
+// column) that TMA stores take out, clipping it at the edges: per-lane global stores with their addresses and bounds cost
 // about ten instructions each and made the weight gradient of small batches instruction-bound (fc6, batch 32: 70 us, 2.1 TB/s).
 __global__ void __launch_bounds__(kFcThreads, 2)
     fc_gemm_kernel(const __grid_constant__ FcGemmParams P, const __grid_constant__ CUtensorMap a_map,
@@ -98,7 +97,9 @@ __global__ void __launch_bounds__(kFcThreads, 2)
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
   const FcSmem L = fc_smem(P.n_pad, P.dual, P.raw_slots, P.lo_slots, P.store_bufs);
-  const uint32_t bars = base + L.bars_off;
+  // 1 KB more than L.total is allocated: either in front of the aligned base or behind the tiles there is room for these
+  constexpr uint32_t kBarBytes = 8u * (3 * kFcRing + 4) + 24u;
+  const uint32_t bars = base - smem_u32(smem_raw) >= kBarBytes ? (smem_u32(smem_raw) + 7u) & ~7u : base + L.total;  // 8-byte aligned
   const uint32_t raw_bar = bars, lo_bar = raw_bar + 8u * kFcRing, done_bar = lo_bar + 8u * kFcRing,
                  acc_full = done_bar + 8u * kFcRing, acc_empty = acc_full + 16u, tmem_slot = acc_empty + 16u;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -285,34 +286,48 @@ __global__ void __launch_bounds__(kFcThreads, 2)
       const int m0 = mt * kTileM + quarter * 32, n0 = nt * P.n_pad;
       const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.acc_cols);
       const int chunks = min(P.n_pad, P.N - n0 + 15) / 16;  // columns behind N are never looked at
-      for (int c = 0; c < chunks; ++c) {
-        float v[16];
-        tmem_ld16(acc + (uint32_t)(c * 16), v);
+      for (int c = 0; c < chunks; c += 2) {  // 32 columns a step: one round of waits, fence and stores for them
+        float v[2][16];
+        const bool two = c + 1 < chunks;
+        tmem_ld16(acc + (uint32_t)(c * 16), v[0]);
+        if (two) tmem_ld16(acc + (uint32_t)(c * 16 + 16), v[1]);
         if (P.dual) {
           float w[16];
           tmem_ld16(acc + (uint32_t)(P.n_pad + c * 16), w);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] += w[j];
+          for (int j = 0; j < 16; ++j) v[0][j] += w[j];
+          if (two) {
+            tmem_ld16(acc + (uint32_t)(P.n_pad + c * 16 + 16), w);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[1][j] += w[j];
+          }
         }
         if (failed || m0 >= P.M) continue;
         if (P.direct) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (m0 + lane < P.M && n0 + c * 16 + j < P.N) P.direct[(long long)(n0 + c * 16 + j) * P.ld_direct + m0 + lane] = v[j];
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const int n = n0 + (c + h) * 16 + j;
+              if (m0 + lane < P.M && n < P.N && (h == 0 || two)) P.direct[(long long)n * P.ld_direct + m0 + lane] = v[h][j];
+            }
           continue;
         }
         const uint32_t slot = P.store_bufs == 2 ? (uint32_t)(stores++ & 1) * kFcStoreTile : 0u;
-        if (lane == 0) {  // the store that read this tile last has done so
+        if (lane == 0) {  // the stores that read this tile last have done so
           if (P.store_bufs == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
           else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         }
         __syncwarp();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) *reinterpret_cast<float*>(out_ptr + slot + j * 128 + lane * 4) = v[j];
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) *reinterpret_cast<float*>(out_ptr + slot + (h * 16 + j) * 128 + lane * 4) = v[h][j];
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
           fc_store_3d(&out_map, out_smem + slot, m0, n0 + c * 16, split);
+          if (two) fc_store_3d(&out_map, out_smem + slot + 2048u, m0, n0 + c * 16 + 16, split);
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
       }
@@ -341,27 +356,43 @@ struct FcReduceParams {
   float drop_scale;
   int rows, cols, pitch, splits, relu;
 };
-template <int VEC>
+// SLICES > 1: a block's eight warps take interleaved slices of the splits of the same 32 x VEC elements and add them in a
+// fixed order - small outputs with many splits, where one thread per element would be a long chain on a few SMs.
+template <int VEC, int SLICES>
 __global__ void __launch_bounds__(256) fc_reduce_kernel(const __grid_constant__ FcReduceParams P) {
   pdl_wait();
+  __shared__ float part[SLICES > 1 ? SLICES : 1][VEC][33];
   const int per_row = (P.cols + VEC - 1) / VEC;
-  const int t = blockIdx.x * 256 + threadIdx.x;
-  if (t >= P.rows * per_row) return;
-  const int row = t / per_row, col = (t - row * per_row) * VEC;
+  const int lane = threadIdx.x & 31, slice = SLICES > 1 ? threadIdx.x >> 5 : 0;
+  const int t = SLICES > 1 ? blockIdx.x * 32 + lane : blockIdx.x * 256 + threadIdx.x;
+  const bool in = t < P.rows * per_row;
+  const int row = in ? t / per_row : 0, col = in ? (t - row * per_row) * VEC : 0;
   const float* src = P.partial + (size_t)row * P.pitch + col;
   const size_t stride = (size_t)P.rows * P.pitch;
   float acc[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
 #pragma unroll 4
-  for (int s = 0; s < P.splits; ++s, src += stride) {
+  for (int s = slice; s < P.splits; s += SLICES) {
+    const float* at = src + s * stride;
     if (VEC == 4) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(src));
+      const float4 v = __ldg(reinterpret_cast<const float4*>(at));
       acc[0] += v.x; acc[VEC > 1 ? 1 : 0] += v.y; acc[VEC > 2 ? 2 : 0] += v.z; acc[VEC > 3 ? 3 : 0] += v.w;
     } else {
-      acc[0] += __ldg(src);
+      acc[0] += __ldg(at);
     }
   }
+  if (SLICES > 1) {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) part[slice][e][lane] = acc[e];
+    __syncthreads();
+    if (slice) return;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+#pragma unroll
+      for (int y = 1; y < SLICES; ++y) acc[e] += part[y][e][lane];
+  }
+  if (!in) return;
   const size_t at = (size_t)row * P.cols + col;
 #pragma unroll
   for (int e = 0; e < VEC; ++e) {
@@ -586,7 +617,10 @@ bool fc_aligned(std::initializer_list<const void*> ptrs) {
 int fc_reduce(cct_ctx* ctx, const FcReduceParams& R) {
   const bool vec = R.cols % 4 == 0 && fc_aligned({R.partial, R.out});
   const long long threads = (long long)R.rows * (vec ? R.cols / 4 : R.cols);
-  launch_pdl(vec ? fc_reduce_kernel<4> : fc_reduce_kernel<1>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, ctx->stream, R);
+  const bool slices = R.splits >= 8 && threads < 256ll * ctx->sm_count;
+  auto kernel = slices ? (vec ? fc_reduce_kernel<4, 8> : fc_reduce_kernel<1, 8>) : (vec ? fc_reduce_kernel<4, 1> : fc_reduce_kernel<1, 1>);
+  const long long per_block = slices ? 32 : 256;
+  launch_pdl(kernel, dim3((unsigned)((threads + per_block - 1) / per_block)), dim3(256), 0, ctx->stream, R);
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
