@@ -59,7 +59,21 @@ class Context:
         capi.check(self.lib.cct_fill_f32(self.h, C.c_void_p(ptr), count, value), "cct_fill_f32", self.h)
 
 
-class LogicalCube:
+class Tracked:
+    """An object whose attributes decide which calls a pass over a network makes (cubes, layers, bridges).  Every assignment
+    raises Tracked.changes, so that a network that has recorded its calls knows when they may no longer be the same.
+    `_untracked` names the attributes that change from pass to pass without changing the calls."""
+
+    changes = 0
+    _untracked = ()
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if name not in self._untracked:
+            Tracked.changes += 1
+
+
+class LogicalCube(Tracked):
     """R x C x D x B fp32 (or int32) cube in device memory; numpy view of it is shaped (B, D, R, C)."""
 
     def __init__(self, ctx, R, C_, D, B, dtype=np.float32, ptr=None):
@@ -101,13 +115,13 @@ class LogicalCube:
             self.ptr = None
 
 
-class Layer:
+class Layer(Tracked):
     def __init__(self, p_data_cube, p_gradient_cube):
         self.p_data_cube = p_data_cube
         self.p_gradient_cube = p_gradient_cube
 
 
-class ConvolutionBridge:
+class ConvolutionBridge(Tracked):
     """forward(): p_input_layer.p_data_cube -> p_output_layer.p_data_cube.
     backward(): p_output_layer.p_gradient_cube (+ input data) -> p_input_layer.p_gradient_cube (iff
     needs_to_calc_backward_grad), model gradient and bias gradient cubes (overwritten)."""
@@ -218,7 +232,7 @@ class ConvolutionBridge:
                 c.free()
 
 
-class FullyConnectedBridge:
+class FullyConnectedBridge(Tracked):
     """The reference's FullyConnectedBridge (src/bridges/FullyConnectedBridge_impl.hxx:171-235, 257-330): Y = X W^T + b
     over the flattened input, weight layout [o][d][r][c].  Runs on the fully connected plan of the C ABI (tensor-core
     GEMMs that read X, W and dY in place); algo=ALGO_SIMT_FP32 runs as a 1x1 convolution over the input viewed as D*R*C

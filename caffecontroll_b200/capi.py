@@ -25,7 +25,8 @@ EXPORTS = [
     "cct_conv_plan_enable_timing", "cct_conv_plan_last_timings", "cct_conv_forward", "cct_conv_backward", "cct_conv_backward_fused",
     "cct_conv_plan_reserve_fusion", "cct_selftest_bounded_wait", "cct_conv_forward_host", "cct_conv_backward_host", "cct_conv_weight_grad_noalloc",
     "cct_maxpool_forward", "cct_maxpool_backward", "cct_relu_forward", "cct_relu_backward",
-    "cct_pool_relu_backward", "cct_sgd_step", "cct_saxpby", "cct_l1_update",
+    "cct_pool_relu_backward", "cct_sgd_step", "cct_sgd_step_multi",
+    "cct_program_begin", "cct_program_end", "cct_program_run", "cct_program_destroy", "cct_saxpby", "cct_l1_update",
     "cct_fc_plan_create", "cct_fc_plan_destroy", "cct_fc_plan_workspace_bytes", "cct_fc_forward", "cct_fc_backward",
     "cct_fc_plan_enable_timing", "cct_fc_plan_last_timings",
     "cct_comm_unique_id", "cct_comm_init_rank", "cct_comm_destroy", "cct_comm_size", "cct_allreduce_sum_begin",
@@ -44,6 +45,12 @@ class BwdFusion(C.Structure):
     """cct_bwd_fusion: what cct_conv_backward_fused folds into the backward pass."""
     _fields_ = [("A", C.c_void_p), ("idx", C.c_void_p), ("dP", C.c_void_p), ("pool_k", C.c_int), ("pool_s", C.c_int),
                 ("relu_mask_dx", C.c_int), ("P", C.c_void_p)]
+
+
+class SgdItem(C.Structure):
+    """cct_sgd_item: one tensor of cct_sgd_step_multi."""
+    _fields_ = [("count", C.c_size_t), ("w", C.c_void_p), ("g", C.c_void_p), ("h", C.c_void_p), ("lr", C.c_float),
+                ("momentum", C.c_float), ("lam", C.c_float)]
 
 
 class ConvDesc(C.Structure):
@@ -103,6 +110,11 @@ def load():
         "cct_relu_backward": [_vp, _vp, _vp, _vp, sz],
         "cct_pool_relu_backward": [_vp, _vp, _vp, _vp, _vp, i, i, i, i],
         "cct_sgd_step": [_vp, sz, _vp, _vp, _vp, f, f, f],
+        "cct_sgd_step_multi": [_vp, i, C.POINTER(SgdItem)],
+        "cct_program_begin": [_vp, C.POINTER(_vp)],
+        "cct_program_end": [_vp],
+        "cct_program_run": [_vp],
+        "cct_program_destroy": [_vp],
         "cct_saxpby": [_vp, sz, f, _vp, f, _vp],
         "cct_l1_update": [_vp, sz, _vp, f, _vp],
         "cct_comm_unique_id": [C.c_char_p],

@@ -398,7 +398,51 @@ int cct_conv_plan_last_timings(cct_conv_plan* plan, float ms[5]) {
   return CCT_OK;
 }
 
+// ---- recorded calls: see include/cct_b200.h
+struct cct_program {
+  cct_ctx* ctx = nullptr;
+  std::vector<std::function<int()>> calls;
+};
+
+int cct_program_begin(cct_ctx* ctx, cct_program** out) {
+  if (!ctx || !out) return CCT_ERR_INVALID;
+  *out = nullptr;
+  if (ctx->recording) {
+    ctx->last_error = "a program is already being recorded on this context";
+    return CCT_ERR_INVALID;
+  }
+  cct_program* p = new (std::nothrow) cct_program();
+  if (!p) return CCT_ERR_NOMEM;
+  p->ctx = ctx;
+  ctx->recording = &p->calls;
+  *out = p;
+  return CCT_OK;
+}
+
+int cct_program_end(cct_program* program) {
+  if (!program || program->ctx->recording != &program->calls) return CCT_ERR_INVALID;
+  program->ctx->recording = nullptr;
+  return CCT_OK;
+}
+
+int cct_program_run(cct_program* program) {
+  if (!program || program->ctx->recording) return CCT_ERR_INVALID;
+  for (const auto& call : program->calls) {
+    const int rc = call();
+    if (rc != CCT_OK) return rc;
+  }
+  return CCT_OK;
+}
+
+int cct_program_destroy(cct_program* program) {
+  if (!program) return CCT_ERR_INVALID;
+  if (program->ctx->recording == &program->calls) program->ctx->recording = nullptr;
+  delete program;
+  return CCT_OK;
+}
+
 int cct_conv_forward(cct_conv_plan* plan, const float* X, const float* W, const float* bias, float* Y, int relu) {
+  if (plan) CCT_RECORD(plan->ctx, cct_conv_forward(plan, X, W, bias, Y, relu))
   if (!plan || !X || !W || !Y) return CCT_ERR_INVALID;
   cct_ctx* ctx = plan->ctx;
   if (plan->G.bias && !bias) return CCT_ERR_INVALID;
@@ -409,6 +453,7 @@ int cct_conv_forward(cct_conv_plan* plan, const float* X, const float* W, const 
 
 int cct_conv_backward(cct_conv_plan* plan, const float* X, const float* W, const float* dY, float* dX, float* dW,
                       float* db) {
+  if (plan) CCT_RECORD(plan->ctx, cct_conv_backward(plan, X, W, dY, dX, dW, db))
   if (!plan || !X || !W || !dY || !dW) return CCT_ERR_INVALID;
   cct_ctx* ctx = plan->ctx;
   if (plan->G.bias && !db) return CCT_ERR_INVALID;
@@ -420,6 +465,10 @@ int cct_conv_backward(cct_conv_plan* plan, const float* X, const float* W, const
 
 int cct_conv_backward_fused(cct_conv_plan* plan, const float* X, const float* W, const float* dY,
                             const cct_bwd_fusion* f, float* dX, float* dW, float* db) {
+  if (plan && f && plan->ctx->recording) {
+    const cct_bwd_fusion kept = *f;
+    CCT_RECORD(plan->ctx, cct_conv_backward_fused(plan, X, W, dY, &kept, dX, dW, db))
+  }
   if (!f) return cct_conv_backward(plan, X, W, dY, dX, dW, db);
   if (!plan || !X || !W || !dW) return CCT_ERR_INVALID;
   cct_ctx* ctx = plan->ctx;

@@ -2,8 +2,10 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <functional>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "../../include/cct_b200.h"
 
@@ -28,7 +30,17 @@ struct cct_ctx {
   volatile int* status_host = nullptr;
   int* status_dev = nullptr;
   std::string last_error;
+  // While a program is being recorded (cct_program_begin .. _end) the bridge calls on this context are kept here instead of
+  // being carried out.
+  std::vector<std::function<int()>>* recording = nullptr;
 };
+
+// First line of every recordable entry point: `call` is the entry point with its own arguments.
+#define CCT_RECORD(ctx, call)                                         \
+  if ((ctx) && (ctx)->recording) {                                    \
+    (ctx)->recording->push_back([=]() -> int { return call; });       \
+    return CCT_OK;                                                    \
+  }
 
 #define CCT_CUDA(ctx, call)                                                                   \
   do {                                                                                        \

@@ -72,6 +72,55 @@ __global__ void sgd_kernel(size_t count, size_t vec, float* __restrict__ w, floa
   }
 }
 
+// The same step for several tensors in one launch.  A block takes kSgdChunk parameters of one tensor (found by its place
+// in the list of first blocks); a thread has the twelve 16-byte loads of its four groups in flight.  CaffeNet's sixteen
+// tensors: 266 -> see the figures at cct_sgd_step_multi's test; launches 16 -> 1.
+constexpr int kSgdItems = 24, kSgdUnroll = 4, kSgdChunk = 256 * 4 * kSgdUnroll;
+struct SgdItems {
+  cct_sgd_item item[kSgdItems];
+  int first[kSgdItems + 1];  // first block of each tensor
+  int vec[kSgdItems];        // 1: 16-byte accesses
+  int n;
+};
+__global__ void __launch_bounds__(256) sgd_multi_kernel(const __grid_constant__ SgdItems P) {
+  pdl_wait();
+  int t = 0;
+  while (t + 1 < P.n && (int)blockIdx.x >= P.first[t + 1]) ++t;
+  const cct_sgd_item& it = P.item[t];
+  const size_t c0 = (size_t)((int)blockIdx.x - P.first[t]) * kSgdChunk;
+  const float lr = it.lr, momentum = it.momentum, lambda = it.lambda;
+  if (P.vec[t]) {
+    float4* w4 = reinterpret_cast<float4*>(it.w);
+    float4* g4 = reinterpret_cast<float4*>(it.g);
+    float4* h4 = reinterpret_cast<float4*>(it.h);
+    const size_t groups = it.count / 4, i0 = c0 / 4 + threadIdx.x;
+    float4 w[kSgdUnroll], g[kSgdUnroll], h[kSgdUnroll];
+#pragma unroll
+    for (int u = 0; u < kSgdUnroll; ++u)
+      if (i0 + u * 256 < groups) { g[u] = g4[i0 + u * 256]; h[u] = h4[i0 + u * 256]; w[u] = w4[i0 + u * 256]; }
+#pragma unroll
+    for (int u = 0; u < kSgdUnroll; ++u)
+      if (i0 + u * 256 < groups) {
+        float4 wo;
+        wo.x = sgd_one(g[u].x, w[u].x, h[u].x, lr, momentum, lambda);
+        wo.y = sgd_one(g[u].y, w[u].y, h[u].y, lr, momentum, lambda);
+        wo.z = sgd_one(g[u].z, w[u].z, h[u].z, lr, momentum, lambda);
+        wo.w = sgd_one(g[u].w, w[u].w, h[u].w, lr, momentum, lambda);
+        if (lambda != 0.f) g4[i0 + u * 256] = g[u];
+        h4[i0 + u * 256] = h[u];
+        w4[i0 + u * 256] = wo;
+      }
+  }
+  // the elements behind the last group of four, or all of them where a pointer is not 16-byte aligned
+  for (size_t i = (P.vec[t] ? max(c0, it.count & ~(size_t)3) : c0) + threadIdx.x; i < min(c0 + kSgdChunk, it.count); i += 256) {
+    float gi = it.g[i], hi = it.h[i];
+    const float wo = sgd_one(gi, it.w[i], hi, lr, momentum, lambda);
+    if (lambda != 0.f) it.g[i] = gi;
+    it.h[i] = hi;
+    it.w[i] = wo;
+  }
+}
+
 // y = alpha x + beta y (12 B moved per element): the saxpy / saxpby calls of the reference's SGD updater
 // (src/algorithms/GradientUpdater.h:163-181), for callers that keep its three-call update.
 __global__ void saxpby_kernel(size_t count, float alpha, const float* __restrict__ x, float beta, float* __restrict__ y) {
@@ -525,6 +574,37 @@ int cct_sgd_step(cct_ctx* ctx, size_t count, float* w, float* g, float* h, float
   return CCT_OK;
 }
 
+int cct_sgd_step_multi(cct_ctx* ctx, int n, const cct_sgd_item* items) {
+  if (!ctx || n < 0 || (n && !items)) return CCT_ERR_INVALID;
+  CCT_CUDA(ctx, cudaSetDevice(ctx->device));
+  SgdItems P;
+  P.n = 0;
+  long long blocks = 0;
+  auto flush = [&]() -> int {
+    if (P.n) launch_pdl(sgd_multi_kernel, dim3((unsigned)blocks), dim3(256), 0, ctx->stream, P);
+    P.n = 0;
+    blocks = 0;
+    CCT_CHECK_LAUNCH(ctx);
+    return CCT_OK;
+  };
+  for (int i = 0; i < n; ++i) {
+    const cct_sgd_item& it = items[i];
+    if (!it.count) continue;
+    if (!it.w || !it.g || !it.h) return CCT_ERR_INVALID;
+    const long long need = (long long)((it.count + kSgdChunk - 1) / kSgdChunk);
+    if (P.n == kSgdItems || blocks + need > 0x7fffffffll) {
+      const int rc = flush();
+      if (rc != CCT_OK) return rc;
+    }
+    P.item[P.n] = it;
+    P.vec[P.n] = vec_groups(4, {it.w, it.g, it.h}) ? 1 : 0;
+    P.first[P.n] = (int)blocks;
+    blocks += need;
+    P.first[++P.n] = (int)blocks;
+  }
+  return flush();
+}
+
 int cct_saxpby(cct_ctx* ctx, size_t count, float alpha, const float* x, float beta, float* y) {
   if (!ctx || ((!x || !y) && count)) return CCT_ERR_INVALID;
   if (!count) return CCT_OK;
@@ -544,6 +624,7 @@ int cct_l1_update(cct_ctx* ctx, size_t count, float* g, float lambda, const floa
 }
 
 int cct_relu_forward(cct_ctx* ctx, const float* X, float* Y, size_t count) {
+  CCT_RECORD(ctx, cct_relu_forward(ctx, X, Y, count))
   if (!ctx || !X || !Y) return CCT_ERR_INVALID;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   launch_pdl(relu_fwd_kernel, dim3(grid_for(ctx, (count + 3) / 4, 256)), dim3(256), 0, ctx->stream, X, Y, count, vec_groups(count, {X, Y}));
@@ -552,6 +633,7 @@ int cct_relu_forward(cct_ctx* ctx, const float* X, float* Y, size_t count) {
 }
 
 int cct_relu_backward(cct_ctx* ctx, const float* X, const float* dY, float* dX, size_t count) {
+  CCT_RECORD(ctx, cct_relu_backward(ctx, X, dY, dX, count))
   if (!ctx || !X || !dY || !dX) return CCT_ERR_INVALID;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   launch_pdl(relu_bwd_kernel, dim3(grid_for(ctx, (count + 3) / 4, 256)), dim3(256), 0, ctx->stream, X, dY, dX, count,
@@ -562,6 +644,7 @@ int cct_relu_backward(cct_ctx* ctx, const float* X, const float* dY, float* dX, 
 
 
 int cct_maxpool_forward(cct_ctx* ctx, const float* X, float* Y, int32_t* idx, int planes, int n, int k, int s) {
+  CCT_RECORD(ctx, cct_maxpool_forward(ctx, X, Y, idx, planes, n, k, s))
   if (!ctx || !X || !Y || !idx || !pool_args_ok(planes, n, k, s)) return CCT_ERR_INVALID;
   const int m = (n - k) / s + 1;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
@@ -574,6 +657,7 @@ int cct_maxpool_forward(cct_ctx* ctx, const float* X, float* Y, int32_t* idx, in
 
 int cct_maxpool_backward(cct_ctx* ctx, const float* dY, const int32_t* idx, float* dX, int planes, int n, int k,
                          int s) {
+  CCT_RECORD(ctx, cct_maxpool_backward(ctx, dY, idx, dX, planes, n, k, s))
   if (!ctx || !dY || !idx || !dX || !pool_args_ok(planes, n, k, s)) return CCT_ERR_INVALID;
   const int m = (n - k) / s + 1;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));

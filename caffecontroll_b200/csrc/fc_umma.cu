@@ -702,6 +702,7 @@ int cct_fc_plan_workspace_bytes(const cct_fc_plan* plan, size_t* bytes) {
 
 int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const float* bias, float* Y, int relu,
                    const uint32_t* drop_mask, float drop_scale) {
+  if (plan) CCT_RECORD(plan->ctx, cct_fc_forward(plan, X, W, bias, Y, relu, drop_mask, drop_scale))
   if (!plan || !X || !W || !Y || (plan->bias && !bias)) return CCT_ERR_INVALID;
   cct_ctx* ctx = plan->ctx;
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
@@ -727,6 +728,7 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
 
 int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const float* dY, float* dX, float* dW, float* db,
                     int in_relu, const uint32_t* in_drop_mask, float in_drop_scale) {
+  if (plan) CCT_RECORD(plan->ctx, cct_fc_backward(plan, X, W, dY, dX, dW, db, in_relu, in_drop_mask, in_drop_scale))
   if (!plan || !X || !W || !dY || !dW || (plan->bias && !db)) return CCT_ERR_INVALID;
   cct_ctx* ctx = plan->ctx;
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;

@@ -365,6 +365,7 @@ extern "C" {
 
 int cct_lrn_forward(cct_ctx* ctx, const float* X, float* Y, float* scale, int batch, int depth, int plane, int local_size,
                     float alpha, float beta) {
+  CCT_RECORD(ctx, cct_lrn_forward(ctx, X, Y, scale, batch, depth, plane, local_size, alpha, beta))
   if (!ctx || !X || !Y || batch <= 0 || depth <= 0 || plane <= 0 || local_size <= 0 || !(local_size & 1))
     return CCT_ERR_INVALID;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
@@ -384,6 +385,7 @@ int cct_lrn_forward(cct_ctx* ctx, const float* X, float* Y, float* scale, int ba
 
 int cct_lrn_backward(cct_ctx* ctx, const float* X, const float* Y, const float* scale, const float* dY, float* dX,
                      int batch, int depth, int plane, int local_size, float alpha, float beta) {
+  CCT_RECORD(ctx, cct_lrn_backward(ctx, X, Y, scale, dY, dX, batch, depth, plane, local_size, alpha, beta))
   if (!ctx || !X || !dY || !dX || batch <= 0 || depth <= 0 || plane <= 0 || local_size <= 0 || !(local_size & 1))
     return CCT_ERR_INVALID;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
@@ -413,6 +415,7 @@ int cct_lrn_backward(cct_ctx* ctx, const float* X, const float* Y, const float* 
 }
 
 int cct_dropout_apply(cct_ctx* ctx, const float* in, const uint32_t* mask, float scale, float* out, size_t count) {
+  CCT_RECORD(ctx, cct_dropout_apply(ctx, in, mask, scale, out, count))
   if (!ctx || !in || !mask || !out) return CCT_ERR_INVALID;
   if (!count) return CCT_OK;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
@@ -434,6 +437,7 @@ int cct_dropout_mask(cct_ctx* ctx, uint32_t* mask, size_t count, float ratio, ui
 
 int cct_softmax_loss_forward(cct_ctx* ctx, const float* X, const float* labels, float* prob, float* image_loss,
                              float* loss, int batch, int classes) {
+  CCT_RECORD(ctx, cct_softmax_loss_forward(ctx, X, labels, prob, image_loss, loss, batch, classes))
   if (!ctx || !X || !labels || !prob || !image_loss || !loss || batch <= 0 || classes <= 0) return CCT_ERR_INVALID;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   launch_pdl(softmax_fwd_kernel, dim3((batch + 3) / 4), dim3(128), 0, ctx->stream, X, labels, prob, image_loss, batch, classes);
@@ -445,6 +449,7 @@ int cct_softmax_loss_forward(cct_ctx* ctx, const float* X, const float* labels, 
 
 int cct_softmax_loss_backward(cct_ctx* ctx, const float* prob, const float* labels, float* dX, int batch, int classes,
                               float scale) {
+  CCT_RECORD(ctx, cct_softmax_loss_backward(ctx, prob, labels, dX, batch, classes, scale))
   if (!ctx || !prob || !labels || !dX || batch <= 0 || classes <= 0) return CCT_ERR_INVALID;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   const size_t total = (size_t)batch * classes;

@@ -9,12 +9,12 @@ import ctypes as C
 import numpy as np
 
 from . import capi
-from .bridge import LogicalCube
+from .bridge import LogicalCube, Tracked
 
 _vp = C.c_void_p
 
 
-class _Bridge:
+class _Bridge(Tracked):
     def __init__(self, p_input_layer, p_output_layer, ctx=None):
         self.p_input_layer, self.p_output_layer = p_input_layer, p_output_layer
         x, y = p_input_layer.p_data_cube, p_output_layer.p_data_cube
@@ -118,6 +118,8 @@ class DropoutBridge(_Bridge):
     input * mask * 1 / (1 - ratio), the same product on the gradient.  The mask is drawn on the device from
     (random_seed, pass counter); set_mask() injects a given one (parity runs use the CPU oracle's)."""
 
+    _untracked = ("calls", "mask_held")
+
     def __init__(self, p_input_layer, p_output_layer, dropout_ratio=0.5, random_seed=1, ctx=None):
         super().__init__(p_input_layer, p_output_layer, ctx)
         self.dropout_ratio = dropout_ratio
@@ -126,13 +128,14 @@ class DropoutBridge(_Bridge):
         self.mask_cube = LogicalCube(self.ctx, self.iR, self.iC, self.iD, self.iB, np.uint32)
         self.calls = 0
         self.injected = False
+        self.mask_held = False  # the owner draws the mask itself (a network that replays its recorded calls)
 
     def set_mask(self, mask):
         self.mask_cube.upload(np.ascontiguousarray(mask, dtype=np.uint32))
         self.injected = True
 
     def draw_mask(self):
-        if self.injected:
+        if self.injected or self.mask_held:
             return
         self.calls += 1
         capi.check(self.lib.cct_dropout_mask(self.ctx.h, _vp(self.mask_cube.ptr), self.mask_cube.n_elements,

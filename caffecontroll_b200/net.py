@@ -13,10 +13,10 @@ import re
 import numpy as np
 
 from . import capi
-from .bridge import ConvolutionBridge, FullyConnectedBridge, Layer, LogicalCube
+from .bridge import ConvolutionBridge, FullyConnectedBridge, Layer, LogicalCube, Tracked
 from .layers import DropoutBridge, LRNBridge, MaxPoolingBridge, ReLUBridge, SoftmaxLossBridge
-from .parallel import (DeviceOps, ModelParallelFullyConnectedBridge, ModelParallelizedBridge, ParallelizedBridge,
-                       SolverParameter, model_parallel_gpus)
+from .parallel import (DeviceOps, ModelParallelFullyConnectedBridge, ModelParallelizedBridge, NetworkUpdate,
+                       ParallelizedBridge, SolverParameter, model_parallel_gpus)
 
 # ------------------------------------------------------------------------------------- protobuf text format
 
@@ -300,6 +300,8 @@ class Net:
         self.in_place = [self.bridges[i].p_input_layer is self.bridges[i].p_output_layer for i in range(len(self.bridges))]
         self.input = next(iter(self.blobs.values()))
         self.fused = []
+        self._update = NetworkUpdate()
+        self._program, self._recorded = None, None
         if fuse:
             self._fuse()
 
@@ -392,6 +394,10 @@ class Net:
             br.forward()
 
     def backward(self):
+        self._backward_passes()
+        self._update.apply([self.pbridges[i] for i in sorted(self.pbridges, reverse=True)])
+
+    def _backward_passes(self):
         # Gradient sums are begun per layer and run on the communicator's stream beside the layers below.  The fully
         # connected layers' sums (most of the bytes) are held back until the first convolution's backward pass is next:
         # the inner-product kernels are single-wave grids that lose a whole wave when NCCL takes SMs away from them,
@@ -413,12 +419,58 @@ class Net:
         for h in held:
             h.begin_allreduce()
         self.ops.allreduce_wait()
-        for i in sorted(self.pbridges, reverse=True):
-            self.pbridges[i].apply_update()
+
+    # The host side of an iteration is a few Python calls per bridge, several times what a small layer's kernels take.  The
+    # bridges make the same library calls on the same buffers every time, so step() records them once and has the library
+    # repeat them; the dropout masks (a new counter every pass) and the update (a rate that may change) stay outside.
+    _RECORDABLE = (ConvolutionBridge, FullyConnectedBridge, ReLUBridge, MaxPoolingBridge, LRNBridge, DropoutBridge, SoftmaxLossBridge)
+
+    def _may_record(self):
+        """Whether the walk over the bridges is nothing but library calls that a program keeps: the library's own bridges,
+        unmodified, on one rank."""
+        plain = [object.__getattribute__(b, "_bridge") if isinstance(b, _WithPrologue) else b for b in self.bridges]
+        return (type(self) is Net and type(self.ops) is DeviceOps and self.ops.world_size() == 1 and
+                not {"forward", "backward"} & set(self.__dict__) and
+                all(type(b) in self._RECORDABLE and not {"forward", "backward"} & set(b.__dict__) for b in plain) and
+                all(type(pb) is ParallelizedBridge for pb in self.pbridges.values()))
+
+    def _release_program(self):
+        if self._program is not None:
+            self.ctx.lib.cct_program_destroy(self._program)
+        self._program = None
+
+    def _record(self):
+        self._release_program()
+        if self._may_record():
+            h = C.c_void_p()
+            capi.check(self.ctx.lib.cct_program_begin(self.ctx.h, C.byref(h)), "cct_program_begin", self.ctx.h)
+            drops = [b for b, t in zip(self.bridges, self.types) if t == "Dropout"]
+            try:
+                for d in drops:
+                    d.mask_held = True
+                self.forward()
+                self._backward_passes()
+            except BaseException:
+                self.ctx.lib.cct_program_destroy(h)
+                raise
+            finally:
+                for d in drops:
+                    d.mask_held = False
+            capi.check(self.ctx.lib.cct_program_end(h), "cct_program_end", self.ctx.h)
+            self._program, self._drops = h, drops
+        self._recorded = (Tracked.changes, list(self.bridges))
 
     def step(self):
-        self.forward()
-        self.backward()
+        if self._recorded is None or self._recorded[0] != Tracked.changes or self._recorded[1] != self.bridges:
+            self._record()
+        if self._program is None or "forward" in self.__dict__ or "backward" in self.__dict__:
+            self.forward()
+            self.backward()
+            return
+        for d in self._drops:
+            DropoutBridge.draw_mask(d)
+        capi.check(self.ctx.lib.cct_program_run(self._program), "cct_program_run", self.ctx.h)
+        self._update.apply([self.pbridges[i] for i in sorted(self.pbridges, reverse=True)])
 
     def set_update_model_gradients(self, flag):
         for pb in self.pbridges.values():
@@ -518,6 +570,8 @@ class Net:
 
     def close(self):
         self.ctx.sync()
+        self._release_program()
+        self._recorded = None
         for br in self.bridges:
             br.close()
         for pb in self.pbridges.values():

@@ -213,6 +213,10 @@ class DeviceOps:
         capi.check(self.ctx.lib.cct_sgd_step(self.ctx.h, count, vp(w), vp(g), vp(h), lr, momentum, lam), "cct_sgd_step",
                    self.ctx.h)
 
+    def sgd_steps(self, items, n):
+        """The "L2" step (or, with lam = 0, the plain one) for `n` tensors described by an array of capi.SgdItem, in one launch."""
+        capi.check(self.ctx.lib.cct_sgd_step_multi(self.ctx.h, n, items), "cct_sgd_step_multi", self.ctx.h)
+
     def zero(self, ptr, count):
         self.ctx.fill(ptr, count, 0.0)
 
@@ -441,6 +445,17 @@ class ParallelizedBridge:
                               float(np.float32(base * self.lr_mult[1])), s.momentum,
                               float(np.float32(s.weight_decay * self.decay_mult[1])), s.regularization_type)
 
+    def update_tensors(self, base):
+        """(count, parameters, gradients, history, rate, momentum, decay) of the weights and of the bias for one update with
+        the base learning rate `base`: what apply_update() passes to the SGD step."""
+        s, out = self.solver, []
+        decay = s.weight_decay if s.regularization_type == "L2" else 0.0
+        for off, n, j in ((0, self.n_w, 0), (4 * self.n_w, self.n_b, 1)):
+            if n:
+                out.append((n, self.params + off, self.grads + off, self.hist + off, float(np.float32(base * self.lr_mult[j])),
+                            s.momentum, float(np.float32(decay * self.decay_mult[j]))))
+        return out
+
     def get_model_grad_cube(self):
         return self.bridge.p_model_gradient_cube
 
@@ -467,6 +482,36 @@ class ParallelizedBridge:
             for p in (self.params, self.grads, self.hist):
                 free(p)
         self.params = self.grads = self.hist = None
+
+
+class NetworkUpdate:
+    """apply_update() of all layers of a network as one launch, where their updaters allow it (device memory, no L1 decay)."""
+
+    def __init__(self):
+        self.key, self.items, self.n = None, None, 0
+
+    def apply(self, pbridges):
+        active = [pb for pb in pbridges if pb.update_model_gradients]
+        if not active:
+            return
+        if any(not isinstance(pb.ops, DeviceOps) or pb.solver.regularization_type == "L1" for pb in active):
+            for pb in active:
+                pb.apply_update()
+            return
+        bases, key = {}, []
+        for pb in active:
+            pb.current_iter += 1  # the updater increments before use (GradientUpdater.h:155)
+            s = pb.solver
+            which = (id(s), pb.current_iter)
+            base = bases.get(which)
+            if base is None:
+                base = bases[which] = get_learning_rate(s.lr_policy, s.base_lr, s.gamma, float(pb.current_iter), float(s.stepsize),
+                                                        s.power, float(s.max_iter))
+            key.append((pb.params, base, pb.lr_mult, pb.decay_mult, s.momentum, s.weight_decay, s.regularization_type))
+        if key != self.key:
+            tensors = [t for pb, k in zip(active, key) for t in pb.update_tensors(k[1])]
+            self.items, self.n, self.key = (capi.SgdItem * len(tensors))(*[capi.SgdItem(*t) for t in tensors]), len(tensors), key
+        active[0].ops.sgd_steps(self.items, self.n)
 
 
 class ModelParallelizedBridge(ParallelizedBridge):

@@ -217,6 +217,18 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
 int cct_fc_plan_enable_timing(cct_fc_plan* plan, int enable);
 int cct_fc_plan_last_timings(cct_fc_plan* plan, float ms[5]);
 
+/* Recorded calls (no counterpart in the reference).  Between cct_program_begin and cct_program_end the bridge calls made on
+ * the context - cct_conv_forward / backward / backward_fused, cct_fc_forward / backward, cct_maxpool_*, cct_relu_*,
+ * cct_lrn_*, cct_dropout_apply, cct_softmax_loss_* - are kept with their arguments instead of being carried out (they
+ * return CCT_OK); every other call takes effect at once.  cct_program_run carries the kept calls out in order, as often as
+ * wanted, and returns the first error.  The plans and buffers they name must still exist then.  A caller whose iteration
+ * repeats the same calls on the same buffers pays for walking its layers once. */
+typedef struct cct_program cct_program;
+int cct_program_begin(cct_ctx* ctx, cct_program** out);
+int cct_program_end(cct_program* program);
+int cct_program_run(cct_program* program);
+int cct_program_destroy(cct_program* program);
+
 /* Failure-path self-test (no counterpart in the reference, whose kernels never wait on anything): launches one warp
  * that waits, through the same bounded wait the convolution kernels use, on a barrier nothing completes, with a limit
  * of `limit_cycles` SM clock cycles (at most the kernels' own limit).  The wait runs out, the kernel returns normally,
@@ -306,6 +318,13 @@ int cct_softmax_loss_backward(cct_ctx* ctx, const float* prob, const float* labe
 /* ---- parameter update: SGDGradientUpdater::update (src/algorithms/GradientUpdater.h:154-193) as one kernel:
  *      g += lambda*w (if lambda != 0);  h = lr*g + momentum*h;  w -= h. ---- */
 int cct_sgd_step(cct_ctx* ctx, size_t count, float* w, float* g, float* h, float lr, float momentum, float lambda);
+/* The same step for several tensors - all layers of a network - in one launch. */
+typedef struct cct_sgd_item {
+  size_t count;
+  float *w, *g, *h;
+  float lr, momentum, lambda;
+} cct_sgd_item;
+int cct_sgd_step_multi(cct_ctx* ctx, int n, const cct_sgd_item* items);
 /* y = alpha * x + beta * y on device vectors: DeviceDriver::math_saxpy (beta = 1) and math_saxpby
  * (src/sched/DeviceDriver.h:197-206), the calls the reference's SGDGradientUpdater makes when it is instantiated on a
  * device driver unchanged. */
