@@ -33,6 +33,8 @@ struct cct_ctx {
   // While a program is being recorded (cct_program_begin .. _end) the bridge calls on this context are kept here instead of
   // being carried out.
   std::vector<std::function<int()>>* recording = nullptr;
+  int timed_plans = 0;                    // plans whose kernel timing is switched on: programs then run call by call
+  cudaStream_t capture_stream = nullptr;  // programs are captured here (the context's own stream may be the legacy one)
 };
 
 // First line of every recordable entry point: `call` is the entry point with its own arguments.

@@ -74,7 +74,7 @@ __global__ void sgd_kernel(size_t count, size_t vec, float* __restrict__ w, floa
 
 // The same step for several tensors in one launch.  A block takes kSgdChunk parameters of one tensor (found by its place
 // in the list of first blocks); a thread has the twelve 16-byte loads of its four groups in flight.  CaffeNet's sixteen
-// tensors: 266 -> see the figures at cct_sgd_step_multi's test; launches 16 -> 1.
+// tensors (61 M parameters, 24 B each): sixteen launches 266 us, this 212 us.
 constexpr int kSgdItems = 24, kSgdUnroll = 4, kSgdChunk = 256 * 4 * kSgdUnroll;
 struct SgdItems {
   cct_sgd_item item[kSgdItems];

@@ -688,6 +688,7 @@ int cct_fc_plan_destroy(cct_fc_plan* plan) {
   cudaSetDevice(plan->ctx->device);
   cudaStreamSynchronize(plan->ctx->stream);
   cudaFree(plan->partial);
+  plan->ctx->timed_plans -= plan->timer.enabled;
   for (cudaEvent_t e : plan->timer.ev)
     if (e) cudaEventDestroy(e);
   delete plan;
@@ -772,6 +773,7 @@ int cct_fc_plan_enable_timing(cct_fc_plan* plan, int enable) {
   PhaseTimer& t = plan->timer;
   if (enable && !t.ev[0])
     for (cudaEvent_t& e : t.ev) CCT_CUDA(ctx, cudaEventCreate(&e));
+  ctx->timed_plans += (enable != 0) - t.enabled;
   t.enabled = enable != 0;
   for (bool& h : t.have) h = false;
   return CCT_OK;
