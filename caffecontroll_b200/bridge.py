@@ -303,11 +303,10 @@ class FullyConnectedBridge(Tracked):
             self._conv.fuse_relu = self.fuse_relu
             self._conv.forward()
             return
-        vp = C.c_void_p
         mask = self.dropout_mask.ptr if self.dropout_mask is not None else None
-        capi.check(self.lib.cct_fc_forward(self.plan, vp(self.p_input_layer.p_data_cube.ptr), vp(self.p_model_cube.ptr),
-                                           vp(self.p_bias_cube.ptr) if self.bias_term else None,
-                                           vp(self.p_output_layer.p_data_cube.ptr), int(self.fuse_relu), mask,
+        capi.check(self.lib.cct_fc_forward(self.plan, self.p_input_layer.p_data_cube.ptr, self.p_model_cube.ptr,
+                                           self.p_bias_cube.ptr if self.bias_term else None,
+                                           self.p_output_layer.p_data_cube.ptr, int(self.fuse_relu), mask,
                                            float(self.dropout_scale)), "cct_fc_forward", self.ctx.h)
 
     def backward(self):
@@ -318,13 +317,12 @@ class FullyConnectedBridge(Tracked):
             self._conv.fuse_relu_backward = self.fuse_relu_backward
             self._conv.backward()
             return
-        vp = C.c_void_p
         dx = self.p_input_layer.p_gradient_cube.ptr if self.needs_to_calc_backward_grad else None
         mask = self.input_dropout_mask.ptr if self.input_dropout_mask is not None else None
-        capi.check(self.lib.cct_fc_backward(self.plan, vp(self.p_input_layer.p_data_cube.ptr), vp(self.p_model_cube.ptr),
-                                            vp(self.p_output_layer.p_gradient_cube.ptr), dx,
-                                            vp(self.p_model_gradient_cube.ptr),
-                                            vp(self.p_bias_gradient_cube.ptr) if self.bias_term else None,
+        capi.check(self.lib.cct_fc_backward(self.plan, self.p_input_layer.p_data_cube.ptr, self.p_model_cube.ptr,
+                                            self.p_output_layer.p_gradient_cube.ptr, dx,
+                                            self.p_model_gradient_cube.ptr,
+                                            self.p_bias_gradient_cube.ptr if self.bias_term else None,
                                             int(self.fuse_relu_backward), mask, float(self.input_dropout_scale)),
                    "cct_fc_backward", self.ctx.h)
 

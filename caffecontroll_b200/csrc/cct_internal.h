@@ -29,6 +29,7 @@ struct cct_ctx {
   // One word in mapped pinned host memory that kernels set when a bounded wait runs out; read by cct_sync().
   volatile int* status_host = nullptr;
   int* status_dev = nullptr;
+  unsigned* ticket = nullptr;  // device word, zero between kernels: which block of a kernel is the last to finish
   std::string last_error;
   // While a program is being recorded (cct_program_begin .. _end) the bridge calls on this context are kept here instead of
   // being carried out.

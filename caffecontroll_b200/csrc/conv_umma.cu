@@ -1187,12 +1187,13 @@ __global__ void __launch_bounds__(32 * SLICES) wgrad_reduce_flat_kernel(const fl
     const int kk = e / n_pad, j = e - kk * n_pad, first = (vg % tiles_per_group) * n_real;
     // the last channel tile of a group may be shorter; the bias row exists only where the kernel produced it
     if (j < min(n_real, og - first) && (kk < k_real || db)) {
-      float t = part[0][tx];
+      float t[4] = {0.f, 0.f, 0.f, 0.f};  // four short chains
 #pragma unroll
-      for (int y = 1; y < SLICES; ++y) t += part[y][tx];
+      for (int y = 0; y < SLICES; ++y) t[y & 3] += part[y][tx];
       const int ch = (vg / tiles_per_group) * og + first + j;
       float* dst = kk < k_real ? dW + (size_t)ch * k_real + kk : db + ch;
-      *dst = accumulate ? *dst + t : t;
+      const float sum = (t[0] + t[1]) + (t[2] + t[3]);
+      *dst = accumulate ? *dst + sum : sum;
     }
   }
 }

@@ -486,6 +486,48 @@ __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
   }
 }
 
+// 2x2 windows with stride 2 (LeNet): the windows do not overlap, an element belongs to one window or to none (the last row
+// and column of an odd plane).  One thread per 2 x 2 block of elements: its window's index and gradient in, four elements out.
+template <bool RELU>
+__global__ void __launch_bounds__(256) maxpool_bwd_2x2_kernel(const float* __restrict__ A, const int32_t* __restrict__ idx,
+                                                              const float* __restrict__ dP, const float* __restrict__ P,
+                                                              float* __restrict__ dA, int items, int n, int m, int half,
+                                                              uint32_t inv_half) {
+  pdl_wait();
+  const int t = blockIdx.x * 256 + threadIdx.x;
+  if (t >= items) return;
+  const int row = (int)fast_div((uint32_t)t, (uint32_t)half, inv_half), b = t - row * half;  // row = plane * half + a
+  const int plane = (int)fast_div((uint32_t)row, (uint32_t)half, inv_half), a = row - plane * half;
+  int where = -1;
+  float g = 0.f;
+  if (a < m && b < m) {
+    const size_t at = (size_t)plane * m * m + a * m + b;
+    where = __ldg(idx + at);
+    g = __ldg(dP + at);
+    // With the pooled tensor P given, its sign is the ReLU mask (see maxpool_bwd_3x3s2_kernel).
+    if (P != nullptr && !(__ldg(P + at) > 0.f)) g = 0.f;
+  }
+  const size_t base = (size_t)plane * n * n;
+  const int e00 = 2 * a * n + 2 * b;
+  const bool wide = 2 * b + 1 < n, tall = 2 * a + 1 < n;
+  float r[4];
+  const int e[4] = {e00, e00 + 1, e00 + n, e00 + n + 1};
+  const bool in[4] = {true, wide, tall, wide && tall};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    r[i] = 0.f + (where == e[i] ? g : 0.f);  // as the sums of the other kernels: -0 becomes 0
+    if (RELU && in[i]) r[i] = __ldg(A + base + e[i]) > 0.f ? r[i] : 0.f;
+  }
+  if ((n & 1) == 0 && (reinterpret_cast<uintptr_t>(dA) & 7) == 0) {
+    *reinterpret_cast<float2*>(dA + base + e[0]) = make_float2(r[0], r[1]);
+    *reinterpret_cast<float2*>(dA + base + e[2]) = make_float2(r[2], r[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (in[i]) dA[base + e[i]] = r[i];
+  }
+}
+
 template <bool RELU>
 int launch_maxpool_bwd(cct_ctx* ctx, const float* A, const int32_t* idx, const float* dP, float* dA, int planes, int n,
                        int m, int k, int s, const float* P = nullptr) {
@@ -507,6 +549,12 @@ int launch_maxpool_bwd(cct_ctx* ctx, const float* A, const int32_t* idx, const f
                  planes, n, m, half, fast_div_magic((uint64_t)group * half * half, (uint32_t)half), group, vec_ok);
       return CCT_OK;
     }
+  }
+  const long long items = (long long)planes * half * half;
+  if (k == 2 && s == 2 && items < (1ll << 31) - 256) {
+    launch_pdl(maxpool_bwd_2x2_kernel<RELU>, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, ctx->stream, A, idx, dP, P, dA, (int)items, n,
+               m, half, fast_div_magic((uint64_t)items, (uint32_t)half));
+    return CCT_OK;
   }
   constexpr int kSlotSmemCap = 56 * 1024;  // four blocks per SM
   if (taps <= 2 && m * m <= kSlotThreads * kSlotWin && (size_t)n * n * 16 + (size_t)n * 4 <= kSlotSmemCap) {

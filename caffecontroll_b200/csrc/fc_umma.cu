@@ -445,6 +445,10 @@ __global__ void __launch_bounds__(256) fc_bias_grad_kernel(const float* __restri
 
 int fc_round_up(int v, int a) { return (v + a - 1) / a * a; }
 
+}  // namespace
+#include "fc_small.cuh"
+namespace {
+
 int fc_encode(cct_ctx* ctx, CUtensorMap* map, const float* ptr, int rank, const cuuint64_t* dim, const cuuint64_t* stride,
               const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn enc = encode_tiled_fn();
@@ -587,6 +591,8 @@ struct cct_fc_plan {
   int B = 0, K = 0, O = 0, bias = 0;
   int K4 = 0, O4 = 0;        // row pitches: multiples of four floats
   FcShape fwd, dgr, wgr;
+  bool small = false;        // all three contractions by fc_small_kernel, with these splits
+  int small_fwd = 1, small_dgr = 1;
   float* partial = nullptr;  // split partial sums of the forward pass and of the data gradient
   float *Xp = nullptr, *Wp = nullptr, *dYp = nullptr;  // copies with padded rows, where K or O is no multiple of four
   size_t bytes = 0;
@@ -606,6 +612,16 @@ int fc_launch(cct_ctx* ctx, const FcShape& s, const FcMap& a, const FcMap& b, co
              a.map, b.map, out.map);
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
+}
+
+// Flops count the tiles' padding, which is most of the work for a handful of images.
+bool use_small_fc(int B, int K, int O) {
+  const double flops = 2.0 * fc_round_up(B, kFsTile) * fc_round_up(K, kFsTile) * fc_round_up(O, kFsTile);
+  return flops <= (K % 4 || O % 4 ? kSmallFcPaddedFlops : kSmallFcFlops);
+}
+
+void fc_small(cct_ctx* ctx, const FcSmallParams& P, int splits) {
+  launch_pdl(fc_small_kernel, dim3((P.M + kFsTile - 1) / kFsTile, (P.N + kFsTile - 1) / kFsTile, splits), dim3(kFsThreads), 0, ctx->stream, P);
 }
 
 bool fc_aligned(std::initializer_list<const void*> ptrs) {
@@ -656,9 +672,13 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
     delete p;
     return CCT_ERR_UNSUPPORTED;
   }
+  p->small = use_small_fc(batch, in_features, out_features);
+  p->small_fwd = fc_small_splits(ctx->sm_count, out_features, batch, in_features);
+  p->small_dgr = fc_small_splits(ctx->sm_count, in_features, batch, out_features);
   // One allocation: split sums, then the padded copies that are needed.
-  const size_t sums = std::max((size_t)p->fwd.P.splits * batch * p->O4, (size_t)p->dgr.P.splits * batch * p->K4);
-  const bool pad_k = p->K4 != p->K, pad_o = p->O4 != p->O;
+  const int f_splits = p->small ? p->small_fwd : p->fwd.P.splits, d_splits = p->small ? p->small_dgr : p->dgr.P.splits;
+  const size_t sums = std::max((size_t)f_splits * batch * p->O4, (size_t)d_splits * batch * p->K4);
+  const bool pad_k = !p->small && p->K4 != p->K, pad_o = !p->small && p->O4 != p->O;
   auto room = [](size_t n) { return (n + 63) & ~(size_t)63; };
   const size_t x = pad_k ? room((size_t)batch * p->K4) : 0, w = pad_k ? room((size_t)out_features * p->K4) : 0,
                dy = pad_o ? room((size_t)batch * p->O4) : 0;
@@ -710,6 +730,17 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   const int B = plan->B, K = plan->K, O = plan->O, K4 = plan->K4, O4 = plan->O4;
   plan->timer.begin(0, ctx->stream);
+  if (plan->small) {
+    const int splits = plan->small_fwd;
+    const FcReduceParams post{plan->partial, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, splits, relu};
+    FcSmallParams S{W, X, K, K, 0, 0, O, B, K, fc_round_up((K + splits - 1) / splits, 32), splits > 1 ? plan->partial : Y,
+                    splits > 1 ? O4 : O, nullptr, post};
+    fc_small(ctx, S, splits);
+    CCT_CHECK_LAUNCH(ctx);
+    const int rc = splits > 1 ? fc_reduce(ctx, post) : CCT_OK;
+    plan->timer.end(0, ctx->stream);
+    return rc;
+  }
   if (plan->Wp) {
     fc_pad(ctx, X, plan->Xp, B, K, K4);
     fc_pad(ctx, W, plan->Wp, O, K, K4);
@@ -738,6 +769,23 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   const float *Xm = X, *dYm = dY;
   // ---- weight gradient: out = dW[o][k] (m = k, n = o), reduction over the batch; both operands MN-major
   plan->timer.begin(1, ctx->stream);
+  if (plan->small) {
+    FcSmallParams S{X, dY, K, O, 1, 1, K, O, B, B, dW, K, plan->bias ? db : nullptr, FcReduceParams{}};
+    fc_small(ctx, S, 1);
+    plan->timer.end(1, ctx->stream);
+    CCT_CHECK_LAUNCH(ctx);
+    if (!dX) return CCT_OK;
+    plan->timer.begin(3, ctx->stream);
+    const int splits = plan->small_dgr;
+    const FcReduceParams post{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4, splits, 0};
+    FcSmallParams D{W, dY, K, O, 1, 0, K, B, O, fc_round_up((O + splits - 1) / splits, 32), splits > 1 ? plan->partial : dX,
+                    splits > 1 ? K4 : K, nullptr, post};
+    fc_small(ctx, D, splits);
+    CCT_CHECK_LAUNCH(ctx);
+    const int rc = splits > 1 ? fc_reduce(ctx, post) : CCT_OK;
+    plan->timer.end(3, ctx->stream);
+    return rc;
+  }
   if (plan->Xp) { fc_pad(ctx, X, plan->Xp, B, K, K4); Xm = plan->Xp; }
   if (plan->dYp) { fc_pad(ctx, dY, plan->dYp, B, O, O4); dYm = plan->dYp; }
   const bool direct = K4 != K || !fc_aligned({dW});  // an output no tensor map describes

@@ -4,14 +4,11 @@ and an output Layer - and the same forward() / backward() pair as PhysicalOperat
 A network may mark a bridge's pass as folded into a neighbouring contraction (skip_forward / skip_backward); the bridge
 then does nothing in that pass.
 """
-import ctypes as C
-
 import numpy as np
 
 from . import capi
 from .bridge import LogicalCube, Tracked
 
-_vp = C.c_void_p
 
 
 class _Bridge(Tracked):
@@ -38,14 +35,14 @@ class ReLUBridge(_Bridge):
         if self.skip_forward:
             return
         x, y = self.p_input_layer.p_data_cube, self.p_output_layer.p_data_cube
-        capi.check(self.lib.cct_relu_forward(self.ctx.h, _vp(x.ptr), _vp(y.ptr), x.n_elements), "cct_relu_forward", self.ctx.h)
+        capi.check(self.lib.cct_relu_forward(self.ctx.h, x.ptr, y.ptr, x.n_elements), "cct_relu_forward", self.ctx.h)
 
     def backward(self):
         if self.skip_backward or not self.needs_to_calc_backward_grad:
             return
         y = self.p_output_layer.p_data_cube
         dy, dx = self.p_output_layer.p_gradient_cube, self.p_input_layer.p_gradient_cube
-        capi.check(self.lib.cct_relu_backward(self.ctx.h, _vp(y.ptr), _vp(dy.ptr), _vp(dx.ptr), y.n_elements),
+        capi.check(self.lib.cct_relu_backward(self.ctx.h, y.ptr, dy.ptr, dx.ptr, y.n_elements),
                    "cct_relu_backward", self.ctx.h)
 
 
@@ -63,7 +60,7 @@ class MaxPoolingBridge(_Bridge):
 
     def forward(self):
         x, y = self.p_input_layer.p_data_cube, self.p_output_layer.p_data_cube
-        capi.check(self.lib.cct_maxpool_forward(self.ctx.h, _vp(x.ptr), _vp(y.ptr), _vp(self.max_index.ptr),
+        capi.check(self.lib.cct_maxpool_forward(self.ctx.h, x.ptr, y.ptr, self.max_index.ptr,
                                                 self.iB * self.iD, self.iR, self.kernel_size, self.stride),
                    "cct_maxpool_forward", self.ctx.h)
 
@@ -71,7 +68,7 @@ class MaxPoolingBridge(_Bridge):
         if self.skip_backward or not self.needs_to_calc_backward_grad:
             return
         dy, dx = self.p_output_layer.p_gradient_cube, self.p_input_layer.p_gradient_cube
-        capi.check(self.lib.cct_maxpool_backward(self.ctx.h, _vp(dy.ptr), _vp(self.max_index.ptr), _vp(dx.ptr),
+        capi.check(self.lib.cct_maxpool_backward(self.ctx.h, dy.ptr, self.max_index.ptr, dx.ptr,
                                                  self.iB * self.iD, self.iR, self.kernel_size, self.stride),
                    "cct_maxpool_backward", self.ctx.h)
 
@@ -95,7 +92,7 @@ class LRNBridge(_Bridge):
 
     def forward(self):
         x, y = self.p_input_layer.p_data_cube, self.p_output_layer.p_data_cube
-        capi.check(self.lib.cct_lrn_forward(self.ctx.h, _vp(x.ptr), _vp(y.ptr), _vp(self.denoms.ptr if self.denoms else None),
+        capi.check(self.lib.cct_lrn_forward(self.ctx.h, x.ptr, y.ptr, self.denoms.ptr if self.denoms else None,
                                             self.iB, self.iD, self.iR * self.iC, self.local_size, self.alpha, self.beta),
                    "cct_lrn_forward", self.ctx.h)
 
@@ -104,8 +101,8 @@ class LRNBridge(_Bridge):
             return
         x, y = self.p_input_layer.p_data_cube, self.p_output_layer.p_data_cube
         dy, dx = self.p_output_layer.p_gradient_cube, self.p_input_layer.p_gradient_cube
-        capi.check(self.lib.cct_lrn_backward(self.ctx.h, _vp(x.ptr), _vp(y.ptr), _vp(self.denoms.ptr if self.denoms else None),
-                                             _vp(dy.ptr), _vp(dx.ptr), self.iB, self.iD, self.iR * self.iC, self.local_size,
+        capi.check(self.lib.cct_lrn_backward(self.ctx.h, x.ptr, y.ptr, self.denoms.ptr if self.denoms else None,
+                                             dy.ptr, dx.ptr, self.iB, self.iD, self.iR * self.iC, self.local_size,
                                              self.alpha, self.beta), "cct_lrn_backward", self.ctx.h)
 
     def close(self):
@@ -138,7 +135,7 @@ class DropoutBridge(_Bridge):
         if self.injected or self.mask_held:
             return
         self.calls += 1
-        capi.check(self.lib.cct_dropout_mask(self.ctx.h, _vp(self.mask_cube.ptr), self.mask_cube.n_elements,
+        capi.check(self.lib.cct_dropout_mask(self.ctx.h, self.mask_cube.ptr, self.mask_cube.n_elements,
                                              self.dropout_ratio, self.random_seed, self.calls), "cct_dropout_mask", self.ctx.h)
 
     def forward(self):
@@ -146,14 +143,14 @@ class DropoutBridge(_Bridge):
         if self.skip_forward:
             return
         x, y = self.p_input_layer.p_data_cube, self.p_output_layer.p_data_cube
-        capi.check(self.lib.cct_dropout_apply(self.ctx.h, _vp(x.ptr), _vp(self.mask_cube.ptr), self.scale, _vp(y.ptr),
+        capi.check(self.lib.cct_dropout_apply(self.ctx.h, x.ptr, self.mask_cube.ptr, self.scale, y.ptr,
                                               x.n_elements), "cct_dropout_apply", self.ctx.h)
 
     def backward(self):
         if self.skip_backward or not self.needs_to_calc_backward_grad:
             return
         dy, dx = self.p_output_layer.p_gradient_cube, self.p_input_layer.p_gradient_cube
-        capi.check(self.lib.cct_dropout_apply(self.ctx.h, _vp(dy.ptr), _vp(self.mask_cube.ptr), self.scale, _vp(dx.ptr),
+        capi.check(self.lib.cct_dropout_apply(self.ctx.h, dy.ptr, self.mask_cube.ptr, self.scale, dx.ptr,
                                               dy.n_elements), "cct_dropout_apply", self.ctx.h)
 
     def close(self):
@@ -177,13 +174,13 @@ class SoftmaxLossBridge(_Bridge):
 
     def forward(self):
         x, y = self.p_input_layer.p_data_cube, self.p_output_layer.p_data_cube
-        capi.check(self.lib.cct_softmax_loss_forward(self.ctx.h, _vp(x.ptr), _vp(self.p_data_labels.ptr), _vp(y.ptr),
-                                                     _vp(self.image_loss.ptr), _vp(self.loss_cube.ptr), self.iB,
+        capi.check(self.lib.cct_softmax_loss_forward(self.ctx.h, x.ptr, self.p_data_labels.ptr, y.ptr,
+                                                     self.image_loss.ptr, self.loss_cube.ptr, self.iB,
                                                      self.classes), "cct_softmax_loss_forward", self.ctx.h)
 
     def backward(self):
         y, dx = self.p_output_layer.p_data_cube, self.p_input_layer.p_gradient_cube
-        capi.check(self.lib.cct_softmax_loss_backward(self.ctx.h, _vp(y.ptr), _vp(self.p_data_labels.ptr), _vp(dx.ptr),
+        capi.check(self.lib.cct_softmax_loss_backward(self.ctx.h, y.ptr, self.p_data_labels.ptr, dx.ptr,
                                                       self.iB, self.classes, 1.0 / self.loss_batch),
                    "cct_softmax_loss_backward", self.ctx.h)
 
@@ -195,7 +192,7 @@ class SoftmaxLossBridge(_Bridge):
         """Queues the copy of the summed loss (one float) into pinned host memory at `host_ptr`, behind the kernels already
         on the stream, without waiting for it: a training loop reads the value once the stream has passed that point
         (an event, or the next synchronisation) and so never stalls the launches of the following iteration."""
-        capi.check(self.lib.cct_memcpy_d2h(self.ctx.h, _vp(host_ptr), _vp(self.loss_cube.ptr), 4), "cct_memcpy_d2h", self.ctx.h)
+        capi.check(self.lib.cct_memcpy_d2h(self.ctx.h, host_ptr, self.loss_cube.ptr, 4), "cct_memcpy_d2h", self.ctx.h)
 
     def close(self):
         self.image_loss.free()
