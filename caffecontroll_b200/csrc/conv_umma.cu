@@ -125,6 +125,11 @@ constexpr int kEpiWarps = 4;
 __host__ __device__ constexpr int gather_threads(int sets) { return (4 * sets + 2 + kEpiWarps) * 32; }  // 704 or 448
 constexpr int kMaxAStages = 4, kMaxAccBufs = 2;
 
+// Channels per table entry where the gathered tensor's channels per group are a multiple of it.  One table read, one bounds
+// test and one branch then serve kRun loads of consecutive channels, and the taps of the same kRun channels follow one
+// another, so that they still find their lines in L1 (the channels of two CTAs' tiles all at once would not fit it).
+constexpr int kRun = 8;
+
 struct alignas(8) ColEnt {  // one accumulator column -> where it lands in the output
   int off;       // element offset from the pixel's output origin
   short cy, cx;  // displacement of the output pixel (depth-to-space), for the bounds test
@@ -165,11 +170,11 @@ struct GatherParams {
   // Weight-gradient mode: the TMEM lanes are rows of the lowered matrix (taps), the reduction runs over pixels.
   // `taps` then points to a table in global memory with one entry per pixel (offset of the pixel's tap origin and
   // the set of tap rows / columns that fall outside the plane there), `out` to the split partial sums.
-  int wg;
   int wg_mtiles, wg_vgroups;  // tiles = splits x channel tiles x M-tiles (M-tile fastest)
   int wg_rows_pad;            // rows of one split's partial-sum slice (M-tiles * 128)
   int wg_k, wg_kreal;         // kernel size, real rows of the lowered matrix
   int taps_smem;              // entries of `taps` staged in shared memory (0 in weight-gradient mode)
+  int run_stride;             // kByRun: elements between consecutive channels of the gathered tensor
   int* status;
 };
 
@@ -177,9 +182,10 @@ struct GatherParams {
 struct TileId {
   int vg, ptile, kb0, split;
 };
+template <bool WG>
 __device__ __forceinline__ TileId decode_tile(const GatherParams& P, int t, int kblocks) {
   TileId id;
-  if (!P.wg) {
+  if (!WG) {
     const int r = t / P.n_pix_tiles, vgroups = P.total_tiles / (P.n_pix_tiles * P.splits);
     id.ptile = t - r * P.n_pix_tiles;
     id.split = P.splits == 1 ? 0 : r / vgroups;
@@ -212,7 +218,10 @@ __host__ __device__ inline GatherSmem gather_smem(int n_pad, int k_pad, int b_st
   return L;
 }
 
-template <int SETS>
+// MODE: what the lanes gather - one table entry per reduction index, one per kRun of them, or (weight gradient) rows of the
+// lowered matrix over pixels.
+enum { kByTap = 0, kByRun = 1, kWeightGrad = 2 };
+template <int SETS, int MODE>
 __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     gather_conv_kernel(const __grid_constant__ GatherParams P, const __grid_constant__ CUtensorMap w_map) {
   pdl_wait();
@@ -221,7 +230,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const GatherSmem L = gather_smem(P.n_pad, P.taps_smem, P.b_stages, P.n_bias, P.wg ? kProducerWarps : 0);
+  const GatherSmem L = gather_smem(P.n_pad, P.taps_smem, P.b_stages, P.n_bias, MODE == kWeightGrad ? kProducerWarps : 0);
   const uint32_t bars = base + L.bars_off;
   // K-block i (running index over this CTA's tiles) uses A slot i % a_stages, weight slot i % b_stages and the
   // barrier pair i % 4: "ready" completes when the four producer warps of the block's set and the weight tile's TMA
@@ -270,10 +279,10 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     const MaskTap* tile_taps = s_taps;   // forward / data gradient: this tile's part of the tap table
     auto setup_tile = [&](int tile_local) {
       const int t = blockIdx.x + tile_local * gridDim.x;
-      const TileId id = decode_tile(P, t, kblocks);
+      const TileId id = decode_tile<MODE == kWeightGrad>(P, t, kblocks);
       const int grp = id.vg / P.tiles_per_group;
       in_px = P.in;
-      if (P.wg) {
+      if (MODE == kWeightGrad) {
         // lane = row of the lowered matrix: (d, kr, kc); `mask` holds the tap's row and column bit
         const int r = id.ptile * kTileM + row;
         mask = kPadBit;
@@ -287,7 +296,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         pix_tab = P.taps + (size_t)id.kb0 * kBlockK;
         return;
       }
-      tile_taps = s_taps + id.kb0 * kBlockK;
+      tile_taps = s_taps + id.kb0 * (kBlockK / (MODE == kByRun ? kRun : 1));
       const int pix = id.ptile * kTileM + row;
       mask = 0;  // which tap rows (bits 0-14) and tap columns (bits 16-30) fall inside the plane
       if (pix < P.n_pix) {
@@ -315,10 +324,10 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     uint2* my_ptab = reinterpret_cast<uint2*>(base_ptr + L.ptab_off) + warp * 64;
     int pbuf = 0;
     auto prefetch_entries = [&](int kb) {
-      if (P.wg) ent_next = __ldg(reinterpret_cast<const uint2*>(pix_tab + kb * kBlockK) + lane);
+      if (MODE == kWeightGrad) ent_next = __ldg(reinterpret_cast<const uint2*>(pix_tab + kb * kBlockK) + lane);
     };
     auto gather = [&](int kb) {
-      if (P.wg) {
+      if (MODE == kWeightGrad) {
         // entry = (offset of the pixel's tap origin, tap rows / columns out of bounds there)
         uint2* slot = my_ptab + pbuf * 32;
         pbuf ^= 1;
@@ -328,6 +337,21 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         for (int e = 0; e < kBlockK; ++e) {
           const uint2 ent = slot[e];
           v[e] = ldg_if_clear(in_px + (int)ent.x, ent.y, mask);
+        }
+        return;
+      }
+      if (MODE == kByRun) {
+        const MaskTap* tp = tile_taps + kb * (kBlockK / kRun);
+#pragma unroll
+        for (int r = 0; r < kBlockK / kRun; ++r) {
+          const MaskTap tap = tp[r];
+#pragma unroll
+          for (int e = 0; e < kRun; ++e) v[r * kRun + e] = 0.f;
+          if ((mask & tap.bits) == tap.bits) {
+            const float* p = in_px + tap.off;
+#pragma unroll
+            for (int e = 0; e < kRun; ++e) v[r * kRun + e] = __ldg(p + e * P.run_stride);
+          }
         }
         return;
       }
@@ -435,7 +459,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       Ring rb;
       int i = 0;  // running k-block index
       for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x) {
-        const TileId id = decode_tile(P, t, kblocks);
+        const TileId id = decode_tile<MODE == kWeightGrad>(P, t, kblocks);
         const int vg = id.vg;
         for (int kb = 0; kb < kblocks; ++kb, ++i) {
           const int sb = rb.idx;
@@ -456,11 +480,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     const int row = quarter * 32 + lane;
     int tile_iter = 0;
     for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x, ++tile_iter) {
-      const TileId id = decode_tile(P, t, kblocks);
+      const TileId id = decode_tile<MODE == kWeightGrad>(P, t, kblocks);
       const int vg = id.vg, ptile = id.ptile;
       const int grp = vg / P.tiles_per_group, ntile = vg % P.tiles_per_group;
       const int buf = tile_iter & (P.acc_bufs - 1), ause = tile_iter >> (P.acc_bufs - 1);
-      if (P.wg) {
+      if (MODE == kWeightGrad) {
         // The accumulator is a 128-row slice of this split's partial sums: row-contiguous stores.
         mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
         tc_fence_after();
@@ -1280,7 +1304,8 @@ __device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, co
 // Forward B operand: [2 (hi, lo)][vg][n_pad][k_pad] <- W[o][Dg*k*k], zero padded.
 __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                 float* __restrict__ lo, int tiles_per_group, int og,
-                                                                int n_real, int n_pad, int k_real, int k_pad) {
+                                                                int n_real, int n_pad, int k_real, int k_pad, int run,
+                                                                int window) {
   pdl_wait();
   const int vg = blockIdx.y / n_pad, j = blockIdx.y - vg * n_pad;
   const int ch = (vg % tiles_per_group) * n_real + j;  // inside the group
@@ -1290,7 +1315,12 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
   for (int kk = (blockIdx.x * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.x * kPackThreads * 4) {
     float v[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] = (live && kk + e < k_real) ? __ldg(src + kk + e) : 0.f;
+    for (int e = 0; e < 4; ++e) {
+      // reduction index -> (channel / run, tap, channel % run) -> element (channel, tap) of the filter
+      const int i = kk + e, r = i / run, chunk = r / window;
+      const int at = run == 1 ? i : (chunk * run + (i - r * run)) * window + (r - chunk * window);
+      v[e] = (live && i < k_real) ? __ldg(src + at) : 0.f;
+    }
     store_split4(hi, lo, row + kk, v);
   }
 }
@@ -1301,7 +1331,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
 __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                   float* __restrict__ lo, int tiles_per_group, int og,
                                                                   int Dg, int k, int s, int taps, int d_tile, int n_real,
-                                                                  int n_pad, int k_real, int k_pad) {
+                                                                  int n_pad, int k_real, int k_pad, int run) {
   pdl_wait();
   const int vg = blockIdx.y / n_pad, j = blockIdx.y - vg * n_pad;
   const int grp = vg / tiles_per_group, d = (vg - grp * tiles_per_group) * d_tile + j / (s * s);
@@ -1310,16 +1340,14 @@ __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* _
   const float* src = W + ((size_t)grp * og * Dg + d) * k * k;
   const size_t row = (size_t)blockIdx.y * k_pad;
   for (int kk = (blockIdx.x * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.x * kPackThreads * 4) {
-    int oc = kk / (taps * taps), jy = (kk - oc * taps * taps) / taps, jx = kk % taps;
     float v[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
+      // reduction index -> (filter / run, jy, jx, filter % run)
+      const int r = (kk + e) / run, chunk = r / (taps * taps), tap = r - chunk * taps * taps;
+      const int oc = chunk * run + (kk + e - r * run), jy = tap / taps, jx = tap - jy * taps;
       const int kr = py + jy * s, kc = px + jx * s;
       v[e] = (live && kk + e < k_real && kr < k && kc < k) ? __ldg(src + (size_t)oc * Dg * k * k + kr * k + kc) : 0.f;
-      if (++jx == taps) {
-        jx = 0;
-        if (++jy == taps) { jy = 0; ++oc; }
-      }
     }
     store_split4(hi, lo, row + kk, v);
   }
@@ -1360,7 +1388,7 @@ struct GatherTiling {
   int tiles = 0, splits = 1, kps = 0;
 };
 GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, int channels, int cols_per_channel, int kblocks,
-                                  int n_bias) {
+                                  int run, int n_bias) {
   GatherTiling best;
   double best_us = 0.0;
   const int t0 = channel_tiles(channels, cols_per_channel);
@@ -1369,7 +1397,7 @@ GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, in
     if (t > t0 && n_pad < 32) break;
     if ((channels + t - 1) / t * (t - 1) >= channels) continue;  // the last tile would be empty
     int slots_unused;
-    const bool two = two_ctas_per_sm(n_pad, kblocks * kBlockK, n_bias, 0, &slots_unused), dual = n_pad <= 64;
+    const bool two = two_ctas_per_sm(n_pad, kblocks * kBlockK / run, n_bias, 0, &slots_unused), dual = n_pad <= 64;
     const int mmas = dual ? 8 : 12;
     const double mhz = 1600.0, exec = mmas * (dual ? n_pad : n_pad / 2.0) / mhz, issue = mmas * 75 / mhz;  // clock under load
     const double alone = std::max({exec, issue, two ? 0.62 : 0.35}), shared = two ? std::max({2 * exec, issue, 0.8}) : alone;
@@ -1406,6 +1434,7 @@ struct GatherProblem {
   int taps_smem = -1;             // tap-table entries staged in shared memory (-1: k_pad)
   size_t map_k = 0;               // extent of the packed operand along the reduction (0: k_pad)
   size_t smem = 0;
+  int run = 1, run_stride = 0;    // reduction order: 1 = (channel, tap); kRun = (channel / kRun, tap, channel % kRun)
   int splits = 1, split_k = 0;    // splits of the reduction and the length of one (a multiple of 32; k_pad without splits)
   float* partial = nullptr;       // split sums
   size_t pix_pad = 0;
@@ -1529,7 +1558,7 @@ bool use_small_wgrad(long long pixels, int vgroups, int n, int k_real) {
 void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias) {
   // Tensor memory (512 columns) = accumulator buffers + A stages of 64 columns.  Narrow problems run "dual" (see the
   // MMA loop): their accumulator is 2*n_pad wide.  Two accumulator buffers let the epilogue overlap the next tile.
-  const int taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k : gp.taps_smem;
+  const int taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k / gp.run : gp.taps_smem;
   const size_t map_k = gp.map_k ? gp.map_k : (size_t)gp.k_pad;
   gp.dual = gp.n_pad <= 64;  // 2 MMAs of width <= 128 instead of 3 narrow ones; wider ones gain nothing
   gp.acc_cols = gp.dual ? 2 * gp.n_pad : gp.n_pad;
@@ -1582,16 +1611,17 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     GatherProblem& f = p->fwd;
     f.k_real = G.Dg * kk;
     f.k_pad = round_up(f.k_real, kBlockK);
+    f.run = G.Dg % kRun == 0 ? kRun : 1; f.run_stride = G.n * G.n;
     const long long pixel_tiles = ((long long)G.B * G.m * G.m + kTileM - 1) / kTileM;
-    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, G.bias ? G.o : 0);
+    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, f.run, G.bias ? G.o : 0);
     f.tiles = tl.tiles;
     f.ch_tile = f.n = (G.og + f.tiles - 1) / f.tiles;
     f.n_pad = round_up(f.n, 16);
     f.splits = tl.splits; f.split_k = tl.kps * kBlockK; f.pix_pad = (size_t)pixel_tiles * kTileM;
-    std::vector<MaskTap> t((size_t)f.splits * f.split_k);  // padding entries behind the last split's real ones
+    std::vector<MaskTap> t((size_t)f.splits * f.split_k / f.run);  // padding entries behind the last split's real ones
     for (int i = 0; i < (int)t.size(); ++i) {
-      if (i < f.k_real) {
-        const int d = i / kk, kr = (i / G.k) % G.k, kc = i % G.k;
+      if (i * f.run < f.k_real) {
+        const int d = i / kk * f.run, kr = (i / G.k) % G.k, kc = i % G.k;
         t[i] = MaskTap{d * G.n * G.n + kr * G.n + kc, (1u << kr) | (1u << (16 + kc))};
       } else {
         t[i] = MaskTap{0, kPadBit};
@@ -1618,17 +1648,18 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     const int J = p->dgr_taps;
     d.k_real = G.og * J * J;
     d.k_pad = round_up(d.k_real, kBlockK);
+    d.run = G.og % kRun == 0 ? kRun : 1; d.run_stride = G.m * G.m;
     const long long pixel_tiles = ((long long)G.B * p->dgr_q * p->dgr_q + kTileM - 1) / kTileM;
-    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.Dg, ss, d.k_pad / kBlockK, 0);
+    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.Dg, ss, d.k_pad / kBlockK, d.run, 0);
     d.tiles = tl.tiles;
     d.ch_tile = (G.Dg + d.tiles - 1) / d.tiles;
     d.n = d.ch_tile * ss;
     d.n_pad = round_up(d.n, 16);
     d.splits = tl.splits; d.split_k = tl.kps * kBlockK; d.pix_pad = (size_t)pixel_tiles * kTileM;
-    std::vector<MaskTap> t((size_t)d.splits * d.split_k);
+    std::vector<MaskTap> t((size_t)d.splits * d.split_k / d.run);
     for (int i = 0; i < (int)t.size(); ++i) {
-      if (i < d.k_real) {
-        const int jx = i % J, jy = (i / J) % J, oc = i / (J * J);
+      if (i * d.run < d.k_real) {
+        const int jx = i % J, jy = (i / J) % J, oc = i / (J * J) * d.run;
         t[i] = MaskTap{oc * G.m * G.m - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
       } else {
         t[i] = MaskTap{0, kPadBit};
@@ -1784,8 +1815,10 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       rc = CCT_ERR_CUDA;
     }
   }
-  if (rc == CCT_OK) rc = set_smem(ctx, gather_conv_kernel<4>, kSmemLimit);
-  if (rc == CCT_OK) rc = set_smem(ctx, gather_conv_kernel<2>, 113 * 1024);
+  for (auto kernel : {gather_conv_kernel<4, kByTap>, gather_conv_kernel<4, kByRun>, gather_conv_kernel<4, kWeightGrad>})
+    if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
+  for (auto kernel : {gather_conv_kernel<2, kByTap>, gather_conv_kernel<2, kByRun>, gather_conv_kernel<2, kWeightGrad>})
+    if (rc == CCT_OK) rc = set_smem(ctx, kernel, 113 * 1024);
   if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad), kSmemLimit);
   if (rc == CCT_OK && p->w_ts) rc = set_smem(ctx, wgrad_ts_kernel, kSmemLimit);
   if (rc != CCT_OK) {
@@ -1813,7 +1846,8 @@ void fill_common(GatherParams& P, const GatherProblem& gp, cct_ctx* ctx, int vgr
   P.n = gp.n; P.n_pad = gp.n_pad; P.k_pad = gp.split_k ? gp.split_k : gp.k_pad;
   P.cols_per_channel = gp.n / gp.ch_tile;
   P.splits = gp.splits; P.partial = gp.partial; P.pix_pad = (int)gp.pix_pad;
-  P.taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k : gp.taps_smem;
+  P.taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k / gp.run : gp.taps_smem;
+  P.run_stride = gp.run_stride;
   P.n_pix_tiles = (P.n_pix + kTileM - 1) / kTileM;
   P.total_tiles = P.n_pix_tiles * vgroups * gp.splits;
   P.a_stages = gp.a_stages; P.b_stages = gp.b_stages; P.acc_bufs = gp.acc_bufs;
@@ -1842,13 +1876,17 @@ void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct) {
 }
 
 // Persistent grid: one CTA per SM (4 producer sets) or two (2 sets); then the reduction over the splits, if any.
-void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp) {
-  if (gp.sets == 2) {
-    const int grid = std::min(P.total_tiles, 2 * ctx->launch_sms());
-    launch_pdl(gather_conv_kernel<2>, dim3(grid), dim3(gather_threads(2)), gp.smem, ctx->stream, P, gp.map);
+void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp, bool weight_grad = false) {
+  auto go = [&](auto kernel, int sets) {
+    const int grid = std::min(P.total_tiles, (sets == 2 ? 2 : 1) * ctx->launch_sms());
+    launch_pdl(kernel, dim3(grid), dim3(gather_threads(sets)), gp.smem, ctx->stream, P, gp.map);
+  };
+  if (weight_grad) {
+    if (gp.sets == 2) go(gather_conv_kernel<2, kWeightGrad>, 2); else go(gather_conv_kernel<4, kWeightGrad>, 4);
+  } else if (gp.run == kRun) {
+    if (gp.sets == 2) go(gather_conv_kernel<2, kByRun>, 2); else go(gather_conv_kernel<4, kByRun>, 4);
   } else {
-    const int grid = std::min(P.total_tiles, ctx->launch_sms());
-    launch_pdl(gather_conv_kernel<4>, dim3(grid), dim3(gather_threads(4)), gp.smem, ctx->stream, P, gp.map);
+    if (gp.sets == 2) go(gather_conv_kernel<2, kByTap>, 2); else go(gather_conv_kernel<4, kByTap>, 4);
   }
   if (P.splits > 1) {
     const int vgroups = P.total_tiles / (P.n_pix_tiles * P.splits), cols = P.n_pix_tiles * vgroups * P.n > 32 * ctx->sm_count ? 8 : 1;
@@ -1878,7 +1916,7 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
   if (repack) {
     t->begin(4, ctx->stream);
     launch_pdl(pack_fwd_kernel, pack_grid(vgroups * f.n_pad, f.k_pad), dim3(kPackThreads), 0, ctx->stream, W, f.w,
-               f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad);
+               f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad, f.run, G.k * G.k);
     t->end(4, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   }
@@ -1930,12 +1968,12 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     P.n_pix = p->wg_mtiles * kTileM;  // lanes = rows of the lowered matrix
     P.in_lim = G.n;
     P.in_group_stride = G.Dg * G.n * G.n;
-    P.wg = 1; P.wg_mtiles = p->wg_mtiles; P.wg_vgroups = vgroups; P.wg_rows_pad = p->wg_mtiles * kTileM;
+    P.wg_mtiles = p->wg_mtiles; P.wg_vgroups = vgroups; P.wg_rows_pad = p->wg_mtiles * kTileM;
     P.wg_k = G.k; P.wg_kreal = f.k_real;
     fill_common(P, w, ctx, vgroups, 0);
     P.taps = p->wg_pix; P.cols = nullptr;
     P.total_tiles = p->wg_splits * vgroups * p->wg_mtiles;
-    launch_gather(ctx, P, w);
+    launch_gather(ctx, P, w, true);
     t->end(1, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
     t->begin(2, ctx->stream);
@@ -2002,7 +2040,7 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
     }
     if (repack) {
       launch_pdl(pack_dgrad_kernel, pack_grid(vgroups * d.n_pad, d.k_pad), dim3(kPackThreads), 0, ctx->stream, W, d.w,
-                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad);
+                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run);
       CCT_CHECK_LAUNCH(ctx);
     }
     GatherParams P{};
