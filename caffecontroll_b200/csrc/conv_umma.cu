@@ -162,8 +162,6 @@ struct GatherParams {
   int n_pix_tiles, total_tiles;
   int a_stages, b_stages, acc_bufs;
   int tmem_cols;           // tensor-memory columns this CTA allocates: 512, or 256 when two CTAs share an SM
-  int dual;                // 1: one MMA covers [B_hi; B_lo] (N = 2*n_pad) and the epilogue adds the two halves
-  int acc_cols;            // accumulator width in tensor-memory columns: n_pad, or 2*n_pad when dual
   int n_bias;              // entries of `bias` (all output channels), staged in shared memory
   int lo_row_offset;       // first row of the "lo" half inside the packed-weight tensor map
   int relu;
@@ -242,7 +240,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   MaskTap* s_taps = reinterpret_cast<MaskTap*>(base_ptr + L.taps_off);
   ColEnt* s_cols = reinterpret_cast<ColEnt*>(base_ptr + L.cols_off);
   float* s_bias = reinterpret_cast<float*>(base_ptr + L.bias_off);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
 
   for (int i = tid; i < P.taps_smem; i += kGatherThreads) s_taps[i] = P.taps[i];
   if (P.cols)
@@ -259,7 +257,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-  const uint32_t a_col0 = (uint32_t)(P.acc_bufs * P.acc_cols);
+  const uint32_t a_col0 = (uint32_t)(P.acc_bufs * P.n_pad);
   const int kblocks = P.k_pad / kBlockK;
   bool failed = false;
 
@@ -369,9 +367,13 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       prefetch_entries(kb);
       gather(kb);
     }
+    int ring_sa = group % P.a_stages;  // A slot of the set's current k-block: index % a_stages
     for (int it = group; it < my_stages; it += SETS) {
-      const int sa = it & (P.a_stages - 1);  // a_stages is 2 or 4
+      // a weight gradient's ring is 2 or 4 deep: no counter (its producers have no register to spare)
+      const int sa = MODE == kWeightGrad ? it & (P.a_stages - 1) : ring_sa;
       const uint32_t st_addr = lane_addr + (uint32_t)(sa * 64);
+      if (MODE != kWeightGrad)
+        for (ring_sa += SETS; ring_sa >= P.a_stages;) ring_sa -= P.a_stages;
       // The set's next k-block: its tile state and (weight gradient) its table entries, requested now so that
       // they have arrived when the gather is issued further down.  v[] still holds the current block.
       const bool has_next = it + SETS < my_stages;
@@ -394,15 +396,15 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         tmem_st8(st_addr + (uint32_t)(c * 8), hi);
         tmem_st8(st_addr + 32u + (uint32_t)(c * 8), lo);
       }
-      // With two stages the hand-over of a filled stage is on the critical path: arrive first, then fetch.
-      if (P.a_stages == 2) {
+      // With few stages the hand-over of a filled stage is on the critical path: arrive first, then fetch.
+      if (P.a_stages < 4) {
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(ready_bar + 8u * (it & 3));
       }
       if (has_next) gather(kb);  // loads in flight across the next wait
-      if (P.a_stages != 2) {
+      if (P.a_stages == 4) {
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -410,47 +412,36 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       }
     }
   } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------------ MMA issue
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(P.acc_cols);
-      int tile_iter = 0;
-      Ring ra, rb, rbar;  // A slot, weight slot, barrier pair of the current k-block
-      for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x, ++tile_iter) {
-        const int buf = tile_iter & (P.acc_bufs - 1), ause = tile_iter >> (P.acc_bufs - 1);  // acc_bufs is 1 or 2
-        if (ause > 0) mbar_wait<false>(acc_empty + 8u * buf, (uint32_t)(ause - 1) & 1u, failed, P.status, 0x20);
+    // ------------------------------------------------------------------ MMA issue (see elect_one)
+    const uint32_t idesc = make_idesc(P.n_pad), tmem = warp_uniform(tmem_base);
+    int tile_iter = 0;
+    Ring ra, rb, rbar;  // A slot, weight slot, barrier pair of the current k-block
+    for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x, ++tile_iter) {
+      const int buf = tile_iter & (P.acc_bufs - 1), ause = tile_iter >> (P.acc_bufs - 1);  // acc_bufs is 1 or 2
+      if (ause > 0) mbar_wait<false>(acc_empty + 8u * buf, (uint32_t)(ause - 1) & 1u, failed, P.status, 0x20);
+      tc_fence_after();
+      const uint32_t d_tmem = tmem + (uint32_t)(buf * P.n_pad);
+      for (int kb = 0; kb < kblocks; ++kb) {
+        mbar_wait<false>(ready_bar + 8u * rbar.idx, (uint32_t)rbar.use & 1u, failed, P.status, 0x40);
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * P.acc_cols);
-        for (int kb = 0; kb < kblocks; ++kb) {
-          mbar_wait<false>(ready_bar + 8u * rbar.idx, (uint32_t)rbar.use & 1u, failed, P.status, 0x40);
-          tc_fence_after();
-          const uint32_t b_hi = base + (uint32_t)rb.idx * L.b_stage_bytes, b_lo = b_hi + (uint32_t)P.n_pad * 128u;
-          const uint64_t dbh = make_desc(b_hi), dbl = make_desc(b_lo);
-          const uint32_t a_hi = tmem_base + a_col0 + (uint32_t)(ra.idx * 64), a_lo = a_hi + 32u;
-          if (P.dual) {
-            // The lo tile sits right behind the hi tile: one descriptor spans both, so a single MMA of width
-            // 2*n_pad produces A*B_hi in the first n_pad columns and A*B_lo in the next (issuing an MMA costs
-            // this thread ~75 cycles however narrow it is, so two wide ones beat three narrow ones).
+        const uint32_t b_hi = base + (uint32_t)rb.idx * L.b_stage_bytes, b_lo = b_hi + (uint32_t)P.n_pad * 128u;
+        const uint64_t dbh = make_desc(b_hi), dbl = make_desc(b_lo);
+        const uint32_t a_hi = tmem + a_col0 + (uint32_t)(ra.idx * 64), a_lo = a_hi + 32u;
+        if (elect_one()) {
 #pragma unroll
-            for (int j = 0; j < kBlockK / 8; ++j) {
-              const uint64_t adv = (uint64_t)(j * 2);
-              umma_tf32_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kb == 0 && j == 0) ? 0u : 1u);
-              umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, 1u);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < kBlockK / 8; ++j) {
-              const uint64_t adv = (uint64_t)(j * 2);
-              umma_tf32_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kb == 0 && j == 0) ? 0u : 1u);
-              umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
-              umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, 1u);
-            }
+          for (int j = 0; j < kBlockK / 8; ++j) {
+            const uint64_t adv = (uint64_t)(j * 2);
+            umma_tf32_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kb == 0 && j == 0) ? 0u : 1u);
+            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
+            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, 1u);
           }
           umma_commit(done_bar + 8u * rbar.idx);  // frees the A slot for the producers and the weight slot for the TMA thread
-          ra.advance(P.a_stages);
-          rb.advance(P.b_stages);
-          rbar.advance(4);
+          if (kb == kblocks - 1) umma_commit(acc_full + 8u * buf);
         }
-        umma_commit(acc_full + 8u * buf);
+        __syncwarp();
+        ra.advance(P.a_stages);
+        rb.advance(P.b_stages);
+        rbar.advance(4);
       }
     }
   } else if (warp == kTmaWarp) {
@@ -488,17 +479,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         // The accumulator is a 128-row slice of this split's partial sums: row-contiguous stores.
         mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
         tc_fence_after();
-        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.acc_cols);
+        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.n_pad);
         float* op = P.out + ((size_t)(id.split * P.wg_vgroups + vg) * P.wg_rows_pad + (size_t)ptile * kTileM + row) * P.n_pad;
         for (int c = 0; c < P.n_pad / 16; ++c) {
           float v[16];
           tmem_ld16(acc + (uint32_t)(c * 16), v);
-          if (P.dual) {
-            float w[16];
-            tmem_ld16(acc + (uint32_t)(P.n_pad + c * 16), w);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] += w[j];
-          }
           if (!failed) {
             float4* o4 = reinterpret_cast<float4*>(op + c * 16);
 #pragma unroll
@@ -515,17 +500,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         // raw sums, lanes along the pixels
         mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
         tc_fence_after();
-        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.acc_cols);
+        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.n_pad);
         float* op = P.partial + (size_t)(id.split * (P.total_tiles / (P.n_pix_tiles * P.splits)) + vg) * P.n_pad * P.pix_pad + pix;
         for (int c = 0; c < P.n_pad / 16; ++c) {
           float v[16];
           tmem_ld16(acc + (uint32_t)(c * 16), v);
-          if (P.dual) {
-            float w[16];
-            tmem_ld16(acc + (uint32_t)(P.n_pad + c * 16), w);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] += w[j];
-          }
           if (!failed) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) op[(size_t)(c * 16 + j) * P.pix_pad] = v[j];
@@ -555,17 +534,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       tc_fence_after();
       const uint32_t live = (pix < P.n_pix && !failed) ? 1u : 0u;
       const uint32_t unchecked = P.check_out ? 0u : 1u;
-      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.acc_cols);
+      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.n_pad);
       const int chunks = P.n_pad / 16;
       for (int c = 0; c < chunks; ++c) {
         float v[16];
         tmem_ld16(acc + (uint32_t)(c * 16), v);
-        if (P.dual) {
-          float w[16];
-          tmem_ld16(acc + (uint32_t)(P.n_pad + c * 16), w);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] += w[j];
-        }
         // Straight-line code: table and bias reads first, then predicated st.global (a generic store could alias
         // shared memory and would pin every following table read behind it; a branch per column costs more than
         // the store it guards).
@@ -714,7 +687,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
   const uint32_t full = bars, empty = full + 8u * kWgMaxStages, acc_full = empty + 8u * kWgMaxStages,
                  tmem_slot = acc_full + 8u;
   MaskTap* s_taps = reinterpret_cast<MaskTap*>(base_ptr + L.taps_off);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
   const int mgroup = blockIdx.x, split = blockIdx.y, vg = blockIdx.z;
   const int grp = vg / P.tiles_per_group, ntile = vg % P.tiles_per_group;
   const int subs = min(SUBS, P.m_tiles - mgroup * SUBS);  // M-tiles this CTA really has
@@ -878,37 +851,34 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
     }
     }
   } else {
-    // ------------------------------------------------------------------ MMA issue
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(kAccCols);
-      Ring ring;
-      for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(P.stages)) {
-        const int s = ring.idx;
-        mbar_wait(full + 8u * s, (uint32_t)ring.use & 1u, failed, P.status, 0x40);  // parked: this thread mostly waits for the producers
-        tc_fence_after();
-        const uint32_t st = base + (uint32_t)s * L.stage_bytes;
-        const uint32_t b_hi = st + SUBS * 2u * kATile, b_lo = b_hi + kBTile;
-        const uint64_t dbh = make_desc(b_hi), dbl = make_desc(b_lo);
-        for (int u = 0; u < subs; ++u) {
-          const uint32_t d_tmem = tmem_base + (uint32_t)(u * kAccCols);
+    // ------------------------------------------------------------------ MMA issue (see elect_one)
+    const uint32_t idesc = make_idesc(kAccCols), tmem = warp_uniform(tmem_base);
+    const int n_subs = (int)warp_uniform((uint32_t)subs);
+    Ring ring;
+    for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(P.stages)) {
+      const int s = ring.idx;
+      mbar_wait(full + 8u * s, (uint32_t)ring.use & 1u, failed, P.status, 0x40);  // parked: this warp mostly waits for the producers
+      tc_fence_after();
+      const uint32_t st = base + (uint32_t)s * L.stage_bytes;
+      const uint32_t b_hi = st + SUBS * 2u * kATile, b_lo = b_hi + kBTile;
+      const uint64_t dbh = make_desc(b_hi), dbl = make_desc(b_lo);
+      if (elect_one()) {
+        for (int u = 0; u < n_subs; ++u) {
+          const uint32_t d_tmem = tmem + (uint32_t)(u * kAccCols);
           const uint32_t a_hi = st + (uint32_t)u * 2u * kATile;
           const uint64_t dah = make_desc(a_hi), dal = make_desc(a_hi + kATile);
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
             const uint64_t adv = (uint64_t)(j * 2);
-            if (kDual) {
-              umma_tf32_ss(d_tmem, dal + adv, dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
-              umma_tf32_ss(d_tmem, dah + adv, dbh + adv, idesc, 1u);
-            } else {
-              umma_tf32_ss(d_tmem, dal + adv, dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
-              umma_tf32_ss(d_tmem, dah + adv, dbl + adv, idesc, 1u);
-              umma_tf32_ss(d_tmem, dah + adv, dbh + adv, idesc, 1u);
-            }
+            umma_tf32_ss(d_tmem, dal + adv, dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
+            if (!kDual) umma_tf32_ss(d_tmem, dah + adv, dbl + adv, idesc, 1u);
+            umma_tf32_ss(d_tmem, dah + adv, dbh + adv, idesc, 1u);
           }
         }
         umma_commit(empty + 8u * s);
+        if (kbl == kblocks - 1) umma_commit(acc_full);
       }
-      umma_commit(acc_full);
+      __syncwarp();
     }
   }
   tc_fence_before();
@@ -1089,19 +1059,19 @@ __global__ void __launch_bounds__(kTsThreads, 1) wgrad_ts_kernel(const __grid_co
       }
     }
   } else {
-    // ------------------------------------------------------------------ MMA issue
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(kTsNTile);
-      Ring ring;
-      for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(kTsStages)) {
-        const int s = ring.idx;
-        mbar_wait(full + 8u * s, (uint32_t)ring.use & 1u, failed, P.status, 0x3040);
-        tc_fence_after();
-        const uint32_t st = base + (uint32_t)s * kTsStage;
-        const uint32_t a_hi = tmem_base + kACol0 + (uint32_t)(s * 64), a_lo = a_hi + 32u;
+    // ------------------------------------------------------------------ MMA issue (see elect_one)
+    const uint32_t idesc = make_idesc(kTsNTile), tmem = warp_uniform(tmem_base);
+    Ring ring;
+    for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(kTsStages)) {
+      const int s = ring.idx;
+      mbar_wait(full + 8u * s, (uint32_t)ring.use & 1u, failed, P.status, 0x3040);
+      tc_fence_after();
+      const uint32_t st = base + (uint32_t)s * kTsStage;
+      const uint32_t a_hi = tmem + kACol0 + (uint32_t)(s * 64), a_lo = a_hi + 32u;
+      if (elect_one()) {
 #pragma unroll
         for (int u = 0; u < kTsRows / kTsNTile; ++u) {
-          const uint32_t d_tmem = tmem_base + (uint32_t)(u * kTsNTile);
+          const uint32_t d_tmem = tmem + (uint32_t)(u * kTsNTile);
           const uint64_t dbh = make_desc(st + (uint32_t)u * kTsNTile * 128u), dbl = make_desc(st + kTsTile + (uint32_t)u * kTsNTile * 128u);
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
@@ -1112,8 +1082,9 @@ __global__ void __launch_bounds__(kTsThreads, 1) wgrad_ts_kernel(const __grid_co
           }
         }
         umma_commit(empty + 8u * s);
+        if (kbl == kblocks - 1) umma_commit(acc_full);
       }
-      umma_commit(acc_full);
+      __syncwarp();
     }
   }
   tc_fence_before();
@@ -1371,14 +1342,13 @@ int gather_slots(int n_pad, int taps_smem, int n_bias, int ptab, size_t limit) {
 // the accumulator is the full 128 columns (each MMA then lasts long enough to cover the refill: CaffeNet conv5 forward
 // 0.189 -> 0.153 ms).
 bool two_ctas_per_sm(int n_pad, int taps_smem, int n_bias, int ptab, int* slots) {
-  const int acc_cols = n_pad <= 64 ? 2 * n_pad : n_pad;
   *slots = gather_slots(n_pad, taps_smem, n_bias, ptab, 113 * 1024);
-  return acc_cols <= 128 && (*slots >= 3 || (*slots == 2 && acc_cols == 128));
+  return n_pad <= 128 && (*slots >= 3 || (*slots == 2 && n_pad == 128));
 }
 
 // Channel tiles and splits of the reduction for the forward pass and the data gradient, by an estimate of the kernel's
 // time in microseconds.  A work unit is (pixel tile, channel tile, split); units are spread over the resident CTAs in whole
-// rounds.  Per k-block a CTA takes what its MMAs take (75 cycles to issue one, half a cycle per column to run it), or what
+// rounds.  Per k-block a CTA takes what its MMAs take (half a cycle per column, 18 cycles at least), or what
 // its producers take to gather (measured: 0.62 us alone on an SM with two producer sets, 0.8 us when two CTAs share one,
 // 0.35 us with four sets); a unit adds an epilogue that grows with its columns (64 columns 1.3 us, 192 columns 2.8 us), a
 // split reduction one more kernel and the traffic of the sums.  So: a last round that is nearly empty (CaffeNet conv3 at
@@ -1397,10 +1367,9 @@ GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, in
     if (t > t0 && n_pad < 32) break;
     if ((channels + t - 1) / t * (t - 1) >= channels) continue;  // the last tile would be empty
     int slots_unused;
-    const bool two = two_ctas_per_sm(n_pad, kblocks * kBlockK / run, n_bias, 0, &slots_unused), dual = n_pad <= 64;
-    const int mmas = dual ? 8 : 12;
-    const double mhz = 1600.0, exec = mmas * (dual ? n_pad : n_pad / 2.0) / mhz, issue = mmas * 75 / mhz;  // clock under load
-    const double alone = std::max({exec, issue, two ? 0.62 : 0.35}), shared = two ? std::max({2 * exec, issue, 0.8}) : alone;
+    const bool two = two_ctas_per_sm(n_pad, kblocks * kBlockK / run, n_bias, 0, &slots_unused);
+    const double mhz = 1600.0, exec = 12 * std::max(n_pad / 2.0, 18.0) / mhz;  // clock under load
+    const double alone = std::max(exec, two ? 0.62 : 0.35), shared = two ? std::max(2 * exec, 0.8) : alone;
     const double epilogue = 0.5 + 0.012 * n_pad;
     for (int s = 1; s <= std::max(1, std::min(32, kblocks / 2)); ++s) {
       const int kps = (kblocks + s - 1) / s;
@@ -1429,7 +1398,7 @@ struct GatherProblem {
   float* w = nullptr;  // [2][vgroups][n_pad][k_pad]
   size_t w_half = 0;   // elements in one half
   CUtensorMap map;
-  int a_stages = 4, b_stages = 4, acc_bufs = 1, dual = 0, acc_cols = 0;
+  int a_stages = 4, b_stages = 4, acc_bufs = 1;
   int sets = 4, tmem_cols = 512;  // kernel shape: 4 producer sets and one CTA per SM, or 2 sets and two CTAs per SM
   int taps_smem = -1;             // tap-table entries staged in shared memory (-1: k_pad)
   size_t map_k = 0;               // extent of the packed operand along the reduction (0: k_pad)
@@ -1556,20 +1525,18 @@ bool use_small_wgrad(long long pixels, int vgroups, int n, int k_real) {
 
 // Tensor-memory and shared-memory budget of a gather problem, room for its packed operand.
 void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias) {
-  // Tensor memory (512 columns) = accumulator buffers + A stages of 64 columns.  Narrow problems run "dual" (see the
-  // MMA loop): their accumulator is 2*n_pad wide.  Two accumulator buffers let the epilogue overlap the next tile.
+  // Tensor memory (512 columns) = accumulator buffers + A stages of 64 columns.  Two accumulator buffers let the epilogue
+  // overlap the next tile.
   const int taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k / gp.run : gp.taps_smem;
   const size_t map_k = gp.map_k ? gp.map_k : (size_t)gp.k_pad;
-  gp.dual = gp.n_pad <= 64;  // 2 MMAs of width <= 128 instead of 3 narrow ones; wider ones gain nothing
-  gp.acc_cols = gp.dual ? 2 * gp.n_pad : gp.n_pad;
-  if (2 * gp.acc_cols + 4 * 64 <= 512) { gp.acc_bufs = 2; gp.a_stages = 4; }
-  else if (2 * gp.acc_cols + 2 * 64 <= 512 && (gp.split_k ? gp.split_k : gp.k_pad) / kBlockK <= 16) { gp.acc_bufs = 2; gp.a_stages = 2; }  // short K: the epilogue matters more
-  else { gp.acc_bufs = 1; gp.a_stages = std::min(4, (512 - gp.acc_cols) / 64); }
+  if (2 * gp.n_pad + 4 * 64 <= 512) { gp.acc_bufs = 2; gp.a_stages = 4; }
+  else if (2 * gp.n_pad + 2 * 64 <= 512 && (gp.split_k ? gp.split_k : gp.k_pad) / kBlockK <= 16) { gp.acc_bufs = 2; gp.a_stages = 2; }  // short K: the epilogue matters more
+  else { gp.acc_bufs = 1; gp.a_stages = std::min(4, (512 - gp.n_pad) / 64); }
   const int ptab = gp.taps_smem == 0 ? 16 : 0;  // weight-gradient mode: per-warp table slices (sized for 16 warps)
   gp.b_stages = gather_slots(gp.n_pad, taps_smem, n_bias, ptab, kSmemLimit);
   int b_two;
   if (two_ctas_per_sm(gp.n_pad, taps_smem, n_bias, ptab, &b_two)) {
-    gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = 2; gp.b_stages = b_two;
+    gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = gp.n_pad <= 64 && !ptab ? 3 : 2; gp.b_stages = b_two;
   }
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
   gp.w_half = (size_t)vgroups * gp.n_pad * map_k;
@@ -1851,7 +1818,7 @@ void fill_common(GatherParams& P, const GatherProblem& gp, cct_ctx* ctx, int vgr
   P.n_pix_tiles = (P.n_pix + kTileM - 1) / kTileM;
   P.total_tiles = P.n_pix_tiles * vgroups * gp.splits;
   P.a_stages = gp.a_stages; P.b_stages = gp.b_stages; P.acc_bufs = gp.acc_bufs;
-  P.dual = gp.dual; P.acc_cols = gp.acc_cols; P.tmem_cols = gp.tmem_cols;
+  P.tmem_cols = gp.tmem_cols;
   P.n_bias = P.bias ? n_bias : 0;
   P.lo_row_offset = vgroups * gp.n_pad;
   P.status = ctx->status_dev;

@@ -37,7 +37,6 @@ constexpr uint32_t kFcStoreTile = 32u * 32u * 4u;  // 32 columns x 32 lanes on t
 struct FcGemmParams {
   int M, N;                 // extents of the output (m fastest in memory)
   int n_pad;                // accumulator columns per tile: N rounded up (a multiple of 32 for MN-major B)
-  int dual, acc_cols;       // dual: B's lo tile sits right behind the raw one and one MMA of width 2 * n_pad covers both
   int m_tiles, n_tiles, splits, kblocks_total, kblocks_per_split;
   int a_mn, b_mn;           // 1: the operand is MN-major (row index contiguous in memory)
   int raw_slots, lo_slots, a_slots, acc_bufs, store_bufs;
@@ -47,18 +46,16 @@ struct FcGemmParams {
   int* status;
 };
 
-// Raw ring (A tile and B tile as TMA delivers them; for `dual` B's lo tile behind them), lo ring (B's lo tiles), the tiles
-// on their way out, barriers.
+// Raw ring (A tile and B tile as TMA delivers them), lo ring (B's lo tiles), the tiles on their way out.
 struct FcSmem {
-  uint32_t b_tile_bytes, raw_bytes, lo_off, lo_stride, store_off, total;
+  uint32_t b_tile_bytes, raw_bytes, lo_off, store_off, total;
 };
-__host__ __device__ inline FcSmem fc_smem(int n_pad, int dual, int raw_slots, int lo_slots, int store_bufs) {
+__host__ __device__ inline FcSmem fc_smem(int n_pad, int raw_slots, int lo_slots, int store_bufs) {
   FcSmem L;
   L.b_tile_bytes = (uint32_t)n_pad * 128u;
-  L.raw_bytes = kFcATile + (dual ? 2u : 1u) * L.b_tile_bytes;
-  L.lo_off = dual ? kFcATile + L.b_tile_bytes : (uint32_t)raw_slots * L.raw_bytes;
-  L.lo_stride = dual ? L.raw_bytes : L.b_tile_bytes;
-  L.store_off = (uint32_t)raw_slots * L.raw_bytes + (dual ? 0u : (uint32_t)lo_slots * L.b_tile_bytes);
+  L.raw_bytes = kFcATile + L.b_tile_bytes;
+  L.lo_off = (uint32_t)raw_slots * L.raw_bytes;
+  L.store_off = L.lo_off + (uint32_t)lo_slots * L.b_tile_bytes;
   L.total = L.store_off + (uint32_t)(kFcEpiWarps * store_bufs) * kFcStoreTile;  // the barriers go where the 1 KB of alignment slack leaves room
   return L;
 }
@@ -96,13 +93,13 @@ __global__ void __launch_bounds__(kFcThreads, 2)
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-  const FcSmem L = fc_smem(P.n_pad, P.dual, P.raw_slots, P.lo_slots, P.store_bufs);
+  const FcSmem L = fc_smem(P.n_pad, P.raw_slots, P.lo_slots, P.store_bufs);
   // 1 KB more than L.total is allocated: either in front of the aligned base or behind the tiles there is room for these
   constexpr uint32_t kBarBytes = 8u * (3 * kFcRing + 4) + 24u;
   const uint32_t bars = base - smem_u32(smem_raw) >= kBarBytes ? (smem_u32(smem_raw) + 7u) & ~7u : base + L.total;  // 8-byte aligned
   const uint32_t raw_bar = bars, lo_bar = raw_bar + 8u * kFcRing, done_bar = lo_bar + 8u * kFcRing,
                  acc_full = done_bar + 8u * kFcRing, acc_empty = acc_full + 16u, tmem_slot = acc_empty + 16u;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < kFcRing; ++s) {
       mbar_init(raw_bar + 8u * s, 1);
@@ -118,7 +115,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-  const uint32_t a_col0 = (uint32_t)(P.acc_bufs * P.acc_cols);  // A slots (64 columns: 32 hi + 32 lo) behind the accumulators
+  const uint32_t a_col0 = (uint32_t)(P.acc_bufs * P.n_pad);  // A slots (64 columns: 32 hi + 32 lo) behind the accumulators
   const int total_tiles = P.m_tiles * P.n_tiles * P.splits;
   bool failed = false;
   // tile t -> (split, n-tile, m-tile), m-tile fastest; k-blocks [kb0, kb1)
@@ -163,43 +160,42 @@ __global__ void __launch_bounds__(kFcThreads, 2)
         }
       }
     }
-  } else if (warp == kFcMmaWarp) {
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(P.acc_cols) | (P.b_mn ? 1u << 16 : 0u);  // A from tensor memory: lanes x K
-      Ring raw, lo, ta;
-      int i = 0, tile_iter = 0;
-      for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_iter) {
-        int mt, nt, split, kb0, kb1;
-        tile_of(t, mt, nt, split, kb0, kb1);
-        const int buf = tile_iter & (P.acc_bufs - 1), use = tile_iter >> (P.acc_bufs - 1);
-        if (use > 0) mbar_wait<false>(acc_empty + 8u * buf, (uint32_t)(use - 1) & 1u, failed, P.status, 0x1200);
+  } else if (warp == kFcMmaWarp) {  // see elect_one
+    const uint32_t idesc = make_idesc(P.n_pad) | (P.b_mn ? 1u << 16 : 0u);  // A from tensor memory: lanes x K
+    const uint32_t tmem = warp_uniform(tmem_base);
+    Ring raw, lo, ta;
+    int i = 0, tile_iter = 0;
+    for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_iter) {
+      int mt, nt, split, kb0, kb1;
+      tile_of(t, mt, nt, split, kb0, kb1);
+      const int buf = tile_iter & (P.acc_bufs - 1), use = tile_iter >> (P.acc_bufs - 1);
+      if (use > 0) mbar_wait<false>(acc_empty + 8u * buf, (uint32_t)(use - 1) & 1u, failed, P.status, 0x1200);
+      tc_fence_after();
+      const uint32_t d_tmem = tmem + (uint32_t)(buf * P.n_pad);
+      for (int kb = kb0; kb < kb1; ++kb, ++i) {
+        mbar_wait<false>(raw_bar + 8u * raw.idx, (uint32_t)raw.use & 1u, failed, P.status, 0x1300);
+        mbar_wait<false>(lo_bar + 8u * (i & 3), (uint32_t)(i >> 2) & 1u, failed, P.status, 0x1400);
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * P.acc_cols);
-        for (int kb = kb0; kb < kb1; ++kb, ++i) {
-          mbar_wait<false>(raw_bar + 8u * raw.idx, (uint32_t)raw.use & 1u, failed, P.status, 0x1300);
-          mbar_wait<false>(lo_bar + 8u * (i & 3), (uint32_t)(i >> 2) & 1u, failed, P.status, 0x1400);
-          tc_fence_after();
-          const uint32_t b_raw = base + (uint32_t)raw.idx * L.raw_bytes + kFcATile;
-          const uint32_t b_lo = base + L.lo_off + (uint32_t)lo.idx * L.lo_stride;
-          const uint32_t t_hi = tmem_base + a_col0 + (uint32_t)(ta.idx * 64), t_lo = t_hi + 32u;
+        const uint32_t b_raw = base + (uint32_t)raw.idx * L.raw_bytes + kFcATile;
+        const uint32_t b_lo = base + L.lo_off + (uint32_t)lo.idx * L.b_tile_bytes;
+        const uint32_t t_hi = tmem + a_col0 + (uint32_t)(ta.idx * 64), t_lo = t_hi + 32u;
+        if (elect_one()) {
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
             // K-major: 8 reduction indices = 32 bytes along the swizzled row; MN-major: 8 rows of 128 bytes
             const uint64_t bh = P.b_mn ? make_desc_mn(b_raw + j * 1024u) : make_desc(b_raw) + (uint64_t)(j * 2);
-            const uint32_t first = (kb == kb0 && j == 0) ? 0u : 1u;
-            umma_tf32_ts(d_tmem, t_lo + (uint32_t)(j * 8), bh, idesc, first);
-            if (!P.dual) {
-              const uint64_t bl = P.b_mn ? make_desc_mn(b_lo + j * 1024u) : make_desc(b_lo) + (uint64_t)(j * 2);
-              umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bl, idesc, 1u);
-            }
+            const uint64_t bl = P.b_mn ? make_desc_mn(b_lo + j * 1024u) : make_desc(b_lo) + (uint64_t)(j * 2);
+            umma_tf32_ts(d_tmem, t_lo + (uint32_t)(j * 8), bh, idesc, (kb == kb0 && j == 0) ? 0u : 1u);
+            umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bl, idesc, 1u);
             umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bh, idesc, 1u);
           }
           umma_commit(done_bar + 8u * (i & 3));
-          raw.advance(P.raw_slots);
-          lo.advance(P.lo_slots);
-          ta.advance(P.a_slots);
+          if (kb == kb1 - 1) umma_commit(acc_full + 8u * buf);
         }
-        umma_commit(acc_full + 8u * buf);
+        __syncwarp();
+        raw.advance(P.raw_slots);
+        lo.advance(P.lo_slots);
+        ta.advance(P.a_slots);
       }
     }
   } else if (warp >= kFcXformWarp0) {
@@ -250,7 +246,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
           tmem_st8(taddr + 32u + (uint32_t)(c * 8), l8);
         }
         const float4* b_raw = reinterpret_cast<const float4*>(st + kFcATile);
-        float4* b_lo = reinterpret_cast<float4*>(base_ptr + L.lo_off + (size_t)lo.idx * L.lo_stride);
+        float4* b_lo = reinterpret_cast<float4*>(base_ptr + L.lo_off + (size_t)lo.idx * L.b_tile_bytes);
 #pragma unroll 4
         for (int v = xt; v < b_vec; v += kXThreads) {
           const float4 r = b_raw[v];
@@ -284,24 +280,13 @@ __global__ void __launch_bounds__(kFcThreads, 2)
       mbar_wait(acc_full + 8u * buf, (uint32_t)use & 1u, failed, P.status, 0x1600);
       tc_fence_after();
       const int m0 = mt * kTileM + quarter * 32, n0 = nt * P.n_pad;
-      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.acc_cols);
+      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.n_pad);
       const int chunks = min(P.n_pad, P.N - n0 + 15) / 16;  // columns behind N are never looked at
       for (int c = 0; c < chunks; c += 2) {  // 32 columns a step: one round of waits, fence and stores for them
         float v[2][16];
         const bool two = c + 1 < chunks;
         tmem_ld16(acc + (uint32_t)(c * 16), v[0]);
         if (two) tmem_ld16(acc + (uint32_t)(c * 16 + 16), v[1]);
-        if (P.dual) {
-          float w[16];
-          tmem_ld16(acc + (uint32_t)(P.n_pad + c * 16), w);
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[0][j] += w[j];
-          if (two) {
-            tmem_ld16(acc + (uint32_t)(P.n_pad + c * 16 + 16), w);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[1][j] += w[j];
-          }
-        }
         if (failed || m0 >= P.M) continue;
         if (P.direct) {
 #pragma unroll
@@ -507,11 +492,11 @@ bool fc_fit_rings(FcShape& s) {
   FcGemmParams& P = s.P;
   const size_t budget = s.pair ? 113 * 1024 : kSmemLimit;
   P.tmem_cols = s.pair ? 256 : 512;
-  P.a_slots = std::min(kFcRing, (P.tmem_cols - P.acc_bufs * P.acc_cols) / 64);
+  P.a_slots = std::min(kFcRing, (P.tmem_cols - P.acc_bufs * P.n_pad) / 64);
   for (int raw = kFcRing; raw >= 2; --raw)
     for (int st = 2; st >= 1; --st) {
-      const int lo = P.dual ? raw : 2;
-      const size_t need = fc_smem(P.n_pad, P.dual, raw, lo, st).total + 1024;
+      const int lo = std::min(raw, P.n_pad <= 64 ? 3 : 2);
+      const size_t need = fc_smem(P.n_pad, raw, lo, st).total + 1024;
       if (need <= budget) {
         P.raw_slots = raw; P.lo_slots = lo; P.store_bufs = st;
         s.smem = need;
@@ -522,8 +507,8 @@ bool fc_fit_rings(FcShape& s) {
 }
 
 // Forward pass and data gradient: M = the layer's output (input) features, N = batch.  The splits of the reduction are
-// chosen by the rounds of (tile, split) units over the resident CTAs: a k-block takes its 12 (dual: 8) MMAs, at least 75
-// cycles to issue each, and two CTAs on an SM share the tensor pipe; a unit adds set-up and epilogue, a split the traffic of
+// chosen by the rounds of (tile, split) units over the resident CTAs: a k-block takes its 12 MMAs, and two CTAs on an SM
+// share the tensor pipe; a unit adds set-up and epilogue, a split the traffic of
 // one more partial sum.
 FcShape fc_batch_shape(int sms, int M, int N, int R) {
   FcShape s;
@@ -532,13 +517,13 @@ FcShape fc_batch_shape(int sms, int M, int N, int R) {
   P.m_tiles = (M + kTileM - 1) / kTileM;
   P.n_tiles = (N + 255) / 256;
   P.n_pad = fc_round_up((N + P.n_tiles - 1) / P.n_tiles, 16);
-  P.dual = P.n_pad <= 64;
-  P.acc_cols = P.dual ? 2 * P.n_pad : P.n_pad;
   P.acc_bufs = 1;
   s.pair = P.n_pad <= 128;
   P.kblocks_total = (R + kBlockK - 1) / kBlockK;
-  const double mmas = P.dual ? 8 : 12, exec = mmas * P.acc_cols / 2.0, alone = std::max(exec, mmas * 75) / 1750.0,
-               shared = std::max(2 * exec, mmas * 75) / 1750.0;
+  // a k-block: its MMAs, or the hand-overs from TMA to transform to MMA (with two raw slots, the room for wide tiles in
+  // half an SM, a CTA waits for its own loads: 1.1 us a k-block at 128 columns)
+  const double exec = 12 * std::max(P.n_pad / 2.0, 18.0) / 1750.0;
+  const double alone = std::max(exec, s.pair && P.n_pad > 64 ? 1.0 : 0.35), shared = std::max(2 * exec, alone);
   const long long slots = (long long)sms * (s.pair ? 2 : 1);
   double best = 0.0;
   for (int n = 1; n <= std::max(1, P.kblocks_total / 2); ++n) {
@@ -568,13 +553,13 @@ FcShape fc_weight_shape(int sms, int K, int O, int B) {
     FcGemmParams& P = s.P;
     P.M = K; P.N = O;
     P.m_tiles = (K + kTileM - 1) / kTileM;
-    P.n_pad = n; P.acc_cols = n; P.acc_bufs = 2;
+    P.n_pad = n; P.acc_bufs = 2;
     P.n_tiles = (O + n - 1) / n;
     P.splits = 1;
     P.kblocks_total = P.kblocks_per_split = (B + kBlockK - 1) / kBlockK;
     P.a_mn = P.b_mn = 1;
     const long long rounds = ((long long)P.m_tiles * P.n_tiles + sms - 1) / sms;
-    const double mma = P.kblocks_total * 12.0 * std::max(75.0, n / 2.0) / 1750.0, out = 0.2 + 0.006 * n;
+    const double mma = P.kblocks_total * std::max(12.0 * n / 2.0 / 1750.0, 0.35), out = 0.2 + 0.006 * n;
     const double us = rounds * std::max(mma, out) + mma + out;
     if (!best.P.n_pad || us < 0.98 * best_us) {
       best = s;

@@ -88,6 +88,19 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
+// One lane of the (converged) warp.  The MMA warps run their loops with all lanes and issue under this predicate: the
+// compiler then knows that descriptors and addresses are the same for every lane and keeps them in uniform registers.  Issued
+// by one lane of a diverged warp instead, each tcgen05.mma cost 50 - 75 cycles however narrow it was; this way it is
+// max(N / 2, 18) (measured with M = 128, A in tensor memory, operand addresses changing from stage to stage: a k-block of 12
+// MMAs of 48 columns takes 318 cycles instead of 599).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// A value that is the same in every lane, as one the compiler knows to be.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // The mbarrier receives one arrival when every MMA issued so far by this thread has finished.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
