@@ -82,6 +82,17 @@ __device__ __forceinline__ float ldg_if_clear(const float* p, uint32_t a, uint32
       : "l"(p), "r"(a), "r"(b));
   return v;
 }
+// p[i * stride], the address as one multiply-add.
+__device__ __forceinline__ float ldg_at(const float* p, int i, int stride) {
+  float v;
+  asm volatile(
+      "{\n\t.reg .b64 a;\n\t"
+      "mad.wide.s32 a, %2, %3, %1;\n\t"
+      "ld.global.nc.f32 %0, [a];\n\t}"
+      : "=f"(v)
+      : "l"(p), "r"(stride), "r"(i * 4));
+  return v;
+}
 // v = flag ? *p : 0, same form.
 __device__ __forceinline__ float ldg_if(const float* p, uint32_t flag) {
   float v;
@@ -172,6 +183,7 @@ struct GatherParams {
   int wg_rows_pad;            // rows of one split's partial-sum slice (M-tiles * 128)
   int wg_k, wg_kreal;         // kernel size, real rows of the lowered matrix
   int taps_smem;              // entries of `taps` staged in shared memory (0 in weight-gradient mode)
+  const float* zero;          // kByRun: what lanes whose tap is out of bounds read
   int run_stride;             // kByRun: elements between consecutive channels of the gathered tensor
   int* status;
 };
@@ -343,13 +355,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
 #pragma unroll
         for (int r = 0; r < kBlockK / kRun; ++r) {
           const MaskTap tap = tp[r];
+          const bool ok = (mask & tap.bits) == tap.bits;
+          const float* p = ok ? in_px + tap.off : P.zero;
+          const int stride = ok ? P.run_stride : 0;
 #pragma unroll
-          for (int e = 0; e < kRun; ++e) v[r * kRun + e] = 0.f;
-          if ((mask & tap.bits) == tap.bits) {
-            const float* p = in_px + tap.off;
-#pragma unroll
-            for (int e = 0; e < kRun; ++e) v[r * kRun + e] = __ldg(p + e * P.run_stride);
-          }
+          for (int e = 0; e < kRun; ++e) v[r * kRun + e] = __ldg(p + e * stride);
         }
         return;
       }
@@ -1297,16 +1307,16 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
 }
 
 // Data-gradient B operand: [2][vg][n_pad][k_pad]; row j = (d, py, px) of channel tile nt of group g (py, px: position
-// inside an s x s block of input pixels), column kk = (oc, jy, jx) <- W[g*og + oc][d][py + jy*s][px + jx*s], zero where
-// the tap index exceeds the kernel.
+// inside a block of s * rows x s input pixels), column kk = (oc, jy, jx) <- W[g*og + oc][d][py + (jy - rows + 1)*s][px + jx*s],
+// zero where the tap index is outside the kernel.
 __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                   float* __restrict__ lo, int tiles_per_group, int og,
-                                                                  int Dg, int k, int s, int taps, int d_tile, int n_real,
-                                                                  int n_pad, int k_real, int k_pad, int run) {
+                                                                  int Dg, int k, int s, int taps, int rows, int d_tile,
+                                                                  int n_real, int n_pad, int k_real, int k_pad, int run) {
   pdl_wait();
   const int vg = blockIdx.y / n_pad, j = blockIdx.y - vg * n_pad;
-  const int grp = vg / tiles_per_group, d = (vg - grp * tiles_per_group) * d_tile + j / (s * s);
-  const int py = (j / s) % s, px = j % s;
+  const int grp = vg / tiles_per_group, d = (vg - grp * tiles_per_group) * d_tile + j / (s * s * rows);
+  const int py = (j / s) % (s * rows), px = j % s, window = taps * (taps + rows - 1);
   const bool live = j < n_real && d < Dg;
   const float* src = W + ((size_t)grp * og * Dg + d) * k * k;
   const size_t row = (size_t)blockIdx.y * k_pad;
@@ -1315,10 +1325,10 @@ __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* _
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       // reduction index -> (filter / run, jy, jx, filter % run)
-      const int r = (kk + e) / run, chunk = r / (taps * taps), tap = r - chunk * taps * taps;
+      const int r = (kk + e) / run, chunk = r / window, tap = r - chunk * window;
       const int oc = chunk * run + (kk + e - r * run), jy = tap / taps, jx = tap - jy * taps;
-      const int kr = py + jy * s, kc = px + jx * s;
-      v[e] = (live && kk + e < k_real && kr < k && kc < k) ? __ldg(src + (size_t)oc * Dg * k * k + kr * k + kc) : 0.f;
+      const int kr = py + (jy - rows + 1) * s, kc = px + jx * s;
+      v[e] = (live && kk + e < k_real && (unsigned)kr < (unsigned)k && kc < k) ? __ldg(src + (size_t)oc * Dg * k * k + kr * k + kc) : 0.f;
     }
     store_split4(hi, lo, row + kk, v);
   }
@@ -1348,19 +1358,19 @@ bool two_ctas_per_sm(int n_pad, int taps_smem, int n_bias, int ptab, int* slots)
 
 // Channel tiles and splits of the reduction for the forward pass and the data gradient, by an estimate of the kernel's
 // time in microseconds.  A work unit is (pixel tile, channel tile, split); units are spread over the resident CTAs in whole
-// rounds.  Per k-block a CTA takes what its MMAs take (half a cycle per column, 18 cycles at least), or what
-// its producers take to gather (measured: 0.62 us alone on an SM with two producer sets, 0.8 us when two CTAs share one,
-// 0.35 us with four sets); a unit adds an epilogue that grows with its columns (64 columns 1.3 us, 192 columns 2.8 us), a
-// split reduction one more kernel and the traffic of the sums.  So: a last round that is nearly empty (CaffeNet conv3 at
-// batch 256: 2 x 338 units on 148 CTAs are five rounds, 3 x 338 half-width ones on 296 are 3.4) asks for narrower tiles, a
-// layer of few pixels (43 tiles at batch 32, 2 at batch 1) for narrower tiles and splits.  A candidate has to win by 3 %.
+// rounds.  The constants are a fit to 754 measured combinations of tiles and splits (CaffeNet's layers at batch 1 to 128 and
+// layers of 20 to 384 channels; 6 % rms): what a k-block takes grows with the accumulator's columns, below that stands what the
+// gather takes; a unit adds its set-up and epilogue, a split reduction one more kernel and the traffic of the sums.  So: a
+// last round that is nearly empty (CaffeNet conv3 at batch 256: 2 x 338 units on 148 CTAs are five rounds, 3 x 338 half-width
+// ones on 296 are 3.4) asks for narrower tiles, a layer of few pixels (43 tiles at batch 32, 2 at batch 1) for narrower tiles
+// and splits.  A candidate has to win by 1 %.
 struct GatherTiling {
   int tiles = 0, splits = 1, kps = 0;
+  double us = 0.0;
 };
 GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, int channels, int cols_per_channel, int kblocks,
-                                  int run, int n_bias) {
+                                  int run, int lane_stride, int n_bias) {
   GatherTiling best;
-  double best_us = 0.0;
   const int t0 = channel_tiles(channels, cols_per_channel);
   for (int t = t0; t > 0 && t <= channels; ++t) {
     const int n_pad = round_up((channels + t - 1) / t * cols_per_channel, 16);
@@ -1368,20 +1378,19 @@ GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, in
     if ((channels + t - 1) / t * (t - 1) >= channels) continue;  // the last tile would be empty
     int slots_unused;
     const bool two = two_ctas_per_sm(n_pad, kblocks * kBlockK / run, n_bias, 0, &slots_unused);
-    const double mhz = 1600.0, exec = 12 * std::max(n_pad / 2.0, 18.0) / mhz;  // clock under load
-    const double alone = std::max(exec, two ? 0.62 : 0.35), shared = two ? std::max(2 * exec, 0.8) : alone;
-    const double epilogue = 0.5 + 0.012 * n_pad;
+    // a k-block of a CTA that shares its SM, of one that has the SM to itself, of the shape with one CTA per SM
+    const double far = lane_stride > 2 ? 1.7 : 1.0;  // lanes 16 bytes and more apart: four wavefronts and more per load
+    const double shared = 2 * std::max(0.11 + 0.0028 * n_pad, (run > 1 ? 0.235 : 0.30) * far);
+    const double alone = std::max(0.19 + 0.0018 * n_pad, 0.27 * far), one = std::max(0.0035 * n_pad, 0.42 * far);
+    const double epilogue = 4.0 + 0.004 * n_pad;
     for (int s = 1; s <= std::max(1, std::min(32, kblocks / 2)); ++s) {
       const int kps = (kblocks + s - 1) / s;
       if ((kblocks + kps - 1) / kps != s) continue;
       const long long units = pixel_tiles * groups * t * s, slots = (long long)sms * (two ? 2 : 1), tail = units % slots;
-      double us = (double)(units / slots) * (kps * shared + 0.4 * epilogue) +
-                  (tail ? kps * (two && tail > sms ? shared : alone) + epilogue : 0.6 * epilogue) + 4.0;
-      if (s > 1) us += 2.3 + units * 128.0 * n_pad * 8.0 / 4e6;
-      if (!best.tiles || us < 0.97 * best_us) {
-        best_us = us;
-        best = GatherTiling{t, s, kps};
-      }
+      double us = (double)(units / slots) * (kps * (two ? shared : one) + 0.4 * epilogue) +
+                  (tail ? kps * (!two ? one : tail > sms ? shared : alone) + epilogue : 0.6 * epilogue) + 2.6;
+      if (s > 1) us += 3.8 + units * 128.0 * n_pad * 4.0 * 0.18e-6;
+      if (!best.tiles || us < 0.99 * best.us) best = GatherTiling{t, s, kps, us};
     }
   }
   return best;
@@ -1403,6 +1412,7 @@ struct GatherProblem {
   int taps_smem = -1;             // tap-table entries staged in shared memory (-1: k_pad)
   size_t map_k = 0;               // extent of the packed operand along the reduction (0: k_pad)
   size_t smem = 0;
+  float* zero = nullptr;          // one 0.f, read by taps out of bounds
   int run = 1, run_stride = 0;    // reduction order: 1 = (channel, tap); kRun = (channel / kRun, tap, channel % kRun)
   int splits = 1, split_k = 0;    // splits of the reduction and the length of one (a multiple of 32; k_pad without splits)
   float* partial = nullptr;       // split sums
@@ -1413,7 +1423,9 @@ struct GatherProblem {
 struct UmmaPlan {
   ConvGeom G;
   GatherProblem fwd, dgr;
-  int dgr_taps = 0, dgr_q = 0, dgr_q0 = 0;  // taps per axis; super-pixels per axis and the first one that holds a pixel
+  // data gradient: taps per axis of one stride period; super-pixels of s * dgr_rows x s pixels, how many and the first that
+  // holds a pixel
+  int dgr_taps = 0, dgr_rows = 1, dgr_q = 0, dgr_q0 = 0, dgr_qy = 0, dgr_qy0 = 0;
   // weight gradient: channel tiles per group, channels per tile (the last one may be shorter), padded to 16
   int wt_tiles = 1, wt_n = 0;
   int w_mtiles, w_subs, w_stages, w_mgroups, w_splits, w_kblocks_total, w_kblocks_per_split, w_npad;
@@ -1580,7 +1592,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     f.k_pad = round_up(f.k_real, kBlockK);
     f.run = G.Dg % kRun == 0 ? kRun : 1; f.run_stride = G.n * G.n;
     const long long pixel_tiles = ((long long)G.B * G.m * G.m + kTileM - 1) / kTileM;
-    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, f.run, G.bias ? G.o : 0);
+    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, f.run, G.s, G.bias ? G.o : 0);
     f.tiles = tl.tiles;
     f.ch_tile = f.n = (G.og + f.tiles - 1) / f.tiles;
     f.n_pad = round_up(f.n, 16);
@@ -1600,6 +1612,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     if (!f.small_ct) {
       mem.table(&f.taps, t);
       mem.table(&f.cols, c);
+      mem.table(&f.zero, std::vector<float>(1, 0.f));
       finish_problem(mem, f, G.g * f.tiles, G.bias ? G.o : 0);
       if (f.splits > 1) sums = std::max(sums, (size_t)f.splits * G.g * f.tiles * f.n_pad * f.pix_pad);
     }
@@ -1608,16 +1621,25 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
   //      columns = (d, py, px), reduction = (oc, jy, jx) with jy, jx < ceil(k/s); depth-to-space in the epilogue.
   {
     GatherProblem& d = p->dgr;
-    const int ss = G.s * G.s;
-    p->dgr_taps = (G.k + G.s - 1) / G.s;
+    const int J = p->dgr_taps = (G.k + G.s - 1) / G.s;
     p->dgr_q0 = G.p / G.s;
     p->dgr_q = (G.n - 1 + G.p) / G.s + 1 - p->dgr_q0;
-    const int J = p->dgr_taps;
-    d.k_real = G.og * J * J;
-    d.k_pad = round_up(d.k_real, kBlockK);
     d.run = G.og % kRun == 0 ? kRun : 1; d.run_stride = G.m * G.m;
-    const long long pixel_tiles = ((long long)G.B * p->dgr_q * p->dgr_q + kTileM - 1) / kTileM;
-    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.Dg, ss, d.k_pad / kBlockK, d.run, 0);
+    GatherTiling tl;
+    long long pixel_tiles = 0;
+    for (int rows = 1; rows <= 4 && J + rows - 1 <= kMaxTapsPerAxis; ++rows) {
+      const int q0 = G.p / (G.s * rows), q = (G.n - 1 + G.p) / (G.s * rows) + 1 - q0, k_real = G.og * J * (J + rows - 1);
+      if (rows > 1 && (k_real > 16384 || channel_tiles(G.Dg, G.s * G.s * rows) == 0)) break;
+      const long long tiles = ((long long)G.B * q * p->dgr_q + kTileM - 1) / kTileM;
+      const GatherTiling c = choose_gather_tiling(ctx->planning_sms(), tiles, G.g, G.Dg, G.s * G.s * rows,
+                                                  round_up(k_real, kBlockK) / kBlockK, d.run, 1, 0);
+      if (rows > 1 && c.us >= 0.99 * tl.us) continue;
+      tl = c; pixel_tiles = tiles;
+      p->dgr_rows = rows; p->dgr_qy0 = q0; p->dgr_qy = q;
+      d.k_real = k_real;
+    }
+    const int ss = G.s * G.s * p->dgr_rows, H = G.s * p->dgr_rows;
+    d.k_pad = round_up(d.k_real, kBlockK);
     d.tiles = tl.tiles;
     d.ch_tile = (G.Dg + d.tiles - 1) / d.tiles;
     d.n = d.ch_tile * ss;
@@ -1626,7 +1648,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     std::vector<MaskTap> t((size_t)d.splits * d.split_k / d.run);
     for (int i = 0; i < (int)t.size(); ++i) {
       if (i * d.run < d.k_real) {
-        const int jx = i % J, jy = (i / J) % J, oc = i / (J * J) * d.run;
+        const int Jy = J + p->dgr_rows - 1, jx = i % J, jy = (i / J) % Jy, oc = i / (J * Jy) * d.run;
         t[i] = MaskTap{oc * G.m * G.m - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
       } else {
         t[i] = MaskTap{0, kPadBit};
@@ -1634,13 +1656,14 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     }
     std::vector<ColEnt> c(d.n_pad);
     for (int j = 0; j < d.n_pad; ++j) {
-      const int dl = j / ss, py = (j / G.s) % G.s, px = j % G.s;
+      const int dl = j / ss, py = (j / G.s) % H, px = j % G.s;
       c[j] = ColEnt{dl * G.n * G.n + py * G.n + px, (short)py, (short)px};
     }
     if (!tensor_only && G.s == 1) d.small_ct = use_small_conv(G.k, 1, (long long)G.B * G.n * G.n, G.g, G.og, G.Dg);
     if (!d.small_ct) {
       mem.table(&d.taps, t);
       mem.table(&d.cols, c);
+      mem.table(&d.zero, std::vector<float>(1, 0.f));
       finish_problem(mem, d, G.g * d.tiles, 0);
       if (d.splits > 1) sums = std::max(sums, (size_t)d.splits * G.g * d.tiles * d.n_pad * d.pix_pad);
     }
@@ -1814,7 +1837,7 @@ void fill_common(GatherParams& P, const GatherProblem& gp, cct_ctx* ctx, int vgr
   P.cols_per_channel = gp.n / gp.ch_tile;
   P.splits = gp.splits; P.partial = gp.partial; P.pix_pad = (int)gp.pix_pad;
   P.taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k / gp.run : gp.taps_smem;
-  P.run_stride = gp.run_stride;
+  P.run_stride = gp.run_stride; P.zero = gp.zero;
   P.n_pix_tiles = (P.n_pix + kTileM - 1) / kTileM;
   P.total_tiles = P.n_pix_tiles * vgroups * gp.splits;
   P.a_stages = gp.a_stages; P.b_stages = gp.b_stages; P.acc_bufs = gp.acc_bufs;
@@ -2007,18 +2030,19 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
     }
     if (repack) {
       launch_pdl(pack_dgrad_kernel, pack_grid(vgroups * d.n_pad, d.k_pad), dim3(kPackThreads), 0, ctx->stream, W, d.w,
-                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run);
+                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, p->dgr_rows, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run);
       CCT_CHECK_LAUNCH(ctx);
     }
     GatherParams P{};
     P.in = dY; P.out = dX; P.bias = nullptr;
-    P.n_pix = B * p->dgr_q * p->dgr_q; P.q_h = p->dgr_q; P.q_w = p->dgr_q;
-    P.iy_mul = 1; P.iy_add = p->dgr_q0; P.ix_mul = 1; P.ix_add = p->dgr_q0;
+    const int rows = p->dgr_rows;
+    P.n_pix = B * p->dgr_qy * p->dgr_q; P.q_h = p->dgr_qy; P.q_w = p->dgr_q;
+    P.iy_mul = rows; P.iy_add = (p->dgr_qy0 + 1) * rows - 1; P.ix_mul = 1; P.ix_add = p->dgr_q0;
     P.in_lim = G.m;
-    P.tap_sign = -1; P.taps_per_axis = p->dgr_taps;
+    P.tap_sign = -1; P.taps_per_axis = p->dgr_taps + rows - 1;
     P.in_batch_stride = (long long)G.o * G.m * G.m;
     P.in_group_stride = G.og * G.m * G.m;
-    P.oy_mul = G.s; P.oy_add = p->dgr_q0 * G.s - G.p; P.ox_mul = G.s; P.ox_add = p->dgr_q0 * G.s - G.p;
+    P.oy_mul = G.s * rows; P.oy_add = p->dgr_qy0 * rows * G.s - G.p; P.ox_mul = G.s; P.ox_add = p->dgr_q0 * G.s - G.p;
     P.out_lim = G.n; P.check_out = 1;
     P.out_pitch = G.n; P.out_plane = G.n * G.n;
     P.out_batch_stride = (long long)G.D * G.n * G.n;
