@@ -134,3 +134,15 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
 int pool_relu_backward_pooled(cct_ctx* ctx, const float* P, const int32_t* idx, const float* dP, float* dA, int planes,
                               int n, int k, int s);
 int maxpool_forward_staged(cct_ctx* ctx, const float* X, float* Y, int32_t* idx, int planes, int n, int m, int k, int s);
+
+// ---- index arithmetic of the pooling kernels
+// x / d for x * d < 2^32 as one multiply-high: inv = floor(2^32 / d) + 1 (host side, fast_div_magic); inv == 0 means
+// "divide".  The GPU has no integer divider, and these kernels would otherwise spend more on index arithmetic than on
+// memory.
+__device__ __forceinline__ uint32_t fast_div(uint32_t x, uint32_t d, uint32_t inv) {
+  return inv ? __umulhi(x, inv) : x / d;
+}
+// Magic for fast_div: valid when max_x * d < 2^32 and d > 1, else 0 (plain division).
+inline uint32_t fast_div_magic(uint64_t max_x, uint32_t d) {
+  return (d > 1 && max_x * d < (1ull << 32)) ? (uint32_t)((1ull << 32) / d) + 1u : 0u;
+}

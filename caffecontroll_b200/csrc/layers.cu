@@ -23,7 +23,7 @@ inline int ew_grid(cct_ctx* ctx, size_t work, int threads) {
 // them as its own).  Splitting the channels keeps the grid large on the late layers (13 x 13 planes).  4 B read + 8 B
 // written per element (Y and scale; the backward pass reads scale instead of recomputing a nine-channel window).
 constexpr int kLrnChunk = 16;
-constexpr int kLrnBwdChunk = 8;
+constexpr int kLrnBwdChunk = 12;
 
 // One short-lived block of 128 threads per 128 items (the kernels' loops then run once): a thread's item is some sixty
 // loads and stores long, and with a grid of a few blocks per SM looping over the items the last round left a third of
@@ -32,8 +32,32 @@ inline int lrn_grid(size_t items) { return (int)std::max<size_t>(1, std::min<siz
 
 // s^(-beta) for s >= 1: exp2(-beta log2 s) on the special-function units (ex2.approx / lg2.approx, each within ~2 ulp:
 // relative error below 1e-6 for the scales and exponents of a normalisation layer, two orders under the path's tolerance;
-// powf costs some thirty instructions and made these kernels compute-bound).
-__device__ __forceinline__ float inv_pow(float s, float beta) { return exp2f(-beta * __log2f(s)); }
+// powf costs some thirty instructions and made these kernels compute-bound).  No argument or result is subnormal, so the
+// flush-to-zero forms give the same bits without the scaling around them.
+__device__ __forceinline__ float inv_pow(float s, float beta) {
+  float l, r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(s));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(-beta * l));
+  return r;
+}
+
+// x[i] = channel c0 + i at `base`, zero outside 0 .. D - 1.  Chunks away from both ends (all but two of them) take the loads
+// without tests; with them a backward thread spent more instructions on addresses and guards than on the layer (128 images,
+// 96 channels, 27 x 27: forward 20 -> 16.6 us, backward 35.6 -> 26.4 with chunks of 12 instead of 8).
+template <int N>
+__device__ __forceinline__ void lrn_load(const float* __restrict__ base, int c0, int D, int plane, float (&x)[N]) {
+  if (c0 >= 0 && c0 + N <= D) {
+    const float* p = base + (size_t)c0 * plane;
+#pragma unroll
+    for (int i = 0; i < N; ++i, p += plane) x[i] = __ldg(p);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int c = c0 + i;
+      x[i] = (c >= 0 && c < D) ? __ldg(base + (size_t)c * plane) : 0.f;
+    }
+  }
+}
 
 template <int LOCAL>
 __global__ void __launch_bounds__(128) lrn_fwd_kernel(const float* __restrict__ X, float* __restrict__ Y,
@@ -48,11 +72,7 @@ __global__ void __launch_bounds__(128) lrn_fwd_kernel(const float* __restrict__ 
     const size_t base = b * (size_t)D * plane + p;
     // the chunk and its halo, all loads issued before the first use (a thread keeps SPAN requests in flight)
     float x[SPAN];
-#pragma unroll
-    for (int i = 0; i < SPAN; ++i) {
-      const int c = d0 + i - W;
-      x[i] = (c >= 0 && c < D) ? __ldg(X + base + (size_t)c * plane) : 0.f;
-    }
+    lrn_load(X + base, d0 - W, D, plane, x);
 #pragma unroll
     for (int j = 0; j < kLrnChunk; ++j) {
       const int d = d0 + j;
@@ -118,18 +138,18 @@ __global__ void __launch_bounds__(128) lrn_bwd_kernel(const float* __restrict__ 
     const size_t base = b * (size_t)D * plane + p;
     // every load of the chunk and its halo is issued before the first use
     float gy[SPAN], sc[SPAN], xx[XSPAN];
+    lrn_load(dY + base, d0 - W, D, plane, gy);
+    lrn_load(X + base, d0 - W - XW, D, plane, xx);
+    if (HAVE_SCALE) {
+      lrn_load(scale + base, d0 - W, D, plane, sc);
 #pragma unroll
-    for (int i = 0; i < SPAN; ++i) {
-      const int c = d0 + i - W;
-      const bool in = c >= 0 && c < D;
-      const size_t at = base + (size_t)(in ? c : 0) * plane;
-      gy[i] = in ? __ldg(dY + at) : 0.f;
-      if (HAVE_SCALE) sc[i] = in ? __ldg(scale + at) : 1.f;
-    }
+      for (int i = 0; i < W; ++i) {  // channels outside: no division by zero below
+        if (d0 + i - W < 0) sc[i] = 1.f;
+        if (d0 + SPAN - 1 - i - W >= D) sc[SPAN - 1 - i] = 1.f;
+      }
 #pragma unroll
-    for (int i = 0; i < XSPAN; ++i) {
-      const int c = d0 + i - W - XW;
-      xx[i] = (c >= 0 && c < D) ? __ldg(X + base + (size_t)c * plane) : 0.f;
+      for (int i = W; i < SPAN - W; ++i)
+        if (d0 + i - W >= D) sc[i] = 1.f;
     }
     if (!HAVE_SCALE) {
 #pragma unroll
@@ -302,11 +322,13 @@ __global__ void softmax_bwd_kernel(const float* __restrict__ prob, const float* 
 // with coalesced loads (every input element crosses HBM -> SM once, four loads in flight per thread), the windows are
 // read from there, Y and idx leave in coalesced runs.  K, S > 0 fix the window at compile time (straight-line
 // compare / select chain); K = 0 keeps run-time loops.  4 B read per input element + 8 B written per output element.
+constexpr int kPoolStrip = 3;   // 27 output rows are nine strips, 13 are five
 constexpr int kPoolFetch = 12;  // 256 * 12 elements: one 55 x 55 plane, four 27 x 27, sixteen 13 x 13
 template <int K, int S>
 __global__ void __launch_bounds__(256) maxpool_fwd_staged_kernel(const float* __restrict__ X, float* __restrict__ Y,
                                                                  int32_t* __restrict__ idx, int planes, int n, int m,
-                                                                 int k_rt, int s_rt, int group) {
+                                                                 int k_rt, int s_rt, int group, uint32_t inv_m,
+                                                                 uint32_t inv_strips) {
   pdl_wait();
   // `group` consecutive planes (contiguous in memory) are staged and pooled together, so that small planes (13 x 13)
   // still give every thread of the block work.
@@ -350,32 +372,69 @@ __global__ void __launch_bounds__(256) maxpool_fwd_staged_kernel(const float* __
       for (; i < total_in; i += 256) plane_smem[i] = __ldg(in + i);
       __syncthreads();
     }
-    for (int t = threadIdx.x; t < total_out; t += 256) {
-      const int pl = t / mm, r = t - pl * mm;
-      const int ph = r / m, pw = r - ph * m;
-      const int origin = ph * s * n + pw * s;
-      const float* win = plane_smem + pl * nn + origin;
-      float best = -FLT_MAX;
-      int where = 0;
-      if (K > 0) {
-#pragma unroll
-        for (int h = 0; h < K; ++h)
+    if (K > 0) {
+      // One thread per column of kPoolStrip windows: a row that two windows share is scanned once, and the divisions that
+      // find the place are paid per strip (12288 planes of 55 x 55: 51.5 -> 46.4 us; strips of 5: 49.2; even and odd columns
+      // apart in shared memory, which spares the two-way conflicts but costs address arithmetic: 49.9).
+      const int strips = (m + kPoolStrip - 1) / kPoolStrip;
+      for (uint32_t t = threadIdx.x; t < (uint32_t)(g * strips * m); t += 256) {
+        const uint32_t r = fast_div(t, (uint32_t)m, inv_m), pl = fast_div(r, (uint32_t)strips, inv_strips);
+        const int pw = (int)(t - r * m), ph0 = (int)(r - pl * strips) * kPoolStrip;
+        const float* col = plane_smem + pl * nn + pw * S;
+        // first maximum of the K elements of a row that lies above -FLT_MAX
+        auto scan = [&](int row, float& best, int& where) {
+          best = -FLT_MAX;
+          where = 0;
 #pragma unroll
           for (int w = 0; w < K; ++w) {
-            const float v = win[h * n + w];
+            const float v = col[row * n + w];
             const bool better = v > best;
             best = better ? v : best;
-            where = better ? h * n + w : where;
+            where = better ? row * n + w : where;
           }
-      } else {
+        };
+        float rb[K > 0 ? K : 1];
+        int rw[K > 0 ? K : 1];
+#pragma unroll
+        for (int h = S; h < K; ++h) scan(ph0 * S + h - S, rb[h], rw[h]);
+#pragma unroll
+        for (int q = 0; q < kPoolStrip; ++q) {
+          const int ph = ph0 + q;
+          if (ph >= m) break;
+#pragma unroll
+          for (int h = 0; h < K; ++h) {
+            if (h + S < K) { rb[h] = rb[h + S]; rw[h] = rw[h + S]; }
+            else scan(ph * S + h, rb[h], rw[h]);
+          }
+          float best = -FLT_MAX;
+          int where = ph * S * n;
+#pragma unroll
+          for (int h = 0; h < K; ++h) {
+            const bool better = rb[h] > best;
+            best = better ? rb[h] : best;
+            where = better ? rw[h] : where;
+          }
+          const size_t at = (size_t)(p0 + (int)pl) * mm + ph * m + pw;
+          Y[at] = best;
+          idx[at] = where + pw * S;
+        }
+      }
+    } else {
+      for (int t = threadIdx.x; t < total_out; t += 256) {
+        const int pl = t / mm, r = t - pl * mm;
+        const int ph = r / m, pw = r - ph * m;
+        const int origin = ph * s * n + pw * s;
+        const float* win = plane_smem + pl * nn + origin;
+        float best = -FLT_MAX;
+        int where = 0;
         for (int h = 0; h < k; ++h)
           for (int w = 0; w < k; ++w) {
             const float v = win[h * n + w];
             if (v > best) { best = v; where = h * n + w; }
           }
+        Y[(size_t)p0 * mm + t] = best;
+        idx[(size_t)p0 * mm + t] = origin + where;
       }
-      Y[(size_t)p0 * mm + t] = best;
-      idx[(size_t)p0 * mm + t] = origin + where;
     }
   }
 }
@@ -391,9 +450,10 @@ int maxpool_forward_staged(cct_ctx* ctx, const float* X, float* Y, int32_t* idx,
                                                                                          : maxpool_fwd_staged_kernel<0, 0>;
   if (smem > 48 * 1024) CCT_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(8, (200 * 1024) / std::max<size_t>(smem, 1)));
-  const int blocks_needed = (planes + group - 1) / group;
+  const int blocks_needed = (planes + group - 1) / group, strips = (m + kPoolStrip - 1) / kPoolStrip;
   const int grid = std::max(1, std::min(blocks_needed, ctx->sm_count * per_sm));
-  launch_pdl(kernel, dim3(grid), dim3(256), smem, ctx->stream, X, Y, idx, planes, n, m, k, s, group);
+  launch_pdl(kernel, dim3(grid), dim3(256), smem, ctx->stream, X, Y, idx, planes, n, m, k, s, group,
+             fast_div_magic((uint64_t)group * strips * m, (uint32_t)m), fast_div_magic((uint64_t)group * strips, (uint32_t)strips));
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
