@@ -344,9 +344,10 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         slot[lane] = ent_next;
         __syncwarp();
 #pragma unroll
-        for (int e = 0; e < kBlockK; ++e) {
-          const uint2 ent = slot[e];
+        for (int e = 0; e < kBlockK; e += 2) {  // two entries per shared-memory read: that pipe is the busiest one here
+          const uint4 ent = reinterpret_cast<const uint4*>(slot)[e / 2];
           v[e] = ldg_if_clear(in_px + (int)ent.x, ent.y, mask);
+          v[e + 1] = ldg_if_clear(in_px + (int)ent.z, ent.w, mask);
         }
         return;
       }
@@ -661,6 +662,7 @@ struct WgradParams {
   int tiles_per_group;
   int n_real, n_pad;
   int m_tiles, subs, stages;
+  int x_count;            // elements of x from the first group's on (wgrad_ts_kernel with wide loads)
   int ones_row;           // index of the all-ones row among the lowered-matrix rows
   int kblocks_total, kblocks_per_split;  // end of this launch's k-block range, k-blocks per split
   int kb_first;                          // first k-block of this launch (a later round of a launch sequence starts further in)
@@ -904,22 +906,54 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
 // the lowered rows from shared memory, 192 of them per instruction (two accumulators of 192 columns): per k-block 24
 // MMAs of 96 cycles each, none paying the shared-memory-A surcharge, where wgrad_kernel issues 36 of 91, and one CTA
 // covers all rows, so dY is staged once per k-block for the whole SM.
-//   warps 0-23  tap producers: warp w stages rows w, w+24, ... (16 rows) of the 384-row tile exactly as wgrad_kernel's.
-//   warps 24-27 dY: warp 24+q owns channels 32q .. 32q+31 (= its tensor-memory lanes): coalesced loads with lane = pixel,
+//   warps 0-23  tap producers: warp w stages rows w, w+24, ... (16 rows) of the 384-row tile exactly as wgrad_kernel's
+//               (WIDE: warps 0-17, two window rows each).
+//   warps 24-27 dY (WIDE: 18-25, two per quadrant): the warp of quadrant q owns channels 32q .. 32q+31 (= the tensor-memory
+//               lanes it reaches): coalesced loads with lane = pixel,
 //               a turn through a private 32 x 33 shared-memory tile, then lane = channel: split and tcgen05.st.
 //               After the last k-block the same warps write the accumulators out (lane = channel = fastest index of the
 //               partial-sum buffer).
-//   warp 28     one thread issues the MMAs.
+//   last warp   issues the MMAs.
 // The partial sums have wgrad_kernel's layout ([split][tile][row][channel]), so the same reduction kernels follow.
-constexpr int kTsTapWarps = 24, kTsDyWarps = 4, kTsMmaWarp = kTsTapWarps + kTsDyWarps;
-constexpr int kTsThreads = (kTsMmaWarp + 1) * 32;  // 928
-constexpr int kTsRows = 384, kTsNTile = 192, kTsStages = 2, kTsRowsPerWarp = kTsRows / kTsTapWarps;  // 16
+__host__ __device__ constexpr int ts_tap_warps(bool wide) { return wide ? 18 : 24; }
+__host__ __device__ constexpr int ts_dy_warps(bool wide) { return wide ? 8 : 4; }
+__host__ __device__ constexpr int ts_threads(bool wide) { return (ts_tap_warps(wide) + ts_dy_warps(wide) + 1) * 32; }  // 864 or 928
+constexpr int kTsRows = 384, kTsNTile = 192, kTsStages = 2;
 constexpr uint32_t kTsTile = kTsRows * 128u;       // one of hi / lo of the lowered rows of a k-block
 constexpr uint32_t kTsStage = 2u * kTsTile;
 constexpr uint32_t kTsTapsOff = kTsStages * kTsStage, kTsTurnOff = kTsTapsOff + kTsRows * 8u,
-                   kTsBarsOff = kTsTurnOff + kTsDyWarps * 32u * 33u * 4u, kTsSmem = kTsBarsOff + 8u * (2 * kTsStages + 1) + 16u;
+                   kTsBarsOff = kTsTurnOff + 4u * 32u * 33u * 4u, kTsSmem = kTsBarsOff + 8u * (2 * kTsStages + 1) + 16u;
 
-__global__ void __launch_bounds__(kTsThreads, 1) wgrad_ts_kernel(const __grid_constant__ WgradParams P) {
+//
+// WIDE (stride a multiple of four, no padding): a tap warp stages whole window rows (input channel, kernel row).  The pixels of
+// an image then lie at the same place in their 16-byte blocks, so the k consecutive elements that a pixel needs come with
+// three or four aligned loads, and which loaded word is which tap is the same for the whole warp: a branch, no selects.  A
+// load per element touched sixteen sectors for the four it used, and the load pipe bound the kernel.  A k-block that crosses
+// images, or the tensor's ends, loads element by element.  18 tap warps and 8 dY warps then: with four the turn of dY was the
+// longest chain of a k-block.  AlexNet conv1 at batch 256 393 -> 358 us (the MMAs alone would take 205), 16 images of
+// 100 x 100 30.4 -> 18.0; what is left is the round of loads, stores and barriers that two stages cannot hide.
+constexpr int kTsWideTaps = 13, kTsWideRows = 2;  // taps that four blocks cover at any alignment; window rows per warp
+
+__device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Splits taps 0 .. k - 1, which start at w[SHIFT], and stores them as lowered rows: row r at dst + off[r & 7] + (r & ~7) * 128.
+template <int SHIFT>
+__device__ __forceinline__ void store_wide(const float* w, int k, uint8_t* dst, const uint32_t* off) {
+#pragma unroll
+  for (int r = 0; r < kTsWideTaps; ++r) {
+    if (r >= k) break;
+    uint32_t h, l;
+    split_tf32_trunc(w[SHIFT + r], h, l);
+    uint8_t* at = dst + off[r & 7] + (r & ~7) * 128;
+    *reinterpret_cast<uint32_t*>(at) = h;
+    *reinterpret_cast<uint32_t*>(at + kTsTile) = l;
+  }
+}
+
+template <bool WIDE>
+__global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __grid_constant__ WgradParams P) {
+  constexpr int kTsTapWarps = ts_tap_warps(WIDE), kTsDyWarps = ts_dy_warps(WIDE), kTsMmaWarp = kTsTapWarps + kTsDyWarps;
+  constexpr int kTsThreads = ts_threads(WIDE), kTsRowsPerWarp = kTsRows / 24;  // 16
   pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -932,7 +966,16 @@ __global__ void __launch_bounds__(kTsThreads, 1) wgrad_ts_kernel(const __grid_co
   const int grp = vg / P.tiles_per_group, ntile = vg % P.tiles_per_group;
   constexpr uint32_t kACol0 = 2 * kTsNTile;  // tensor memory: two accumulators of 192 columns, then 2 x 64 columns of A
 
-  for (int i = tid; i < kTsRows; i += kTsThreads) s_taps[i] = P.taps[i];
+  if (WIDE) {  // lowered rows that no warp stages: zeros
+    const int words = (kTsRows - P.ones_row - 1) * 32;
+    for (int i = tid; i < words * 2 * kTsStages; i += kTsThreads) {
+      const int part = i / words;
+      reinterpret_cast<uint32_t*>(base_ptr + (size_t)part * kTsTile + (size_t)(P.ones_row + 1) * 128)[i - part * words] = 0u;
+    }
+    fence_proxy_async_smem();
+  } else {
+    for (int i = tid; i < kTsRows; i += kTsThreads) s_taps[i] = P.taps[i];
+  }
   if (tid == 0) {
     for (int s = 0; s < kTsStages; ++s) { mbar_init(full + 8u * s, kTsTapWarps + kTsDyWarps); mbar_init(empty + 8u * s, 1); }
     mbar_init(acc_full, 1);
@@ -964,7 +1007,90 @@ __global__ void __launch_bounds__(kTsThreads, 1) wgrad_ts_kernel(const __grid_co
       while (pc >= P.m) { pc -= P.m; ++pr; }
       while (pr >= P.m) { pr -= P.m; ++pb; }
     };
-    if (warp < kTsTapWarps) {
+    if (WIDE && warp < kTsTapWarps) {
+      // ---- window rows u = 2 warp and 2 warp + 1: lowered rows u * k + kc, whose swizzle phases repeat after eight
+      const int k = P.k, units = P.ones_row / k, mine = min(kTsWideRows, max(0, units - kTsWideRows * warp));
+      const float* x = P.x + (long long)grp * P.x_group_stride;
+      int unit_at[kTsWideRows];
+      uint32_t lane_off[kTsWideRows][8];
+#pragma unroll
+      for (int i = 0; i < kTsWideRows; ++i) {
+        const int u = kTsWideRows * warp + i, d = u / k;
+        unit_at[i] = d * P.n * P.n + (u - d * k) * P.n;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) lane_off[i][r] = (uint32_t)((u * k + r) * 128 + (((lane >> 2) ^ ((u * k + r) & 7)) << 4) + (lane & 3) * 4);
+      }
+      const int ones = warp == kTsTapWarps - 1 ? P.ones_row : -1;
+      const int misaligned = (int)((reinterpret_cast<uintptr_t>(x) >> 2) & 3);  // words between x and its 16-byte block
+      float w[kTsWideRows][16];
+      int shift[kTsWideRows] = {0, 0};
+      bool ok = false;
+      auto load_rows = [&]() {
+        ok = pix < P.n_pix;
+        const int at0 = pb * (int)P.x_batch_stride + pr * P.s * P.n + pc * P.s;
+        // The lines of the k-block after the next one (if it lies in the same image), every eighth lane one line: with one
+        // k-block's loads in flight a trip to HBM was longer than the MMAs it hid behind.
+        int far_r = pr, far_c = pc + 2 * kBlockK;
+        while (far_c >= P.m) { far_c -= P.m; ++far_r; }
+        const bool far_in = far_r < P.m && (lane & 7) == 0;
+        const int far0 = pb * (int)P.x_batch_stride + far_r * P.s * P.n + far_c * P.s;
+        const int pb0 = __shfl_sync(0xffffffffu, pb, 0);
+        const bool one_image = __all_sync(0xffffffffu, ok && pb == pb0);
+#pragma unroll
+        for (int i = 0; i < kTsWideRows; ++i) {
+          if (i >= mine) break;
+          const int at = at0 + unit_at[i];
+          if (far_in && ok) prefetch_l2(x + far0 + unit_at[i]);
+          shift[i] = (at + misaligned) & 3;  // of this lane; of every lane where the pixels are one image's
+          const int first = at - shift[i];
+          if (__all_sync(0xffffffffu, one_image && first >= 0 && first + 16 <= P.x_count)) {
+            const float4* block = reinterpret_cast<const float4*>(x + first);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (4 * j >= k + shift[i]) break;
+              const float4 v = __ldg(block + j);
+              w[i][4 * j] = v.x; w[i][4 * j + 1] = v.y; w[i][4 * j + 2] = v.z; w[i][4 * j + 3] = v.w;
+            }
+          } else {
+            shift[i] = 0;
+#pragma unroll
+            for (int r = 0; r < kTsWideTaps; ++r) {
+              if (r >= k) break;
+              w[i][r] = ok ? __ldg(x + at + r) : 0.f;
+            }
+          }
+        }
+      };
+      load_rows();
+      Ring ring;
+      for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(kTsStages)) {
+        const int s = ring.idx, use = ring.use;
+        if (use > 0) mbar_wait(empty + 8u * s, (uint32_t)(use - 1) & 1u, failed, P.status, 0x3010);
+#pragma unroll
+        for (int i = 0; i < kTsWideRows; ++i) {
+          if (i >= mine) break;
+          uint8_t* dst = base_ptr + (size_t)s * kTsStage;
+          switch ((int)warp_uniform((uint32_t)shift[i])) {
+            case 0: store_wide<0>(w[i], k, dst, lane_off[i]); break;
+            case 1: store_wide<1>(w[i], k, dst, lane_off[i]); break;
+            case 2: store_wide<2>(w[i], k, dst, lane_off[i]); break;
+            default: store_wide<3>(w[i], k, dst, lane_off[i]); break;
+          }
+        }
+        if (ones >= 0) {
+          uint8_t* dst = base_ptr + (size_t)s * kTsStage + ones * 128 + (((lane >> 2) ^ (ones & 7)) << 4) + (lane & 3) * 4;
+          *reinterpret_cast<float*>(dst) = ok ? 1.f : 0.f;
+          *reinterpret_cast<float*>(dst + kTsTile) = 0.f;
+        }
+        if (kbl + 1 < kblocks) {  // the next k-block's loads go in flight before the barrier work
+          next_pixel();
+          load_rows();
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + 8u * s);
+      }
+    } else if (warp < kTsTapWarps) {
       // ---- lowered rows warp + 24*i: row offsets 3072 bytes apart, all with the swizzle phase of row `warp`
       const float* xg = P.x + (long long)grp * P.x_group_stride;
       const bool mine = P.ones_row % kTsTapWarps == warp;
@@ -1012,27 +1138,43 @@ __global__ void __launch_bounds__(kTsThreads, 1) wgrad_ts_kernel(const __grid_co
         if (lane == 0) mbar_arrive(full + 8u * s);
       }
     } else {
-      // ---- dY: channels 32q .. 32q+31 of the tile; tensor-memory lanes of the same numbers
-      const int q = warp - kTsTapWarps;
-      const float* dyg = P.dy + (long long)(grp * P.dy_group_channels + ntile * P.n_real + q * 32) * P.mm;
+      // ---- dY: channels 32q .. 32q+31 of the tile; tensor-memory lanes of the same numbers.  With eight warps two share a
+      // quadrant: each loads half of its channels and stores half of the pixels.
+      constexpr int kHalves = kTsDyWarps / 4, kChannels = 32 / kHalves;
+      const int q = warp & 3, half = (warp - kTsTapWarps) >> 2;  // a warp reaches the tensor-memory lanes of its number mod 4
+      const int ch0 = q * 32 + half * kChannels;
+      const float* dyg = P.dy + (long long)(grp * P.dy_group_channels + ntile * P.n_real + ch0) * P.mm;
       const int n_live = min(P.n_real, P.dy_group_channels - ntile * P.n_real);  // the last tile of a group may be shorter
-      const int live = min(32, max(0, n_live - q * 32));  // real channels of this quadrant
+      const int live = min(kChannels, max(0, n_live - ch0));  // real channels of this warp
       float* turn = reinterpret_cast<float*>(base_ptr + kTsTurnOff) + q * (32 * 33);
-      const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + kACol0;
-      float vb[32];
+      const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + kACol0 + (uint32_t)(half * kChannels);
+      auto quadrant_sync = [&]() {
+        if (kHalves == 1) __syncwarp();
+        else asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+      };
+      float vb[kChannels];
       auto load_rows = [&]() {
         const bool ok = pix < P.n_pix;
         const float* dsrc = dyg + (long long)pb * P.dy_batch_stride + pr * P.m + pc;
+        // one lane per channel: the line two k-blocks on
+        if (WIDE && lane < live && pr * P.m + pc + 2 * kBlockK < P.mm && ok) prefetch_l2(dsrc + (long long)lane * P.mm + 2 * kBlockK - lane);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) vb[i] = ldg_if(dsrc + (long long)i * P.mm, (ok && i < live) ? 1u : 0u);
+        for (int i = 0; i < kChannels; ++i) {
+          if (WIDE) {
+            vb[i] = ok && i < live ? __ldg(dsrc) : 0.f;
+            dsrc += P.mm;
+          } else {
+            vb[i] = ldg_if(dsrc + (long long)i * P.mm, (ok && i < live) ? 1u : 0u);
+          }
+        }
       };
       load_rows();
       Ring ring;
       for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(kTsStages)) {
         const int s = ring.idx, use = ring.use;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) turn[i * 33 + lane] = vb[i];  // row = channel, column = pixel
-        __syncwarp();
+        for (int i = 0; i < kChannels; ++i) turn[(half * kChannels + i) * 33 + lane] = vb[i];  // row = channel, column = pixel
+        quadrant_sync();
         if (kbl + 1 < kblocks) {
           next_pixel();
           load_rows();
@@ -1042,16 +1184,16 @@ __global__ void __launch_bounds__(kTsThreads, 1) wgrad_ts_kernel(const __grid_co
         tc_fence_after();
         const uint32_t st_addr = lane_addr + (uint32_t)(s * 64);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {  // lane = channel now: its 32 pixels, eight at a time
+        for (int c = 0; c < kChannels / 8; ++c) {  // lane = channel now: its pixels, eight at a time
           uint32_t hi[8], lo[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) split_tf32_trunc(turn[lane * 33 + c * 8 + e], hi[e], lo[e]);
+          for (int e = 0; e < 8; ++e) split_tf32_trunc(turn[lane * 33 + half * kChannels + c * 8 + e], hi[e], lo[e]);
           tmem_st8(st_addr + (uint32_t)(c * 8), hi);
           tmem_st8(st_addr + 32u + (uint32_t)(c * 8), lo);
         }
         tmem_wait_st();
         tc_fence_before();
-        __syncwarp();  // also: every lane has read the tile before the next k-block overwrites it
+        quadrant_sync();  // also: every lane has read the tile before the next k-block overwrites it
         if (lane == 0) mbar_arrive(full + 8u * s);
       }
       // ---- epilogue: lane = channel, one accumulator column = one lowered row
@@ -1059,7 +1201,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) wgrad_ts_kernel(const __grid_co
       tc_fence_after();
       const int ch = q * 32 + lane;
       float* op = P.partial + ((size_t)split * gridDim.z + vg) * kTsRows * P.n_pad + ch;
-      for (int c = 0; c < kTsRows / 16; ++c) {
+      for (int c = half; c < kTsRows / 16; c += kHalves) {
         float acc[16];
         tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 16), acc);
         if (!failed && ch < P.n_pad) {
@@ -1810,7 +1952,9 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
   for (auto kernel : {gather_conv_kernel<2, kByTap>, gather_conv_kernel<2, kByRun>, gather_conv_kernel<2, kWeightGrad>})
     if (rc == CCT_OK) rc = set_smem(ctx, kernel, 113 * 1024);
   if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad), kSmemLimit);
-  if (rc == CCT_OK && p->w_ts) rc = set_smem(ctx, wgrad_ts_kernel, kSmemLimit);
+  if (p->w_ts)
+    for (auto kernel : {wgrad_ts_kernel<false>, wgrad_ts_kernel<true>})
+      if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
   if (rc != CCT_OK) {
     umma_plan_destroy(ctx, p);
     return rc;
@@ -1996,8 +2140,12 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       rows_pad = p->ws_rows * kSwTile;
       launch_pdl(small_wgrad_kernel, dim3(p->ws_rows * p->ws_cols * vgroups, p->w_splits), dim3(kSwThreads), 0, ctx->stream, P,
                  rows_pad, p->ws_rows, p->ws_cols, p->ws_pix);
-    } else if (p->w_ts)
-      launch_pdl(wgrad_ts_kernel, dim3(grid), dim3(kTsThreads), p->w_smem, ctx->stream, P);
+    } else if (p->w_ts) {
+      // Wide loads: see the kernel.  Below eight taps a window row has fewer than three blocks' worth.
+      P.x_count = (int)((long long)G.B * G.D * G.n * G.n - (G.g - 1) * P.x_group_stride);
+      const bool wide = G.s % 4 == 0 && G.p == 0 && G.k >= 8 && G.k <= kTsWideTaps && G.Dg * G.k <= kTsWideRows * ts_tap_warps(true);
+      launch_pdl(wide ? wgrad_ts_kernel<true> : wgrad_ts_kernel<false>, dim3(grid), dim3(ts_threads(wide)), p->w_smem, ctx->stream, P);
+    }
     else
       launch_pdl(wgrad_pick(p->w_subs, f.n_pad), dim3(grid), dim3(kWgThreads), p->w_smem, ctx->stream, P);
     t->end(1, ctx->stream);
