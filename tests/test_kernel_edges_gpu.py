@@ -1,0 +1,144 @@
+"""The branches that a layer's sizes choose between, each at the sizes where it can go wrong: edges of tiles, remainders, the
+smallest and largest of its range."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from caffecontroll_b200 import FullyConnectedBridge, Layer, LogicalCube, capi
+from oracle import pyoracle
+from tests.parity import assert_close, make_inputs
+
+pytestmark = pytest.mark.gpu
+
+TENSOR = 2
+
+
+def vp(p):
+    return C.c_void_p(p)
+
+
+# Window rows loaded in 16-byte blocks (stride a multiple of four, no padding), k-blocks that cross images, odd planes whose
+# blocks are misaligned, the tensor's ends, groups; then narrow data gradients, whose accumulator holds several rows of pixels,
+# with a last block that is cut off, padding and stride.  Tolerance: tests/parity.py (1e-4; the split operands stay below 2e-5).
+@pytest.mark.parametrize("shape", [
+    (1, 3, 11, 8, 11, 4, 0, 1), (3, 3, 47, 24, 11, 4, 0, 1), (5, 4, 23, 17, 8, 4, 0, 1), (2, 2, 61, 128, 13, 8, 0, 1),
+    (2, 6, 39, 40, 11, 4, 0, 2), (2, 4, 30, 9, 9, 4, 0, 1), (2, 3, 40, 16, 11, 4, 5, 1),
+    (6, 20, 28, 32, 5, 1, 2, 1), (9, 16, 33, 64, 3, 1, 1, 1), (4, 24, 29, 80, 5, 2, 2, 1), (3, 3, 57, 96, 11, 4, 0, 1),
+])
+def test_convolution_shapes(ctx, port, shape):
+    from caffecontroll_b200 import conv_layer
+    B, D, n, o, k, s, p, g = shape
+    X, W, b, dY = make_inputs(29, B, D, n, o, k, s, p, g)
+    Y, dX, dW, db, used = conv_layer(ctx, X, W, b, dY, k, s, p, g, algo=TENSOR)
+    assert used == TENSOR
+    dXr, dWr, dbr = port.conv_backward(X, W, dY, k, s, p, g)
+    for a, r, name in ((Y, port.conv_forward(X, W, b, k, s, p, g), "Y"), (dX, dXr, "dX"), (dW, dWr, "dW"), (db, dbr, "db")):
+        assert_close(a, r.reshape(a.shape), name)
+
+
+# Inner products: one product, features that are no multiple of four (padded copies or the fp32 kernel), both sides of the
+# line between the fp32 and the tensor-core kernel, batches at the accumulator widths of 64, 128 and 256 columns.
+# Tolerance: products of unit values summed over K: split operands leave 2^-20 of the sum of magnitudes, far below 1e-4.
+@pytest.mark.parametrize("B,K,o", [(1, 1, 1), (3, 5, 7), (50, 500, 10), (33, 1023, 129), (64, 515, 2050), (65, 2049, 513),
+                                   (128, 1026, 514), (129, 770, 1027), (257, 301, 260)])
+def test_inner_product_sizes(ctx, B, K, o):
+    rng = np.random.default_rng(B + K + o)
+    X, W, b, dY = (rng.standard_normal(s).astype(np.float32) for s in ((B, K, 1, 1), (o, K, 1, 1), (o,), (B, o, 1, 1)))
+    xin = Layer(LogicalCube.from_numpy(ctx, X), LogicalCube(ctx, 1, 1, K, B))
+    out = Layer(LogicalCube(ctx, 1, 1, o, B), LogicalCube.from_numpy(ctx, dY))
+    fc = FullyConnectedBridge(xin, out, True)
+    fc.p_model_cube.upload(W)
+    fc.p_bias_cube.upload(b)
+    fc.forward()
+    fc.backward()
+    ctx.sync()
+    X2, W2, dY2 = X.reshape(B, K).astype(np.float64), W.reshape(o, K).astype(np.float64), dY.reshape(B, o).astype(np.float64)
+    for cube, r, name in ((out.p_data_cube, X2 @ W2.T + b, "Y"), (xin.p_gradient_cube, dY2 @ W2, "dX"),
+                          (fc.p_model_gradient_cube, dY2.T @ X2, "dW"), (fc.p_bias_gradient_cube, dY2.sum(0), "db")):
+        got = cube.download()
+        assert_close(got, r.astype(np.float32).reshape(got.shape), name)
+    fc.close()
+
+
+def test_sgd_in_one_launch_equals_one_launch_per_tensor(ctx):
+    """Bit for bit, over tails, chunks of one tensor that end inside a vector, and buffers off a 16-byte boundary."""
+    rng = np.random.default_rng(5)
+    items, cubes = (capi.SgdItem * 6)(), []
+    for i, (n, shift, lam) in enumerate([(1, 0, 0.0), (7, 1, 5e-4), (4096, 0, 5e-4), (4099, 0, 0.0), (100003, 0, 5e-4), (70001, 3, 5e-4)]):
+        values = [rng.standard_normal(n + shift).astype(np.float32) for _ in range(3)]
+        pair = [[LogicalCube.from_numpy(ctx, v.reshape(1, -1, 1, 1)) for v in values] for _ in range(2)]
+        one, many = ([c.ptr + 4 * shift for c in cs] for cs in pair)
+        capi.check(ctx.lib.cct_sgd_step(ctx.h, n, vp(one[0]), vp(one[1]), vp(one[2]), 0.01, 0.9, lam), "sgd", ctx.h)
+        items[i] = capi.SgdItem(n, many[0], many[1], many[2], 0.01, 0.9, lam)
+        cubes.append(pair)
+    capi.check(ctx.lib.cct_sgd_step_multi(ctx.h, 6, items), "sgd multi", ctx.h)
+    ctx.sync()
+    for one, many in cubes:
+        for a, b in zip(one, many):
+            assert np.array_equal(a.download(), b.download())
+
+
+# Strips of windows and of 2 x 2 blocks: planes smaller than a strip, strips that are cut off, odd and even planes.
+@pytest.mark.parametrize("B,D,n,k,s", [(1, 1, 3, 3, 2), (2, 3, 4, 3, 2), (3, 5, 8, 3, 2), (1, 7, 23, 3, 2), (5, 17, 13, 3, 2),
+                                       (1, 3, 2, 2, 2), (3, 5, 7, 2, 2), (2, 9, 24, 2, 2)])
+def test_pooling_planes(ctx, port, B, D, n, k, s):
+    m = (n - k) // s + 1
+    rng = np.random.default_rng(n)
+    A = rng.integers(-3, 4, (B, D, n, n)).astype(np.float32)  # many equal values: the first maximum has to win
+    dP = rng.standard_normal((B, D, m, m)).astype(np.float32)
+    Yr, idxr = port.maxpool_forward(A, k, s)
+    cA, cdP = LogicalCube.from_numpy(ctx, A), LogicalCube.from_numpy(ctx, dP)
+    cY, cI, cdA = LogicalCube(ctx, m, m, D, B), LogicalCube(ctx, m, m, D, B), LogicalCube(ctx, n, n, D, B)
+    capi.check(ctx.lib.cct_maxpool_forward(ctx.h, vp(cA.ptr), vp(cY.ptr), vp(cI.ptr), B * D, n, k, s), "pool fwd", ctx.h)
+    capi.check(ctx.lib.cct_maxpool_backward(ctx.h, vp(cdP.ptr), vp(cI.ptr), vp(cdA.ptr), B * D, n, k, s), "pool bwd", ctx.h)
+    ctx.sync()
+    assert np.array_equal(cY.download(), Yr) and np.array_equal(cI.download().view(np.int32), idxr.reshape(B, D, m, m))
+    assert np.array_equal(cdA.download(), port.maxpool_backward(dP, idxr, n))
+
+
+@pytest.mark.parametrize("B,classes", [(1, 1), (1, 2), (7, 1024), (5, 1025), (3, 4001)])
+def test_softmax_class_counts(ctx, B, classes):
+    """Tolerance: parity's 1e-4 against the fp32 sums' (classes + B) * 2^-24 < 3e-4 of terms that are positive, in practice 1e-6."""
+    rng = np.random.default_rng(classes)
+    X = (3 * rng.standard_normal((B, classes, 1, 1))).astype(np.float32)
+    labels = rng.integers(0, classes, B).astype(np.float32)
+    pr, lr, gr = pyoracle.np_softmax_loss(X, labels, scale=1.0 / B)
+    cX, cL = LogicalCube.from_numpy(ctx, X), LogicalCube.from_numpy(ctx, labels.reshape(B, 1, 1, 1))
+    cP, cG, cIL, cLoss = (LogicalCube(ctx, 1, 1, d, b) for d, b in ((classes, B), (classes, B), (1, B), (1, 1)))
+    for _ in range(2):  # the second call finds the counter that the first one left
+        capi.check(ctx.lib.cct_softmax_loss_forward(ctx.h, vp(cX.ptr), vp(cL.ptr), vp(cP.ptr), vp(cIL.ptr), vp(cLoss.ptr), B,
+                                                    classes), "softmax fwd", ctx.h)
+        capi.check(ctx.lib.cct_softmax_loss_backward(ctx.h, vp(cP.ptr), vp(cL.ptr), vp(cG.ptr), B, classes, 1.0 / B),
+                   "softmax bwd", ctx.h)
+        ctx.sync()
+        assert_close(cP.download(), pr, "probabilities")
+        assert abs(float(cLoss.download().reshape(-1)[0]) - lr) <= 1e-4 * abs(lr) + 1e-6
+        assert_close(cG.download(), gr, "gradient")
+
+
+def test_recorded_step_equals_the_bridges_one_by_one(ctx):
+    """Three steps through the recorded program (its first run call by call, the later ones as a graph), a change of a
+    bridge's switch that has to be noticed, one more step: the same bits as a network whose bridges are walked through."""
+    from caffecontroll_b200.net import Net, parse_prototxt, solver_from_message
+    from tests.test_net_gpu import B, NET, SOLVER
+    net_param, solver = parse_prototxt(NET.replace("dropout_ratio: 0.5", "dropout_ratio: 0.4")), solver_from_message(parse_prototxt(SOLVER))
+    rng = np.random.default_rng(3)
+    X, labels = rng.standard_normal((B, 3, 67, 67)).astype(np.float32), rng.integers(0, 12, B).astype(np.float32)
+    results = []
+    for recorded in (True, False):
+        net = Net(ctx, net_param, solver, B, fuse=True)
+        net.set_input(X, labels)
+        for i in range(4):
+            if i == 3:
+                net.bridges[net.names.index("fc7")].needs_to_calc_backward_grad = False
+            if recorded:
+                net.step()
+            else:
+                net.forward()
+                net.backward()
+        ctx.sync()
+        results.append([pb.get_model_cube().download() for _, pb in net.param_bridges()])
+        net.close()
+    for a, b in zip(*results):
+        assert np.array_equal(a, b)
