@@ -1357,7 +1357,8 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
   // One warp per plane at a time, eight loads in flight per lane; no block-wide synchronisation.
   const int lane = threadIdx.x & 31;
   const int warp0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int plane = warp0; plane < planes; plane += nwarps) {
+  for (int turn = warp0; turn < planes; turn += nwarps) {
+    const int plane = planes - 1 - turn;  // what the kernel before wrote last is still in L2
     const int b = plane / channels, c = plane - b * channels;
     const int grp = c / og, j = c - grp * og;
     const int tile = j / ch_tile, within = j - tile * ch_tile;

@@ -348,8 +348,12 @@ __global__ void __launch_bounds__(256) maxpool_fwd_staged_kernel(const float* __
       r[j] = i < total_in ? __ldg(in + i) : 0.f;
     }
   };
-  if (via_regs && (int)blockIdx.x * group < planes) fetch(blockIdx.x * group);
-  for (int p0 = blockIdx.x * group; p0 < planes; p0 += gridDim.x * group) {
+  // From the last group to the first: X is usually what the kernel before has written, and its last tens of megabytes are
+  // still in L2.
+  const int groups = (planes + group - 1) / group;
+  if (via_regs && (int)blockIdx.x < groups) fetch((groups - 1 - (int)blockIdx.x) * group);
+  for (int turn = blockIdx.x; turn < groups; turn += gridDim.x) {
+    const int p0 = (groups - 1 - turn) * group;
     const int g = min(group, planes - p0);
     const float* in = X + (size_t)p0 * nn;
     const int total_in = g * nn, total_out = g * mm;
@@ -361,8 +365,8 @@ __global__ void __launch_bounds__(256) maxpool_fwd_staged_kernel(const float* __
         if (i < total_in) plane_smem[i] = r[j];
       }
       __syncthreads();
-      const int next = p0 + gridDim.x * group;
-      if (next < planes) fetch(next);
+      const int next = p0 - (int)gridDim.x * group;
+      if (next >= 0) fetch(next);
     } else {
       int i = threadIdx.x;
       for (; i + 3 * 256 < total_in; i += 4 * 256) {
