@@ -407,8 +407,10 @@ def run_conv_stack(args, rank, world, local_rank):
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     barrier()
     e0.record(stream)
+    counted = capi.kernel_launches()
     for _ in range(args.steps):
         step()
+    timed_launches = capi.kernel_launches() - counted
     e1.record(stream)
     barrier()
     ms_total = e0.elapsed_time(e1)
@@ -452,7 +454,7 @@ def run_conv_stack(args, rank, world, local_rank):
                          "peak_source": "%s: bf16 burst %.1f TFLOP/s / 2 / 3 - of measured; sustained figure %.1f" %
                                         (peaks["source"], peaks["bf16_tflops"], (peaks.get("bf16_tflops_sustained") or 0) / 6.0),
                          "flops_per_step": flops, "layers": per_layer},
-            "cpu_baseline": None, "e2e": None, "clocks": clocks, "gpu_launches": None,
+            "cpu_baseline": None, "e2e": None, "clocks": clocks, "gpu_launches": timed_launches,
         }
         print(json.dumps(line), flush=True)
     if world > 1:
@@ -601,8 +603,10 @@ def run_caffenet(args, rank, world, local_rank):
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     barrier()
     e0.record(stream)
+    counted = capi.kernel_launches()
     for _ in range(args.steps):
         net.step()
+    timed_launches = capi.kernel_launches() - counted
     e1.record(stream)
     barrier()
     ms_step = max_over_ranks(e0.elapsed_time(e1)) / args.steps
@@ -814,7 +818,7 @@ def run_caffenet(args, rank, world, local_rank):
                            "the iteration, the loss copied back to pinned host memory and read by the host one step later",
                     "last_loss": e2e_losses[-1] if e2e_losses else None, "h2d_ms_per_upload": h2d_ms,
                     "h2d_gbs": X.nbytes / (h2d_ms * 1e-3) / 1e9 if h2d_ms > 0 else None},
-            "clocks": clocks, "gpu_launches": net.launches_per_step() * args.steps,
+            "clocks": clocks, "gpu_launches": timed_launches,
             "allreduce_bytes_per_step": 4 * net.num_parameters() if world > 1 else 0,
             "allreduce_ms_alone": ar_alone_ms,
         }
@@ -1025,8 +1029,10 @@ def main():
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     barrier()
     e0.record(stream)
+    counted = capi.kernel_launches()
     for _ in range(args.steps):
         step()
+    timed_launches = capi.kernel_launches() - counted
     e1.record(stream)
     barrier()
     ms_total = e0.elapsed_time(e1)
@@ -1106,9 +1112,6 @@ def main():
         if world == 1 and not args.no_cpu_baseline:
             cpu = cpu_reference_time(w, 3, 1, False)
             cpu.pop("seconds_per_step", None)
-        # tcgen05 path: pack + gather (forward); dY split + gather + reduce + bias sums (or wgrad + reduce for short
-        # lowered matrices), pack + gather (backward); two SGD kernels
-        launches_per_step = (2 + (6 if wg_gather else 4) + 2) if algo.value == 2 else (1 + 3 + 2)
         line = {
             "metric": METRIC, "value": world * B / (ms_step * 1e-3), "unit": "images/s", "n_gpus": world,
             "steps": args.steps, "warmup": warm_steps, "ms_per_step": ms_step, "higher_is_better": True,
@@ -1118,7 +1121,7 @@ def main():
             "roofline": roofline, "cpu_baseline": cpu,
             "e2e": {"value": world * B / e2e_s, "unit": "images/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "ms_per_step": e2e_s * 1e3, "steps": args.e2e_steps},
-            "clocks": clocks, "gpu_launches": (launches_per_step + (1 if w.get("pool") else 0)) * args.steps,
+            "clocks": clocks, "gpu_launches": timed_launches,
         }
         if remnants:
             line["hbm_bound_passes"] = remnants

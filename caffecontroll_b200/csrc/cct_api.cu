@@ -413,6 +413,7 @@ struct cct_program {
   // microseconds per kernel (LeNet's iteration: 30 kernels, 127 us with 100 us of work in them), the graph about ten in all.
   int runs = 0;
   cudaGraphExec_t graph = nullptr;
+  uint64_t graph_kernels = 0;
   bool no_graph = false;  // capturing failed once: call by call for good
 };
 
@@ -432,7 +433,10 @@ bool capture_program(cct_program* p) {
   const cudaStream_t own = ctx->stream;
   ctx->stream = ctx->capture_stream;
   bool ok = true;
+  const uint64_t counted = thread_launches;
   for (const auto& call : p->calls) ok = ok && call() == CCT_OK;
+  p->graph_kernels = thread_launches - counted;  // captured, not launched
+  kernel_launches -= p->graph_kernels;
   ctx->stream = own;
   cudaGraph_t graph = nullptr;
   ok = cudaStreamEndCapture(ctx->capture_stream, &graph) == cudaSuccess && graph && ok;
@@ -481,6 +485,7 @@ int cct_program_run(cct_program* program) {
     if (free_stream && !program->graph) program->no_graph = !capture_program(program);
     if (free_stream && program->graph) {
       CCT_CUDA(ctx, cudaGraphLaunch(program->graph, ctx->stream));
+      kernel_launches += program->graph_kernels;
       return CCT_OK;
     }
   }
@@ -488,6 +493,12 @@ int cct_program_run(cct_program* program) {
     const int rc = call();
     if (rc != CCT_OK) return rc;
   }
+  return CCT_OK;
+}
+
+int cct_kernel_launches(unsigned long long* count) {
+  if (!count) return CCT_ERR_INVALID;
+  *count = kernel_launches;
   return CCT_OK;
 }
 

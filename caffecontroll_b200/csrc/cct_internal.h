@@ -1,5 +1,6 @@
 // Internal declarations shared by the translation units behind include/cct_b200.h.
 #pragma once
+#include <atomic>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <functional>
@@ -62,6 +63,9 @@ struct cct_ctx {
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+inline std::atomic<uint64_t> kernel_launches{0};  // cct_kernel_launches
+inline thread_local uint64_t thread_launches = 0; // those of this thread, captured ones included
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               Args&&... args) {
@@ -75,6 +79,8 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  ++thread_launches;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 #endif

@@ -302,6 +302,7 @@ class Net:
         self.fused = []
         self._update = NetworkUpdate()
         self._program, self._recorded = None, None
+        self._step_launches = 0
         if fuse:
             self._fuse()
 
@@ -461,6 +462,11 @@ class Net:
         self._recorded = (Tracked.changes, list(self.bridges))
 
     def step(self):
+        before = capi.kernel_launches()
+        self._step()
+        self._step_launches = capi.kernel_launches() - before
+
+    def _step(self):
         if self._recorded is None or self._recorded[0] != Tracked.changes or self._recorded[1] != self.bridges:
             self._record()
         if self._program is None or "forward" in self.__dict__ or "backward" in self.__dict__:
@@ -544,29 +550,8 @@ class Net:
         return sum(pb.count for pb in self.pbridges.values())
 
     def launches_per_step(self):
-        """Kernels one forward + backward + update launches, counted from the structure of the calls: convolution
-        forward = weight pack + contraction; its backward = weight gradient (dY split + contraction + split reduction +
-        bias sums for lowered matrices of 512 rows or more, else contraction + reduction), data gradient (pack +
-        contraction), plus one pass per folded mask; fully connected = contraction + reduction per pass, bias sums;
-        one kernel per parameter-free bridge pass; two SGD kernels per parameterised layer."""
-        n = 0
-        for i, br in enumerate(self.bridges):
-            t = self.types[i]
-            if t == "Convolution":
-                wg = 4 if (br.iD // br.group) * br.K * br.K >= 512 else 2
-                n += 2 + wg + (2 if br.needs_to_calc_backward_grad else 0)
-                n += (1 if br.pool_fusion is not None else 0) + (1 if br.fuse_relu_backward and br.needs_to_calc_backward_grad else 0)
-            elif t == "InnerProduct":
-                n += 2 + 2 + (2 if br.needs_to_calc_backward_grad else 0)
-            elif t == "SoftmaxWithLoss":
-                n += 3
-            elif t == "Dropout":
-                n += 1 + (0 if br.skip_forward else 1) + (0 if br.skip_backward else 1)
-            elif t == "Pooling":
-                n += 1 + (0 if br.skip_backward else 1)
-            else:
-                n += (0 if br.skip_forward else 1) + (0 if br.skip_backward else 1)
-        return n + 2 * len(self.pbridges)
+        """Kernels the last step() launched (0 before the first)."""
+        return self._step_launches
 
     def close(self):
         self.ctx.sync()

@@ -230,6 +230,9 @@ int cct_program_end(cct_program* program);
 int cct_program_run(cct_program* program);
 int cct_program_destroy(cct_program* program);
 
+/* Kernels that the library has launched in this process so far, those of recorded calls' graphs included. */
+int cct_kernel_launches(unsigned long long* count);
+
 /* Failure-path self-test (no counterpart in the reference, whose kernels never wait on anything): launches one warp
  * that waits, through the same bounded wait the convolution kernels use, on a barrier nothing completes, with a limit
  * of `limit_cycles` SM clock cycles (at most the kernels' own limit).  The wait runs out, the kernel returns normally,
