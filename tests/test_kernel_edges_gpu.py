@@ -142,3 +142,26 @@ def test_recorded_step_equals_the_bridges_one_by_one(ctx):
         net.close()
     for a, b in zip(*results):
         assert np.array_equal(a, b)
+
+
+# Host-buffer calls that move the batch in slices: a last slice of one image, a weight gradient begun before it (both kernels
+# that can be), one that cannot be split so (512 lowered rows and more), without an input gradient.
+@pytest.mark.parametrize("shape", [(17, 3, 47, 24, 11, 4, 0, 1), (33, 6, 31, 40, 5, 1, 2, 1), (16, 64, 9, 48, 3, 1, 1, 1)])
+@pytest.mark.parametrize("with_dx", [True, False])
+def test_sliced_host_calls(ctx, port, shape, with_dx):
+    B, D, n, o, k, s, p, g = shape
+    X, W, b, dY = make_inputs(31, B, D, n, o, k, s, p, g)
+    plan = C.c_void_p()
+    desc = capi.ConvDesc(B, D, n, o, k, s, p, g, 1, TENSOR)
+    capi.check(ctx.lib.cct_conv_plan_create(ctx.h, C.byref(desc), C.byref(plan)), "plan", ctx.h)
+    Y, dX, dW, db = np.zeros_like(dY), np.zeros_like(X), np.zeros_like(W), np.zeros_like(b)
+    host = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    capi.check(ctx.lib.cct_conv_forward_host(plan, host(X), host(W), host(b), host(Y), 0), "forward", ctx.h)
+    for _ in range(2):
+        capi.check(ctx.lib.cct_conv_backward_host(plan, None, None, host(dY), host(dX) if with_dx else None, host(dW), host(db)),
+                   "backward", ctx.h)
+    ctx.lib.cct_conv_plan_destroy(plan)
+    dXr, dWr, dbr = port.conv_backward(X, W, dY, k, s, p, g)
+    pairs = [(Y, port.conv_forward(X, W, b, k, s, p, g), "Y"), (dW, dWr, "dW"), (db, dbr, "db")] + ([(dX, dXr, "dX")] if with_dx else [])
+    for a, r, name in pairs:
+        assert_close(a, r.reshape(a.shape), name)
