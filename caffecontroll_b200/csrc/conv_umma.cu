@@ -122,16 +122,16 @@ __device__ __forceinline__ void stg_if(float* p, float v, uint32_t flag) {
 //               32 lowered values, splits them hi/lo and writes them with tcgen05.st into an A slot in tensor memory
 //               (sets of four warps; set g takes the k-blocks with running index == g mod SETS, each set covers
 //               all 128 lanes).
-//   MMA warp    one thread issues the MMAs: A from tensor memory, B from shared memory.
+//   MMA warp    issues the MMAs (see elect_one): A from tensor memory, B from shared memory.
 //   TMA warp    one thread streams the pre-split weight tiles (B) into shared memory with TMA (128-byte swizzle).
 //   epilogue    (4 warps) tcgen05.ld the finished accumulator, add bias / clamp, store NCHW (or depth-to-space for
 //               the strided data gradient); overlaps the next tile's MMAs when two accumulators fit.
 // Tensor memory: [accumulator(s) | A slots of 64 columns: 32 hi + 32 lo].
 // The kernel comes in two shapes.  SETS = 4: sixteen producer warps (four sets of four; set g fills the k-blocks with
 // running index == g mod 4), 704 threads, one CTA per SM with all 512 tensor-memory columns.  SETS = 2: eight producer
-// warps, 448 threads, 256 columns, two stages, one accumulator - two such CTAs share an SM, so two threads issue MMAs
-// into the SM's tensor pipe (one thread cannot issue them faster than one per ~75 cycles, however narrow they are)
-// and one CTA's epilogue overlaps the other's main loop.
+// warps, 448 threads, 256 columns, two or three A slots, one accumulator - two such CTAs share an SM, so that one CTA's
+// hand-overs and epilogue overlap the other's MMAs (CaffeNet conv2's data gradient, 48 columns: 525 us, one CTA with four
+// sets 660).
 constexpr int kEpiWarps = 4;
 __host__ __device__ constexpr int gather_threads(int sets) { return (4 * sets + 2 + kEpiWarps) * 32; }  // 704 or 448
 constexpr int kMaxAStages = 4, kMaxAccBufs = 2;
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(128) gather_reduce_kernel(const __grid_constan
 //               st.shared per row; the loads of the next k-block are issued before the warp waits for the stage
 //               buffer to drain.
 //   warps 16-23 dY producers: warp 16+w stages channel rows w, w+8, ... of the dY tile the same way.
-//   warp 24     one thread issues the MMAs (both operands from shared memory).
+//   warp 24     issues the MMAs (both operands from shared memory).
 // The producers run at about one instruction per eight cycles each (latency bound), so their number, not their
 // instruction count alone, sets the staging rate.  The finished accumulators are written to the split's slice of the
 // scratch buffer by warps 0-15.
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
   constexpr uint32_t kATile = kTileM * 128u, kBTile = NB * 16u * 128u;
   constexpr int kNPad = NB * 16;
   // Narrow dY tiles run "dual": the lo tile sits right behind the hi tile, one MMA of width 2*kNPad covers both (an
-  // MMA costs the issuing thread about 75 cycles however narrow it is), and the epilogue adds the two halves of the
+  // MMA pays some 43 cycles for reading A from shared memory, however narrow it is), and the epilogue adds the two halves of the
   // accumulator.
   constexpr bool kDual = kNPad <= 64;  // operands from shared memory: an MMA wider than 128 is slower than two narrow ones
   constexpr int kAccCols = kDual ? 2 * kNPad : kNPad;
