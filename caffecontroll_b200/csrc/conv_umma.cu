@@ -127,6 +127,12 @@ __device__ __forceinline__ void stg_if(float* p, float v, uint32_t flag) {
 //   epilogue    (4 warps) tcgen05.ld the finished accumulator, add bias / clamp, store NCHW (or depth-to-space for
 //               the strided data gradient); overlaps the next tile's MMAs when two accumulators fit.
 // Tensor memory: [accumulator(s) | A slots of 64 columns: 32 hi + 32 lo].
+// The tensor core truncates every sum it writes to the accumulator, so an accumulator loses about half a place in the last
+// per MMA.  Tiles of at most kCrossCols columns therefore have a second one for the cross terms (lo*hi + hi*lo, a factor of
+// 2^11 smaller), which the epilogue adds: one truncation at full magnitude per eight products instead of three.  Wider tiles
+// have no tensor memory to spare for it next to their A slots.  Error against 64-bit sums, 5x5, 96 -> 41 channels, positive
+// data: forward 3.8e-5 with one accumulator, 1.7e-5 with two; the price is an A slot (two instead of three at 48 and 64
+// columns) and a second tcgen05.ld in the epilogue: CaffeNet conv2's data gradient (48 columns) 531 -> 545 us.
 // The kernel comes in two shapes.  SETS = 4: sixteen producer warps (four sets of four; set g fills the k-blocks with
 // running index == g mod 4), 704 threads, one CTA per SM with all 512 tensor-memory columns.  SETS = 2: eight producer
 // warps, 448 threads, 256 columns, two or three A slots, one accumulator - two such CTAs share an SM, so that one CTA's
@@ -134,7 +140,9 @@ __device__ __forceinline__ void stg_if(float* p, float v, uint32_t flag) {
 // sets 660).
 constexpr int kEpiWarps = 4;
 __host__ __device__ constexpr int gather_threads(int sets) { return (4 * sets + 2 + kEpiWarps) * 32; }  // 704 or 448
-constexpr int kMaxAStages = 4, kMaxAccBufs = 2;
+constexpr int kMaxAStages = 4, kMaxAccBufs = 2, kCrossCols = 64;
+// Columns of one accumulator buffer: hi*hi and behind it, on narrow tiles, the cross terms.
+__host__ __device__ constexpr int acc_columns(int n_pad) { return n_pad <= kCrossCols ? 2 * n_pad : n_pad; }
 
 // Channels per table entry where the gathered tensor's channels per group are a multiple of it.  One table read, one bounds
 // test and one branch then serve kRun loads of consecutive channels, and the taps of the same kRun channels follow one
@@ -269,9 +277,20 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-  const uint32_t a_col0 = (uint32_t)(P.acc_bufs * P.n_pad);
+  const uint32_t acc_cols = (uint32_t)acc_columns(P.n_pad), cross = acc_cols - (uint32_t)P.n_pad;  // cross: 0 = one accumulator
+  const uint32_t a_col0 = (uint32_t)P.acc_bufs * acc_cols;
   const int kblocks = P.k_pad / kBlockK;
   bool failed = false;
+  // 16 columns of a finished accumulator
+  auto load_acc = [&](uint32_t taddr, float* v) {
+    tmem_ld16(taddr, v);
+    if (cross) {
+      float c[16];
+      tmem_ld16(taddr + cross, c);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] += c[j];
+    }
+  };
 
   if (warp < kProducerWarps) {
     // ------------------------------------------------------------------ producers
@@ -431,7 +450,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       const int buf = tile_iter & (P.acc_bufs - 1), ause = tile_iter >> (P.acc_bufs - 1);  // acc_bufs is 1 or 2
       if (ause > 0) mbar_wait<false>(acc_empty + 8u * buf, (uint32_t)(ause - 1) & 1u, failed, P.status, 0x20);
       tc_fence_after();
-      const uint32_t d_tmem = tmem + (uint32_t)(buf * P.n_pad);
+      const uint32_t d_tmem = tmem + (uint32_t)buf * acc_cols, d_cross = d_tmem + cross;
       for (int kb = 0; kb < kblocks; ++kb) {
         mbar_wait<false>(ready_bar + 8u * rbar.idx, (uint32_t)rbar.use & 1u, failed, P.status, 0x40);
         tc_fence_after();
@@ -442,9 +461,10 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
             const uint64_t adv = (uint64_t)(j * 2);
-            umma_tf32_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kb == 0 && j == 0) ? 0u : 1u);
-            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
-            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, 1u);
+            const uint32_t add = kb == 0 && j == 0 ? 0u : 1u;
+            umma_tf32_ts(d_cross, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, add);
+            umma_tf32_ts(d_cross, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
+            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, cross ? add : 1u);
           }
           umma_commit(done_bar + 8u * rbar.idx);  // frees the A slot for the producers and the weight slot for the TMA thread
           if (kb == kblocks - 1) umma_commit(acc_full + 8u * buf);
@@ -490,11 +510,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         // The accumulator is a 128-row slice of this split's partial sums: row-contiguous stores.
         mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
         tc_fence_after();
-        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.n_pad);
+        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * acc_cols;
         float* op = P.out + ((size_t)(id.split * P.wg_vgroups + vg) * P.wg_rows_pad + (size_t)ptile * kTileM + row) * P.n_pad;
         for (int c = 0; c < P.n_pad / 16; ++c) {
           float v[16];
-          tmem_ld16(acc + (uint32_t)(c * 16), v);
+          load_acc(acc + (uint32_t)(c * 16), v);
           if (!failed) {
             float4* o4 = reinterpret_cast<float4*>(op + c * 16);
 #pragma unroll
@@ -511,11 +531,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         // raw sums, lanes along the pixels
         mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
         tc_fence_after();
-        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.n_pad);
+        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * acc_cols;
         float* op = P.partial + (size_t)(id.split * (P.total_tiles / (P.n_pix_tiles * P.splits)) + vg) * P.n_pad * P.pix_pad + pix;
         for (int c = 0; c < P.n_pad / 16; ++c) {
           float v[16];
-          tmem_ld16(acc + (uint32_t)(c * 16), v);
+          load_acc(acc + (uint32_t)(c * 16), v);
           if (!failed) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) op[(size_t)(c * 16 + j) * P.pix_pad] = v[j];
@@ -545,11 +565,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       tc_fence_after();
       const uint32_t live = (pix < P.n_pix && !failed) ? 1u : 0u;
       const uint32_t unchecked = P.check_out ? 0u : 1u;
-      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * P.n_pad);
+      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * acc_cols;
       const int chunks = P.n_pad / 16;
       for (int c = 0; c < chunks; ++c) {
         float v[16];
-        tmem_ld16(acc + (uint32_t)(c * 16), v);
+        load_acc(acc + (uint32_t)(c * 16), v);
         // Straight-line code: table and bias reads first, then predicated st.global (a generic store could alias
         // shared memory and would pin every following table read behind it; a branch per column costs more than
         // the store it guards).
@@ -1682,16 +1702,17 @@ bool use_small_wgrad(long long pixels, int vgroups, int n, int k_real) {
 void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias) {
   // Tensor memory (512 columns) = accumulator buffers + A stages of 64 columns.  Two accumulator buffers let the epilogue
   // overlap the next tile.
+  const int acc = acc_columns(gp.n_pad);
   const int taps_smem = gp.taps_smem < 0 ? gp.splits * gp.split_k / gp.run : gp.taps_smem;
   const size_t map_k = gp.map_k ? gp.map_k : (size_t)gp.k_pad;
-  if (2 * gp.n_pad + 4 * 64 <= 512) { gp.acc_bufs = 2; gp.a_stages = 4; }
-  else if (2 * gp.n_pad + 2 * 64 <= 512 && (gp.split_k ? gp.split_k : gp.k_pad) / kBlockK <= 16) { gp.acc_bufs = 2; gp.a_stages = 2; }  // short K: the epilogue matters more
-  else { gp.acc_bufs = 1; gp.a_stages = std::min(4, (512 - gp.n_pad) / 64); }
+  if (2 * acc + 4 * 64 <= 512) { gp.acc_bufs = 2; gp.a_stages = 4; }
+  else if (2 * acc + 2 * 64 <= 512 && (gp.split_k ? gp.split_k : gp.k_pad) / kBlockK <= 16) { gp.acc_bufs = 2; gp.a_stages = 2; }  // short K: the epilogue matters more
+  else { gp.acc_bufs = 1; gp.a_stages = std::min(4, (512 - acc) / 64); }
   const int ptab = gp.taps_smem == 0 ? 16 : 0;  // weight-gradient mode: per-warp table slices (sized for 16 warps)
   gp.b_stages = gather_slots(gp.n_pad, taps_smem, n_bias, ptab, kSmemLimit);
   int b_two;
   if (two_ctas_per_sm(gp.n_pad, taps_smem, n_bias, ptab, &b_two)) {
-    gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = gp.n_pad <= 64 && !ptab ? 3 : 2; gp.b_stages = b_two;
+    gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = acc <= 64 && !ptab ? 3 : 2; gp.b_stages = b_two;
   }
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
   gp.w_half = (size_t)vgroups * gp.n_pad * map_k;
