@@ -46,6 +46,10 @@ def test_convolution_shapes(ctx, port, shape):
 @pytest.mark.parametrize("shape,which,chain", [
     ((48, 96, 24, 41, 5, 1, 2, 1), "Y", 75), ((64, 64, 20, 64, 3, 1, 1, 1), "dX", 18),
     ((48, 96, 24, 41, 5, 1, 2, 1), "dW", 58), ((64, 64, 20, 64, 3, 1, 1, 1), "dW", 28),
+    # taller pixel blocks (one row of pixels: 38 blocks, 76 at the two additions that narrow tiles may take); units of the weight
+    # gradient's splits, three additions per block on wide tiles; uneven channel tiles
+    ((32, 30, 40, 134, 3, 1, 1, 1), "dX", 76), ((32, 48, 28, 134, 3, 1, 1, 1), "dX", 76),
+    ((8, 158, 45, 136, 5, 1, 2, 1), "dW", 3 * 57), ((5, 272, 25, 208, 5, 1, 2, 2), "dW", 3 * 20), ((40, 64, 30, 337, 3, 1, 1, 1), "dW", 3 * 58),
 ])
 def test_accumulation_error(ctx, shape, which, chain):
     from caffecontroll_b200 import conv_layer
