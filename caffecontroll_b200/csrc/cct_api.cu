@@ -634,8 +634,7 @@ int cct_conv_backward_host(cct_conv_plan* plan, const float* hX, const float* hW
   const int per = slice_images(plan);
   if (per > 0) {
     // dY arrives in slices; the data gradient of a slice runs as soon as the slice is there and its dX goes back while
-    // the next slice is still arriving; the weight gradient is begun before the last slice and completed behind it (AlexNet
-    // conv1, 32 images: the link idled while 63 us of weight gradient ran).
+    // the next slice is still arriving; the weight gradient (the whole batch) follows the last slice.
     rc = host_call_begin(plan);
     if (rc != CCT_OK) return rc;
     const size_t ix = (size_t)G.D * G.n * G.n, iy = (size_t)G.o * G.m * G.m;
@@ -647,30 +646,19 @@ int cct_conv_backward_host(cct_conv_plan* plan, const float* hX, const float* hW
       CCT_CUDA(ctx, cudaMemcpyAsync(plan->sdY + b0 * iy, hdY + b0 * iy, nb * iy * 4, cudaMemcpyHostToDevice, ctx->copy_in));
       CCT_CUDA(ctx, cudaEventRecord(plan->ev_in[slices], ctx->copy_in));
     }
-    // Both directions share the link's rate: what can go back while the weight gradient runs alone at the end does not
-    // compete with the uploads that it waits for.
-    const int last = slices - 1;
-    const double held = umma_wgrad_tail_us(plan->umma) * 50e3;  // bytes
     PhaseTimer untimed;
-    WgradPart part;
     slices = 0;
     for (int b0 = 0; b0 < G.B; b0 += per, ++slices) {
       const int nb = std::min(per, G.B - b0);
       CCT_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, plan->ev_in[slices], 0));
-      if (hdX) {
-        rc = umma_conv_dgrad(ctx, plan->umma, plan->sW, plan->sdY + b0 * iy, plan->sdX + b0 * ix, &untimed, nb, slices == 0);
-        if (rc != CCT_OK) return rc;
-        CCT_CUDA(ctx, cudaEventRecord(plan->ev_out[slices], ctx->stream));
-        if ((G.B - b0) * ix * 4.0 <= held) CCT_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_out, plan->ev_in[last], 0));
-        CCT_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_out, plan->ev_out[slices], 0));
-        CCT_CUDA(ctx, cudaMemcpyAsync(hdX + b0 * ix, plan->sdX + b0 * ix, nb * ix * 4, cudaMemcpyDeviceToHost, ctx->copy_out));
-      }
-      if (b0 + nb < G.B && b0 + nb + per >= G.B) {  // the weight gradient of all slices but the last, while that one arrives
-        rc = umma_conv_wgrad(ctx, plan->umma, plan->sX, plan->sdY, plan->sdW, plan->sdb, &untimed, &part, b0 + nb);
-        if (rc != CCT_OK) return rc;
-      }
+      if (!hdX) continue;
+      rc = umma_conv_dgrad(ctx, plan->umma, plan->sW, plan->sdY + b0 * iy, plan->sdX + b0 * ix, &untimed, nb, slices == 0);
+      if (rc != CCT_OK) return rc;
+      CCT_CUDA(ctx, cudaEventRecord(plan->ev_out[slices], ctx->stream));
+      CCT_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_out, plan->ev_out[slices], 0));
+      CCT_CUDA(ctx, cudaMemcpyAsync(hdX + b0 * ix, plan->sdX + b0 * ix, nb * ix * 4, cudaMemcpyDeviceToHost, ctx->copy_out));
     }
-    rc = umma_conv_wgrad(ctx, plan->umma, plan->sX, plan->sdY, plan->sdW, plan->sdb, &untimed, &part);
+    rc = umma_conv_wgrad(ctx, plan->umma, plan->sX, plan->sdY, plan->sdW, plan->sdb, &untimed);
     if (rc != CCT_OK) return rc;
     CCT_CUDA(ctx, cudaEventRecord(plan->ev_out[0], ctx->stream));
     CCT_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_out, plan->ev_out[0], 0));

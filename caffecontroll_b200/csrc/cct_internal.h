@@ -132,14 +132,7 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
                       int relu, PhaseTimer* t, int batch = 0, bool repack = true);
 int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dY, float* dX,
                        float* dW, float* db, PhaseTimer* t);
-// A weight gradient may be begun with the first `images` of the batch (their partial sums only; `part` says what is done, or
-// stays empty where the layer's kernel has no use for it) and is then completed by a call without `images`.
-struct WgradPart {
-  int kblocks = 0, splits = 0;
-};
-int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t,
-                    WgradPart* part = nullptr, int images = 0);
-double umma_wgrad_tail_us(const UmmaPlan* p);  // about what the completing call takes
+int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t);
 int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, float* dX, PhaseTimer* t, int batch,
                     bool repack);
 

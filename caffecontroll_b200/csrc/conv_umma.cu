@@ -1772,7 +1772,9 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
   UmmaPlan* p = new UmmaPlan();
   p->G = G;
   PlanMemory mem;
-  size_t sums = 0;  // floats of the split sums: one buffer for all passes, none needs its sums after its own reduction
+  // Floats of the split sums: one buffer for all passes.  A pass therefore ends with its own reduction - no entry point may
+  // leave sums there while another pass of the plan is launched.
+  size_t sums = 0;
   const int kk = G.k * G.k;
   // ---- forward: accumulator columns = output channels of a tile, reduction = (d, kr, kc)
   {
@@ -2141,18 +2143,10 @@ int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W
   return rc;
 }
 
-double umma_wgrad_tail_us(const UmmaPlan* p) {
-  const ConvGeom& G = p->G;
-  const double flops = 2.0 * G.B * G.m * G.m * G.o * G.Dg * G.k * G.k;
-  return p->wg_gather ? 30.0 + flops / 1.8e8 : 45.0;  // gathered: the whole batch at some 180 TFLOP/s, else the last part
-}
-
 // Weight + bias gradient over the whole batch.
-int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t,
-                    WgradPart* part, int images) {
+int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t) {
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   const ConvGeom& G = p->G;
-  if (images > 0 && (p->wg_gather || p->w_small || p->w_splits < 6)) return CCT_OK;
   if (p->wg_gather) {
     struct { int tiles, n, n_pad, k_real; } f = {p->wt_tiles, p->wt_n, p->w_npad, p->fwd.k_real};
     GatherProblem& w = p->wgp;
@@ -2199,19 +2193,6 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     const int vgroups = G.g * f.tiles;
     dim3 grid(p->w_mgroups, p->w_splits, vgroups);
     int rows_pad = p->w_mtiles * kTileM;
-    if (images > 0) {  // whole k-blocks of these images, over two thirds of the splits' room
-      P.kblocks_total = (int)((long long)images * P.mm / kBlockK);
-      P.kblocks_per_split = (P.kblocks_total + p->w_splits * 2 / 3 - 1) / (p->w_splits * 2 / 3);
-      if (P.kblocks_total == 0 || P.kblocks_per_split > kMaxChainKblocks) return CCT_OK;
-      grid.y = (P.kblocks_total + P.kblocks_per_split - 1) / P.kblocks_per_split;
-      *part = WgradPart{P.kblocks_total, (int)grid.y};
-    } else if (part && part->kblocks) {  // the rest, over the splits that are left
-      const int rest = P.kblocks_total - part->kblocks, room = p->w_splits - part->splits;
-      P.kb_first = part->kblocks;
-      P.kblocks_per_split = (rest + room - 1) / room;
-      grid.y = (rest + P.kblocks_per_split - 1) / P.kblocks_per_split;
-      P.partial += (size_t)part->splits * vgroups * rows_pad * P.n_pad;
-    }
     t->begin(1, ctx->stream);
     if (p->w_small) {
       P.n_pad = p->ws_cols * kSwTile;
@@ -2228,10 +2209,8 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       launch_pdl(wgrad_pick(p->w_subs, f.n_pad), dim3(grid), dim3(kWgThreads), p->w_smem, ctx->stream, P);
     t->end(1, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
-    if (images > 0) return CCT_OK;
     t->begin(2, ctx->stream);
-    const int splits = p->w_small ? p->w_splits : (int)grid.y + (part ? part->splits : 0);
-    launch_wgrad_reduce(ctx, p->w_partial, dW, G.bias ? db : nullptr, splits, vgroups, f.tiles, rows_pad, f.n, P.n_pad,
+    launch_wgrad_reduce(ctx, p->w_partial, dW, G.bias ? db : nullptr, p->w_splits, vgroups, f.tiles, rows_pad, f.n, P.n_pad,
                         f.k_real, G.og);
     t->end(2, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);

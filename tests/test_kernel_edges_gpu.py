@@ -174,24 +174,30 @@ def test_recorded_step_equals_the_bridges_one_by_one(ctx):
         assert np.array_equal(a, b)
 
 
-# Host-buffer calls that move the batch in slices: a last slice of one image, a weight gradient begun before it (both kernels
-# that can be), one that cannot be split so (512 lowered rows and more), without an input gradient.
-@pytest.mark.parametrize("shape", [(17, 3, 47, 24, 11, 4, 0, 1), (33, 6, 31, 40, 5, 1, 2, 1), (16, 64, 9, 48, 3, 1, 1, 1)])
+# Host-buffer calls that move the batch in slices: a last slice of one image, the kernels that the weight gradient can be, and
+# layers of few pixels and many filters, whose data gradient leaves split sums in the buffer that the weight gradient uses too.
+@pytest.mark.parametrize("shape", [(17, 3, 47, 24, 11, 4, 0, 1), (33, 6, 31, 40, 5, 1, 2, 1), (16, 64, 9, 48, 3, 1, 1, 1),
+                                   (16, 48, 14, 256, 3, 1, 1, 1), (32, 48, 14, 256, 3, 1, 1, 1), (16, 32, 13, 384, 3, 1, 1, 1),
+                                   (16, 16, 28, 192, 5, 1, 2, 1), (16, 16, 7, 64, 3, 1, 1, 1), (33, 1, 65, 136, 11, 4, 5, 1),
+                                   (19, 14, 16, 208, 5, 1, 0, 1)])
 @pytest.mark.parametrize("with_dx", [True, False])
-def test_sliced_host_calls(ctx, port, shape, with_dx):
+@pytest.mark.parametrize("algo", [capi.ALGO_AUTO, TENSOR])
+def test_sliced_host_calls(ctx, port, shape, with_dx, algo):
     B, D, n, o, k, s, p, g = shape
     X, W, b, dY = make_inputs(31, B, D, n, o, k, s, p, g)
     plan = C.c_void_p()
-    desc = capi.ConvDesc(B, D, n, o, k, s, p, g, 1, TENSOR)
+    desc = capi.ConvDesc(B, D, n, o, k, s, p, g, 1, algo)
     capi.check(ctx.lib.cct_conv_plan_create(ctx.h, C.byref(desc), C.byref(plan)), "plan", ctx.h)
-    Y, dX, dW, db = np.zeros_like(dY), np.zeros_like(X), np.zeros_like(W), np.zeros_like(b)
+    Y, dX, dW, db = (np.full_like(a, np.nan) for a in (dY, X, W, b))
     host = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
     capi.check(ctx.lib.cct_conv_forward_host(plan, host(X), host(W), host(b), host(Y), 0), "forward", ctx.h)
+    dXr, dWr, dbr = port.conv_backward(X, W, dY, k, s, p, g)
+    assert_close(Y, port.conv_forward(X, W, b, k, s, p, g).reshape(Y.shape), "Y")
     for _ in range(2):
+        for a in (dX, dW, db):
+            a.fill(np.nan)
         capi.check(ctx.lib.cct_conv_backward_host(plan, None, None, host(dY), host(dX) if with_dx else None, host(dW), host(db)),
                    "backward", ctx.h)
+        for a, r, name in [(dW, dWr, "dW"), (db, dbr, "db")] + ([(dX, dXr, "dX")] if with_dx else []):
+            assert_close(a, r.reshape(a.shape), name)
     ctx.lib.cct_conv_plan_destroy(plan)
-    dXr, dWr, dbr = port.conv_backward(X, W, dY, k, s, p, g)
-    pairs = [(Y, port.conv_forward(X, W, b, k, s, p, g), "Y"), (dW, dWr, "dW"), (db, dbr, "db")] + ([(dX, dXr, "dX")] if with_dx else [])
-    for a, r, name in pairs:
-        assert_close(a, r.reshape(a.shape), name)
