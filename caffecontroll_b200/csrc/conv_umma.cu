@@ -1432,7 +1432,7 @@ __global__ void bias_grad_kernel(const float* __restrict__ plane_sums, float* __
 }
 
 // ------------------------------------------------------------------------------------------ weight packing
-// A block writes one row of the packed operand (blockIdx.y = (vg, j)), four consecutive reduction indices per thread and
+// A block writes one row of the packed operand (blockIdx.x = (vg, j): there may be more than 65 535 of them), four consecutive reduction indices per thread and
 // step: one decode per four elements and 16-byte stores (a flat grid-stride loop spent most of its time dividing: CaffeNet
 // conv3's 0.9 M weights 8.0 / 11.6 us for the two operands, bound by neither memory nor launch).
 constexpr int kPackThreads = 128;
@@ -1451,12 +1451,12 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
                                                                 int n_real, int n_pad, int k_real, int k_pad, int run,
                                                                 int window) {
   pdl_wait();
-  const int vg = blockIdx.y / n_pad, j = blockIdx.y - vg * n_pad;
+  const int vg = blockIdx.x / n_pad, j = blockIdx.x - vg * n_pad;
   const int ch = (vg % tiles_per_group) * n_real + j;  // inside the group
   const bool live = j < n_real && ch < og;
   const float* src = W + (size_t)((vg / tiles_per_group) * og + ch) * k_real;
-  const size_t row = (size_t)blockIdx.y * k_pad;
-  for (int kk = (blockIdx.x * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.x * kPackThreads * 4) {
+  const size_t row = (size_t)blockIdx.x * k_pad;
+  for (int kk = (blockIdx.y * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.y * kPackThreads * 4) {
     float v[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -1477,13 +1477,13 @@ __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* _
                                                                   int Dg, int k, int s, int taps, int rows, int d_tile,
                                                                   int n_real, int n_pad, int k_real, int k_pad, int run) {
   pdl_wait();
-  const int vg = blockIdx.y / n_pad, j = blockIdx.y - vg * n_pad;
+  const int vg = blockIdx.x / n_pad, j = blockIdx.x - vg * n_pad;
   const int grp = vg / tiles_per_group, d = (vg - grp * tiles_per_group) * d_tile + j / (s * s * rows);
   const int py = (j / s) % (s * rows), px = j % s, window = taps * (taps + rows - 1);
   const bool live = j < n_real && d < Dg;
   const float* src = W + ((size_t)grp * og * Dg + d) * k * k;
-  const size_t row = (size_t)blockIdx.y * k_pad;
-  for (int kk = (blockIdx.x * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.x * kPackThreads * 4) {
+  const size_t row = (size_t)blockIdx.x * k_pad;
+  for (int kk = (blockIdx.y * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.y * kPackThreads * 4) {
     float v[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -1702,7 +1702,7 @@ void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* d
   }
 }
 
-dim3 pack_grid(int rows, int k_pad) { return dim3((k_pad / 4 + kPackThreads - 1) / kPackThreads, rows); }
+dim3 pack_grid(int rows, int k_pad) { return dim3(rows, (k_pad / 4 + kPackThreads - 1) / kPackThreads); }
 
 // Where the fp32 kernels of conv_small.cuh are the faster ones (measured, kernels alone, tensor cores -> fp32): forward of
 // 37 MFLOP (LeNet conv1, batch 64) 9.7 -> 5.0 us, 58 MFLOP (64 channels, 14 x 14, 3 x 3) 13.7 -> 6.8, 148 MFLOP 17 -> 12,
@@ -1715,6 +1715,7 @@ constexpr double kSmallConvFlops = 1.5e8, kSmallWideFlops = 8e7, kSmallWgradFlop
 int use_small_conv(int k, int s, long long out_pixels, int groups, int ci, int co) {
   const int ct = small_conv_ct(co);
   if (!small_conv_pick(k, s, ct) || small_conv_smem(k, ct, ci, 0) > 48 * 1024) return 0;
+  if ((long long)groups * ((co + 3) / 4) > 65535) return 0;  // channel tiles (of four at least) are a grid's y
   const double flops = 2.0 * out_pixels * groups * ((co + ct - 1) / ct * ct) * ci * k * k;
   return flops <= (k >= 7 ? kSmallWideFlops : kSmallConvFlops) ? ct : 0;
 }

@@ -38,6 +38,21 @@ def test_convolution_shapes(ctx, port, shape):
         assert_close(a, r.reshape(a.shape), name)
 
 
+@pytest.mark.parametrize("algo", [capi.ALGO_AUTO, TENSOR])
+def test_many_groups(ctx, port, algo):
+    """4096 groups of one channel are 65 536 rows of a packed operand; 65 600 groups (forward only) are more channel tiles than a
+    grid has in y."""
+    from caffecontroll_b200 import conv_layer
+    for B, g, n, backward in ((2, 4096, 5, True), (1, 65600, 3, False)):
+        X, W, b, dY = make_inputs(37, B, g, n, g, 3, 1, 1, g, bias=backward)  # (65 600 biases do not fit in shared memory)
+        Y, dX, dW, db, used = conv_layer(ctx, X, W, b, dY if backward else None, 3, 1, 1, g, algo=algo)
+        assert used == TENSOR
+        assert_close(Y, port.conv_forward(X, W, b if backward else np.zeros(g, np.float32), 3, 1, 1, g).reshape(Y.shape), "Y")
+        if backward:
+            for a, r, name in zip((dX, dW, db), port.conv_backward(X, W, dY, 3, 1, 1, g), ("dX", "dW", "db")):
+                assert_close(a, r.reshape(a.shape), name)
+
+
 # The tensor core truncates.  An instruction adds eight products to a sum: the sum loses half a place on average, each product,
 # aligned to it and cut two bits below its last place, an eighth - 1.5 places in all.  A place is 2^-23 .. 2^-24 of the sum
 # (0.72 * 2^-23 on average) and over positive data the sum grows steadily (half its final value on average), so N instructions
