@@ -615,6 +615,13 @@ bool fc_aligned(std::initializer_list<const void*> ptrs) {
   return true;
 }
 
+// Splits of fc_small_kernel for a pass of this plan.  A plan of the tensor-core kernel takes it where an operand is not on a
+// 16-byte boundary, which no tensor map can describe (and which the kernel's scalar loads do not mind); the room for split
+// sums is then what the other kernel's splits need.
+int fc_small_pass_splits(const cct_fc_plan* plan, int wanted, const FcShape& tensor) {
+  return plan->small ? wanted : std::min(wanted, tensor.P.splits);
+}
+
 int fc_reduce(cct_ctx* ctx, const FcReduceParams& R) {
   const bool vec = R.cols % 4 == 0 && fc_aligned({R.partial, R.out});
   const long long threads = (long long)R.rows * (vec ? R.cols / 4 : R.cols);
@@ -715,8 +722,8 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   const int B = plan->B, K = plan->K, O = plan->O, K4 = plan->K4, O4 = plan->O4;
   plan->timer.begin(0, ctx->stream);
-  if (plan->small) {
-    const int splits = plan->small_fwd;
+  if (plan->small || !(plan->Wp || fc_aligned({X, W}))) {
+    const int splits = fc_small_pass_splits(plan, plan->small_fwd, plan->fwd);
     const FcReduceParams post{plan->partial, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, splits, relu};
     FcSmallParams S{W, X, K, K, 0, 0, O, B, K, fc_round_up((K + splits - 1) / splits, 32), splits > 1 ? plan->partial : Y,
                     splits > 1 ? O4 : O, nullptr, post};
@@ -751,40 +758,41 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   const int B = plan->B, K = plan->K, O = plan->O, K4 = plan->K4, O4 = plan->O4;
+  const bool x_ok = plan->Xp || fc_aligned({X}), w_ok = plan->Wp || fc_aligned({W}), dy_ok = plan->dYp || fc_aligned({dY});
+  const bool w_small = plan->small || !(x_ok && dy_ok), d_small = plan->small || !(w_ok && dy_ok);
   const float *Xm = X, *dYm = dY;
+  int rc = CCT_OK;
   // ---- weight gradient: out = dW[o][k] (m = k, n = o), reduction over the batch; both operands MN-major
   plan->timer.begin(1, ctx->stream);
-  if (plan->small) {
+  if (plan->dYp && !(w_small && d_small)) { fc_pad(ctx, dY, plan->dYp, B, O, O4); dYm = plan->dYp; }
+  if (w_small) {
     FcSmallParams S{X, dY, K, O, 1, 1, K, O, B, B, dW, K, plan->bias ? db : nullptr, FcReduceParams{}};
     fc_small(ctx, S, 1);
-    plan->timer.end(1, ctx->stream);
-    CCT_CHECK_LAUNCH(ctx);
-    if (!dX) return CCT_OK;
+  } else {
+    if (plan->Xp) { fc_pad(ctx, X, plan->Xp, B, K, K4); Xm = plan->Xp; }
+    const bool direct = K4 != K || !fc_aligned({dW});  // an output no tensor map describes
+    rc = fc_operand_map(ctx, &plan->x_wgr, Xm, B, K, K4, 32, true);
+    if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_wgr, dYm, B, O, O4, 32, true);
+    if (rc == CCT_OK && !direct) rc = fc_output_map(ctx, &plan->out_wgr, dW, K, O, 1, K);
+    if (rc == CCT_OK)
+      rc = fc_launch(ctx, plan->wgr, plan->x_wgr, plan->dy_wgr, direct ? plan->x_wgr : plan->out_wgr, direct ? dW : nullptr, K);
+    if (rc != CCT_OK) return rc;
+    if (plan->bias) launch_pdl(fc_bias_grad_kernel, dim3((O + 31) / 32), dim3(256), 0, ctx->stream, dY, db, B, O);
+  }
+  plan->timer.end(1, ctx->stream);
+  CCT_CHECK_LAUNCH(ctx);
+  // ---- data gradient: out = dX[b][k] (m = k, n = b), reduction over o; A = W read MN-major, B = dY K-major
+  if (dX && d_small) {
     plan->timer.begin(3, ctx->stream);
-    const int splits = plan->small_dgr;
+    const int splits = fc_small_pass_splits(plan, plan->small_dgr, plan->dgr);
     const FcReduceParams post{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4, splits, 0};
     FcSmallParams D{W, dY, K, O, 1, 0, K, B, O, fc_round_up((O + splits - 1) / splits, 32), splits > 1 ? plan->partial : dX,
                     splits > 1 ? K4 : K, nullptr, post};
     fc_small(ctx, D, splits);
     CCT_CHECK_LAUNCH(ctx);
-    const int rc = splits > 1 ? fc_reduce(ctx, post) : CCT_OK;
+    rc = splits > 1 ? fc_reduce(ctx, post) : CCT_OK;
     plan->timer.end(3, ctx->stream);
-    return rc;
-  }
-  if (plan->Xp) { fc_pad(ctx, X, plan->Xp, B, K, K4); Xm = plan->Xp; }
-  if (plan->dYp) { fc_pad(ctx, dY, plan->dYp, B, O, O4); dYm = plan->dYp; }
-  const bool direct = K4 != K || !fc_aligned({dW});  // an output no tensor map describes
-  int rc = fc_operand_map(ctx, &plan->x_wgr, Xm, B, K, K4, 32, true);
-  if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_wgr, dYm, B, O, O4, 32, true);
-  if (rc == CCT_OK && !direct) rc = fc_output_map(ctx, &plan->out_wgr, dW, K, O, 1, K);
-  if (rc == CCT_OK)
-    rc = fc_launch(ctx, plan->wgr, plan->x_wgr, plan->dy_wgr, direct ? plan->x_wgr : plan->out_wgr, direct ? dW : nullptr, K);
-  if (rc != CCT_OK) return rc;
-  if (plan->bias) launch_pdl(fc_bias_grad_kernel, dim3((O + 31) / 32), dim3(256), 0, ctx->stream, dY, db, B, O);
-  plan->timer.end(1, ctx->stream);
-  CCT_CHECK_LAUNCH(ctx);
-  // ---- data gradient: out = dX[b][k] (m = k, n = b), reduction over o; A = W read MN-major, B = dY K-major
-  if (dX) {
+  } else if (dX) {
     plan->timer.begin(3, ctx->stream);
     if (plan->Wp) { fc_pad(ctx, W, plan->Wp, O, K, K4); W = plan->Wp; }
     rc = fc_operand_map(ctx, &plan->w_dgr, W, O, K, K4, 32, true);

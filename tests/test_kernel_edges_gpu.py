@@ -106,6 +106,34 @@ def test_inner_product_sizes(ctx, B, K, o):
     fc.close()
 
 
+# Operands four bytes off a 16-byte boundary, which no tensor map describes: all of them, or one at a time, with feature counts
+# that are and are not multiples of four, above the size of the fp32 kernel.  Tolerance as above.
+@pytest.mark.parametrize("B,K,o", [(129, 772, 1027), (129, 770, 1028), (130, 1024, 512), (40, 2051, 1030)])
+@pytest.mark.parametrize("shifted", ["X", "W", "dY", "X W dY dX dW Y"])
+def test_inner_product_alignment(ctx, B, K, o, shifted):
+    rng = np.random.default_rng(B + K + o)
+    sizes = {"X": (B, K), "W": (o, K), "b": (1, o), "dY": (B, o), "Y": (B, o), "dX": (B, K), "dW": (o, K), "db": (1, o)}
+    host, base, ptr = {}, {}, {}
+    for name, sh in sizes.items():
+        host[name] = rng.standard_normal(sh).astype(np.float32)
+        shift = 1 if name in shifted.split() else 0
+        base[name] = LogicalCube.from_numpy(ctx, np.concatenate([np.full(shift, 7, np.float32), host[name].ravel(), np.full(3, 7, np.float32)]))
+        ptr[name] = base[name].ptr + 4 * shift
+    plan = C.c_void_p()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(plan)), "plan", ctx.h)
+    capi.check(ctx.lib.cct_fc_forward(plan, ptr["X"], ptr["W"], ptr["b"], ptr["Y"], 0, None, 1.0), "forward", ctx.h)
+    capi.check(ctx.lib.cct_fc_backward(plan, ptr["X"], ptr["W"], ptr["dY"], ptr["dX"], ptr["dW"], ptr["db"], 0, None, 1.0),
+               "backward", ctx.h)
+    ctx.sync()
+    ctx.lib.cct_fc_plan_destroy(plan)
+    X, W, dY = (host[n].astype(np.float64) for n in ("X", "W", "dY"))
+    for name, r in (("Y", X @ W.T + host["b"]), ("dX", dY @ W), ("dW", dY.T @ X), ("db", dY.sum(0)[None])):
+        shift = 1 if name in shifted.split() else 0
+        got = base[name].download().ravel()
+        assert_close(got[shift:shift + r.size].reshape(r.shape), r.astype(np.float32), name)
+        assert np.all(got[:shift] == 7) and np.all(got[shift + r.size:] == 7)  # nothing beside the output
+
+
 def test_sgd_in_one_launch_equals_one_launch_per_tensor(ctx):
     """Bit for bit, over tails, chunks of one tensor that end inside a vector, and buffers off a 16-byte boundary."""
     rng = np.random.default_rng(5)
