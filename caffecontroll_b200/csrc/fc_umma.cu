@@ -349,9 +349,10 @@ __global__ void __launch_bounds__(256) fc_reduce_kernel(const __grid_constant__ 
   __shared__ float part[SLICES > 1 ? SLICES : 1][VEC][33];
   const int per_row = (P.cols + VEC - 1) / VEC;
   const int lane = threadIdx.x & 31, slice = SLICES > 1 ? threadIdx.x >> 5 : 0;
-  const int t = SLICES > 1 ? blockIdx.x * 32 + lane : blockIdx.x * 256 + threadIdx.x;
-  const bool in = t < P.rows * per_row;
-  const int row = in ? t / per_row : 0, col = in ? (t - row * per_row) * VEC : 0;
+  const long long t = SLICES > 1 ? blockIdx.x * 32ll + lane : blockIdx.x * 256ll + threadIdx.x;
+  const bool in = t < (long long)P.rows * per_row;
+  const int row = !in ? 0 : t <= 0x7fffffffll ? (int)t / per_row : (int)(t / per_row);
+  const int col = in ? (int)(t - (long long)row * per_row) * VEC : 0;
   const float* src = P.partial + (size_t)row * P.pitch + col;
   const size_t stride = (size_t)P.rows * P.pitch;
   float acc[VEC];
@@ -646,10 +647,6 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   if (!ctx || !out) return CCT_ERR_INVALID;
   *out = nullptr;
   if (batch <= 0 || in_features <= 0 || out_features <= 0) return CCT_ERR_INVALID;
-  if ((double)batch * std::max(in_features, out_features) > 2147483647.0 || (double)in_features * out_features > 4e9) {
-    ctx->last_error = "fully connected layer too large";
-    return CCT_ERR_UNSUPPORTED;
-  }
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   cct_fc_plan* p = new (std::nothrow) cct_fc_plan();
   if (!p) return CCT_ERR_NOMEM;

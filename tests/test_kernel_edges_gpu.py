@@ -134,6 +134,33 @@ def test_inner_product_alignment(ctx, B, K, o, shifted):
         assert np.all(got[:shift] == 7) and np.all(got[shift + r.size:] == 7)  # nothing beside the output
 
 
+# More than 2^31 elements in X and dX, more than 2^32 in W and dW.  Tolerance: parity (dW for the second only: its reduction over
+# the batch is one chain, whose truncation alone is 2e-3 after 270 000 images).
+@pytest.mark.parametrize("B,K,o", [(270000, 8192, 16), (4, 65536, 66000)])
+def test_inner_product_beyond_32_bits(ctx, B, K, o):
+    if torch.cuda.mem_get_info()[0] < 60 << 30:
+        pytest.skip("needs 60 GB")
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    make = lambda r, c: torch.empty(r * c, device="cuda").uniform_(-1, 1, generator=gen).view(r, c)  # noqa: E731
+    X, W, dY, b = make(B, K), make(o, K), make(B, o), make(1, o)
+    Y, dX, dW, db = torch.zeros_like(dY), torch.zeros_like(X), torch.zeros_like(W), torch.zeros_like(b)
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(plan)), "plan", ctx.h)
+    capi.check(ctx.lib.cct_fc_forward(plan, q(X), q(W), q(b), q(Y), 0, None, 1.0), "forward", ctx.h)
+    capi.check(ctx.lib.cct_fc_backward(plan, q(X), q(W), q(dY), q(dX), q(dW), q(db), 0, None, 1.0), "backward", ctx.h)
+    ctx.sync()
+    ctx.lib.cct_fc_plan_destroy(plan)
+    rows, outs = sorted({0, 1, B // 2, B - 1}), sorted({0, 1, o // 2, o - 1})  # 64-bit products of some rows, the last among them
+    Xd, Wd, dYd = X[rows].double(), W[outs].double(), dY[rows].double()
+    checks = [(Y[rows][:, outs], Xd @ Wd.T + b[0, outs].double(), "Y"),
+              (dX[rows], sum(dYd[:, j:j + 4096] @ W[j:j + 4096].double() for j in range(0, o, 4096)), "dX")]
+    if B < 1000:
+        checks.append((dW[outs], dY[:, outs].double().T @ X.double(), "dW"))
+    for got, ref, name in checks:
+        assert_close(got.cpu().numpy(), ref.float().cpu().numpy(), name)
+
+
 def test_sgd_in_one_launch_equals_one_launch_per_tensor(ctx):
     """Bit for bit, over tails, chunks of one tensor that end inside a vector, and buffers off a 16-byte boundary."""
     rng = np.random.default_rng(5)
