@@ -485,16 +485,24 @@ class ParallelizedBridge:
 
 
 class NetworkUpdate:
-    """apply_update() of all layers of a network as one launch, where their updaters allow it (device memory, no L1 decay)."""
+    """apply_update() of all layers of a network as one launch, where their updaters are the library's own (device memory, no L1
+    decay, neither apply_update() nor the step replaced)."""
 
     def __init__(self):
         self.key, self.items, self.n = None, None, 0
+
+    @staticmethod
+    def _plain(pb):
+        ops = pb.ops
+        return (type(pb).apply_update is ParallelizedBridge.apply_update and "apply_update" not in pb.__dict__ and
+                isinstance(ops, DeviceOps) and type(ops).sgd_step is DeviceOps.sgd_step and "sgd_step" not in ops.__dict__ and
+                pb.solver.regularization_type != "L1")
 
     def apply(self, pbridges):
         active = [pb for pb in pbridges if pb.update_model_gradients]
         if not active:
             return
-        if any(not isinstance(pb.ops, DeviceOps) or pb.solver.regularization_type == "L1" for pb in active):
+        if not all(self._plain(pb) and pb.ops.ctx is active[0].ops.ctx for pb in active):
             for pb in active:
                 pb.apply_update()
             return
@@ -507,9 +515,11 @@ class NetworkUpdate:
             if base is None:
                 base = bases[which] = get_learning_rate(s.lr_policy, s.base_lr, s.gamma, float(pb.current_iter), float(s.stepsize),
                                                         s.power, float(s.max_iter))
-            key.append((pb.params, base, pb.lr_mult, pb.decay_mult, s.momentum, s.weight_decay, s.regularization_type))
+            # everything update_tensors() reads, by value
+            key.append((pb.n_w, pb.n_b, pb.params, pb.grads, pb.hist, base, *pb.lr_mult, *pb.decay_mult, s.momentum, s.weight_decay,
+                        s.regularization_type))
         if key != self.key:
-            tensors = [t for pb, k in zip(active, key) for t in pb.update_tensors(k[1])]
+            tensors = [t for pb, k in zip(active, key) for t in pb.update_tensors(k[5])]
             self.items, self.n, self.key = (capi.SgdItem * len(tensors))(*[capi.SgdItem(*t) for t in tensors]), len(tensors), key
         active[0].ops.sgd_steps(self.items, self.n)
 

@@ -183,3 +183,67 @@ def test_against_reference_parallelized_bridge_with_two_partitions(port, referen
     mine = ops.view(pb.params, pb.count)
     assert maxnorm_rel(mine[:W.size], Wref.ravel()) <= 1e-5
     assert maxnorm_rel(mine[W.size:], bref) <= 1e-5
+
+
+def test_network_update_follows_its_updaters():
+    """One launch for all layers reads what each layer's apply_update() would read at that moment - buffers and multipliers that
+    were replaced or changed in place among them - and is not taken where an updater or its step has been replaced."""
+    from types import SimpleNamespace
+    from caffecontroll_b200.parallel import DeviceOps, NetworkUpdate
+
+    class Ops(DeviceOps):
+        def __init__(self):
+            super().__init__(ctx="device 0")
+            self.next, self.launches = 1000, []
+
+        def alloc(self, count):
+            self.next += 4 * count
+            return self.next
+
+        def zero(self, ptr, count):
+            pass
+
+        def copy(self, dst, src, count):
+            pass
+
+        def sgd_steps(self, items, n):
+            self.launches.append([(t.count, t.w, t.g, t.h, t.lr, t.momentum, t.lam) for t in items[:n]])
+
+    cube = lambda n: SimpleNamespace(n_elements=n, ptr=0, own_data=False, free=lambda: None)  # noqa: E731
+    bridge = lambda n: SimpleNamespace(p_model_cube=cube(n), p_bias_cube=cube(2), p_model_gradient_cube=cube(n),  # noqa: E731
+                                       p_bias_gradient_cube=cube(2), bias_term=True)
+    f32 = lambda v: float(np.float32(v))  # noqa: E731
+    ops, solver = Ops(), SolverParameter(base_lr=0.5, lr_policy="fixed", momentum=0.25, weight_decay=0.125)
+    pbs = [ParallelizedBridge(bridge(n), solver, ops, [1.0, 2.0], [1.0, 0.0], defer_update=True) for n in (7, 5)]
+    expected = lambda: [t for pb in pbs for t in (  # noqa: E731
+        (pb.n_w, pb.params, pb.grads, pb.hist, f32(0.5 * pb.lr_mult[0]), f32(solver.momentum), f32(solver.weight_decay * pb.decay_mult[0])),
+        (2, pb.params + 4 * pb.n_w, pb.grads + 4 * pb.n_w, pb.hist + 4 * pb.n_w, f32(0.5 * pb.lr_mult[1]), f32(solver.momentum),
+         f32(solver.weight_decay * pb.decay_mult[1])))]
+    update = NetworkUpdate()
+
+    def change(what):
+        if what == "gradients":
+            pbs[0].grads += 400
+        elif what == "history":
+            pbs[1].hist += 800
+        elif what == "rate of a layer":
+            pbs[0].lr_mult[0] = 0.0
+        elif what == "decay of a layer":
+            pbs[1].decay_mult[1] = 3.0
+        elif what == "momentum":
+            solver.momentum = 0.75
+
+    for what in ("nothing", "gradients", "history", "rate of a layer", "decay of a layer", "momentum"):
+        change(what)
+        update.apply(pbs)
+        assert ops.launches.pop() == expected() and not ops.launches, what
+    assert [pb.current_iter for pb in pbs] == [6, 6]
+
+    calls = []
+    pbs[1].apply_update = lambda: calls.append("replaced")
+    ops.sgd_step = lambda *a: calls.append(a[0])
+    update.apply(pbs)
+    assert calls == [7, 2, "replaced"] and not ops.launches
+    del pbs[1].apply_update
+    update.apply(pbs)  # the step is still replaced
+    assert calls[3:] == [7, 2, 5, 2] and not ops.launches
