@@ -138,7 +138,7 @@ static int ctx_create_common(int device_id, cudaStream_t stream, bool make_strea
   if (e == cudaSuccess) {
     ctx->sm_count = prop.multiProcessorCount;
     if (make_stream) {
-      e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
+      e = cudaStreamCreateWithFlags(&ctx->stream.own, cudaStreamNonBlocking);
       ctx->owns_stream = true;
     } else {
       ctx->stream = stream;
@@ -177,7 +177,6 @@ int cct_ctx_destroy(cct_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   if (ctx->copy_in) cudaStreamDestroy(ctx->copy_in);
   if (ctx->copy_out) cudaStreamDestroy(ctx->copy_out);
-  if (ctx->capture_stream) cudaStreamDestroy(ctx->capture_stream);
   if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
   if (ctx->status_host) cudaFreeHost((void*)ctx->status_host);
   cudaFree(ctx->ticket);
@@ -413,39 +412,38 @@ struct cct_program {
   // microseconds per kernel (LeNet's iteration: 30 kernels, 127 us with 100 us of work in them), the graph about ten in all.
   int runs = 0;
   cudaGraphExec_t graph = nullptr;
-  uint64_t graph_kernels = 0;
+  uint64_t graph_kernels = 0, graph_launches = 0;
   bool no_graph = false;  // capturing failed once: call by call for good
 };
 
 namespace {
 
-// Captures the program's calls into a graph.  False (and no graph) if that does not work; errors are cleared.
+// Captures the program's calls into a graph, on a stream of its own (the context's may be the legacy one, and other threads
+// may be using it).  False (and no graph) if that does not work; errors are cleared.
 bool capture_program(cct_program* p) {
-  cct_ctx* ctx = p->ctx;
-  if (!ctx->capture_stream && cudaStreamCreateWithFlags(&ctx->capture_stream, cudaStreamNonBlocking) != cudaSuccess) {
+  cudaStream_t stream = nullptr;
+  if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  if (cudaStreamBeginCapture(ctx->capture_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
+  bool ok = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+  if (ok) {
+    const uint64_t counted = thread_launches;
+    capture_here = stream;
+    for (const auto& call : p->calls) ok = ok && call() == CCT_OK;
+    capture_here = nullptr;
+    p->graph_kernels = thread_launches - counted;  // captured, not launched
+    kernel_launches -= p->graph_kernels;
+    cudaGraph_t graph = nullptr;
+    ok = cudaStreamEndCapture(stream, &graph) == cudaSuccess && graph && ok;
+    if (ok) ok = cudaGraphInstantiate(&p->graph, graph, 0) == cudaSuccess;
+    if (graph) cudaGraphDestroy(graph);
   }
-  const cudaStream_t own = ctx->stream;
-  ctx->stream = ctx->capture_stream;
-  bool ok = true;
-  const uint64_t counted = thread_launches;
-  for (const auto& call : p->calls) ok = ok && call() == CCT_OK;
-  p->graph_kernels = thread_launches - counted;  // captured, not launched
-  kernel_launches -= p->graph_kernels;
-  ctx->stream = own;
-  cudaGraph_t graph = nullptr;
-  ok = cudaStreamEndCapture(ctx->capture_stream, &graph) == cudaSuccess && graph && ok;
-  if (ok) ok = cudaGraphInstantiate(&p->graph, graph, 0) == cudaSuccess;
-  if (graph) cudaGraphDestroy(graph);
   if (!ok) {
     cudaGetLastError();
     p->graph = nullptr;
   }
+  cudaStreamDestroy(stream);
   return ok;
 }
 
@@ -454,26 +452,26 @@ bool capture_program(cct_program* p) {
 int cct_program_begin(cct_ctx* ctx, cct_program** out) {
   if (!ctx || !out) return CCT_ERR_INVALID;
   *out = nullptr;
-  if (ctx->recording) {
-    ctx->last_error = "a program is already being recorded on this context";
+  if (recording_here.calls) {
+    ctx->last_error = "this thread is already recording a program";
     return CCT_ERR_INVALID;
   }
   cct_program* p = new (std::nothrow) cct_program();
   if (!p) return CCT_ERR_NOMEM;
   p->ctx = ctx;
-  ctx->recording = &p->calls;
+  recording_here = Recording{ctx, &p->calls};
   *out = p;
   return CCT_OK;
 }
 
 int cct_program_end(cct_program* program) {
-  if (!program || program->ctx->recording != &program->calls) return CCT_ERR_INVALID;
-  program->ctx->recording = nullptr;
+  if (!program || recording_here.calls != &program->calls) return CCT_ERR_INVALID;
+  recording_here = Recording{};
   return CCT_OK;
 }
 
 int cct_program_run(cct_program* program) {
-  if (!program || program->ctx->recording) return CCT_ERR_INVALID;
+  if (!program || recording_here.ctx == program->ctx) return CCT_ERR_INVALID;
   cct_ctx* ctx = program->ctx;
   if (program->runs++ && !program->no_graph && ctx->timed_plans == 0) {
     if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
@@ -486,6 +484,7 @@ int cct_program_run(cct_program* program) {
     if (free_stream && program->graph) {
       CCT_CUDA(ctx, cudaGraphLaunch(program->graph, ctx->stream));
       kernel_launches += program->graph_kernels;
+      ++program->graph_launches;
       return CCT_OK;
     }
   }
@@ -493,6 +492,12 @@ int cct_program_run(cct_program* program) {
     const int rc = call();
     if (rc != CCT_OK) return rc;
   }
+  return CCT_OK;
+}
+
+int cct_program_graph_launches(const cct_program* program, unsigned long long* count) {
+  if (!program || !count) return CCT_ERR_INVALID;
+  *count = program->graph_launches;
   return CCT_OK;
 }
 
@@ -504,7 +509,7 @@ int cct_kernel_launches(unsigned long long* count) {
 
 int cct_program_destroy(cct_program* program) {
   if (!program) return CCT_ERR_INVALID;
-  if (program->ctx->recording == &program->calls) program->ctx->recording = nullptr;
+  if (recording_here.calls == &program->calls) recording_here = Recording{};
   if (program->graph) {
     cudaSetDevice(program->ctx->device);
     cudaGraphExecDestroy(program->graph);
@@ -537,7 +542,7 @@ int cct_conv_backward(cct_conv_plan* plan, const float* X, const float* W, const
 
 int cct_conv_backward_fused(cct_conv_plan* plan, const float* X, const float* W, const float* dY,
                             const cct_bwd_fusion* f, float* dX, float* dW, float* db) {
-  if (plan && f && plan->ctx->recording) {
+  if (plan && f && recording_here.ctx == plan->ctx) {
     const cct_bwd_fusion kept = *f;
     CCT_RECORD(plan->ctx, cct_conv_backward_fused(plan, X, W, dY, &kept, dX, dW, db))
   }

@@ -10,9 +10,27 @@
 
 #include "../../include/cct_b200.h"
 
+struct cct_ctx;
+
+// What a program (cct_program_begin) does with a context's calls concerns the thread that does it alone; other threads' calls
+// on the same context are carried out on the context's stream meanwhile.
+struct Recording {  // between cct_program_begin and _end: this thread's bridge calls on `ctx` are kept in `calls`
+  cct_ctx* ctx = nullptr;
+  std::vector<std::function<int()>>* calls = nullptr;
+};
+inline thread_local Recording recording_here;
+inline thread_local cudaStream_t capture_here = nullptr;  // set while this thread captures a program: its launches go there
+
+// The stream a context's work is enqueued on, as seen from this thread.
+struct CtxStream {
+  cudaStream_t own = nullptr;
+  CtxStream& operator=(cudaStream_t s) { own = s; return *this; }
+  operator cudaStream_t() const { return capture_here ? capture_here : own; }
+};
+
 struct cct_ctx {
   int device = 0;
-  cudaStream_t stream = nullptr;
+  CtxStream stream;
   bool owns_stream = false;
   // Side streams of the host-buffer entry points: uploads and downloads overlap each other and the kernels.
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
@@ -32,18 +50,18 @@ struct cct_ctx {
   int* status_dev = nullptr;
   unsigned* ticket = nullptr;  // device word, zero between kernels: which block of a kernel is the last to finish
   std::string last_error;
-  // While a program is being recorded (cct_program_begin .. _end) the bridge calls on this context are kept here instead of
-  // being carried out.
-  std::vector<std::function<int()>>* recording = nullptr;
-  int timed_plans = 0;                    // plans whose kernel timing is switched on: programs then run call by call
-  cudaStream_t capture_stream = nullptr;  // programs are captured here (the context's own stream may be the legacy one)
+  int timed_plans = 0;  // plans whose kernel timing is switched on: programs then run call by call
 };
 
 // First line of every recordable entry point: `call` is the entry point with its own arguments.
-#define CCT_RECORD(ctx, call)                                         \
-  if ((ctx) && (ctx)->recording) {                                    \
-    (ctx)->recording->push_back([=]() -> int { return call; });       \
-    return CCT_OK;                                                    \
+#define CCT_RECORD(context, call)                                               \
+  if ((context) && recording_here.ctx == (context)) {                           \
+    try {                                                                       \
+      recording_here.calls->push_back([=]() -> int { return call; });           \
+    } catch (...) {                                                             \
+      return CCT_ERR_NOMEM;                                                     \
+    }                                                                           \
+    return CCT_OK;                                                              \
   }
 
 #define CCT_CUDA(ctx, call)                                                                   \

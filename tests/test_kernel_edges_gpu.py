@@ -244,6 +244,50 @@ def test_recorded_step_equals_the_bridges_one_by_one(ctx):
         assert np.array_equal(a, b)
 
 
+def test_recording_is_one_threads_own(ctx):
+    """While a thread records, another thread's calls on the same context are carried out, and it may record itself."""
+    import threading
+    from caffecontroll_b200.layers import ReLUBridge
+    x = np.linspace(-1, 1, 64, dtype=np.float32).reshape(2, 2, 4, 4)
+    mk = lambda v: Layer(LogicalCube.from_numpy(ctx, v), LogicalCube.from_numpy(ctx, 0 * v))  # noqa: E731
+    mine, theirs = [(mk(x), mk(7 + 0 * x)) for _ in range(2)]
+    relu, other = ReLUBridge(*mine, ctx), ReLUBridge(*theirs, ctx)
+    program, failures = C.c_void_p(), []
+
+    def beside():
+        try:
+            own = C.c_void_p()
+            other.forward()
+            capi.check(ctx.lib.cct_program_begin(ctx.h, C.byref(own)), "begin", ctx.h)
+            other.backward()
+            capi.check(ctx.lib.cct_program_end(own), "end", ctx.h)
+            ctx.lib.cct_program_destroy(own)
+        except Exception as e:
+            failures.append(e)
+
+    capi.check(ctx.lib.cct_program_begin(ctx.h, C.byref(program)), "begin", ctx.h)
+    relu.forward()
+    t = threading.Thread(target=beside)
+    t.start()
+    t.join()
+    capi.check(ctx.lib.cct_program_end(program), "end", ctx.h)
+    ctx.sync()
+    assert not failures
+    assert np.array_equal(theirs[1].p_data_cube.download(), np.maximum(x, 0))
+    assert np.all(mine[1].p_data_cube.download() == 7)  # recorded, not carried out
+    launches = C.c_ulonglong()
+    for run in range(3):
+        theirs[1].p_data_cube.upload(7 + 0 * x)
+        mine[1].p_data_cube.upload(7 + 0 * x)
+        capi.check(ctx.lib.cct_program_run(program), "run", ctx.h)
+        ctx.sync()
+        assert np.array_equal(mine[1].p_data_cube.download(), np.maximum(x, 0))
+        assert np.all(theirs[1].p_data_cube.download() == 7)  # the other thread's call is no part of it
+        capi.check(ctx.lib.cct_program_graph_launches(program, C.byref(launches)), "graph launches", ctx.h)
+        assert launches.value == run  # the first run call by call
+    ctx.lib.cct_program_destroy(program)
+
+
 # Host-buffer calls that move the batch in slices: a last slice of one image, the kernels that the weight gradient can be, and
 # layers of few pixels and many filters, whose data gradient leaves split sums in the buffer that the weight gradient uses too.
 @pytest.mark.parametrize("shape", [(17, 3, 47, 24, 11, 4, 0, 1), (33, 6, 31, 40, 5, 1, 2, 1), (16, 64, 9, 48, 3, 1, 1, 1),
