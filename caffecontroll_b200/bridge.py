@@ -59,18 +59,56 @@ class Context:
         capi.check(self.lib.cct_fill_f32(self.h, C.c_void_p(ptr), count, value), "cct_fill_f32", self.h)
 
 
-class Tracked:
-    """An object whose attributes decide which calls a pass over a network makes (cubes, layers, bridges).  Every assignment
-    raises Tracked.changes, so that a network that has recorded its calls knows when they may no longer be the same.
-    `_untracked` names the attributes that change from pass to pass without changing the calls."""
+class Watch:
+    """What happened to the objects a network watches: `changed` - an attribute has another value; `rewired` - one names another
+    object, so that the network has to look again at what it consists of."""
 
-    changes = 0
+    __slots__ = ("changed", "rewired")
+
+    def __init__(self):
+        self.changed = self.rewired = False
+
+
+class Tracked:
+    """An object whose attributes decide which calls a pass over a network makes (cubes, layers, bridges, updaters).  A network
+    that keeps its calls watches the objects they come from; an attribute that gets another value tells it.  `_untracked` names
+    the attributes that change from pass to pass without changing the calls."""
+
     _untracked = ()
 
     def __setattr__(self, name, value):
+        d = self.__dict__
+        old = d.get(name, Tracked)
         object.__setattr__(self, name, value)
-        if name not in self._untracked:
-            Tracked.changes += 1
+        if "_watches" not in d or name in self._untracked or old is value:
+            return
+        t = type(value)
+        if t is type(old) and (old == value if t in (int, bool, str) else t is float and old.hex() == value.hex()):
+            return
+        for w in d["_watches"]:
+            w.changed = True
+            w.rewired |= t not in (int, bool, str, float)
+
+    def __delattr__(self, name):
+        object.__delattr__(self, name)
+        for w in self.__dict__.get("_watches", ()):
+            w.changed = w.rewired = True
+
+
+def watch(roots, w):
+    """Lets `w` know of changes to every tracked object that can be reached from `roots`."""
+    seen, todo = set(), list(roots)
+    while todo:
+        o = todo.pop()
+        if isinstance(o, (list, tuple)):
+            todo.extend(o)
+        elif isinstance(o, Tracked) and id(o) not in seen:
+            seen.add(id(o))
+            watches = o.__dict__.get("_watches", ())
+            if w not in watches:
+                o.__dict__["_watches"] = (*watches, w)
+            if not isinstance(o, LogicalCube):  # a cube refers to no other object
+                todo.extend([v for v in o.__dict__.values() if isinstance(v, (Tracked, list, tuple))])
 
 
 class LogicalCube(Tracked):

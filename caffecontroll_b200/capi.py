@@ -26,7 +26,7 @@ EXPORTS = [
     "cct_conv_plan_reserve_fusion", "cct_selftest_bounded_wait", "cct_conv_forward_host", "cct_conv_backward_host", "cct_conv_weight_grad_noalloc",
     "cct_maxpool_forward", "cct_maxpool_backward", "cct_relu_forward", "cct_relu_backward",
     "cct_pool_relu_backward", "cct_sgd_step", "cct_sgd_step_multi",
-    "cct_program_begin", "cct_program_end", "cct_program_run", "cct_program_graph_launches", "cct_program_destroy", "cct_kernel_launches", "cct_saxpby", "cct_l1_update",
+    "cct_program_begin", "cct_program_begin_live", "cct_program_end", "cct_program_run", "cct_program_graph_launches", "cct_program_destroy", "cct_kernel_launches", "cct_saxpby", "cct_l1_update",
     "cct_fc_plan_create", "cct_fc_plan_destroy", "cct_fc_plan_workspace_bytes", "cct_fc_forward", "cct_fc_backward",
     "cct_fc_plan_enable_timing", "cct_fc_plan_last_timings",
     "cct_comm_unique_id", "cct_comm_init_rank", "cct_comm_destroy", "cct_comm_size", "cct_allreduce_sum_begin",
@@ -112,6 +112,7 @@ def load():
         "cct_sgd_step": [_vp, sz, _vp, _vp, _vp, f, f, f],
         "cct_sgd_step_multi": [_vp, i, C.POINTER(SgdItem)],
         "cct_program_begin": [_vp, C.POINTER(_vp)],
+        "cct_program_begin_live": [_vp, C.POINTER(_vp)],
         "cct_program_end": [_vp],
         "cct_program_run": [_vp],
         "cct_program_graph_launches": [_vp, C.POINTER(C.c_ulonglong)],

@@ -177,6 +177,7 @@ int cct_ctx_destroy(cct_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   if (ctx->copy_in) cudaStreamDestroy(ctx->copy_in);
   if (ctx->copy_out) cudaStreamDestroy(ctx->copy_out);
+  if (cudaStream_t spare = ctx->spare_stream.load()) cudaStreamDestroy(spare);
   if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
   if (ctx->status_host) cudaFreeHost((void*)ctx->status_host);
   cudaFree(ctx->ticket);
@@ -421,8 +422,8 @@ namespace {
 // Captures the program's calls into a graph, on a stream of its own (the context's may be the legacy one, and other threads
 // may be using it).  False (and no graph) if that does not work; errors are cleared.
 bool capture_program(cct_program* p) {
-  cudaStream_t stream = nullptr;
-  if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) {
+  cudaStream_t stream = p->ctx->spare_stream.exchange(nullptr);
+  if (!stream && cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -443,13 +444,12 @@ bool capture_program(cct_program* p) {
     cudaGetLastError();
     p->graph = nullptr;
   }
-  cudaStreamDestroy(stream);
+  stream = p->ctx->spare_stream.exchange(stream);  // kept for the next capture (creating one takes as long as a small graph)
+  if (stream) cudaStreamDestroy(stream);
   return ok;
 }
 
-}  // namespace
-
-int cct_program_begin(cct_ctx* ctx, cct_program** out) {
+int begin_program(cct_ctx* ctx, bool live, cct_program** out) {
   if (!ctx || !out) return CCT_ERR_INVALID;
   *out = nullptr;
   if (recording_here.calls) {
@@ -459,10 +459,16 @@ int cct_program_begin(cct_ctx* ctx, cct_program** out) {
   cct_program* p = new (std::nothrow) cct_program();
   if (!p) return CCT_ERR_NOMEM;
   p->ctx = ctx;
-  recording_here = Recording{ctx, &p->calls};
+  p->runs = live;
+  recording_here = Recording{ctx, &p->calls, live};
   *out = p;
   return CCT_OK;
 }
+
+}  // namespace
+
+int cct_program_begin(cct_ctx* ctx, cct_program** out) { return begin_program(ctx, false, out); }
+int cct_program_begin_live(cct_ctx* ctx, cct_program** out) { return begin_program(ctx, true, out); }
 
 int cct_program_end(cct_program* program) {
   if (!program || recording_here.calls != &program->calls) return CCT_ERR_INVALID;

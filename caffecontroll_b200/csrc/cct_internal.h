@@ -17,6 +17,7 @@ struct cct_ctx;
 struct Recording {  // between cct_program_begin and _end: this thread's bridge calls on `ctx` are kept in `calls`
   cct_ctx* ctx = nullptr;
   std::vector<std::function<int()>>* calls = nullptr;
+  bool live = false;  // and carried out as well
 };
 inline thread_local Recording recording_here;
 inline thread_local cudaStream_t capture_here = nullptr;  // set while this thread captures a program: its launches go there
@@ -50,18 +51,31 @@ struct cct_ctx {
   int* status_dev = nullptr;
   unsigned* ticket = nullptr;  // device word, zero between kernels: which block of a kernel is the last to finish
   std::string last_error;
+  std::atomic<cudaStream_t> spare_stream{nullptr};  // for the next capture of a program
   int timed_plans = 0;  // plans whose kernel timing is switched on: programs then run call by call
 };
 
 // First line of every recordable entry point: `call` is the entry point with its own arguments.
-#define CCT_RECORD(context, call)                                               \
-  if ((context) && recording_here.ctx == (context)) {                           \
-    try {                                                                       \
-      recording_here.calls->push_back([=]() -> int { return call; });           \
-    } catch (...) {                                                             \
-      return CCT_ERR_NOMEM;                                                     \
-    }                                                                           \
-    return CCT_OK;                                                              \
+inline int record_call(std::function<int()> call) {
+  const Recording here = recording_here;
+  try {
+    here.calls->push_back(call);
+  } catch (...) {
+    return CCT_ERR_NOMEM;
+  }
+  if (!here.live) return CCT_OK;
+  recording_here = Recording{};  // an entry point may use others
+  const int rc = call();
+  recording_here = here;
+  return rc;
+}
+#define CCT_RECORD(context, call)                                                    \
+  if ((context) && recording_here.ctx == (context)) {                                \
+    try {                                                                            \
+      return record_call([=]() -> int { return call; });                             \
+    } catch (...) {                                                                  \
+      return CCT_ERR_NOMEM;                                                          \
+    }                                                                                \
   }
 
 #define CCT_CUDA(ctx, call)                                                                   \

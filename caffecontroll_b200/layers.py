@@ -115,7 +115,7 @@ class DropoutBridge(_Bridge):
     input * mask * 1 / (1 - ratio), the same product on the gradient.  The mask is drawn on the device from
     (random_seed, pass counter); set_mask() injects a given one (parity runs use the CPU oracle's)."""
 
-    _untracked = ("calls", "mask_held")
+    _untracked = ("calls",)
 
     def __init__(self, p_input_layer, p_output_layer, dropout_ratio=0.5, random_seed=1, ctx=None):
         super().__init__(p_input_layer, p_output_layer, ctx)
@@ -125,14 +125,13 @@ class DropoutBridge(_Bridge):
         self.mask_cube = LogicalCube(self.ctx, self.iR, self.iC, self.iD, self.iB, np.uint32)
         self.calls = 0
         self.injected = False
-        self.mask_held = False  # the owner draws the mask itself (a network that replays its recorded calls)
 
     def set_mask(self, mask):
         self.mask_cube.upload(np.ascontiguousarray(mask, dtype=np.uint32))
         self.injected = True
 
     def draw_mask(self):
-        if self.injected or self.mask_held:
+        if self.injected:
             return
         self.calls += 1
         capi.check(self.lib.cct_dropout_mask(self.ctx.h, self.mask_cube.ptr, self.mask_cube.n_elements,

@@ -13,7 +13,7 @@ import re
 import numpy as np
 
 from . import capi
-from .bridge import ConvolutionBridge, FullyConnectedBridge, Layer, LogicalCube, Tracked
+from .bridge import ConvolutionBridge, FullyConnectedBridge, Layer, LogicalCube, Watch, watch
 from .layers import DropoutBridge, LRNBridge, MaxPoolingBridge, ReLUBridge, SoftmaxLossBridge
 from .parallel import (DeviceOps, ModelParallelFullyConnectedBridge, ModelParallelizedBridge, NetworkUpdate,
                        ParallelizedBridge, SolverParameter, model_parallel_gpus)
@@ -301,10 +301,12 @@ class Net:
         self.input = next(iter(self.blobs.values()))
         self.fused = []
         self._update = NetworkUpdate()
-        self._program, self._recorded = None, None
+        self._program, self._recorded, self._watch = None, None, Watch()
+        self._walks, self._patience, self._runs = 1, 1, 0
         self._step_launches = 0
         if fuse:
             self._fuse()
+        self._look_again()
 
     # ---- construction helpers
     def _layer(self, R, Cc, D, with_grad=True):
@@ -365,7 +367,7 @@ class Net:
                 drop.skip_forward = drop.skip_backward = True
                 # the mask must exist before the layer that applies it runs: draw it in the producer's slot
                 self.bridges[i] = _WithPrologue(br, drop.draw_mask)
-                drop.draw_mask = lambda: None
+                drop.draw_mask = _drawn_by_the_producer
                 self.fused.append("%s+%s+%s, masks in %s" % (self.names[i], self.names[r], self.names[nxt],
                                                              self.names[consumer_of(nxt)]))
 
@@ -421,45 +423,72 @@ class Net:
             h.begin_allreduce()
         self.ops.allreduce_wait()
 
-    # The host side of an iteration is a few Python calls per bridge, several times what a small layer's kernels take.  The
-    # bridges make the same library calls on the same buffers every time, so step() records them once and has the library
-    # repeat them; the dropout masks (a new counter every pass) and the update (a rate that may change) stay outside.
+    # The host side of an iteration is a few Python calls per bridge, several times what a small layer's kernels take.  Where the
+    # bridges make the same library calls on the same buffers every time, step() records them once and has the library repeat
+    # them; the dropout masks (a new counter every pass) and the update (a rate that may change) stay outside.  A recording lasts
+    # until one of the network's objects changes.  The first step walks, and a network that keeps changing (a loader that
+    # alternates between input buffers) walks nearly always: each recording that did not last doubles the number of steps, up
+    # to 64, before the next is made.
     _RECORDABLE = (ConvolutionBridge, FullyConnectedBridge, ReLUBridge, MaxPoolingBridge, LRNBridge, DropoutBridge, SoftmaxLossBridge)
+
+    def _own_methods(self):
+        """Whether nothing that an iteration calls on the network and its operations has been replaced, on one rank."""
+        return (type(self) is Net and not {"forward", "backward"} & self.__dict__.keys() and type(self.ops) is DeviceOps and
+                not {"world_size", "allreduce_begin", "allreduce_wait", "allreduce_sum"} & self.ops.__dict__.keys() and
+                self.ops.world_size() == 1)
 
     def _may_record(self):
         """Whether the walk over the bridges is nothing but library calls that a program keeps: the library's own bridges,
         unmodified, on one rank."""
         plain = [object.__getattribute__(b, "_bridge") if isinstance(b, _WithPrologue) else b for b in self.bridges]
-        return (type(self) is Net and type(self.ops) is DeviceOps and self.ops.world_size() == 1 and
-                not {"forward", "backward"} & set(self.__dict__) and
-                all(type(b) in self._RECORDABLE and not {"forward", "backward"} & set(b.__dict__) for b in plain) and
-                all(type(pb) is ParallelizedBridge for pb in self.pbridges.values()))
+        return (self._own_methods() and
+                all(type(b) in self._RECORDABLE and not {"forward", "backward"} & b.__dict__.keys() and
+                    b.__dict__.get("draw_mask", _drawn_by_the_producer) is _drawn_by_the_producer for b in plain) and
+                all(type(pb) is ParallelizedBridge and pb.defer_update and pb.ops is self.ops and
+                    not {"backward", "begin_allreduce"} & pb.__dict__.keys() for pb in self.pbridges.values()))
+
+    def _same_parts(self):
+        bridges, pbridges, ops = self._recorded
+        return bridges == self.bridges and pbridges == self.pbridges and ops is self.ops
+
+    def _look_again(self):
+        """Watches what the network consists of now."""
+        self._watch.rewired, self._recorded = False, (list(self.bridges), dict(self.pbridges), self.ops)
+        watch([object.__getattribute__(b, "_bridge") if isinstance(b, _WithPrologue) else b for b in self.bridges] +
+              list(self.pbridges.values()), self._watch)
 
     def _release_program(self):
         if self._program is not None:
             self.ctx.lib.cct_program_destroy(self._program)
         self._program = None
 
-    def _record(self):
+    def _postpone(self):
+        """The program (if any) goes; the next one is recorded after some steps."""
+        lasted = self._program is not None and self._runs > 2 * self._patience
         self._release_program()
-        if self._may_record():
-            h = C.c_void_p()
-            capi.check(self.ctx.lib.cct_program_begin(self.ctx.h, C.byref(h)), "cct_program_begin", self.ctx.h)
-            drops = [b for b, t in zip(self.bridges, self.types) if t == "Dropout"]
-            try:
-                for d in drops:
-                    d.mask_held = True
-                self.forward()
-                self._backward_passes()
-            except BaseException:
-                self.ctx.lib.cct_program_destroy(h)
-                raise
-            finally:
-                for d in drops:
-                    d.mask_held = False
+        self._patience = 1 if lasted else min(2 * self._patience, 64)
+        self._walks = self._patience
+
+    def _record(self):
+        """Forward and backward passes whose calls are kept, if they may be; False (and nothing done) otherwise."""
+        if self._watch.rewired or not self._same_parts():
+            self._look_again()
+        self._watch.changed = False  # from here on: what changes while the walk is recorded counts
+        self._runs = 0
+        if not self._may_record():
+            self._postpone()
+            return False
+        h = C.c_void_p()
+        capi.check(self.ctx.lib.cct_program_begin_live(self.ctx.h, C.byref(h)), "cct_program_begin_live", self.ctx.h)
+        try:
+            self.forward()
+            self._backward_passes()
             capi.check(self.ctx.lib.cct_program_end(h), "cct_program_end", self.ctx.h)
-            self._program, self._drops = h, drops
-        self._recorded = (Tracked.changes, list(self.bridges))
+        except BaseException:
+            self.ctx.lib.cct_program_destroy(h)
+            raise
+        self._program, self._drops = h, [b for b, t in zip(self.bridges, self.types) if t == "Dropout"]
+        return True
 
     def step(self):
         before = capi.kernel_launches()
@@ -467,15 +496,18 @@ class Net:
         self._step_launches = capi.kernel_launches() - before
 
     def _step(self):
-        if self._recorded is None or self._recorded[0] != Tracked.changes or self._recorded[1] != self.bridges:
-            self._record()
-        if self._program is None or "forward" in self.__dict__ or "backward" in self.__dict__:
+        if self._program is not None and (self._watch.changed or not self._same_parts() or not self._own_methods()):
+            self._postpone()
+        if self._program is not None:
+            self._runs += 1
+            for d in self._drops:
+                DropoutBridge.draw_mask(d)
+            capi.check(self.ctx.lib.cct_program_run(self._program), "cct_program_run", self.ctx.h)
+        elif self._walks or not self._record():
+            self._walks = max(0, self._walks - 1)
             self.forward()
             self.backward()
             return
-        for d in self._drops:
-            DropoutBridge.draw_mask(d)
-        capi.check(self.ctx.lib.cct_program_run(self._program), "cct_program_run", self.ctx.h)
         self._update.apply([self.pbridges[i] for i in sorted(self.pbridges, reverse=True)])
 
     def set_update_model_gradients(self, flag):
@@ -556,7 +588,6 @@ class Net:
     def close(self):
         self.ctx.sync()
         self._release_program()
-        self._recorded = None
         for br in self.bridges:
             br.close()
         for pb in self.pbridges.values():
@@ -564,6 +595,10 @@ class Net:
         for c in self._cubes:
             c.free()
         self._cubes = []
+
+
+def _drawn_by_the_producer():
+    """draw_mask() of a dropout bridge whose mask the layer in front draws."""
 
 
 class _WithPrologue:

@@ -11,10 +11,12 @@ learning-rate policy, per-blob multipliers) can be exercised with gloo ranks on 
 """
 import ctypes as C
 import math
+import struct
 
 import numpy as np
 
 from . import capi
+from .bridge import Tracked
 
 
 def partition_batch(global_batch, n_partitions):
@@ -355,13 +357,15 @@ class ModelParallelFullyConnectedBridge:
         self.staging.free()
 
 
-class ParallelizedBridge:
+class ParallelizedBridge(Tracked):
     """One rank's share of a data-parallel convolution layer.
 
     `bridge` is this rank's sub-bridge over its batch slice (a ConvolutionBridge).  Its model, bias and gradient cubes
     are re-pointed into one flat buffer owned here, as the reference's ParallelizedBridge owns p_model_cube and hands
     the pointer to its sub-bridges (ParallelizedBridge_impl.hxx:519-532).
     """
+
+    _untracked = ("current_iter", "update_model_gradients", "lr_mult", "decay_mult", "solver")  # the update reads them every time
 
     def __init__(self, bridge, solver, ops, lr_mult=(1.0, 2.0), decay_mult=(1.0, 0.0), defer_update=False):
         self.bridge, self.solver, self.ops = bridge, solver, ops
@@ -484,6 +488,10 @@ class ParallelizedBridge:
         self.params = self.grads = self.hist = None
 
 
+_SGD_ITEM = struct.Struct("@NPPPfff4x")  # capi.SgdItem (a ctypes structure takes four times as long to fill)
+assert _SGD_ITEM.size == C.sizeof(capi.SgdItem)
+
+
 class NetworkUpdate:
     """apply_update() of all layers of a network as one launch, where their updaters are the library's own (device memory, no L1
     decay, neither apply_update() nor the step replaced)."""
@@ -492,35 +500,43 @@ class NetworkUpdate:
         self.key, self.items, self.n = None, None, 0
 
     @staticmethod
-    def _plain(pb):
-        ops = pb.ops
-        return (type(pb).apply_update is ParallelizedBridge.apply_update and "apply_update" not in pb.__dict__ and
-                isinstance(ops, DeviceOps) and type(ops).sgd_step is DeviceOps.sgd_step and "sgd_step" not in ops.__dict__ and
-                pb.solver.regularization_type != "L1")
+    def _plain(active):
+        ops = active[0].ops
+        if not isinstance(ops, DeviceOps):
+            return False
+        for pb in active:
+            if pb.ops is not ops and not (isinstance(pb.ops, DeviceOps) and pb.ops.ctx is ops.ctx):
+                return False
+            if (type(pb.ops).sgd_step is not DeviceOps.sgd_step or "sgd_step" in pb.ops.__dict__ or
+                    type(pb).apply_update is not ParallelizedBridge.apply_update or "apply_update" in pb.__dict__ or
+                    pb.solver.regularization_type == "L1"):
+                return False
+        return True
 
     def apply(self, pbridges):
         active = [pb for pb in pbridges if pb.update_model_gradients]
         if not active:
             return
-        if not all(self._plain(pb) and pb.ops.ctx is active[0].ops.ctx for pb in active):
+        if not self._plain(active):
             for pb in active:
                 pb.apply_update()
             return
         bases, key = {}, []
         for pb in active:
-            pb.current_iter += 1  # the updater increments before use (GradientUpdater.h:155)
+            it = pb.current_iter + 1  # the updater increments before use (GradientUpdater.h:155)
+            pb.__dict__["current_iter"] = it  # (untracked)
             s = pb.solver
-            which = (id(s), pb.current_iter)
-            base = bases.get(which)
+            base = bases.get((id(s), it))
             if base is None:
-                base = bases[which] = get_learning_rate(s.lr_policy, s.base_lr, s.gamma, float(pb.current_iter), float(s.stepsize),
-                                                        s.power, float(s.max_iter))
+                base = bases[id(s), it] = get_learning_rate(s.lr_policy, s.base_lr, s.gamma, float(it), float(s.stepsize), s.power,
+                                                            float(s.max_iter))
             # everything update_tensors() reads, by value
-            key.append((pb.n_w, pb.n_b, pb.params, pb.grads, pb.hist, base, *pb.lr_mult, *pb.decay_mult, s.momentum, s.weight_decay,
+            key.append((base, pb.n_w, pb.n_b, pb.params, pb.grads, pb.hist, *pb.lr_mult, *pb.decay_mult, s.momentum, s.weight_decay,
                         s.regularization_type))
         if key != self.key:
-            tensors = [t for pb, k in zip(active, key) for t in pb.update_tensors(k[5])]
-            self.items, self.n, self.key = (capi.SgdItem * len(tensors))(*[capi.SgdItem(*t) for t in tensors]), len(tensors), key
+            tensors = [t for pb, k in zip(active, key) for t in pb.update_tensors(k[0])]
+            self.items = (capi.SgdItem * len(tensors)).from_buffer_copy(b"".join([_SGD_ITEM.pack(*t) for t in tensors]))
+            self.n, self.key = len(tensors), key
         active[0].ops.sgd_steps(self.items, self.n)
 
 

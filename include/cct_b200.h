@@ -221,13 +221,15 @@ int cct_fc_plan_last_timings(cct_fc_plan* plan, float ms[5]);
  * same thread makes on the context - cct_conv_forward / backward / backward_fused, cct_fc_forward / backward, cct_maxpool_*,
  * cct_relu_*, cct_lrn_*, cct_dropout_apply, cct_softmax_loss_* - are kept with their arguments instead of being carried out
  * (they return CCT_OK); every other call takes effect at once, and so do the calls of other threads.  A thread records one
- * program at a time and ends it itself.  cct_program_run carries the kept calls out in order, as often as wanted, and returns
+ * program at a time and ends it itself.  After cct_program_begin_live the calls are carried out as well as kept, which counts
+ * as the program's first run.  cct_program_run carries the kept calls out in order, as often as wanted, and returns
  * the first error; from the second run on as one CUDA graph launch, unless a plan's timing is switched on or the context's
  * stream is being captured by the caller.  The plans and buffers they name must still exist then.  A caller whose iteration
  * repeats the same calls on the same buffers pays for walking its layers once.  cct_program_graph_launches: how many of the
  * runs so far were a graph launch. */
 typedef struct cct_program cct_program;
 int cct_program_begin(cct_ctx* ctx, cct_program** out);
+int cct_program_begin_live(cct_ctx* ctx, cct_program** out);
 int cct_program_end(cct_program* program);
 int cct_program_run(cct_program* program);
 int cct_program_graph_launches(const cct_program* program, unsigned long long* count);

@@ -217,31 +217,109 @@ def test_softmax_class_counts(ctx, B, classes):
         assert_close(cG.download(), gr, "gradient")
 
 
-def test_recorded_step_equals_the_bridges_one_by_one(ctx):
-    """Three steps through the recorded program (its first run call by call, the later ones as a graph), a change of a
-    bridge's switch that has to be noticed, one more step: the same bits as a network whose bridges are walked through."""
+def small_network(ctx):
     from caffecontroll_b200.net import Net, parse_prototxt, solver_from_message
     from tests.test_net_gpu import B, NET, SOLVER
     net_param, solver = parse_prototxt(NET.replace("dropout_ratio: 0.5", "dropout_ratio: 0.4")), solver_from_message(parse_prototxt(SOLVER))
     rng = np.random.default_rng(3)
-    X, labels = rng.standard_normal((B, 3, 67, 67)).astype(np.float32), rng.integers(0, 12, B).astype(np.float32)
+    net = Net(ctx, net_param, solver, B, fuse=True)
+    data = [(rng.standard_normal((B, 3, 67, 67)).astype(np.float32), rng.integers(0, 12, B).astype(np.float32)) for _ in range(2)]
+    net.set_input(*data[0])
+    return net, data
+
+
+def graph_launches(ctx, net):
+    n = C.c_ulonglong()
+    capi.check(ctx.lib.cct_program_graph_launches(net._program, C.byref(n)), "cct_program_graph_launches", ctx.h)
+    return n.value
+
+
+def parameters(net):
+    net.ctx.sync()
+    return [pb.get_model_cube().download() for _, pb in net.param_bridges()]
+
+
+def test_recorded_step_equals_the_bridges_one_by_one(ctx):
+    """Steps through the recorded program (the first walks, the second records its walk, the later ones are graph launches), a
+    change of a bridge's switch that has to be noticed, a second recording: the same bits as a network whose bridges are walked
+    through."""
     results = []
     for recorded in (True, False):
-        net = Net(ctx, net_param, solver, B, fuse=True)
-        net.set_input(X, labels)
-        for i in range(4):
-            if i == 3:
+        net, _ = small_network(ctx)
+        for i in range(9):
+            if i == 5:
                 net.bridges[net.names.index("fc7")].needs_to_calc_backward_grad = False
-            if recorded:
-                net.step()
-            else:
+            if not recorded:
                 net.forward()
                 net.backward()
-        ctx.sync()
-        results.append([pb.get_model_cube().download() for _, pb in net.param_bridges()])
+                continue
+            net.step()
+            other = LogicalCube(ctx, 1, 1, 1, 1)  # objects that are not the network's do not matter, nor does an equal value
+            other.ptr, net.labels.ptr = other.ptr, net.labels.ptr + 0
+            other.free()
+            assert (net._program is None) == (i in (0, 5)), i
+            if net._program is not None:
+                assert graph_launches(ctx, net) == {1: 0, 2: 1, 3: 2, 4: 3, 6: 0, 7: 1, 8: 2}[i]
+        results.append(parameters(net))
         net.close()
     for a, b in zip(*results):
         assert np.array_equal(a, b)
+
+
+def test_steps_that_alternate_between_input_buffers(ctx):
+    """A double-buffered loader: the same bits as copying each batch into one buffer, and next to no recordings."""
+    results = []
+    for alternate in (True, False):
+        net, data = small_network(ctx)
+        buffers = [tuple(LogicalCube.from_numpy(ctx, a if a.ndim == 4 else a.reshape(-1, 1, 1, 1)) for a in d) for d in data]
+        own = net.input.p_data_cube.ptr, net.labels.ptr
+        recordings, record = [], net._record
+        net._record = lambda: recordings.append(1) or record()
+        for i in range(40):
+            if alternate:
+                net.input.p_data_cube.ptr, net.labels.ptr = (c.ptr for c in buffers[i % 2])
+                net.loss_bridge.p_data_labels = net.labels
+            else:
+                net.set_input(*data[i % 2])
+            net.step()
+        assert len(recordings) == (5 if alternate else 1)  # at steps 1, 4, 9, 18 and 35, each given up at the next
+        results.append(parameters(net))
+        net.input.p_data_cube.ptr, net.labels.ptr = own
+        net.close()
+        for pair in buffers:
+            for c in pair:
+                c.free()
+    for a, b in zip(*results):
+        assert np.array_equal(a, b)
+
+
+def test_replaced_methods_end_a_recording(ctx):
+    """What a program replaces on a network that has recorded its calls is called from the next step on."""
+    net, _ = small_network(ctx)
+    for _ in range(3):
+        net.step()
+    assert graph_launches(ctx, net) == 1
+    calls = []
+    name, pb = net.param_bridges()[0]
+    backward = pb.backward
+    pb.backward = lambda begin_allreduce=True: (calls.append(name), backward(begin_allreduce))
+    net.step()
+    assert calls == [name] and net._program is None
+    del pb.backward
+    while net._program is None:
+        net.step()
+    net.step()
+    net.ops.allreduce_begin = lambda ptr, count: calls.append(count)
+    net.step()
+    assert len(calls) == 1 + len(net.pbridges)
+    del net.ops.allreduce_begin
+    while net._program is None:
+        net.step()
+    net.ops.world_size = lambda: 2  # a process group that was set up later
+    net.ops.allreduce_begin = lambda ptr, count: calls.append(count)
+    net.step()
+    assert len(calls) == 1 + 2 * len(net.pbridges) and net._program is None
+    net.close()
 
 
 def test_recording_is_one_threads_own(ctx):

@@ -98,3 +98,42 @@ def test_model_parallel_placement_fields_follow_the_reference_rules():
         with pytest.raises(ValueError):
             model_parallel_gpus(bad, depth)
 
+
+
+def test_a_watch_sees_the_objects_it_reaches_and_no_others():
+    from caffecontroll_b200.bridge import Layer, LogicalCube, Tracked, Watch, watch
+    cube = lambda: LogicalCube(None, 2, 2, 1, 1, ptr=4096)  # noqa: E731
+    inner, a, b = cube(), Layer(cube(), cube()), Layer(cube(), None)
+    a.fused = (inner, 3)
+    first, second = Watch(), Watch()
+    watch([a], first)
+    watch([a, b], first)  # once more: no second entry
+    watch([b], second)
+    assert len(a._watches) == 1
+
+    def seen(change):
+        for w in (first, second):
+            w.changed = w.rewired = False
+        change()
+        return (first.changed, first.rewired), (second.changed, second.rewired)
+
+    none, value, object_ = (False, False), (True, False), (True, True)
+    assert seen(lambda: setattr(a.p_data_cube, "ptr", 4096)) == (none, none)  # the same value
+    assert seen(lambda: setattr(a.p_data_cube, "ptr", 8192)) == (value, none)
+    assert seen(lambda: setattr(inner, "ptr", 8192)) == (value, none)
+    assert seen(lambda: setattr(b, "p_data_cube", b.p_data_cube)) == (none, none)
+    assert seen(lambda: setattr(b, "p_data_cube", cube())) == (object_, object_)
+    assert seen(lambda: setattr(a, "scale", 0.0)) == (value, none)
+    assert seen(lambda: setattr(a, "scale", 0.0)) == (none, none)
+    assert seen(lambda: setattr(a, "scale", -0.0)) == (value, none)
+    assert seen(lambda: setattr(a, "scale", 0)) == (value, none)
+    assert seen(lambda: delattr(a, "scale")) == (object_, none)
+    assert seen(cube) == (none, none)
+
+    class Counting(Tracked):
+        _untracked = ("calls",)
+
+    c = Counting()
+    watch([c], first)
+    assert seen(lambda: setattr(c, "calls", 1)) == (none, none)
+    assert seen(lambda: setattr(c, "forward", None)) == (object_, none)
