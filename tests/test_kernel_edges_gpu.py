@@ -197,6 +197,25 @@ def test_pooling_planes(ctx, port, B, D, n, k, s):
     assert np.array_equal(cdA.download(), port.maxpool_backward(dP, idxr, n))
 
 
+def test_normalisation_with_subnormal_powers(ctx):
+    """scale^-beta below 2^-126 times a large x: the product is an ordinary number.  Tolerance: the exponent -beta log2(scale), up
+    to 130 in fp32, is off by up to 130 * 2^-23 = 1.6e-5 (relative error ln 2 of that), a subnormal power keeps 18 bits or more:
+    below 1e-4."""
+    B, D, n, alpha, beta = 1, 24, 4, 1.0, 1.3
+    X = np.zeros((B, D, n, n), np.float32)
+    X[0, ::8] = np.float32(10.0) ** np.linspace(14.0, 15.6, n * n, dtype=np.float32).reshape(n, n)
+    x = X.astype(np.float64)
+    pad = np.pad(x * x, ((0, 0), (2, 2), (0, 0), (0, 0)))
+    scale = 1 + alpha / 5 * sum(pad[:, j:j + D] for j in range(5))
+    power = scale ** -beta
+    assert (power < 2.0 ** -126).any() and (power > 2.0 ** -132).all()
+    cX, cY = LogicalCube.from_numpy(ctx, X), LogicalCube(ctx, n, n, D, B)
+    capi.check(ctx.lib.cct_lrn_forward(ctx.h, cX.ptr, cY.ptr, None, B, D, n * n, 5, alpha, beta), "lrn fwd", ctx.h)
+    ctx.sync()
+    got, want = cY.download()[0, ::8], (x * power)[0, ::8]
+    assert np.max(np.abs(got - want) / want) < 1e-4
+
+
 @pytest.mark.parametrize("B,classes", [(1, 1), (1, 2), (7, 1024), (5, 1025), (3, 4001)])
 def test_softmax_class_counts(ctx, B, classes):
     """Tolerance: parity's 1e-4 against the fp32 sums' (classes + B) * 2^-24 < 3e-4 of terms that are positive, in practice 1e-6."""
