@@ -151,12 +151,9 @@ static int ctx_create_common(int device_id, cudaStream_t stream, bool make_strea
     ctx->status_host = hs;
     e = cudaHostGetDevicePointer((void**)&ctx->status_dev, hs, 0);
   }
-  if (e == cudaSuccess) e = cudaMalloc((void**)&ctx->ticket, 256);
-  if (e == cudaSuccess) e = cudaMemset(ctx->ticket, 0, 256);
   if (e != cudaSuccess) {
     std::fprintf(stderr, "cct_b200: context creation failed: %s\n", cudaGetErrorString(e));
     if (hs) cudaFreeHost(hs);
-    if (ctx->ticket) cudaFree(ctx->ticket);
     if (ctx->owns_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return CCT_ERR_CUDA;
@@ -180,7 +177,6 @@ int cct_ctx_destroy(cct_ctx* ctx) {
   if (cudaStream_t spare = ctx->spare_stream.load()) cudaStreamDestroy(spare);
   if (ctx->owns_stream) cudaStreamDestroy(ctx->stream);
   if (ctx->status_host) cudaFreeHost((void*)ctx->status_host);
-  cudaFree(ctx->ticket);
   delete ctx;
   return CCT_OK;
 }

@@ -49,7 +49,6 @@ struct cct_ctx {
   // One word in mapped pinned host memory that kernels set when a bounded wait runs out; read by cct_sync().
   volatile int* status_host = nullptr;
   int* status_dev = nullptr;
-  unsigned* ticket = nullptr;  // device word, zero between kernels: which block of a kernel is the last to finish
   std::string last_error;
   std::atomic<cudaStream_t> spare_stream{nullptr};  // for the next capture of a program
   int timed_plans = 0;  // plans whose kernel timing is switched on: programs then run call by call
@@ -98,22 +97,31 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 inline std::atomic<uint64_t> kernel_launches{0};  // cct_kernel_launches
 inline thread_local uint64_t thread_launches = 0; // those of this thread, captured ones included
 
+// `cluster` blocks (a divisor of the grid's x) form a thread-block cluster.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                              Args&&... args) {
+inline cudaError_t launch_pdl_cluster(unsigned cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                      cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   kernel_launches.fetch_add(1, std::memory_order_relaxed);
   ++thread_launches;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              Args&&... args) {
+  return launch_pdl_cluster(1, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 #endif
 

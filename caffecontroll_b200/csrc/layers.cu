@@ -235,17 +235,37 @@ __global__ void dropout_mask_kernel(uint32_t* __restrict__ mask, size_t count, u
 
 // -------------------------------------------------------------------------------------------- softmax loss
 // SoftmaxLossBridge (src/kernels/softmax.hxx:17-50): per image prob = exp(x - max) / sum, loss -= log(max(prob[label],
-// FLT_MIN)).  One warp per image; the per-image losses are added in image order by the block that finishes last, so the
-// result does not depend on the grid.  Labels are floats, as in the reference's label cube.  Up to 1024 classes a lane
-// keeps its logits in registers, all loads in flight at once (256 images x 1000 classes: 8.0 us with three passes over the
-// row and 4.8 us for a kernel of its own that added the losses one load at a time).
-constexpr int kSoftmaxVals = 32;
-template <bool IN_REGS>
-__global__ void __launch_bounds__(128) softmax_fwd_kernel(const float* __restrict__ X, const float* __restrict__ labels,
-                                                          float* __restrict__ prob, float* __restrict__ image_loss,
-                                                          float* __restrict__ loss, unsigned* __restrict__ ticket, int B, int C) {
+// FLT_MIN)).  One warp per image; the per-image losses are added in image order by one warp afterwards, so the result does
+// not depend on the grid.  Labels are floats, as in the reference's label cube.  Up to 1024 classes a lane keeps its logits
+// in registers, all loads in flight at once; beyond that a warp makes three passes over its row.
+// A few images are one cluster, whose barrier stands between the images and their sum (64 images, 10 classes: 4.3 us); more
+// take a second launch for it (256 images, 1000 classes: 7.9 us, one cluster of 256 warps 12.5).  Nothing is shared between
+// calls: calls of one context may run beside one another, replayed from graphs on several streams.
+constexpr int kSoftmaxVals = 32, kSoftmaxCluster = 8, kSoftmaxWarps = 8;
+
+// out = v[0] + v[1] + ... + v[n - 1], added in order by one warp: one load per lane, then the additions.
+__device__ __forceinline__ void sum_in_order(const float* v, float* out, int n, int lane) {
+  float acc = 0.f;
+  for (int i0 = 0; i0 < n; i0 += 32) {
+    const float mine = i0 + lane < n ? __ldcg(v + i0 + lane) : 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const float one = __shfl_sync(0xffffffffu, mine, j);
+      if (i0 + j < n) acc += one;
+    }
+  }
+  if (lane == 0) *out = acc;
+}
+__global__ void __launch_bounds__(32) sum_in_order_kernel(const float* __restrict__ v, float* __restrict__ out, int n) {
   pdl_wait();
-  __shared__ bool last;
+  sum_in_order(v, out, n, threadIdx.x);
+}
+
+template <bool IN_REGS, bool CLUSTER>
+__global__ void __launch_bounds__(CLUSTER ? 32 * kSoftmaxWarps : 128) softmax_fwd_kernel(const float* __restrict__ X, const float* __restrict__ labels,
+                                                                           float* __restrict__ prob, float* image_loss,
+                                                                           float* __restrict__ loss, int B, int C) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int img = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
   if (img < B) {
@@ -286,30 +306,14 @@ __global__ void __launch_bounds__(128) softmax_fwd_kernel(const float* __restric
       const int label = (int)labels[img];
       const float p = (label >= 0 && label < C) ? expf(x[label] - mx) / sum : 0.f;
       image_loss[img] = -logf(fmaxf(p, FLT_MIN));
-      __threadfence();
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last || threadIdx.x >= 32) return;
-  float acc = 0.f;
-  for (int i0 = 0; i0 < B; i0 += 32) {  // one load per lane, then the additions in image order
-    const float mine = i0 + lane < B ? __ldcg(image_loss + i0 + lane) : 0.f;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float one = __shfl_sync(0xffffffffu, mine, j);
-      if (i0 + j < B) acc += one;
-    }
-  }
-  if (lane == 0) {
-    *loss = acc;
-    *ticket = 0u;
+  if (CLUSTER) {  // the grid is one cluster: every image's loss is there and visible behind this barrier
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (blockIdx.x == 0 && threadIdx.x < 32) sum_in_order(image_loss, loss, B, lane);
   }
 }
 
-// Gradient of the loss with respect to the bridge's input (src/kernels/softmax.hxx:62-80):
-// dX = (prob - onehot(label)) * scale, scale = 1 / (batch the loss is averaged over).
 __global__ void softmax_bwd_kernel(const float* __restrict__ prob, const float* __restrict__ labels,
                                    float* __restrict__ dX, size_t total, int C, float scale) {
   pdl_wait();
@@ -554,8 +558,17 @@ int cct_softmax_loss_forward(cct_ctx* ctx, const float* X, const float* labels, 
   CCT_RECORD(ctx, cct_softmax_loss_forward(ctx, X, labels, prob, image_loss, loss, batch, classes))
   if (!ctx || !X || !labels || !prob || !image_loss || !loss || batch <= 0 || classes <= 0) return CCT_ERR_INVALID;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
-  launch_pdl(classes <= 32 * kSoftmaxVals ? softmax_fwd_kernel<true> : softmax_fwd_kernel<false>, dim3((batch + 3) / 4), dim3(128), 0,
-             ctx->stream, X, labels, prob, image_loss, loss, ctx->ticket, batch, classes);
+  const bool in_regs = classes <= 32 * kSoftmaxVals;
+  if (in_regs && batch <= kSoftmaxCluster * kSoftmaxWarps) {
+    const int warps = (batch + kSoftmaxCluster - 1) / kSoftmaxCluster;
+    launch_pdl_cluster(kSoftmaxCluster, softmax_fwd_kernel<true, true>, dim3(kSoftmaxCluster), dim3(32 * warps), 0, ctx->stream, X, labels,
+                       prob, image_loss, loss, batch, classes);
+  } else {
+    launch_pdl(in_regs ? softmax_fwd_kernel<true, false> : softmax_fwd_kernel<false, false>, dim3((batch + 3) / 4), dim3(128), 0,
+               ctx->stream, X, labels, prob, image_loss, loss, batch, classes);
+    CCT_CHECK_LAUNCH(ctx);
+    launch_pdl(sum_in_order_kernel, dim3(1), dim3(32), 0, ctx->stream, image_loss, loss, batch);
+  }
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }

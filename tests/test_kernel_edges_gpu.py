@@ -216,7 +216,7 @@ def test_normalisation_with_subnormal_powers(ctx):
     assert np.max(np.abs(got - want) / want) < 1e-4
 
 
-@pytest.mark.parametrize("B,classes", [(1, 1), (1, 2), (7, 1024), (5, 1025), (3, 4001)])
+@pytest.mark.parametrize("B,classes", [(1, 1), (1, 2), (7, 1024), (5, 1025), (3, 4001), (63, 1000), (64, 40), (65, 40), (33, 1030), (1030, 1030)])
 def test_softmax_class_counts(ctx, B, classes):
     """Tolerance: parity's 1e-4 against the fp32 sums' (classes + B) * 2^-24 < 3e-4 of terms that are positive, in practice 1e-6."""
     rng = np.random.default_rng(classes)
@@ -225,7 +225,7 @@ def test_softmax_class_counts(ctx, B, classes):
     pr, lr, gr = pyoracle.np_softmax_loss(X, labels, scale=1.0 / B)
     cX, cL = LogicalCube.from_numpy(ctx, X), LogicalCube.from_numpy(ctx, labels.reshape(B, 1, 1, 1))
     cP, cG, cIL, cLoss = (LogicalCube(ctx, 1, 1, d, b) for d, b in ((classes, B), (classes, B), (1, B), (1, 1)))
-    for _ in range(2):  # the second call finds the counter that the first one left
+    for _ in range(2):
         capi.check(ctx.lib.cct_softmax_loss_forward(ctx.h, vp(cX.ptr), vp(cL.ptr), vp(cP.ptr), vp(cIL.ptr), vp(cLoss.ptr), B,
                                                     classes), "softmax fwd", ctx.h)
         capi.check(ctx.lib.cct_softmax_loss_backward(ctx.h, vp(cP.ptr), vp(cL.ptr), vp(cG.ptr), B, classes, 1.0 / B),
@@ -234,6 +234,40 @@ def test_softmax_class_counts(ctx, B, classes):
         assert_close(cP.download(), pr, "probabilities")
         assert abs(float(cLoss.download().reshape(-1)[0]) - lr) <= 1e-4 * abs(lr) + 1e-6
         assert_close(cG.download(), gr, "gradient")
+
+
+@pytest.mark.parametrize("B", [64, 3000])
+def test_losses_beside_one_another(B):
+    """Two calls of one context, captured into graphs and replayed on two streams at once: each gives its own sum."""
+    from caffecontroll_b200 import Context
+    C_, streams = 1000, [torch.cuda.Stream() for _ in range(2)]
+    own = Context(0, stream=streams[0].cuda_stream)
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    graphs, losses, want = [], [], []
+    for i in range(2):
+        X = 3 * torch.randn((B, C_), generator=gen, device="cuda")
+        labels = torch.randint(0, C_, (B,), generator=gen, device="cuda").float()
+        prob, image, loss = torch.zeros_like(X), torch.zeros(B, device="cuda"), torch.zeros(1, device="cuda")
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=streams[0]):
+            for _ in range(20):
+                capi.check(own.lib.cct_softmax_loss_forward(own.h, X.data_ptr(), labels.data_ptr(), prob.data_ptr(), image.data_ptr(),
+                                                            loss.data_ptr(), B, C_), "softmax", own.h)
+        graphs.append((g, X, labels, prob, image))
+        losses.append(loss)
+        want.append(float(torch.nn.functional.cross_entropy(X.double(), labels.long(), reduction="sum")))
+    for _ in range(20):
+        for i in range(2):
+            losses[i].fill_(-1)
+        torch.cuda.synchronize()
+        for i in range(2):
+            with torch.cuda.stream(streams[i]):
+                graphs[i][0].replay()
+        torch.cuda.synchronize()
+        for i in range(2):
+            assert abs(float(losses[i]) - want[i]) <= 1e-4 * want[i]
+    own.close()
 
 
 def small_network(ctx):
