@@ -143,20 +143,6 @@ __device__ __forceinline__ void split_tf32_trunc(float x, uint32_t& hi, uint32_t
   lo = __float_as_uint(x - __uint_as_float(hi));
 }
 
-// The same for two values, the subtractions as one packed instruction (hi * -1 + x is exact).
-__device__ __forceinline__ void split_tf32_trunc2(float x0, float x1, uint32_t* hi, uint32_t* lo) {
-  hi[0] = __float_as_uint(x0) & 0xFFFFE000u;
-  hi[1] = __float_as_uint(x1) & 0xFFFFE000u;
-  asm("{\n\t.reg .b64 x, h, m, l;\n\t"
-      "mov.b64 x, {%2, %3};\n\t"
-      "mov.b64 h, {%4, %5};\n\t"
-      "mov.b64 m, {%6, %6};\n\t"
-      "fma.rn.f32x2 l, h, m, x;\n\t"
-      "mov.b64 {%0, %1}, l;\n\t}"
-      : "=r"(lo[0]), "=r"(lo[1])
-      : "f"(x0), "f"(x1), "r"(hi[0]), "r"(hi[1]), "r"(0xBF800000u));
-}
-
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
