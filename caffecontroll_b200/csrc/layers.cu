@@ -262,9 +262,9 @@ __global__ void __launch_bounds__(32) sum_in_order_kernel(const float* __restric
 }
 
 template <bool IN_REGS, bool CLUSTER>
-__global__ void __launch_bounds__(CLUSTER ? 32 * kSoftmaxWarps : 128) softmax_fwd_kernel(const float* __restrict__ X, const float* __restrict__ labels,
-                                                                           float* __restrict__ prob, float* image_loss,
-                                                                           float* __restrict__ loss, int B, int C) {
+__global__ void __launch_bounds__(CLUSTER ? 32 * kSoftmaxWarps : 128)
+    softmax_fwd_kernel(const float* __restrict__ X, const float* __restrict__ labels, float* __restrict__ prob, float* image_loss,
+                       float* __restrict__ loss, int B, int C) {
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int img = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
@@ -314,6 +314,8 @@ __global__ void __launch_bounds__(CLUSTER ? 32 * kSoftmaxWarps : 128) softmax_fw
   }
 }
 
+// Gradient of the loss with respect to the bridge's input (src/kernels/softmax.hxx:62-80):
+// dX = (prob - onehot(label)) * scale, scale = 1 / (batch the loss is averaged over).
 __global__ void softmax_bwd_kernel(const float* __restrict__ prob, const float* __restrict__ labels,
                                    float* __restrict__ dX, size_t total, int C, float scale) {
   pdl_wait();
