@@ -1432,8 +1432,8 @@ __global__ void bias_grad_kernel(const float* __restrict__ plane_sums, float* __
 }
 
 // ------------------------------------------------------------------------------------------ weight packing
-// A block writes one row of the packed operand (blockIdx.x = (vg, j): there may be more than 65 535 of them), four consecutive reduction indices per thread and
-// step: one decode per four elements and 16-byte stores (a flat grid-stride loop spent most of its time dividing: CaffeNet
+// A block writes one row of the packed operand (blockIdx.x = (vg, j): there may be more than 65 535 of them), four consecutive
+// reduction indices per thread and step: one decode per four elements and 16-byte stores (a flat grid-stride loop spent most of its time dividing: CaffeNet
 // conv3's 0.9 M weights 8.0 / 11.6 us for the two operands, bound by neither memory nor launch).
 constexpr int kPackThreads = 128;
 
@@ -1470,16 +1470,16 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
 }
 
 // Data-gradient B operand: [2][vg][n_pad][k_pad]; row j = (d, py, px) of channel tile nt of group g (py, px: position
-// inside a block of s * rows x s input pixels), column kk = (oc, jy, jx) <- W[g*og + oc][d][py + (jy - rows + 1)*s][px + jx*s],
-// zero where the tap index is outside the kernel.
+// inside a block of s x s input pixels), column kk = (oc, jy, jx) <- W[g*og + oc][d][py + jy*s][px + jx*s], zero where the tap
+// index is outside the kernel.
 __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                   float* __restrict__ lo, int tiles_per_group, int og,
-                                                                  int Dg, int k, int s, int taps, int rows, int d_tile,
+                                                                  int Dg, int k, int s, int taps, int d_tile,
                                                                   int n_real, int n_pad, int k_real, int k_pad, int run) {
   pdl_wait();
   const int vg = blockIdx.x / n_pad, j = blockIdx.x - vg * n_pad;
-  const int grp = vg / tiles_per_group, d = (vg - grp * tiles_per_group) * d_tile + j / (s * s * rows);
-  const int py = (j / s) % (s * rows), px = j % s, window = taps * (taps + rows - 1);
+  const int grp = vg / tiles_per_group, d = (vg - grp * tiles_per_group) * d_tile + j / (s * s);
+  const int py = (j / s) % s, px = j % s, window = taps * taps;
   const bool live = j < n_real && d < Dg;
   const float* src = W + ((size_t)grp * og * Dg + d) * k * k;
   const size_t row = (size_t)blockIdx.x * k_pad;
@@ -1490,8 +1490,8 @@ __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* _
       // reduction index -> (filter / run, jy, jx, filter % run)
       const int r = (kk + e) / run, chunk = r / window, tap = r - chunk * window;
       const int oc = chunk * run + (kk + e - r * run), jy = tap / taps, jx = tap - jy * taps;
-      const int kr = py + (jy - rows + 1) * s, kc = px + jx * s;
-      v[e] = (live && kk + e < k_real && (unsigned)kr < (unsigned)k && kc < k) ? __ldg(src + (size_t)oc * Dg * k * k + kr * k + kc) : 0.f;
+      const int kr = py + jy * s, kc = px + jx * s;
+      v[e] = (live && kk + e < k_real && kr < k && kc < k) ? __ldg(src + (size_t)oc * Dg * k * k + kr * k + kc) : 0.f;
     }
     store_split4(hi, lo, row + kk, v);
   }
@@ -1549,14 +1549,13 @@ bool two_ctas_per_sm(int n_pad, int taps_smem, int n_bias, int ptab, int* slots)
 // gather takes; a unit adds its set-up and epilogue, a split reduction one more kernel and the traffic of the sums.  So: a
 // last round that is nearly empty (CaffeNet conv3 at batch 256: 2 x 338 units on 148 CTAs are five rounds, 3 x 338 half-width
 // ones on 296 are 3.4) asks for narrower tiles, a layer of few pixels (43 tiles at batch 32, 2 at batch 1) for narrower tiles
-// and splits.  A candidate has to win by 1 % and to keep its accumulation chain within `limit` (chain_limit); `dense`: the part
-// of the reduction's k-blocks that add anything to one accumulator column.
+// and splits.  A candidate has to win by 1 % and to keep its accumulation chain within `limit` (chain_limit).
 struct GatherTiling {
   int tiles = 0, splits = 1, kps = 0;
   double us = 0.0;
 };
 GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, int channels, int cols_per_channel, int kblocks,
-                                  int run, int lane_stride, int n_bias, double limit, double dense) {
+                                  int run, int lane_stride, int n_bias, double limit) {
   GatherTiling best;
   const int t0 = channel_tiles(channels, cols_per_channel);
   for (int t = t0; t > 0 && t <= channels; ++t) {
@@ -1572,7 +1571,7 @@ GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, in
     const double epilogue = 4.0 + 0.004 * n_pad;
     for (int s = 1; s <= std::max(1, std::min(32, kblocks / 2)); ++s) {
       const int kps = (kblocks + s - 1) / s;
-      if ((kblocks + kps - 1) / kps != s || kps * dense * (n_pad <= kCrossCols ? 1.0 : 3.0) > limit) continue;
+      if ((kblocks + kps - 1) / kps != s || kps * (n_pad <= kCrossCols ? 1.0 : 3.0) > limit) continue;
       const long long units = pixel_tiles * groups * t * s, slots = (long long)sms * (two ? 2 : 1), tail = units % slots;
       double us = (double)(units / slots) * (kps * (two ? shared : one) + 0.4 * epilogue) +
                   (tail ? kps * (!two ? one : tail > sms ? shared : alone) + epilogue : 0.6 * epilogue) + 2.6;
@@ -1610,9 +1609,9 @@ struct GatherProblem {
 struct UmmaPlan {
   ConvGeom G;
   GatherProblem fwd, dgr;
-  // data gradient: taps per axis of one stride period; super-pixels of s * dgr_rows x s pixels, how many and the first that
+  // data gradient: taps per axis of one stride period; super-pixels of s x s pixels, how many per axis and the first that
   // holds a pixel
-  int dgr_taps = 0, dgr_rows = 1, dgr_q = 0, dgr_q0 = 0, dgr_qy = 0, dgr_qy0 = 0;
+  int dgr_taps = 0, dgr_q = 0, dgr_q0 = 0;
   // weight gradient: channel tiles per group, channels per tile (the last one may be shorter), padded to 16; longest
   // accumulation chain in k-blocks
   int wt_tiles = 1, wt_n = 0, w_chain = kMaxChainKblocks;
@@ -1785,7 +1784,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     f.run = G.Dg % kRun == 0 ? kRun : 1; f.run_stride = G.n * G.n;
     const long long pixel_tiles = ((long long)G.B * G.m * G.m + kTileM - 1) / kTileM;
     const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, f.run, G.s,
-                                                 G.bias ? G.o : 0, chain_limit(G.og, 1, f.k_pad / kBlockK), 1.0);
+                                                 G.bias ? G.o : 0, chain_limit(G.og, 1, f.k_pad / kBlockK));
     f.tiles = tl.tiles;
     f.ch_tile = f.n = (G.og + f.tiles - 1) / f.tiles;
     f.n_pad = round_up(f.n, 16);
@@ -1818,24 +1817,14 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     p->dgr_q0 = G.p / G.s;
     p->dgr_q = (G.n - 1 + G.p) / G.s + 1 - p->dgr_q0;
     d.run = G.og % kRun == 0 ? kRun : 1; d.run_stride = G.m * G.m;
-    GatherTiling tl;
-    long long pixel_tiles = 0;
-    const double limit = chain_limit(G.Dg, G.s * G.s, (G.og * J * J + kBlockK - 1) / kBlockK);
-    for (int rows = 1; rows <= 4 && J + rows - 1 <= kMaxTapsPerAxis; ++rows) {
-      const int q0 = G.p / (G.s * rows), q = (G.n - 1 + G.p) / (G.s * rows) + 1 - q0, k_real = G.og * J * (J + rows - 1);
-      if (rows > 1 && (k_real > 16384 || channel_tiles(G.Dg, G.s * G.s * rows) == 0)) break;
-      const long long tiles = ((long long)G.B * q * p->dgr_q + kTileM - 1) / kTileM;
-      const GatherTiling c = choose_gather_tiling(ctx->planning_sms(), tiles, G.g, G.Dg, G.s * G.s * rows,
-                                                  round_up(k_real, kBlockK) / kBlockK, d.run, 1, 0, limit,
-                                                  // the taps that a pixel of a taller block does not have: whole runs of eight
-                                                  // products, or (in tap order) single ones among the others
-                                                  d.run == kRun ? (double)J / (J + rows - 1) : 1.0);
-      if (!c.tiles || (tl.tiles && c.us >= 0.99 * tl.us)) continue;
-      tl = c; pixel_tiles = tiles;
-      p->dgr_rows = rows; p->dgr_qy0 = q0; p->dgr_qy = q;
-      d.k_real = k_real;
-    }
-    const int ss = G.s * G.s * p->dgr_rows, H = G.s * p->dgr_rows;
+    d.k_real = G.og * J * J;
+    // One stride period of rows per super pixel: a taller one gathers less per pixel, but the taps that one of its pixels does
+    // not have would be products with a zero weight, and a dY that is not finite would reach pixels whose window does not hold it.
+    const int ss = G.s * G.s;
+    const long long pixel_tiles = ((long long)G.B * p->dgr_q * p->dgr_q + kTileM - 1) / kTileM;
+    const int kblocks = round_up(d.k_real, kBlockK) / kBlockK;
+    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.Dg, ss, kblocks, d.run, 1, 0,
+                                                 chain_limit(G.Dg, ss, kblocks));
     d.k_pad = round_up(d.k_real, kBlockK);
     d.tiles = tl.tiles;
     d.ch_tile = (G.Dg + d.tiles - 1) / d.tiles;
@@ -1845,7 +1834,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     std::vector<MaskTap> t((size_t)d.splits * d.split_k / d.run);
     for (int i = 0; i < (int)t.size(); ++i) {
       if (i * d.run < d.k_real) {
-        const int Jy = J + p->dgr_rows - 1, jx = i % J, jy = (i / J) % Jy, oc = i / (J * Jy) * d.run;
+        const int jx = i % J, jy = (i / J) % J, oc = i / (J * J) * d.run;
         t[i] = MaskTap{oc * G.m * G.m - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
       } else {
         t[i] = MaskTap{0, kPadBit};
@@ -1853,7 +1842,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     }
     std::vector<ColEnt> c(d.n_pad);
     for (int j = 0; j < d.n_pad; ++j) {
-      const int dl = j / ss, py = (j / G.s) % H, px = j % G.s;
+      const int dl = j / ss, py = (j / G.s) % G.s, px = j % G.s;
       c[j] = ColEnt{dl * G.n * G.n + py * G.n + px, (short)py, (short)px};
     }
     if (!tensor_only && G.s == 1) d.small_ct = use_small_conv(G.k, 1, (long long)G.B * G.n * G.n, G.g, G.og, G.Dg);
@@ -2238,19 +2227,18 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
     }
     if (repack) {
       launch_pdl(pack_dgrad_kernel, pack_grid(vgroups * d.n_pad, d.k_pad), dim3(kPackThreads), 0, ctx->stream, W, d.w,
-                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, p->dgr_rows, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run);
+                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run);
       CCT_CHECK_LAUNCH(ctx);
     }
     GatherParams P{};
     P.in = dY; P.out = dX; P.bias = nullptr;
-    const int rows = p->dgr_rows;
-    P.n_pix = B * p->dgr_qy * p->dgr_q; P.q_h = p->dgr_qy; P.q_w = p->dgr_q;
-    P.iy_mul = rows; P.iy_add = (p->dgr_qy0 + 1) * rows - 1; P.ix_mul = 1; P.ix_add = p->dgr_q0;
+    P.n_pix = B * p->dgr_q * p->dgr_q; P.q_h = p->dgr_q; P.q_w = p->dgr_q;
+    P.iy_mul = 1; P.iy_add = p->dgr_q0; P.ix_mul = 1; P.ix_add = p->dgr_q0;
     P.in_lim = G.m;
-    P.tap_sign = -1; P.taps_per_axis = p->dgr_taps + rows - 1;
+    P.tap_sign = -1; P.taps_per_axis = p->dgr_taps;
     P.in_batch_stride = (long long)G.o * G.m * G.m;
     P.in_group_stride = G.og * G.m * G.m;
-    P.oy_mul = G.s * rows; P.oy_add = p->dgr_qy0 * rows * G.s - G.p; P.ox_mul = G.s; P.ox_add = p->dgr_q0 * G.s - G.p;
+    P.oy_mul = G.s; P.oy_add = p->dgr_q0 * G.s - G.p; P.ox_mul = G.s; P.ox_add = p->dgr_q0 * G.s - G.p;
     P.out_lim = G.n; P.check_out = 1;
     P.out_pitch = G.n; P.out_plane = G.n * G.n;
     P.out_batch_stride = (long long)G.D * G.n * G.n;

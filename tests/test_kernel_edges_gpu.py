@@ -20,8 +20,8 @@ def vp(p):
 
 
 # Window rows loaded in 16-byte blocks (stride a multiple of four, no padding), k-blocks that cross images, odd planes whose
-# blocks are misaligned, the tensor's ends, groups; then narrow data gradients, whose accumulator holds several rows of pixels,
-# with a last block that is cut off, padding and stride.  Tolerance: tests/parity.py (1e-4; the split operands stay below 2e-5).
+# blocks are misaligned, the tensor's ends, groups; then narrow data gradients with padding and stride.  Tolerance:
+# tests/parity.py (1e-4; the split operands stay below 2e-5).
 @pytest.mark.parametrize("shape", [
     (1, 3, 11, 8, 11, 4, 0, 1), (3, 3, 47, 24, 11, 4, 0, 1), (5, 4, 23, 17, 8, 4, 0, 1), (2, 2, 61, 128, 13, 8, 0, 1),
     (2, 6, 39, 40, 11, 4, 0, 2), (2, 4, 30, 9, 9, 4, 0, 1), (2, 3, 40, 16, 11, 4, 5, 1),
@@ -36,6 +36,32 @@ def test_convolution_shapes(ctx, port, shape):
     dXr, dWr, dbr = port.conv_backward(X, W, dY, k, s, p, g)
     for a, r, name in ((Y, port.conv_forward(X, W, b, k, s, p, g), "Y"), (dX, dXr, "dX"), (dW, dWr, "dW"), (db, dbr, "db")):
         assert_close(a, r.reshape(a.shape), name)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("shape", [
+    (32, 30, 40, 134, 3, 1, 1, 1), (9, 16, 33, 64, 3, 1, 1, 1), (6, 20, 28, 32, 5, 1, 2, 1), (4, 8, 14, 24, 3, 1, 0, 1),
+    (32, 96, 27, 256, 5, 1, 2, 2),
+])
+def test_a_gradient_that_is_not_finite_stays_in_its_window(ctx, shape, value):
+    """dX outside the window of one element of dY does not depend on that element, whatever it is: bit for bit."""
+    from caffecontroll_b200 import conv_layer
+    B, D, n, o, k, s, p, g = shape
+    X, W, b, dY = make_inputs(31, B, D, n, o, k, s, p, g)
+    W = np.where(W == 0, np.float32(0.01), W)
+    m = (n + 2 * p - k) // s + 1
+    where = (B - 1, o // g - 1, m // 2, m // 2 + 1)
+    dY[where] = 0
+    _, clean, _, _, _ = conv_layer(ctx, X, W, b, dY, k, s, p, g, algo=TENSOR)
+    dY[where] = value
+    _, dX, _, _, used = conv_layer(ctx, X, W, b, dY, k, s, p, g, algo=TENSOR)
+    assert used == TENSOR
+    bad = ~np.isfinite(dX)
+    window = np.zeros(dX.shape, bool)
+    y, x = where[2] - p, where[3] - p
+    window[B - 1, :D // g, max(y, 0):y + k, max(x, 0):x + k] = True
+    assert np.array_equal(bad, window)
+    assert np.array_equal(dX[~window], clean[~window])
 
 
 @pytest.mark.parametrize("algo", [capi.ALGO_AUTO, TENSOR])
@@ -61,8 +87,8 @@ def test_many_groups(ctx, port, algo):
 @pytest.mark.parametrize("shape,which,chain", [
     ((48, 96, 24, 41, 5, 1, 2, 1), "Y", 75), ((64, 64, 20, 64, 3, 1, 1, 1), "dX", 18),
     ((48, 96, 24, 41, 5, 1, 2, 1), "dW", 58), ((64, 64, 20, 64, 3, 1, 1, 1), "dW", 28),
-    # taller pixel blocks (one row of pixels: 38 blocks, 76 at the two additions that narrow tiles may take); units of the weight
-    # gradient's splits, three additions per block on wide tiles; uneven channel tiles
+    # 38 blocks, 76 at the two additions per block that narrow tiles may take; units of the weight gradient's splits, three
+    # additions per block on wide tiles; uneven channel tiles
     ((32, 30, 40, 134, 3, 1, 1, 1), "dX", 76), ((32, 48, 28, 134, 3, 1, 1, 1), "dX", 76),
     ((8, 158, 45, 136, 5, 1, 2, 1), "dW", 3 * 57), ((5, 272, 25, 208, 5, 1, 2, 2), "dW", 3 * 20), ((40, 64, 30, 337, 3, 1, 1, 1), "dW", 3 * 58),
 ])
