@@ -64,9 +64,10 @@ __global__ void __launch_bounds__(kFsThreads) fc_small_kernel(const __grid_const
   __shared__ float s_db[kFsWarps][kFsTile];
   float *s_a = s_ab, *s_b = s_ab + kFsChunk * kFsPitch;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ty = lane >> 2, tx = lane & 3;
-  const int m0 = blockIdx.x * kFsTile, n0 = blockIdx.y * kFsTile;
-  const int r_begin = blockIdx.z * P.r_per_split, r_end = min(P.R, r_begin + P.r_per_split);
-  const bool sum_b = P.db != nullptr && blockIdx.x == 0;
+  const int m_tiles = (P.M + kFsTile - 1) / kFsTile, n_tile = blockIdx.x / m_tiles;  // one grid axis: y ends at 65 535
+  const int m0 = (blockIdx.x - n_tile * m_tiles) * kFsTile, n0 = n_tile * kFsTile;
+  const int r_begin = blockIdx.y * P.r_per_split, r_end = min(P.R, r_begin + P.r_per_split);
+  const bool sum_b = P.db != nullptr && m0 == 0;
   float acc[4][8], db = 0.f;
 #pragma unroll
   for (int u = 0; u < 4; ++u)
@@ -107,8 +108,8 @@ __global__ void __launch_bounds__(kFsThreads) fc_small_kernel(const __grid_const
     float t = 0.f;
 #pragma unroll
     for (int w = 0; w < kFsWarps; ++w) t += s_ab[w * kFsTile * kFsTile + i];
-    if (gridDim.z > 1) {
-      P.out[((long long)blockIdx.z * P.N + n) * P.ld + m] = t;
+    if (gridDim.y > 1) {
+      P.out[((long long)blockIdx.y * P.N + n) * P.ld + m] = t;
       continue;
     }
     const long long at = (long long)n * P.ld + m;

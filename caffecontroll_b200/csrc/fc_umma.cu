@@ -607,7 +607,7 @@ bool use_small_fc(int B, int K, int O) {
 }
 
 void fc_small(cct_ctx* ctx, const FcSmallParams& P, int splits) {
-  launch_pdl(fc_small_kernel, dim3((P.M + kFsTile - 1) / kFsTile, (P.N + kFsTile - 1) / kFsTile, splits), dim3(kFsThreads), 0, ctx->stream, P);
+  launch_pdl(fc_small_kernel, dim3((unsigned)((P.M + kFsTile - 1) / kFsTile) * ((P.N + kFsTile - 1) / kFsTile), splits), dim3(kFsThreads), 0, ctx->stream, P);
 }
 
 bool fc_aligned(std::initializer_list<const void*> ptrs) {

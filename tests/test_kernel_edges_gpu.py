@@ -160,6 +160,26 @@ def test_inner_product_alignment(ctx, B, K, o, shifted):
         assert np.all(got[:shift] == 7) and np.all(got[shift + r.size:] == 7)  # nothing beside the output
 
 
+def test_inner_product_of_many_rows_off_the_boundary(ctx):
+    """More row tiles than a grid has in y, in the kernel that takes an X off a 16-byte boundary.  Tolerance: parity (dW adds
+    2 097 169 / 8 rounded products per chain: 2^-25 sqrt(n / 2) of the sum, 1.1e-5)."""
+    B, K, o = 65536 * 32 + 17, 8, 12
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    make = lambda n: torch.empty(n, device="cuda").uniform_(-1, 1, generator=gen)  # noqa: E731
+    X, W, b, dY = make(B * K + 1)[1:], make(o * K), make(o), make(B * o)
+    Y, dX, dW, db = torch.zeros(B * o, device="cuda"), torch.zeros(B * K, device="cuda"), torch.zeros_like(W), torch.zeros_like(b)
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(plan)), "plan", ctx.h)
+    capi.check(ctx.lib.cct_fc_forward(plan, q(X), q(W), q(b), q(Y), 0, None, 1.0), "forward", ctx.h)
+    capi.check(ctx.lib.cct_fc_backward(plan, q(X), q(W), q(dY), q(dX), q(dW), q(db), 0, None, 1.0), "backward", ctx.h)
+    ctx.sync()
+    ctx.lib.cct_fc_plan_destroy(plan)
+    Xd, Wd, dYd = X.double().view(B, K), W.double().view(o, K), dY.double().view(B, o)
+    for got, ref, name in ((Y, Xd @ Wd.T + b.double(), "Y"), (dX, dYd @ Wd, "dX"), (dW, dYd.T @ Xd, "dW"), (db, dYd.sum(0), "db")):
+        assert_close(got.cpu().numpy(), ref.float().flatten().cpu().numpy(), name)
+
+
 # More than 2^31 elements in X and dX, more than 2^32 in W and dW.  Tolerance: parity (dW for the second only: its reduction over
 # the batch is one chain, whose truncation alone is 2e-3 after 270 000 images).
 @pytest.mark.parametrize("B,K,o", [(270000, 8192, 16), (4, 65536, 66000)])
