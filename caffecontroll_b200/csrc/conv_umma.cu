@@ -4,7 +4,8 @@
 // tensor memory).  The lowered matrix of the reference (type-1 lowering, one row of k*k*D values per output pixel)
 // is never written to global memory: producer threads gather each 128 x 32 tile of it straight from the NCHW
 // tensors, splitting every fp32 value into hi = its tf32 part and lo = x - hi on the way.  Three MMAs per k-step
-// (hi*hi + hi*lo + lo*hi) recover fp32-level accuracy ("3xTF32"); flops are counted once.
+// (hi*hi + hi*lo + lo*hi) recover fp32-level accuracy ("3xTF32"), or two where the cross terms are formed in bf16 (cross_word);
+// flops are counted once.
 //
 //   forward        Y[pix][o]   = sum_k  Lowered(X)[pix][k] * W[o][k]            (+ bias, optional ReLU)
 //   data gradient  dX[q][(d,py,px)] = sum_kk Gathered(dY)[q][kk] * Wd[(d,py,px)][kk]   kk = (filter, jy, jx)
@@ -239,7 +240,8 @@ __host__ __device__ inline GatherSmem gather_smem(int n_pad, int k_pad, int b_st
 // MODE: what the lanes gather - one table entry per reduction index, one per kRun of them, or (weight gradient) rows of the
 // lowered matrix over pixels.
 enum { kByTap = 0, kByRun = 1, kWeightGrad = 2 };
-template <int SETS, int MODE>
+// MIXED: cross terms in bf16 (cross_word), "lo" operands are their words; tiles of more than kCrossCols columns.
+template <int SETS, int MODE, bool MIXED>
 __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     gather_conv_kernel(const __grid_constant__ GatherParams P, const __grid_constant__ CUtensorMap w_map) {
   pdl_wait();
@@ -277,7 +279,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-  const uint32_t acc_cols = (uint32_t)acc_columns(P.n_pad), cross = acc_cols - (uint32_t)P.n_pad;  // cross: 0 = one accumulator
+  const uint32_t acc_cols = (uint32_t)acc_columns(P.n_pad), cross = MIXED ? 0u : acc_cols - (uint32_t)P.n_pad;  // cross: 0 = one accumulator
   const uint32_t a_col0 = (uint32_t)P.acc_bufs * acc_cols;
   const int kblocks = P.k_pad / kBlockK;
   bool failed = false;
@@ -422,7 +424,10 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       for (int c = 0; c < kBlockK / 8; ++c) {
         uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) split_tf32_trunc(v[c * 8 + e], hi[e], lo[e]);
+        for (int e = 0; e < 8; ++e) {
+          if (MIXED) split_mixed_a(v[c * 8 + e], hi[e], lo[e]);
+          else split_tf32_trunc(v[c * 8 + e], hi[e], lo[e]);
+        }
         tmem_st8(st_addr + (uint32_t)(c * 8), hi);
         tmem_st8(st_addr + 32u + (uint32_t)(c * 8), lo);
       }
@@ -443,7 +448,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issue (see elect_one)
-    const uint32_t idesc = make_idesc(P.n_pad), tmem = warp_uniform(tmem_base);
+    const uint32_t idesc = make_idesc(P.n_pad), idesc_cross = make_idesc_bf16(P.n_pad), tmem = warp_uniform(tmem_base);
     int tile_iter = 0;
     Ring ra, rb, rbar;  // A slot, weight slot, barrier pair of the current k-block
     for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x, ++tile_iter) {
@@ -458,13 +463,22 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         const uint64_t dbh = make_desc(b_hi), dbl = make_desc(b_lo);
         const uint32_t a_hi = tmem + a_col0 + (uint32_t)(ra.idx * 64), a_lo = a_hi + 32u;
         if (elect_one()) {
+          if (MIXED) {  // one accumulator; the second halves of the slot and of the weight tile are words of cross terms
 #pragma unroll
-          for (int j = 0; j < kBlockK / 8; ++j) {
-            const uint64_t adv = (uint64_t)(j * 2);
-            const uint32_t add = kb == 0 && j == 0 ? 0u : 1u;
-            umma_tf32_ts(d_cross, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, add);
-            umma_tf32_ts(d_cross, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
-            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, cross ? add : 1u);
+            for (int j = 0; j < kBlockK / 8; ++j)
+              umma_bf16_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbl + (uint64_t)(j * 2), idesc_cross, kb == 0 && j == 0 ? 0u : 1u);
+#pragma unroll
+            for (int j = 0; j < kBlockK / 8; ++j)
+              umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + (uint64_t)(j * 2), idesc, 1u);
+          } else {
+#pragma unroll
+            for (int j = 0; j < kBlockK / 8; ++j) {
+              const uint64_t adv = (uint64_t)(j * 2);
+              const uint32_t add = kb == 0 && j == 0 ? 0u : 1u;
+              umma_tf32_ts(d_cross, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, add);
+              umma_tf32_ts(d_cross, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
+              umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, cross ? add : 1u);
+            }
           }
           umma_commit(done_bar + 8u * rbar.idx);  // frees the A slot for the producers and the weight slot for the TMA thread
           if (kb == kblocks - 1) umma_commit(acc_full + 8u * buf);
@@ -1372,7 +1386,7 @@ __global__ void __launch_bounds__(32 * SLICES) wgrad_reduce_flat_kernel(const fl
 __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__ dY, float* __restrict__ hi,
                                                        float* __restrict__ lo, float* __restrict__ plane_sums,
                                                        int planes, int channels, int mm, int og, int ch_tile,
-                                                       int tiles_per_group, int n_pad, size_t row_len) {
+                                                       int tiles_per_group, int n_pad, size_t row_len, int mixed) {
   pdl_wait();
   // One warp per plane at a time, eight loads in flight per lane; no block-wide synchronisation.
   const int lane = threadIdx.x & 31;
@@ -1403,6 +1417,7 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
         const int i = i0 + u * 32 + lane;
         uint32_t h, l;
         split_tf32_trunc(x[u], h, l);
+        if (mixed) l = cross_word(__uint_as_float(l), x[u]);
         if (i >= 0 && i < mm) {
           dh[i] = __uint_as_float(h);
           dl[i] = __uint_as_float(l);
@@ -1437,10 +1452,13 @@ __global__ void bias_grad_kernel(const float* __restrict__ plane_sums, float* __
 // conv3's 0.9 M weights 8.0 / 11.6 us for the two operands, bound by neither memory nor launch).
 constexpr int kPackThreads = 128;
 
-__device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, const float* v) {
+__device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, const float* v, int mixed) {
   float h[4], l[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) split_tf32(v[e], h[e], l[e]);
+  for (int e = 0; e < 4; ++e) {
+    split_tf32(v[e], h[e], l[e]);
+    if (mixed) l[e] = __uint_as_float(cross_word(l[e], v[e]));
+  }
   *reinterpret_cast<float4*>(hi + at) = make_float4(h[0], h[1], h[2], h[3]);
   *reinterpret_cast<float4*>(lo + at) = make_float4(l[0], l[1], l[2], l[3]);
 }
@@ -1449,7 +1467,7 @@ __device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, co
 __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                 float* __restrict__ lo, int tiles_per_group, int og,
                                                                 int n_real, int n_pad, int k_real, int k_pad, int run,
-                                                                int window) {
+                                                                int window, int mixed) {
   pdl_wait();
   const int vg = blockIdx.x / n_pad, j = blockIdx.x - vg * n_pad;
   const int ch = (vg % tiles_per_group) * n_real + j;  // inside the group
@@ -1465,7 +1483,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
       const int at = run == 1 ? i : (chunk * run + (i - r * run)) * window + (r - chunk * window);
       v[e] = (live && i < k_real) ? __ldg(src + at) : 0.f;
     }
-    store_split4(hi, lo, row + kk, v);
+    store_split4(hi, lo, row + kk, v, mixed);
   }
 }
 
@@ -1475,7 +1493,8 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
 __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                   float* __restrict__ lo, int tiles_per_group, int og,
                                                                   int Dg, int k, int s, int taps, int d_tile,
-                                                                  int n_real, int n_pad, int k_real, int k_pad, int run) {
+                                                                  int n_real, int n_pad, int k_real, int k_pad, int run,
+                                                                  int mixed) {
   pdl_wait();
   const int vg = blockIdx.x / n_pad, j = blockIdx.x - vg * n_pad;
   const int grp = vg / tiles_per_group, d = (vg - grp * tiles_per_group) * d_tile + j / (s * s);
@@ -1493,7 +1512,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* _
       const int kr = py + jy * s, kc = px + jx * s;
       v[e] = (live && kk + e < k_real && kr < k && kc < k) ? __ldg(src + (size_t)oc * Dg * k * k + kr * k + kc) : 0.f;
     }
-    store_split4(hi, lo, row + kk, v);
+    store_split4(hi, lo, row + kk, v, mixed);
   }
 }
 
@@ -1603,6 +1622,7 @@ struct GatherProblem {
   int splits = 1, split_k = 0;    // splits of the reduction and the length of one (a multiple of 32; k_pad without splits)
   float* partial = nullptr;       // split sums
   size_t pix_pad = 0;
+  bool mixed = false;             // cross terms in bf16 (cross_word)
   int small_ct = 0;               // > 0: small_conv_kernel with this many channels per block instead of gather_conv_kernel
 };
 
@@ -1739,6 +1759,7 @@ void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias)
   if (two_ctas_per_sm(gp.n_pad, taps_smem, n_bias, ptab, &b_two)) {
     gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = acc <= 64 && !ptab ? 3 : 2; gp.b_stages = b_two;
   }
+  gp.mixed = gp.n_pad > kCrossCols && (gp.split_k ? gp.split_k : gp.k_pad) / kBlockK >= kMixedChain;  // see cross_word
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
   gp.w_half = (size_t)vgroups * gp.n_pad * map_k;
   mem.room(&gp.w, 2 * gp.w_half);
@@ -1996,9 +2017,11 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       rc = CCT_ERR_CUDA;
     }
   }
-  for (auto kernel : {gather_conv_kernel<4, kByTap>, gather_conv_kernel<4, kByRun>, gather_conv_kernel<4, kWeightGrad>})
+  for (auto kernel : {gather_conv_kernel<4, kByTap, false>, gather_conv_kernel<4, kByRun, false>, gather_conv_kernel<4, kWeightGrad, false>,
+                      gather_conv_kernel<4, kByTap, true>, gather_conv_kernel<4, kByRun, true>, gather_conv_kernel<4, kWeightGrad, true>})
     if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
-  for (auto kernel : {gather_conv_kernel<2, kByTap>, gather_conv_kernel<2, kByRun>, gather_conv_kernel<2, kWeightGrad>})
+  for (auto kernel : {gather_conv_kernel<2, kByTap, false>, gather_conv_kernel<2, kByRun, false>, gather_conv_kernel<2, kWeightGrad, false>,
+                      gather_conv_kernel<2, kByTap, true>, gather_conv_kernel<2, kByRun, true>, gather_conv_kernel<2, kWeightGrad, true>})
     if (rc == CCT_OK) rc = set_smem(ctx, kernel, 113 * 1024);
   if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad), kSmemLimit);
   if (p->w_ts)
@@ -2064,13 +2087,17 @@ void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp,
     const int grid = std::min(P.total_tiles, (sets == 2 ? 2 : 1) * ctx->launch_sms());
     launch_pdl(kernel, dim3(grid), dim3(gather_threads(sets)), gp.smem, ctx->stream, P, gp.map);
   };
-  if (weight_grad) {
-    if (gp.sets == 2) go(gather_conv_kernel<2, kWeightGrad>, 2); else go(gather_conv_kernel<4, kWeightGrad>, 4);
-  } else if (gp.run == kRun) {
-    if (gp.sets == 2) go(gather_conv_kernel<2, kByRun>, 2); else go(gather_conv_kernel<4, kByRun>, 4);
-  } else {
-    if (gp.sets == 2) go(gather_conv_kernel<2, kByTap>, 2); else go(gather_conv_kernel<4, kByTap>, 4);
-  }
+  auto pick = [&](auto mixed) {
+    constexpr bool M = decltype(mixed)::value;
+    if (weight_grad) {
+      if (gp.sets == 2) go(gather_conv_kernel<2, kWeightGrad, M>, 2); else go(gather_conv_kernel<4, kWeightGrad, M>, 4);
+    } else if (gp.run == kRun) {
+      if (gp.sets == 2) go(gather_conv_kernel<2, kByRun, M>, 2); else go(gather_conv_kernel<4, kByRun, M>, 4);
+    } else {
+      if (gp.sets == 2) go(gather_conv_kernel<2, kByTap, M>, 2); else go(gather_conv_kernel<4, kByTap, M>, 4);
+    }
+  };
+  if (gp.mixed) pick(std::true_type{}); else pick(std::false_type{});
   if (P.splits > 1) {
     const int vgroups = P.total_tiles / (P.n_pix_tiles * P.splits), cols = P.n_pix_tiles * vgroups * P.n > 32 * ctx->sm_count ? 8 : 1;
     const int col_tiles = (P.n + cols - 1) / cols;
@@ -2099,7 +2126,7 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
   if (repack) {
     t->begin(4, ctx->stream);
     launch_pdl(pack_fwd_kernel, pack_grid(vgroups * f.n_pad, f.k_pad), dim3(kPackThreads), 0, ctx->stream, W, f.w,
-               f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad, f.run, G.k * G.k);
+               f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad, f.run, G.k * G.k, (int)f.mixed);
     t->end(4, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   }
@@ -2144,7 +2171,7 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     t->begin(1, ctx->stream);
     launch_pdl(split_dy_kernel, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, 
         dY, w.w, w.w + w.w_half, G.bias ? p->wg_plane_sums : nullptr, G.B * G.o, G.o, mm, G.og, f.n, f.tiles,
-        f.n_pad, w.map_k);
+        f.n_pad, w.map_k, (int)w.mixed);
     CCT_CHECK_LAUNCH(ctx);
     GatherParams P{};
     P.in = X; P.out = p->w_partial; P.bias = nullptr;
@@ -2227,7 +2254,8 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
     }
     if (repack) {
       launch_pdl(pack_dgrad_kernel, pack_grid(vgroups * d.n_pad, d.k_pad), dim3(kPackThreads), 0, ctx->stream, W, d.w,
-                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run);
+                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run,
+                 (int)d.mixed);
       CCT_CHECK_LAUNCH(ctx);
     }
     GatherParams P{};

@@ -108,6 +108,41 @@ def test_accumulation_error(ctx, shape, which, chain):
     assert err <= 4 * chain * 2.0 ** -23.9 + 2.0 ** -21, "%s: relative error %.2e, chain of %d" % (which, err, chain)
 
 
+# Both sides of the lines behind which cross terms are bf16 (chains of 8 blocks of 32, more than 64 columns), reductions that are
+# no multiple of 32 or of eight channels, data of random sign.  Relative 2-norms: per product lo (below 2^-10 of x) is rounded to
+# eight bits, twice, of random sign: below 2^-19; the truncating additions as above, three per block at the most.
+@pytest.mark.parametrize("shape", [
+    (3, 224, 14, 80, 1, 1, 0, 1), (3, 256, 14, 80, 1, 1, 0, 1), (3, 257, 14, 65, 1, 1, 0, 1), (3, 264, 14, 64, 1, 1, 0, 1),
+    (5, 29, 15, 130, 3, 1, 1, 1), (2, 160, 17, 272, 3, 1, 1, 2), (4, 40, 19, 300, 5, 2, 2, 1),
+])
+def test_cross_terms_in_bf16(ctx, shape):
+    from caffecontroll_b200 import conv_layer
+    B, D, n, o, k, s, p, g = shape
+    m = (n + 2 * p - k) // s + 1
+    gen = torch.Generator().manual_seed(D + o)
+    X, W, dY = (torch.randn(sh, generator=gen) for sh in ((B, D, n, n), (o, D // g, k, k), (B, o, m, m)))
+    Y, dX, dW, db, used = conv_layer(ctx, X.numpy(), W.numpy(), np.zeros(o, np.float32), dY.numpy(), k, s, p, g, algo=TENSOR)
+    assert used == TENSOR
+    Xd, Wd, dYd = X.double().requires_grad_(), W.double().requires_grad_(), dY.double()
+    Yr = torch.nn.functional.conv2d(Xd, Wd, None, s, p, 1, g)
+    Yr.backward(dYd)
+    for got, ref, products in ((Y, Yr.detach(), D // g * k * k), (dX, Xd.grad, o // g * k * k), (dW, Wd.grad, B * m * m)):
+        err = float((torch.from_numpy(got).double() - ref).norm() / ref.norm())
+        assert err <= 4 * 3 * (products // 32 + 1) * 2.0 ** -23.9 + 2.0 ** -19, "relative error %.2e" % err
+
+
+def test_cross_terms_of_the_largest_values(ctx):
+    """The largest fp32 numbers, which bf16 would round to Inf, times small ones."""
+    from caffecontroll_b200 import conv_layer
+    B, D, n, o = 2, 320, 8, 96
+    rng = np.random.default_rng(5)
+    X = rng.choice(np.float32([3.4028234e38, -3.4e38, 1.0]), (B, D, n, n)).astype(np.float32)
+    W = (1e-12 * rng.standard_normal((o, D, 1, 1))).astype(np.float32)
+    Y = conv_layer(ctx, X, W, np.zeros(o, np.float32), None, 1, 1, 0, 1, algo=TENSOR)[0]
+    ref = np.einsum("bdyx,od->boyx", X.astype(np.float64), W[:, :, 0, 0].astype(np.float64))
+    assert np.isfinite(Y).all() and np.linalg.norm(Y / 1e26 - ref / 1e26) <= 1e-5 * np.linalg.norm(ref / 1e26)
+
+
 # Inner products: one product, features that are no multiple of four (padded copies or the fp32 kernel), both sides of the
 # line between the fp32 and the tensor-core kernel, batches at the accumulator widths of 64, 128 and 256 columns.
 # Tolerance: products of unit values summed over K: split operands leave 2^-20 of the sum of magnitudes, far below 1e-4.
