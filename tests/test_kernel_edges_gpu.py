@@ -167,6 +167,27 @@ def test_inner_product_sizes(ctx, B, K, o):
     fc.close()
 
 
+# Chains of eight blocks of 32 and more (cross terms in bf16): padded and ragged features, batches at the edges of the accumulator
+# widths.  Relative 2-norms: see test_cross_terms_in_bf16.
+@pytest.mark.parametrize("B,K,o", [(130, 2050, 4224), (70, 2304, 5000), (17, 4164, 4100), (256, 4608, 4608)])
+def test_inner_product_long_chains(ctx, B, K, o):
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    make = lambda *sh: torch.randn(sh, generator=gen, device="cuda")  # noqa: E731
+    X, W, b, dY = make(B, K), make(o, K), make(o), make(B, o)
+    Y, dX, dW, db = torch.zeros_like(dY), torch.zeros_like(X), torch.zeros_like(W), torch.zeros_like(b)
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(plan)), "plan", ctx.h)
+    capi.check(ctx.lib.cct_fc_forward(plan, q(X), q(W), q(b), q(Y), 0, None, 1.0), "forward", ctx.h)
+    capi.check(ctx.lib.cct_fc_backward(plan, q(X), q(W), q(dY), q(dX), q(dW), q(db), 0, None, 1.0), "backward", ctx.h)
+    ctx.sync()
+    ctx.lib.cct_fc_plan_destroy(plan)
+    Xd, Wd, dYd = X.double(), W.double(), dY.double()
+    for got, ref, products in ((Y, Xd @ Wd.T + b.double(), K), (dX, dYd @ Wd, o), (dW, dYd.T @ Xd, B)):
+        err = float((got.double() - ref).norm() / ref.norm())
+        assert err <= 4 * 3 * (min(products, 96 * 32) // 32 + 1) * 2.0 ** -23.9 + 2.0 ** -19, "relative error %.2e" % err
+
+
 # Operands four bytes off a 16-byte boundary, which no tensor map describes: all of them, or one at a time, with feature counts
 # that are and are not multiples of four, above the size of the fp32 kernel.  Tolerance as above.
 @pytest.mark.parametrize("B,K,o", [(129, 772, 1027), (129, 770, 1028), (130, 1024, 512), (40, 2051, 1030)])
