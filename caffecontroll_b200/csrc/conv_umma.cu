@@ -239,7 +239,11 @@ __host__ __device__ inline GatherSmem gather_smem(int n_pad, int k_pad, int b_st
 
 // MODE: what the lanes gather - one table entry per reduction index, one per kRun of them, or (weight gradient) rows of the
 // lowered matrix over pixels.
-enum { kByTap = 0, kByRun = 1, kWeightGrad = 2 };
+// kInside: one offset per reduction index (four to a shared-memory read) and no bounds test - a forward pass without padding,
+// whose windows lie inside the plane: 5.3 instructions per value instead of 9, AlexNet conv1 at batch 256 288 -> 270 us.  (Entries
+// behind the last real index read the window's first element against a weight of zero; lanes behind the last pixel read the last
+// pixel's window, their columns are not stored.)
+enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3 };
 // MIXED: cross terms in bf16 (cross_word), "lo" operands are their words; tiles of more than kCrossCols columns.
 template <int SETS, int MODE, bool MIXED>
 __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
@@ -264,7 +268,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   float* s_bias = reinterpret_cast<float*>(base_ptr + L.bias_off);
   const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
 
-  for (int i = tid; i < P.taps_smem; i += kGatherThreads) s_taps[i] = P.taps[i];
+  int* s_offsets = reinterpret_cast<int*>(s_taps);  // kInside: the offsets alone
+  for (int i = tid; i < P.taps_smem; i += kGatherThreads) {
+    if (MODE == kInside) s_offsets[i] = P.taps[i].off;
+    else s_taps[i] = P.taps[i];
+  }
   if (P.cols)
     for (int i = tid; i < P.n_pad; i += kGatherThreads) s_cols[i] = P.cols[i];
   for (int i = tid; i < P.n_bias + kBiasPad; i += kGatherThreads) s_bias[i] = i < P.n_bias ? P.bias[i] : 0.f;
@@ -307,6 +315,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     const float* in_px = P.in;
     uint32_t mask = 0;                   // forward / data gradient: which taps are in bounds for this lane's pixel
     const MaskTap* pix_tab = P.taps;     // weight gradient: this tile's slice of the per-pixel table
+    const int* tile_offsets = s_offsets;
     const MaskTap* tile_taps = s_taps;   // forward / data gradient: this tile's part of the tap table
     auto setup_tile = [&](int tile_local) {
       const int t = blockIdx.x + tile_local * gridDim.x;
@@ -328,6 +337,13 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         return;
       }
       tile_taps = s_taps + id.kb0 * (kBlockK / (MODE == kByRun ? kRun : 1));
+      if (MODE == kInside) {
+        tile_offsets = s_offsets + id.kb0 * kBlockK;
+        const int pix = min(id.ptile * kTileM + row, P.n_pix - 1), per_img = P.q_h * P.q_w;
+        const int b = pix / per_img, r = pix - b * per_img, qy = r / P.q_w, qx = r - qy * P.q_w;
+        in_px = P.in + (long long)b * P.in_batch_stride + (long long)grp * P.in_group_stride + (long long)(qy * P.iy_mul) * P.in_lim + qx * P.ix_mul;
+        return;
+      }
       const int pix = id.ptile * kTileM + row;
       mask = 0;  // which tap rows (bits 0-14) and tap columns (bits 16-30) fall inside the plane
       if (pix < P.n_pix) {
@@ -382,6 +398,18 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
           const int stride = ok ? P.run_stride : 0;
 #pragma unroll
           for (int e = 0; e < kRun; ++e) v[r * kRun + e] = __ldg(p + e * stride);
+        }
+        return;
+      }
+      if (MODE == kInside) {
+        const int4* tp = reinterpret_cast<const int4*>(tile_offsets + kb * kBlockK);
+#pragma unroll
+        for (int e = 0; e < kBlockK; e += 4) {
+          const int4 off = tp[e / 4];
+          v[e] = __ldg(in_px + off.x);
+          v[e + 1] = __ldg(in_px + off.y);
+          v[e + 2] = __ldg(in_px + off.z);
+          v[e + 3] = __ldg(in_px + off.w);
         }
         return;
       }
@@ -970,21 +998,30 @@ constexpr int kTsWideTaps = 13, kTsWideRows = 2;  // taps that four blocks cover
 
 __device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// A lowered value as the shared-memory operand of wgrad_ts_kernel.
+template <bool MIXED>
+__device__ __forceinline__ void split_lowered(float x, uint32_t& h, uint32_t& l) {
+  split_tf32_trunc(x, h, l);
+  if (MIXED) l = cross_word(__uint_as_float(l), x);
+}
+
 // Splits taps 0 .. k - 1, which start at w[SHIFT], and stores them as lowered rows: row r at dst + off[r & 7] + (r & ~7) * 128.
-template <int SHIFT>
+template <int SHIFT, bool MIXED>
 __device__ __forceinline__ void store_wide(const float* w, int k, uint8_t* dst, const uint32_t* off) {
 #pragma unroll
   for (int r = 0; r < kTsWideTaps; ++r) {
     if (r >= k) break;
     uint32_t h, l;
-    split_tf32_trunc(w[SHIFT + r], h, l);
+    split_lowered<MIXED>(w[SHIFT + r], h, l);
     uint8_t* at = dst + off[r & 7] + (r & ~7) * 128;
     *reinterpret_cast<uint32_t*>(at) = h;
     *reinterpret_cast<uint32_t*>(at + kTsTile) = l;
   }
 }
 
-template <bool WIDE>
+// MIXED (chains of kMixedChain and more): cross terms in bf16 (cross_word), "lo" operands are their words.  AlexNet conv1 at batch
+// 256 348 -> 346 us alone, 362 -> 349 within CaffeNet's iteration (the MMAs are not what bounds it, but take a third less power).
+template <bool WIDE, bool MIXED>
 __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __grid_constant__ WgradParams P) {
   constexpr int kTsTapWarps = ts_tap_warps(WIDE), kTsDyWarps = ts_dy_warps(WIDE), kTsMmaWarp = kTsTapWarps + kTsDyWarps;
   constexpr int kTsThreads = ts_threads(WIDE), kTsRowsPerWarp = kTsRows / 24;  // 16
@@ -1105,16 +1142,16 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
           if (i >= mine) break;
           uint8_t* dst = base_ptr + (size_t)s * kTsStage;
           switch ((int)warp_uniform((uint32_t)shift[i])) {
-            case 0: store_wide<0>(w[i], k, dst, lane_off[i]); break;
-            case 1: store_wide<1>(w[i], k, dst, lane_off[i]); break;
-            case 2: store_wide<2>(w[i], k, dst, lane_off[i]); break;
-            default: store_wide<3>(w[i], k, dst, lane_off[i]); break;
+            case 0: store_wide<0, MIXED>(w[i], k, dst, lane_off[i]); break;
+            case 1: store_wide<1, MIXED>(w[i], k, dst, lane_off[i]); break;
+            case 2: store_wide<2, MIXED>(w[i], k, dst, lane_off[i]); break;
+            default: store_wide<3, MIXED>(w[i], k, dst, lane_off[i]); break;
           }
         }
         if (ones >= 0) {
           uint8_t* dst = base_ptr + (size_t)s * kTsStage + ones * 128 + (((lane >> 2) ^ (ones & 7)) << 4) + (lane & 3) * 4;
           *reinterpret_cast<float*>(dst) = ok ? 1.f : 0.f;
-          *reinterpret_cast<float*>(dst + kTsTile) = 0.f;
+          *reinterpret_cast<uint32_t*>(dst + kTsTile) = MIXED && ok ? cross_word(0.f, 1.f) : 0u;
         }
         if (kbl + 1 < kblocks) {  // the next k-block's loads go in flight before the barrier work
           next_pixel();
@@ -1158,7 +1195,7 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
 #pragma unroll
         for (int i = 0; i < kTsRowsPerWarp; ++i) {
           uint32_t h, l;
-          split_tf32_trunc(va[i], h, l);
+          split_lowered<MIXED>(va[i], h, l);
           uint8_t* dst = st + i * (kTsTapWarps * 128);
           *reinterpret_cast<uint32_t*>(dst) = h;
           *reinterpret_cast<uint32_t*>(dst + kTsTile) = l;
@@ -1221,7 +1258,11 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
         for (int c = 0; c < kChannels / 8; ++c) {  // lane = channel now: its pixels, eight at a time
           uint32_t hi[8], lo[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) split_tf32_trunc(turn[lane * 33 + half * kChannels + c * 8 + e], hi[e], lo[e]);
+          for (int e = 0; e < 8; ++e) {
+            const float x = turn[lane * 33 + half * kChannels + c * 8 + e];
+            if (MIXED) split_mixed_a(x, hi[e], lo[e]);
+            else split_tf32_trunc(x, hi[e], lo[e]);
+          }
           tmem_st8(st_addr + (uint32_t)(c * 8), hi);
           tmem_st8(st_addr + 32u + (uint32_t)(c * 8), lo);
         }
@@ -1246,7 +1287,7 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
     }
   } else {
     // ------------------------------------------------------------------ MMA issue (see elect_one)
-    const uint32_t idesc = make_idesc(kTsNTile), tmem = warp_uniform(tmem_base);
+    const uint32_t idesc = make_idesc(kTsNTile), idesc_cross = make_idesc_bf16(kTsNTile), tmem = warp_uniform(tmem_base);
     Ring ring;
     for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(kTsStages)) {
       const int s = ring.idx;
@@ -1262,8 +1303,12 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
             const uint64_t adv = (uint64_t)(j * 2);
-            umma_tf32_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
-            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
+            if (MIXED) {
+              umma_bf16_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbl + adv, idesc_cross, (kbl == 0 && j == 0) ? 0u : 1u);
+            } else {
+              umma_tf32_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
+              umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
+            }
             umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, 1u);
           }
         }
@@ -1618,6 +1663,7 @@ struct GatherProblem {
   size_t map_k = 0;               // extent of the packed operand along the reduction (0: k_pad)
   size_t smem = 0;
   float* zero = nullptr;          // one 0.f, read by taps out of bounds
+  bool inside = false;            // kInside
   int run = 1, run_stride = 0;    // reduction order: 1 = (channel, tap); kRun = (channel / kRun, tap, channel % kRun)
   int splits = 1, split_k = 0;    // splits of the reduction and the length of one (a multiple of 32; k_pad without splits)
   float* partial = nullptr;       // split sums
@@ -1803,6 +1849,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     f.k_real = G.Dg * kk;
     f.k_pad = round_up(f.k_real, kBlockK);
     f.run = G.Dg % kRun == 0 ? kRun : 1; f.run_stride = G.n * G.n;
+    f.inside = f.run == 1 && G.p == 0;
     const long long pixel_tiles = ((long long)G.B * G.m * G.m + kTileM - 1) / kTileM;
     const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, f.run, G.s,
                                                  G.bias ? G.o : 0, chain_limit(G.og, 1, f.k_pad / kBlockK));
@@ -2018,14 +2065,16 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     }
   }
   for (auto kernel : {gather_conv_kernel<4, kByTap, false>, gather_conv_kernel<4, kByRun, false>, gather_conv_kernel<4, kWeightGrad, false>,
-                      gather_conv_kernel<4, kByTap, true>, gather_conv_kernel<4, kByRun, true>, gather_conv_kernel<4, kWeightGrad, true>})
+                      gather_conv_kernel<4, kByTap, true>, gather_conv_kernel<4, kByRun, true>, gather_conv_kernel<4, kWeightGrad, true>,
+                      gather_conv_kernel<4, kInside, false>, gather_conv_kernel<4, kInside, true>})
     if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
   for (auto kernel : {gather_conv_kernel<2, kByTap, false>, gather_conv_kernel<2, kByRun, false>, gather_conv_kernel<2, kWeightGrad, false>,
-                      gather_conv_kernel<2, kByTap, true>, gather_conv_kernel<2, kByRun, true>, gather_conv_kernel<2, kWeightGrad, true>})
+                      gather_conv_kernel<2, kByTap, true>, gather_conv_kernel<2, kByRun, true>, gather_conv_kernel<2, kWeightGrad, true>,
+                      gather_conv_kernel<2, kInside, false>, gather_conv_kernel<2, kInside, true>})
     if (rc == CCT_OK) rc = set_smem(ctx, kernel, 113 * 1024);
   if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad), kSmemLimit);
   if (p->w_ts)
-    for (auto kernel : {wgrad_ts_kernel<false>, wgrad_ts_kernel<true>})
+    for (auto kernel : {wgrad_ts_kernel<false, false>, wgrad_ts_kernel<true, false>, wgrad_ts_kernel<false, true>, wgrad_ts_kernel<true, true>})
       if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
   if (rc != CCT_OK) {
     umma_plan_destroy(ctx, p);
@@ -2093,6 +2142,8 @@ void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp,
       if (gp.sets == 2) go(gather_conv_kernel<2, kWeightGrad, M>, 2); else go(gather_conv_kernel<4, kWeightGrad, M>, 4);
     } else if (gp.run == kRun) {
       if (gp.sets == 2) go(gather_conv_kernel<2, kByRun, M>, 2); else go(gather_conv_kernel<4, kByRun, M>, 4);
+    } else if (gp.inside) {
+      if (gp.sets == 2) go(gather_conv_kernel<2, kInside, M>, 2); else go(gather_conv_kernel<4, kInside, M>, 4);
     } else {
       if (gp.sets == 2) go(gather_conv_kernel<2, kByTap, M>, 2); else go(gather_conv_kernel<4, kByTap, M>, 4);
     }
@@ -2220,7 +2271,10 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       // Wide loads: see the kernel.  Below eight taps a window row has fewer than three blocks' worth.
       P.x_count = (int)((long long)G.B * G.D * G.n * G.n - (G.g - 1) * P.x_group_stride);
       const bool wide = G.s % 4 == 0 && G.p == 0 && G.k >= 8 && G.k <= kTsWideTaps && G.Dg * G.k <= kTsWideRows * ts_tap_warps(true);
-      launch_pdl(wide ? wgrad_ts_kernel<true> : wgrad_ts_kernel<false>, dim3(grid), dim3(ts_threads(wide)), p->w_smem, ctx->stream, P);
+      const bool mixed = P.kblocks_per_split >= kMixedChain;
+      const auto kernel = wide ? (mixed ? wgrad_ts_kernel<true, true> : wgrad_ts_kernel<true, false>)
+                               : (mixed ? wgrad_ts_kernel<false, true> : wgrad_ts_kernel<false, false>);
+      launch_pdl(kernel, dim3(grid), dim3(ts_threads(wide)), p->w_smem, ctx->stream, P);
     }
     else
       launch_pdl(wgrad_pick(p->w_subs, f.n_pad), dim3(grid), dim3(kWgThreads), p->w_smem, ctx->stream, P);

@@ -64,6 +64,30 @@ def test_a_gradient_that_is_not_finite_stays_in_its_window(ctx, shape, value):
     assert np.array_equal(dX[~window], clean[~window])
 
 
+# Forward passes without padding (no bounds test on the gathered operand), reductions that end inside a block of 32, fewer pixels
+# than a tile, groups; and one with padding.
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("shape", [(1, 3, 11, 8, 11, 4, 0, 1), (3, 3, 47, 96, 11, 4, 0, 1), (2, 10, 15, 130, 3, 1, 0, 2), (5, 7, 12, 70, 2, 2, 0, 1),
+                                   (9, 33, 9, 80, 1, 1, 0, 1), (2, 3, 20, 72, 7, 2, 3, 1)])
+def test_an_input_that_is_not_finite_stays_in_its_windows(ctx, shape, value):
+    """Y outside the windows that hold one element of X does not depend on that element: bit for bit."""
+    from caffecontroll_b200 import conv_layer
+    B, D, n, o, k, s, p, g = shape
+    X, W, b, _ = make_inputs(41, B, D, n, o, k, s, p, g)
+    W = np.where(W == 0, np.float32(0.01), W)
+    m = (n + 2 * p - k) // s + 1
+    where = (B - 1, 0, n // 2, n // 2)
+    X[where] = 0
+    clean = conv_layer(ctx, X, W, b, None, k, s, p, g, algo=TENSOR)[0]
+    X[where] = value
+    Y = conv_layer(ctx, X, W, b, None, k, s, p, g, algo=TENSOR)[0]
+    inside = [r * s - p <= n // 2 < r * s - p + k for r in range(m)]
+    window = np.zeros(Y.shape, bool)
+    window[B - 1, :o // g] = np.outer(inside, inside)
+    assert np.array_equal(~np.isfinite(Y), window)
+    assert np.array_equal(Y[~window], clean[~window])
+
+
 @pytest.mark.parametrize("algo", [capi.ALGO_AUTO, TENSOR])
 def test_many_groups(ctx, port, algo):
     """4096 groups of one channel are 65 536 rows of a packed operand; 65 600 groups (forward only) are more channel tiles than a
