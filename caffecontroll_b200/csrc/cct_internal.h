@@ -129,7 +129,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 
 // Optional per-kernel-group timing with CUDA events on the context's stream (measurement only).
 struct PhaseTimer {
-  static constexpr int kSlots = 5;  // 0 forward, 1 wgrad, 2 wgrad reduce, 3 dgrad (with its repacking), 4 forward repack
+  static constexpr int kSlots = 5;  // 0 forward, 1 wgrad, 2 wgrad reduce (with the repacking for dgrad), 3 dgrad, 4 forward repack
   bool enabled = false;
   cudaEvent_t ev[2 * kSlots] = {};
   bool have[kSlots] = {};
@@ -167,12 +167,14 @@ void umma_plan_destroy(cct_ctx* ctx, UmmaPlan* p);
 size_t umma_plan_workspace_bytes(const UmmaPlan* p);
 bool umma_supported(const ConvGeom& G);
 // `batch` > 0 restricts a call to the first `batch` images of the tensors it is given; `repack` = rewrite the packed
-// weight operand from W first (needed once per new W).
+// weight operand from W first (needed once per new W).  `pack_W`: the weight gradient's last launch does that for the data
+// gradient.
 int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* bias, float* Y,
                       int relu, PhaseTimer* t, int batch = 0, bool repack = true);
 int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dY, float* dX,
                        float* dW, float* db, PhaseTimer* t);
-int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t);
+int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t,
+                    const float* pack_W = nullptr);
 int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, float* dX, PhaseTimer* t, int batch,
                     bool repack);
 

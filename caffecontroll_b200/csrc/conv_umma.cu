@@ -83,17 +83,6 @@ __device__ __forceinline__ float ldg_if_clear(const float* p, uint32_t a, uint32
       : "l"(p), "r"(a), "r"(b));
   return v;
 }
-// p[i * stride], the address as one multiply-add.
-__device__ __forceinline__ float ldg_at(const float* p, int i, int stride) {
-  float v;
-  asm volatile(
-      "{\n\t.reg .b64 a;\n\t"
-      "mad.wide.s32 a, %2, %3, %1;\n\t"
-      "ld.global.nc.f32 %0, [a];\n\t}"
-      : "=f"(v)
-      : "l"(p), "r"(stride), "r"(i * 4));
-  return v;
-}
 // v = flag ? *p : 0, same form.
 __device__ __forceinline__ float ldg_if(const float* p, uint32_t flag) {
   float v;
@@ -1346,17 +1335,113 @@ WgradKernel wgrad_pick(int subs, int n_pad) {
 #include "conv_small.cuh"
 namespace {
 
+// ------------------------------------------------------------------------------------------ weight packing
+// A block writes one row of the packed operand (blockIdx.x = (vg, j): there may be more than 65 535 of them), four consecutive
+// reduction indices per thread and step: one decode per four elements and 16-byte stores (a flat grid-stride loop spent most of its time dividing: CaffeNet
+// conv3's 0.9 M weights 8.0 / 11.6 us for the two operands, bound by neither memory nor launch).
+constexpr int kPackThreads = 128;
+
+template <bool MIXED>
+__device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, const float* v) {
+  float h[4], l[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    split_tf32(v[e], h[e], l[e]);
+    if (MIXED) l[e] = __uint_as_float(cross_word(l[e], v[e]));
+  }
+  *reinterpret_cast<float4*>(hi + at) = make_float4(h[0], h[1], h[2], h[3]);
+  *reinterpret_cast<float4*>(lo + at) = make_float4(l[0], l[1], l[2], l[3]);
+}
+
+// Data-gradient B operand: [2][vg][n_pad][k_pad]; row j = (d, py, px) of channel tile nt of group g (py, px: position
+// inside a block of s x s input pixels), column kk = (oc, jy, jx) <- W[g*og + oc][d][py + jy*s][px + jx*s], zero where the tap
+// index is outside the kernel.
+struct PackDgrad {
+  const float* W;
+  float *hi, *lo;
+  int tiles_per_group, og, Dg, k, s, taps, d_tile, n_real, n_pad, k_real, k_pad, run, mixed;
+  int parts;   // blocks per row
+  int blocks;  // rows * parts
+};
+__device__ __forceinline__ void pack_dgrad_block(const PackDgrad& J, int block) {
+  const int r0 = block / J.parts, part = block - r0 * J.parts;
+  const int vg = r0 / J.n_pad, j = r0 - vg * J.n_pad;
+  const int grp = vg / J.tiles_per_group, d = (vg - grp * J.tiles_per_group) * J.d_tile + j / (J.s * J.s);
+  const int py = (j / J.s) % J.s, px = j % J.s, window = J.taps * J.taps;
+  const bool live = j < J.n_real && d < J.Dg;
+  const float* src = J.W + ((size_t)grp * J.og * J.Dg + d) * J.k * J.k;
+  const size_t row = (size_t)r0 * J.k_pad;
+  for (int kk = (part * (int)blockDim.x + (int)threadIdx.x) * 4; kk < J.k_pad; kk += J.parts * (int)blockDim.x * 4) {
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      // reduction index -> (filter / run, jy, jx, filter % run)
+      const int r = (kk + e) / J.run, chunk = r / window, tap = r - chunk * window;
+      const int oc = chunk * J.run + (kk + e - r * J.run), jy = tap / J.taps, jx = tap - jy * J.taps;
+      const int kr = py + jy * J.s, kc = px + jx * J.s;
+      v[e] = (live && kk + e < J.k_real && kr < J.k && kc < J.k) ? __ldg(src + (size_t)oc * J.Dg * J.k * J.k + kr * J.k + kc) : 0.f;
+    }
+    if (J.mixed) store_split4<true>(J.hi, J.lo, row + kk, v);
+    else store_split4<false>(J.hi, J.lo, row + kk, v);
+  }
+}
+__global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const __grid_constant__ PackDgrad J) {
+  pdl_wait();
+  pack_dgrad_block(J, blockIdx.x);
+}
+
+// db[c] = sum over the batch of the plane sums (ConvolutionBridge_impl.hxx:575-599), in a fixed order.
+struct BiasSum {
+  const float* plane_sums;
+  float* db;
+  int batch, channels;
+  int blocks;
+};
+__device__ __forceinline__ void bias_grad_block(const BiasSum& J, int block) {
+  // one warp per channel: lane l adds images l, l + 32, ... in order, then a fixed shuffle tree
+  const int c = (int)((block * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (c >= J.channels) return;
+  float t = 0.f;
+  for (int b = lane; b < J.batch; b += 32) t += J.plane_sums[(size_t)b * J.channels + c];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) J.db[c] = t;
+}
+
+// What else goes between the weight gradient and the data gradient of a layer, in blocks behind those that add the split sums:
+// the weights are packed for the data gradient, the plane sums of dY are added to the bias gradient.  In launches of their own
+// they were 2 - 7 and 2 - 3 us each, most of it the launch: ragged layer of 37 images 42.5 -> 40.5 us, CaffeNet's iteration at
+// batch 32 1 214 -> 1 196.
+struct ReduceExtras {
+  PackDgrad pack;
+  BiasSum bias;
+};
+// True if this block was one of them; `first` of the grid's x are not.
+__device__ __forceinline__ bool extra_block(const ReduceExtras& E, int first) {
+  int block = (int)blockIdx.x - first;
+  if (block < 0) return false;
+  if (block < E.pack.blocks) {
+    pack_dgrad_block(E.pack, block);
+    return true;
+  }
+  block -= E.pack.blocks;
+  if (block < E.bias.blocks) bias_grad_block(E.bias, block);
+  return true;
+}
+
 // dW[o][kk] and db[o] from the split partial sums, added in split order (deterministic).  One block per 32 x 32
 // tile of (kk, channel): the partial sums are read along the channels (their fastest index), the tile is turned in
 // shared memory, and dW is written along kk (its fastest index) - both sides coalesced, no division per element.
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dW,
                                                            float* __restrict__ db, int splits, int vgroups,
                                                            int tiles_per_group, int rows_pad, int n_real, int n_pad,
-                                                           int k_real, int og, int accumulate) {
+                                                           int k_real, int og, int accumulate, int row_tiles, int col_tiles,
+                                                           const __grid_constant__ ReduceExtras extras) {
   pdl_wait();
   __shared__ float tile[32][33];
-  const int vg = blockIdx.z;
-  const int kk0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+  if (extra_block(extras, row_tiles * col_tiles * vgroups)) return;
+  const int across = blockIdx.x / row_tiles, vg = across / col_tiles;
+  const int kk0 = (blockIdx.x - across * row_tiles) * 32, j0 = (across - vg * col_tiles) * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
   const int ch0 = (vg / tiles_per_group) * og + (vg % tiles_per_group) * n_real;
   n_real = min(n_real, og - (vg % tiles_per_group) * n_real);  // the last channel tile of a group may be shorter
@@ -1394,11 +1479,13 @@ __global__ void __launch_bounds__(32 * SLICES) wgrad_reduce_flat_kernel(const fl
                                                                         float* __restrict__ dW, float* __restrict__ db,
                                                                         int splits, int vgroups, int tiles_per_group,
                                                                         int rows_pad, int n_real, int n_pad, int k_real,
-                                                                        int og, int accumulate) {
+                                                                        int og, int accumulate, int per_group,
+                                                                        const __grid_constant__ ReduceExtras extras) {
   pdl_wait();
   __shared__ float part[SLICES][33];
+  if (extra_block(extras, per_group * vgroups)) return;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int vg = blockIdx.y, e = blockIdx.x * 32 + tx;  // e = kk * n_pad + channel
+  const int vg = blockIdx.x / per_group, e = (blockIdx.x - vg * per_group) * 32 + tx;  // e = kk * n_pad + channel
   const size_t split_stride = (size_t)vgroups * rows_pad * n_pad;
   const bool in = e < (k_real + 1) * n_pad;
   float acc = 0.f;
@@ -1478,41 +1565,12 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
   }
 }
 
-// db[c] = sum over the batch of the plane sums (ConvolutionBridge_impl.hxx:575-599), in a fixed order.
-__global__ void bias_grad_kernel(const float* __restrict__ plane_sums, float* __restrict__ db, int batch, int channels) {
-  pdl_wait();
-  // one warp per channel: lane l adds images l, l + 32, ... in order, then a fixed shuffle tree
-  const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (c >= channels) return;
-  float t = 0.f;
-  for (int b = lane; b < batch; b += 32) t += plane_sums[(size_t)b * channels + c];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (lane == 0) db[c] = t;
-}
-
-// ------------------------------------------------------------------------------------------ weight packing
-// A block writes one row of the packed operand (blockIdx.x = (vg, j): there may be more than 65 535 of them), four consecutive
-// reduction indices per thread and step: one decode per four elements and 16-byte stores (a flat grid-stride loop spent most of its time dividing: CaffeNet
-// conv3's 0.9 M weights 8.0 / 11.6 us for the two operands, bound by neither memory nor launch).
-constexpr int kPackThreads = 128;
-
-__device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, const float* v, int mixed) {
-  float h[4], l[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    split_tf32(v[e], h[e], l[e]);
-    if (mixed) l[e] = __uint_as_float(cross_word(l[e], v[e]));
-  }
-  *reinterpret_cast<float4*>(hi + at) = make_float4(h[0], h[1], h[2], h[3]);
-  *reinterpret_cast<float4*>(lo + at) = make_float4(l[0], l[1], l[2], l[3]);
-}
-
 // Forward B operand: [2 (hi, lo)][vg][n_pad][k_pad] <- W[o][Dg*k*k], zero padded.
+template <bool MIXED>
 __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                 float* __restrict__ lo, int tiles_per_group, int og,
                                                                 int n_real, int n_pad, int k_real, int k_pad, int run,
-                                                                int window, int mixed) {
+                                                                int window) {
   pdl_wait();
   const int vg = blockIdx.x / n_pad, j = blockIdx.x - vg * n_pad;
   const int ch = (vg % tiles_per_group) * n_real + j;  // inside the group
@@ -1528,36 +1586,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
       const int at = run == 1 ? i : (chunk * run + (i - r * run)) * window + (r - chunk * window);
       v[e] = (live && i < k_real) ? __ldg(src + at) : 0.f;
     }
-    store_split4(hi, lo, row + kk, v, mixed);
-  }
-}
-
-// Data-gradient B operand: [2][vg][n_pad][k_pad]; row j = (d, py, px) of channel tile nt of group g (py, px: position
-// inside a block of s x s input pixels), column kk = (oc, jy, jx) <- W[g*og + oc][d][py + jy*s][px + jx*s], zero where the tap
-// index is outside the kernel.
-__global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const float* __restrict__ W, float* __restrict__ hi,
-                                                                  float* __restrict__ lo, int tiles_per_group, int og,
-                                                                  int Dg, int k, int s, int taps, int d_tile,
-                                                                  int n_real, int n_pad, int k_real, int k_pad, int run,
-                                                                  int mixed) {
-  pdl_wait();
-  const int vg = blockIdx.x / n_pad, j = blockIdx.x - vg * n_pad;
-  const int grp = vg / tiles_per_group, d = (vg - grp * tiles_per_group) * d_tile + j / (s * s);
-  const int py = (j / s) % s, px = j % s, window = taps * taps;
-  const bool live = j < n_real && d < Dg;
-  const float* src = W + ((size_t)grp * og * Dg + d) * k * k;
-  const size_t row = (size_t)blockIdx.x * k_pad;
-  for (int kk = (blockIdx.y * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.y * kPackThreads * 4) {
-    float v[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      // reduction index -> (filter / run, jy, jx, filter % run)
-      const int r = (kk + e) / run, chunk = r / window, tap = r - chunk * window;
-      const int oc = chunk * run + (kk + e - r * run), jy = tap / taps, jx = tap - jy * taps;
-      const int kr = py + jy * s, kc = px + jx * s;
-      v[e] = (live && kk + e < k_real && kr < k && kc < k) ? __ldg(src + (size_t)oc * Dg * k * k + kr * k + kc) : 0.f;
-    }
-    store_split4(hi, lo, row + kk, v, mixed);
+    store_split4<MIXED>(hi, lo, row + kk, v);
   }
 }
 
@@ -1747,22 +1776,27 @@ int set_smem(cct_ctx* ctx, K kernel, size_t bytes) {
   return CCT_OK;
 }
 
-// Split reduction: tiles when they fill the machine, the flat form otherwise (both add in a fixed order).
+// Split reduction: tiles when they fill the machine, the flat form otherwise (both add in a fixed order).  `extras`: see there;
+// their block counts are set here, for the block size that is taken.
 void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* db, int splits, int vgroups,
                          int tiles_per_group, int rows_pad, int n_real, int n_pad, int k_real, int og,
-                         int accumulate = 0) {
-  const dim3 tiles((k_real + 1 + 31) / 32, (n_real + 31) / 32, vgroups);
-  if ((int)(tiles.x * tiles.y * tiles.z) >= ctx->sm_count)
-    launch_pdl(wgrad_reduce_kernel, dim3(tiles), dim3(256), 0, ctx->stream, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad,
-                                                       n_real, n_pad, k_real, og, accumulate);
+                         int accumulate = 0, ReduceExtras extras = ReduceExtras()) {
+  auto extra_blocks = [&](int threads) {
+    if (extras.bias.db) extras.bias.blocks = (extras.bias.channels + threads / 32 - 1) / (threads / 32);
+    return extras.pack.blocks + extras.bias.blocks;
+  };
+  const int row_tiles = (k_real + 1 + 31) / 32, col_tiles = (n_real + 31) / 32;
+  if (row_tiles * col_tiles * vgroups >= ctx->sm_count)
+    launch_pdl(wgrad_reduce_kernel, dim3(row_tiles * col_tiles * vgroups + extra_blocks(256)), dim3(256), 0, ctx->stream, partial, dW, db,
+               splits, vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate, row_tiles, col_tiles, extras);
   else {
-    const dim3 grid(((k_real + 1) * n_pad + 31) / 32, vgroups);
+    const int per_group = ((k_real + 1) * n_pad + 31) / 32;
     auto go = [&](auto kernel, int slices) {
-      launch_pdl(kernel, grid, dim3(32 * slices), 0, ctx->stream, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real,
-                 n_pad, k_real, og, accumulate);
+      launch_pdl(kernel, dim3(per_group * vgroups + extra_blocks(32 * slices)), dim3(32 * slices), 0, ctx->stream, partial, dW, db, splits,
+                 vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate, per_group, extras);
     };
     if (splits < 16) go(wgrad_reduce_flat_kernel<4>, 4);
-    else if (splits < 64 || grid.x * grid.y > 2u * ctx->sm_count) go(wgrad_reduce_flat_kernel<8>, 8);
+    else if (splits < 64 || per_group * vgroups > 2 * ctx->sm_count) go(wgrad_reduce_flat_kernel<8>, 8);
     else go(wgrad_reduce_flat_kernel<32>, 32);
   }
 }
@@ -2112,6 +2146,15 @@ void fill_common(GatherParams& P, const GatherProblem& gp, cct_ctx* ctx, int vgr
   P.status = ctx->status_dev;
 }
 
+PackDgrad pack_dgrad_job(const UmmaPlan* p, const float* W) {
+  const ConvGeom& G = p->G;
+  const GatherProblem& d = p->dgr;
+  PackDgrad J{W, d.w, d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run, (int)d.mixed, 0, 0};
+  J.parts = (d.k_pad / 4 + kPackThreads - 1) / kPackThreads;
+  J.blocks = G.g * d.tiles * d.n_pad * J.parts;
+  return J;
+}
+
 void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct) {
   const int jr = small_rows(k);
   P.row_groups = (P.n_out + jr - 1) / jr;
@@ -2176,8 +2219,8 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
   }
   if (repack) {
     t->begin(4, ctx->stream);
-    launch_pdl(pack_fwd_kernel, pack_grid(vgroups * f.n_pad, f.k_pad), dim3(kPackThreads), 0, ctx->stream, W, f.w,
-               f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad, f.run, G.k * G.k, (int)f.mixed);
+    launch_pdl(f.mixed ? pack_fwd_kernel<true> : pack_fwd_kernel<false>, pack_grid(vgroups * f.n_pad, f.k_pad), dim3(kPackThreads), 0, ctx->stream, W, f.w,
+               f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad, f.run, G.k * G.k);
     t->end(4, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   }
@@ -2206,15 +2249,18 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
 
 int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dY, float* dX,
                        float* dW, float* db, PhaseTimer* t) {
-  int rc = umma_conv_wgrad(ctx, p, X, dY, dW, db, t);
-  if (rc == CCT_OK && dX) rc = umma_conv_dgrad(ctx, p, W, dY, dX, t, 0, true);
+  int rc = umma_conv_wgrad(ctx, p, X, dY, dW, db, t, dX ? W : nullptr);
+  if (rc == CCT_OK && dX) rc = umma_conv_dgrad(ctx, p, W, dY, dX, t, 0, false);
   return rc;
 }
 
-// Weight + bias gradient over the whole batch.
-int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t) {
+// Weight + bias gradient over the whole batch; `pack_W`: the weights to pack for the data gradient on the way.
+int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t,
+                    const float* pack_W) {
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   const ConvGeom& G = p->G;
+  ReduceExtras extras{};
+  if (pack_W && !p->dgr.small_ct) extras.pack = pack_dgrad_job(p, pack_W);
   if (p->wg_gather) {
     struct { int tiles, n, n_pad, k_real; } f = {p->wt_tiles, p->wt_n, p->w_npad, p->fwd.k_real};
     GatherProblem& w = p->wgp;
@@ -2237,10 +2283,10 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     launch_gather(ctx, P, w, true);
     t->end(1, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
+    if (G.bias) extras.bias = BiasSum{p->wg_plane_sums, db, G.B, G.o, 0};
     t->begin(2, ctx->stream);
     launch_wgrad_reduce(ctx, p->w_partial, dW, nullptr, p->wg_splits, vgroups, f.tiles, p->wg_mtiles * kTileM, f.n,
-                        f.n_pad, f.k_real, G.og);
-    if (G.bias) launch_pdl(bias_grad_kernel, dim3((G.o + 7) / 8), dim3(256), 0, ctx->stream, p->wg_plane_sums, db, G.B, G.o);
+                        f.n_pad, f.k_real, G.og, 0, extras);
     t->end(2, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   } else {
@@ -2282,7 +2328,7 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     CCT_CHECK_LAUNCH(ctx);
     t->begin(2, ctx->stream);
     launch_wgrad_reduce(ctx, p->w_partial, dW, G.bias ? db : nullptr, p->w_splits, vgroups, f.tiles, rows_pad, f.n, P.n_pad,
-                        f.k_real, G.og);
+                        f.k_real, G.og, 0, extras);
     t->end(2, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   }
@@ -2307,9 +2353,8 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
       return CCT_OK;
     }
     if (repack) {
-      launch_pdl(pack_dgrad_kernel, pack_grid(vgroups * d.n_pad, d.k_pad), dim3(kPackThreads), 0, ctx->stream, W, d.w,
-                 d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run,
-                 (int)d.mixed);
+      const PackDgrad J = pack_dgrad_job(p, W);
+      launch_pdl(pack_dgrad_kernel, dim3(J.blocks), dim3(kPackThreads), 0, ctx->stream, J);
       CCT_CHECK_LAUNCH(ctx);
     }
     GatherParams P{};

@@ -349,6 +349,46 @@ __global__ void __launch_bounds__(kFcThreads, 2)
   if (warp == 0) tmem_dealloc(tmem_base, (uint32_t)P.tmem_cols);
 }
 
+// db[o] = sum_b dY[b][o] (FullyConnectedBridge_impl.hxx:298: backward_bias_fc).  A block of 32 x 8 threads owns 32
+// outputs: thread (x, y) adds the images y, y + 8, ... in order with sixteen loads in flight, then the eight partial sums
+// of an output are added in a fixed order - deterministic, and two memory round trips instead of B.
+struct FcBiasSum {
+  const float* dY;
+  float* db;
+  int B, O;
+};
+__device__ __forceinline__ void fc_bias_grad_block(const FcBiasSum& J, int block) {
+  __shared__ float part[8][33];
+  const float* dY = J.dY;
+  const int B = J.B, O = J.O;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int o = block * 32 + tx;
+  float acc = 0.f;
+  if (o < O) {
+    int b = ty;
+    for (; b + 8 * 15 < B; b += 8 * 16) {
+      float v[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = __ldg(dY + (size_t)(b + 8 * j) * O + o);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) acc += v[j];
+    }
+    for (; b < B; b += 8) acc += dY[(size_t)b * O + o];
+  }
+  part[ty][tx] = acc;
+  __syncthreads();
+  if (ty == 0 && o < O) {
+    float t = part[0][tx];
+#pragma unroll
+    for (int y = 1; y < 8; ++y) t += part[y][tx];
+    J.db[o] = t;
+  }
+}
+__global__ void __launch_bounds__(256) fc_bias_grad_kernel(const __grid_constant__ FcBiasSum J) {
+  pdl_wait();
+  fc_bias_grad_block(J, blockIdx.x);
+}
+
 // Sums the splits of a contraction in split order and applies what surrounds it, VEC columns of a row per thread.
 //   forward        Y[b][o] = act(bias[o] + sum), act = optional ReLU then optional dropout (DropoutBridge forward:
 //                  x * mask * scale, src/bridges/DropoutBridge_impl.hxx:71-74)
@@ -362,12 +402,20 @@ struct FcReduceParams {
   const uint32_t* drop_mask;
   float drop_scale;
   int rows, cols, pitch, splits, relu;
+  // data gradient: the layer's bias gradient in blocks behind the others (a launch less; `sum_blocks` of the grid are not)
+  unsigned sum_blocks = 0;
+  FcBiasSum bias_sum{};
 };
 // SLICES > 1: a block's eight warps take interleaved slices of the splits of the same 32 x VEC elements and add them in a
 // fixed order - small outputs with many splits, where one thread per element would be a long chain on a few SMs.
-template <int VEC, int SLICES>
+// BIAS: blocks behind the others add the layer's bias gradient (data gradient).
+template <int VEC, int SLICES, bool BIAS>
 __global__ void __launch_bounds__(256) fc_reduce_kernel(const __grid_constant__ FcReduceParams P) {
   pdl_wait();
+  if (BIAS && blockIdx.x >= P.sum_blocks) {
+    fc_bias_grad_block(P.bias_sum, (int)(blockIdx.x - P.sum_blocks));
+    return;
+  }
   __shared__ float part[SLICES > 1 ? SLICES : 1][VEC][33];
   const int per_row = (P.cols + VEC - 1) / VEC;
   const int lane = threadIdx.x & 31, slice = SLICES > 1 ? threadIdx.x >> 5 : 0;
@@ -419,36 +467,6 @@ __global__ void __launch_bounds__(256) fc_pad_kernel(const float* __restrict__ s
   for (int r = blockIdx.y; r < rows; r += gridDim.y)
     for (int c = blockIdx.x * 256 + threadIdx.x; c < pitch; c += gridDim.x * 256)
       dst[(size_t)r * pitch + c] = c < cols ? __ldg(src + (size_t)r * cols + c) : 0.f;
-}
-
-// db[o] = sum_b dY[b][o] (FullyConnectedBridge_impl.hxx:298: backward_bias_fc).  A block of 32 x 8 threads owns 32
-// outputs: thread (x, y) adds the images y, y + 8, ... in order with sixteen loads in flight, then the eight partial sums
-// of an output are added in a fixed order - deterministic, and two memory round trips instead of B.
-__global__ void __launch_bounds__(256) fc_bias_grad_kernel(const float* __restrict__ dY, float* __restrict__ db, int B, int O) {
-  pdl_wait();
-  __shared__ float part[8][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int o = blockIdx.x * 32 + tx;
-  float acc = 0.f;
-  if (o < O) {
-    int b = ty;
-    for (; b + 8 * 15 < B; b += 8 * 16) {
-      float v[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = __ldg(dY + (size_t)(b + 8 * j) * O + o);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) acc += v[j];
-    }
-    for (; b < B; b += 8) acc += dY[(size_t)b * O + o];
-  }
-  part[ty][tx] = acc;
-  __syncthreads();
-  if (ty == 0 && o < O) {
-    float t = part[0][tx];
-#pragma unroll
-    for (int y = 1; y < 8; ++y) t += part[y][tx];
-    db[o] = t;
-  }
 }
 
 int fc_round_up(int v, int a) { return (v + a - 1) / a * a; }
@@ -648,13 +666,19 @@ int fc_small_pass_splits(const cct_fc_plan* plan, int wanted, const FcShape& ten
   return plan->small ? wanted : std::min(wanted, tensor.P.splits);
 }
 
-int fc_reduce(cct_ctx* ctx, const FcReduceParams& R) {
+int fc_reduce(cct_ctx* ctx, FcReduceParams R) {
   const bool vec = R.cols % 4 == 0 && fc_aligned({R.partial, R.out});
   const long long threads = (long long)R.rows * (vec ? R.cols / 4 : R.cols);
   const bool slices = R.splits >= 8 && threads < 256ll * ctx->sm_count;
-  auto kernel = slices ? (vec ? fc_reduce_kernel<4, 8> : fc_reduce_kernel<1, 8>) : (vec ? fc_reduce_kernel<4, 1> : fc_reduce_kernel<1, 1>);
+  auto pick = [&](auto bias) {
+    constexpr bool kBias = decltype(bias)::value;
+    return slices ? (vec ? fc_reduce_kernel<4, 8, kBias> : fc_reduce_kernel<1, 8, kBias>)
+                  : (vec ? fc_reduce_kernel<4, 1, kBias> : fc_reduce_kernel<1, 1, kBias>);
+  };
+  auto kernel = R.bias_sum.db ? pick(std::true_type{}) : pick(std::false_type{});
   const long long per_block = slices ? 32 : 256;
-  launch_pdl(kernel, dim3((unsigned)((threads + per_block - 1) / per_block)), dim3(256), 0, ctx->stream, R);
+  R.sum_blocks = (unsigned)((threads + per_block - 1) / per_block);
+  launch_pdl(kernel, dim3(R.sum_blocks + (R.bias_sum.db ? (R.bias_sum.O + 31) / 32 : 0)), dim3(256), 0, ctx->stream, R);
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
@@ -784,6 +808,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   const bool x_ok = plan->Xp || fc_aligned({X}), w_ok = plan->Wp || fc_aligned({W}), dy_ok = plan->dYp || fc_aligned({dY});
   const bool w_small = plan->small || !(x_ok && dy_ok), d_small = plan->small || !(w_ok && dy_ok);
   const float *Xm = X, *dYm = dY;
+  FcBiasSum bias_sum{};
   int rc = CCT_OK;
   // ---- weight gradient: out = dW[o][k] (m = k, n = o), reduction over the batch; both operands MN-major
   plan->timer.begin(1, ctx->stream);
@@ -800,7 +825,13 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     if (rc == CCT_OK)
       rc = fc_launch(ctx, plan->wgr, plan->x_wgr, plan->dy_wgr, direct ? plan->x_wgr : plan->out_wgr, direct ? dW : nullptr, K);
     if (rc != CCT_OK) return rc;
-    if (plan->bias) launch_pdl(fc_bias_grad_kernel, dim3((O + 31) / 32), dim3(256), 0, ctx->stream, dY, db, B, O);
+    if (plan->bias) {
+      bias_sum = FcBiasSum{dY, db, B, O};
+      if (!dX || (d_small && fc_small_pass_splits(plan, plan->small_dgr, plan->dgr) == 1)) {  // no reduction follows
+        launch_pdl(fc_bias_grad_kernel, dim3((O + 31) / 32), dim3(256), 0, ctx->stream, bias_sum);
+        bias_sum = FcBiasSum{};
+      }
+    }
   }
   plan->timer.end(1, ctx->stream);
   CCT_CHECK_LAUNCH(ctx);
@@ -808,7 +839,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   if (dX && d_small) {
     plan->timer.begin(3, ctx->stream);
     const int splits = fc_small_pass_splits(plan, plan->small_dgr, plan->dgr);
-    const FcReduceParams post{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4, splits, 0};
+    const FcReduceParams post{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4, splits, 0, 0, bias_sum};
     FcSmallParams D{W, dY, K, O, 1, 0, K, B, O, fc_round_up((O + splits - 1) / splits, 32), splits > 1 ? plan->partial : dX,
                     splits > 1 ? K4 : K, nullptr, post};
     fc_small(ctx, D, splits);
@@ -824,7 +855,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     if (rc == CCT_OK) rc = fc_launch(ctx, plan->dgr, plan->w_dgr, plan->dy_dgr, plan->out_dgr);
     if (rc == CCT_OK)
       rc = fc_reduce(ctx, FcReduceParams{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4,
-                                         plan->dgr.P.splits, 0});
+                                         plan->dgr.P.splits, 0, 0, bias_sum});
     plan->timer.end(3, ctx->stream);
   }
   return rc;
