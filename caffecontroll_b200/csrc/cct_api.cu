@@ -561,6 +561,14 @@ int cct_conv_backward_fused(cct_conv_plan* plan, const float* X, const float* W,
       ctx->last_error = "cct_conv_backward_fused with a pooled gradient needs cct_conv_plan_reserve_fusion(plan) first";
       return CCT_ERR_INVALID;
     }
+    DyRows rows;
+    if (f->P && plan->algo == CCT_ALGO_UMMA_3XTF32 && umma_dy_rows(plan->umma, &rows)) {
+      // straight into the form the contractions read
+      int rc = pool_relu_backward_rows(ctx, f->P, f->idx, f->dP, rows, G.B * G.o, G.m, f->pool_k, f->pool_s);
+      if (rc == CCT_OK) rc = umma_conv_backward(ctx, plan->umma, X, W, nullptr, dX, dW, db, &plan->timer);
+      if (rc == CCT_OK && f->relu_mask_dx && dX) rc = cct_relu_backward(ctx, X, dX, dX, (size_t)G.B * G.D * G.n * G.n);
+      if (rc != CCT_ERR_UNSUPPORTED) return rc;
+    }
     const int rc = f->P ? pool_relu_backward_pooled(ctx, f->P, f->idx, f->dP, plan->mask_dY, G.B * G.o, G.m, f->pool_k, f->pool_s)
                         : cct_pool_relu_backward(ctx, f->A, f->idx, f->dP, plan->mask_dY, G.B * G.o, G.m, f->pool_k, f->pool_s);
     if (rc != CCT_OK) return rc;

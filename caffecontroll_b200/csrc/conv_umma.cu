@@ -1755,6 +1755,7 @@ struct UmmaPlan {
   // pre-split TMA operand [hi|lo][channel tile][channel][pixel]
   bool wg_gather = false;
   GatherProblem wgp;
+  MaskTap* dgr_row_taps = nullptr; // the data gradient's table for a dY in rows (DyRows), where that can be
   MaskTap* wg_pix = nullptr;       // per pixel: offset of the tap origin, taps out of bounds (padded to splits * kps * 32)
   float* wg_plane_sums = nullptr;  // [batch][channel] sums of dY for the bias gradient
   int wg_splits = 1, wg_kps = 1, wg_mtiles = 1;
@@ -2117,6 +2118,17 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     mem.table(&p->wg_pix, t);
     finish_problem(mem, w, vgroups, 0);
     if (G.bias) mem.room(&p->wg_plane_sums, (size_t)G.B * G.o);
+    // dY in rows serves the data gradient too, where rows are channels and the offsets fit.
+    if (w.n == w.n_pad && w.tiles * w.n == G.og && !p->dgr.small_ct && (double)G.o * w.map_k < 2147483648.0) {
+      const GatherProblem& d = p->dgr;
+      const int J = p->dgr_taps;
+      std::vector<MaskTap> rt((size_t)d.splits * d.split_k / d.run, MaskTap{0, kPadBit});
+      for (int i = 0; i * d.run < d.k_real; ++i) {
+        const int jx = i % J, jy = (i / J) % J, oc = i / (J * J) * d.run;
+        rt[i] = MaskTap{(int)(oc * w.map_k) - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
+      }
+      mem.table(&p->dgr_row_taps, rt);
+    }
     sums = std::max(sums, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
   }
   float* sum_memory = nullptr;
@@ -2281,6 +2293,12 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
   return CCT_OK;
 }
 
+bool umma_dy_rows(const UmmaPlan* p, DyRows* rows) {
+  if (!p->wg_gather || !p->dgr_row_taps) return false;
+  *rows = DyRows{p->wgp.w, p->wgp.w_half, p->wgp.map_k, p->G.bias ? p->wg_plane_sums : nullptr, p->G.o, (int)p->wgp.mixed};
+  return true;
+}
+
 int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dY, float* dX,
                        float* dW, float* db, PhaseTimer* t) {
   int rc = umma_conv_wgrad(ctx, p, X, dY, dW, db, t, dX ? W : nullptr);
@@ -2300,7 +2318,8 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     GatherProblem& w = p->wgp;
     const int vgroups = G.g * f.tiles, mm = G.m * G.m;
     t->begin(1, ctx->stream);
-    launch_pdl(split_dy_kernel, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, 
+    if (dY)  // (else the kernel that made it has written the rows)
+      launch_pdl(split_dy_kernel, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, 
         dY, w.w, w.w + w.w_half, G.bias ? p->wg_plane_sums : nullptr, G.B * G.o, G.o, mm, G.og, f.n, f.tiles,
         f.n_pad, w.map_k, (int)w.mixed);
     CCT_CHECK_LAUNCH(ctx);
@@ -2399,6 +2418,12 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
     P.tap_sign = -1; P.taps_per_axis = p->dgr_taps;
     P.in_batch_stride = (long long)G.o * G.m * G.m;
     P.in_group_stride = G.og * G.m * G.m;
+    const bool rows = !dY;
+    if (rows) {  // DyRows
+      P.in = p->wgp.w;
+      P.in_batch_stride = G.m * G.m;
+      P.in_group_stride = (int)(G.og * p->wgp.map_k);
+    }
     P.oy_mul = G.s; P.oy_add = p->dgr_q0 * G.s - G.p; P.ox_mul = G.s; P.ox_add = p->dgr_q0 * G.s - G.p;
     P.out_lim = G.n; P.check_out = 1;
     P.out_pitch = G.n; P.out_plane = G.n * G.n;
@@ -2406,6 +2431,10 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
     P.out_group_channels = G.Dg;
     P.relu = 0;
     fill_common(P, d, ctx, vgroups, 0);
+    if (rows) {
+      P.taps = p->dgr_row_taps;
+      P.run_stride = (int)p->wgp.map_k;
+    }
     launch_gather(ctx, P, d);
     t->end(3, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);

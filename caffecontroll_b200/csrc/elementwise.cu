@@ -386,18 +386,24 @@ __global__ void __launch_bounds__(kSlotThreads) maxpool_bwd_slots_kernel(
 // building the result in shared memory as well, to store it in 16-byte pieces, was slower than either.
 constexpr int kPool32Threads = 256, kPool32Strip = 4;
 constexpr int kPool32Items = 12 * kPool32Threads;  // 2 x 2 blocks a thread block takes on per group
-constexpr size_t kPool32SmemCap = 64 * 1024;
+constexpr size_t kPool32SmemCap = 64 * 1024, kPool32RowsSmem = 28 * 1024;
 
-template <bool RELU>
+// ROWS: the result goes out as DyRows.  Written as a cube, read again and split by a kernel of its own it crossed HBM three times
+// more: CaffeNet conv2 at batch 256 66 + 102 us, this 118; conv5 21 + 31, this 30; at batch 32 10.6 + 11.1, this 17.8.  With two
+// stores per element it pays to turn the planes in shared memory, so that a warp stores whole lines (157 us straight from the 2 x 2
+// blocks), and to keep a block's planes few (28 KB; 36 KB 119 us, 56 KB 123).
+template <bool RELU, bool ROWS>
 __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
     const float* __restrict__ A, const int32_t* __restrict__ idx, const float* __restrict__ dP, const float* __restrict__ P,
-    float* __restrict__ dA, int planes, int n, int m, int half, uint32_t inv_half, int strips, uint32_t inv_strips, int group, int vec_ok) {
+    float* __restrict__ dA, int planes, int n, int m, int half, uint32_t inv_half, int strips, uint32_t inv_strips, int group, int vec_ok,
+    const __grid_constant__ DyRows rows, uint32_t inv_channels) {
   extern __shared__ __align__(16) float pool32_smem[];
   pdl_wait();
   const int nn = n * n, mm = m * m;
   const int in_pad = (group * mm + 3) & ~3;
   int32_t* s_idx = reinterpret_cast<int32_t*>(pool32_smem);
   float* s_g = pool32_smem + in_pad;
+  float* s_out = s_g + in_pad;  // ROWS: the planes, on their way out
   for (int g0 = blockIdx.x * group; g0 < planes; g0 += gridDim.x * group) {
     const int cnt = min(group, planes - g0);
     const size_t in_base = (size_t)g0 * mm;
@@ -446,7 +452,7 @@ __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
         gl = in && left ? wg[ph * m - 1] : 0.f;
         gr = in && right ? wg[ph * m] : 0.f;
       };
-      const size_t plane_at = out_base + (size_t)pl * nn;
+      const size_t plane_at = ROWS ? (size_t)pl * nn : out_base + (size_t)pl * nn;
       int32_t i00, i01, i10, i11;
       float g00, g01, g10, g11;
       load(a0 - 1, i00, i01, g00, g01);
@@ -468,7 +474,7 @@ __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
         r10 += i11 == e10 ? g11 : 0.f;
         r11 += i11 == e11 ? g11 : 0.f;
         const bool wide = w0 + 1 < n, tall = h0 + 1 < n;
-        float* out = dA + plane_at;
+        float* out = (ROWS ? s_out : dA) + plane_at;
         if (RELU) {
           const float* ap = A + plane_at;
           r00 = __ldg(ap + e00) > 0.f ? r00 : 0.f;
@@ -484,6 +490,32 @@ __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
       }
     }
     __syncthreads();
+    if (ROWS) {
+      // A warp per plane, a lane per float of the destination's 128-byte lines; the sums are added as split_dy_kernel adds them.
+      const int lane = threadIdx.x & 31;
+      for (int pl = threadIdx.x >> 5; pl < cnt; pl += kPool32Threads / 32) {
+        const uint32_t plane = (uint32_t)(g0 + pl), b = fast_div(plane, (uint32_t)rows.channels, inv_channels);
+        float* hi = rows.rows + (size_t)(plane - b * rows.channels) * rows.row_len + (size_t)b * nn;
+        const float* src = s_out + pl * nn;
+        float sum = 0.f;
+#pragma unroll 4
+        for (int i = lane - (int)(((size_t)b * nn) & 31); i < nn; i += 32) {
+          const float x = i >= 0 ? src[i] : 0.f;
+          const float l = x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
+          if (i >= 0) {
+            hi[i] = x;
+            hi[rows.lo + i] = rows.mixed ? __uint_as_float(cross_word(l, x)) : l;
+          }
+          sum += x;
+        }
+        if (rows.plane_sums) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+          if (lane == 0) rows.plane_sums[plane] = sum;
+        }
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -529,6 +561,29 @@ __global__ void __launch_bounds__(256) maxpool_bwd_2x2_kernel(const float* __res
   }
 }
 
+// The kernel for windows of 3x3 with stride 2; false if a group of planes does not fit.
+template <bool RELU, bool ROWS>
+int launch_maxpool_bwd_3x3s2(cct_ctx* ctx, const float* A, const int32_t* idx, const float* dP, const float* P, float* dA, int planes, int n,
+                             int m, const DyRows& rows, bool* fits) {
+  // Planes per block: a multiple of four, so that every group starts on a 16-byte boundary of the pooled tensors.
+  const int half = (n + 1) / 2, strips = (half + kPool32Strip - 1) / kPool32Strip;
+  const int group = ROWS ? std::max(4, (int)(kPool32RowsSmem / ((2 * m * m + n * n) * 4)) & ~3)
+                         : std::max(4, (kPool32Items / (half * half) + 3) & ~3);
+  const size_t smem = ((size_t)2 * ((group * m * m + 3) & ~3) + (ROWS ? (size_t)group * n * n : 0)) * 4;
+  *fits = smem <= kPool32SmemCap;
+  if (!*fits) return CCT_OK;
+  const int vec_ok = ((reinterpret_cast<uintptr_t>(idx) | reinterpret_cast<uintptr_t>(dP) |
+                       reinterpret_cast<uintptr_t>(P)) & 15) == 0;
+  if (smem > 48 * 1024)
+    CCT_CUDA(ctx, cudaFuncSetAttribute(maxpool_bwd_3x3s2_kernel<RELU, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int blocks = std::max(1, std::min((planes + group - 1) / group, ctx->sm_count * 64));
+  launch_pdl(maxpool_bwd_3x3s2_kernel<RELU, ROWS>, dim3(blocks), dim3(kPool32Threads), smem, ctx->stream, A, idx, dP, P, dA,
+             planes, n, m, half, fast_div_magic((uint64_t)group * strips * half, (uint32_t)half), strips,
+             fast_div_magic((uint64_t)group * strips, (uint32_t)strips), group, vec_ok, rows,
+             rows.channels ? fast_div_magic((uint64_t)planes, (uint32_t)rows.channels) : 0u);
+  return CCT_OK;
+}
+
 template <bool RELU>
 int launch_maxpool_bwd(cct_ctx* ctx, const float* A, const int32_t* idx, const float* dP, float* dA, int planes, int n,
                        int m, int k, int s, const float* P = nullptr) {
@@ -537,21 +592,9 @@ int launch_maxpool_bwd(cct_ctx* ctx, const float* A, const int32_t* idx, const f
   const int taps = (k + s - 1) / s;
   const int half = (n + 1) / 2;
   if (k == 3 && s == 2) {
-    // Planes per block: a multiple of four, so that every group starts on a 16-byte boundary of the pooled tensors.
-    const int strips = (half + kPool32Strip - 1) / kPool32Strip;
-    const int group = std::max(4, (kPool32Items / (half * half) + 3) & ~3);
-    const size_t smem = (size_t)2 * ((group * m * m + 3) & ~3) * 4;
-    if (smem <= kPool32SmemCap) {
-      const int vec_ok = ((reinterpret_cast<uintptr_t>(idx) | reinterpret_cast<uintptr_t>(dP) |
-                           reinterpret_cast<uintptr_t>(P)) & 15) == 0;
-      if (smem > 48 * 1024)
-        CCT_CUDA(ctx, cudaFuncSetAttribute(maxpool_bwd_3x3s2_kernel<RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      const int blocks = std::max(1, std::min((planes + group - 1) / group, ctx->sm_count * 64));
-      launch_pdl(maxpool_bwd_3x3s2_kernel<RELU>, dim3(blocks), dim3(kPool32Threads), smem, ctx->stream, A, idx, dP, P, dA,
-                 planes, n, m, half, fast_div_magic((uint64_t)group * strips * half, (uint32_t)half), strips,
-                 fast_div_magic((uint64_t)group * strips, (uint32_t)strips), group, vec_ok);
-      return CCT_OK;
-    }
+    bool fits = false;
+    const int rc = launch_maxpool_bwd_3x3s2<RELU, false>(ctx, A, idx, dP, P, dA, planes, n, m, DyRows(), &fits);
+    if (rc != CCT_OK || fits) return rc;
   }
   const long long items = (long long)planes * half * half;
   if (k == 2 && s == 2 && items < (1ll << 31) - 256) {
@@ -600,6 +643,19 @@ int pool_relu_backward_pooled(cct_ctx* ctx, const float* P, const int32_t* idx, 
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   const int rc = launch_maxpool_bwd<false>(ctx, nullptr, idx, dP, dA, planes, n, m, k, s, P);
   if (rc != CCT_OK) return rc;
+  CCT_CHECK_LAUNCH(ctx);
+  return CCT_OK;
+}
+
+int pool_relu_backward_rows(cct_ctx* ctx, const float* P, const int32_t* idx, const float* dP, const DyRows& out, int planes,
+                            int n, int k, int s) {
+  if (!ctx || !P || !idx || !dP || !pool_args_ok(planes, n, k, s)) return CCT_ERR_INVALID;
+  if (k != 3 || s != 2) return CCT_ERR_UNSUPPORTED;
+  CCT_CUDA(ctx, cudaSetDevice(ctx->device));
+  bool fits = false;
+  const int rc = launch_maxpool_bwd_3x3s2<false, true>(ctx, nullptr, idx, dP, P, out.rows, planes, n, (n - k) / s + 1, out, &fits);
+  if (rc != CCT_OK) return rc;
+  if (!fits) return CCT_ERR_UNSUPPORTED;
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }

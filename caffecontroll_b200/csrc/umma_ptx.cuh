@@ -158,11 +158,7 @@ __device__ __forceinline__ void split_tf32_trunc(float x, uint32_t& hi, uint32_t
 // CaffeNet at batch 256, forward / weight gradient / data gradient, us: conv2 407 -> 317 / 405 -> 359 / -, conv3 263 -> 195 /
 // 257 -> 194 / 271 -> 208, conv4 215 -> 162 / 211 -> 161 / 216 -> 159, conv5 144 -> 111 / 157 -> 141 / 153 -> 113.
 constexpr int kMixedChain = 8;  // k-blocks of 32 of an accumulation chain from which on it is the more accurate form
-__device__ __forceinline__ uint32_t cross_word(float lower, float upper) {
-  uint32_t w;
-  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(upper), "f"(lower));  // (the largest fp32 values would round to Inf)
-  return w;
-}
+// (cross_word itself: cct_internal.h, for the kernels that write operands)
 // hi = x truncated to tf32 and A's word of the cross terms.
 __device__ __forceinline__ void split_mixed_a(float x, uint32_t& hi, uint32_t& word) {
   hi = __float_as_uint(x) & 0xFFFFE000u;

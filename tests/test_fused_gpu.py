@@ -118,3 +118,41 @@ def test_fused_backward_argument_checks(ctx):
     assert rc == capi.CCT_ERR_INVALID
     capi.check(lib.cct_conv_plan_destroy(plan), "destroy", ctx.h)
     buf.free()
+
+
+# With the pooled tensor at hand the masked gradient goes straight into the rows that the contractions read, where the weight
+# gradient is a gather over at least 512 lowered rows and the channel tiles are multiples of 16: one and two tiles, groups, planes
+# of 25 to 729 elements, chains on both sides of the line for bf16 cross terms; uneven tiles, planes too large for the kernel and
+# other windows, which take the cube.  Bit-identical to the cube's path.
+@pytest.mark.parametrize("shape", [
+    (3, 64, 15, 48, 3, 1, 1, 1, 3, 2), (2, 128, 20, 160, 3, 1, 1, 2, 3, 2), (5, 64, 5, 16, 3, 1, 1, 1, 3, 2), (70, 64, 7, 256, 3, 1, 1, 1, 3, 2),
+    (2, 32, 27, 512, 5, 1, 2, 1, 3, 2), (2, 60, 28, 272, 3, 1, 0, 1, 3, 2), (1, 64, 57, 16, 3, 1, 1, 1, 3, 2), (3, 64, 16, 32, 3, 1, 1, 1, 2, 2),
+    (3, 72, 21, 64, 3, 2, 1, 1, 3, 2),
+])
+def test_pooled_gradient_in_rows(ctx, shape):
+    B, D, n, o, k, s, p, g, pk, ps = shape
+    m = (n + 2 * p - k) // s + 1
+    mp = (m - pk) // ps + 1
+    rng = np.random.default_rng(n + o)
+    lib, vp = ctx.lib, C.c_void_p
+    desc, plan = capi.ConvDesc(B, D, n, o, k, s, p, g, 1, capi.ALGO_UMMA_3XTF32), C.c_void_p()
+    capi.check(lib.cct_conv_plan_create(ctx.h, C.byref(desc), C.byref(plan)), "plan", ctx.h)
+    capi.check(lib.cct_conv_plan_reserve_fusion(plan), "reserve", ctx.h)
+    cX, cW, cY, cdP = (LogicalCube.from_numpy(ctx, rng.standard_normal(sh).astype(np.float32))
+                       for sh in ((B, D, n, n), (o, D // g, k, k), (B, o, m, m), (B, o, mp, mp)))
+    cP, cidx = LogicalCube(ctx, mp, mp, o, B), LogicalCube(ctx, mp, mp, o, B, np.int32)
+    capi.check(lib.cct_maxpool_forward(ctx.h, vp(cY.ptr), vp(cP.ptr), vp(cidx.ptr), B * o, m, pk, ps), "pool", ctx.h)
+    cdX, cdW, cdb = LogicalCube(ctx, n, n, D, B), LogicalCube(ctx, k, k, D // g, o), LogicalCube(ctx, 1, 1, o, 1)
+    results = []
+    for A, P, dX in ((cY.ptr, None, cdX.ptr), (None, cP.ptr, cdX.ptr), (cY.ptr, None, cdX.ptr), (None, cP.ptr, None)):
+        f = capi.BwdFusion(A, cidx.ptr, cdP.ptr, pk, ps, 0, P)
+        capi.check(lib.cct_conv_backward_fused(plan, vp(cX.ptr), vp(cW.ptr), None, C.byref(f), vp(dX) if dX else None, vp(cdW.ptr),
+                                               vp(cdb.ptr)), "backward", ctx.h)
+        ctx.sync()
+        results.append((cdX.download(), cdW.download(), cdb.download()))
+    capi.check(lib.cct_conv_plan_destroy(plan), "destroy", ctx.h)
+    for other in results[1:]:
+        for got, want in zip(other, results[0]):
+            assert np.array_equal(got, want)
+    for c in (cX, cW, cY, cdP, cP, cidx, cdX, cdW, cdb):
+        c.free()
