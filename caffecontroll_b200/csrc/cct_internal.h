@@ -86,7 +86,8 @@ inline int record_call(std::function<int()> call) {
     }                                                                                         \
   } while (0)
 
-// Programmatic dependent launch: every kernel of the library starts with pdl_wait() (griddepcontrol.wait: returns once
+// Programmatic dependent launch: every kernel of the library starts with pdl_wait() - the persistent
+// ones once barriers, tensor memory and the plan's constant tables are set up - (griddepcontrol.wait: returns once
 // the kernel before it in the stream has completed and its writes are visible) and is launched with the programmatic
 // stream-serialisation attribute, so the launch itself - grid set-up, parameter upload - overlaps the tail of its
 // predecessor instead of following it.  No kernel signals its dependents early: the order of execution stays the

@@ -20,7 +20,8 @@
 // streamed by TMA into swizzled shared memory, warp-specialised roles.  Shorter lowered matrices have their own weight-
 // gradient kernels: wgrad_ts_kernel (257 .. 384 rows: dY through tensor memory, the lowered rows staged in shared memory)
 // and wgrad_kernel (anything shorter, and the allocation-free entry point: both operands staged in shared memory).
-// Every kernel starts with pdl_wait() and is launched with launch_pdl (cct_internal.h).  Every mbarrier wait is bounded: when it runs out the thread
+// Every kernel is launched with launch_pdl and calls pdl_wait() before it touches anything but its plan's tables (cct_internal.h).
+// Every mbarrier wait is bounded: when it runs out the thread
 // sets the context's status word, stops waiting on anything else, and the kernel still frees its tensor memory.
 #include <algorithm>
 #include <cstdio>
@@ -237,7 +238,6 @@ enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3 };
 template <int SETS, int MODE, bool MIXED>
 __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     gather_conv_kernel(const __grid_constant__ GatherParams P, const __grid_constant__ CUtensorMap w_map) {
-  pdl_wait();
   constexpr int kProducerWarps = 4 * SETS, kMmaWarp = kProducerWarps, kTmaWarp = kMmaWarp + 1;
   constexpr int kGatherThreads = gather_threads(SETS);
   extern __shared__ uint8_t smem_raw[];
@@ -264,13 +264,15 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   }
   if (P.cols)
     for (int i = tid; i < P.n_pad; i += kGatherThreads) s_cols[i] = P.cols[i];
-  for (int i = tid; i < P.n_bias + kBiasPad; i += kGatherThreads) s_bias[i] = i < P.n_bias ? P.bias[i] : 0.f;
   if (tid == 0) {
     for (int s = 0; s < kMaxAStages; ++s) { mbar_init(ready_bar + 8u * s, 5); mbar_init(done_bar + 8u * s, 1); }  // 4 producer warps + the TMA thread
     for (int s = 0; s < kMaxAccBufs; ++s) { mbar_init(acc_full + 8u * s, 1); mbar_init(acc_empty + 8u * s, kEpiWarps); }
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(tmem_slot, (uint32_t)P.tmem_cols);
+  if (warp == kTmaWarp) prefetch_map(&w_map);
+  pdl_wait();  // so far the plan's tables alone have been read: set-up beside the end of the kernel before (15.6 -> 15.35 us for conv3 of one image)
+  for (int i = tid; i < P.n_bias + kBiasPad; i += kGatherThreads) s_bias[i] = i < P.n_bias ? P.bias[i] : 0.f;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1014,7 +1016,6 @@ template <bool WIDE, bool MIXED>
 __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __grid_constant__ WgradParams P) {
   constexpr int kTsTapWarps = ts_tap_warps(WIDE), kTsDyWarps = ts_dy_warps(WIDE), kTsMmaWarp = kTsTapWarps + kTsDyWarps;
   constexpr int kTsThreads = ts_threads(WIDE), kTsRowsPerWarp = kTsRows / 24;  // 16
-  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -1042,6 +1043,7 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(tmem_slot, 512);
+  pdl_wait();  // so far the plan's table alone has been read
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

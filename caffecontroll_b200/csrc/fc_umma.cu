@@ -93,7 +93,6 @@ template <bool MIXED>
 __global__ void __launch_bounds__(kFcThreads, 2)
     fc_gemm_kernel(const __grid_constant__ FcGemmParams P, const __grid_constant__ CUtensorMap a_map,
                    const __grid_constant__ CUtensorMap b_map, const __grid_constant__ CUtensorMap out_map) {
-  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -114,6 +113,8 @@ __global__ void __launch_bounds__(kFcThreads, 2)
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(tmem_slot, (uint32_t)P.tmem_cols);
+  if (warp == kFcTmaWarp) { prefetch_map(&a_map); prefetch_map(&b_map); }
+  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -177,6 +177,8 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int 
       "l"(tmap), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
+// The descriptor of a tensor map (a kernel parameter) fetched ahead of its first copy.
+__device__ __forceinline__ void prefetch_map(const void* tmap) { asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory"); }
 // D[tmem] (+)= A[tmem] * B[smem]^T.
 __device__ __forceinline__ void umma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                              uint32_t accumulate) {
