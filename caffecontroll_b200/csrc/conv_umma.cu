@@ -1374,14 +1374,24 @@ __device__ __forceinline__ void pack_dgrad_block(const PackDgrad& J, int block) 
   const float* src = J.W + ((size_t)grp * J.og * J.Dg + d) * J.k * J.k;
   const size_t row = (size_t)r0 * J.k_pad;
   for (int kk = (part * (int)blockDim.x + (int)threadIdx.x) * 4; kk < J.k_pad; kk += J.parts * (int)blockDim.x * 4) {
+    // reduction index -> (filter / run, jy, jx, filter % run); four in a row are four filters of one tap where run is kRun, and
+    // one decode serves them (with one each the divisions bound the packing kernels)
     float v[4];
+    const size_t filter = (size_t)J.Dg * J.k * J.k;
+    if (J.run == kRun) {
+      const int r = kk / kRun, chunk = r / window, tap = r - chunk * window;
+      const int jy = tap / J.taps, kr = py + jy * J.s, kc = px + (tap - jy * J.taps) * J.s;
+      const bool in = live && kk < J.k_real && kr < J.k && kc < J.k;
+      const float* at = src + (size_t)(chunk * kRun + (kk & (kRun - 1))) * filter + kr * J.k + kc;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      // reduction index -> (filter / run, jy, jx, filter % run)
-      const int r = (kk + e) / J.run, chunk = r / window, tap = r - chunk * window;
-      const int oc = chunk * J.run + (kk + e - r * J.run), jy = tap / J.taps, jx = tap - jy * J.taps;
-      const int kr = py + jy * J.s, kc = px + jx * J.s;
-      v[e] = (live && kk + e < J.k_real && kr < J.k && kc < J.k) ? __ldg(src + (size_t)oc * J.Dg * J.k * J.k + kr * J.k + kc) : 0.f;
+      for (int e = 0; e < 4; ++e) v[e] = in ? __ldg(at + e * filter) : 0.f;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int oc = (kk + e) / window, tap = kk + e - oc * window, jy = tap / J.taps;
+        const int kr = py + jy * J.s, kc = px + (tap - jy * J.taps) * J.s;
+        v[e] = (live && kk + e < J.k_real && kr < J.k && kc < J.k) ? __ldg(src + oc * filter + kr * J.k + kc) : 0.f;
+      }
     }
     if (J.mixed) store_split4<true>(J.hi, J.lo, row + kk, v);
     else store_split4<false>(J.hi, J.lo, row + kk, v);
@@ -1614,14 +1624,12 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
   const float* src = W + (size_t)((vg / tiles_per_group) * og + ch) * k_real;
   const size_t row = (size_t)blockIdx.x * k_pad;
   for (int kk = (blockIdx.y * kPackThreads + threadIdx.x) * 4; kk < k_pad; kk += gridDim.y * kPackThreads * 4) {
+    // reduction index -> (channel / run, tap, channel % run) -> element (channel, tap) of the filter, one decode for four
     float v[4];
+    const int r = kk / kRun, chunk = r / window;
+    const int at = run == 1 ? kk : (chunk * kRun + (kk & (kRun - 1))) * window + (r - chunk * window), step = run == 1 ? 1 : window;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      // reduction index -> (channel / run, tap, channel % run) -> element (channel, tap) of the filter
-      const int i = kk + e, r = i / run, chunk = r / window;
-      const int at = run == 1 ? i : (chunk * run + (i - r * run)) * window + (r - chunk * window);
-      v[e] = (live && i < k_real) ? __ldg(src + at) : 0.f;
-    }
+    for (int e = 0; e < 4; ++e) v[e] = (live && kk + e < k_real) ? __ldg(src + at + e * step) : 0.f;
     store_split4<MIXED>(hi, lo, row + kk, v);
   }
 }
