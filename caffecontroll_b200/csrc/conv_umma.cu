@@ -678,6 +678,13 @@ __global__ void __launch_bounds__(128) gather_reduce_kernel(const __grid_constan
   }
 }
 
+// A value as the shared-memory operand B: hi and the low part or word.
+template <bool MIXED>
+__device__ __forceinline__ void split_lowered(float x, uint32_t& h, uint32_t& l) {
+  split_tf32_trunc(x, h, l);
+  if (MIXED) l = cross_word(__uint_as_float(l), x);
+}
+
 // ---------------------------------------------------------------------------------- weight-gradient kernel
 //
 // dW[kk][o] (+ the bias row) = sum over pixels of Lowered(X)[pix][kk] * dY[pix][o], split over pixel ranges.
@@ -741,7 +748,10 @@ __host__ __device__ inline WgSmem wg_smem(int n_pad, int subs, int stages) {
 // compile time every warp stages exactly 8*SUBS tap rows and NB channel rows per k-block, all loads of a k-block are
 // in flight together, and the shared-memory addresses are one per-warp base plus immediates: row warp+16*i of a
 // 128-byte-swizzled tile has the same swizzle phase ((warp+16*i) & 7 == warp & 7) for every i.
-template <int SUBS, int NB>
+// MIXED (more than 64 columns, chains of kMixedChain and more): cross terms in bf16 (cross_word), "lo" tiles are their words.
+// With two M-tiles per CTA: 64 images of 28 x 40 x 40 to 100 / 160 / 176 channels 47.6 -> 45.0, 60.3 -> 56.8, 63.8 -> 59.9 us.  One
+// M-tile with wide dY tiles stays with three tf32 products (200 channels 79.6 -> 89.4).
+template <int SUBS, int NB, bool MIXED>
 __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_constant__ WgradParams P) {
   pdl_wait();
   extern __shared__ uint8_t smem_raw[];
@@ -837,7 +847,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
 #pragma unroll
         for (int i = 0; i < kARows; ++i) {  // tile i/8 (hi then lo), row warp + 16*(i%8)
           uint32_t h, l;
-          split_tf32_trunc(va[i], h, l);
+          if (MIXED) split_mixed_a(va[i], h, l);
+          else split_tf32_trunc(va[i], h, l);
           uint8_t* dst = st + (i / 8) * 2 * kATile + (i % 8) * 2048;
           *reinterpret_cast<uint32_t*>(dst) = h;
           *reinterpret_cast<uint32_t*>(dst + kATile) = l;
@@ -875,7 +886,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
 #pragma unroll
         for (int i = 0; i < kDyRows; ++i) {
           uint32_t h, l;
-          split_tf32_trunc(vb[i], h, l);
+          split_lowered<MIXED>(vb[i], h, l);
           uint8_t* dst = st + i * (kWgDyWarps * 128);
           *reinterpret_cast<uint32_t*>(dst) = h;
           *reinterpret_cast<uint32_t*>(dst + kBTile) = l;
@@ -917,7 +928,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
     }
   } else {
     // ------------------------------------------------------------------ MMA issue (see elect_one)
-    const uint32_t idesc = make_idesc(kAccCols), tmem = warp_uniform(tmem_base);
+    const uint32_t idesc = make_idesc(kAccCols), idesc_cross = make_idesc_bf16(kAccCols), tmem = warp_uniform(tmem_base);
     const int n_subs = (int)warp_uniform((uint32_t)subs);
     Ring ring;
     for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(P.stages)) {
@@ -935,8 +946,12 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
             const uint64_t adv = (uint64_t)(j * 2);
-            umma_tf32_ss(d_tmem, dal + adv, dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
-            if (!kDual) umma_tf32_ss(d_tmem, dah + adv, dbl + adv, idesc, 1u);
+            if (MIXED) {
+              umma_bf16_ss(d_tmem, dal + adv, dbl + adv, idesc_cross, (kbl == 0 && j == 0) ? 0u : 1u);
+            } else {
+              umma_tf32_ss(d_tmem, dal + adv, dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
+              if (!kDual) umma_tf32_ss(d_tmem, dah + adv, dbl + adv, idesc, 1u);
+            }
             umma_tf32_ss(d_tmem, dah + adv, dbh + adv, idesc, 1u);
           }
         }
@@ -988,13 +1003,6 @@ constexpr uint32_t kTsTapsOff = kTsStages * kTsStage, kTsTurnOff = kTsTapsOff + 
 constexpr int kTsWideTaps = 13, kTsWideRows = 2;  // taps that four blocks cover at any alignment; window rows per warp
 
 __device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
-// A lowered value as the shared-memory operand of wgrad_ts_kernel.
-template <bool MIXED>
-__device__ __forceinline__ void split_lowered(float x, uint32_t& h, uint32_t& l) {
-  split_tf32_trunc(x, h, l);
-  if (MIXED) l = cross_word(__uint_as_float(l), x);
-}
 
 // Splits taps 0 .. k - 1, which start at w[SHIFT], and stores them as lowered rows: row r at dst + off[r & 7] + (r & ~7) * 128.
 template <int SHIFT, bool MIXED>
@@ -1315,22 +1323,24 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
 }
 
 typedef void (*WgradKernel)(const WgradParams);
-template <int SUBS>
+template <int SUBS, bool MIXED>
 WgradKernel wgrad_pick_nb(int nb) {
   switch (nb) {
-    case 1: return wgrad_kernel<SUBS, 1>;   case 2: return wgrad_kernel<SUBS, 2>;
-    case 3: return wgrad_kernel<SUBS, 3>;   case 4: return wgrad_kernel<SUBS, 4>;
-    case 5: return wgrad_kernel<SUBS, 5>;   case 6: return wgrad_kernel<SUBS, 6>;
-    case 7: return wgrad_kernel<SUBS, 7>;   case 8: return wgrad_kernel<SUBS, 8>;
-    case 9: return wgrad_kernel<SUBS, 9>;   case 10: return wgrad_kernel<SUBS, 10>;
-    case 11: return wgrad_kernel<SUBS, 11>; case 12: return wgrad_kernel<SUBS, 12>;
-    case 13: return wgrad_kernel<SUBS, 13>; case 14: return wgrad_kernel<SUBS, 14>;
-    case 15: return wgrad_kernel<SUBS, 15>; case 16: return wgrad_kernel<SUBS, 16>;
+    case 1: return wgrad_kernel<SUBS, 1, false>;   case 2: return wgrad_kernel<SUBS, 2, false>;
+    case 3: return wgrad_kernel<SUBS, 3, false>;   case 4: return wgrad_kernel<SUBS, 4, false>;
+    case 5: return wgrad_kernel<SUBS, 5, MIXED>;   case 6: return wgrad_kernel<SUBS, 6, MIXED>;
+    case 7: return wgrad_kernel<SUBS, 7, MIXED>;   case 8: return wgrad_kernel<SUBS, 8, MIXED>;
+    case 9: return wgrad_kernel<SUBS, 9, MIXED>;   case 10: return wgrad_kernel<SUBS, 10, MIXED>;
+    case 11: return wgrad_kernel<SUBS, 11, MIXED>; case 12: return wgrad_kernel<SUBS, 12, MIXED>;
+    case 13: return wgrad_kernel<SUBS, 13, MIXED>; case 14: return wgrad_kernel<SUBS, 14, MIXED>;
+    case 15: return wgrad_kernel<SUBS, 15, MIXED>; case 16: return wgrad_kernel<SUBS, 16, MIXED>;
   }
   return nullptr;
 }
-WgradKernel wgrad_pick(int subs, int n_pad) {
-  return subs == 2 ? wgrad_pick_nb<2>(n_pad / 16) : wgrad_pick_nb<1>(n_pad / 16);
+WgradKernel wgrad_pick(int subs, int n_pad, int chain) {
+  const int nb = n_pad / 16;
+  if (chain >= kMixedChain && subs == 2) return wgrad_pick_nb<2, true>(nb);
+  return subs == 2 ? wgrad_pick_nb<2, false>(nb) : wgrad_pick_nb<1, false>(nb);
 }
 
 }  // namespace
@@ -2162,7 +2172,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
                       gather_conv_kernel<2, kByTap, true>, gather_conv_kernel<2, kByRun, true>, gather_conv_kernel<2, kWeightGrad, true>,
                       gather_conv_kernel<2, kInside, false>, gather_conv_kernel<2, kInside, true>})
     if (rc == CCT_OK) rc = set_smem(ctx, kernel, 113 * 1024);
-  if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad), kSmemLimit);
+  if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad, p->w_kblocks_per_split), kSmemLimit);
   if (p->w_ts)
     for (auto kernel : {wgrad_ts_kernel<false, false>, wgrad_ts_kernel<true, false>, wgrad_ts_kernel<false, true>, wgrad_ts_kernel<true, true>})
       if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
@@ -2386,7 +2396,7 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       launch_pdl(kernel, dim3(grid), dim3(ts_threads(wide)), p->w_smem, ctx->stream, P);
     }
     else
-      launch_pdl(wgrad_pick(p->w_subs, f.n_pad), dim3(grid), dim3(kWgThreads), p->w_smem, ctx->stream, P);
+      launch_pdl(wgrad_pick(p->w_subs, f.n_pad, P.kblocks_per_split), dim3(grid), dim3(kWgThreads), p->w_smem, ctx->stream, P);
     t->end(1, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
     t->begin(2, ctx->stream);
@@ -2552,7 +2562,7 @@ extern "C" int cct_conv_weight_grad_noalloc(cct_ctx* ctx, const cct_conv_desc* d
 
   MaskTap* taps = reinterpret_cast<MaskTap*>(scratch);
   float* partial = reinterpret_cast<float*>(scratch + taps_bytes);
-  WgradKernel kernel = wgrad_pick(subs, n_pad);
+  WgradKernel kernel = wgrad_pick(subs, n_pad, kblocks_per_split);
   CCT_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
   launch_pdl(noalloc_taps_kernel, dim3(8), dim3(256), 0, ctx->stream, taps, m_tiles * kTileM, k_real, G.k, G.n);
   CCT_CHECK_LAUNCH(ctx);

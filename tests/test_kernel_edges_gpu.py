@@ -138,6 +138,7 @@ def test_accumulation_error(ctx, shape, which, chain):
 @pytest.mark.parametrize("shape", [
     (3, 224, 14, 80, 1, 1, 0, 1), (3, 256, 14, 80, 1, 1, 0, 1), (3, 257, 14, 65, 1, 1, 0, 1), (3, 264, 14, 64, 1, 1, 0, 1),
     (5, 29, 15, 130, 3, 1, 1, 1), (2, 160, 17, 272, 3, 1, 1, 2), (4, 40, 19, 300, 5, 2, 2, 1),
+    (24, 28, 40, 75, 3, 1, 1, 1), (25, 28, 40, 170, 3, 1, 1, 1),  # both operands of the weight gradient in shared memory
 ])
 def test_cross_terms_in_bf16(ctx, shape):
     from caffecontroll_b200 import conv_layer
