@@ -161,12 +161,12 @@ int simt_conv_backward(cct_ctx* ctx, const ConvGeom& G, const float* X, const fl
 
 // ---- tcgen05 3xTF32 path (conv_umma.cu) ----
 // dY as the weight gradient's operand: rows of one channel over all images (`row_len` floats, a multiple of 32), the values and
-// behind them, `lo` floats on, their low parts or (mixed) words of cross terms; the plane sums for the bias gradient, or null.
+// behind them, `lo` floats on, their low parts; the plane sums for the bias gradient, or null.
 struct DyRows {
   float* rows = nullptr;
   size_t lo = 0, row_len = 0;
   float* plane_sums = nullptr;
-  int channels = 0, mixed = 0;
+  int channels = 0;
 };
 struct UmmaPlan;  // opaque: tables, packed weights, split-K scratch
 // `tensor_only`: every pass on the tensor cores, however small the layer (CCT_ALGO_UMMA_3XTF32 by name); otherwise small
@@ -196,15 +196,6 @@ int pool_relu_backward_rows(cct_ctx* ctx, const float* P, const int32_t* idx, co
 int pool_relu_backward_pooled(cct_ctx* ctx, const float* P, const int32_t* idx, const float* dP, float* dA, int planes,
                               int n, int k, int s);
 int maxpool_forward_staged(cct_ctx* ctx, const float* X, float* Y, int32_t* idx, int planes, int n, int m, int k, int s);
-
-// ---- one word of two bf16 numbers, see "Cross terms in bf16" in umma_ptx.cuh
-#ifdef __CUDACC__
-__device__ __forceinline__ uint32_t cross_word(float lower, float upper) {
-  uint32_t w;
-  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(upper), "f"(lower));  // (the largest fp32 values would round to Inf)
-  return w;
-}
-#endif
 
 // ---- index arithmetic of the pooling kernels
 // x / d for x * d < 2^32 as one multiply-high: inv = floor(2^32 / d) + 1 (host side, fast_div_magic); inv == 0 means

@@ -4,8 +4,7 @@
 // tensor memory).  The lowered matrix of the reference (type-1 lowering, one row of k*k*D values per output pixel)
 // is never written to global memory: producer threads gather each 128 x 32 tile of it straight from the NCHW
 // tensors, splitting every fp32 value into hi = its tf32 part and lo = x - hi on the way.  Three MMAs per k-step
-// (hi*hi + hi*lo + lo*hi) recover fp32-level accuracy ("3xTF32"), or two where the cross terms are formed in bf16 (cross_word);
-// flops are counted once.
+// (hi*hi + hi*lo + lo*hi) recover fp32-level accuracy ("3xTF32"); flops are counted once.
 //
 //   forward        Y[pix][o]   = sum_k  Lowered(X)[pix][k] * W[o][k]            (+ bias, optional ReLU)
 //   data gradient  dX[q][(d,py,px)] = sum_kk Gathered(dY)[q][kk] * Wd[(d,py,px)][kk]   kk = (filter, jy, jx)
@@ -234,8 +233,7 @@ __host__ __device__ inline GatherSmem gather_smem(int n_pad, int k_pad, int b_st
 // behind the last real index read the window's first element against a weight of zero; lanes behind the last pixel read the last
 // pixel's window, their columns are not stored.)
 enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3 };
-// MIXED: cross terms in bf16 (cross_word), "lo" operands are their words; tiles of more than kCrossCols columns.
-template <int SETS, int MODE, bool MIXED>
+template <int SETS, int MODE>
 __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     gather_conv_kernel(const __grid_constant__ GatherParams P, const __grid_constant__ CUtensorMap w_map) {
   constexpr int kProducerWarps = 4 * SETS, kMmaWarp = kProducerWarps, kTmaWarp = kMmaWarp + 1;
@@ -278,7 +276,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-  const uint32_t acc_cols = (uint32_t)acc_columns(P.n_pad), cross = MIXED ? 0u : acc_cols - (uint32_t)P.n_pad;  // cross: 0 = one accumulator
+  const uint32_t acc_cols = (uint32_t)acc_columns(P.n_pad), cross = acc_cols - (uint32_t)P.n_pad;  // cross: 0 = one accumulator
   const uint32_t a_col0 = (uint32_t)P.acc_bufs * acc_cols;
   const int kblocks = P.k_pad / kBlockK;
   bool failed = false;
@@ -443,10 +441,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       for (int c = 0; c < kBlockK / 8; ++c) {
         uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          if (MIXED) split_mixed_a(v[c * 8 + e], hi[e], lo[e]);
-          else split_tf32_trunc(v[c * 8 + e], hi[e], lo[e]);
-        }
+        for (int e = 0; e < 8; ++e) split_tf32_trunc(v[c * 8 + e], hi[e], lo[e]);
         tmem_st8(st_addr + (uint32_t)(c * 8), hi);
         tmem_st8(st_addr + 32u + (uint32_t)(c * 8), lo);
       }
@@ -467,7 +462,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------------ MMA issue (see elect_one)
-    const uint32_t idesc = make_idesc(P.n_pad), idesc_cross = make_idesc_bf16(P.n_pad), tmem = warp_uniform(tmem_base);
+    const uint32_t idesc = make_idesc(P.n_pad), tmem = warp_uniform(tmem_base);
     int tile_iter = 0;
     Ring ra, rb, rbar;  // A slot, weight slot, barrier pair of the current k-block
     for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x, ++tile_iter) {
@@ -482,22 +477,13 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         const uint64_t dbh = make_desc(b_hi), dbl = make_desc(b_lo);
         const uint32_t a_hi = tmem + a_col0 + (uint32_t)(ra.idx * 64), a_lo = a_hi + 32u;
         if (elect_one()) {
-          if (MIXED) {  // one accumulator; the second halves of the slot and of the weight tile are words of cross terms
 #pragma unroll
-            for (int j = 0; j < kBlockK / 8; ++j)
-              umma_bf16_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbl + (uint64_t)(j * 2), idesc_cross, kb == 0 && j == 0 ? 0u : 1u);
-#pragma unroll
-            for (int j = 0; j < kBlockK / 8; ++j)
-              umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + (uint64_t)(j * 2), idesc, 1u);
-          } else {
-#pragma unroll
-            for (int j = 0; j < kBlockK / 8; ++j) {
-              const uint64_t adv = (uint64_t)(j * 2);
-              const uint32_t add = kb == 0 && j == 0 ? 0u : 1u;
-              umma_tf32_ts(d_cross, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, add);
-              umma_tf32_ts(d_cross, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
-              umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, cross ? add : 1u);
-            }
+          for (int j = 0; j < kBlockK / 8; ++j) {
+            const uint64_t adv = (uint64_t)(j * 2);
+            const uint32_t add = kb == 0 && j == 0 ? 0u : 1u;
+            umma_tf32_ts(d_cross, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, add);
+            umma_tf32_ts(d_cross, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
+            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, cross ? add : 1u);
           }
           umma_commit(done_bar + 8u * rbar.idx);  // frees the A slot for the producers and the weight slot for the TMA thread
           if (kb == kblocks - 1) umma_commit(acc_full + 8u * buf);
@@ -678,13 +664,6 @@ __global__ void __launch_bounds__(128) gather_reduce_kernel(const __grid_constan
   }
 }
 
-// A value as the shared-memory operand B: hi and the low part or word.
-template <bool MIXED>
-__device__ __forceinline__ void split_lowered(float x, uint32_t& h, uint32_t& l) {
-  split_tf32_trunc(x, h, l);
-  if (MIXED) l = cross_word(__uint_as_float(l), x);
-}
-
 // ---------------------------------------------------------------------------------- weight-gradient kernel
 //
 // dW[kk][o] (+ the bias row) = sum over pixels of Lowered(X)[pix][kk] * dY[pix][o], split over pixel ranges.
@@ -748,10 +727,7 @@ __host__ __device__ inline WgSmem wg_smem(int n_pad, int subs, int stages) {
 // compile time every warp stages exactly 8*SUBS tap rows and NB channel rows per k-block, all loads of a k-block are
 // in flight together, and the shared-memory addresses are one per-warp base plus immediates: row warp+16*i of a
 // 128-byte-swizzled tile has the same swizzle phase ((warp+16*i) & 7 == warp & 7) for every i.
-// MIXED (more than 64 columns, chains of kMixedChain and more): cross terms in bf16 (cross_word), "lo" tiles are their words.
-// With two M-tiles per CTA: 64 images of 28 x 40 x 40 to 100 / 160 / 176 channels 47.6 -> 45.0, 60.3 -> 56.8, 63.8 -> 59.9 us.  One
-// M-tile with wide dY tiles stays with three tf32 products (200 channels 79.6 -> 89.4).
-template <int SUBS, int NB, bool MIXED>
+template <int SUBS, int NB>
 __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_constant__ WgradParams P) {
   pdl_wait();
   extern __shared__ uint8_t smem_raw[];
@@ -847,8 +823,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
 #pragma unroll
         for (int i = 0; i < kARows; ++i) {  // tile i/8 (hi then lo), row warp + 16*(i%8)
           uint32_t h, l;
-          if (MIXED) split_mixed_a(va[i], h, l);
-          else split_tf32_trunc(va[i], h, l);
+          split_tf32_trunc(va[i], h, l);
           uint8_t* dst = st + (i / 8) * 2 * kATile + (i % 8) * 2048;
           *reinterpret_cast<uint32_t*>(dst) = h;
           *reinterpret_cast<uint32_t*>(dst + kATile) = l;
@@ -886,7 +861,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
 #pragma unroll
         for (int i = 0; i < kDyRows; ++i) {
           uint32_t h, l;
-          split_lowered<MIXED>(vb[i], h, l);
+          split_tf32_trunc(vb[i], h, l);
           uint8_t* dst = st + i * (kWgDyWarps * 128);
           *reinterpret_cast<uint32_t*>(dst) = h;
           *reinterpret_cast<uint32_t*>(dst + kBTile) = l;
@@ -928,7 +903,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
     }
   } else {
     // ------------------------------------------------------------------ MMA issue (see elect_one)
-    const uint32_t idesc = make_idesc(kAccCols), idesc_cross = make_idesc_bf16(kAccCols), tmem = warp_uniform(tmem_base);
+    const uint32_t idesc = make_idesc(kAccCols), tmem = warp_uniform(tmem_base);
     const int n_subs = (int)warp_uniform((uint32_t)subs);
     Ring ring;
     for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(P.stages)) {
@@ -946,12 +921,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
             const uint64_t adv = (uint64_t)(j * 2);
-            if (MIXED) {
-              umma_bf16_ss(d_tmem, dal + adv, dbl + adv, idesc_cross, (kbl == 0 && j == 0) ? 0u : 1u);
-            } else {
-              umma_tf32_ss(d_tmem, dal + adv, dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
-              if (!kDual) umma_tf32_ss(d_tmem, dah + adv, dbl + adv, idesc, 1u);
-            }
+            umma_tf32_ss(d_tmem, dal + adv, dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
+            if (!kDual) umma_tf32_ss(d_tmem, dah + adv, dbl + adv, idesc, 1u);
             umma_tf32_ss(d_tmem, dah + adv, dbh + adv, idesc, 1u);
           }
         }
@@ -1005,22 +976,20 @@ constexpr int kTsWideTaps = 13, kTsWideRows = 2;  // taps that four blocks cover
 __device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // Splits taps 0 .. k - 1, which start at w[SHIFT], and stores them as lowered rows: row r at dst + off[r & 7] + (r & ~7) * 128.
-template <int SHIFT, bool MIXED>
+template <int SHIFT>
 __device__ __forceinline__ void store_wide(const float* w, int k, uint8_t* dst, const uint32_t* off) {
 #pragma unroll
   for (int r = 0; r < kTsWideTaps; ++r) {
     if (r >= k) break;
     uint32_t h, l;
-    split_lowered<MIXED>(w[SHIFT + r], h, l);
+    split_tf32_trunc(w[SHIFT + r], h, l);
     uint8_t* at = dst + off[r & 7] + (r & ~7) * 128;
     *reinterpret_cast<uint32_t*>(at) = h;
     *reinterpret_cast<uint32_t*>(at + kTsTile) = l;
   }
 }
 
-// MIXED (chains of kMixedChain and more): cross terms in bf16 (cross_word), "lo" operands are their words.  AlexNet conv1 at batch
-// 256 348 -> 346 us alone, 362 -> 349 within CaffeNet's iteration (the MMAs are not what bounds it, but take a third less power).
-template <bool WIDE, bool MIXED>
+template <bool WIDE>
 __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __grid_constant__ WgradParams P) {
   constexpr int kTsTapWarps = ts_tap_warps(WIDE), kTsDyWarps = ts_dy_warps(WIDE), kTsMmaWarp = kTsTapWarps + kTsDyWarps;
   constexpr int kTsThreads = ts_threads(WIDE), kTsRowsPerWarp = kTsRows / 24;  // 16
@@ -1141,16 +1110,16 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
           if (i >= mine) break;
           uint8_t* dst = base_ptr + (size_t)s * kTsStage;
           switch ((int)warp_uniform((uint32_t)shift[i])) {
-            case 0: store_wide<0, MIXED>(w[i], k, dst, lane_off[i]); break;
-            case 1: store_wide<1, MIXED>(w[i], k, dst, lane_off[i]); break;
-            case 2: store_wide<2, MIXED>(w[i], k, dst, lane_off[i]); break;
-            default: store_wide<3, MIXED>(w[i], k, dst, lane_off[i]); break;
+            case 0: store_wide<0>(w[i], k, dst, lane_off[i]); break;
+            case 1: store_wide<1>(w[i], k, dst, lane_off[i]); break;
+            case 2: store_wide<2>(w[i], k, dst, lane_off[i]); break;
+            default: store_wide<3>(w[i], k, dst, lane_off[i]); break;
           }
         }
         if (ones >= 0) {
           uint8_t* dst = base_ptr + (size_t)s * kTsStage + ones * 128 + (((lane >> 2) ^ (ones & 7)) << 4) + (lane & 3) * 4;
           *reinterpret_cast<float*>(dst) = ok ? 1.f : 0.f;
-          *reinterpret_cast<uint32_t*>(dst + kTsTile) = MIXED && ok ? cross_word(0.f, 1.f) : 0u;
+          *reinterpret_cast<float*>(dst + kTsTile) = 0.f;
         }
         if (kbl + 1 < kblocks) {  // the next k-block's loads go in flight before the barrier work
           next_pixel();
@@ -1194,7 +1163,7 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
 #pragma unroll
         for (int i = 0; i < kTsRowsPerWarp; ++i) {
           uint32_t h, l;
-          split_lowered<MIXED>(va[i], h, l);
+          split_tf32_trunc(va[i], h, l);
           uint8_t* dst = st + i * (kTsTapWarps * 128);
           *reinterpret_cast<uint32_t*>(dst) = h;
           *reinterpret_cast<uint32_t*>(dst + kTsTile) = l;
@@ -1257,11 +1226,7 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
         for (int c = 0; c < kChannels / 8; ++c) {  // lane = channel now: its pixels, eight at a time
           uint32_t hi[8], lo[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float x = turn[lane * 33 + half * kChannels + c * 8 + e];
-            if (MIXED) split_mixed_a(x, hi[e], lo[e]);
-            else split_tf32_trunc(x, hi[e], lo[e]);
-          }
+          for (int e = 0; e < 8; ++e) split_tf32_trunc(turn[lane * 33 + half * kChannels + c * 8 + e], hi[e], lo[e]);
           tmem_st8(st_addr + (uint32_t)(c * 8), hi);
           tmem_st8(st_addr + 32u + (uint32_t)(c * 8), lo);
         }
@@ -1286,7 +1251,7 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
     }
   } else {
     // ------------------------------------------------------------------ MMA issue (see elect_one)
-    const uint32_t idesc = make_idesc(kTsNTile), idesc_cross = make_idesc_bf16(kTsNTile), tmem = warp_uniform(tmem_base);
+    const uint32_t idesc = make_idesc(kTsNTile), tmem = warp_uniform(tmem_base);
     Ring ring;
     for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(kTsStages)) {
       const int s = ring.idx;
@@ -1302,12 +1267,8 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
             const uint64_t adv = (uint64_t)(j * 2);
-            if (MIXED) {
-              umma_bf16_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbl + adv, idesc_cross, (kbl == 0 && j == 0) ? 0u : 1u);
-            } else {
-              umma_tf32_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
-              umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
-            }
+            umma_tf32_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
+            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
             umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, 1u);
           }
         }
@@ -1323,24 +1284,22 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
 }
 
 typedef void (*WgradKernel)(const WgradParams);
-template <int SUBS, bool MIXED>
+template <int SUBS>
 WgradKernel wgrad_pick_nb(int nb) {
   switch (nb) {
-    case 1: return wgrad_kernel<SUBS, 1, false>;   case 2: return wgrad_kernel<SUBS, 2, false>;
-    case 3: return wgrad_kernel<SUBS, 3, false>;   case 4: return wgrad_kernel<SUBS, 4, false>;
-    case 5: return wgrad_kernel<SUBS, 5, MIXED>;   case 6: return wgrad_kernel<SUBS, 6, MIXED>;
-    case 7: return wgrad_kernel<SUBS, 7, MIXED>;   case 8: return wgrad_kernel<SUBS, 8, MIXED>;
-    case 9: return wgrad_kernel<SUBS, 9, MIXED>;   case 10: return wgrad_kernel<SUBS, 10, MIXED>;
-    case 11: return wgrad_kernel<SUBS, 11, MIXED>; case 12: return wgrad_kernel<SUBS, 12, MIXED>;
-    case 13: return wgrad_kernel<SUBS, 13, MIXED>; case 14: return wgrad_kernel<SUBS, 14, MIXED>;
-    case 15: return wgrad_kernel<SUBS, 15, MIXED>; case 16: return wgrad_kernel<SUBS, 16, MIXED>;
+    case 1: return wgrad_kernel<SUBS, 1>;   case 2: return wgrad_kernel<SUBS, 2>;
+    case 3: return wgrad_kernel<SUBS, 3>;   case 4: return wgrad_kernel<SUBS, 4>;
+    case 5: return wgrad_kernel<SUBS, 5>;   case 6: return wgrad_kernel<SUBS, 6>;
+    case 7: return wgrad_kernel<SUBS, 7>;   case 8: return wgrad_kernel<SUBS, 8>;
+    case 9: return wgrad_kernel<SUBS, 9>;   case 10: return wgrad_kernel<SUBS, 10>;
+    case 11: return wgrad_kernel<SUBS, 11>; case 12: return wgrad_kernel<SUBS, 12>;
+    case 13: return wgrad_kernel<SUBS, 13>; case 14: return wgrad_kernel<SUBS, 14>;
+    case 15: return wgrad_kernel<SUBS, 15>; case 16: return wgrad_kernel<SUBS, 16>;
   }
   return nullptr;
 }
-WgradKernel wgrad_pick(int subs, int n_pad, int chain) {
-  const int nb = n_pad / 16;
-  if (chain >= kMixedChain && subs == 2) return wgrad_pick_nb<2, true>(nb);
-  return subs == 2 ? wgrad_pick_nb<2, false>(nb) : wgrad_pick_nb<1, false>(nb);
+WgradKernel wgrad_pick(int subs, int n_pad) {
+  return subs == 2 ? wgrad_pick_nb<2>(n_pad / 16) : wgrad_pick_nb<1>(n_pad / 16);
 }
 
 }  // namespace
@@ -1353,14 +1312,10 @@ namespace {
 // conv3's 0.9 M weights 8.0 / 11.6 us for the two operands, bound by neither memory nor launch).
 constexpr int kPackThreads = 128;
 
-template <bool MIXED>
 __device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, const float* v) {
   float h[4], l[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    split_tf32(v[e], h[e], l[e]);
-    if (MIXED) l[e] = __uint_as_float(cross_word(l[e], v[e]));
-  }
+  for (int e = 0; e < 4; ++e) split_tf32(v[e], h[e], l[e]);
   *reinterpret_cast<float4*>(hi + at) = make_float4(h[0], h[1], h[2], h[3]);
   *reinterpret_cast<float4*>(lo + at) = make_float4(l[0], l[1], l[2], l[3]);
 }
@@ -1371,7 +1326,7 @@ __device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, co
 struct PackDgrad {
   const float* W;
   float *hi, *lo;
-  int tiles_per_group, og, Dg, k, s, taps, d_tile, n_real, n_pad, k_real, k_pad, run, mixed;
+  int tiles_per_group, og, Dg, k, s, taps, d_tile, n_real, n_pad, k_real, k_pad, run;
   int parts;   // blocks per row
   int blocks;  // rows * parts
 };
@@ -1403,8 +1358,7 @@ __device__ __forceinline__ void pack_dgrad_block(const PackDgrad& J, int block) 
         v[e] = (live && kk + e < J.k_real && kr < J.k && kc < J.k) ? __ldg(src + oc * filter + kr * J.k + kc) : 0.f;
       }
     }
-    if (J.mixed) store_split4<true>(J.hi, J.lo, row + kk, v);
-    else store_split4<false>(J.hi, J.lo, row + kk, v);
+    store_split4(J.hi, J.lo, row + kk, v);
   }
 }
 __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const __grid_constant__ PackDgrad J) {
@@ -1545,7 +1499,7 @@ __global__ void __launch_bounds__(32 * SLICES) wgrad_reduce_flat_kernel(const fl
 __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__ dY, float* __restrict__ hi,
                                                        float* __restrict__ lo, float* __restrict__ plane_sums,
                                                        int planes, int channels, int mm, int og, int ch_tile,
-                                                       int tiles_per_group, int n_pad, size_t row_len, int mixed) {
+                                                       int tiles_per_group, int n_pad, size_t row_len) {
   pdl_wait();
   // One warp per plane at a time in chunks of 256 elements, the next chunk's loads (of this plane or the warp's next one) in
   // flight while the current one is stored; no block-wide synchronisation.  One chunk at a time left planes of 169 elements at
@@ -1599,7 +1553,6 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
       const int i = q.i0 + u * 32 + lane;
       uint32_t h, l;
       split_tf32_trunc(x[u], h, l);
-      if (mixed) l = cross_word(__uint_as_float(l), x[u]);
       if (i >= 0 && i < mm) {
         hi[q.at + i] = __uint_as_float(h);
         lo[q.at + i] = __uint_as_float(l);
@@ -1622,7 +1575,6 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
 }
 
 // Forward B operand: [2 (hi, lo)][vg][n_pad][k_pad] <- W[o][Dg*k*k], zero padded.
-template <bool MIXED>
 __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                 float* __restrict__ lo, int tiles_per_group, int og,
                                                                 int n_real, int n_pad, int k_real, int k_pad, int run,
@@ -1640,7 +1592,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
     const int at = run == 1 ? kk : (chunk * kRun + (kk & (kRun - 1))) * window + (r - chunk * window), step = run == 1 ? 1 : window;
 #pragma unroll
     for (int e = 0; e < 4; ++e) v[e] = (live && kk + e < k_real) ? __ldg(src + at + e * step) : 0.f;
-    store_split4<MIXED>(hi, lo, row + kk, v);
+    store_split4(hi, lo, row + kk, v);
   }
 }
 
@@ -1751,7 +1703,6 @@ struct GatherProblem {
   int splits = 1, split_k = 0;    // splits of the reduction and the length of one (a multiple of 32; k_pad without splits)
   float* partial = nullptr;       // split sums
   size_t pix_pad = 0;
-  bool mixed = false;             // cross terms in bf16 (cross_word)
   int small_ct = 0;               // > 0: small_conv_kernel with this many channels per block instead of gather_conv_kernel
 };
 
@@ -1894,7 +1845,6 @@ void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias)
   if (two_ctas_per_sm(gp.n_pad, taps_smem, n_bias, ptab, &b_two)) {
     gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = acc <= 64 && !ptab ? 3 : 2; gp.b_stages = b_two;
   }
-  gp.mixed = gp.n_pad > kCrossCols && (gp.split_k ? gp.split_k : gp.k_pad) / kBlockK >= kMixedChain;  // see cross_word
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
   gp.w_half = (size_t)vgroups * gp.n_pad * map_k;
   mem.room(&gp.w, 2 * gp.w_half);
@@ -2164,17 +2114,13 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       rc = CCT_ERR_CUDA;
     }
   }
-  for (auto kernel : {gather_conv_kernel<4, kByTap, false>, gather_conv_kernel<4, kByRun, false>, gather_conv_kernel<4, kWeightGrad, false>,
-                      gather_conv_kernel<4, kByTap, true>, gather_conv_kernel<4, kByRun, true>, gather_conv_kernel<4, kWeightGrad, true>,
-                      gather_conv_kernel<4, kInside, false>, gather_conv_kernel<4, kInside, true>})
+  for (auto kernel : {gather_conv_kernel<4, kByTap>, gather_conv_kernel<4, kByRun>, gather_conv_kernel<4, kWeightGrad>, gather_conv_kernel<4, kInside>})
     if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
-  for (auto kernel : {gather_conv_kernel<2, kByTap, false>, gather_conv_kernel<2, kByRun, false>, gather_conv_kernel<2, kWeightGrad, false>,
-                      gather_conv_kernel<2, kByTap, true>, gather_conv_kernel<2, kByRun, true>, gather_conv_kernel<2, kWeightGrad, true>,
-                      gather_conv_kernel<2, kInside, false>, gather_conv_kernel<2, kInside, true>})
+  for (auto kernel : {gather_conv_kernel<2, kByTap>, gather_conv_kernel<2, kByRun>, gather_conv_kernel<2, kWeightGrad>, gather_conv_kernel<2, kInside>})
     if (rc == CCT_OK) rc = set_smem(ctx, kernel, 113 * 1024);
-  if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad, p->w_kblocks_per_split), kSmemLimit);
+  if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad), kSmemLimit);
   if (p->w_ts)
-    for (auto kernel : {wgrad_ts_kernel<false, false>, wgrad_ts_kernel<true, false>, wgrad_ts_kernel<false, true>, wgrad_ts_kernel<true, true>})
+    for (auto kernel : {wgrad_ts_kernel<false>, wgrad_ts_kernel<true>})
       if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
   if (rc != CCT_OK) {
     umma_plan_destroy(ctx, p);
@@ -2215,7 +2161,7 @@ void fill_common(GatherParams& P, const GatherProblem& gp, cct_ctx* ctx, int vgr
 PackDgrad pack_dgrad_job(const UmmaPlan* p, const float* W) {
   const ConvGeom& G = p->G;
   const GatherProblem& d = p->dgr;
-  PackDgrad J{W, d.w, d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run, (int)d.mixed, 0, 0};
+  PackDgrad J{W, d.w, d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run, 0, 0};
   J.parts = (d.k_pad / 4 + kPackThreads - 1) / kPackThreads;
   J.blocks = G.g * d.tiles * d.n_pad * J.parts;
   return J;
@@ -2245,19 +2191,15 @@ void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp,
     const int grid = std::min(P.total_tiles, (sets == 2 ? 2 : 1) * ctx->launch_sms());
     launch_pdl(kernel, dim3(grid), dim3(gather_threads(sets)), gp.smem, ctx->stream, P, gp.map);
   };
-  auto pick = [&](auto mixed) {
-    constexpr bool M = decltype(mixed)::value;
-    if (weight_grad) {
-      if (gp.sets == 2) go(gather_conv_kernel<2, kWeightGrad, M>, 2); else go(gather_conv_kernel<4, kWeightGrad, M>, 4);
-    } else if (gp.run == kRun) {
-      if (gp.sets == 2) go(gather_conv_kernel<2, kByRun, M>, 2); else go(gather_conv_kernel<4, kByRun, M>, 4);
-    } else if (gp.inside) {
-      if (gp.sets == 2) go(gather_conv_kernel<2, kInside, M>, 2); else go(gather_conv_kernel<4, kInside, M>, 4);
-    } else {
-      if (gp.sets == 2) go(gather_conv_kernel<2, kByTap, M>, 2); else go(gather_conv_kernel<4, kByTap, M>, 4);
-    }
-  };
-  if (gp.mixed) pick(std::true_type{}); else pick(std::false_type{});
+  if (weight_grad) {
+    if (gp.sets == 2) go(gather_conv_kernel<2, kWeightGrad>, 2); else go(gather_conv_kernel<4, kWeightGrad>, 4);
+  } else if (gp.run == kRun) {
+    if (gp.sets == 2) go(gather_conv_kernel<2, kByRun>, 2); else go(gather_conv_kernel<4, kByRun>, 4);
+  } else if (gp.inside) {
+    if (gp.sets == 2) go(gather_conv_kernel<2, kInside>, 2); else go(gather_conv_kernel<4, kInside>, 4);
+  } else {
+    if (gp.sets == 2) go(gather_conv_kernel<2, kByTap>, 2); else go(gather_conv_kernel<4, kByTap>, 4);
+  }
   if (P.splits > 1) {
     const int vgroups = P.total_tiles / (P.n_pix_tiles * P.splits), cols = P.n_pix_tiles * vgroups * P.n > 32 * ctx->sm_count ? 8 : 1;
     const int col_tiles = (P.n + cols - 1) / cols;
@@ -2285,7 +2227,7 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
   }
   if (repack) {
     t->begin(4, ctx->stream);
-    launch_pdl(f.mixed ? pack_fwd_kernel<true> : pack_fwd_kernel<false>, pack_grid(vgroups * f.n_pad, f.k_pad), dim3(kPackThreads), 0, ctx->stream, W, f.w,
+    launch_pdl(pack_fwd_kernel, pack_grid(vgroups * f.n_pad, f.k_pad), dim3(kPackThreads), 0, ctx->stream, W, f.w,
                f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad, f.run, G.k * G.k);
     t->end(4, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
@@ -2315,7 +2257,7 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
 
 bool umma_dy_rows(const UmmaPlan* p, DyRows* rows) {
   if (!p->wg_gather || !p->dgr_row_taps) return false;
-  *rows = DyRows{p->wgp.w, p->wgp.w_half, p->wgp.map_k, p->G.bias ? p->wg_plane_sums : nullptr, p->G.o, (int)p->wgp.mixed};
+  *rows = DyRows{p->wgp.w, p->wgp.w_half, p->wgp.map_k, p->G.bias ? p->wg_plane_sums : nullptr, p->G.o};
   return true;
 }
 
@@ -2341,7 +2283,7 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     if (dY)  // (else the kernel that made it has written the rows)
       launch_pdl(split_dy_kernel, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, 
         dY, w.w, w.w + w.w_half, G.bias ? p->wg_plane_sums : nullptr, G.B * G.o, G.o, mm, G.og, f.n, f.tiles,
-        f.n_pad, w.map_k, (int)w.mixed);
+        f.n_pad, w.map_k);
     CCT_CHECK_LAUNCH(ctx);
     GatherParams P{};
     P.in = X; P.out = p->w_partial; P.bias = nullptr;
@@ -2390,13 +2332,10 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       // Wide loads: see the kernel.  Below eight taps a window row has fewer than three blocks' worth.
       P.x_count = (int)((long long)G.B * G.D * G.n * G.n - (G.g - 1) * P.x_group_stride);
       const bool wide = G.s % 4 == 0 && G.p == 0 && G.k >= 8 && G.k <= kTsWideTaps && G.Dg * G.k <= kTsWideRows * ts_tap_warps(true);
-      const bool mixed = P.kblocks_per_split >= kMixedChain;
-      const auto kernel = wide ? (mixed ? wgrad_ts_kernel<true, true> : wgrad_ts_kernel<true, false>)
-                               : (mixed ? wgrad_ts_kernel<false, true> : wgrad_ts_kernel<false, false>);
-      launch_pdl(kernel, dim3(grid), dim3(ts_threads(wide)), p->w_smem, ctx->stream, P);
+      launch_pdl(wide ? wgrad_ts_kernel<true> : wgrad_ts_kernel<false>, dim3(grid), dim3(ts_threads(wide)), p->w_smem, ctx->stream, P);
     }
     else
-      launch_pdl(wgrad_pick(p->w_subs, f.n_pad, P.kblocks_per_split), dim3(grid), dim3(kWgThreads), p->w_smem, ctx->stream, P);
+      launch_pdl(wgrad_pick(p->w_subs, f.n_pad), dim3(grid), dim3(kWgThreads), p->w_smem, ctx->stream, P);
     t->end(1, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
     t->begin(2, ctx->stream);
@@ -2562,7 +2501,7 @@ extern "C" int cct_conv_weight_grad_noalloc(cct_ctx* ctx, const cct_conv_desc* d
 
   MaskTap* taps = reinterpret_cast<MaskTap*>(scratch);
   float* partial = reinterpret_cast<float*>(scratch + taps_bytes);
-  WgradKernel kernel = wgrad_pick(subs, n_pad, kblocks_per_split);
+  WgradKernel kernel = wgrad_pick(subs, n_pad);
   CCT_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
   launch_pdl(noalloc_taps_kernel, dim3(8), dim3(256), 0, ctx->stream, taps, m_tiles * kTileM, k_real, G.k, G.n);
   CCT_CHECK_LAUNCH(ctx);

@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
           const float l = x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
           if (i >= 0) {
             hi[i] = x;
-            hi[rows.lo + i] = rows.mixed ? __uint_as_float(cross_word(l, x)) : l;
+            hi[rows.lo + i] = l;
           }
           sum += x;
         }

@@ -14,7 +14,7 @@
 //
 // 3xTF32: kind::tf32 reads the upper 19 bits of every fp32 operand word, so the raw tile is the "hi" operand as it
 // stands; transform warps compute lo = x - hi element-wise into a second tile of the same layout (an element-wise pass
-// is layout-agnostic, so it serves both swizzles), and three MMAs per k-step (lo*hi + hi*lo + hi*hi; or two, MIXED) accumulate in
+// is layout-agnostic, so it serves both swizzles), and three MMAs per k-step (lo*hi + hi*lo + hi*hi) accumulate in
 // fp32 in tensor memory.  Long reductions are split over CTAs (bounded accumulation chains, as in the convolution
 // kernels); a small kernel adds the partial sums in split order and applies bias / ReLU / dropout (forward) or the
 // masks of the bridges in front of the layer (data gradient).
@@ -74,8 +74,7 @@ __device__ __forceinline__ void fc_store_3d(const void* tmap, uint32_t src, int 
                : "memory");
 }
 
-// What bounds it: at batch 256 the shared-memory port (a k-block of 256 columns: operand reads 64 KB, TMA writes 48, the
-// transform's reads and writes 80, at 128 bytes a cycle half as much again as its 8 MMAs take), at small batches the stream of W (or,
+// What bounds it: at batch 256 the tensor pipe (12 MMAs of N / 2 cycles per k-block), at small batches the stream of W (or,
 // for the weight gradient, of dW) - so the same roles in two shapes.
 //   N > 128 columns: one CTA per SM, the whole batch in one accumulator, so that a weight tile is split into tensor memory
 //   once (two CTAs with half the batch each split it twice and waited for it: 61 % of the tensor pipe, now see below).
@@ -87,9 +86,6 @@ __device__ __forceinline__ void fc_store_3d(const void* tmap, uint32_t src, int 
 // The epilogue turns 32 accumulator columns at a time into a 32 x 32 tile in shared memory (one conflict-free store per
 // column) that TMA stores take out, clipping it at the edges: per-lane global stores with their addresses and bounds cost
 // about ten instructions each and made the weight gradient of small batches instruction-bound (fc6, batch 32: 70 us, 2.1 TB/s).
-// MIXED: cross terms in bf16 (cross_word), the "lo" tile and slots hold their words.  fc6 at batch 256, forward 82.4 -> 74.8 us,
-// data gradient 75.6 -> 68.5; errors against 64-bit sums 1.6e-5 -> 1.1e-5, 1.5e-5 -> 1.0e-5.
-template <bool MIXED>
 __global__ void __launch_bounds__(kFcThreads, 2)
     fc_gemm_kernel(const __grid_constant__ FcGemmParams P, const __grid_constant__ CUtensorMap a_map,
                    const __grid_constant__ CUtensorMap b_map, const __grid_constant__ CUtensorMap out_map) {
@@ -167,7 +163,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
     }
   } else if (warp == kFcMmaWarp) {  // see elect_one
     const uint32_t idesc = make_idesc(P.n_pad) | (P.b_mn ? 1u << 16 : 0u);  // A from tensor memory: lanes x K
-    const uint32_t idesc_cross = make_idesc_bf16(P.n_pad), tmem = warp_uniform(tmem_base);
+    const uint32_t tmem = warp_uniform(tmem_base);
     Ring raw, lo, ta;
     int i = 0, tile_iter = 0;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_iter) {
@@ -185,23 +181,14 @@ __global__ void __launch_bounds__(kFcThreads, 2)
         const uint32_t b_lo = base + L.lo_off + (uint32_t)lo.idx * L.b_tile_bytes;
         const uint32_t t_hi = tmem + a_col0 + (uint32_t)(ta.idx * 64), t_lo = t_hi + 32u;
         if (elect_one()) {
-          if (MIXED) {
-            const uint64_t bh = make_desc(b_raw), bl = make_desc(b_lo);
 #pragma unroll
-            for (int j = 0; j < kBlockK / 8; ++j)
-              umma_bf16_ts(d_tmem, t_lo + (uint32_t)(j * 8), bl + (uint64_t)(j * 2), idesc_cross, (kb == kb0 && j == 0) ? 0u : 1u);
-#pragma unroll
-            for (int j = 0; j < kBlockK / 8; ++j) umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bh + (uint64_t)(j * 2), idesc, 1u);
-          } else {
-#pragma unroll
-            for (int j = 0; j < kBlockK / 8; ++j) {
-              // K-major: 8 reduction indices = 32 bytes along the swizzled row; MN-major: 8 rows of 128 bytes
-              const uint64_t bh = P.b_mn ? make_desc_mn(b_raw + j * 1024u) : make_desc(b_raw) + (uint64_t)(j * 2);
-              const uint64_t bl = P.b_mn ? make_desc_mn(b_lo + j * 1024u) : make_desc(b_lo) + (uint64_t)(j * 2);
-              umma_tf32_ts(d_tmem, t_lo + (uint32_t)(j * 8), bh, idesc, (kb == kb0 && j == 0) ? 0u : 1u);
-              umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bl, idesc, 1u);
-              umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bh, idesc, 1u);
-            }
+          for (int j = 0; j < kBlockK / 8; ++j) {
+            // K-major: 8 reduction indices = 32 bytes along the swizzled row; MN-major: 8 rows of 128 bytes
+            const uint64_t bh = P.b_mn ? make_desc_mn(b_raw + j * 1024u) : make_desc(b_raw) + (uint64_t)(j * 2);
+            const uint64_t bl = P.b_mn ? make_desc_mn(b_lo + j * 1024u) : make_desc(b_lo) + (uint64_t)(j * 2);
+            umma_tf32_ts(d_tmem, t_lo + (uint32_t)(j * 8), bh, idesc, (kb == kb0 && j == 0) ? 0u : 1u);
+            umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bl, idesc, 1u);
+            umma_tf32_ts(d_tmem, t_hi + (uint32_t)(j * 8), bh, idesc, 1u);
           }
           umma_commit(done_bar + 8u * (i & 3));
           if (kb == kb1 - 1) umma_commit(acc_full + 8u * buf);
@@ -255,10 +242,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
         for (int c = 0; c < 2; ++c) {
           uint32_t hi[8], l8[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            if (MIXED) split_mixed_a(x[c * 8 + e], hi[e], l8[e]);
-            else split_tf32_trunc(x[c * 8 + e], hi[e], l8[e]);
-          }
+          for (int e = 0; e < 8; ++e) split_tf32_trunc(x[c * 8 + e], hi[e], l8[e]);
           tmem_st8(taddr + (uint32_t)(c * 8), hi);
           tmem_st8(taddr + 32u + (uint32_t)(c * 8), l8);
         }
@@ -272,12 +256,6 @@ __global__ void __launch_bounds__(kFcThreads, 2)
           l.y = r.y - __uint_as_float(__float_as_uint(r.y) & 0xFFFFE000u);
           l.z = r.z - __uint_as_float(__float_as_uint(r.z) & 0xFFFFE000u);
           l.w = r.w - __uint_as_float(__float_as_uint(r.w) & 0xFFFFE000u);
-          if (MIXED) {
-            l.x = __uint_as_float(cross_word(l.x, r.x));
-            l.y = __uint_as_float(cross_word(l.y, r.y));
-            l.z = __uint_as_float(cross_word(l.z, r.z));
-            l.w = __uint_as_float(cross_word(l.w, r.w));
-          }
           b_lo[v] = l;
         }
         fence_proxy_async_smem();
@@ -635,10 +613,7 @@ int fc_launch(cct_ctx* ctx, const FcShape& s, const FcMap& a, const FcMap& b, co
   P.direct = direct; P.ld_direct = ld_direct;
   P.status = ctx->status_dev;
   const int tiles = P.m_tiles * P.n_tiles * P.splits;
-  // Cross terms in bf16: a B that is K-major (the words pair what follows along K) and chains for which they are the more accurate
-  // form; at batch 32, where the stream of W is the bound, that is all they change.
-  const bool mixed = !P.b_mn && P.kblocks_per_split >= kMixedChain;
-  launch_pdl(mixed ? fc_gemm_kernel<true> : fc_gemm_kernel<false>, dim3(std::min(tiles, (s.pair ? 2 : 1) * ctx->launch_sms())), dim3(kFcThreads), s.smem, ctx->stream, P,
+  launch_pdl(fc_gemm_kernel, dim3(std::min(tiles, (s.pair ? 2 : 1) * ctx->launch_sms())), dim3(kFcThreads), s.smem, ctx->stream, P,
              a.map, b.map, out.map);
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
@@ -731,8 +706,7 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   float* at = p->partial + room(sums);
   if (pad_k) { p->Xp = at; p->Wp = at + x; }
   if (pad_o) p->dYp = at + x + w;
-  cudaError_t e = cudaFuncSetAttribute(fc_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+  const cudaError_t e = cudaFuncSetAttribute(fc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   if (e != cudaSuccess) {
     ctx->last_error = std::string("cudaFuncSetAttribute(fc_gemm_kernel): ") + cudaGetErrorString(e);
     cudaFree(p->partial);

@@ -129,10 +129,6 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
 __host__ __device__ constexpr uint32_t make_idesc(int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
 }
-// kind::f16 with bf16 A and B, otherwise the same.
-__host__ __device__ constexpr uint32_t make_idesc_bf16(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
-}
 
 // hi = x rounded to tf32 (10 explicit mantissa bits), lo = x - hi (exact in fp32).
 __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
@@ -144,25 +140,6 @@ __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
 __device__ __forceinline__ void split_tf32_trunc(float x, uint32_t& hi, uint32_t& lo) {
   hi = __float_as_uint(x) & 0xFFFFE000u;
   lo = __float_as_uint(x - __uint_as_float(hi));
-}
-
-// Cross terms in bf16.  lo needs no more than bf16's eight bits (and has fp32's exponents there), and for hi * lo eight bits of
-// hi do as well.  One word then holds what a value contributes to both cross terms: (x, lo) of A against (lo, x) of B, lower half
-// first, is x_a * lo_b + lo_a * x_b.  kind::f16 takes 16 reduction indices where kind::tf32 takes 8, in the same time: a block
-// of 32 values is 4 + 4 MMAs instead of 4 + 8, and has two truncating additions per eight products instead of three.  What it
-// costs is 2^-9 of lo per term: 1.0e-6 of a sum of products of random sign, whatever its length, where the additions cost
-// 9.5e-9 per product with 3xTF32 in one accumulator (relative 2-norms).  Hence kMixedChain: 64 products 0.7e-6 -> 1.1e-6, 128
-// 1.24 -> 1.29, 192 1.8 -> 1.5, 512 4.9 -> 3.3, 1024 9.6 -> 6.3.  Tiles with an accumulator for the cross terms stay with 3xTF32:
-// they would gain accuracy from 2 000 products on only, and what bounds them is the producers' instructions (one more per
-// value: CaffeNet conv2's data gradient 541 -> 574 us).
-// CaffeNet at batch 256, forward / weight gradient / data gradient, us: conv2 407 -> 317 / 405 -> 359 / -, conv3 263 -> 195 /
-// 257 -> 194 / 271 -> 208, conv4 215 -> 162 / 211 -> 161 / 216 -> 159, conv5 144 -> 111 / 157 -> 141 / 153 -> 113.
-constexpr int kMixedChain = 8;  // k-blocks of 32 of an accumulation chain from which on it is the more accurate form
-// (cross_word itself: cct_internal.h, for the kernels that write operands)
-// hi = x truncated to tf32 and A's word of the cross terms.
-__device__ __forceinline__ void split_mixed_a(float x, uint32_t& hi, uint32_t& word) {
-  hi = __float_as_uint(x) & 0xFFFFE000u;
-  word = cross_word(x, x - __uint_as_float(hi));
 }
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
@@ -190,17 +167,6 @@ __device__ __forceinline__ void umma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, u
       : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// The same with bf16 operands: 16 of them along K, two to a word of A's tensor memory and of B's shared memory.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      :
-      : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
                "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -216,18 +182,6 @@ __device__ __forceinline__ void umma_tf32_ss(uint32_t d_tmem, uint64_t a_desc, u
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      :
-      : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same with bf16 operands (16 along K).
-__device__ __forceinline__ void umma_bf16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       :
       : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");

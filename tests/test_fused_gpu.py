@@ -122,7 +122,7 @@ def test_fused_backward_argument_checks(ctx):
 
 # With the pooled tensor at hand the masked gradient goes straight into the rows that the contractions read, where the weight
 # gradient is a gather over at least 512 lowered rows and the channel tiles are multiples of 16: one and two tiles, groups, planes
-# of 25 to 729 elements, chains on both sides of the line for bf16 cross terms; uneven tiles, planes too large for the kernel and
+# of 25 to 729 elements; uneven tiles, planes too large for the kernel and
 # other windows, which take the cube.  Bit-identical to the cube's path.
 @pytest.mark.parametrize("shape", [
     (3, 64, 15, 48, 3, 1, 1, 1, 3, 2), (2, 128, 20, 160, 3, 1, 1, 2, 3, 2), (5, 64, 5, 16, 3, 1, 1, 1, 3, 2), (70, 64, 7, 256, 3, 1, 1, 1, 3, 2),
