@@ -449,6 +449,10 @@ __global__ void __launch_bounds__(256) fc_pad_kernel(const float* __restrict__ s
 }
 
 int fc_round_up(int v, int a) { return (v + a - 1) / a * a; }
+bool fc_overlap(const float* a, size_t a_count, const float* b, size_t b_count) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + b_count * sizeof(float) && y < x + a_count * sizeof(float);
+}
 
 }  // namespace
 #include "fc_small.cuh"
@@ -801,8 +805,10 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
       rc = fc_launch(ctx, plan->wgr, plan->x_wgr, plan->dy_wgr, direct ? plan->x_wgr : plan->out_wgr, direct ? dW : nullptr, K);
     if (rc != CCT_OK) return rc;
     if (plan->bias) {
+      // With the data gradient's reduction, unless there is none, or it writes where the sum reads (dX over dY).
       bias_sum = FcBiasSum{dY, db, B, O};
-      if (!dX || (d_small && fc_small_pass_splits(plan, plan->small_dgr, plan->dgr) == 1)) {  // no reduction follows
+      if (!dX || (d_small && fc_small_pass_splits(plan, plan->small_dgr, plan->dgr) == 1) ||
+          fc_overlap(dX, (size_t)B * K, dY, (size_t)B * O)) {
         launch_pdl(fc_bias_grad_kernel, dim3((O + 31) / 32), dim3(256), 0, ctx->stream, bias_sum);
         bias_sum = FcBiasSum{};
       }

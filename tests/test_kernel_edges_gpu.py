@@ -341,6 +341,30 @@ def test_inner_product_long_chains(ctx, B, K, o):
         assert err <= 4 * 3 * (min(products, 96 * 32) // 32 + 1) * 2.0 ** -23.9 + 2.0 ** -21, "relative error %.2e" % err
 
 
+# dX written over dY, the whole of it or a part, where the bias gradient would ride with the launch that writes dX: bit for bit what
+# separate buffers give, every time.
+@pytest.mark.parametrize("B,K,shift", [(256, 1024, 0), (40, 2048, 0), (130, 1024, 64), (130, 1024, -64)])
+def test_inner_product_gradient_in_place(ctx, B, K, shift):
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    make = lambda *sh: torch.randn(sh, generator=gen, device="cuda")  # noqa: E731
+    X, W, dY = make(B, K), make(K, K), make(B, K)
+    apart, dWs, dbs = torch.zeros_like(X), [torch.zeros_like(W) for _ in range(2)], [torch.zeros(K, device="cuda") for _ in range(2)]
+    both, plan, q = torch.zeros(B * K + 128, device="cuda"), C.c_void_p(), lambda t: t.data_ptr()
+    over, inside = both[64:64 + B * K], both[64 + shift:64 + shift + B * K]  # dY, dX
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, K, 1, C.byref(plan)), "plan", ctx.h)
+    run = lambda dy, dx, k: capi.check(ctx.lib.cct_fc_backward(plan, q(X), q(W), q(dy), q(dx), q(dWs[k]), q(dbs[k]), 0, None, 1.0),  # noqa: E731
+                                       "backward", ctx.h)
+    run(dY, apart, 0)
+    for _ in range(5):
+        over.copy_(dY.view(-1))
+        torch.cuda.synchronize()
+        run(over, inside, 1)
+        ctx.sync()
+        assert torch.equal(inside.view(B, K), apart) and torch.equal(dWs[0], dWs[1]) and torch.equal(dbs[0], dbs[1])
+    ctx.lib.cct_fc_plan_destroy(plan)
+
+
 # Operands four bytes off a 16-byte boundary, which no tensor map describes: all of them, or one at a time, with feature counts
 # that are and are not multiples of four, above the size of the fp32 kernel.  Tolerance as above.
 @pytest.mark.parametrize("B,K,o", [(129, 772, 1027), (129, 770, 1028), (130, 1024, 512), (40, 2051, 1030)])
