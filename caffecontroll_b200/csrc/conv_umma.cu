@@ -1404,15 +1404,20 @@ __device__ __forceinline__ bool extra_block(const ReduceExtras& E, int first) {
   if (block < E.bias.blocks) bias_grad_block(E.bias, block);
   return true;
 }
+// A reduction with nothing beside it (small layers, whose gradients need neither) is a kernel without that code: with it a network
+// of 10 images, two such reductions of 4 us in its iteration, took 88.0 us instead of 86.2.
+struct NoExtras {};
+__device__ __forceinline__ bool extra_block(const NoExtras&, int) { return false; }
 
 // dW[o][kk] and db[o] from the split partial sums, added in split order (deterministic).  One block per 32 x 32
 // tile of (kk, channel): the partial sums are read along the channels (their fastest index), the tile is turned in
 // shared memory, and dW is written along kk (its fastest index) - both sides coalesced, no division per element.
+template <class Extras>
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dW,
                                                            float* __restrict__ db, int splits, int vgroups,
                                                            int tiles_per_group, int rows_pad, int n_real, int n_pad,
                                                            int k_real, int og, int accumulate, int row_tiles, int col_tiles,
-                                                           const __grid_constant__ ReduceExtras extras) {
+                                                           const __grid_constant__ Extras extras) {
   pdl_wait();
   __shared__ float tile[32][33];
   if (extra_block(extras, row_tiles * col_tiles * vgroups)) return;
@@ -1455,13 +1460,13 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
 // elements of the partial sums' (row, channel) plane and SLICES interleaved slices of the splits, the slice sums added in a
 // fixed order - the result does not depend on the grid, and a thread's chain is splits / SLICES long.  dW is written
 // without coalescing (a few ten thousand elements).
-template <int SLICES>
+template <int SLICES, class Extras>
 __global__ void __launch_bounds__(32 * SLICES) wgrad_reduce_flat_kernel(const float* __restrict__ partial,
                                                                         float* __restrict__ dW, float* __restrict__ db,
                                                                         int splits, int vgroups, int tiles_per_group,
                                                                         int rows_pad, int n_real, int n_pad, int k_real,
                                                                         int og, int accumulate, int per_group,
-                                                                        const __grid_constant__ ReduceExtras extras) {
+                                                                        const __grid_constant__ Extras extras) {
   pdl_wait();
   __shared__ float part[SLICES][33];
   if (extra_block(extras, per_group * vgroups)) return;
@@ -1782,29 +1787,38 @@ int set_smem(cct_ctx* ctx, K kernel, size_t bytes) {
   return CCT_OK;
 }
 
-// Split reduction: tiles when they fill the machine, the flat form otherwise (both add in a fixed order).  `extras`: see there;
-// their block counts are set here, for the block size that is taken.
-void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* db, int splits, int vgroups,
-                         int tiles_per_group, int rows_pad, int n_real, int n_pad, int k_real, int og,
-                         int accumulate = 0, ReduceExtras extras = ReduceExtras()) {
-  auto extra_blocks = [&](int threads) {
-    if (extras.bias.db) extras.bias.blocks = (extras.bias.channels + threads / 32 - 1) / (threads / 32);
-    return extras.pack.blocks + extras.bias.blocks;
+// Blocks that go with a reduction; those of the bias gradient are counted here, for the block size that is taken.
+int extra_blocks(ReduceExtras& E, int threads) {
+  if (E.bias.db) E.bias.blocks = (E.bias.channels + threads / 32 - 1) / (threads / 32);
+  return E.pack.blocks + E.bias.blocks;
+}
+int extra_blocks(NoExtras&, int) { return 0; }
+
+// Split reduction: tiles when they fill the machine, the flat form otherwise (both add in a fixed order).
+template <class Extras>
+void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* db, int splits, int vgroups, int tiles_per_group,
+                         int rows_pad, int n_real, int n_pad, int k_real, int og, int accumulate, Extras extras) {
+  auto go = [&](auto kernel, int threads, int blocks, auto... shape) {
+    blocks += extra_blocks(extras, threads);
+    launch_pdl(kernel, dim3(blocks), dim3(threads), 0, ctx->stream, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real,
+               n_pad, k_real, og, accumulate, shape..., extras);
   };
-  const int row_tiles = (k_real + 1 + 31) / 32, col_tiles = (n_real + 31) / 32;
-  if (row_tiles * col_tiles * vgroups >= ctx->sm_count)
-    launch_pdl(wgrad_reduce_kernel, dim3(row_tiles * col_tiles * vgroups + extra_blocks(256)), dim3(256), 0, ctx->stream, partial, dW, db,
-               splits, vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate, row_tiles, col_tiles, extras);
-  else {
-    const int per_group = ((k_real + 1) * n_pad + 31) / 32;
-    auto go = [&](auto kernel, int slices) {
-      launch_pdl(kernel, dim3(per_group * vgroups + extra_blocks(32 * slices)), dim3(32 * slices), 0, ctx->stream, partial, dW, db, splits,
-                 vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate, per_group, extras);
-    };
-    if (splits < 16) go(wgrad_reduce_flat_kernel<4>, 4);
-    else if (splits < 64 || per_group * vgroups > 2 * ctx->sm_count) go(wgrad_reduce_flat_kernel<8>, 8);
-    else go(wgrad_reduce_flat_kernel<32>, 32);
-  }
+  const int row_tiles = (k_real + 1 + 31) / 32, col_tiles = (n_real + 31) / 32, per_group = ((k_real + 1) * n_pad + 31) / 32;
+  const int tiles = row_tiles * col_tiles * vgroups, flat = per_group * vgroups;
+  if (tiles >= ctx->sm_count) go(wgrad_reduce_kernel<Extras>, 256, tiles, row_tiles, col_tiles);
+  else if (splits < 16) go(wgrad_reduce_flat_kernel<4, Extras>, 128, flat, per_group);
+  else if (splits < 64 || flat > 2 * ctx->sm_count) go(wgrad_reduce_flat_kernel<8, Extras>, 256, flat, per_group);
+  else go(wgrad_reduce_flat_kernel<32, Extras>, 1024, flat, per_group);
+}
+void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* db, int splits, int vgroups, int tiles_per_group,
+                         int rows_pad, int n_real, int n_pad, int k_real, int og, int accumulate = 0,
+                         const ReduceExtras& extras = ReduceExtras()) {
+  if (extras.pack.blocks || extras.bias.db)
+    launch_wgrad_reduce<ReduceExtras>(ctx, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate,
+                                      extras);
+  else
+    launch_wgrad_reduce<NoExtras>(ctx, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate,
+                                  NoExtras());
 }
 
 dim3 pack_grid(int rows, int k_pad) { return dim3(rows, (k_pad / 4 + kPackThreads - 1) / kPackThreads); }
