@@ -1739,6 +1739,25 @@ struct UmmaPlan {
   size_t bytes = 0;
 };
 
+namespace {
+typedef void (*GatherKernel)(const GatherParams, const CUtensorMap);
+GatherKernel gather_kernel(const GatherProblem& gp, bool weight_grad) {
+  const bool two = gp.sets == 2;
+  if (weight_grad) return two ? gather_conv_kernel<2, kWeightGrad> : gather_conv_kernel<4, kWeightGrad>;
+  if (gp.run == kRun) return two ? gather_conv_kernel<2, kByRun> : gather_conv_kernel<4, kByRun>;
+  if (gp.inside) return two ? gather_conv_kernel<2, kInside> : gather_conv_kernel<4, kInside>;
+  return two ? gather_conv_kernel<2, kByTap> : gather_conv_kernel<4, kByTap>;
+}
+// wgrad_ts_kernel's wide loads: see there.  Below eight taps a window row has fewer than three blocks' worth.
+bool ts_wide(const ConvGeom& G) {
+  return G.s % 4 == 0 && G.p == 0 && G.k >= 8 && G.k <= kTsWideTaps && G.Dg * G.k <= kTsWideRows * ts_tap_warps(true);
+}
+WgradKernel short_wgrad_kernel(const UmmaPlan* p) {
+  if (!p->w_ts) return wgrad_pick(p->w_subs, p->w_npad);
+  return ts_wide(p->G) ? wgrad_ts_kernel<true> : wgrad_ts_kernel<false>;
+}
+}  // namespace
+
 bool umma_supported(const ConvGeom& G) {
   if (channel_tiles(G.og, 1) == 0 || channel_tiles(G.Dg, G.s * G.s) == 0) return false;
   if (G.k > kMaxTapsPerAxis || G.n > 8000) return false;  // tap rows / columns are bits of a 32-bit validity mask
@@ -2128,14 +2147,10 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       rc = CCT_ERR_CUDA;
     }
   }
-  for (auto kernel : {gather_conv_kernel<4, kByTap>, gather_conv_kernel<4, kByRun>, gather_conv_kernel<4, kWeightGrad>, gather_conv_kernel<4, kInside>})
-    if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
-  for (auto kernel : {gather_conv_kernel<2, kByTap>, gather_conv_kernel<2, kByRun>, gather_conv_kernel<2, kWeightGrad>, gather_conv_kernel<2, kInside>})
-    if (rc == CCT_OK) rc = set_smem(ctx, kernel, 113 * 1024);
-  if (rc == CCT_OK) rc = set_smem(ctx, wgrad_pick(p->w_subs, p->w_npad), kSmemLimit);
-  if (p->w_ts)
-    for (auto kernel : {wgrad_ts_kernel<false>, wgrad_ts_kernel<true>})
-      if (rc == CCT_OK) rc = set_smem(ctx, kernel, kSmemLimit);
+  // The kernels that this plan launches, and no others: each is one to load at its first use.
+  for (const GatherProblem* gp : {&p->fwd, &p->dgr, &p->wgp})
+    if (rc == CCT_OK && gp->w) rc = set_smem(ctx, gather_kernel(*gp, gp == &p->wgp), gp->sets == 2 ? 113 * 1024 : kSmemLimit);
+  if (rc == CCT_OK && !p->w_small && !p->wg_gather) rc = set_smem(ctx, short_wgrad_kernel(p), kSmemLimit);
   if (rc != CCT_OK) {
     umma_plan_destroy(ctx, p);
     return rc;
@@ -2201,19 +2216,8 @@ void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct) {
 
 // Persistent grid: one CTA per SM (4 producer sets) or two (2 sets); then the reduction over the splits, if any.
 void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp, bool weight_grad = false) {
-  auto go = [&](auto kernel, int sets) {
-    const int grid = std::min(P.total_tiles, (sets == 2 ? 2 : 1) * ctx->launch_sms());
-    launch_pdl(kernel, dim3(grid), dim3(gather_threads(sets)), gp.smem, ctx->stream, P, gp.map);
-  };
-  if (weight_grad) {
-    if (gp.sets == 2) go(gather_conv_kernel<2, kWeightGrad>, 2); else go(gather_conv_kernel<4, kWeightGrad>, 4);
-  } else if (gp.run == kRun) {
-    if (gp.sets == 2) go(gather_conv_kernel<2, kByRun>, 2); else go(gather_conv_kernel<4, kByRun>, 4);
-  } else if (gp.inside) {
-    if (gp.sets == 2) go(gather_conv_kernel<2, kInside>, 2); else go(gather_conv_kernel<4, kInside>, 4);
-  } else {
-    if (gp.sets == 2) go(gather_conv_kernel<2, kByTap>, 2); else go(gather_conv_kernel<4, kByTap>, 4);
-  }
+  const int grid = std::min(P.total_tiles, (gp.sets == 2 ? 2 : 1) * ctx->launch_sms());
+  launch_pdl(gather_kernel(gp, weight_grad), dim3(grid), dim3(gather_threads(gp.sets)), gp.smem, ctx->stream, P, gp.map);
   if (P.splits > 1) {
     const int vgroups = P.total_tiles / (P.n_pix_tiles * P.splits), cols = P.n_pix_tiles * vgroups * P.n > 32 * ctx->sm_count ? 8 : 1;
     const int col_tiles = (P.n + cols - 1) / cols;
@@ -2342,14 +2346,10 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       rows_pad = p->ws_rows * kSwTile;
       launch_pdl(small_wgrad_kernel, dim3(p->ws_rows * p->ws_cols * vgroups, p->w_splits), dim3(kSwThreads), 0, ctx->stream, P,
                  rows_pad, p->ws_rows, p->ws_cols, p->ws_pix);
-    } else if (p->w_ts) {
-      // Wide loads: see the kernel.  Below eight taps a window row has fewer than three blocks' worth.
-      P.x_count = (int)((long long)G.B * G.D * G.n * G.n - (G.g - 1) * P.x_group_stride);
-      const bool wide = G.s % 4 == 0 && G.p == 0 && G.k >= 8 && G.k <= kTsWideTaps && G.Dg * G.k <= kTsWideRows * ts_tap_warps(true);
-      launch_pdl(wide ? wgrad_ts_kernel<true> : wgrad_ts_kernel<false>, dim3(grid), dim3(ts_threads(wide)), p->w_smem, ctx->stream, P);
+    } else {
+      if (p->w_ts) P.x_count = (int)((long long)G.B * G.D * G.n * G.n - (G.g - 1) * P.x_group_stride);
+      launch_pdl(short_wgrad_kernel(p), dim3(grid), dim3(p->w_ts ? ts_threads(ts_wide(G)) : kWgThreads), p->w_smem, ctx->stream, P);
     }
-    else
-      launch_pdl(wgrad_pick(p->w_subs, f.n_pad), dim3(grid), dim3(kWgThreads), p->w_smem, ctx->stream, P);
     t->end(1, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
     t->begin(2, ctx->stream);
