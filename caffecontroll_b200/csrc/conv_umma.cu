@@ -2106,6 +2106,18 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     w.k_pad = p->wg_kps * kBlockK;
     w.taps_smem = 0;
     w.map_k = (size_t)kb_total * kBlockK;
+    // dY in rows serves the data gradient too, where rows are channels and the offsets fit.  (Its table goes before the next one, which
+    // is long: behind it, it made the tables grow, and the long one was copied once more.)
+    if (w.n == w.n_pad && w.tiles * w.n == G.og && !p->dgr.small_ct && (double)G.o * w.map_k < 2147483648.0) {
+      const GatherProblem& d = p->dgr;
+      const int J = p->dgr_taps;
+      std::vector<MaskTap> rt((size_t)d.splits * d.split_k / d.run, MaskTap{0, kPadBit});
+      for (int i = 0; i * d.run < d.k_real; ++i) {
+        const int jx = i % J, jy = (i / J) % J, oc = i / (J * J) * d.run;
+        rt[i] = MaskTap{(int)(oc * w.map_k) - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
+      }
+      mem.table(&p->dgr_row_taps, rt);
+    }
     // Per-pixel table: where the pixel's window starts, and which of its rows and columns lie outside the plane.
     std::vector<uint32_t> outside(G.m);  // the same for rows and columns: bit a = window row a of output row r is outside
     for (int r = 0; r < G.m; ++r)
@@ -2121,17 +2133,6 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     mem.table(&p->wg_pix, t);
     finish_problem(mem, w, vgroups, 0);
     if (G.bias) mem.room(&p->wg_plane_sums, (size_t)G.B * G.o);
-    // dY in rows serves the data gradient too, where rows are channels and the offsets fit.
-    if (w.n == w.n_pad && w.tiles * w.n == G.og && !p->dgr.small_ct && (double)G.o * w.map_k < 2147483648.0) {
-      const GatherProblem& d = p->dgr;
-      const int J = p->dgr_taps;
-      std::vector<MaskTap> rt((size_t)d.splits * d.split_k / d.run, MaskTap{0, kPadBit});
-      for (int i = 0; i * d.run < d.k_real; ++i) {
-        const int jx = i % J, jy = (i / J) % J, oc = i / (J * J) * d.run;
-        rt[i] = MaskTap{(int)(oc * w.map_k) - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
-      }
-      mem.table(&p->dgr_row_taps, rt);
-    }
     sums = std::max(sums, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
   }
   float* sum_memory = nullptr;
