@@ -186,9 +186,11 @@ int cct_conv_weight_grad_noalloc(cct_ctx* ctx, const cct_conv_desc* desc, const 
 
 /* Per-kernel device times of the plan's most recent forward and backward call, for measurement: when enabled,
  * CUDA events are recorded around each kernel group on the context's stream.  ms[0] forward contraction,
- * ms[1] weight(+bias)-gradient contraction, ms[2] its split reduction, ms[3] data-gradient contraction(s),
- * ms[4] weight repacking (all calls).  The getter synchronises the stream.  No counterpart in the reference
- * (its Report objects hold host wall-clock: src/Report.h:13-91). */
+ * ms[1] weight-gradient contraction, with the pass over dY in front of it, ms[2] its split reduction, with the bias gradient and
+ * the packing of the weights for the data gradient, ms[3] data-gradient contraction(s), with that packing in calls of one slice
+ * of the batch (host buffers), ms[4] packing of the weights for the forward pass.  The pooling and ReLU masks of
+ * cct_conv_backward_fused are in none of them, nor is the pass over dY where the pooling mask's kernel does it too.  The getter
+ * synchronises the stream.  No counterpart in the reference (its Report objects hold host wall-clock: src/Report.h:13-91). */
 int cct_conv_plan_enable_timing(cct_conv_plan* plan, int enable);
 int cct_conv_plan_last_timings(cct_conv_plan* plan, float ms[5]);
 
@@ -214,7 +216,8 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
 int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const float* dY, float* dX, float* dW, float* db,
                     int in_relu, const uint32_t* in_drop_mask, float in_drop_scale);
 /* Per-kernel-group device times of the most recent calls (as cct_conv_plan_last_timings): ms[0] forward, ms[1] weight
- * and bias gradient, ms[3] data gradient. */
+ * gradient, with the bias gradient where no launch of the data gradient adds it, ms[3] data gradient, with the bias gradient
+ * where its reduction adds it. */
 int cct_fc_plan_enable_timing(cct_fc_plan* plan, int enable);
 int cct_fc_plan_last_timings(cct_fc_plan* plan, float ms[5]);
 
