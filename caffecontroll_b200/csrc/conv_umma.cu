@@ -229,7 +229,7 @@ __host__ __device__ inline GatherSmem gather_smem(int n_pad, int k_pad, int b_st
 // MODE: what the lanes gather - one table entry per reduction index, one per kRun of them, or (weight gradient) rows of the
 // lowered matrix over pixels.
 // kInside: one offset per reduction index (four to a shared-memory read) and no bounds test - a forward pass without padding,
-// whose windows lie inside the plane: 5.3 instructions per value instead of 9, AlexNet conv1 at batch 256 288 -> 270 us.  (Entries
+// whose windows lie inside the plane: 5.3 instructions per value instead of 9, AlexNet conv1 at batch 256 320 -> 293 us.  (Entries
 // behind the last real index read the window's first element against a weight of zero; lanes behind the last pixel read the last
 // pixel's window, their columns are not stored.)
 enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3 };
