@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <functional>
+#include <initializer_list>
 #include <string>
 #include <utility>
 #include <vector>
@@ -76,6 +77,16 @@ inline int record_call(std::function<int()> call) {
       return CCT_ERR_NOMEM;                                                          \
     }                                                                                \
   }
+
+// Whether `n` words at `out` lie outside all of `others` (address and words; null: none).
+inline bool apart(const void* out, size_t n, std::initializer_list<std::pair<const void*, size_t>> others) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(out);
+  for (const auto& o : others) {
+    const uintptr_t b = reinterpret_cast<uintptr_t>(o.first);
+    if (o.first && a < b + o.second * 4 && b < a + n * 4) return false;
+  }
+  return true;
+}
 
 #define CCT_CUDA(ctx, call)                                                                   \
   do {                                                                                        \

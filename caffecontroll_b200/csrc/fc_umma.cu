@@ -450,11 +450,6 @@ __global__ void __launch_bounds__(256) fc_pad_kernel(const float* __restrict__ s
 }
 
 int fc_round_up(int v, int a) { return (v + a - 1) / a * a; }
-bool fc_overlap(const float* a, size_t a_count, const float* b, size_t b_count) {
-  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-  return x < y + b_count * sizeof(float) && y < x + a_count * sizeof(float);
-}
-
 }  // namespace
 #include "fc_small.cuh"
 namespace {
@@ -602,7 +597,7 @@ struct cct_fc_plan {
   int K4 = 0, O4 = 0;        // row pitches: multiples of four floats
   FcShape fwd, dgr, wgr;
   bool small = false;        // all three contractions by fc_small_kernel, with these splits
-  int small_fwd = 1, small_dgr = 1;
+  int small_fwd = 1, small_dgr = 1;  // (fwd: for operands off a 16-byte boundary; a plan of the tensor-core kernel takes no more splits than that has room for)
   float* partial = nullptr;  // split partial sums of the forward pass and of the data gradient
   float *Xp = nullptr, *Wp = nullptr, *dYp = nullptr;  // copies with padded rows, where K or O is no multiple of four
   size_t bytes = 0;
@@ -630,21 +625,26 @@ bool use_small_fc(int B, int K, int O) {
   return flops <= (K % 4 || O % 4 ? kSmallFcPaddedFlops : kSmallFcFlops);
 }
 
-void fc_small(cct_ctx* ctx, const FcSmallParams& P, int splits) {
-  launch_pdl(fc_small_kernel, dim3((unsigned)((P.M + kFsTile - 1) / kFsTile) * ((P.N + kFsTile - 1) / kFsTile), splits), dim3(kFsThreads), 0, ctx->stream, P);
+// One launch for one or two contractions.
+int fc_small(cct_ctx* ctx, std::initializer_list<FcSmallParams> jobs) {
+  FcSmallJobs J{};
+  unsigned blocks = 0;
+  int n = 0;
+  for (const FcSmallParams& P : jobs) {
+    J.job[n] = P;
+    J.first = n++ ? J.first : ~0u;
+    if (n == 2) J.first = blocks;
+    blocks += (unsigned)((P.M + kFsTile - 1) / kFsTile) * ((P.N + kFsTile - 1) / kFsTile) * P.splits;
+  }
+  launch_pdl(fc_small_kernel, dim3(blocks), dim3(kFsThreads), 0, ctx->stream, J);
+  CCT_CHECK_LAUNCH(ctx);
+  return CCT_OK;
 }
 
 bool fc_aligned(std::initializer_list<const void*> ptrs) {
   for (const void* p : ptrs)
     if (reinterpret_cast<uintptr_t>(p) & 15u) return false;
   return true;
-}
-
-// Splits of fc_small_kernel for a pass of this plan.  A plan of the tensor-core kernel takes it where an operand is not on a
-// 16-byte boundary, which no tensor map can describe (and which the kernel's scalar loads do not mind); the room for split
-// sums is then what the other kernel's splits need.
-int fc_small_pass_splits(const cct_fc_plan* plan, int wanted, const FcShape& tensor) {
-  return plan->small ? wanted : std::min(wanted, tensor.P.splits);
 }
 
 int fc_reduce(cct_ctx* ctx, FcReduceParams R) {
@@ -662,6 +662,26 @@ int fc_reduce(cct_ctx* ctx, FcReduceParams R) {
   launch_pdl(kernel, dim3(R.sum_blocks + (R.bias_sum.db ? (R.bias_sum.O + 31) / 32 : 0)), dim3(256), 0, ctx->stream, R);
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
+}
+
+// Forward pass of a small layer.  Where Y lies over an operand that other blocks still read, the sums go through `scratch`.
+int fc_dot(cct_ctx* ctx, const float* W, const float* X, int K, FcReduceParams post, float* scratch) {
+  FcDotParams P{W, X, post.cols, post.rows, K, post};
+  const bool clear = apart(post.out, (size_t)post.rows * post.cols, {{X, (size_t)post.rows * K}, {W, (size_t)post.cols * K}});
+  if (!clear) {
+    P.post = FcReduceParams{};
+    P.post.out = scratch;
+    P.post.cols = post.cols;
+    post.partial = scratch;
+    post.pitch = post.cols;
+    post.splits = 1;
+  }
+  const bool vec = K % 4 == 0 && fc_aligned({W, X});
+  const int steps = (K + (vec ? 127 : 31)) / (vec ? 128 : 32);
+  launch_pdl(vec ? fc_dot_kernel<4> : fc_dot_kernel<1>, dim3((unsigned)((P.M + kFdTile - 1) / kFdTile) * ((P.N + kFdTile - 1) / kFdTile)),
+             dim3(32 * std::min(steps, kFdMaxWarps)), 0, ctx->stream, P);
+  CCT_CHECK_LAUNCH(ctx);
+  return clear ? CCT_OK : fc_reduce(ctx, post);
 }
 
 void fc_pad(cct_ctx* ctx, const float* src, float* dst, int rows, int cols, int pitch) {
@@ -695,7 +715,7 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   p->small_fwd = fc_small_splits(ctx->sm_count, out_features, batch, in_features);
   p->small_dgr = fc_small_splits(ctx->sm_count, in_features, batch, out_features);
   // One allocation: split sums, then the padded copies that are needed.
-  const int f_splits = p->small ? p->small_fwd : p->fwd.P.splits, d_splits = p->small ? p->small_dgr : p->dgr.P.splits;
+  const int f_splits = p->small ? 1 : p->fwd.P.splits, d_splits = p->small ? p->small_dgr : p->dgr.P.splits;
   const size_t sums = std::max((size_t)f_splits * batch * p->O4, (size_t)d_splits * batch * p->K4);
   const bool pad_k = !p->small && p->K4 != p->K, pad_o = !p->small && p->O4 != p->O;
   auto room = [](size_t n) { return (n + 63) & ~(size_t)63; };
@@ -749,14 +769,18 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   const int B = plan->B, K = plan->K, O = plan->O, K4 = plan->K4, O4 = plan->O4;
   plan->timer.begin(0, ctx->stream);
-  if (plan->small || !(plan->Wp || fc_aligned({X, W}))) {
-    const int splits = fc_small_pass_splits(plan, plan->small_fwd, plan->fwd);
+  if (plan->small) {
+    const int rc = fc_dot(ctx, W, X, K, FcReduceParams{nullptr, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, 1, relu},
+                          plan->partial);
+    plan->timer.end(0, ctx->stream);
+    return rc;
+  }
+  if (!(plan->Wp || fc_aligned({X, W}))) {
+    const int splits = std::min(plan->small_fwd, plan->fwd.P.splits);
     const FcReduceParams post{plan->partial, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, splits, relu};
-    FcSmallParams S{W, X, K, K, 0, 0, O, B, K, fc_round_up((K + splits - 1) / splits, 32), splits > 1 ? plan->partial : Y,
-                    splits > 1 ? O4 : O, nullptr, post};
-    fc_small(ctx, S, splits);
-    CCT_CHECK_LAUNCH(ctx);
-    const int rc = splits > 1 ? fc_reduce(ctx, post) : CCT_OK;
+    int rc = fc_small(ctx, {FcSmallParams{W, X, K, K, 0, 0, O, B, K, splits, fc_round_up((K + splits - 1) / splits, 32),
+                                          splits > 1 ? plan->partial : Y, splits > 1 ? O4 : O, nullptr, post}});
+    if (rc == CCT_OK && splits > 1) rc = fc_reduce(ctx, post);
     plan->timer.end(0, ctx->stream);
     return rc;
   }
@@ -793,9 +817,16 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   // ---- weight gradient: out = dW[o][k] (m = k, n = o), reduction over the batch; both operands MN-major
   plan->timer.begin(1, ctx->stream);
   if (plan->dYp && !(w_small && d_small)) { fc_pad(ctx, dY, plan->dYp, B, O, O4); dYm = plan->dYp; }
+  const FcSmallParams W_job{X, dY, K, O, 1, 1, K, O, B, 1, B, dW, K, plan->bias ? db : nullptr, FcReduceParams{}};
+  // Both contractions of a small layer in one launch, where neither writes what the other reads or writes.
+  const size_t nx = (size_t)B * K, ny = (size_t)B * O, nw = (size_t)O * K, nb = plan->bias ? O : 0;
+  const int d_splits = plan->small ? plan->small_dgr : std::min(plan->small_dgr, plan->dgr.P.splits);
+  const bool together = w_small && d_small && dX && !plan->timer.enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, nb}}) &&
+                        apart(dW, nw, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}}) &&
+                        apart(db, nb, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}});
   if (w_small) {
-    FcSmallParams S{X, dY, K, O, 1, 1, K, O, B, B, dW, K, plan->bias ? db : nullptr, FcReduceParams{}};
-    fc_small(ctx, S, 1);
+    if (!together) rc = fc_small(ctx, {W_job});
+    if (rc != CCT_OK) return rc;
   } else {
     if (plan->Xp) { fc_pad(ctx, X, plan->Xp, B, K, K4); Xm = plan->Xp; }
     const bool direct = K4 != K || !fc_aligned({dW});  // an output no tensor map describes
@@ -808,8 +839,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     if (plan->bias) {
       // With the data gradient's reduction, unless there is none, or it writes where the sum reads (dX over dY).
       bias_sum = FcBiasSum{dY, db, B, O};
-      if (!dX || (d_small && fc_small_pass_splits(plan, plan->small_dgr, plan->dgr) == 1) ||
-          fc_overlap(dX, (size_t)B * K, dY, (size_t)B * O)) {
+      if (!dX || (d_small && d_splits == 1) || !apart(dX, nx, {{dY, ny}})) {
         launch_pdl(fc_bias_grad_kernel, dim3((O + 31) / 32), dim3(256), 0, ctx->stream, bias_sum);
         bias_sum = FcBiasSum{};
       }
@@ -820,13 +850,11 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   // ---- data gradient: out = dX[b][k] (m = k, n = b), reduction over o; A = W read MN-major, B = dY K-major
   if (dX && d_small) {
     plan->timer.begin(3, ctx->stream);
-    const int splits = fc_small_pass_splits(plan, plan->small_dgr, plan->dgr);
-    const FcReduceParams post{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4, splits, 0, 0, bias_sum};
-    FcSmallParams D{W, dY, K, O, 1, 0, K, B, O, fc_round_up((O + splits - 1) / splits, 32), splits > 1 ? plan->partial : dX,
-                    splits > 1 ? K4 : K, nullptr, post};
-    fc_small(ctx, D, splits);
-    CCT_CHECK_LAUNCH(ctx);
-    rc = splits > 1 ? fc_reduce(ctx, post) : CCT_OK;
+    const FcReduceParams post{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4, d_splits, 0, 0, bias_sum};
+    const FcSmallParams D_job{W, dY, K, O, 1, 0, K, B, O, d_splits, fc_round_up((O + d_splits - 1) / d_splits, 32),
+                              d_splits > 1 ? plan->partial : dX, d_splits > 1 ? K4 : K, nullptr, post};
+    rc = together ? fc_small(ctx, {W_job, D_job}) : fc_small(ctx, {D_job});
+    if (rc == CCT_OK && d_splits > 1) rc = fc_reduce(ctx, post);
     plan->timer.end(3, ctx->stream);
   } else if (dX) {
     plan->timer.begin(3, ctx->stream);

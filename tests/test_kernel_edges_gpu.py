@@ -725,3 +725,44 @@ def test_sliced_host_calls(ctx, port, shape, with_dx, algo):
         for a, r, name in [(dW, dWr, "dW"), (db, dbr, "db")] + ([(dX, dXr, "dX")] if with_dx else []):
             assert_close(a, r.reshape(a.shape), name)
     ctx.lib.cct_conv_plan_destroy(plan)
+
+
+# Inner products of the fp32 kernels: one feature, rows that are and are not multiples of four floats or on a 16-byte boundary, tiles of four
+# images and outputs that are not full, fewer and more steps of the reduction than a block has warps, a data gradient with and without
+# splits; the two gradients in one launch.  Tolerance: n products added in fp32 in any order, n * 2^-24 of the sum of their magnitudes,
+# and a few roundings more.
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("B,K,o", [(1, 1, 1), (3, 5, 7), (5, 36, 130), (50, 4096, 10), (64, 500, 10), (33, 127, 257), (4, 60, 1021), (9, 2052, 21)])
+def test_small_inner_products(ctx, B, K, o, shift):
+    gen = torch.Generator(device="cuda").manual_seed(B + K + o)
+    make = lambda r, c: torch.randn(r * c + shift, device="cuda", generator=gen)[shift:].view(r, c)  # noqa: E731
+    X, W, b, dY = make(B, K), make(o, K), make(1, o), make(B, o)
+    keep, keep_in = ((torch.rand(s, device="cuda", generator=gen) < 0.5).int() for s in ((B, o), (B, K)))
+    Y, dX, dW, db = torch.zeros_like(dY), torch.zeros_like(X), torch.zeros_like(W), torch.zeros_like(b)
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(plan)), "plan", ctx.h)
+    before = capi.kernel_launches()
+    capi.check(ctx.lib.cct_fc_forward(plan, q(X), q(W), q(b), q(Y), 1, q(keep), 2.0), "forward", ctx.h)
+    forward = capi.kernel_launches()
+    capi.check(ctx.lib.cct_fc_backward(plan, q(X), q(W), q(dY), q(dX), q(dW), q(db), 1, q(keep_in), 2.0), "backward", ctx.h)
+    assert forward - before == 1 and capi.kernel_launches() - forward == (2 if o >= 256 else 1)
+    ctx.sync()
+    Xd, Wd, dYd = X.double(), W.double(), dY.double()
+    back = keep_in * 2.0 * (X > 0)
+    checks = [(Y, (Xd @ Wd.T + b.double()).clamp(min=0) * keep * 2, (Xd.abs() @ Wd.abs().T + b.double().abs()) * 2, K + 2, "Y"),
+              (dX, dYd @ Wd * back, dYd.abs() @ Wd.abs() * 2, o + 2, "dX"), (dW, dYd.T @ Xd, dYd.abs().T @ Xd.abs(), B, "dW"),
+              (db, dYd.sum(0)[None], dYd.abs().sum(0)[None], B, "db")]
+    for got, ref, size, n, name in checks:
+        assert torch.all((got.double() - ref).abs() <= (n + 4) * 2.0 ** -24 * size), name
+    # an output over an operand: the same bits as apart
+    for out, over, call in ((Y, X, lambda t: ctx.lib.cct_fc_forward(plan, q(t), q(W), q(b), q(t), 1, q(keep), 2.0)),
+                            (dW, W, lambda t: ctx.lib.cct_fc_backward(plan, q(X), q(t), q(dY), None, q(t), q(db), 0, None, 1.0)),
+                            (dX, X, lambda t: ctx.lib.cct_fc_backward(plan, q(t), q(W), q(dY), q(t), q(dW), q(db), 1, q(keep_in), 2.0))):
+        if out.numel() <= over.numel():
+            both = over.clone()
+            torch.cuda.synchronize()
+            capi.check(call(both), "over", ctx.h)
+            ctx.sync()
+            assert torch.equal(both.view(-1)[:out.numel()], out.view(-1))
+    ctx.lib.cct_fc_plan_destroy(plan)
