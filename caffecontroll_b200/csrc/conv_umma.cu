@@ -2197,22 +2197,37 @@ PackDgrad pack_dgrad_job(const UmmaPlan* p, const float* W) {
   return J;
 }
 
-void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct) {
-  const int jr = small_rows(k);
+// Grid of a pass by small_conv_block, and its shared memory; `warps` > 0: that many per block.
+struct SmallConvShape {
+  int ct, warps, x, y;
+  size_t smem;
+};
+SmallConvShape shape_small_conv(cct_ctx* ctx, SmallConv& P, int k, int ct, int warps = 0) {
+  const int jr = small_rows(k, ct);  // (the same for four and eight channels)
   P.row_groups = (P.n_out + jr - 1) / jr;
   P.positions = P.batch * P.row_groups * P.n_out;
   // Narrower channel tiles and more warps on the input channels until the SMs have about sixteen warps each.
   const long long lots = (P.positions + 31) / 32, want = 16ll * ctx->launch_sms();
   if (ct == 8 && lots * P.groups * ((P.co + 7) / 8) * std::min(16, std::max(1, P.ci / 2)) < want) ct = 4;
   P.col_tiles = (P.co + ct - 1) / ct;
-  int warps = 4;
   P.share = P.ci >= 4 && lots * P.groups * P.col_tiles < want;
-  while (P.share && warps < 16 && P.ci >= 4 * warps && lots * P.groups * P.col_tiles * warps < want &&
-         small_conv_smem(k, ct, P.ci, 2 * warps) <= 48 * 1024)
-    warps *= 2;
+  if (!warps) {
+    warps = 4;
+    while (P.share && warps < 16 && P.ci >= 4 * warps && lots * P.groups * P.col_tiles * warps < want &&
+           small_conv_smem(k, ct, P.ci, 2 * warps) <= 48 * 1024)
+      warps *= 2;
+  }
   const int per_block = P.share ? 32 : 32 * warps;
-  launch_pdl(small_conv_pick(k, s, ct), dim3((P.positions + per_block - 1) / per_block, P.groups * P.col_tiles), dim3(32 * warps),
-             small_conv_smem(k, ct, P.ci, P.share ? warps : 0), ctx->stream, P);
+  return SmallConvShape{ct, warps, (P.positions + per_block - 1) / per_block, P.groups * P.col_tiles,
+                        small_conv_smem(k, ct, P.ci, P.share ? warps : 0)};
+}
+void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct) {
+  const SmallConvShape g = shape_small_conv(ctx, P, k, ct);
+  launch_pdl(small_conv_pick(k, s, g.ct), dim3(g.x, g.y), dim3(32 * g.warps), g.smem, ctx->stream, P);
+}
+// The data gradient of a stride-1 layer as a convolution of dY.
+SmallConv small_dgrad(const ConvGeom& G, const float* dY, const float* W, float* dX, int batch) {
+  return SmallConv{dY, W, nullptr, dX, batch, G.m, G.n, G.k - 1 - G.p, G.og, G.Dg, G.g, 1, 0};
 }
 
 // Persistent grid: one CTA per SM (4 producer sets) or two (2 sets); then the reduction over the splits, if any.
@@ -2280,16 +2295,31 @@ bool umma_dy_rows(const UmmaPlan* p, DyRows* rows) {
   return true;
 }
 
+namespace {
+int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t, const float* pack_W,
+                    SmallConv* with);
+}
+
 int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dY, float* dX,
                        float* dW, float* db, PhaseTimer* t) {
+  const ConvGeom& G = p->G;
+  const size_t nx = (size_t)G.B * G.D * G.n * G.n, ny = (size_t)G.B * G.o * G.m * G.m, nw = (size_t)G.o * G.Dg * G.k * G.k;
+  // Small layers: the data gradient goes with the weight gradient, unless one writes where the other reads.
+  if (p->w_small && p->dgr.small_ct && dX && !t->enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, G.o}}) &&
+      apart(dW, nw, {{W, nw}, {dY, ny}}) && (!G.bias || apart(db, G.o, {{W, nw}, {dY, ny}}))) {
+    SmallConv d = small_dgrad(G, dY, W, dX, G.B);
+    return weight_gradient(ctx, p, X, dY, dW, db, t, nullptr, &d);
+  }
   int rc = umma_conv_wgrad(ctx, p, X, dY, dW, db, t, dX ? W : nullptr);
   if (rc == CCT_OK && dX) rc = umma_conv_dgrad(ctx, p, W, dY, dX, t, 0, false);
   return rc;
 }
 
-// Weight + bias gradient over the whole batch; `pack_W`: the weights to pack for the data gradient on the way.
-int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t,
-                    const float* pack_W) {
+// Weight + bias gradient over the whole batch; `pack_W`: the weights to pack for the data gradient on the way; `with`: the data
+// gradient of a small layer, in the same launch.
+namespace {
+int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t, const float* pack_W,
+                    SmallConv* with) {
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   const ConvGeom& G = p->G;
   ReduceExtras extras{};
@@ -2345,8 +2375,15 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     if (p->w_small) {
       P.n_pad = p->ws_cols * kSwTile;
       rows_pad = p->ws_rows * kSwTile;
-      launch_pdl(small_wgrad_kernel, dim3(p->ws_rows * p->ws_cols * vgroups, p->w_splits), dim3(kSwThreads), 0, ctx->stream, P,
-                 rows_pad, p->ws_rows, p->ws_cols, p->ws_pix);
+      const SmallWgrad J{P, rows_pad, p->ws_rows, p->ws_cols, p->ws_pix, p->ws_rows * p->ws_cols * vgroups};
+      const int blocks = J.tiles * p->w_splits;
+      if (with) {
+        const SmallConvShape g = shape_small_conv(ctx, *with, G.k, p->dgr.small_ct, kSwWarps);
+        launch_pdl(small_backward_pick(G.k, g.ct), dim3(blocks + g.x * g.y), dim3(kSwThreads), std::max(kSwSmem, g.smem), ctx->stream,
+                   SmallBackward{J, *with, g.x, g.x * g.y});
+      } else {
+        launch_pdl(small_wgrad_kernel, dim3(blocks), dim3(kSwThreads), kSwSmem, ctx->stream, J);
+      }
     } else {
       if (p->w_ts) P.x_count = (int)((long long)G.B * G.D * G.n * G.n - (G.g - 1) * P.x_group_stride);
       launch_pdl(short_wgrad_kernel(p), dim3(grid), dim3(p->w_ts ? ts_threads(ts_wide(G)) : kWgThreads), p->w_smem, ctx->stream, P);
@@ -2362,6 +2399,11 @@ int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
   return CCT_OK;
 }
 
+}  // namespace
+int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t, const float* pack_W) {
+  return weight_gradient(ctx, p, X, dY, dW, db, t, pack_W, nullptr);
+}
+
 // Data gradient of the first `batch` images (0: all of them); `repack` rewrites the packed weights from W first.
 int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, float* dX, PhaseTimer* t, int batch,
                     bool repack) {
@@ -2373,7 +2415,7 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
     const int vgroups = G.g * d.tiles;
     t->begin(3, ctx->stream);
     if (d.small_ct) {
-      SmallConv P{dY, W, nullptr, dX, B, G.m, G.n, G.k - 1 - G.p, G.og, G.Dg, G.g, 1, 0};
+      SmallConv P = small_dgrad(G, dY, W, dX, B);
       launch_small_conv(ctx, P, G.k, 1, d.small_ct);
       t->end(3, ctx->stream);
       CCT_CHECK_LAUNCH(ctx);

@@ -766,3 +766,36 @@ def test_small_inner_products(ctx, B, K, o, shift):
             ctx.sync()
             assert torch.equal(both.view(-1)[:out.numel()], out.view(-1))
     ctx.lib.cct_fc_plan_destroy(plan)
+
+
+# Both gradients of a small layer with stride 1 in one launch and, where dX lies over X, one after the other.  Tolerance: parity (fp32
+# products, sums of at most 24 x 25 and 36 864 of them).
+@pytest.mark.parametrize("shape", [(5, 1, 9, 7, 5, 1, 0, 1), (6, 2, 11, 24, 3, 1, 1, 2), (3, 8, 10, 5, 1, 1, 0, 1), (2, 3, 13, 9, 7, 1, 3, 1),
+                                   (64, 1, 28, 20, 5, 1, 0, 1), (4, 12, 8, 16, 3, 1, 1, 1)])
+def test_small_gradients_in_one_launch(ctx, shape):
+    B, D, n, o, k, s, p, g = shape
+    m = (n + 2 * p - k) // s + 1
+    gen = torch.Generator(device="cuda").manual_seed(o)
+    X, W, dY = (torch.randn(sh, device="cuda", generator=gen) for sh in ((B, D, n, n), (o, D // g, k, k), (B, o, m, m)))
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    desc = capi.ConvDesc(B, D, n, o, k, s, p, g, 1, capi.ALGO_AUTO)
+    capi.check(ctx.lib.cct_conv_plan_create(ctx.h, C.byref(desc), C.byref(plan)), "plan", ctx.h)
+
+    def run(x, w, dx, dw):
+        db = torch.zeros(o, device="cuda")
+        torch.cuda.synchronize()
+        before = capi.kernel_launches()
+        capi.check(ctx.lib.cct_conv_backward(plan, q(x), q(w), q(dY), q(dx), q(dw), q(db)), "backward", ctx.h)
+        ctx.sync()
+        return dx, dw, db, capi.kernel_launches() - before
+
+    dX, dW, db, launches = run(X, W, torch.zeros_like(X), torch.zeros_like(W))
+    assert launches == 2
+    x = X.clone()
+    over = run(x, W, x, torch.zeros_like(W))
+    ctx.lib.cct_conv_plan_destroy(plan)
+    assert over[3] == 3 and torch.equal(over[1], dW) and torch.equal(over[2], db)
+    Xd, Wd = X.double().requires_grad_(), W.double().requires_grad_()
+    torch.nn.functional.conv2d(Xd, Wd, None, s, p, 1, g).backward(dY.double())
+    for got, ref, name in ((dX, Xd.grad, "dX"), (over[0], Xd.grad, "dX over X"), (dW, Wd.grad, "dW"), (db, dY.double().sum((0, 2, 3)), "db")):
+        assert_close(got.cpu().numpy(), ref.float().cpu().numpy(), name)
