@@ -2008,28 +2008,32 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     for (int u = 2; u <= kWgMaxSubs; ++u)
       if (u <= p->w_mtiles && u * (f.n_pad <= 64 ? 2 : 1) * f.n_pad <= 512 && 2 * wg_smem(f.n_pad, u, 2).stage_bytes + 8192 <= (uint32_t)kSmemLimit)
         subs = u;
-    p->w_subs = subs;
-    p->w_mgroups = (p->w_mtiles + subs - 1) / subs;
     // 257 .. 384 rows and one channel tile of at most 128: the role-exchanged kernel, one CTA for all rows
     p->w_ts = p->w_mtiles * kTileM == kTsRows && f.n_pad <= kTileM;
-    if (p->w_ts) p->w_mgroups = 1;
+    const int n_pix = G.B * G.m * G.m;
+    p->w_kblocks_total = (n_pix + kBlockK - 1) / kBlockK;
+    for (;; subs = 1) {
+      p->w_mgroups = p->w_ts ? 1 : (p->w_mtiles + subs - 1) / subs;
+      const int out_tiles = p->w_mgroups * G.g * f.tiles;
+      // Whole waves of CTAs (one CTA per SM), as few as keep a partial sum's accumulation chain within
+      // kMaxChainKblocks: the tensor core's fp32 accumulation truncates, so the error of a partial sum grows with the
+      // length of its chain, while the reduction over splits adds with proper rounding.
+      int splits = 1;
+      for (int waves = 1; waves <= 64; ++waves) {
+        splits = std::max(1, waves * ctx->sm_count / out_tiles);
+        if ((p->w_kblocks_total + splits - 1) / splits <= p->w_chain) break;
+      }
+      splits = std::min(splits, std::max(1, p->w_kblocks_total / 3));  // at least 3 k-blocks per CTA
+      p->w_kblocks_per_split = (p->w_kblocks_total + splits - 1) / splits;
+      p->w_splits = (p->w_kblocks_total + p->w_kblocks_per_split - 1) / p->w_kblocks_per_split;
+      // Few pixels: where a CTA for every M-tile has an SM of its own, the same splits with half the MMAs in a row (about 1 us per
+      // k-block of two M-tiles): 37 images, 50 -> 75 channels 21 x 21, kernel 14.1 -> 10.0 us, LeNet conv2 at batch 64 12.6 -> 9.1.
+      if (subs == 1 || p->w_ts || p->w_mtiles * G.g * f.tiles * p->w_splits > ctx->sm_count) break;
+    }
+    p->w_subs = subs;
     const uint32_t stage_bytes = wg_smem(f.n_pad, subs, 2).stage_bytes;
     p->w_stages = std::max(2, std::min(kWgMaxStages, (int)((kSmemLimit - 8192) / stage_bytes)));
     p->w_smem = p->w_ts ? kTsSmem + 1024 : wg_smem(f.n_pad, subs, p->w_stages).total + 1024;
-    const int n_pix = G.B * G.m * G.m;
-    p->w_kblocks_total = (n_pix + kBlockK - 1) / kBlockK;
-    const int out_tiles = p->w_mgroups * G.g * f.tiles;
-    // Whole waves of CTAs (one CTA per SM), as few as keep a partial sum's accumulation chain within
-    // kMaxChainKblocks: the tensor core's fp32 accumulation truncates, so the error of a partial sum grows with the
-    // length of its chain, while the reduction over splits adds with proper rounding.
-    int splits = 1;
-    for (int waves = 1; waves <= 64; ++waves) {
-      splits = std::max(1, waves * ctx->sm_count / out_tiles);
-      if ((p->w_kblocks_total + splits - 1) / splits <= p->w_chain) break;
-    }
-    splits = std::min(splits, std::max(1, p->w_kblocks_total / 3));  // at least 3 k-blocks per CTA
-    p->w_kblocks_per_split = (p->w_kblocks_total + splits - 1) / splits;
-    p->w_splits = (p->w_kblocks_total + p->w_kblocks_per_split - 1) / p->w_kblocks_per_split;
     p->w_small = !tensor_only && use_small_wgrad(n_pix, G.g * f.tiles, f.n, f.k_real);
     if (p->w_small) {
       // About one block per SM (two where a block keeps at least two chunks of pixels).
