@@ -238,54 +238,63 @@ __global__ void dropout_mask_kernel(uint32_t* __restrict__ mask, size_t count, u
 // FLT_MIN)).  One warp per image; the per-image losses are added in image order by one warp afterwards, so the result does
 // not depend on the grid.  Labels are floats, as in the reference's label cube.  Up to 1024 classes a lane keeps its logits
 // in registers, all loads in flight at once; beyond that a warp makes three passes over its row.
-// A few images are one cluster, whose barrier stands between the images and their sum (64 images, 10 classes: 4.3 us); more
-// take a second launch for it (256 images, 1000 classes: 7.9 us, one cluster of 256 warps 12.5).  Nothing is shared between
-// calls: calls of one context may run beside one another, replayed from graphs on several streams.
-constexpr int kSoftmaxVals = 32, kSoftmaxCluster = 8, kSoftmaxWarps = 8;
+// Few images are one block or one cluster, whose barrier stands between the images and their sum; more take a second launch for
+// it.  One block where a lane has one logit (64 images, 10 classes 4.9 -> 3.5 us: launching a cluster costs that much); with up to
+// 1024 classes a block's images are too much for one SM (32 images, 1000 classes: one block 10.6 us, a cluster 6.2).
+// Nothing is shared between calls: calls of one context may run beside one another, replayed from graphs on several streams.
+constexpr int kSoftmaxVals = 32, kSoftmaxCluster = 8, kSoftmaxWarps = 8, kSoftmaxBlockWarps = 32, kSoftmaxBlockImages = 128;
+enum { kApart = 0, kOneBlock = 1, kCluster = 2 };
 
-// out = v[0] + v[1] + ... + v[n - 1], added in order by one warp: one load per lane, then the additions.
-__device__ __forceinline__ void sum_in_order(const float* v, float* out, int n, int lane) {
-  float acc = 0.f;
-  for (int i0 = 0; i0 < n; i0 += 32) {
-    const float mine = i0 + lane < n ? __ldcg(v + i0 + lane) : 0.f;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float one = __shfl_sync(0xffffffffu, mine, j);
-      if (i0 + j < n) acc += one;
-    }
-  }
-  if (lane == 0) *out = acc;
+// v[0] + v[1] + ... + v[n - 1], added in order by one thread (v in shared memory; by a warp, from global memory, 256 values took
+// 5.6 us, this 2.8).
+__device__ __forceinline__ float sum_in_order(const float* v, int n, float acc) {
+#pragma unroll 16
+  for (int i = 0; i < n; ++i) acc += v[i];
+  return acc;
 }
-__global__ void __launch_bounds__(32) sum_in_order_kernel(const float* __restrict__ v, float* __restrict__ out, int n) {
+__global__ void __launch_bounds__(256) sum_in_order_kernel(const float* __restrict__ v, float* __restrict__ out, int n) {
   pdl_wait();
-  sum_in_order(v, out, n, threadIdx.x);
+  __shared__ float s_v[1024];
+  float acc = 0.f;
+  for (int i0 = 0; i0 < n; i0 += 1024) {
+    if (i0) __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = k * 256 + (int)threadIdx.x;
+      s_v[i] = i0 + i < n ? __ldcg(v + i0 + i) : 0.f;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) acc = sum_in_order(s_v, min(1024, n - i0), acc);
+  }
+  if (threadIdx.x == 0) *out = acc;
 }
 
-template <bool IN_REGS, bool CLUSTER>
-__global__ void __launch_bounds__(CLUSTER ? 32 * kSoftmaxWarps : 128)
+// VALS: logits per lane in registers - one, 32, or none.
+template <int VALS, int TOGETHER>
+__global__ void __launch_bounds__(TOGETHER == kOneBlock ? 32 * kSoftmaxBlockWarps : TOGETHER == kCluster ? 32 * kSoftmaxWarps : 128)
     softmax_fwd_kernel(const float* __restrict__ X, const float* __restrict__ labels, float* __restrict__ prob, float* image_loss,
                        float* __restrict__ loss, int B, int C) {
   pdl_wait();
+  __shared__ float s_loss[kSoftmaxBlockImages];
   const int lane = threadIdx.x & 31;
-  const int img = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-  if (img < B) {
+  for (int img = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5); img < B; img += (int)(blockDim.x >> 5)) {
     const float* x = X + (size_t)img * C;
     float* pr = prob + (size_t)img * C;
-    float v[IN_REGS ? kSoftmaxVals : 1];
+    float v[VALS ? VALS : 1];
     float mx = -FLT_MAX, sum = 0.f;
-    if (IN_REGS) {
+    if (VALS) {
 #pragma unroll
-      for (int j = 0; j < kSoftmaxVals; ++j) v[j] = lane + 32 * j < C ? __ldg(x + lane + 32 * j) : -FLT_MAX;
+      for (int j = 0; j < VALS; ++j) v[j] = lane + 32 * j < C ? __ldg(x + lane + 32 * j) : -FLT_MAX;
 #pragma unroll
-      for (int j = 0; j < kSoftmaxVals; ++j) mx = fmaxf(mx, v[j]);
+      for (int j = 0; j < VALS; ++j) mx = fmaxf(mx, v[j]);
     } else {
       for (int i = lane; i < C; i += 32) mx = fmaxf(mx, x[i]);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (IN_REGS) {
+    if (VALS) {
 #pragma unroll
-      for (int j = 0; j < kSoftmaxVals; ++j)
+      for (int j = 0; j < VALS; ++j)
         if (32 * j < C) {
           v[j] = expf(v[j] - mx);
           if (lane + 32 * j < C) sum += v[j];
@@ -295,9 +304,9 @@ __global__ void __launch_bounds__(CLUSTER ? 32 * kSoftmaxWarps : 128)
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (IN_REGS) {
+    if (VALS) {
 #pragma unroll
-      for (int j = 0; j < kSoftmaxVals; ++j)
+      for (int j = 0; j < VALS; ++j)
         if (lane + 32 * j < C) pr[lane + 32 * j] = v[j] / sum;
     } else {
       for (int i = lane; i < C; i += 32) pr[i] = expf(x[i] - mx) / sum;
@@ -305,13 +314,22 @@ __global__ void __launch_bounds__(CLUSTER ? 32 * kSoftmaxWarps : 128)
     if (lane == 0) {
       const int label = (int)labels[img];
       const float p = (label >= 0 && label < C) ? expf(x[label] - mx) / sum : 0.f;
-      image_loss[img] = -logf(fmaxf(p, FLT_MIN));
+      const float one = -logf(fmaxf(p, FLT_MIN));
+      image_loss[img] = one;
+      if (TOGETHER == kOneBlock) s_loss[img] = one;
     }
+    if (TOGETHER != kOneBlock) break;
   }
-  if (CLUSTER) {  // the grid is one cluster: every image's loss is there and visible behind this barrier
+  if (TOGETHER == kApart) return;
+  if (TOGETHER == kOneBlock) {
+    __syncthreads();
+  } else {  // the grid is one cluster: every image's loss is there and visible behind this barrier
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (blockIdx.x == 0 && threadIdx.x < 32) sum_in_order(image_loss, loss, B, lane);
+    if (blockIdx.x) return;
+    if ((int)threadIdx.x < B) s_loss[threadIdx.x] = __ldcg(image_loss + threadIdx.x);
+    __syncthreads();
   }
+  if (threadIdx.x == 0) *loss = sum_in_order(s_loss, B, 0.f);
 }
 
 // Gradient of the loss with respect to the bridge's input (src/kernels/softmax.hxx:62-80):
@@ -560,16 +578,19 @@ int cct_softmax_loss_forward(cct_ctx* ctx, const float* X, const float* labels, 
   CCT_RECORD(ctx, cct_softmax_loss_forward(ctx, X, labels, prob, image_loss, loss, batch, classes))
   if (!ctx || !X || !labels || !prob || !image_loss || !loss || batch <= 0 || classes <= 0) return CCT_ERR_INVALID;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
-  const bool in_regs = classes <= 32 * kSoftmaxVals;
-  if (in_regs && batch <= kSoftmaxCluster * kSoftmaxWarps) {
+  const int vals = classes <= 32 ? 1 : classes <= 32 * kSoftmaxVals ? kSoftmaxVals : 0;
+  if (vals == 1 && batch <= kSoftmaxBlockImages) {
+    launch_pdl(softmax_fwd_kernel<1, kOneBlock>, dim3(1), dim3(32 * std::min(batch, kSoftmaxBlockWarps)), 0, ctx->stream, X, labels, prob,
+               image_loss, loss, batch, classes);
+  } else if (vals > 1 && batch <= kSoftmaxCluster * kSoftmaxWarps) {
     const int warps = (batch + kSoftmaxCluster - 1) / kSoftmaxCluster;
-    launch_pdl_cluster(kSoftmaxCluster, softmax_fwd_kernel<true, true>, dim3(kSoftmaxCluster), dim3(32 * warps), 0, ctx->stream, X, labels,
-                       prob, image_loss, loss, batch, classes);
+    launch_pdl_cluster(kSoftmaxCluster, softmax_fwd_kernel<kSoftmaxVals, kCluster>, dim3(kSoftmaxCluster), dim3(32 * warps), 0, ctx->stream, X,
+                       labels, prob, image_loss, loss, batch, classes);
   } else {
-    launch_pdl(in_regs ? softmax_fwd_kernel<true, false> : softmax_fwd_kernel<false, false>, dim3((batch + 3) / 4), dim3(128), 0,
-               ctx->stream, X, labels, prob, image_loss, loss, batch, classes);
+    launch_pdl(vals == 1 ? softmax_fwd_kernel<1, kApart> : vals ? softmax_fwd_kernel<kSoftmaxVals, kApart> : softmax_fwd_kernel<0, kApart>,
+               dim3((batch + 3) / 4), dim3(128), 0, ctx->stream, X, labels, prob, image_loss, loss, batch, classes);
     CCT_CHECK_LAUNCH(ctx);
-    launch_pdl(sum_in_order_kernel, dim3(1), dim3(32), 0, ctx->stream, image_loss, loss, batch);
+    launch_pdl(sum_in_order_kernel, dim3(1), dim3(256), 0, ctx->stream, image_loss, loss, batch);
   }
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;

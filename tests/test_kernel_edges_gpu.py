@@ -727,6 +727,12 @@ def test_sliced_host_calls(ctx, port, shape, with_dx, algo):
     ctx.lib.cct_conv_plan_destroy(plan)
 
 
+# At most 32 classes: the largest batch of one block, one more, sums in several pieces; 33 classes: the largest batch of a cluster and one more.
+@pytest.mark.parametrize("B,classes", [(1, 32), (31, 10), (128, 32), (129, 32), (2049, 3), (64, 33), (65, 33)])
+def test_softmax_of_few_classes(ctx, B, classes):
+    test_softmax_class_counts(ctx, B, classes)
+
+
 # Inner products of the fp32 kernels: one feature, rows that are and are not multiples of four floats or on a 16-byte boundary, tiles of four
 # images and outputs that are not full, fewer and more steps of the reduction than a block has warps, a data gradient with and without
 # splits; the two gradients in one launch.  Tolerance: n products added in fp32 in any order, n * 2^-24 of the sum of their magnitudes,
