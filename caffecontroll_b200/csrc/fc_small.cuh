@@ -15,9 +15,10 @@
 namespace {
 
 constexpr int kFsThreads = 256, kFsWarps = 8, kFsTile = 32, kFsChunk = 128, kFsPitch = 36;
-// Measured against fc_gemm_kernel, forward + backward: 4096 -> 10, 50 images (17 MFLOP with the padding to 32) 23 -> 14 us;
-// 512 -> 128, 128 images (17) 24 -> 15; 800 -> 500, 64 images (52) 22 -> 26.  Where feature counts are no multiples of four
-// the other path copies its operands first: 999 -> 333, 37 images (46) 42 -> 23.
+// Measured against fc_gemm_kernel, forward + backward, when each contraction was a launch: 4096 -> 10, 50 images (17 MFLOP with the
+// padding to 32) 23 -> 14 us; 512 -> 128, 128 images (17) 24 -> 15; 800 -> 500, 64 images (52) 22 -> 26.  Where feature counts are no
+// multiples of four the other path copies its operands first: 999 -> 333, 37 images (46) 42 -> 23.  Layers within these lines stay
+// with the fp32 products whatever fc_small_faster() says of their backward pass.
 constexpr double kSmallFcFlops = 4e7, kSmallFcPaddedFlops = 1e8;
 
 struct FcSmallParams {
@@ -137,58 +138,69 @@ __global__ void __launch_bounds__(kFsThreads, 3) fc_small_kernel(const __grid_co
   }
 }
 
-// Forward pass of a small layer: out[n][m] = sum_r A[m][r] B[n][r], rows along the reduction.  A block owns 4 images x 4 outputs,
+// Forward pass of a small layer: out[n][m] = sum_r A[m][r] B[n][r], rows along the reduction.  A block owns NT images x 4 outputs,
 // its warps interleaved steps of 32 (x 4 where rows are on 16-byte boundaries) reduction indices; operands go from L2 straight
-// to registers, eight loads for sixteen products per lane and index, a warp's sums are added by shuffles and the warps' in
-// order.  With the 32 x 32 tiles of fc_small_kernel a few outputs with a long reduction took 32 splits, and a launch to add
-// them; with the splits in a cluster, adding through distributed shared memory, 512 indices per block took longer than that
-// launch.  4096 -> 10, 50 images: 4.4 + 2.7 -> 3.4 us, 500 -> 10, 64 images: 6.3 + 2.4 -> 2.3.  Traffic is a quarter of a word per product: layers that are not small have other kernels.
-constexpr int kFdTile = 4, kFdMaxWarps = 16;
+// to registers, a warp's sums are added by shuffles and the warps' in order.  With the 32 x 32 tiles of fc_small_kernel a few outputs
+// with a long reduction took 32 splits, and a launch to add them; with the splits in a cluster, adding through distributed shared
+// memory, 512 indices per block took longer than that launch.  4096 -> 10, 50 images: 4.4 + 2.7 -> 3.4 us, 500 -> 10, 64 images:
+// 6.3 + 2.4 -> 2.3.
+// What bounds it is the traffic from L2, a quarter of a word per product and more; fc_gemm_kernel's two launches take five
+// microseconds however little there is to do.  Where the line lies (products; tensor cores -> this): 512 -> 128, 256 images (17 M)
+// 10.5 -> 4.5 us; 512 -> 512, 64 images (17 M) 6.7 -> 4.5, 128 (34 M) 8.2 -> 7.7, 256 (67 M) 11.6 -> 13.3; 800 -> 500, 64 images
+// (26 M) 7.7 -> 8.0; 4096 -> 1000, one image 8.5 -> 3.2, four 8.8 -> 5.4, eight (33 M) 8.8 -> 6.5, 16 (66 M) 8.8 -> 11.8; 4096 ->
+// 4096, one image (17 M) 17.1 -> 15.1, two 17.2 -> 17.9.  Eight images per block where that leaves kDotWideBlocks blocks (512 -> 512,
+// 64 images: four 5.5 us, eight 4.5; 2304 -> 64, 32 images, 64 blocks of eight: 2.9 and 3.1) and the loads are wide (999 -> 333, 32
+// images: 6.6 and 7.8); one or two images take fewer registers and loads (4096 -> 1000, one image: 6.2 us with eight).
+constexpr int kFdM = 4, kFdMaxWarps = 16;
+constexpr double kDotProducts = 2.4e7;
+constexpr int kDotWideBlocks = 128;
 struct FcDotParams {
   const float *a, *b;
   int M, N, R;
   FcReduceParams post;  // out, ld = cols; bias / ReLU / dropout
 };
-template <int VEC>
+template <int VEC, int NT>
 __global__ void __launch_bounds__(32 * kFdMaxWarps) fc_dot_kernel(const __grid_constant__ FcDotParams P) {
   pdl_wait();
-  __shared__ float s_part[kFdMaxWarps][kFdTile * kFdTile];
+  constexpr int kSums = NT * kFdM;  // 4 ... 32
+  __shared__ float s_part[kFdMaxWarps][kSums];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
-  const int m_tiles = (P.M + kFdTile - 1) / kFdTile, n_tile = blockIdx.x / m_tiles;
-  const int m0 = (blockIdx.x - n_tile * m_tiles) * kFdTile, n0 = n_tile * kFdTile;
-  const float *a[kFdTile], *b[kFdTile];  // rows behind the last one repeat it; their sums are not stored
+  const int n_tiles = (P.N + NT - 1) / NT, m_tile = blockIdx.x / n_tiles;
+  const int n0 = (blockIdx.x - m_tile * n_tiles) * NT, m0 = m_tile * kFdM;
+  const float *a[kFdM], *b[NT];  // rows behind the last one repeat it; their sums are not stored
 #pragma unroll
-  for (int i = 0; i < kFdTile; ++i) {
-    a[i] = P.a + (long long)min(m0 + i, P.M - 1) * P.R;
-    b[i] = P.b + (long long)min(n0 + i, P.N - 1) * P.R;
-  }
-  float acc[kFdTile * kFdTile];
+  for (int i = 0; i < kFdM; ++i) a[i] = P.a + (long long)min(m0 + i, P.M - 1) * P.R;
 #pragma unroll
-  for (int i = 0; i < kFdTile * kFdTile; ++i) acc[i] = 0.f;
+  for (int i = 0; i < NT; ++i) b[i] = P.b + (long long)min(n0 + i, P.N - 1) * P.R;
+  float acc[kSums];
+#pragma unroll
+  for (int i = 0; i < kSums; ++i) acc[i] = 0.f;
 #pragma unroll 2
   for (int r = (warp * 32 + lane) * VEC; r < P.R; r += warps * 32 * VEC) {
-    float x[kFdTile][VEC], w[kFdTile][VEC];
-#pragma unroll
-    for (int i = 0; i < kFdTile; ++i) {
+    float x[NT][VEC], w[kFdM][VEC];
+    auto load = [&](float (&v)[VEC], const float* p) {
       if (VEC == 4) {
-        const float4 xv = __ldg(reinterpret_cast<const float4*>(b[i] + r)), wv = __ldg(reinterpret_cast<const float4*>(a[i] + r));
-        x[i][0] = xv.x; x[i][VEC > 1 ? 1 : 0] = xv.y; x[i][VEC > 2 ? 2 : 0] = xv.z; x[i][VEC > 3 ? 3 : 0] = xv.w;
-        w[i][0] = wv.x; w[i][VEC > 1 ? 1 : 0] = wv.y; w[i][VEC > 2 ? 2 : 0] = wv.z; w[i][VEC > 3 ? 3 : 0] = wv.w;
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p + r));
+        v[0] = t.x; v[VEC > 1 ? 1 : 0] = t.y; v[VEC > 2 ? 2 : 0] = t.z; v[VEC > 3 ? 3 : 0] = t.w;
       } else {
-        x[i][0] = __ldg(b[i] + r);
-        w[i][0] = __ldg(a[i] + r);
+        v[0] = __ldg(p + r);
       }
-    }
+    };
 #pragma unroll
-    for (int n = 0; n < kFdTile; ++n)
+    for (int i = 0; i < kFdM; ++i) load(w[i], a[i]);
 #pragma unroll
-      for (int m = 0; m < kFdTile; ++m)
+    for (int i = 0; i < NT; ++i) load(x[i], b[i]);
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) acc[n * kFdTile + m] = fmaf(w[m][e], x[n][e], acc[n * kFdTile + m]);
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int m = 0; m < kFdM; ++m)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[n * kFdM + m] = fmaf(w[m][e], x[n][e], acc[n * kFdM + m]);
   }
-  // Sixteen sums over 32 lanes: halves of the sums are exchanged for halves of the lanes, lane l ends with sum l >> 1.
+  // kSums sums over 32 lanes: halves of the sums are exchanged for halves of the lanes; lane l ends with sum l / kLanes.
+  constexpr int kLanes = 32 / kSums;
 #pragma unroll
-  for (int half = 8, o = 16; half > 0; half >>= 1, o >>= 1) {
+  for (int half = kSums / 2, o = 16; half > 0; half >>= 1, o >>= 1) {
     const bool upper = lane & o;
 #pragma unroll
     for (int i = 0; i < half; ++i) {
@@ -196,11 +208,12 @@ __global__ void __launch_bounds__(32 * kFdMaxWarps) fc_dot_kernel(const __grid_c
       acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
     }
   }
-  acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
-  if (!(lane & 1)) s_part[warp][lane >> 1] = acc[0];
+#pragma unroll
+  for (int o = kLanes / 2; o > 0; o >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+  if (lane % kLanes == 0) s_part[warp][lane / kLanes] = acc[0];
   __syncthreads();
-  const int n = n0 + tid / kFdTile, m = m0 + (tid & (kFdTile - 1));
-  if (tid >= kFdTile * kFdTile || n >= P.N || m >= P.M) return;
+  const int n = n0 + tid / kFdM, m = m0 + (tid & (kFdM - 1));
+  if (tid >= kSums || n >= P.N || m >= P.M) return;
   float t = 0.f;
   for (int w = 0; w < warps; ++w) t += s_part[w][tid];
   const FcReduceParams& F = P.post;
@@ -210,11 +223,29 @@ __global__ void __launch_bounds__(32 * kFdMaxWarps) fc_dot_kernel(const __grid_c
   if (F.drop_mask) t = t * (float)(F.drop_mask[at] != 0u) * F.drop_scale;
   F.out[at] = t;
 }
+template <int VEC>
+void (*fc_dot_pick(int nt))(const FcDotParams) {
+  return nt == 1 ? fc_dot_kernel<VEC, 1> : nt == 2 ? fc_dot_kernel<VEC, 2> : nt == 4 ? fc_dot_kernel<VEC, 4> : fc_dot_kernel<VEC, 8>;
+}
 
 // Splits of the reduction: about two blocks per SM, at least 64 indices each.
 int fc_small_splits(int sms, int M, int N, int R) {
   const int tiles = ((M + kFsTile - 1) / kFsTile) * ((N + kFsTile - 1) / kFsTile);
   return std::max(1, std::min(2 * sms / tiles, R / 128));
+}
+
+// Whether a backward pass is faster by fc_small_kernel: a fit to both paths' times (us).  Chunks of 128 indices of the two jobs' blocks,
+// 2.0 - 2.9 us for every one that an SM has, against 8.7 us for five launches of the tensor-core path, the stream of the weights and
+// their gradient, and wider tiles.  1000 -> 100, 256 images 18.1 -> 11.8 (estimate 16.8, 12.3); 512 -> 512, 64 images 11.1 -> 9.9
+// (11.1, 10.9), 128 images 13.6 -> 15.3 (13.1, 14.2); 4096 -> 1000, one image 15.6 -> 60 (15.7, 64).
+bool fc_small_faster(int sms, int B, int K, int O) {
+  auto up = [](int a, int b) { return (double)((a + b - 1) / b); };
+  const int splits = fc_small_splits(sms, K, B, O);
+  auto cost = [](double r) { return 2.0 + 0.9 * std::min(1.0, r / kFsChunk); };  // of a chunk with r indices
+  const double k = up(K, kFsTile), w = k * up(O, kFsTile) * up(B, kFsChunk) * cost(B);
+  const double d = k * up(B, kFsTile) * splits * up((O + splits - 1) / splits, kFsChunk) * cost((double)O / splits);
+  const double small = 2.6 + (w + d) / sms + (splits > 1 ? 1.6 : 0.0);
+  return small < 8.7 + 1.7e-6 * K * O + 0.031 * B + (K % 4 || O % 4 ? 5.0 : 0.0);
 }
 
 }  // namespace

@@ -596,8 +596,9 @@ struct cct_fc_plan {
   int B = 0, K = 0, O = 0, bias = 0;
   int K4 = 0, O4 = 0;        // row pitches: multiples of four floats
   FcShape fwd, dgr, wgr;
-  bool small = false;        // all three contractions by fc_small_kernel, with these splits
-  int small_fwd = 1, small_dgr = 1;  // (fwd: for operands off a 16-byte boundary; a plan of the tensor-core kernel takes no more splits than that has room for)
+  bool dot = false;          // forward pass by fc_dot_kernel
+  bool small_forward = false, small = false;  // forward, backward pass by fc_small_kernel, with these splits (where an operand is off a
+  int small_fwd = 1, small_dgr = 1;           // 16-byte boundary too, as far as there is room for their sums)
   float* partial = nullptr;  // split partial sums of the forward pass and of the data gradient
   float *Xp = nullptr, *Wp = nullptr, *dYp = nullptr;  // copies with padded rows, where K or O is no multiple of four
   size_t bytes = 0;
@@ -678,7 +679,9 @@ int fc_dot(cct_ctx* ctx, const float* W, const float* X, int K, FcReduceParams p
   }
   const bool vec = K % 4 == 0 && fc_aligned({W, X});
   const int steps = (K + (vec ? 127 : 31)) / (vec ? 128 : 32);
-  launch_pdl(vec ? fc_dot_kernel<4> : fc_dot_kernel<1>, dim3((unsigned)((P.M + kFdTile - 1) / kFdTile) * ((P.N + kFdTile - 1) / kFdTile)),
+  const bool wide = vec && P.N >= 8 && (long long)((P.N + 7) / 8) * ((P.M + kFdM - 1) / kFdM) >= kDotWideBlocks;
+  const int nt = wide ? 8 : P.N > 2 ? 4 : P.N;
+  launch_pdl(vec ? fc_dot_pick<4>(nt) : fc_dot_pick<1>(nt), dim3((unsigned)((P.M + kFdM - 1) / kFdM) * ((P.N + nt - 1) / nt)),
              dim3(32 * std::min(steps, kFdMaxWarps)), 0, ctx->stream, P);
   CCT_CHECK_LAUNCH(ctx);
   return clear ? CCT_OK : fc_reduce(ctx, post);
@@ -711,13 +714,16 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
     delete p;
     return CCT_ERR_UNSUPPORTED;
   }
-  p->small = use_small_fc(batch, in_features, out_features);
+  const bool few = use_small_fc(batch, in_features, out_features);
+  p->dot = (double)batch * in_features * out_features <= kDotProducts;
+  p->small_forward = few && !p->dot;
+  p->small = few || fc_small_faster(ctx->sm_count, batch, in_features, out_features);
   p->small_fwd = fc_small_splits(ctx->sm_count, out_features, batch, in_features);
   p->small_dgr = fc_small_splits(ctx->sm_count, in_features, batch, out_features);
   // One allocation: split sums, then the padded copies that are needed.
-  const int f_splits = p->small ? 1 : p->fwd.P.splits, d_splits = p->small ? p->small_dgr : p->dgr.P.splits;
+  const int f_splits = p->dot ? 1 : p->small_forward ? p->small_fwd : p->fwd.P.splits, d_splits = p->small ? p->small_dgr : p->dgr.P.splits;
   const size_t sums = std::max((size_t)f_splits * batch * p->O4, (size_t)d_splits * batch * p->K4);
-  const bool pad_k = !p->small && p->K4 != p->K, pad_o = !p->small && p->O4 != p->O;
+  const bool pad_k = !((p->dot || p->small_forward) && p->small) && p->K4 != p->K, pad_o = !p->small && p->O4 != p->O;
   auto room = [](size_t n) { return (n + 63) & ~(size_t)63; };
   const size_t x = pad_k ? room((size_t)batch * p->K4) : 0, w = pad_k ? room((size_t)out_features * p->K4) : 0,
                dy = pad_o ? room((size_t)batch * p->O4) : 0;
@@ -769,14 +775,14 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   const int B = plan->B, K = plan->K, O = plan->O, K4 = plan->K4, O4 = plan->O4;
   plan->timer.begin(0, ctx->stream);
-  if (plan->small) {
+  if (plan->dot) {
     const int rc = fc_dot(ctx, W, X, K, FcReduceParams{nullptr, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, 1, relu},
                           plan->partial);
     plan->timer.end(0, ctx->stream);
     return rc;
   }
-  if (!(plan->Wp || fc_aligned({X, W}))) {
-    const int splits = std::min(plan->small_fwd, plan->fwd.P.splits);
+  if (plan->small_forward || !(plan->Wp || fc_aligned({X, W}))) {
+    const int splits = plan->small_forward ? plan->small_fwd : std::min(plan->small_fwd, plan->fwd.P.splits);
     const FcReduceParams post{plan->partial, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, splits, relu};
     int rc = fc_small(ctx, {FcSmallParams{W, X, K, K, 0, 0, O, B, K, splits, fc_round_up((K + splits - 1) / splits, 32),
                                           splits > 1 ? plan->partial : Y, splits > 1 ? O4 : O, nullptr, post}});

@@ -738,7 +738,8 @@ def test_softmax_of_few_classes(ctx, B, classes):
 # splits; the two gradients in one launch.  Tolerance: n products added in fp32 in any order, n * 2^-24 of the sum of their magnitudes,
 # and a few roundings more.
 @pytest.mark.parametrize("shift", [0, 1])
-@pytest.mark.parametrize("B,K,o", [(1, 1, 1), (3, 5, 7), (5, 36, 130), (50, 4096, 10), (64, 500, 10), (33, 127, 257), (4, 60, 1021), (9, 2052, 21)])
+@pytest.mark.parametrize("B,K,o", [(1, 1, 1), (2, 68, 9), (3, 5, 7), (5, 36, 130), (50, 4096, 10), (64, 500, 10), (33, 127, 257), (4, 60, 1021), (9, 2052, 21),
+                                   (13, 1028, 300), (100, 400, 300)])
 def test_small_inner_products(ctx, B, K, o, shift):
     gen = torch.Generator(device="cuda").manual_seed(B + K + o)
     make = lambda r, c: torch.randn(r * c + shift, device="cuda", generator=gen)[shift:].view(r, c)  # noqa: E731
@@ -772,6 +773,27 @@ def test_small_inner_products(ctx, B, K, o, shift):
             ctx.sync()
             assert torch.equal(both.view(-1)[:out.numel()], out.view(-1))
     ctx.lib.cct_fc_plan_destroy(plan)
+
+
+# Layers whose passes take different kernels: dot products forward, tensor cores backward (with padded rows too); tensor cores forward, fp32
+# tiles backward; fp32 tiles with splits forward.  Rows on and off a 16-byte boundary.  Tolerance: parity.
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("B,K,o", [(1, 4096, 1000), (4, 4093, 1001), (256, 1000, 100), (128, 999, 333)])
+def test_inner_products_of_mixed_plans(ctx, B, K, o, shift):
+    gen = torch.Generator(device="cuda").manual_seed(B + K + o)
+    make = lambda r, c: torch.randn(r * c + shift, device="cuda", generator=gen)[shift:].view(r, c)  # noqa: E731
+    X, W, b, dY = make(B, K), make(o, K), make(1, o), make(B, o)
+    Y, dX, dW, db = torch.zeros_like(dY), torch.zeros_like(X), torch.zeros_like(W), torch.zeros_like(b)
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(plan)), "plan", ctx.h)
+    capi.check(ctx.lib.cct_fc_forward(plan, q(X), q(W), q(b), q(Y), 0, None, 1.0), "forward", ctx.h)
+    capi.check(ctx.lib.cct_fc_backward(plan, q(X), q(W), q(dY), q(dX), q(dW), q(db), 0, None, 1.0), "backward", ctx.h)
+    ctx.sync()
+    ctx.lib.cct_fc_plan_destroy(plan)
+    Xd, Wd, dYd = X.double(), W.double(), dY.double()
+    for got, ref, name in ((Y, Xd @ Wd.T + b.double(), "Y"), (dX, dYd @ Wd, "dX"), (dW, dYd.T @ Xd, "dW"), (db, dYd.sum(0)[None], "db")):
+        assert_close(got.cpu().numpy(), ref.float().cpu().numpy(), name)
 
 
 # Both gradients of a small layer with stride 1 in one launch and, where dX lies over X, one after the other.  Tolerance: parity (fp32
