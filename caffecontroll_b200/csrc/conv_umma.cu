@@ -233,7 +233,14 @@ __host__ __device__ inline GatherSmem gather_smem(int n_pad, int k_pad, int b_st
 // behind the last real index read the window's first element against a weight of zero; lanes behind the last pixel read the last
 // pixel's window, their columns are not stored.)
 enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3 };
-template <int SETS, int MODE>
+// ONE: every CTA has one tile, a short one (kOneKblocks).  There is no next tile then for the epilogue to overlap with, and the producers,
+// who are through, take their share of its columns (six chunks of 16 took four warps 1.2 us); in front of the first k-block stood three
+// trips to L2 for the tables and the bias, one behind the other, and the allocation of tensor memory (1.3 us in all), now one trip
+// beside the allocation.  conv3 of one image 13.6 -> 12.9 us, 37 images of 50 -> 75 channels both ways 36.3 -> 35.1.  Not for the
+// persistent kernels' last tiles, nor for the other two modes: the registers it takes spill (AlexNet conv1 at batch 256 1 211 -> 1 227
+// us both ways; LeNet conv2's forward kernel 9.9 -> 11.1).  Where a tile is long it gains nothing (CaffeNet at batch 32 1 238 -> 1 245 us).
+constexpr int kOneKblocks = 32;
+template <int SETS, int MODE, bool ONE>
 __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     gather_conv_kernel(const __grid_constant__ GatherParams P, const __grid_constant__ CUtensorMap w_map) {
   constexpr int kProducerWarps = 4 * SETS, kMmaWarp = kProducerWarps, kTmaWarp = kMmaWarp + 1;
@@ -256,21 +263,41 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
 
   int* s_offsets = reinterpret_cast<int*>(s_taps);  // kInside: the offsets alone
-  for (int i = tid; i < P.taps_smem; i += kGatherThreads) {
-    if (MODE == kInside) s_offsets[i] = P.taps[i].off;
-    else s_taps[i] = P.taps[i];
-  }
-  if (P.cols)
-    for (int i = tid; i < P.n_pad; i += kGatherThreads) s_cols[i] = P.cols[i];
-  if (tid == 0) {
+  auto init_barriers = [&]() {
     for (int s = 0; s < kMaxAStages; ++s) { mbar_init(ready_bar + 8u * s, 5); mbar_init(done_bar + 8u * s, 1); }  // 4 producer warps + the TMA thread
     for (int s = 0; s < kMaxAccBufs; ++s) { mbar_init(acc_full + 8u * s, 1); mbar_init(acc_empty + 8u * s, kEpiWarps); }
     fence_mbar_init();
+  };
+  if constexpr (ONE) {
+    static_assert(MODE == kByTap || MODE == kByRun, "the other modes have no registers to spare");
+    if (warp == 0) tmem_alloc(tmem_slot, (uint32_t)P.tmem_cols);
+    else if (tid == 32) init_barriers();
+    if (warp == kTmaWarp) prefetch_map(&w_map);
+    MaskTap tap0{};
+    ColEnt col0{};
+    if (tid < P.taps_smem) tap0 = P.taps[tid];
+    if (tid < P.n_pad) col0 = P.cols[tid];
+    pdl_wait();  // so far the plan's tables alone have been read
+    const float bias0 = tid < P.n_bias ? P.bias[tid] : 0.f;
+    if (tid < P.taps_smem) s_taps[tid] = tap0;
+    if (tid < P.n_pad) s_cols[tid] = col0;
+    if (tid < P.n_bias + kBiasPad) s_bias[tid] = bias0;
+#pragma unroll 4
+    for (int i = tid + kGatherThreads; i < P.taps_smem; i += kGatherThreads) s_taps[i] = P.taps[i];
+    for (int i = tid + kGatherThreads; i < P.n_bias + kBiasPad; i += kGatherThreads) s_bias[i] = i < P.n_bias ? P.bias[i] : 0.f;
+  } else {
+    for (int i = tid; i < P.taps_smem; i += kGatherThreads) {
+      if (MODE == kInside) s_offsets[i] = P.taps[i].off;
+      else s_taps[i] = P.taps[i];
+    }
+    if (P.cols)
+      for (int i = tid; i < P.n_pad; i += kGatherThreads) s_cols[i] = P.cols[i];
+    if (tid == 0) init_barriers();
+    if (warp == 0) tmem_alloc(tmem_slot, (uint32_t)P.tmem_cols);
+    if (warp == kTmaWarp) prefetch_map(&w_map);
+    pdl_wait();  // so far the plan's tables alone have been read: set-up beside the end of the kernel before (15.6 -> 15.35 us for conv3 of one image)
+    for (int i = tid; i < P.n_bias + kBiasPad; i += kGatherThreads) s_bias[i] = i < P.n_bias ? P.bias[i] : 0.f;
   }
-  if (warp == 0) tmem_alloc(tmem_slot, (uint32_t)P.tmem_cols);
-  if (warp == kTmaWarp) prefetch_map(&w_map);
-  pdl_wait();  // so far the plan's tables alone have been read: set-up beside the end of the kernel before (15.6 -> 15.35 us for conv3 of one image)
-  for (int i = tid; i < P.n_bias + kBiasPad; i += kGatherThreads) s_bias[i] = i < P.n_bias ? P.bias[i] : 0.f;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -515,7 +542,7 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
         }
       }
     }
-  } else {
+  } else if constexpr (!ONE) {
     // ------------------------------------------------------------------ epilogue
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
@@ -617,6 +644,42 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
+    }
+  }
+  if constexpr (ONE) {
+    // The tile's chunks of 16 columns in turn to the epilogue warps and the producers' sets.
+    if (warp < kProducerWarps || warp > kTmaWarp) {
+      const TileId id = decode_tile<false>(P, blockIdx.x, kblocks);
+      const int grp = id.vg / P.tiles_per_group, ntile = id.vg - grp * P.tiles_per_group;
+      const int quarter = warp & 3, pix = id.ptile * kTileM + quarter * 32 + lane, per_img = P.q_h * P.q_w;
+      const int b = pix / per_img, r = pix - b * per_img, qy = r / P.q_w, qx = r - qy * P.q_w;
+      const int oy0 = qy * P.oy_mul + P.oy_add, ox0 = qx * P.ox_mul + P.ox_add;
+      const int ch0 = grp * P.out_group_channels + ntile * P.out_tile_channels;
+      float* op = P.out + (long long)b * P.out_batch_stride + (long long)ch0 * P.out_plane + (long long)oy0 * P.out_pitch + ox0;
+      float* sums = P.partial + (size_t)(id.split * (P.total_tiles / (P.n_pix_tiles * P.splits)) + id.vg) * P.n_pad * P.pix_pad + pix;
+      const float* bias = s_bias + (P.n_bias ? ch0 : 0);
+      const int n_live = min(P.n, (P.out_group_channels - ntile * P.out_tile_channels) * P.cols_per_channel);
+      mbar_wait(acc_full, 0u, failed, P.status, 0x210);
+      tc_fence_after();
+      const bool live = pix < P.n_pix && !failed;
+      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16);
+      for (int c0 = warp < kProducerWarps ? 16 + (warp >> 2) * 16 : 0; c0 < P.n_pad; c0 += 16 * (1 + SETS)) {
+        float v[16];
+        load_acc(acc + (uint32_t)c0, v);
+        if (P.splits > 1) {
+          if (failed) continue;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) sums[(size_t)(c0 + j) * P.pix_pad] = v[j];  // raw sums, lanes along the pixels
+          continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const ColEnt ce = s_cols[c0 + j];
+          const bool in = !P.check_out || ((unsigned)(oy0 + ce.cy) < (unsigned)P.out_lim && (unsigned)(ox0 + ce.cx) < (unsigned)P.out_lim);
+          const float y = v[j] + bias[c0 + j];
+          stg_if(op + ce.off, P.relu ? fmaxf(y, 0.f) : y, live && c0 + j < n_live && in ? 1u : 0u);
+        }
+      }
     }
   }
   tc_fence_before();
@@ -729,7 +792,6 @@ __host__ __device__ inline WgSmem wg_smem(int n_pad, int subs, int stages) {
 // 128-byte-swizzled tile has the same swizzle phase ((warp+16*i) & 7 == warp & 7) for every i.
 template <int SUBS, int NB>
 __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_constant__ WgradParams P) {
-  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -751,14 +813,16 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad_kernel(const __grid_const
   constexpr bool kDual = kNPad <= 64;  // operands from shared memory: an MMA wider than 128 is slower than two narrow ones
   constexpr int kAccCols = kDual ? 2 * kNPad : kNPad;
 
-  for (int i = tid; i < SUBS * kTileM; i += kWgThreads)
-    s_taps[i] = i < subs * kTileM ? P.taps[mgroup * SUBS * kTileM + i] : MaskTap{0, kWgPadBit};
-  if (tid == 0) {
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, 512);
+  } else if (tid == 32) {
     for (int s = 0; s < kWgMaxStages; ++s) { mbar_init(full + 8u * s, kWgProdWarps); mbar_init(empty + 8u * s, 1); }
     mbar_init(acc_full, 1);
     fence_mbar_init();
   }
-  if (warp == 0) tmem_alloc(tmem_slot, 512);
+  pdl_wait();  // (the table too may come from a kernel)
+  for (int i = tid; i < SUBS * kTileM; i += kWgThreads)
+    s_taps[i] = i < subs * kTileM ? P.taps[mgroup * SUBS * kTileM + i] : MaskTap{0, kWgPadBit};
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1704,6 +1768,7 @@ struct GatherProblem {
   size_t smem = 0;
   float* zero = nullptr;          // one 0.f, read by taps out of bounds
   bool inside = false;            // kInside
+  bool one = false;               // ONE: the tiles of the whole batch are short and have a slot each
   int run = 1, run_stride = 0;    // reduction order: 1 = (channel, tap); kRun = (channel / kRun, tap, channel % kRun)
   int splits = 1, split_k = 0;    // splits of the reduction and the length of one (a multiple of 32; k_pad without splits)
   float* partial = nullptr;       // split sums
@@ -1741,12 +1806,15 @@ struct UmmaPlan {
 
 namespace {
 typedef void (*GatherKernel)(const GatherParams, const CUtensorMap);
+template <int MODE, bool ONE = false>
+GatherKernel gather_kernel_of(const GatherProblem& gp) {
+  return gp.sets == 2 ? gather_conv_kernel<2, MODE, ONE> : gather_conv_kernel<4, MODE, ONE>;
+}
 GatherKernel gather_kernel(const GatherProblem& gp, bool weight_grad) {
-  const bool two = gp.sets == 2;
-  if (weight_grad) return two ? gather_conv_kernel<2, kWeightGrad> : gather_conv_kernel<4, kWeightGrad>;
-  if (gp.run == kRun) return two ? gather_conv_kernel<2, kByRun> : gather_conv_kernel<4, kByRun>;
-  if (gp.inside) return two ? gather_conv_kernel<2, kInside> : gather_conv_kernel<4, kInside>;
-  return two ? gather_conv_kernel<2, kByTap> : gather_conv_kernel<4, kByTap>;
+  if (weight_grad) return gather_kernel_of<kWeightGrad>(gp);
+  if (gp.run == kRun) return gp.one ? gather_kernel_of<kByRun, true>(gp) : gather_kernel_of<kByRun>(gp);
+  if (gp.inside) return gather_kernel_of<kInside>(gp);
+  return gp.one ? gather_kernel_of<kByTap, true>(gp) : gather_kernel_of<kByTap>(gp);
 }
 // wgrad_ts_kernel's wide loads: see there.  Below eight taps a window row has fewer than three blocks' worth.
 bool ts_wide(const ConvGeom& G) {
@@ -1863,7 +1931,7 @@ bool use_small_wgrad(long long pixels, int vgroups, int n, int k_real) {
 }
 
 // Tensor-memory and shared-memory budget of a gather problem, room for its packed operand.
-void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias) {
+void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias, int sms, long long tiles) {
   // Tensor memory (512 columns) = accumulator buffers + A stages of 64 columns.  Two accumulator buffers let the epilogue
   // overlap the next tile.
   const int acc = acc_columns(gp.n_pad);
@@ -1879,6 +1947,7 @@ void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias)
     gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = acc <= 64 && !ptab ? 3 : 2; gp.b_stages = b_two;
   }
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
+  gp.one = gp.taps_smem && !gp.inside && gp.split_k <= kOneKblocks * kBlockK && tiles <= (long long)sms * (gp.sets == 2 ? 2 : 1);
   gp.w_half = (size_t)vgroups * gp.n_pad * map_k;
   mem.room(&gp.w, 2 * gp.w_half);
 }
@@ -1945,7 +2014,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       mem.table(&f.taps, t);
       mem.table(&f.cols, c);
       mem.table(&f.zero, std::vector<float>(1, 0.f));
-      finish_problem(mem, f, G.g * f.tiles, G.bias ? G.o : 0);
+      finish_problem(mem, f, G.g * f.tiles, G.bias ? G.o : 0, ctx->planning_sms(), pixel_tiles * G.g * f.tiles * f.splits);
       if (f.splits > 1) sums = std::max(sums, (size_t)f.splits * G.g * f.tiles * f.n_pad * f.pix_pad);
     }
   }
@@ -1990,7 +2059,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       mem.table(&d.taps, t);
       mem.table(&d.cols, c);
       mem.table(&d.zero, std::vector<float>(1, 0.f));
-      finish_problem(mem, d, G.g * d.tiles, 0);
+      finish_problem(mem, d, G.g * d.tiles, 0, ctx->planning_sms(), pixel_tiles * G.g * d.tiles * d.splits);
       if (d.splits > 1) sums = std::max(sums, (size_t)d.splits * G.g * d.tiles * d.n_pad * d.pix_pad);
     }
   }
@@ -2135,7 +2204,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
         for (int q = 0; q < G.m; ++q, ++i) t[i] = MaskTap{row + q * G.s, outside[r] | (outside[q] << 16) | 0x80008000u};
       }
     mem.table(&p->wg_pix, t);
-    finish_problem(mem, w, vgroups, 0);
+    finish_problem(mem, w, vgroups, 0, ctx->planning_sms(), (long long)base_tiles * p->wg_splits);
     if (G.bias) mem.room(&p->wg_plane_sums, (size_t)G.B * G.o);
     sums = std::max(sums, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
   }
@@ -2234,9 +2303,9 @@ SmallConv small_dgrad(const ConvGeom& G, const float* dY, const float* W, float*
   return SmallConv{dY, W, nullptr, dX, batch, G.m, G.n, G.k - 1 - G.p, G.og, G.Dg, G.g, 1, 0};
 }
 
-// Persistent grid: one CTA per SM (4 producer sets) or two (2 sets); then the reduction over the splits, if any.
+// A CTA per tile, or a persistent grid: one CTA per SM (4 producer sets) or two (2 sets); then the reduction over the splits, if any.
 void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp, bool weight_grad = false) {
-  const int grid = std::min(P.total_tiles, (gp.sets == 2 ? 2 : 1) * ctx->launch_sms());
+  const int grid = gp.one ? P.total_tiles : std::min(P.total_tiles, (gp.sets == 2 ? 2 : 1) * ctx->launch_sms());
   launch_pdl(gather_kernel(gp, weight_grad), dim3(grid), dim3(gather_threads(gp.sets)), gp.smem, ctx->stream, P, gp.map);
   if (P.splits > 1) {
     const int vgroups = P.total_tiles / (P.n_pix_tiles * P.splits), cols = P.n_pix_tiles * vgroups * P.n > 32 * ctx->sm_count ? 8 : 1;
