@@ -8,8 +8,8 @@
 // the contraction itself (bias, ReLU, dropout; the masks of the bridges in front); the weight gradient's blocks of the first
 // row of tiles sum the bias gradient on the way.  What bounds these layers is the number of launches (1.5 us each at the least,
 // and as long for the host), so both contractions of a backward pass are one, and forward passes have fc_dot_kernel: 4096 -> 10,
-// 50 images, both ways 13.4 -> 8.9 us.  Three blocks per SM (80 registers): the backward launch took 7.0 us with two, whose 384
-// blocks were two waves, and 6.6 with four; the two launches 3.6 + 4.5.
+// 50 images, both ways 13.4 -> 8.9 us.  Three blocks per SM (80 registers) for two jobs: the backward launch took 7.0 us with two, whose
+// 384 blocks were two waves, and 6.6 with four; the two launches 3.6 + 4.5.  One job keeps its registers.
 #pragma once
 
 namespace {
@@ -66,18 +66,17 @@ __device__ __forceinline__ void fs_stage(float* dst, const float* src, long long
   }
 }
 
-__global__ void __launch_bounds__(kFsThreads, 3) fc_small_kernel(const __grid_constant__ FcSmallJobs J) {
-  pdl_wait();
-  const bool second = blockIdx.x >= J.first;
-  const FcSmallParams& P = J.job[second];
-  const unsigned block = blockIdx.x - (second ? J.first : 0u);
+// TWO: tile and split of one of two jobs (else the grid's x and y, said as such: with variables in their place 290 -> 1200, 97 images
+// forward took 13.4 us instead of 11.3).
+template <bool TWO>
+__device__ __forceinline__ void fc_small_body(const FcSmallParams& P, unsigned tile, unsigned split) {
   __shared__ __align__(16) float s_ab[2 * kFsChunk * kFsPitch];
   __shared__ float s_db[kFsWarps][kFsTile];
   float *s_a = s_ab, *s_b = s_ab + kFsChunk * kFsPitch;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ty = lane >> 2, tx = lane & 3;
-  const int m_tiles = (P.M + kFsTile - 1) / kFsTile, split = (int)(block % (unsigned)P.splits), tile = (int)(block / (unsigned)P.splits);
-  const int n_tile = tile / m_tiles, m0 = (tile - n_tile * m_tiles) * kFsTile, n0 = n_tile * kFsTile;
-  const int r_begin = split * P.r_per_split, r_end = min(P.R, r_begin + P.r_per_split);
+  const int m_tiles = (P.M + kFsTile - 1) / kFsTile, n_tile = (TWO ? tile : blockIdx.x) / m_tiles;  // one grid axis: y ends at 65 535
+  const int m0 = ((TWO ? tile : blockIdx.x) - n_tile * m_tiles) * kFsTile, n0 = n_tile * kFsTile;
+  const int r_begin = (TWO ? split : blockIdx.y) * P.r_per_split, r_end = min(P.R, r_begin + P.r_per_split);
   const bool sum_b = P.db != nullptr && m0 == 0;
   float acc[4][8], db = 0.f;
 #pragma unroll
@@ -119,8 +118,8 @@ __global__ void __launch_bounds__(kFsThreads, 3) fc_small_kernel(const __grid_co
     float t = 0.f;
 #pragma unroll
     for (int w = 0; w < kFsWarps; ++w) t += s_ab[w * kFsTile * kFsTile + i];
-    if (P.splits > 1) {
-      P.out[((long long)split * P.N + n) * P.ld + m] = t;
+    if (TWO ? P.splits > 1 : gridDim.y > 1) {
+      P.out[((long long)(TWO ? split : blockIdx.y) * P.N + n) * P.ld + m] = t;
       continue;
     }
     const long long at = (long long)n * P.ld + m;
@@ -137,6 +136,18 @@ __global__ void __launch_bounds__(kFsThreads, 3) fc_small_kernel(const __grid_co
     P.db[n0 + tid] = t;
   }
 }
+__global__ void __launch_bounds__(kFsThreads) fc_small_kernel(const __grid_constant__ FcSmallParams P) {
+  pdl_wait();
+  fc_small_body<false>(P, 0, 0);
+}
+// Three blocks per SM: see above.
+__global__ void __launch_bounds__(kFsThreads, 3) fc_small_two_kernel(const __grid_constant__ FcSmallJobs J) {
+  pdl_wait();
+  const bool second = blockIdx.x >= J.first;
+  const FcSmallParams& P = J.job[second];
+  const unsigned block = blockIdx.x - (second ? J.first : 0u);
+  fc_small_body<true>(P, block / (unsigned)P.splits, block % (unsigned)P.splits);
+}
 
 // Forward pass of a small layer: out[n][m] = sum_r A[m][r] B[n][r], rows along the reduction.  A block owns NT images x 4 outputs,
 // its warps interleaved steps of 32 (x 4 where rows are on 16-byte boundaries) reduction indices; operands go from L2 straight
@@ -152,7 +163,8 @@ __global__ void __launch_bounds__(kFsThreads, 3) fc_small_kernel(const __grid_co
 // 64 images: four 5.5 us, eight 4.5; 2304 -> 64, 32 images, 64 blocks of eight: 2.9 and 3.1) and the loads are wide (999 -> 333, 32
 // images: 6.6 and 7.8); one or two images take fewer registers and loads (4096 -> 1000, one image: 6.2 us with eight).
 constexpr int kFdM = 4, kFdMaxWarps = 16;
-constexpr double kDotProducts = 2.4e7;
+// (Loads of one word, where K is no multiple of four: 86 -> 960, 187 images (15 M) 6.1 us by the fp32 tiles and 12.9 this way.)
+constexpr double kDotProducts = 2.4e7, kDotNarrowProducts = 5e6;
 constexpr int kDotWideBlocks = 128;
 struct FcDotParams {
   const float *a, *b;

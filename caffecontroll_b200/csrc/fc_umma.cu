@@ -626,18 +626,16 @@ bool use_small_fc(int B, int K, int O) {
   return flops <= (K % 4 || O % 4 ? kSmallFcPaddedFlops : kSmallFcFlops);
 }
 
-// One launch for one or two contractions.
-int fc_small(cct_ctx* ctx, std::initializer_list<FcSmallParams> jobs) {
-  FcSmallJobs J{};
-  unsigned blocks = 0;
-  int n = 0;
-  for (const FcSmallParams& P : jobs) {
-    J.job[n] = P;
-    J.first = n++ ? J.first : ~0u;
-    if (n == 2) J.first = blocks;
-    blocks += (unsigned)((P.M + kFsTile - 1) / kFsTile) * ((P.N + kFsTile - 1) / kFsTile) * P.splits;
-  }
-  launch_pdl(fc_small_kernel, dim3(blocks), dim3(kFsThreads), 0, ctx->stream, J);
+unsigned fc_small_tiles(const FcSmallParams& P) { return (unsigned)((P.M + kFsTile - 1) / kFsTile) * ((P.N + kFsTile - 1) / kFsTile); }
+int fc_small(cct_ctx* ctx, const FcSmallParams& P) {
+  launch_pdl(fc_small_kernel, dim3(fc_small_tiles(P), P.splits), dim3(kFsThreads), 0, ctx->stream, P);
+  CCT_CHECK_LAUNCH(ctx);
+  return CCT_OK;
+}
+int fc_small_two(cct_ctx* ctx, const FcSmallParams& first, const FcSmallParams& second) {
+  const unsigned blocks = fc_small_tiles(first) * first.splits;
+  launch_pdl(fc_small_two_kernel, dim3(blocks + fc_small_tiles(second) * second.splits), dim3(kFsThreads), 0, ctx->stream,
+             FcSmallJobs{{first, second}, blocks});
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
@@ -715,7 +713,7 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
     return CCT_ERR_UNSUPPORTED;
   }
   const bool few = use_small_fc(batch, in_features, out_features);
-  p->dot = (double)batch * in_features * out_features <= kDotProducts;
+  p->dot = (double)batch * in_features * out_features <= (few && in_features % 4 ? kDotNarrowProducts : kDotProducts);
   p->small_forward = few && !p->dot;
   p->small = few || fc_small_faster(ctx->sm_count, batch, in_features, out_features);
   p->small_fwd = fc_small_splits(ctx->sm_count, out_features, batch, in_features);
@@ -784,8 +782,8 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
   if (plan->small_forward || !(plan->Wp || fc_aligned({X, W}))) {
     const int splits = plan->small_forward ? plan->small_fwd : std::min(plan->small_fwd, plan->fwd.P.splits);
     const FcReduceParams post{plan->partial, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, splits, relu};
-    int rc = fc_small(ctx, {FcSmallParams{W, X, K, K, 0, 0, O, B, K, splits, fc_round_up((K + splits - 1) / splits, 32),
-                                          splits > 1 ? plan->partial : Y, splits > 1 ? O4 : O, nullptr, post}});
+    int rc = fc_small(ctx, FcSmallParams{W, X, K, K, 0, 0, O, B, K, splits, fc_round_up((K + splits - 1) / splits, 32),
+                                         splits > 1 ? plan->partial : Y, splits > 1 ? O4 : O, nullptr, post});
     if (rc == CCT_OK && splits > 1) rc = fc_reduce(ctx, post);
     plan->timer.end(0, ctx->stream);
     return rc;
@@ -831,7 +829,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
                         apart(dW, nw, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}}) &&
                         apart(db, nb, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}});
   if (w_small) {
-    if (!together) rc = fc_small(ctx, {W_job});
+    if (!together) rc = fc_small(ctx, W_job);
     if (rc != CCT_OK) return rc;
   } else {
     if (plan->Xp) { fc_pad(ctx, X, plan->Xp, B, K, K4); Xm = plan->Xp; }
@@ -859,7 +857,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     const FcReduceParams post{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4, d_splits, 0, 0, bias_sum};
     const FcSmallParams D_job{W, dY, K, O, 1, 0, K, B, O, d_splits, fc_round_up((O + d_splits - 1) / d_splits, 32),
                               d_splits > 1 ? plan->partial : dX, d_splits > 1 ? K4 : K, nullptr, post};
-    rc = together ? fc_small(ctx, {W_job, D_job}) : fc_small(ctx, {D_job});
+    rc = together ? fc_small_two(ctx, W_job, D_job) : fc_small(ctx, D_job);
     if (rc == CCT_OK && d_splits > 1) rc = fc_reduce(ctx, post);
     plan->timer.end(3, ctx->stream);
   } else if (dX) {

@@ -778,7 +778,7 @@ def test_small_inner_products(ctx, B, K, o, shift):
 # Layers whose passes take different kernels: dot products forward, tensor cores backward (with padded rows too); tensor cores forward, fp32
 # tiles backward; fp32 tiles with splits forward.  Rows on and off a 16-byte boundary.  Tolerance: parity.
 @pytest.mark.parametrize("shift", [0, 1])
-@pytest.mark.parametrize("B,K,o", [(1, 4096, 1000), (4, 4093, 1001), (256, 1000, 100), (128, 999, 333)])
+@pytest.mark.parametrize("B,K,o", [(1, 4096, 1000), (4, 4093, 1001), (256, 1000, 100), (128, 999, 333), (60, 333, 300)])
 def test_inner_products_of_mixed_plans(ctx, B, K, o, shift):
     gen = torch.Generator(device="cuda").manual_seed(B + K + o)
     make = lambda r, c: torch.randn(r * c + shift, device="cuda", generator=gen)[shift:].view(r, c)  # noqa: E731
