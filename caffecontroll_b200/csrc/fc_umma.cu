@@ -87,9 +87,11 @@ __device__ __forceinline__ void fc_store_3d(const void* tmap, uint32_t src, int 
 // The epilogue turns 32 accumulator columns at a time into a 32 x 32 tile in shared memory (one conflict-free store per
 // column) that TMA stores take out, clipping it at the edges: per-lane global stores with their addresses and bounds cost
 // about ten instructions each and made the weight gradient of small batches instruction-bound (fc6, batch 32: 70 us, 2.1 TB/s).
-__global__ void __launch_bounds__(kFcThreads, 2)
-    fc_gemm_kernel(const __grid_constant__ FcGemmParams P, const __grid_constant__ CUtensorMap a_map,
-                   const __grid_constant__ CUtensorMap b_map, const __grid_constant__ CUtensorMap out_map) {
+// TWO: block `block0` of `blocks` that share the tiles (else the grid's: said of the loops as such, since with variables in their place fc6
+// at batch 256 took 308 us both ways instead of 300).
+template <bool TWO>
+__device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtensorMap& a_map, const CUtensorMap& b_map, const CUtensorMap& out_map,
+                                             unsigned block0, unsigned blocks) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
     if (lane == 0) {
       Ring ring;
       int i = 0;
-      for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+      for (int t = TWO ? block0 : blockIdx.x; t < total_tiles; t += TWO ? blocks : gridDim.x) {
         int mt, nt, split, kb0, kb1;
         tile_of(t, mt, nt, split, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb, ++i, ring.advance(P.raw_slots)) {
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
     const uint32_t tmem = warp_uniform(tmem_base);
     Ring raw, lo, ta;
     int i = 0, tile_iter = 0;
-    for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_iter) {
+    for (int t = TWO ? block0 : blockIdx.x; t < total_tiles; t += TWO ? blocks : gridDim.x, ++tile_iter) {
       int mt, nt, split, kb0, kb1;
       tile_of(t, mt, nt, split, kb0, kb1);
       const int buf = tile_iter & (P.acc_bufs - 1), use = tile_iter >> (P.acc_bufs - 1);
@@ -210,7 +212,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
     const int back = min(P.lo_slots, P.a_slots);
     Ring raw, lo, ta;
     int i = 0;
-    for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+    for (int t = TWO ? block0 : blockIdx.x; t < total_tiles; t += TWO ? blocks : gridDim.x) {
       int mt, nt, split, kb0, kb1;
       tile_of(t, mt, nt, split, kb0, kb1);
       for (int kb = kb0; kb < kb1; ++kb, ++i) {
@@ -275,7 +277,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
     uint8_t* out_ptr = base_ptr + L.store_off + (size_t)(warp * P.store_bufs) * kFcStoreTile;
     const uint32_t out_smem = base + L.store_off + (uint32_t)(warp * P.store_bufs) * kFcStoreTile;
     int tile_iter = 0, stores = 0;
-    for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_iter) {
+    for (int t = TWO ? block0 : blockIdx.x; t < total_tiles; t += TWO ? blocks : gridDim.x, ++tile_iter) {
       int mt, nt, split, kb0, kb1;
       tile_of(t, mt, nt, split, kb0, kb1);
       const int buf = tile_iter & (P.acc_bufs - 1), use = tile_iter >> (P.acc_bufs - 1);
@@ -327,6 +329,24 @@ __global__ void __launch_bounds__(kFcThreads, 2)
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, (uint32_t)P.tmem_cols);
+}
+__global__ void __launch_bounds__(kFcThreads, 2)
+    fc_gemm_kernel(const __grid_constant__ FcGemmParams P, const __grid_constant__ CUtensorMap a_map,
+                   const __grid_constant__ CUtensorMap b_map, const __grid_constant__ CUtensorMap out_map) {
+  fc_gemm_body<false>(P, a_map, b_map, out_map, 0, 0);
+}
+// The two contractions of a backward pass of few tiles in one launch: blocks [0, first) work on the weight gradient, those behind them on
+// the data gradient.  Each of such a layer's launches is five microseconds of set-up and hand-overs however little it does: 800 -> 500,
+// 64 images, both ways 19.4 -> 15.2 us, LeNet's iteration 93.6 -> 89.5.
+struct FcJob {
+  FcGemmParams P;
+  CUtensorMap a, b, out;
+};
+__global__ void __launch_bounds__(kFcThreads, 2) fc_gemm_two_kernel(const __grid_constant__ FcJob w, const __grid_constant__ FcJob d, unsigned first) {
+  const bool second = blockIdx.x >= first;
+  const FcGemmParams P = second ? d.P : w.P;
+  const FcJob& J = second ? d : w;
+  fc_gemm_body<true>(P, J.a, J.b, J.out, blockIdx.x - (second ? first : 0u), second ? gridDim.x - first : first);
 }
 
 // db[o] = sum_b dY[b][o] (FullyConnectedBridge_impl.hxx:298: backward_bias_fc).  A block of 32 x 8 threads owns 32
@@ -589,13 +609,35 @@ FcShape fc_weight_shape(int sms, int K, int O, int B) {
   return best;
 }
 
+// The weight gradient's shape in half an SM, and its blocks there: where there are at most two tiles of both contractions for each of
+// the slots; in proportion to the tiles where there are not slots for all.
+FcShape fc_weight_pair_shape(int K, int O, int B) {
+  FcShape s;
+  FcGemmParams& P = s.P;
+  P.M = K; P.N = O;
+  P.m_tiles = (K + kTileM - 1) / kTileM;
+  P.n_pad = O <= 32 ? 32 : 64; P.acc_bufs = 2;
+  P.n_tiles = (O + P.n_pad - 1) / P.n_pad;
+  P.splits = 1;
+  P.kblocks_total = P.kblocks_per_split = (B + kBlockK - 1) / kBlockK;
+  P.a_mn = P.b_mn = 1;
+  s.pair = true;
+  return s;
+}
+int fc_pair_blocks(int sms, FcShape& w, const FcShape& d) {
+  const long long tw = (long long)w.P.m_tiles * w.P.n_tiles, td = (long long)d.P.m_tiles * d.P.n_tiles * d.P.splits, slots = 2ll * sms;
+  if (!d.pair || tw + td > 2 * slots || !fc_fit_rings(w)) return 0;
+  return (int)(tw + td <= slots ? tw : std::max(1ll, slots * tw / (tw + td)));
+}
+
 }  // namespace
 
 struct cct_fc_plan {
   cct_ctx* ctx = nullptr;
   int B = 0, K = 0, O = 0, bias = 0;
   int K4 = 0, O4 = 0;        // row pitches: multiples of four floats
-  FcShape fwd, dgr, wgr;
+  FcShape fwd, dgr, wgr, wgr_pair;  // wgr_pair: the weight gradient's, beside the data gradient in one launch
+  int two = 0;               // blocks of the weight gradient there (0: two launches)
   bool dot = false;          // forward pass by fc_dot_kernel
   bool small_forward = false, small = false;  // forward, backward pass by fc_small_kernel, with these splits (where an operand is off a
   int small_fwd = 1, small_dgr = 1;           // 16-byte boundary too, as far as there is room for their sums)
@@ -616,6 +658,19 @@ int fc_launch(cct_ctx* ctx, const FcShape& s, const FcMap& a, const FcMap& b, co
   const int tiles = P.m_tiles * P.n_tiles * P.splits;
   launch_pdl(fc_gemm_kernel, dim3(std::min(tiles, (s.pair ? 2 : 1) * ctx->launch_sms())), dim3(kFcThreads), s.smem, ctx->stream, P,
              a.map, b.map, out.map);
+  CCT_CHECK_LAUNCH(ctx);
+  return CCT_OK;
+}
+
+int fc_launch_two(cct_ctx* ctx, const cct_fc_plan* plan, float* direct, long long ld_direct) {
+  FcGemmParams W = plan->wgr_pair.P, D = plan->dgr.P;
+  W.direct = direct; W.ld_direct = ld_direct;
+  W.status = D.status = ctx->status_dev;
+  const int tiles = D.m_tiles * D.n_tiles * D.splits, blocks = std::min(tiles, std::max(1, 2 * ctx->launch_sms() - plan->two));
+  const FcJob w{W, plan->x_wgr.map, plan->dy_wgr.map, (direct ? plan->x_wgr : plan->out_wgr).map};
+  const FcJob d{D, plan->w_dgr.map, plan->dy_dgr.map, plan->out_dgr.map};
+  launch_pdl(fc_gemm_two_kernel, dim3(plan->two + blocks), dim3(kFcThreads), std::max(plan->wgr_pair.smem, plan->dgr.smem), ctx->stream, w, d,
+             (unsigned)plan->two);
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
@@ -735,7 +790,9 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   float* at = p->partial + room(sums);
   if (pad_k) { p->Xp = at; p->Wp = at + x; }
   if (pad_o) p->dYp = at + x + w;
-  const cudaError_t e = cudaFuncSetAttribute(fc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+  if (!p->small) p->two = fc_pair_blocks(ctx->sm_count, p->wgr_pair = fc_weight_pair_shape(in_features, out_features, batch), p->dgr);
+  cudaError_t e = cudaFuncSetAttribute(fc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+  if (e == cudaSuccess && p->two) e = cudaFuncSetAttribute(fc_gemm_two_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024);
   if (e != cudaSuccess) {
     ctx->last_error = std::string("cudaFuncSetAttribute(fc_gemm_kernel): ") + cudaGetErrorString(e);
     cudaFree(p->partial);
@@ -822,22 +879,22 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   plan->timer.begin(1, ctx->stream);
   if (plan->dYp && !(w_small && d_small)) { fc_pad(ctx, dY, plan->dYp, B, O, O4); dYm = plan->dYp; }
   const FcSmallParams W_job{X, dY, K, O, 1, 1, K, O, B, 1, B, dW, K, plan->bias ? db : nullptr, FcReduceParams{}};
-  // Both contractions of a small layer in one launch, where neither writes what the other reads or writes.
+  // Both contractions of a layer with few tiles in one launch, where neither writes what the other reads or writes.
   const size_t nx = (size_t)B * K, ny = (size_t)B * O, nw = (size_t)O * K, nb = plan->bias ? O : 0;
   const int d_splits = plan->small ? plan->small_dgr : std::min(plan->small_dgr, plan->dgr.P.splits);
-  const bool together = w_small && d_small && dX && !plan->timer.enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, nb}}) &&
-                        apart(dW, nw, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}}) &&
-                        apart(db, nb, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}});
+  const bool clear = dX && !plan->timer.enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, nb}}) &&
+                     apart(dW, nw, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}}) && apart(db, nb, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}});
+  const bool together = clear && w_small && d_small, two = clear && plan->two && !w_small && !d_small;
+  const bool direct = K4 != K || !fc_aligned({dW});  // dW: an output no tensor map describes
   if (w_small) {
     if (!together) rc = fc_small(ctx, W_job);
     if (rc != CCT_OK) return rc;
   } else {
     if (plan->Xp) { fc_pad(ctx, X, plan->Xp, B, K, K4); Xm = plan->Xp; }
-    const bool direct = K4 != K || !fc_aligned({dW});  // an output no tensor map describes
     rc = fc_operand_map(ctx, &plan->x_wgr, Xm, B, K, K4, 32, true);
     if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_wgr, dYm, B, O, O4, 32, true);
     if (rc == CCT_OK && !direct) rc = fc_output_map(ctx, &plan->out_wgr, dW, K, O, 1, K);
-    if (rc == CCT_OK)
+    if (rc == CCT_OK && !two)
       rc = fc_launch(ctx, plan->wgr, plan->x_wgr, plan->dy_wgr, direct ? plan->x_wgr : plan->out_wgr, direct ? dW : nullptr, K);
     if (rc != CCT_OK) return rc;
     if (plan->bias) {
@@ -866,7 +923,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     rc = fc_operand_map(ctx, &plan->w_dgr, W, O, K, K4, 32, true);
     if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_dgr, dYm, B, O, O4, plan->dgr.P.n_pad, false);
     if (rc == CCT_OK) rc = fc_output_map(ctx, &plan->out_dgr, plan->partial, K, B, plan->dgr.P.splits, K4);
-    if (rc == CCT_OK) rc = fc_launch(ctx, plan->dgr, plan->w_dgr, plan->dy_dgr, plan->out_dgr);
+    if (rc == CCT_OK) rc = two ? fc_launch_two(ctx, plan, direct ? dW : nullptr, K) : fc_launch(ctx, plan->dgr, plan->w_dgr, plan->dy_dgr, plan->out_dgr);
     if (rc == CCT_OK)
       rc = fc_reduce(ctx, FcReduceParams{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4,
                                          plan->dgr.P.splits, 0, 0, bias_sum});

@@ -827,3 +827,34 @@ def test_small_gradients_in_one_launch(ctx, shape):
     torch.nn.functional.conv2d(Xd, Wd, None, s, p, 1, g).backward(dY.double())
     for got, ref, name in ((dX, Xd.grad, "dX"), (over[0], Xd.grad, "dX over X"), (dW, Wd.grad, "dW"), (db, dY.double().sum((0, 2, 3)), "db")):
         assert_close(got.cpu().numpy(), ref.float().cpu().numpy(), name)
+
+
+# Both contractions of a backward pass in one launch of the tensor-core kernel: a slot for every tile and up to two tiles a slot, one output
+# tile, outputs that no tensor map describes, and the sum of dY where there is a bias; dX over X: one launch more.  Tolerance: parity.
+@pytest.mark.parametrize("B,K,o,bias", [(64, 800, 500, 1), (16, 2048, 1000, 0), (128, 516, 512, 1), (40, 2051, 1030, 1), (1, 1300, 1028, 0)])
+def test_two_contractions_in_one_launch(ctx, B, K, o, bias):
+    gen = torch.Generator(device="cuda").manual_seed(B + K + o)
+    make = lambda r, c: torch.randn(r, c, device="cuda", generator=gen)  # noqa: E731
+    X, W, dY, keep = make(B, K), make(o, K), make(B, o), (torch.rand(B, K, device="cuda", generator=gen) < 0.5).int()
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, bias, C.byref(plan)), "plan", ctx.h)
+
+    def run(x, dx):
+        dW, db = torch.zeros_like(W), torch.zeros(o, device="cuda")
+        torch.cuda.synchronize()
+        before = capi.kernel_launches()
+        capi.check(ctx.lib.cct_fc_backward(plan, q(x), q(W), q(dY), q(dx), q(dW), q(db), 1, q(keep), 2.0), "backward", ctx.h)
+        ctx.sync()
+        return dx, dW, db, capi.kernel_launches() - before
+
+    dX, dW, db, launches = run(X, torch.zeros_like(X))
+    x = X.clone()
+    over = run(x, x)
+    ctx.lib.cct_fc_plan_destroy(plan)
+    pads = 2 * (K % 4 != 0) + (o % 4 != 0)
+    assert launches == 2 + pads and over[3] == 3 + pads
+    Xd, Wd, dYd = X.double(), W.double(), dY.double()
+    refs = [(dYd @ Wd) * keep * 2 * (X > 0), dYd.T @ Xd] + [dYd.sum(0)] * bias
+    for got in ((dX, dW, db), over):
+        for a, r, name in zip(got, refs, ("dX", "dW", "db")):
+            assert_close(a.cpu().numpy(), r.float().cpu().numpy(), name)
