@@ -31,23 +31,36 @@ struct SmallConv {
   int positions, row_groups;        // batch * row_groups * n_out lanes
   int col_tiles;                    // channel tiles of CT per group
   int share;                        // 1: the block's warps split the input channels of the same 32 positions
+  static constexpr int kThreads = 512;  // at most
+  __host__ __device__ static constexpr int blocks(int) { return 0; }  // per SM at the least: not said (with 1 the compiler takes twice the registers)
 };
 
-// Rows per lane (row and column masks share 32 bits); with one channel there are registers for eight, which load 3 values for 2
-// outputs where four load 2 for 1 (5 x 5; the pass above with four: 20.0 us).
-__host__ __device__ constexpr int small_rows(int K, int CT) { return K >= 11 ? 2 : CT == 1 ? 8 : 4; }
+// Rows per lane (row and column masks share 32 bits).  With one channel there are registers for eight, which load 3 values of a 5 x 5 window
+// for 2 outputs where four load 2 for 1 (LeNet conv1, both passes, with four: 20.0 us, not 19.3); a 3 x 3 window gains no such thing
+// (44 images 32 x 32, two groups: 6.0 us with four, 6.5 with eight).
+__host__ __device__ constexpr int small_rows(int K, int S, int CT) { return K >= 11 ? 2 : CT == 1 && S == 1 && K == 5 ? 8 : 4; }
 // Shared memory: the weights, afterwards the warps' sums.
-inline size_t small_conv_smem(int K, int ct, int ci, int sharing_warps) {
-  return std::max((size_t)ci * K * K * ct, (size_t)sharing_warps * small_rows(K, ct) * ct * 32) * sizeof(float);
+inline size_t small_conv_smem(int K, int s, int ct, int ci, int sharing_warps) {
+  return std::max((size_t)ci * K * K * ct, (size_t)sharing_warps * small_rows(K, s, ct) * ct * 32) * sizeof(float);
 }
 
-// Block (bx, by) of the pass's grid: positions, channel tile.
-template <int K, int S, int CT>
-__device__ __forceinline__ void small_conv_block(const SmallConv& P, float* small_smem, int bx, int by) {
-  constexpr int JR = small_rows(K, CT), R = (JR - 1) * S + K;
+// JOB: SmallConv, the pass alone, whose grid's x is positions and y channel tiles; or SmallBackward below, both gradients of a layer.  The
+// pass's text stands in the kernel: as a function called from two kernels 6 images 16 x 16, 3 -> 8 channels 5 x 5 by 2 took 6.5 us, not 6.0.
+template <int K, int S, int CT, typename JOB>
+__global__ void __launch_bounds__(JOB::kThreads, JOB::blocks(CT)) small_conv_kernel(const __grid_constant__ JOB J) {
+  pdl_wait();
+  constexpr bool ALONE = std::is_same<JOB, SmallConv>::value;
+  int bx = 0, by = 0;
+  if constexpr (!ALONE) {
+    if (J.weight_gradient()) return;
+    by = blockIdx.x / J.grid_x, bx = blockIdx.x - by * J.grid_x;
+  }
+  const SmallConv& P = J;
+  constexpr int JR = small_rows(K, S, CT), R = (JR - 1) * S + K;
   static_assert(R + K <= 32, "row and column bits share a word");
+  extern __shared__ __align__(16) float small_smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int grp = by / P.col_tiles, c0 = (by - grp * P.col_tiles) * CT;
+  const int grp = (ALONE ? blockIdx.y : by) / P.col_tiles, c0 = ((ALONE ? blockIdx.y : by) - grp * P.col_tiles) * CT;
   const int nwarps = blockDim.x >> 5;
   // weights of this block's channels; consecutive threads read consecutive elements of a channel's window
   for (int e = tid; e < P.ci * K * K; e += blockDim.x) {
@@ -63,7 +76,7 @@ __device__ __forceinline__ void small_conv_block(const SmallConv& P, float* smal
     for (int c = 0; c < CT; ++c) small_smem[((d * K + uc) * K + ur) * CT + c] = wv[c];
   }
   // where this lane works: image, first row, column
-  const int want = P.share ? bx * 32 + lane : bx * (int)blockDim.x + tid;
+  const int want = P.share ? (ALONE ? blockIdx.x : bx) * 32 + lane : (ALONE ? blockIdx.x : bx) * blockDim.x + tid;
   const int pos = min(want, P.positions - 1);
   const int bg = pos / P.n_out, x = pos - bg * P.n_out;
   const int b = bg / P.row_groups, y0 = (bg - b * P.row_groups) * JR;
@@ -150,22 +163,16 @@ __device__ __forceinline__ void small_conv_block(const SmallConv& P, float* smal
     finish(y, i / CT, i % CT);
   }
 }
-template <int K, int S, int CT>
-__global__ void __launch_bounds__(512) small_conv_kernel(const __grid_constant__ SmallConv P) {
-  pdl_wait();
-  extern __shared__ __align__(16) float small_smem[];
-  small_conv_block<K, S, CT>(P, small_smem, blockIdx.x, blockIdx.y);
-}
 
 typedef void (*SmallConvKernel)(const SmallConv);
 template <int CT>
 SmallConvKernel small_conv_pick_ks(int k, int s) {
   switch (k * 10 + s) {
-    case 11: return small_conv_kernel<1, 1, CT>;
-    case 31: return small_conv_kernel<3, 1, CT>;   case 32: return small_conv_kernel<3, 2, CT>;
-    case 51: return small_conv_kernel<5, 1, CT>;   case 52: return small_conv_kernel<5, 2, CT>;
-    case 71: return small_conv_kernel<7, 1, CT>;   case 72: return small_conv_kernel<7, 2, CT>;
-    case 114: return small_conv_kernel<11, 4, CT>;
+    case 11: return small_conv_kernel<1, 1, CT, SmallConv>;
+    case 31: return small_conv_kernel<3, 1, CT, SmallConv>;   case 32: return small_conv_kernel<3, 2, CT, SmallConv>;
+    case 51: return small_conv_kernel<5, 1, CT, SmallConv>;   case 52: return small_conv_kernel<5, 2, CT, SmallConv>;
+    case 71: return small_conv_kernel<7, 1, CT, SmallConv>;   case 72: return small_conv_kernel<7, 2, CT, SmallConv>;
+    case 114: return small_conv_kernel<11, 4, CT, SmallConv>;
   }
   return nullptr;
 }
@@ -278,25 +285,31 @@ __global__ void __launch_bounds__(kSwThreads) small_wgrad_kernel(const __grid_co
 }
 
 // Both gradients of a layer with stride 1 in one launch: neither reads what the other writes.  Blocks [0, conv_blocks) are the data
-// gradient's.  LeNet conv1 at batch 64, forward and
-// backward: 22.2 -> 19.4 us, three launches instead of four (three blocks per SM; with two 19.6, with four, and spills, 20.4).
-struct SmallBackward {
+// gradient's.  LeNet conv1 at batch 64, forward and backward: 22.2 -> 19.3 us, three launches instead of four (three blocks per SM for
+// one-channel data gradients; with two 19.6, with four, and spills, 20.4).  Up to kSmallRounds rounds of blocks: 64 images 20 x 20, 3 -> 16
+// channels 5 x 5 9.4 + 7.9 -> 13.4 us (1.3 rounds), 16 images 30 x 30, 6 -> 12 channels 3 x 3 6.3 + 4.8 -> 9.9 (1.6); 21 images 18 x 18, 42
+// -> 24 channels 1 x 1 4.5 + 5.4 -> 11.7 (2.6).  Not where the data gradient alone has more warps per block than go here: 3 images 9 x 9,
+// 3 -> 259 channels 3 x 3 4.5 + 17.3 -> 23.8.
+constexpr int kSmallRounds = 2;
+struct SmallBackward : SmallConv {  // the base: the data gradient
   SmallWgrad w;
-  SmallConv d;
-  int d_grid_x, conv_blocks;
+  int grid_x, conv_blocks;  // of the data gradient
+  static constexpr int kThreads = kSwThreads;
+  __host__ __device__ static constexpr int blocks(int ct) { return ct == 1 ? 3 : 2; }  // per SM
+  __device__ bool weight_gradient() const {
+    extern __shared__ __align__(16) float small_smem[];
+    const int block = (int)blockIdx.x - conv_blocks;
+    if (block >= 0) small_wgrad_block(w, small_smem, block % w.tiles, block / w.tiles);
+    return block >= 0;
+  }
 };
-template <int K, int CT>
-__global__ void __launch_bounds__(kSwThreads, CT == 1 ? 3 : 2) small_backward_kernel(const __grid_constant__ SmallBackward J) {
-  pdl_wait();
-  extern __shared__ __align__(16) float small_smem[];
-  const int block = (int)blockIdx.x - J.conv_blocks;
-  if (block >= 0) small_wgrad_block(J.w, small_smem, block % J.w.tiles, block / J.w.tiles);
-  else small_conv_block<K, 1, CT>(J.d, small_smem, blockIdx.x % J.d_grid_x, blockIdx.x / J.d_grid_x);
-}
 typedef void (*SmallBackwardKernel)(const SmallBackward);
 template <int CT>
 SmallBackwardKernel small_backward_pick_k(int k) {
-  return k == 1 ? small_backward_kernel<1, CT> : k == 3 ? small_backward_kernel<3, CT> : k == 5 ? small_backward_kernel<5, CT> : small_backward_kernel<7, CT>;
+  return k == 1   ? small_conv_kernel<1, 1, CT, SmallBackward>
+         : k == 3 ? small_conv_kernel<3, 1, CT, SmallBackward>
+         : k == 5 ? small_conv_kernel<5, 1, CT, SmallBackward>
+                  : small_conv_kernel<7, 1, CT, SmallBackward>;
 }
 SmallBackwardKernel small_backward_pick(int k, int ct) {
   return ct == 8 ? small_backward_pick_k<8>(k) : ct == 4 ? small_backward_pick_k<4>(k) : small_backward_pick_k<1>(k);

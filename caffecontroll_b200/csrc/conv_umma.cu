@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 #include <cuda.h>
@@ -236,7 +237,7 @@ enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3 };
 // ONE: every CTA has one tile, a short one (kOneKblocks).  There is no next tile then for the epilogue to overlap with, and the producers,
 // who are through, take their share of its columns (six chunks of 16 took four warps 1.2 us); in front of the first k-block stood three
 // trips to L2 for the tables and the bias, one behind the other, and the allocation of tensor memory (1.3 us in all), now one trip
-// beside the allocation.  conv3 of one image 13.6 -> 12.9 us, 37 images of 50 -> 75 channels both ways 36.3 -> 35.1.  Not for the
+// beside the allocation.  conv3 of one image 13.6 -> 13.0 us, 37 images of 50 -> 75 channels both ways 36.3 -> 34.9.  Not for the
 // persistent kernels' last tiles, nor for the other two modes: the registers it takes spill (AlexNet conv1 at batch 256 1 211 -> 1 227
 // us both ways; LeNet conv2's forward kernel 9.9 -> 11.1).  Where a tile is long it gains nothing (CaffeNet at batch 32 1 238 -> 1 245 us).
 constexpr int kOneKblocks = 32;
@@ -1920,7 +1921,7 @@ constexpr double kSmallConvFlops = 1.5e8, kSmallWideFlops = 8e7, kSmallWgradFlop
 // Channels per block of small_conv_kernel for one pass (0: the tensor-core kernel).
 int use_small_conv(int k, int s, long long out_pixels, int groups, int ci, int co) {
   const int ct = small_conv_ct(co);
-  if (!small_conv_pick(k, s, ct) || small_conv_smem(k, ct, ci, 0) > 48 * 1024) return 0;
+  if (!small_conv_pick(k, s, ct) || small_conv_smem(k, s, ct, ci, 0) > 48 * 1024) return 0;
   if ((long long)groups * ((co + 3) / 4) > 65535) return 0;  // channel tiles (of four at least) are a grid's y
   const double flops = 2.0 * out_pixels * groups * ((co + ct - 1) / ct * ct) * ci * k * k;
   return flops <= (k >= 7 ? kSmallWideFlops : kSmallConvFlops) ? ct : 0;
@@ -2270,13 +2271,13 @@ PackDgrad pack_dgrad_job(const UmmaPlan* p, const float* W) {
   return J;
 }
 
-// Grid of a pass by small_conv_block, and its shared memory; `warps` > 0: that many per block.
+// Grid of a pass by small_conv_kernel, and its shared memory; `warps` > 0: that many per block.
 struct SmallConvShape {
   int ct, warps, x, y;
   size_t smem;
 };
-SmallConvShape shape_small_conv(cct_ctx* ctx, SmallConv& P, int k, int ct, int warps = 0) {
-  const int jr = small_rows(k, ct);  // (the same for four and eight channels)
+SmallConvShape shape_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct, int warps = 0) {
+  const int jr = small_rows(k, s, ct);  // (the same for four and eight channels)
   P.row_groups = (P.n_out + jr - 1) / jr;
   P.positions = P.batch * P.row_groups * P.n_out;
   // Narrower channel tiles and more warps on the input channels until the SMs have about sixteen warps each.
@@ -2287,15 +2288,15 @@ SmallConvShape shape_small_conv(cct_ctx* ctx, SmallConv& P, int k, int ct, int w
   if (!warps) {
     warps = 4;
     while (P.share && warps < 16 && P.ci >= 4 * warps && lots * P.groups * P.col_tiles * warps < want &&
-           small_conv_smem(k, ct, P.ci, 2 * warps) <= 48 * 1024)
+           small_conv_smem(k, s, ct, P.ci, 2 * warps) <= 48 * 1024)
       warps *= 2;
   }
   const int per_block = P.share ? 32 : 32 * warps;
   return SmallConvShape{ct, warps, (P.positions + per_block - 1) / per_block, P.groups * P.col_tiles,
-                        small_conv_smem(k, ct, P.ci, P.share ? warps : 0)};
+                        small_conv_smem(k, s, ct, P.ci, P.share ? warps : 0)};
 }
 void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct) {
-  const SmallConvShape g = shape_small_conv(ctx, P, k, ct);
+  const SmallConvShape g = shape_small_conv(ctx, P, k, s, ct);
   launch_pdl(small_conv_pick(k, s, g.ct), dim3(g.x, g.y), dim3(32 * g.warps), g.smem, ctx->stream, P);
 }
 // The data gradient of a stride-1 layer as a convolution of dY.
@@ -2381,7 +2382,11 @@ int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W
   if (p->w_small && p->dgr.small_ct && dX && !t->enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, G.o}}) &&
       apart(dW, nw, {{W, nw}, {dY, ny}}) && (!G.bias || apart(db, G.o, {{W, nw}, {dY, ny}}))) {
     SmallConv d = small_dgrad(G, dY, W, dX, G.B);
-    return weight_gradient(ctx, p, X, dY, dW, db, t, nullptr, &d);
+    const int warps = shape_small_conv(ctx, d, G.k, 1, p->dgr.small_ct).warps;
+    const SmallConvShape g = shape_small_conv(ctx, d, G.k, 1, p->dgr.small_ct, kSwWarps);
+    const long long blocks = (long long)p->ws_rows * p->ws_cols * G.g * p->wt_tiles * p->w_splits + (long long)g.x * g.y;
+    if (warps <= kSwWarps && blocks <= (long long)kSmallRounds * SmallBackward::blocks(g.ct) * ctx->sm_count)
+      return weight_gradient(ctx, p, X, dY, dW, db, t, nullptr, &d);
   }
   int rc = umma_conv_wgrad(ctx, p, X, dY, dW, db, t, dX ? W : nullptr);
   if (rc == CCT_OK && dX) rc = umma_conv_dgrad(ctx, p, W, dY, dX, t, 0, false);
@@ -2451,9 +2456,9 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       const SmallWgrad J{P, rows_pad, p->ws_rows, p->ws_cols, p->ws_pix, p->ws_rows * p->ws_cols * vgroups};
       const int blocks = J.tiles * p->w_splits;
       if (with) {
-        const SmallConvShape g = shape_small_conv(ctx, *with, G.k, p->dgr.small_ct, kSwWarps);
+        const SmallConvShape g = shape_small_conv(ctx, *with, G.k, 1, p->dgr.small_ct, kSwWarps);
         launch_pdl(small_backward_pick(G.k, g.ct), dim3(blocks + g.x * g.y), dim3(kSwThreads), std::max(kSwSmem, g.smem), ctx->stream,
-                   SmallBackward{J, *with, g.x, g.x * g.y});
+                   SmallBackward{*with, J, g.x, g.x * g.y});
       } else {
         launch_pdl(small_wgrad_kernel, dim3(blocks), dim3(kSwThreads), kSwSmem, ctx->stream, J);
       }
