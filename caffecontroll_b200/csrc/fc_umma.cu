@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kFcThreads, 2)
 }
 // The two contractions of a backward pass of few tiles in one launch: blocks [0, first) work on the weight gradient, those behind them on
 // the data gradient.  Each of such a layer's launches is five microseconds of set-up and hand-overs however little it does: 800 -> 500,
-// 64 images, both ways 19.4 -> 15.2 us, LeNet's iteration 93.6 -> 89.5.
+// 64 images, both ways 19.4 -> 15.2 us, LeNet's iteration 94.2 -> 89.9.
 struct FcJob {
   FcGemmParams P;
   CUtensorMap a, b, out;
