@@ -838,10 +838,12 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
   }
   if (plan->small_forward || !(plan->Wp || fc_aligned({X, W}))) {
     const int splits = plan->small_forward ? plan->small_fwd : std::min(plan->small_fwd, plan->fwd.P.splits);
+    // through sums: splits, or an output over an operand that other blocks still read
+    const bool sums = splits > 1 || !apart(Y, (size_t)B * O, {{X, (size_t)B * K}, {W, (size_t)O * K}});
     const FcReduceParams post{plan->partial, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, splits, relu};
     int rc = fc_small(ctx, FcSmallParams{W, X, K, K, 0, 0, O, B, K, splits, fc_round_up((K + splits - 1) / splits, 32),
-                                         splits > 1 ? plan->partial : Y, splits > 1 ? O4 : O, nullptr, post});
-    if (rc == CCT_OK && splits > 1) rc = fc_reduce(ctx, post);
+                                         sums ? plan->partial : Y, sums ? O4 : O, nullptr, sums ? FcReduceParams{} : post});
+    if (rc == CCT_OK && sums) rc = fc_reduce(ctx, post);
     plan->timer.end(0, ctx->stream);
     return rc;
   }
@@ -882,6 +884,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   // Both contractions of a layer with few tiles in one launch, where neither writes what the other reads or writes.
   const size_t nx = (size_t)B * K, ny = (size_t)B * O, nw = (size_t)O * K, nb = plan->bias ? O : 0;
   const int d_splits = plan->small ? plan->small_dgr : std::min(plan->small_dgr, plan->dgr.P.splits);
+  const bool d_sums = d_splits > 1 || !apart(dX, nx, {{dY, ny}, {W, nw}});  // as in the forward pass
   const bool clear = dX && !plan->timer.enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, nb}}) &&
                      apart(dW, nw, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}}) && apart(db, nb, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}});
   const bool together = clear && w_small && d_small, two = clear && plan->two && !w_small && !d_small;
@@ -900,7 +903,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     if (plan->bias) {
       // With the data gradient's reduction, unless there is none, or it writes where the sum reads (dX over dY).
       bias_sum = FcBiasSum{dY, db, B, O};
-      if (!dX || (d_small && d_splits == 1) || !apart(dX, nx, {{dY, ny}})) {
+      if (!dX || (d_small && !d_sums) || !apart(dX, nx, {{dY, ny}})) {
         launch_pdl(fc_bias_grad_kernel, dim3((O + 31) / 32), dim3(256), 0, ctx->stream, bias_sum);
         bias_sum = FcBiasSum{};
       }
@@ -913,9 +916,9 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     plan->timer.begin(3, ctx->stream);
     const FcReduceParams post{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4, d_splits, 0, 0, bias_sum};
     const FcSmallParams D_job{W, dY, K, O, 1, 0, K, B, O, d_splits, fc_round_up((O + d_splits - 1) / d_splits, 32),
-                              d_splits > 1 ? plan->partial : dX, d_splits > 1 ? K4 : K, nullptr, post};
+                              d_sums ? plan->partial : dX, d_sums ? K4 : K, nullptr, d_sums ? FcReduceParams{} : post};
     rc = together ? fc_small_two(ctx, W_job, D_job) : fc_small(ctx, D_job);
-    if (rc == CCT_OK && d_splits > 1) rc = fc_reduce(ctx, post);
+    if (rc == CCT_OK && d_sums) rc = fc_reduce(ctx, post);
     plan->timer.end(3, ctx->stream);
   } else if (dX) {
     plan->timer.begin(3, ctx->stream);

@@ -211,8 +211,8 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
                    const uint32_t* drop_mask, float drop_scale);
 /* dW = dY^T * X and db = column sums of dY (both overwritten); dX = dY * W when dX != NULL.  The bridges in front of the
  * layer can be folded into dX: in_drop_mask != NULL multiplies dX by (mask != 0) * in_drop_scale (DropoutBridge::backward),
- * in_relu != 0 by [X > 0] (ReLUBridge::backward; X is this layer's input, i.e. the output of those bridges).  On the tensor
- * cores dX may overlap dY (in_features == out_features); in small layers, which the fp32 kernels take, it may not. */
+ * in_relu != 0 by [X > 0] (ReLUBridge::backward; X is this layer's input, i.e. the output of those bridges).  dX may overlap
+ * dY, as Y may overlap X in the forward pass: the results are those of separate buffers. */
 int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const float* dY, float* dX, float* dW, float* db,
                     int in_relu, const uint32_t* in_drop_mask, float in_drop_scale);
 /* Per-kernel-group device times of the most recent calls (as cct_conv_plan_last_timings): ms[0] forward, ms[1] weight

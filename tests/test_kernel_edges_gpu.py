@@ -365,6 +365,49 @@ def test_inner_product_gradient_in_place(ctx, B, K, shift):
     ctx.lib.cct_fc_plan_destroy(plan)
 
 
+# Outputs over operands in layers of the fp32 kernels, with and without splits of a reduction, and where an operand off a 16-byte boundary
+# brings a layer of the tensor cores there: Y over X, dX over dY, dX over the weights, bit for bit what separate buffers give, every time.
+@pytest.mark.parametrize("B,K,off", [(64, 32, 0), (256, 200, 0), (450, 210, 0), (577, 256, 0), (640, 256, 0), (385, 200, 0), (40, 256, 0), (256, 640, 1)])
+def test_inner_products_over_their_operands(ctx, B, K, off):
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    make = lambda *sh: torch.randn(sh, generator=gen, device="cuda")  # noqa: E731
+    X, W, dY, b = make(B, K), make(K, K), make(B, K), make(K)
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, K, 1, C.byref(plan)), "plan", ctx.h)
+
+    def run(over):
+        words = off + (B + K) * K
+        spare = lambda: torch.zeros(words, device="cuda")[off:]  # noqa: E731
+        x, w, dy, y, dx, dw, db = (spare() for _ in range(7))
+        for buffer, values in ((x, X), (w, W), (dy, dY)):
+            buffer[:values.numel()].copy_(values.view(-1))
+        if over == "Y over X":
+            y = x
+        elif over == "dX over dY":
+            dx = dy
+        elif over == "dX over W":
+            dx = w
+        torch.cuda.synchronize()
+        if over in ("", "Y over X"):
+            capi.check(ctx.lib.cct_fc_forward(plan, q(x), q(w), q(b), q(y), 1, None, 1.0), "forward", ctx.h)
+        if over != "Y over X":
+            capi.check(ctx.lib.cct_fc_backward(plan, q(x), q(w), q(dy), q(dx), q(dw), q(db), 0, None, 1.0), "backward", ctx.h)
+        ctx.sync()
+        return y[:B * K], dx[:B * K], dw[:K * K], db[:K]
+
+    apart = run("")
+    for _ in range(5):
+        assert torch.equal(run("Y over X")[0], apart[0])
+        for over in ("dX over dY", "dX over W"):
+            for got, want, name in zip(run(over)[1:], apart[1:], ("dX", "dW", "db")):
+                assert torch.equal(got, want), (over, name)
+    ctx.lib.cct_fc_plan_destroy(plan)
+    for got, ref, name in zip(apart, ((X.double() @ W.double().T + b.double()).clamp(min=0), dY.double() @ W.double(),
+                                      dY.double().T @ X.double(), dY.double().sum(0)), ("Y", "dX", "dW", "db")):
+        assert_close(got.cpu().numpy(), ref.float().view(-1).cpu().numpy(), name)
+
+
 # Operands four bytes off a 16-byte boundary, which no tensor map describes: all of them, or one at a time, with feature counts
 # that are and are not multiples of four, above the size of the fp32 kernel.  Tolerance as above.
 @pytest.mark.parametrize("B,K,o", [(129, 772, 1027), (129, 770, 1028), (130, 1024, 512), (40, 2051, 1030)])
