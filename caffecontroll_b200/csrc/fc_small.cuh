@@ -155,16 +155,11 @@ __global__ void __launch_bounds__(kFsThreads, 3) fc_small_two_kernel(const __gri
 // with a long reduction took 32 splits, and a launch to add them; with the splits in a cluster, adding through distributed shared
 // memory, 512 indices per block took longer than that launch.  4096 -> 10, 50 images: 4.4 + 2.7 -> 3.4 us, 500 -> 10, 64 images:
 // 6.3 + 2.4 -> 2.3.
-// What bounds it is the traffic from L2, a quarter of a word per product and more; fc_gemm_kernel's two launches take five
-// microseconds however little there is to do.  Where the line lies (products; tensor cores -> this): 512 -> 128, 256 images (17 M)
-// 10.5 -> 4.5 us; 512 -> 512, 64 images (17 M) 6.7 -> 4.5, 128 (34 M) 8.2 -> 7.7, 256 (67 M) 11.6 -> 13.3; 800 -> 500, 64 images
-// (26 M) 7.7 -> 8.0; 4096 -> 1000, one image 8.5 -> 3.2, four 8.8 -> 5.4, eight (33 M) 8.8 -> 6.5, 16 (66 M) 8.8 -> 11.8; 4096 ->
-// 4096, one image (17 M) 17.1 -> 15.1, two 17.2 -> 17.9.  Eight images per block where that leaves kDotWideBlocks blocks (512 -> 512,
+// What bounds it is the traffic from L2 (3/8 of a word per product with eight images, 1/2 with four, 5/4 with one); fc_gemm_kernel's two
+// launches take five microseconds however little there is to do.  Eight images per block where that leaves kDotWideBlocks blocks (512 -> 512,
 // 64 images: four 5.5 us, eight 4.5; 2304 -> 64, 32 images, 64 blocks of eight: 2.9 and 3.1) and the loads are wide (999 -> 333, 32
 // images: 6.6 and 7.8); one or two images take fewer registers and loads (4096 -> 1000, one image: 6.2 us with eight).
 constexpr int kFdM = 4, kFdMaxWarps = 16;
-// (Loads of one word, where K is no multiple of four: 86 -> 960, 187 images (15 M) 6.1 us by the fp32 tiles and 12.9 this way.)
-constexpr double kDotProducts = 2.4e7, kDotNarrowProducts = 5e6;
 constexpr int kDotWideBlocks = 128;
 struct FcDotParams {
   const float *a, *b;
@@ -240,10 +235,30 @@ void (*fc_dot_pick(int nt))(const FcDotParams) {
   return nt == 1 ? fc_dot_kernel<VEC, 1> : nt == 2 ? fc_dot_kernel<VEC, 2> : nt == 4 ? fc_dot_kernel<VEC, 4> : fc_dot_kernel<VEC, 8>;
 }
 
-// Splits of the reduction: about two blocks per SM, at least 64 indices each.
+// Splits of the reduction: about two blocks per SM, about 128 indices each at the least.
 int fc_small_splits(int sms, int M, int N, int R) {
   const int tiles = ((M + kFsTile - 1) / kFsTile) * ((N + kFsTile - 1) / kFsTile);
   return std::max(1, std::min(2 * sms / tiles, R / 128));
+}
+
+// Whether a forward pass is faster by fc_dot_kernel.  Its time follows the products with the reduction rounded up, since lanes behind its
+// end have none (a warp's step is 128 indices, 32 off a 16-byte boundary, where short steps also pay for their blocks: 64 in their place):
+// 1.8 us + 0.18 per million by wide loads, 0.35 and more by narrow ones.
+// Against one launch of fc_small_kernel (`one_launch`: a small layer without splits; 3.6 us up to 64 indices, 4.0 - 5.5 to 255), us there ->
+// here, on both sides of each line: wide 64 -> 512, 128 images (8 M) 4.0 -> 3.2, 256 (17 M) 4.0 -> 5.0; 16 -> 130, 640 (11 M) 3.6 -> 4.0;
+// 128 -> 1000, 64 (8 M) 4.5 -> 3.1, 128 (16 M) 4.6 -> 5.0; narrow 16 -> 2048, 32 (4.2 M) 3.7 -> 4.0; 130 -> 500, 64 (6.1 M) 5.4 -> 5.0; 128 ->
+// 128, 1024 (17 M) 4.6 -> 11.2.
+// Against two launches, of fc_small_kernel with splits or of the tensor cores: wide 512 -> 128, 256 images (17 M) 6.2 -> 4.6; 512 -> 512, 64
+// (17 M) 6.7 -> 4.5, 128 (34 M) 8.2 -> 7.7, 256 (67 M) 11.6 -> 13.3; 1024 -> 1000, 20 (20 M) 6.45 -> 6.45; 800 -> 500, 64 (29 M) 7.7 -> 8.0;
+// 16 -> 2048, 384 (101 M) 9.6 -> 18.2.  Narrow ones against the tiles, whose splits grow with the reduction: 256 -> 500, 64 images (8.2 M) 6.1 ->
+// 6.7; 1024 -> 1000, eight (8.2 M) 7.4 -> 5.2, 16 (16 M) 7.7 -> 8.6; 512 -> 500, 64 (16 M) 6.3 -> 12.8; 2048 -> 100, 64 (13 M) 6.2 -> 6.0; 4096
+// -> 100, 50 (20 M) 8.4 -> 8.5.  Up to four images are the stream of the weights, which the tiles read for images that are not there: 4096
+// -> 1000, four (16 M) 15.9 -> 5.4; `padded`: the tensor cores' four launches, 4093 -> 1001, four 16.3 -> 5.4.
+bool fc_dot_faster(int B, int K, int O, bool wide, bool one_launch, bool padded) {
+  const int step = wide ? 128 : 64;
+  const double products = (double)B * O * ((K + step - 1) / step) * step;
+  if (one_launch) return products <= (wide ? (K <= 64 ? 1e7 : 1.3e7) : (K <= 64 ? 4e6 : 6.4e6));
+  return products <= (wide || padded || B <= 4 ? 2.4e7 : std::min(2.4e7, 6.5e6 + 5e3 * K));
 }
 
 // Whether a backward pass is faster by fc_small_kernel: a fit to both paths' times (us).  Chunks of 128 indices of the two jobs' blocks,

@@ -638,9 +638,9 @@ struct cct_fc_plan {
   int K4 = 0, O4 = 0;        // row pitches: multiples of four floats
   FcShape fwd, dgr, wgr, wgr_pair;  // wgr_pair: the weight gradient's, beside the data gradient in one launch
   int two = 0;               // blocks of the weight gradient there (0: two launches)
-  bool dot = false;          // forward pass by fc_dot_kernel
-  bool small_forward = false, small = false;  // forward, backward pass by fc_small_kernel, with these splits (where an operand is off a
-  int small_fwd = 1, small_dgr = 1;           // 16-byte boundary too, as far as there is room for their sums)
+  bool dot = false, dot_narrow = false;  // forward pass by fc_dot_kernel: rows on 16-byte boundaries, and off them
+  bool small_forward = false, small = false;  // else the forward pass, and the backward pass, by fc_small_kernel, with these splits (where an
+  int small_fwd = 1, small_dgr = 1;           // operand is off a 16-byte boundary too, as far as there is room for their sums)
   float* partial = nullptr;  // split partial sums of the forward pass and of the data gradient
   float *Xp = nullptr, *Wp = nullptr, *dYp = nullptr;  // copies with padded rows, where K or O is no multiple of four
   size_t bytes = 0;
@@ -718,8 +718,9 @@ int fc_reduce(cct_ctx* ctx, FcReduceParams R) {
   return CCT_OK;
 }
 
-// Forward pass of a small layer.  Where Y lies over an operand that other blocks still read, the sums go through `scratch`.
-int fc_dot(cct_ctx* ctx, const float* W, const float* X, int K, FcReduceParams post, float* scratch) {
+// Forward pass of a small layer; `vec`: all rows on 16-byte boundaries.  Where Y lies over an operand that other blocks still read, the
+// sums go through `scratch`.
+int fc_dot(cct_ctx* ctx, bool vec, const float* W, const float* X, int K, FcReduceParams post, float* scratch) {
   FcDotParams P{W, X, post.cols, post.rows, K, post};
   const bool clear = apart(post.out, (size_t)post.rows * post.cols, {{X, (size_t)post.rows * K}, {W, (size_t)post.cols * K}});
   if (!clear) {
@@ -730,7 +731,6 @@ int fc_dot(cct_ctx* ctx, const float* W, const float* X, int K, FcReduceParams p
     post.pitch = post.cols;
     post.splits = 1;
   }
-  const bool vec = K % 4 == 0 && fc_aligned({W, X});
   const int steps = (K + (vec ? 127 : 31)) / (vec ? 128 : 32);
   const bool wide = vec && P.N >= 8 && (long long)((P.N + 7) / 8) * ((P.M + kFdM - 1) / kFdM) >= kDotWideBlocks;
   const int nt = wide ? 8 : P.N > 2 ? 4 : P.N;
@@ -768,15 +768,17 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
     return CCT_ERR_UNSUPPORTED;
   }
   const bool few = use_small_fc(batch, in_features, out_features);
-  p->dot = (double)batch * in_features * out_features <= (few && in_features % 4 ? kDotNarrowProducts : kDotProducts);
-  p->small_forward = few && !p->dot;
+  p->small_forward = few;
   p->small = few || fc_small_faster(ctx->sm_count, batch, in_features, out_features);
   p->small_fwd = fc_small_splits(ctx->sm_count, out_features, batch, in_features);
   p->small_dgr = fc_small_splits(ctx->sm_count, in_features, batch, out_features);
+  const bool one_launch = few && p->small_fwd == 1;
+  p->dot = in_features % 4 == 0 && fc_dot_faster(batch, in_features, out_features, true, one_launch, false);
+  p->dot_narrow = fc_dot_faster(batch, in_features, out_features, false, one_launch, !few && in_features % 4);
   // One allocation: split sums, then the padded copies that are needed.
-  const int f_splits = p->dot ? 1 : p->small_forward ? p->small_fwd : p->fwd.P.splits, d_splits = p->small ? p->small_dgr : p->dgr.P.splits;
+  const int f_splits = few ? p->small_fwd : p->fwd.P.splits, d_splits = p->small ? p->small_dgr : p->dgr.P.splits;
   const size_t sums = std::max((size_t)f_splits * batch * p->O4, (size_t)d_splits * batch * p->K4);
-  const bool pad_k = !((p->dot || p->small_forward) && p->small) && p->K4 != p->K, pad_o = !p->small && p->O4 != p->O;
+  const bool pad_k = !((p->dot_narrow || few) && p->small) && p->K4 != p->K, pad_o = !p->small && p->O4 != p->O;
   auto room = [](size_t n) { return (n + 63) & ~(size_t)63; };
   const size_t x = pad_k ? room((size_t)batch * p->K4) : 0, w = pad_k ? room((size_t)out_features * p->K4) : 0,
                dy = pad_o ? room((size_t)batch * p->O4) : 0;
@@ -830,8 +832,9 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   const int B = plan->B, K = plan->K, O = plan->O, K4 = plan->K4, O4 = plan->O4;
   plan->timer.begin(0, ctx->stream);
-  if (plan->dot) {
-    const int rc = fc_dot(ctx, W, X, K, FcReduceParams{nullptr, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, 1, relu},
+  const bool wide = K % 4 == 0 && fc_aligned({X, W});
+  if (wide ? plan->dot : plan->dot_narrow) {
+    const int rc = fc_dot(ctx, wide, W, X, K, FcReduceParams{nullptr, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4, 1, relu},
                           plan->partial);
     plan->timer.end(0, ctx->stream);
     return rc;
