@@ -262,17 +262,22 @@ bool fc_dot_faster(int B, int K, int O, bool wide, bool one_launch, bool padded)
 }
 
 // Whether a backward pass is faster by fc_small_kernel: a fit to both paths' times (us).  Chunks of 128 indices of the two jobs' blocks,
-// 2.0 - 2.9 us for every one that an SM has, against 8.7 us for five launches of the tensor-core path, the stream of the weights and
-// their gradient, and wider tiles.  1000 -> 100, 256 images 18.1 -> 11.8 (estimate 16.8, 12.3); 512 -> 512, 64 images 11.1 -> 9.9
-// (11.1, 10.9), 128 images 13.6 -> 15.3 (13.1, 14.2); 4096 -> 1000, one image 15.6 -> 60 (15.7, 64).
-bool fc_small_faster(int sms, int B, int K, int O) {
+// 2.0 - 2.9 us for every one that an SM has (0.85 of that beyond 6 us, where blocks overlap), but no less than the chunks
+// of the longest block, which walks the whole batch for its tile of the weight gradient; against 8.7 us for five launches of the
+// tensor-core path (6.5: `pair`, both contractions in one), the stream of the weights and their gradient, and wider tiles, whose chain over
+// the batch is 0.67 us per block of 32.  Us there -> here (estimates): 1000 -> 100, 256 images 18.1 -> 11.8 (16.8, 11.7); 784 -> 128, 256
+// images 17.9 -> 10.8 (16.8, 10.2); 64 -> 512, 8192 images 173 -> 147 (187, 169).  Where the tensor cores stay: 800 -> 256, 128 images 8.9
+// (10.8 here; 10.8, 11.8); 200 -> 1024, 128 images 8.5 (13.4); 1000 -> 100, 640 images 23.7 (24.3; 25.0, 24.1); 784 -> 128, 4096 images 100 (103;
+// 99, 110); 4096 -> 1000, one image 15.6 (60).
+bool fc_small_faster(int sms, int B, int K, int O, bool pair) {
   auto up = [](int a, int b) { return (double)((a + b - 1) / b); };
   const int splits = fc_small_splits(sms, K, B, O);
   auto cost = [](double r) { return 2.0 + 0.9 * std::min(1.0, r / kFsChunk); };  // of a chunk with r indices
   const double k = up(K, kFsTile), w = k * up(O, kFsTile) * up(B, kFsChunk) * cost(B);
-  const double d = k * up(B, kFsTile) * splits * up((O + splits - 1) / splits, kFsChunk) * cost((double)O / splits);
-  const double small = 2.6 + (w + d) / sms + (splits > 1 ? 1.6 : 0.0);
-  return small < 8.7 + 1.7e-6 * K * O + 0.031 * B + (K % 4 || O % 4 ? 5.0 : 0.0);
+  const double d = k * up(B, kFsTile) * splits * up((O + splits - 1) / splits, kFsChunk) * cost((double)O / splits), even = (w + d) / sms;
+  const double small = 2.6 + std::max(std::min(even, 0.9 + 0.85 * even), 2.6 * up(B, kFsChunk)) + (splits > 1 ? 1.6 : 0.0);
+  const double tensor = (pair ? 6.5 : 8.7) + 1.7e-6 * K * O + (B <= 256 ? 0.031 * B : 2.4 + 0.0215 * B) + (K % 4 || O % 4 ? 5.0 : 0.0);
+  return small < 0.95 * tensor;
 }
 
 }  // namespace

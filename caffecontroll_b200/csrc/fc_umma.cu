@@ -769,7 +769,9 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   }
   const bool few = use_small_fc(batch, in_features, out_features);
   p->small_forward = few;
-  p->small = few || fc_small_faster(ctx->sm_count, batch, in_features, out_features);
+  p->two = fc_pair_blocks(ctx->sm_count, p->wgr_pair = fc_weight_pair_shape(in_features, out_features, batch), p->dgr);
+  p->small = few || fc_small_faster(ctx->sm_count, batch, in_features, out_features, p->two > 0);
+  if (p->small) p->two = 0;
   p->small_fwd = fc_small_splits(ctx->sm_count, out_features, batch, in_features);
   p->small_dgr = fc_small_splits(ctx->sm_count, in_features, batch, out_features);
   const bool one_launch = few && p->small_fwd == 1;
@@ -792,7 +794,6 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   float* at = p->partial + room(sums);
   if (pad_k) { p->Xp = at; p->Wp = at + x; }
   if (pad_o) p->dYp = at + x + w;
-  if (!p->small) p->two = fc_pair_blocks(ctx->sm_count, p->wgr_pair = fc_weight_pair_shape(in_features, out_features, batch), p->dgr);
   cudaError_t e = cudaFuncSetAttribute(fc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
   if (e == cudaSuccess && p->two) e = cudaFuncSetAttribute(fc_gemm_two_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024);
   if (e != cudaSuccess) {

@@ -860,6 +860,26 @@ def test_lines_of_the_dot_products(ctx, B, K, o, shift, launches):
     assert_close(Y.cpu().numpy(), (X.double() @ W.double().T + b.double()).float().cpu().numpy(), "Y")
 
 
+# Both sides of the line between the fp32 tiles and the tensor cores in backward passes of layers that are not small: a batch that makes one
+# block's chain long, blocks for every SM several times over.  Tolerance: parity.
+@pytest.mark.parametrize("B,K,o,launches", [(256, 784, 128, 1), (640, 1000, 100, 3), (4096, 784, 128, 3), (8192, 64, 512, 1), (1024, 256, 256, 1)])
+def test_backward_passes_of_long_batches(ctx, B, K, o, launches):
+    gen = torch.Generator(device="cuda").manual_seed(B + K + o)
+    make = lambda r, c: torch.randn(r, c, device="cuda", generator=gen)  # noqa: E731
+    X, W, dY = make(B, K), make(o, K), make(B, o)
+    dX, dW, db = torch.zeros_like(X), torch.zeros_like(W), torch.zeros(o, device="cuda")
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(plan)), "plan", ctx.h)
+    before = capi.kernel_launches()
+    capi.check(ctx.lib.cct_fc_backward(plan, q(X), q(W), q(dY), q(dX), q(dW), q(db), 0, None, 1.0), "backward", ctx.h)
+    assert capi.kernel_launches() - before == launches
+    ctx.sync()
+    ctx.lib.cct_fc_plan_destroy(plan)
+    for got, ref, name in ((dX, dY.double() @ W.double(), "dX"), (dW, dY.double().T @ X.double(), "dW"), (db, dY.double().sum(0), "db")):
+        assert_close(got.cpu().numpy(), ref.float().cpu().numpy(), name)
+
+
 # Both gradients of a small layer with stride 1 in one launch and, where dX lies over X, one after the other.  Tolerance: parity (fp32
 # products, sums of at most 24 x 25 and 36 864 of them).
 @pytest.mark.parametrize("shape", [(5, 1, 9, 7, 5, 1, 0, 1), (6, 2, 11, 24, 3, 1, 1, 2), (3, 8, 10, 5, 1, 1, 0, 1), (2, 3, 13, 9, 7, 1, 3, 1),
