@@ -88,6 +88,14 @@ inline bool apart(const void* out, size_t n, std::initializer_list<std::pair<con
   return true;
 }
 
+// Blocks of the first of two jobs, of `a` and `b` tiles, in one launch over `slots` resident blocks: one per tile where there are slots for all,
+// else the slots in proportion to the tiles; 0 where there are more than two tiles for each of them.
+inline int share_slots(long long slots, long long a, long long b) {
+  if (a + b > 2 * slots) return 0;
+  const long long mine = a + b <= slots ? a : slots * a / (a + b);
+  return (int)(mine < 1 ? 1 : mine);
+}
+
 #define CCT_CUDA(ctx, call)                                                                   \
   do {                                                                                        \
     cudaError_t e__ = (call);                                                                 \

@@ -609,8 +609,7 @@ FcShape fc_weight_shape(int sms, int K, int O, int B) {
   return best;
 }
 
-// The weight gradient's shape in half an SM, and its blocks there: where there are at most two tiles of both contractions for each of
-// the slots; in proportion to the tiles where there are not slots for all.
+// The weight gradient's shape in half an SM, beside the data gradient's.
 FcShape fc_weight_pair_shape(int K, int O, int B) {
   FcShape s;
   FcGemmParams& P = s.P;
@@ -624,11 +623,7 @@ FcShape fc_weight_pair_shape(int K, int O, int B) {
   s.pair = true;
   return s;
 }
-int fc_pair_blocks(int sms, FcShape& w, const FcShape& d) {
-  const long long tw = (long long)w.P.m_tiles * w.P.n_tiles, td = (long long)d.P.m_tiles * d.P.n_tiles * d.P.splits, slots = 2ll * sms;
-  if (!d.pair || tw + td > 2 * slots || !fc_fit_rings(w)) return 0;
-  return (int)(tw + td <= slots ? tw : std::max(1ll, slots * tw / (tw + td)));
-}
+long long fc_tiles(const FcShape& s) { return (long long)s.P.m_tiles * s.P.n_tiles * s.P.splits; }
 
 }  // namespace
 
@@ -637,7 +632,7 @@ struct cct_fc_plan {
   int B = 0, K = 0, O = 0, bias = 0;
   int K4 = 0, O4 = 0;        // row pitches: multiples of four floats
   FcShape fwd, dgr, wgr, wgr_pair;  // wgr_pair: the weight gradient's, beside the data gradient in one launch
-  int two = 0;               // blocks of the weight gradient there (0: two launches)
+  bool pair = false;         // both gradients in one launch, where the SMs that a call has can take their tiles
   bool dot = false, dot_narrow = false;  // forward pass by fc_dot_kernel: rows on 16-byte boundaries, and off them
   bool small_forward = false, small = false;  // else the forward pass, and the backward pass, by fc_small_kernel, with these splits (where an
   int small_fwd = 1, small_dgr = 1;           // operand is off a 16-byte boundary too, as far as there is room for their sums)
@@ -662,15 +657,17 @@ int fc_launch(cct_ctx* ctx, const FcShape& s, const FcMap& a, const FcMap& b, co
   return CCT_OK;
 }
 
-int fc_launch_two(cct_ctx* ctx, const cct_fc_plan* plan, float* direct, long long ld_direct) {
+// `blocks` of the grid are the weight gradient's.  Both jobs give up their share of SMs that a reduction in flight takes: with
+// eight fewer 6272 -> 256, 128 images, has 186 blocks for 196 tiles and 94 for 98, not 196 and 84.
+int fc_launch_two(cct_ctx* ctx, const cct_fc_plan* plan, int blocks, float* direct, long long ld_direct) {
   FcGemmParams W = plan->wgr_pair.P, D = plan->dgr.P;
   W.direct = direct; W.ld_direct = ld_direct;
   W.status = D.status = ctx->status_dev;
-  const int tiles = D.m_tiles * D.n_tiles * D.splits, blocks = std::min(tiles, std::max(1, 2 * ctx->launch_sms() - plan->two));
+  const int behind = (int)std::min(fc_tiles(plan->dgr), std::max(1ll, 2ll * ctx->launch_sms() - blocks));
   const FcJob w{W, plan->x_wgr.map, plan->dy_wgr.map, (direct ? plan->x_wgr : plan->out_wgr).map};
   const FcJob d{D, plan->w_dgr.map, plan->dy_dgr.map, plan->out_dgr.map};
-  launch_pdl(fc_gemm_two_kernel, dim3(plan->two + blocks), dim3(kFcThreads), std::max(plan->wgr_pair.smem, plan->dgr.smem), ctx->stream, w, d,
-             (unsigned)plan->two);
+  launch_pdl(fc_gemm_two_kernel, dim3(blocks + behind), dim3(kFcThreads), std::max(plan->wgr_pair.smem, plan->dgr.smem), ctx->stream, w, d,
+             (unsigned)blocks);
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
@@ -769,9 +766,9 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   }
   const bool few = use_small_fc(batch, in_features, out_features);
   p->small_forward = few;
-  p->two = fc_pair_blocks(ctx->sm_count, p->wgr_pair = fc_weight_pair_shape(in_features, out_features, batch), p->dgr);
-  p->small = few || fc_small_faster(ctx->sm_count, batch, in_features, out_features, p->two > 0);
-  if (p->small) p->two = 0;
+  p->wgr_pair = fc_weight_pair_shape(in_features, out_features, batch);
+  p->pair = p->dgr.pair && share_slots(2ll * ctx->sm_count, fc_tiles(p->wgr_pair), fc_tiles(p->dgr)) && fc_fit_rings(p->wgr_pair);
+  p->small = few || fc_small_faster(ctx->sm_count, batch, in_features, out_features, p->pair);
   p->small_fwd = fc_small_splits(ctx->sm_count, out_features, batch, in_features);
   p->small_dgr = fc_small_splits(ctx->sm_count, in_features, batch, out_features);
   const bool one_launch = few && p->small_fwd == 1;
@@ -795,7 +792,7 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   if (pad_k) { p->Xp = at; p->Wp = at + x; }
   if (pad_o) p->dYp = at + x + w;
   cudaError_t e = cudaFuncSetAttribute(fc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-  if (e == cudaSuccess && p->two) e = cudaFuncSetAttribute(fc_gemm_two_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024);
+  if (e == cudaSuccess && p->pair && !p->small) e = cudaFuncSetAttribute(fc_gemm_two_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024);
   if (e != cudaSuccess) {
     ctx->last_error = std::string("cudaFuncSetAttribute(fc_gemm_kernel): ") + cudaGetErrorString(e);
     cudaFree(p->partial);
@@ -891,7 +888,8 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   const bool d_sums = d_splits > 1 || !apart(dX, nx, {{dY, ny}, {W, nw}});  // as in the forward pass
   const bool clear = dX && !plan->timer.enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, nb}}) &&
                      apart(dW, nw, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}}) && apart(db, nb, {{W, nw}, {dY, ny}, {X, nx}, {in_drop_mask, nx}});
-  const bool together = clear && w_small && d_small, two = clear && plan->two && !w_small && !d_small;
+  const bool together = clear && w_small && d_small;
+  const int two = clear && plan->pair && !w_small && !d_small ? share_slots(2ll * ctx->launch_sms(), fc_tiles(plan->wgr_pair), fc_tiles(plan->dgr)) : 0;
   const bool direct = K4 != K || !fc_aligned({dW});  // dW: an output no tensor map describes
   if (w_small) {
     if (!together) rc = fc_small(ctx, W_job);
@@ -930,7 +928,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     rc = fc_operand_map(ctx, &plan->w_dgr, W, O, K, K4, 32, true);
     if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_dgr, dYm, B, O, O4, plan->dgr.P.n_pad, false);
     if (rc == CCT_OK) rc = fc_output_map(ctx, &plan->out_dgr, plan->partial, K, B, plan->dgr.P.splits, K4);
-    if (rc == CCT_OK) rc = two ? fc_launch_two(ctx, plan, direct ? dW : nullptr, K) : fc_launch(ctx, plan->dgr, plan->w_dgr, plan->dy_dgr, plan->out_dgr);
+    if (rc == CCT_OK) rc = two ? fc_launch_two(ctx, plan, two, direct ? dW : nullptr, K) : fc_launch(ctx, plan->dgr, plan->w_dgr, plan->dy_dgr, plan->out_dgr);
     if (rc == CCT_OK)
       rc = fc_reduce(ctx, FcReduceParams{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4,
                                          plan->dgr.P.splits, 0, 0, bias_sum});
