@@ -1769,7 +1769,7 @@ struct GatherProblem {
   size_t smem = 0;
   float* zero = nullptr;          // one 0.f, read by taps out of bounds
   bool inside = false;            // kInside
-  bool one = false;               // ONE: the tiles of the whole batch are short and have a slot each
+  bool one = false;               // ONE: the tiles of the whole batch are short and have a slot each, if no SMs are kept
   int run = 1, run_stride = 0;    // reduction order: 1 = (channel, tap); kRun = (channel / kRun, tap, channel % kRun)
   int splits = 1, split_k = 0;    // splits of the reduction and the length of one (a multiple of 32; k_pad without splits)
   float* partial = nullptr;       // split sums
@@ -1811,12 +1811,13 @@ template <int MODE, bool ONE = false>
 GatherKernel gather_kernel_of(const GatherProblem& gp) {
   return gp.sets == 2 ? gather_conv_kernel<2, MODE, ONE> : gather_conv_kernel<4, MODE, ONE>;
 }
-GatherKernel gather_kernel(const GatherProblem& gp, bool weight_grad) {
+GatherKernel gather_kernel(const GatherProblem& gp, bool weight_grad, bool one) {
   if (weight_grad) return gather_kernel_of<kWeightGrad>(gp);
-  if (gp.run == kRun) return gp.one ? gather_kernel_of<kByRun, true>(gp) : gather_kernel_of<kByRun>(gp);
+  if (gp.run == kRun) return one ? gather_kernel_of<kByRun, true>(gp) : gather_kernel_of<kByRun>(gp);
   if (gp.inside) return gather_kernel_of<kInside>(gp);
-  return gp.one ? gather_kernel_of<kByTap, true>(gp) : gather_kernel_of<kByTap>(gp);
+  return one ? gather_kernel_of<kByTap, true>(gp) : gather_kernel_of<kByTap>(gp);
 }
+int gather_smem_limit(const GatherProblem& gp) { return gp.sets == 2 ? 113 * 1024 : kSmemLimit; }
 // wgrad_ts_kernel's wide loads: see there.  Below eight taps a window row has fewer than three blocks' worth.
 bool ts_wide(const ConvGeom& G) {
   return G.s % 4 == 0 && G.p == 0 && G.k >= 8 && G.k <= kTsWideTaps && G.Dg * G.k <= kTsWideRows * ts_tap_warps(true);
@@ -2224,7 +2225,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
   }
   // The kernels that this plan launches, and no others: each is one to load at its first use.
   for (const GatherProblem* gp : {&p->fwd, &p->dgr, &p->wgp})
-    if (rc == CCT_OK && gp->w) rc = set_smem(ctx, gather_kernel(*gp, gp == &p->wgp), gp->sets == 2 ? 113 * 1024 : kSmemLimit);
+    if (rc == CCT_OK && gp->w) rc = set_smem(ctx, gather_kernel(*gp, gp == &p->wgp, gp->one), gather_smem_limit(*gp));
   if (rc == CCT_OK && !p->w_small && !p->wg_gather) rc = set_smem(ctx, short_wgrad_kernel(p), kSmemLimit);
   if (rc != CCT_OK) {
     umma_plan_destroy(ctx, p);
@@ -2304,10 +2305,15 @@ SmallConv small_dgrad(const ConvGeom& G, const float* dY, const float* W, float*
   return SmallConv{dY, W, nullptr, dX, batch, G.m, G.n, G.k - 1 - G.p, G.og, G.Dg, G.g, 1, 0};
 }
 
-// A CTA per tile, or a persistent grid: one CTA per SM (4 producer sets) or two (2 sets); then the reduction over the splits, if any.
+// A CTA per tile where each has a slot (ONE), or a persistent grid: one CTA per SM (4 producer sets) or two (2 sets); then the reduction over
+// the splits, if any.  A plan whose tiles all had slots takes the persistent kernel while a reduction in flight keeps some of them; its
+// attribute is set then, since a plan made beside a communicator never comes here.
 void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp, bool weight_grad = false) {
-  const int grid = gp.one ? P.total_tiles : std::min(P.total_tiles, (gp.sets == 2 ? 2 : 1) * ctx->launch_sms());
-  launch_pdl(gather_kernel(gp, weight_grad), dim3(grid), dim3(gather_threads(gp.sets)), gp.smem, ctx->stream, P, gp.map);
+  const int slots = (gp.sets == 2 ? 2 : 1) * ctx->launch_sms();
+  const bool one = gp.one && P.total_tiles <= slots;
+  const GatherKernel kernel = gather_kernel(gp, weight_grad, one);
+  if (gp.one && !one) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gather_smem_limit(gp));  // (or the launch fails)
+  launch_pdl(kernel, dim3(std::min(P.total_tiles, slots)), dim3(gather_threads(gp.sets)), gp.smem, ctx->stream, P, gp.map);
   if (P.splits > 1) {
     const int vgroups = P.total_tiles / (P.n_pix_tiles * P.splits), cols = P.n_pix_tiles * vgroups * P.n > 32 * ctx->sm_count ? 8 : 1;
     const int col_tiles = (P.n + cols - 1) / cols;

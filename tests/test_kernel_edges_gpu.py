@@ -1,6 +1,9 @@
 """The branches that a layer's sizes choose between, each at the sizes where it can go wrong: edges of tiles, remainders, the
 smallest and largest of its range."""
 import ctypes as C
+import os
+import re
+import subprocess
 
 import numpy as np
 import pytest
@@ -942,3 +945,103 @@ def test_two_contractions_in_one_launch(ctx, B, K, o, bias):
     for got in ((dX, dW, db), over):
         for a, r, name in zip(got, refs, ("dX", "dW", "db")):
             assert_close(a.cpu().numpy(), r.float().cpu().numpy(), name)
+
+
+@pytest.fixture(scope="session")
+def keep_sms(ctx, tmp_path_factory):
+    """keep_sms(n): launches leave n SMs free from now on, as while a gradient reduction is in flight."""
+    at = tmp_path_factory.mktemp("keep")
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "caffecontroll_b200", "csrc")
+    (at / "keep.cu").write_text('#include "%s/cct_internal.h"\nextern "C" void keep(cct_ctx* ctx, int sms) { ctx->reserved_sms = sms; }\n' % csrc)
+    subprocess.run([os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-gencode",
+                    "arch=compute_100a,code=sm_100a", "-o", str(at / "keep.so"), str(at / "keep.cu")], check=True)
+    lib = C.CDLL(str(at / "keep.so"))
+    lib.keep.argtypes = [C.c_void_p, C.c_int]
+    return lambda n: lib.keep(ctx.h, n)
+
+
+def kernels_of(ctx, call):
+    """Names of the library's kernels that a call launches, template arguments included."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        ctx.sync()
+    names = [re.match(r"(?:void )?(\w+(?:<[^(]*>)?)\(", e.name.replace("(anonymous namespace)::", "")) for e in prof.events()]
+    return [n.group(1) for n in names if n]
+
+
+# gather_conv_kernel<SETS, MODE, ONE> with a CTA per tile (ONE) by tap and by run of channels, two and four producer sets, with and without
+# splits, strides and groups; the last slot and one tile past it; 32 k-blocks and 33; wgrad_kernel<M-tiles, ...> with one M-tile per CTA where more
+# would fit, and with two.  Persistent (all SMs but one kept), the same bits; tolerance against float64: parity.
+@pytest.mark.parametrize("shape,forward,weight,data", [
+    ((37, 50, 21, 75, 3, 2, 1, 1), "<2, 0, true>", "<1, 5>", "<2, 0, true>"), ((1, 256, 13, 384, 3, 1, 1, 1), "<2, 1, true>", None, "<2, 1, true>"),
+    ((1, 96, 27, 256, 5, 1, 2, 2), "<2, 1, true>", None, "<2, 1, true>"), ((9, 17, 33, 65, 3, 1, 1, 1), "<2, 0, true>", "<2, 5>", "<2, 0, true>"),
+    ((74, 32, 16, 130, 3, 1, 1, 1), "<4, 1, true>", "<2, 9>", "<2, 0, false>"), ((75, 32, 16, 130, 3, 1, 1, 1), "<2, 1, false>", "<2, 9>", "<2, 0, false>"),
+    ((74, 31, 16, 130, 3, 1, 1, 1), "<4, 0, true>", "<2, 9>", "<2, 0, false>"), ((4, 100, 29, 300, 5, 1, 1, 1), "<4, 0, true>", None, "<4, 0, false>"),
+    ((38, 96, 10, 300, 5, 1, 1, 1), "<4, 1, true>", None, "<4, 0, false>"), ((52, 33, 31, 40, 3, 2, 1, 1), "<2, 0, true>", None, "<4, 1, true>"),
+    ((58, 64, 7, 17, 1, 2, 0, 1), "<2, 1, true>", "<1, 2>", "<2, 0, true>"), ((2, 33, 17, 300, 3, 1, 1, 1), "<2, 0, true>", "<1, 10>", "<2, 0, true>"),
+    ((37, 1024, 16, 130, 1, 1, 0, 1), "<2, 1, true>", None, "<2, 0, false>"), ((37, 1056, 16, 130, 1, 1, 0, 1), "<2, 1, false>", None, "<4, 0, false>"),
+])
+def test_a_cta_per_tile(ctx, keep_sms, shape, forward, weight, data):
+    B, D, n, o, k, s, p, g = shape
+    m = (n + 2 * p - k) // s + 1
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    X, W, b, dY = (torch.randn(sh, device="cuda", generator=gen) for sh in ((B, D, n, n), (o, D // g, k, k), (o,), (B, o, m, m)))
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    desc = capi.ConvDesc(B, D, n, o, k, s, p, g, 1, TENSOR)
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_conv_plan_create(ctx.h, C.byref(desc), C.byref(plan)), "plan", ctx.h)
+
+    def run():
+        Y, dX, dW, db = (torch.full_like(t, 7) for t in (dY, X, W, b))
+        torch.cuda.synchronize()
+        there = kernels_of(ctx, lambda: capi.check(ctx.lib.cct_conv_forward(plan, q(X), q(W), q(b), q(Y), 1), "forward", ctx.h))
+        back = kernels_of(ctx, lambda: capi.check(ctx.lib.cct_conv_backward(plan, q(X), q(W), q(dY), q(dX), q(dW), q(db)), "backward", ctx.h))
+        last = [name for name in back if name.startswith("gather_conv_kernel")][-1]
+        return (Y, dX, dW, db), ["".join(x for x in there if x.startswith("gather_conv")), "".join(x for x in back if x.startswith("wgrad_kernel")), last]
+
+    got, names = run()
+    assert names[0] == "gather_conv_kernel" + forward and names[2] == "gather_conv_kernel" + data
+    assert weight is None or names[1] == "wgrad_kernel" + weight
+    keep_sms(torch.cuda.get_device_properties(0).multi_processor_count - 1)
+    try:
+        kept, kept_names = run()
+    finally:
+        keep_sms(0)
+    ctx.lib.cct_conv_plan_destroy(plan)
+    assert "true" not in kept_names[0] + kept_names[2]
+    Xd, Wd, bd = (t.double().requires_grad_() for t in (X, W, b))
+    out = torch.nn.functional.conv2d(Xd, Wd, bd, s, p, 1, g)
+    out.backward(dY.double())
+    for a, c, r, name in zip(got, kept, (out.detach().clamp(min=0), Xd.grad, Wd.grad, bd.grad), ("Y", "dX", "dW", "db")):
+        assert torch.equal(a, c), name
+        assert_close(a.cpu().numpy(), r.float().cpu().numpy(), name)
+
+
+def test_two_contractions_beside_a_reduction(ctx, keep_sms):
+    """Both contractions of an inner product's backward pass with fewer SMs: in one launch where there are at most two tiles a slot, else in two;
+    the same bits."""
+    B, K, o = 64, 800, 500
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    X, W, dY = (torch.randn(sh, device="cuda", generator=gen) for sh in ((B, K), (o, K), (B, o)))
+    plan, q, results = C.c_void_p(), lambda t: t.data_ptr(), []
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(plan)), "plan", ctx.h)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for kept, launches in ((0, 2), (8, 2), (sms - 40, 2), (sms - 4, 3), (sms - 1, 3)):
+        dX, dW, db = torch.zeros_like(X), torch.zeros_like(W), torch.zeros(o, device="cuda")
+        torch.cuda.synchronize()
+        before = capi.kernel_launches()
+        keep_sms(kept)
+        try:
+            capi.check(ctx.lib.cct_fc_backward(plan, q(X), q(W), q(dY), q(dX), q(dW), q(db), 0, None, 1.0), "backward", ctx.h)
+        finally:
+            keep_sms(0)
+        ctx.sync()
+        assert capi.kernel_launches() - before == launches, kept
+        results.append((dX, dW, db))
+    ctx.lib.cct_fc_plan_destroy(plan)
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
+    for a, r, name in zip(results[0], (dY.double() @ W.double(), dY.double().T @ X.double(), dY.double().sum(0)), ("dX", "dW", "db")):
+        assert_close(a.cpu().numpy(), r.float().cpu().numpy(), name)
