@@ -4,7 +4,7 @@
 // their own, tensor-memory allocation, the hand-overs between its roles) and half a microsecond for every further k-block
 // of a tile; a layer of a few ten million multiply-adds - LeNet's first layers, a narrow data gradient - is all latency
 // there.  These kernels do such a layer in one launch of short blocks: exact fp32 products, fp32 accumulation in a fixed
-// order, no packed operand.  use_small_gather() / use_small_wgrad() draw the line.
+// order, no packed operand.  use_small_conv() / use_small_wgrad() draw the line.
 #pragma once
 
 namespace {
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(JOB::kThreads, JOB::blocks(CT)) small_conv_ker
   int bx = 0, by = 0;
   if constexpr (!ALONE) {
     if (J.weight_gradient()) return;
-    by = blockIdx.x / J.grid_x, bx = blockIdx.x - by * J.grid_x;
+    bx = (int)blockIdx.x - J.conv_at; by = bx / J.grid_x, bx -= by * J.grid_x;
   }
   const SmallConv& P = J;
   constexpr int JR = small_rows(K, S, CT), R = (JR - 1) * S + K;
@@ -284,23 +284,27 @@ __global__ void __launch_bounds__(kSwThreads) small_wgrad_kernel(const __grid_co
   small_wgrad_block(J, small_smem, blockIdx.x % J.tiles, blockIdx.x / J.tiles);
 }
 
-// Both gradients of a layer with stride 1 in one launch: neither reads what the other writes.  Blocks [0, conv_blocks) are the data
-// gradient's.  LeNet conv1 at batch 64, forward and backward: 22.2 -> 19.3 us, three launches instead of four (three blocks per SM for
-// one-channel data gradients; with two 19.6, with four, and spills, 20.4).  Up to kSmallRounds rounds of blocks: 64 images 20 x 20, 3 -> 16
-// channels 5 x 5 9.4 + 7.9 -> 13.4 us (1.3 rounds), 16 images 30 x 30, 6 -> 12 channels 3 x 3 6.3 + 4.8 -> 9.9 (1.6); 21 images 18 x 18, 42
-// -> 24 channels 1 x 1 4.5 + 5.4 -> 11.7 (2.6).  Not where the data gradient alone has more warps per block than go here: 3 images 9 x 9,
-// 3 -> 259 channels 3 x 3 4.5 + 17.3 -> 23.8.
+// Both gradients of a layer with stride 1 in one launch: neither reads what the other writes.  LeNet conv1 at batch 64, forward and
+// backward: 22.2 -> 19.3 us, three launches instead of four (three blocks per SM for one-channel data gradients; with two 19.6, with
+// four 20.4).  The weight gradient's blocks go first, since a few of them behind the others are a round of their own (44 images 18 x 18, 7 -> 16
+// channels 1 x 1: two launches 9.1 us, the data gradient first 10.5, the weight gradient first 8.1; 32 images 24 x 24, 4 -> 12 channels 3 x 3
+// 12.4, 12.8 and 11.0) - unless the data gradient's are the longer ones: three and more channels a warp against one chunk of pixels, in one
+// round or with one channel (LeNet conv1's backward pass 14.9 us, the weight gradient first 15.7; 8 images 18 x 18, 7 -> 23 channels 5 x 5 10.2 and 11.6;
+// in more rounds 46 x 46, 44 -> 28 channels 3 x 3 12.9 and 11.2).  Up to kSmallRounds rounds of blocks: 21 images 18 x 18, 42 -> 24 channels 1 x 1 4.5
+// + 5.4 -> 11.7 us (2.6 rounds).  Not where the data gradient alone has more warps per block than go here: 3 images 9 x 9, 3 -> 259
+// channels 3 x 3 4.5 + 17.3 -> 23.8.
 constexpr int kSmallRounds = 2;
 struct SmallBackward : SmallConv {  // the base: the data gradient
   SmallWgrad w;
-  int grid_x, conv_blocks;  // of the data gradient
+  int grid_x, conv_at;         // of the data gradient: its grid, and its first block
+  int wgrad_at, wgrad_blocks;
   static constexpr int kThreads = kSwThreads;
   __host__ __device__ static constexpr int blocks(int ct) { return ct == 1 ? 3 : 2; }  // per SM
   __device__ bool weight_gradient() const {
     extern __shared__ __align__(16) float small_smem[];
-    const int block = (int)blockIdx.x - conv_blocks;
-    if (block >= 0) small_wgrad_block(w, small_smem, block % w.tiles, block / w.tiles);
-    return block >= 0;
+    const unsigned block = blockIdx.x - (unsigned)wgrad_at;
+    if (block < (unsigned)wgrad_blocks) small_wgrad_block(w, small_smem, (int)block % w.tiles, (int)block / w.tiles);
+    return block < (unsigned)wgrad_blocks;
   }
 };
 typedef void (*SmallBackwardKernel)(const SmallBackward);

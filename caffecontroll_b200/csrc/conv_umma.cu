@@ -2463,8 +2463,10 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       const int blocks = J.tiles * p->w_splits;
       if (with) {
         const SmallConvShape g = shape_small_conv(ctx, *with, G.k, 1, p->dgr.small_ct, kSwWarps);
-        launch_pdl(small_backward_pick(G.k, g.ct), dim3(blocks + g.x * g.y), dim3(kSwThreads), std::max(kSwSmem, g.smem), ctx->stream,
-                   SmallBackward{*with, J, g.x, g.x * g.y});
+        const int others = g.x * g.y;
+        const bool conv_first = with->ci > 2 * kSwWarps && p->ws_pix == kSwPix && (g.ct == 1 || blocks + others <= SmallBackward::blocks(g.ct) * ctx->sm_count);
+        launch_pdl(small_backward_pick(G.k, g.ct), dim3(blocks + others), dim3(kSwThreads), std::max(kSwSmem, g.smem), ctx->stream,
+                   SmallBackward{*with, J, g.x, conv_first ? 0 : blocks, conv_first ? others : 0, blocks});
       } else {
         launch_pdl(small_wgrad_kernel, dim3(blocks), dim3(kSwThreads), kSwSmem, ctx->stream, J);
       }
