@@ -35,18 +35,23 @@ struct SmallConv {
   __host__ __device__ static constexpr int blocks(int) { return 0; }  // per SM at the least: not said (with 1 the compiler takes twice the registers)
 };
 
-// Rows per lane (row and column masks share 32 bits).  With one channel there are registers for eight, which load 3 values of a 5 x 5 window
-// for 2 outputs where four load 2 for 1 (LeNet conv1, both passes, with four: 20.0 us, not 19.3); a 3 x 3 window gains no such thing
-// (44 images 32 x 32, two groups: 6.0 us with four, 6.5 with eight).
-__host__ __device__ constexpr int small_rows(int K, int S, int CT) { return K >= 11 ? 2 : CT == 1 && S == 1 && K == 5 ? 8 : 4; }
+// Rows per lane (row and column masks share 32 bits).  One channel leaves registers for kSmallTall, with which 3 values of a 5 x 5 window are
+// loaded for 2 outputs where four load 2 for 1 (LeNet conv1, both passes, with four: 20.0 us, not 19.3; a 3 x 3 window gains no such
+// thing: 44 images 32 x 32, two groups 6.0 us with four, 6.5 with eight).  Taken where four rows are more than one lot of 32 lanes for every
+// SM and eight leave as many, or hardly a row behind the plane's last one: backward passes, four rows and eight: one image 28 x 28, 20
+// channels 6.5 us and 7.9; 128 images 12 x 12, 32 channels 10.8 and 12.1 (144 lots of four); 16 images 40 x 40, 32 channels 17.5 and 15.3 (200,
+// 100 of eight); 64 images 32 x 32, 32 channels 25.4 and 23.5 (512, 256); 64 images 28 x 28, 32 channels, four rows too many 19.9 and 20.4, though not
+// beside a weight gradient (20 channels 17.4 and 14.7).
+__host__ __device__ constexpr int small_rows(int K) { return K >= 11 ? 2 : 4; }
+constexpr int kSmallTall = 8;
 // Shared memory: the weights, afterwards the warps' sums.
-inline size_t small_conv_smem(int K, int s, int ct, int ci, int sharing_warps) {
-  return std::max((size_t)ci * K * K * ct, (size_t)sharing_warps * small_rows(K, s, ct) * ct * 32) * sizeof(float);
+inline size_t small_conv_smem(int K, int rows, int ct, int ci, int sharing_warps) {
+  return std::max((size_t)ci * K * K * ct, (size_t)sharing_warps * rows * ct * 32) * sizeof(float);
 }
 
 // JOB: SmallConv, the pass alone, whose grid's x is positions and y channel tiles; or SmallBackward below, both gradients of a layer.  The
 // pass's text stands in the kernel: as a function called from two kernels 6 images 16 x 16, 3 -> 8 channels 5 x 5 by 2 took 6.5 us, not 6.0.
-template <int K, int S, int CT, typename JOB>
+template <int K, int S, int CT, typename JOB, int JR = small_rows(K)>
 __global__ void __launch_bounds__(JOB::kThreads, JOB::blocks(CT)) small_conv_kernel(const __grid_constant__ JOB J) {
   pdl_wait();
   constexpr bool ALONE = std::is_same<JOB, SmallConv>::value;
@@ -56,7 +61,7 @@ __global__ void __launch_bounds__(JOB::kThreads, JOB::blocks(CT)) small_conv_ker
     bx = (int)blockIdx.x - J.conv_at; by = bx / J.grid_x, bx -= by * J.grid_x;
   }
   const SmallConv& P = J;
-  constexpr int JR = small_rows(K, S, CT), R = (JR - 1) * S + K;
+  constexpr int R = (JR - 1) * S + K;
   static_assert(R + K <= 32, "row and column bits share a word");
   extern __shared__ __align__(16) float small_smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -176,7 +181,8 @@ SmallConvKernel small_conv_pick_ks(int k, int s) {
   }
   return nullptr;
 }
-SmallConvKernel small_conv_pick(int k, int s, int ct) {
+SmallConvKernel small_conv_pick(int k, int s, int ct, int rows = 0) {
+  if (rows == kSmallTall) return small_conv_kernel<5, 1, 1, SmallConv, kSmallTall>;
   return ct == 8 ? small_conv_pick_ks<8>(k, s) : ct == 4 ? small_conv_pick_ks<4>(k, s) : small_conv_pick_ks<1>(k, s);
 }
 // Output channels per block: the fewest idle ones, eight where four would leave as many idle.
@@ -285,15 +291,17 @@ __global__ void __launch_bounds__(kSwThreads) small_wgrad_kernel(const __grid_co
 }
 
 // Both gradients of a layer with stride 1 in one launch: neither reads what the other writes.  LeNet conv1 at batch 64, forward and
-// backward: 22.2 -> 19.3 us, three launches instead of four (three blocks per SM for one-channel data gradients; with two 19.6, with
-// four 20.4).  The weight gradient's blocks go first, since a few of them behind the others are a round of their own (44 images 18 x 18, 7 -> 16
+// backward: 22.2 -> 19.3 us, three launches instead of four (three blocks per SM for one-channel data gradients, at 80 registers and
+// 136 bytes of spills in tall lanes; with two blocks 19.6, with four 20.4).  The weight gradient's blocks go first, since a few of them behind the others are a round of their own (44 images 18 x 18, 7 -> 16
 // channels 1 x 1: two launches 9.1 us, the data gradient first 10.5, the weight gradient first 8.1; 32 images 24 x 24, 4 -> 12 channels 3 x 3
 // 12.4, 12.8 and 11.0) - unless the data gradient's are the longer ones: three and more channels a warp against one chunk of pixels, in one
 // round or with one channel (LeNet conv1's backward pass 14.9 us, the weight gradient first 15.7; 8 images 18 x 18, 7 -> 23 channels 5 x 5 10.2 and 11.6;
-// in more rounds 46 x 46, 44 -> 28 channels 3 x 3 12.9 and 11.2).  Up to kSmallRounds rounds of blocks: 21 images 18 x 18, 42 -> 24 channels 1 x 1 4.5
+// in more rounds 46 x 46, 44 -> 28 channels 3 x 3 12.9 and 11.2), or tall lanes in more than a round (64 images 32 x 32, 12 channels, padding 2 16.5
+// and 17.9).  Up to kSmallRounds rounds of blocks: 21 images 18 x 18, 42 -> 24 channels 1 x 1 4.5
 // + 5.4 -> 11.7 us (2.6 rounds).  Not where the data gradient alone has more warps per block than go here: 3 images 9 x 9, 3 -> 259
-// channels 3 x 3 4.5 + 17.3 -> 23.8.
-constexpr int kSmallRounds = 2;
+// channels 3 x 3 4.5 + 17.3 -> 23.8.  Nor tall lanes with fewer than kSmallTallChannels in more than a round, which the pass alone shares
+// between four warps, not eight (64 images 32 x 32, eight channels, padding 2: 16.1 -> 17.1).
+constexpr int kSmallRounds = 2, kSmallTallChannels = 12;
 struct SmallBackward : SmallConv {  // the base: the data gradient
   SmallWgrad w;
   int grid_x, conv_at;         // of the data gradient: its grid, and its first block
@@ -315,7 +323,8 @@ SmallBackwardKernel small_backward_pick_k(int k) {
          : k == 5 ? small_conv_kernel<5, 1, CT, SmallBackward>
                   : small_conv_kernel<7, 1, CT, SmallBackward>;
 }
-SmallBackwardKernel small_backward_pick(int k, int ct) {
+SmallBackwardKernel small_backward_pick(int k, int ct, int rows) {
+  if (rows == kSmallTall) return small_conv_kernel<5, 1, 1, SmallBackward, kSmallTall>;
   return ct == 8 ? small_backward_pick_k<8>(k) : ct == 4 ? small_backward_pick_k<4>(k) : small_backward_pick_k<1>(k);
 }
 

@@ -1922,7 +1922,7 @@ constexpr double kSmallConvFlops = 1.5e8, kSmallWideFlops = 8e7, kSmallWgradFlop
 // Channels per block of small_conv_kernel for one pass (0: the tensor-core kernel).
 int use_small_conv(int k, int s, long long out_pixels, int groups, int ci, int co) {
   const int ct = small_conv_ct(co);
-  if (!small_conv_pick(k, s, ct) || small_conv_smem(k, s, ct, ci, 0) > 48 * 1024) return 0;
+  if (!small_conv_pick(k, s, ct) || small_conv_smem(k, small_rows(k), ct, ci, 0) > 48 * 1024) return 0;
   if ((long long)groups * ((co + 3) / 4) > 65535) return 0;  // channel tiles (of four at least) are a grid's y
   const double flops = 2.0 * out_pixels * groups * ((co + ct - 1) / ct * ct) * ci * k * k;
   return flops <= (k >= 7 ? kSmallWideFlops : kSmallConvFlops) ? ct : 0;
@@ -2272,33 +2272,35 @@ PackDgrad pack_dgrad_job(const UmmaPlan* p, const float* W) {
   return J;
 }
 
-// Grid of a pass by small_conv_kernel, and its shared memory; `warps` > 0: that many per block.
+// Grid of a pass by small_conv_kernel, and its shared memory; `block_warps` > 0: that many per block, beside a weight gradient.
 struct SmallConvShape {
-  int ct, warps, x, y;
+  int ct, rows, warps, x, y;
   size_t smem;
 };
-SmallConvShape shape_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct, int warps = 0) {
-  const int jr = small_rows(k, s, ct);  // (the same for four and eight channels)
-  P.row_groups = (P.n_out + jr - 1) / jr;
+SmallConvShape shape_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct, int block_warps = 0) {
+  // Tall lanes: see small_rows().
+  auto lots_of = [&](int rows) { return ((long long)P.batch * ((P.n_out + rows - 1) / rows) * P.n_out + 31) / 32; };
+  const long long few = lots_of(small_rows(k)), tall = lots_of(kSmallTall), sms = ctx->launch_sms();
+  const bool eight = k == 5 && s == 1 && ct == 1 && few > sms && (tall < sms || 40 * tall <= (block_warps ? 23 : 22) * few);
+  const int rows = eight ? kSmallTall : small_rows(k);
+  P.row_groups = (P.n_out + rows - 1) / rows;
   P.positions = P.batch * P.row_groups * P.n_out;
   // Narrower channel tiles and more warps on the input channels until the SMs have about sixteen warps each.
-  const long long lots = (P.positions + 31) / 32, want = 16ll * ctx->launch_sms();
+  const long long lots = (P.positions + 31) / 32, want = 16ll * sms;
   if (ct == 8 && lots * P.groups * ((P.co + 7) / 8) * std::min(16, std::max(1, P.ci / 2)) < want) ct = 4;
   P.col_tiles = (P.co + ct - 1) / ct;
   P.share = P.ci >= 4 && lots * P.groups * P.col_tiles < want;
-  if (!warps) {
-    warps = 4;
-    while (P.share && warps < 16 && P.ci >= 4 * warps && lots * P.groups * P.col_tiles * warps < want &&
-           small_conv_smem(k, s, ct, P.ci, 2 * warps) <= 48 * 1024)
-      warps *= 2;
-  }
+  int warps = block_warps ? block_warps : 4;
+  while (!block_warps && P.share && warps < 16 && P.ci >= 4 * warps && lots * P.groups * P.col_tiles * warps < want &&
+         small_conv_smem(k, rows, ct, P.ci, 2 * warps) <= 48 * 1024)
+    warps *= 2;
   const int per_block = P.share ? 32 : 32 * warps;
-  return SmallConvShape{ct, warps, (P.positions + per_block - 1) / per_block, P.groups * P.col_tiles,
-                        small_conv_smem(k, s, ct, P.ci, P.share ? warps : 0)};
+  return SmallConvShape{ct, rows, warps, (P.positions + per_block - 1) / per_block, P.groups * P.col_tiles,
+                        small_conv_smem(k, rows, ct, P.ci, P.share ? warps : 0)};
 }
 void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct) {
   const SmallConvShape g = shape_small_conv(ctx, P, k, s, ct);
-  launch_pdl(small_conv_pick(k, s, g.ct), dim3(g.x, g.y), dim3(32 * g.warps), g.smem, ctx->stream, P);
+  launch_pdl(small_conv_pick(k, s, g.ct, g.rows), dim3(g.x, g.y), dim3(32 * g.warps), g.smem, ctx->stream, P);
 }
 // The data gradient of a stride-1 layer as a convolution of dY.
 SmallConv small_dgrad(const ConvGeom& G, const float* dY, const float* W, float* dX, int batch) {
@@ -2391,7 +2393,8 @@ int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W
     const int warps = shape_small_conv(ctx, d, G.k, 1, p->dgr.small_ct).warps;
     const SmallConvShape g = shape_small_conv(ctx, d, G.k, 1, p->dgr.small_ct, kSwWarps);
     const long long blocks = (long long)p->ws_rows * p->ws_cols * G.g * p->wt_tiles * p->w_splits + (long long)g.x * g.y;
-    if (warps <= kSwWarps && blocks <= (long long)kSmallRounds * SmallBackward::blocks(g.ct) * ctx->sm_count)
+    const long long slots = (long long)SmallBackward::blocks(g.ct) * ctx->sm_count;
+    if (warps <= kSwWarps && blocks <= kSmallRounds * slots && (g.rows != kSmallTall || G.og >= kSmallTallChannels || blocks <= slots))
       return weight_gradient(ctx, p, X, dY, dW, db, t, nullptr, &d);
   }
   int rc = umma_conv_wgrad(ctx, p, X, dY, dW, db, t, dX ? W : nullptr);
@@ -2464,8 +2467,9 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       if (with) {
         const SmallConvShape g = shape_small_conv(ctx, *with, G.k, 1, p->dgr.small_ct, kSwWarps);
         const int others = g.x * g.y;
-        const bool conv_first = with->ci > 2 * kSwWarps && p->ws_pix == kSwPix && (g.ct == 1 || blocks + others <= SmallBackward::blocks(g.ct) * ctx->sm_count);
-        launch_pdl(small_backward_pick(G.k, g.ct), dim3(blocks + others), dim3(kSwThreads), std::max(kSwSmem, g.smem), ctx->stream,
+        const bool one_round = blocks + others <= SmallBackward::blocks(g.ct) * ctx->sm_count;
+        const bool conv_first = with->ci > 2 * kSwWarps ? p->ws_pix == kSwPix && (g.ct == 1 || one_round) : g.rows == kSmallTall && !one_round;
+        launch_pdl(small_backward_pick(G.k, g.ct, g.rows), dim3(blocks + others), dim3(kSwThreads), std::max(kSwSmem, g.smem), ctx->stream,
                    SmallBackward{*with, J, g.x, conv_first ? 0 : blocks, conv_first ? others : 0, blocks});
       } else {
         launch_pdl(small_wgrad_kernel, dim3(blocks), dim3(kSwThreads), kSwSmem, ctx->stream, J);

@@ -1045,3 +1045,29 @@ def test_two_contractions_beside_a_reduction(ctx, keep_sms):
         assert all(torch.equal(a, b) for a, b in zip(results[0], other))
     for a, r, name in zip(results[0], (dY.double() @ W.double(), dY.double().T @ X.double(), dY.double().sum(0)), ("dX", "dW", "db")):
         assert_close(a.cpu().numpy(), r.float().cpu().numpy(), name)
+
+
+# One-channel data gradients of 5 x 5 windows: four and eight rows per lane on both sides of one lot of four for every SM, planes that end inside
+# a lane's rows, alone and beside the weight gradient.  Tolerance: parity.
+@pytest.mark.parametrize("shape,rows,launches", [
+    ((1, 1, 28, 20, 5, 1, 0, 1), 4, 2), ((64, 1, 28, 20, 5, 1, 0, 1), 8, 2), ((128, 1, 12, 32, 5, 1, 0, 1), 4, 3), ((16, 1, 40, 32, 5, 1, 0, 1), 8, 3),
+    ((64, 1, 28, 32, 5, 1, 0, 1), 8, 2), ((128, 1, 28, 20, 5, 1, 2, 1), 4, 3), ((64, 1, 32, 32, 5, 1, 2, 1), 8, 3), ((118, 1, 6, 42, 5, 1, 2, 1), 4, 3), ((64, 1, 32, 8, 5, 1, 2, 1), 8, 3),
+])
+def test_rows_of_one_channel(ctx, shape, rows, launches):
+    B, D, n, o, k, s, p, g = shape
+    m = n + 2 * p - k + 1
+    gen = torch.Generator(device="cuda").manual_seed(n + o)
+    X, W, dY = (torch.randn(sh, device="cuda", generator=gen) for sh in ((B, D, n, n), (o, D, k, k), (B, o, m, m)))
+    dX, dW, db = torch.full_like(X, 7), torch.zeros_like(W), torch.zeros(o, device="cuda")
+    plan, q = C.c_void_p(), lambda t: t.data_ptr()
+    desc = capi.ConvDesc(B, D, n, o, k, s, p, g, 1, capi.ALGO_AUTO)
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_conv_plan_create(ctx.h, C.byref(desc), C.byref(plan)), "plan", ctx.h)
+    names = kernels_of(ctx, lambda: capi.check(ctx.lib.cct_conv_backward(plan, q(X), q(W), q(dY), q(dX), q(dW), q(db)), "backward", ctx.h))
+    ctx.lib.cct_conv_plan_destroy(plan)
+    mine = [name for name in names if name.startswith("small_conv_kernel")]
+    assert len(names) == launches and len(mine) == 1 and mine[0].endswith(", %d>" % rows), names
+    Xd, Wd = X.double().requires_grad_(), W.double().requires_grad_()
+    torch.nn.functional.conv2d(Xd, Wd, None, s, p).backward(dY.double())
+    for got, ref, name in ((dX, Xd.grad, "dX"), (dW, Wd.grad, "dW"), (db, dY.double().sum((0, 2, 3)), "db")):
+        assert_close(got.cpu().numpy(), ref.float().cpu().numpy(), name)
