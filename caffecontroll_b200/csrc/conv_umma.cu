@@ -2272,7 +2272,8 @@ PackDgrad pack_dgrad_job(const UmmaPlan* p, const float* W) {
   return J;
 }
 
-// Grid of a pass by small_conv_kernel, and its shared memory; `block_warps` > 0: that many per block, beside a weight gradient.
+// Grid of a pass by small_conv_kernel, and its shared memory; `block_warps` > 0: that many per block, which
+// may go beside a weight gradient.
 struct SmallConvShape {
   int ct, rows, warps, x, y;
   size_t smem;
@@ -2298,13 +2299,25 @@ SmallConvShape shape_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct
   return SmallConvShape{ct, rows, warps, (P.positions + per_block - 1) / per_block, P.groups * P.col_tiles,
                         small_conv_smem(k, rows, ct, P.ci, P.share ? warps : 0)};
 }
-void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct) {
-  const SmallConvShape g = shape_small_conv(ctx, P, k, s, ct);
+void launch_small_conv(cct_ctx* ctx, SmallConv& P, int k, int s, int ct, int block_warps = 0) {
+  const SmallConvShape g = shape_small_conv(ctx, P, k, s, ct, block_warps);
   launch_pdl(small_conv_pick(k, s, g.ct, g.rows), dim3(g.x, g.y), dim3(32 * g.warps), g.smem, ctx->stream, P);
 }
 // The data gradient of a stride-1 layer as a convolution of dY.
 SmallConv small_dgrad(const ConvGeom& G, const float* dY, const float* W, float* dX, int batch) {
   return SmallConv{dY, W, nullptr, dX, batch, G.m, G.n, G.k - 1 - G.p, G.og, G.Dg, G.g, 1, 0};
+}
+
+// Whether both gradients of a small layer go in one launch (kSmallRounds and so on).
+bool small_together(cct_ctx* ctx, const UmmaPlan* p) {
+  const ConvGeom& G = p->G;
+  if (!p->w_small || !p->dgr.small_ct) return false;
+  SmallConv d = small_dgrad(G, nullptr, nullptr, nullptr, G.B);
+  if (shape_small_conv(ctx, d, G.k, 1, p->dgr.small_ct).warps > kSwWarps) return false;
+  const SmallConvShape g = shape_small_conv(ctx, d, G.k, 1, p->dgr.small_ct, kSwWarps);
+  const long long blocks = (long long)p->ws_rows * p->ws_cols * G.g * p->wt_tiles * p->w_splits + (long long)g.x * g.y;
+  const long long slots = (long long)SmallBackward::blocks(g.ct) * ctx->sm_count;
+  return blocks <= kSmallRounds * slots && (g.rows != kSmallTall || G.og >= kSmallTallChannels || blocks <= slots);
 }
 
 // A CTA per tile where each has a slot (ONE), or a persistent grid: one CTA per SM (4 producer sets) or two (2 sets); then the reduction over
@@ -2387,15 +2400,10 @@ int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W
   const ConvGeom& G = p->G;
   const size_t nx = (size_t)G.B * G.D * G.n * G.n, ny = (size_t)G.B * G.o * G.m * G.m, nw = (size_t)G.o * G.Dg * G.k * G.k;
   // Small layers: the data gradient goes with the weight gradient, unless one writes where the other reads.
-  if (p->w_small && p->dgr.small_ct && dX && !t->enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, G.o}}) &&
+  if (dX && p->w_small && p->dgr.small_ct && !t->enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, G.o}}) &&
       apart(dW, nw, {{W, nw}, {dY, ny}}) && (!G.bias || apart(db, G.o, {{W, nw}, {dY, ny}}))) {
     SmallConv d = small_dgrad(G, dY, W, dX, G.B);
-    const int warps = shape_small_conv(ctx, d, G.k, 1, p->dgr.small_ct).warps;
-    const SmallConvShape g = shape_small_conv(ctx, d, G.k, 1, p->dgr.small_ct, kSwWarps);
-    const long long blocks = (long long)p->ws_rows * p->ws_cols * G.g * p->wt_tiles * p->w_splits + (long long)g.x * g.y;
-    const long long slots = (long long)SmallBackward::blocks(g.ct) * ctx->sm_count;
-    if (warps <= kSwWarps && blocks <= kSmallRounds * slots && (g.rows != kSmallTall || G.og >= kSmallTallChannels || blocks <= slots))
-      return weight_gradient(ctx, p, X, dY, dW, db, t, nullptr, &d);
+    if (small_together(ctx, p)) return weight_gradient(ctx, p, X, dY, dW, db, t, nullptr, &d);
   }
   int rc = umma_conv_wgrad(ctx, p, X, dY, dW, db, t, dX ? W : nullptr);
   if (rc == CCT_OK && dX) rc = umma_conv_dgrad(ctx, p, W, dY, dX, t, 0, false);
@@ -2506,7 +2514,7 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
     t->begin(3, ctx->stream);
     if (d.small_ct) {
       SmallConv P = small_dgrad(G, dY, W, dX, B);
-      launch_small_conv(ctx, P, G.k, 1, d.small_ct);
+      launch_small_conv(ctx, P, G.k, 1, d.small_ct, small_together(ctx, p) ? kSwWarps : 0);  // the same sums with and without company
       t->end(3, ctx->stream);
       CCT_CHECK_LAUNCH(ctx);
       return CCT_OK;

@@ -1071,3 +1071,31 @@ def test_rows_of_one_channel(ctx, shape, rows, launches):
     torch.nn.functional.conv2d(Xd, Wd, None, s, p).backward(dY.double())
     for got, ref, name in ((dX, Xd.grad, "dX"), (dW, Wd.grad, "dW"), (db, dY.double().sum((0, 2, 3)), "db")):
         assert_close(got.cpu().numpy(), ref.float().cpu().numpy(), name)
+
+
+# The data gradient of a small layer beside its weight gradient, in a launch of its own with the timing switched on, and over X, from few channels for
+# eight warps to more than two a warp: the same bits.
+@pytest.mark.parametrize("shape", [(16, 6, 30, 12, 3, 1, 1, 1), (3, 8, 10, 5, 1, 1, 0, 1), (5, 1, 9, 7, 5, 1, 0, 1), (6, 2, 11, 24, 3, 1, 1, 2), (64, 1, 28, 20, 5, 1, 0, 1),
+                                   (2, 3, 13, 9, 7, 1, 3, 1), (4, 12, 8, 4, 3, 1, 1, 1), (4, 12, 8, 3, 3, 1, 1, 1), (8, 7, 18, 23, 5, 1, 2, 1)])
+def test_small_data_gradients_alone_and_in_company(ctx, shape):
+    B, D, n, o, k, s, p, g = shape
+    m = n + 2 * p - k + 1
+    gen = torch.Generator(device="cuda").manual_seed(o)
+    X, W, dY = (torch.randn(sh, device="cuda", generator=gen) for sh in ((B, D, n, n), (o, D // g, k, k), (B, o, m, m)))
+    plan, q, results = C.c_void_p(), lambda t: t.data_ptr(), []
+    desc = capi.ConvDesc(B, D, n, o, k, s, p, g, 1, capi.ALGO_AUTO)
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_conv_plan_create(ctx.h, C.byref(desc), C.byref(plan)), "plan", ctx.h)
+    for timed, over in ((0, False), (1, False), (0, True)):
+        capi.check(ctx.lib.cct_conv_plan_enable_timing(plan, timed), "timing", ctx.h)
+        x = X.clone()
+        dX, dW, db = x if over else torch.zeros_like(X), torch.zeros_like(W), torch.zeros(o, device="cuda")
+        torch.cuda.synchronize()
+        before = capi.kernel_launches()
+        capi.check(ctx.lib.cct_conv_backward(plan, q(x), q(W), q(dY), q(dX), q(dW), q(db)), "backward", ctx.h)
+        ctx.sync()
+        assert capi.kernel_launches() - before == (3 if timed or over else 2)
+        results.append((dX, dW, db))
+    ctx.lib.cct_conv_plan_destroy(plan)
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
