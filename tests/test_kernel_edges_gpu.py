@@ -209,64 +209,6 @@ def test_single_products_of_inner_products(ctx, B, K, o):
 # reduction, of the weight gradient at most 19 blocks of 32 pixels (1 200 and 1 250 blocks in splits of nine for the last two), which
 # keeps the bound at 1.6e-5 where a missing cross term gives 4e-4.
 @pytest.mark.parametrize("shape", [
-    (3, 224, 14, 80, 1, 1, 0, 1), (3, 256, 14, 200, 1, 1, 0, 1), (3, 264, 14, 64, 1, 1, 0, 1), (4, 300, 13, 136, 3, 1, 1, 1),
-    (8, 512, 27, 272, 1, 1, 0, 2), (24, 28, 40, 100, 3, 1, 1, 1), (24, 12, 40, 28, 3, 1, 1, 1), (40, 3, 115, 96, 11, 4, 0, 1),
-])
-def test_single_products(ctx, shape):
-    from caffecontroll_b200 import conv_layer
-    B, D, n, o, k, s, p, g = shape
-    m = (n + 2 * p - k) // s + 1
-    rng = np.random.default_rng(D + o)
-    X, dY = (rng.standard_normal(sh).astype(np.float32) for sh in ((B, D, n, n), (B, o, m, m)))
-    W = np.zeros((o, D // g, k, k), np.float32)
-    at = np.arange(o)
-    W[at, at % (o // g) % (D // g), at % k, at // k % k] = rng.standard_normal(o)
-    one = np.zeros_like(dY)
-    one[at % B, at, at % m, at // m % m] = rng.standard_normal(o)
-    conv = lambda x, w, dy: conv_layer(ctx, x, w, np.zeros(o, np.float32), dy, k, s, p, g, algo=TENSOR)  # noqa: E731
-    Y, dX, _, _, used = conv(X, W, dY)
-    dW = conv(X, W, one)[2]
-    assert used == TENSOR
-
-    def exact(dy):
-        x, w = (torch.from_numpy(t).double().requires_grad_() for t in (X, W))
-        y = torch.nn.functional.conv2d(x, w, None, s, p, 1, g)
-        y.backward(torch.from_numpy(dy).double())
-        return y.detach().numpy(), x.grad.numpy(), w.grad.numpy()
-
-    y, dx, _ = exact(dY)
-    assert_products(Y, y, "Y")
-    if o <= D:  # (otherwise several filters share a channel)
-        assert_products(dX, dx, "dX")
-    assert_products(dW, exact(one)[2].reshape(dW.shape), "dW")
-
-
-# One feature per image, one output per image: every sum of the three passes is a single product.
-@pytest.mark.parametrize("B,K,o", [(130, 2052, 4224), (70, 2304, 5000), (17, 4164, 4100), (256, 4608, 4608)])
-def test_single_products_of_inner_products(ctx, B, K, o):
-    rng = np.random.default_rng(K)
-    W, at = rng.standard_normal((o, K)).astype(np.float32), np.arange(B)
-    X, dY, b = np.zeros((B, K), np.float32), np.zeros((B, o), np.float32), np.zeros(o, np.float32)
-    X[at, rng.permutation(K)[:B]], dY[at, rng.permutation(o)[:B]] = rng.standard_normal((2, B))
-    c = {name: LogicalCube.from_numpy(ctx, t.reshape(1, 1, *t.reshape(-1, t.shape[-1]).shape))
-         for name, t in (("X", X), ("W", W), ("b", b), ("dY", dY), ("Y", 0 * dY), ("dX", 0 * X), ("dW", 0 * W), ("db", 0 * b))}
-    plan, q = C.c_void_p(), {name: cube.ptr for name, cube in c.items()}
-    capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(plan)), "plan", ctx.h)
-    capi.check(ctx.lib.cct_fc_forward(plan, q["X"], q["W"], q["b"], q["Y"], 0, None, 1.0), "forward", ctx.h)
-    capi.check(ctx.lib.cct_fc_backward(plan, q["X"], q["W"], q["dY"], q["dX"], q["dW"], q["db"], 0, None, 1.0), "backward", ctx.h)
-    ctx.sync()
-    ctx.lib.cct_fc_plan_destroy(plan)
-    X, W, dY = (t.astype(np.float64) for t in (X, W, dY))
-    for name, ref in (("Y", X @ W.T), ("dX", dY @ W), ("dW", dY.T @ X)):
-        assert_products(c[name].download().reshape(ref.shape), ref, name)
-    for cube in c.values():
-        cube.free()
-
-
-# Both sides of the lines behind which cross terms are bf16 (chains of 8 blocks of 32, more than 64 columns), reductions that are
-# no multiple of 32 or of eight channels, data of random sign.  Relative 2-norms: per product lo (below 2^-10 of x) is rounded to
-# eight bits, twice, of random sign: below 2^-19; the truncating additions as above, three per block at the most.
-@pytest.mark.parametrize("shape", [
     (3, 224, 14, 80, 1, 1, 0, 1), (3, 256, 14, 80, 1, 1, 0, 1), (3, 257, 14, 65, 1, 1, 0, 1), (3, 264, 14, 64, 1, 1, 0, 1),
     (5, 29, 15, 130, 3, 1, 1, 1), (2, 160, 17, 272, 3, 1, 1, 2), (4, 40, 19, 300, 5, 2, 2, 1),
     (24, 28, 40, 75, 3, 1, 1, 1), (25, 28, 40, 170, 3, 1, 1, 1),  # both operands of the weight gradient in shared memory
