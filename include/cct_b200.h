@@ -185,7 +185,8 @@ int cct_conv_weight_grad_noalloc(cct_ctx* ctx, const cct_conv_desc* desc, const 
                                  float* db);
 
 /* Per-kernel device times of the plan's most recent forward and backward call, for measurement: when enabled,
- * CUDA events are recorded around each kernel group on the context's stream.  ms[0] forward contraction,
+ * CUDA events are recorded around each kernel group on the context's stream.  Small layers, whose gradients are otherwise one
+ * launch, then have one launch for each: the same results, but not the launches of an untimed call.  ms[0] forward contraction,
  * ms[1] weight-gradient contraction, with the pass over dY in front of it, ms[2] its split reduction, with the bias gradient and
  * the packing of the weights for the data gradient, ms[3] data-gradient contraction(s), with that packing in calls of one slice
  * of the batch (host buffers), ms[4] packing of the weights for the forward pass.  The pooling and ReLU masks of
@@ -199,7 +200,8 @@ int cct_conv_plan_last_timings(cct_conv_plan* plan, float ms[5]);
  *      backward_bias_fc: src/sched/DeviceDriver_GPU.cu:1142-1160).  X is [batch][in_features] (a cube of any R x C x D
  *      with R*C*D = in_features, flattened as the reference does), W is [out_features][in_features], Y is
  *      [batch][out_features].  The three contractions run as 3xTF32 on the tensor cores with the operands read in place by
- *      TMA (nothing is transposed or packed); feature counts that are no multiples of 4 take copies with padded rows first. ---- */
+ *      TMA (nothing is transposed or packed; feature counts that are no multiples of 4 take copies with padded rows first), those of
+ *      small layers, of forward passes with few products and of operands off a 16-byte boundary in fp32. ---- */
 typedef struct cct_fc_plan cct_fc_plan;
 int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_features, int bias_term, cct_fc_plan** out);
 int cct_fc_plan_destroy(cct_fc_plan* plan);
@@ -215,7 +217,8 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
  * dY, as Y may overlap X in the forward pass: the results are those of separate buffers. */
 int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const float* dY, float* dX, float* dW, float* db,
                     int in_relu, const uint32_t* in_drop_mask, float in_drop_scale);
-/* Per-kernel-group device times of the most recent calls (as cct_conv_plan_last_timings): ms[0] forward, ms[1] weight
+/* Per-kernel-group device times of the most recent calls (as cct_conv_plan_last_timings; a call with the timing on has a launch for
+ * each contraction, where both of a backward pass may be one without): ms[0] forward, ms[1] weight
  * gradient, with the bias gradient where no launch of the data gradient adds it, ms[3] data gradient, with the bias gradient
  * where its reduction adds it. */
 int cct_fc_plan_enable_timing(cct_fc_plan* plan, int enable);

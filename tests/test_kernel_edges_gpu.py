@@ -310,9 +310,10 @@ def test_inner_product_gradient_in_place(ctx, B, K, shift):
     ctx.lib.cct_fc_plan_destroy(plan)
 
 
-# Outputs over operands in layers of the fp32 kernels, with and without splits of a reduction, and where an operand off a 16-byte boundary
-# brings a layer of the tensor cores there: Y over X, dX over dY, dX over the weights, bit for bit what separate buffers give, every time.
-@pytest.mark.parametrize("B,K,off", [(64, 32, 0), (256, 200, 0), (450, 210, 0), (577, 256, 0), (640, 256, 0), (385, 200, 0), (40, 256, 0), (256, 640, 1)])
+# Outputs over operands in layers of the fp32 kernels, with and without splits of a reduction, where an operand off a 16-byte boundary brings a
+# layer of the tensor cores there, and on the tensor cores (alone, both contractions together, rows in padded copies): Y over X, dX over dY, dX over the weights, bit for bit what separate buffers give, every time.
+@pytest.mark.parametrize("B,K,off", [(64, 32, 0), (256, 200, 0), (450, 210, 0), (577, 256, 0), (640, 256, 0), (385, 200, 0), (40, 256, 0), (256, 640, 1),
+                                     (256, 640, 0), (64, 800, 0), (130, 1026, 0)])
 def test_inner_products_over_their_operands(ctx, B, K, off):
     gen = torch.Generator(device="cuda").manual_seed(B)
     make = lambda *sh: torch.randn(sh, generator=gen, device="cuda")  # noqa: E731
