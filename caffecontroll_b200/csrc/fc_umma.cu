@@ -624,6 +624,17 @@ FcShape fc_weight_pair_shape(int K, int O, int B) {
   return s;
 }
 long long fc_tiles(const FcShape& s) { return (long long)s.P.m_tiles * s.P.n_tiles * s.P.splits; }
+// Whether both are faster in one launch.  With a slot for every tile always (272 layers of 8 to 128 images: by 25 - 50 %).  In more rounds not
+// where the data gradient's tiles alone have an SM each and more than two k-blocks of images make the weight gradient's wider tiles
+// worth while, unless those leave most of a second round empty: 4096 -> 512, 128 images, two launches 18.0 us, one 19.4; 2304 -> 1000 19.2
+// and 20.8; 6272 -> 552 22.5 and 23.2; with 64 images 14.7 and 13.8, 15.3 and 14.3, 16.7 and 16.4 (the same layers), but 3136 -> 1000, eight k-blocks
+// a tile of the data gradient, 17.7 and 18.4; 128 images, tiles that share SMs alone too: 6272 -> 512 23.2 and 20.6; 215 wide tiles: 5436 -> 400 21.9 and 19.9.
+bool fc_pair_faster(int sms, const FcShape& w, const FcShape& d, const FcShape& w_alone) {
+  const long long tw = fc_tiles(w), td = fc_tiles(d), alone = fc_tiles(w_alone), slots = 2ll * sms;
+  if (!d.pair || !share_slots(slots, tw, td)) return false;
+  const bool second_round_empty = alone > sms && 5 * alone < 8 * sms;
+  return 20 * (tw + td) <= 21 * slots || td > sms || (w.P.kblocks_total <= 2 && d.P.kblocks_per_split < 8) || second_round_empty;
+}
 
 }  // namespace
 
@@ -767,7 +778,7 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   const bool few = use_small_fc(batch, in_features, out_features);
   p->small_forward = few;
   p->wgr_pair = fc_weight_pair_shape(in_features, out_features, batch);
-  p->pair = p->dgr.pair && share_slots(2ll * ctx->sm_count, fc_tiles(p->wgr_pair), fc_tiles(p->dgr)) && fc_fit_rings(p->wgr_pair);
+  p->pair = fc_pair_faster(ctx->sm_count, p->wgr_pair, p->dgr, p->wgr) && fc_fit_rings(p->wgr_pair);
   p->small = few || fc_small_faster(ctx->sm_count, batch, in_features, out_features, p->pair);
   p->small_fwd = fc_small_splits(ctx->sm_count, out_features, batch, in_features);
   p->small_dgr = fc_small_splits(ctx->sm_count, in_features, batch, out_features);

@@ -806,6 +806,13 @@ def test_lines_of_the_dot_products(ctx, B, K, o, shift, launches):
     assert_close(Y.cpu().numpy(), (X.double() @ W.double().T + b.double()).float().cpu().numpy(), "Y")
 
 
+# Both sides of the line between one launch and two for both contractions on the tensor cores, in one round of tiles and in more.  Tolerance: parity.
+@pytest.mark.parametrize("B,K,o,launches", [(128, 4096, 256, 2), (128, 4096, 512, 3), (64, 4096, 512, 2), (64, 3136, 1000, 3), (128, 6272, 512, 2), (128, 5436, 400, 2),
+                                            (128, 6272, 552, 3)])
+def test_lines_of_the_merged_launch(ctx, B, K, o, launches):
+    test_backward_passes_of_long_batches(ctx, B, K, o, launches)
+
+
 # Both sides of the line between the fp32 tiles and the tensor cores in backward passes of layers that are not small: a batch that makes one
 # block's chain long, blocks for every SM several times over.  Tolerance: parity.
 @pytest.mark.parametrize("B,K,o,launches", [(256, 784, 128, 1), (640, 1000, 100, 3), (4096, 784, 128, 3), (8192, 64, 512, 1), (1024, 256, 256, 1)])
