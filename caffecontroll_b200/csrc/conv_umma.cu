@@ -240,7 +240,8 @@ enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3 };
 // beside the allocation.  conv3 of one image 13.6 -> 13.0 us, 37 images of 50 -> 75 channels both ways 36.3 -> 34.9.  Not for the
 // persistent kernels' last tiles, nor for the other two modes: the registers it takes spill (AlexNet conv1 at batch 256 1 211 -> 1 227
 // us both ways; LeNet conv2's forward kernel 9.9 -> 11.1).  Where a tile is long it gains nothing (CaffeNet at batch 32 1 238 -> 1 245 us).
-// Data gradients with a stride, which store every other word and further apart, only up to kOneScattered columns per SM: beyond, all warps storing
+// Data gradients with a stride, which store every other word and further apart, only up to kOneScattered columns per SM (stride 2; half as many
+// above: 4 -> 12 channels 148 x 148, 11 x 11 by 4, 8 images, 37 columns per SM, 7.7 -> 7.7 us, 23 images, 106, 10.3 -> 11.5): beyond, all warps storing
 // at once are slower than the persistent kernel's four in turn (64 -> 8 channels 21 x 21, 3 x 3 by 2: 78 images, 296 tiles of 64 columns, 8.5 -> 8.3
 // us, 148 images, 280 of 128, 10.9 -> 11.8; 256 -> 51 channels 13 x 13, 48 images, 133 of 160, 13.1 -> 13.5).
 constexpr int kOneKblocks = 32, kOneScattered = 128;
@@ -1952,9 +1953,9 @@ void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias,
     gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = acc <= 64 && !ptab ? 3 : 2; gp.b_stages = b_two;
   }
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
-  const bool scattered = gp.splits == 1 && gp.n != gp.ch_tile;  // columns are the pixels of a stride period
+  const int period = gp.splits == 1 ? gp.n / gp.ch_tile : 1;  // pixels of a stride period, which are columns, where they are stored as such
   gp.one = gp.taps_smem && !gp.inside && gp.split_k <= kOneKblocks * kBlockK && tiles <= (long long)sms * (gp.sets == 2 ? 2 : 1) &&
-           (!scattered || tiles * gp.n_pad <= (long long)sms * kOneScattered);
+           (period == 1 || tiles * gp.n_pad <= (long long)sms * (period <= 4 ? kOneScattered : kOneScattered / 2));
   gp.w_half = (size_t)vgroups * gp.n_pad * map_k;
   mem.room(&gp.w, 2 * gp.w_half);
 }

@@ -931,7 +931,8 @@ def kernels_of(ctx, call):
     ((38, 96, 10, 300, 5, 1, 1, 1), "<4, 1, true>", None, "<4, 0, false>"), ((52, 33, 31, 40, 3, 2, 1, 1), "<2, 0, true>", None, "<4, 1, true>"),
     ((58, 64, 7, 17, 1, 2, 0, 1), "<2, 1, true>", "<1, 2>", "<2, 0, true>"), ((2, 33, 17, 300, 3, 1, 1, 1), "<2, 0, true>", "<1, 10>", "<2, 0, true>"),
     ((78, 64, 21, 8, 3, 2, 1, 1), "<2, 1, true>", None, "<2, 1, true>"), ((148, 64, 21, 8, 3, 2, 1, 1), "<2, 1, true>", None, "<2, 1, false>"),
-    ((48, 256, 13, 51, 3, 2, 1, 1), "<2, 1, true>", None, "<4, 0, false>"),
+    ((48, 256, 13, 51, 3, 2, 1, 1), "<2, 1, true>", None, "<4, 0, false>"), ((32, 16, 31, 24, 11, 4, 2, 1), "<2, 1, true>", None, "<2, 1, true>"),
+    ((64, 16, 31, 24, 11, 4, 2, 1), "<2, 1, true>", None, "<2, 1, false>"),
     ((37, 1024, 16, 130, 1, 1, 0, 1), "<2, 1, true>", None, "<2, 0, false>"), ((37, 1056, 16, 130, 1, 1, 0, 1), "<2, 1, false>", None, "<4, 0, false>"),
 ])
 def test_a_cta_per_tile(ctx, keep_sms, shape, forward, weight, data):
