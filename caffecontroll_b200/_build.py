@@ -21,6 +21,7 @@ def sources():
 
 def _headers():
     return glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh")) + \
+        glob.glob(os.path.join(CSRC, "*.inc")) + \
         glob.glob(os.path.join(HERE, "..", "include", "*.h"))
 
 

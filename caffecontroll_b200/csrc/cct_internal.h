@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/cct_b200.h"
+#include "half_pairs.cuh"
 
 struct cct_ctx;
 
@@ -185,7 +186,8 @@ struct DyRows {
   float* rows = nullptr;
   size_t lo = 0, row_len = 0;
   float* plane_sums = nullptr;
-  int channels = 0;
+  int channels = 0, batch = 0;
+  const HalfScale* half = nullptr;  // set, and X and dY ok: pairs of fp16 of scaled dY in place of the low parts (half_word)
 };
 struct UmmaPlan;  // opaque: tables, packed weights, split-K scratch
 // `tensor_only`: every pass on the tensor cores, however small the layer (CCT_ALGO_UMMA_3XTF32 by name); otherwise small
@@ -201,8 +203,10 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
                       int relu, PhaseTimer* t, int batch = 0, bool repack = true);
 int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dY, float* dX,
                        float* dW, float* db, PhaseTimer* t);
-// Whether umma_conv_backward takes dY in the form of `rows` (then dY = null), written there by the kernel that makes it.
+// Whether umma_conv_backward takes dY in the form of `rows` (then dY = null), written there by the kernel that makes it;
+// umma_rows_scales comes before that kernel: dY is what a 3x3 / stride 2 pooling of P's windows makes of dP.
 bool umma_dy_rows(const UmmaPlan* p, DyRows* rows);
+int umma_rows_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, size_t pooled);
 int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t,
                     const float* pack_W = nullptr);
 int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, float* dX, PhaseTimer* t, int batch,

@@ -4,7 +4,8 @@
 // tensor memory).  The lowered matrix of the reference (type-1 lowering, one row of k*k*D values per output pixel)
 // is never written to global memory: producer threads gather each 128 x 32 tile of it straight from the NCHW
 // tensors, splitting every fp32 value into hi = its tf32 part and lo = x - hi on the way.  Three MMAs per k-step
-// (hi*hi + hi*lo + lo*hi) recover fp32-level accuracy ("3xTF32"); flops are counted once.
+// (hi*hi + hi*lo + lo*hi) recover fp32-level accuracy ("3xTF32"); flops are counted once.  Larger contractions split
+// scaled values into two fp16 parts instead, at twice the rate, where the operands' values allow it (operand_scale.cuh).
 //
 //   forward        Y[pix][o]   = sum_k  Lowered(X)[pix][k] * W[o][k]            (+ bias, optional ReLU)
 //   data gradient  dX[q][(d,py,px)] = sum_kk Gathered(dY)[q][kk] * Wd[(d,py,px)][kk]   kk = (filter, jy, jx)
@@ -31,6 +32,7 @@
 #include <cuda.h>
 
 #include "cct_internal.h"
+#include "operand_scale.cuh"
 #include "umma_ptx.cuh"
 
 namespace {
@@ -181,6 +183,11 @@ struct GatherParams {
   int wg_mtiles, wg_vgroups;  // tiles = splits x channel tiles x M-tiles (M-tile fastest)
   int wg_rows_pad;            // rows of one split's partial-sum slice (M-tiles * 128)
   int wg_k, wg_kreal;         // kernel size, real rows of the lowered matrix
+  // HALF: the scales of the plan's operands, which two of them this contraction has (gathered, packed), the first row of the packed
+  // operand in pairs of fp16, and the stages that there is room for then.
+  const HalfScale* half;
+  int half_gathered, half_packed, half_row_offset;
+  int a_stages_half, b_stages_half, acc_bufs_half;
   int taps_smem;              // entries of `taps` staged in shared memory (0 in weight-gradient mode)
   const float* zero;          // kByRun: what lanes whose tap is out of bounds read
   int run_stride;             // kByRun: elements between consecutive channels of the gathered tensor
@@ -233,7 +240,7 @@ __host__ __device__ inline GatherSmem gather_smem(int n_pad, int k_pad, int b_st
 // whose windows lie inside the plane: 5.3 instructions per value instead of 9, AlexNet conv1 at batch 256 320 -> 293 us.  (Entries
 // behind the last real index read the window's first element against a weight of zero; lanes behind the last pixel read the last
 // pixel's window, their columns are not stored.)
-enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3 };
+enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3, kHalf = 4 };  // FORM: one of the first four, + kHalf (HALF)
 // ONE: every CTA has one tile, a short one (kOneKblocks).  There is no next tile then for the epilogue to overlap with, and the producers,
 // who are through, take their share of its columns (six chunks of 16 took four warps 1.2 us); in front of the first k-block stood three
 // trips to L2 for the tables and the bias, one behind the other, and the allocation of tensor memory (1.3 us in all), now one trip
@@ -245,9 +252,17 @@ enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3 };
 // at once are slower than the persistent kernel's four in turn (64 -> 8 channels 21 x 21, 3 x 3 by 2: 78 images, 296 tiles of 64 columns, 8.5 -> 8.3
 // us, 148 images, 280 of 128, 10.9 -> 11.8; 256 -> 51 channels 13 x 13, 48 images, 133 of 160, 13.1 -> 13.5).
 constexpr int kOneKblocks = 32, kOneScattered = 128;
-template <int SETS, int MODE, bool ONE>
+// HALF: the operands as pairs of fp16 where the scales of this call say so (operand_scale.cuh), of tf32 otherwise: an A slot has 32 columns
+// then (16 of hi, 16 of lo, two values to a column), a weight slot one row of 128 bytes per column, 32 hi and 32 lo.  Half the MMAs:
+// CaffeNet at batch 256, conv2 forward 387 -> 280 us, conv3 256 / 253 / 273 (forward, weight, data gradient) -> 150 / 165 / 176, conv4 213 /
+// 210 / 211 -> 116 / 138 / 119, conv5 141 / 159 / 149 -> 98 / 138 / 85, 14 - 26 us for each look at the operands; what is left is the gather of the
+// producers (tensor pipe and load-store unit wait for it).  Errors against 64 bits are half as large (conv3, 64 images of 14 x 14, positive
+// data: Y 1.44e-5 -> 7.9e-6, dX 7.8e-6 -> 4.6e-6, dW 2.2e-5 -> 1.1e-5), since the accumulator is truncated half as often.
+template <int SETS, int FORM, bool ONE>
 __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     gather_conv_kernel(const __grid_constant__ GatherParams P, const __grid_constant__ CUtensorMap w_map) {
+  constexpr int MODE = FORM % kHalf;
+  constexpr bool HALF = FORM >= kHalf;
   constexpr int kProducerWarps = 4 * SETS, kMmaWarp = kProducerWarps, kTmaWarp = kMmaWarp + 1;
   constexpr int kGatherThreads = gather_threads(SETS);
   extern __shared__ uint8_t smem_raw[];
@@ -267,6 +282,8 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   float* s_bias = reinterpret_cast<float*>(base_ptr + L.bias_off);
   const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
 
+  // HALF: the gathered operand's scale (0: tf32 instead) and what takes both operands' scales back
+  float* s_scale = reinterpret_cast<float*>(base_ptr + (tmem_slot + 4 - base));
   int* s_offsets = reinterpret_cast<int*>(s_taps);  // kInside: the offsets alone
   auto init_barriers = [&]() {
     for (int s = 0; s < kMaxAStages; ++s) { mbar_init(ready_bar + 8u * s, 5); mbar_init(done_bar + 8u * s, 1); }  // 4 producer warps + the TMA thread
@@ -302,6 +319,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     if (warp == kTmaWarp) prefetch_map(&w_map);
     pdl_wait();  // so far the plan's tables alone have been read: set-up beside the end of the kernel before (15.6 -> 15.35 us for conv3 of one image)
     for (int i = tid; i < P.n_bias + kBiasPad; i += kGatherThreads) s_bias[i] = i < P.n_bias ? P.bias[i] : 0.f;
+    if (HALF && tid == 0) {
+      const HalfScale a = P.half[P.half_gathered], b = P.half[P.half_packed];
+      s_scale[0] = a.ok && b.ok ? a.scale : 0.f;
+      s_scale[1] = a.inverse * b.inverse;
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -309,383 +331,22 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
   const uint32_t acc_cols = (uint32_t)acc_columns(P.n_pad), cross = acc_cols - (uint32_t)P.n_pad;  // cross: 0 = one accumulator
-  const uint32_t a_col0 = (uint32_t)P.acc_bufs * acc_cols;
   const int kblocks = P.k_pad / kBlockK;
   bool failed = false;
-  // 16 columns of a finished accumulator
-  auto load_acc = [&](uint32_t taddr, float* v) {
-    tmem_ld16(taddr, v);
-    if (cross) {
-      float c[16];
-      tmem_ld16(taddr + cross, c);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] += c[j];
+  // The roles' text stands in a file of its own because the half kernels need it twice, each time with `half` known: by a flag in one text
+  // <2, kWeightGrad> spilled (CaffeNet conv2's weight gradient 332 -> 372 us); as a function or a lambda the kernels of single tiles
+  // came out with more registers (37 images of 50 -> 75 channels both ways 35.0 -> 36.4).
+  if constexpr (HALF) {
+    if (s_scale[0] != 0.f) {
+      constexpr bool half = true;
+#include "gather_roles.inc"
+    } else {
+      constexpr bool half = false;
+#include "gather_roles.inc"
     }
-  };
-
-  if (warp < kProducerWarps) {
-    // ------------------------------------------------------------------ producers
-    // Set `group` fills the A stages of the k-blocks with running index == group (mod SETS).  The raw
-    // values of the set's next k-block are already in flight (in registers) while the current one is split and
-    // stored, so the global-load latency is paid once per k-block per set, off the critical path.
-    const int group = warp >> 2, quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + a_col0;
-    const int my_tiles = (P.total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int my_stages = my_tiles * kblocks;
-    const float* in_px = P.in;
-    uint32_t mask = 0;                   // forward / data gradient: which taps are in bounds for this lane's pixel
-    const MaskTap* pix_tab = P.taps;     // weight gradient: this tile's slice of the per-pixel table
-    const int* tile_offsets = s_offsets;
-    const MaskTap* tile_taps = s_taps;   // forward / data gradient: this tile's part of the tap table
-    auto setup_tile = [&](int tile_local) {
-      const int t = blockIdx.x + tile_local * gridDim.x;
-      const TileId id = decode_tile<MODE == kWeightGrad>(P, t, kblocks);
-      const int grp = id.vg / P.tiles_per_group;
-      in_px = P.in;
-      if (MODE == kWeightGrad) {
-        // lane = row of the lowered matrix: (d, kr, kc); `mask` holds the tap's row and column bit
-        const int r = id.ptile * kTileM + row;
-        mask = kPadBit;
-        if (r < P.wg_kreal) {
-          const int kk = P.wg_k * P.wg_k;
-          const int d = r / kk, rem = r - d * kk;
-          const int kr = rem / P.wg_k, kc = rem - kr * P.wg_k;
-          in_px = P.in + (long long)grp * P.in_group_stride + (long long)d * P.in_lim * P.in_lim + kr * P.in_lim + kc;
-          mask = (1u << kr) | (1u << (16 + kc));
-        }
-        pix_tab = P.taps + (size_t)id.kb0 * kBlockK;
-        return;
-      }
-      tile_taps = s_taps + id.kb0 * (kBlockK / (MODE == kByRun ? kRun : 1));
-      if (MODE == kInside) {
-        tile_offsets = s_offsets + id.kb0 * kBlockK;
-        const int pix = min(id.ptile * kTileM + row, P.n_pix - 1), per_img = P.q_h * P.q_w;
-        const int b = pix / per_img, r = pix - b * per_img, qy = r / P.q_w, qx = r - qy * P.q_w;
-        in_px = P.in + (long long)b * P.in_batch_stride + (long long)grp * P.in_group_stride + (long long)(qy * P.iy_mul) * P.in_lim + qx * P.ix_mul;
-        return;
-      }
-      const int pix = id.ptile * kTileM + row;
-      mask = 0;  // which tap rows (bits 0-14) and tap columns (bits 16-30) fall inside the plane
-      if (pix < P.n_pix) {
-        const int per_img = P.q_h * P.q_w;
-        const int b = pix / per_img;
-        const int r = pix - b * per_img;
-        const int qy = r / P.q_w;
-        const int qx = r - qy * P.q_w;
-        const int iy0 = qy * P.iy_mul + P.iy_add, ix0 = qx * P.ix_mul + P.ix_add;
-        in_px = P.in + (long long)b * P.in_batch_stride + (long long)grp * P.in_group_stride +
-                (long long)iy0 * P.in_lim + ix0;
-        if (P.tap_sign > 0)  // coordinate origin + i in [0, lim)
-          mask = bit_range(-iy0, min(P.taps_per_axis, P.in_lim - iy0)) |
-                 (bit_range(-ix0, min(P.taps_per_axis, P.in_lim - ix0)) << 16);
-        else  // coordinate origin - i in [0, lim)
-          mask = bit_range(iy0 - P.in_lim + 1, min(P.taps_per_axis, iy0 + 1)) |
-                 (bit_range(ix0 - P.in_lim + 1, min(P.taps_per_axis, ix0 + 1)) << 16);
-      }
-    };
-    float v[kBlockK];
-    // Weight gradient: the 32 table entries of a k-block are the same for every lane.  Lane e fetches entry e one
-    // step ahead (`ent_next`, in flight while the current block is split and stored), the warp passes them round
-    // through its own slice of shared memory.
-    uint2 ent_next = make_uint2(0u, 0xffffffffu);
-    uint2* my_ptab = reinterpret_cast<uint2*>(base_ptr + L.ptab_off) + warp * 64;
-    int pbuf = 0;
-    auto prefetch_entries = [&](int kb) {
-      if (MODE == kWeightGrad) ent_next = __ldg(reinterpret_cast<const uint2*>(pix_tab + kb * kBlockK) + lane);
-    };
-    auto gather = [&](int kb) {
-      if (MODE == kWeightGrad) {
-        // entry = (offset of the pixel's tap origin, tap rows / columns out of bounds there)
-        uint2* slot = my_ptab + pbuf * 32;
-        pbuf ^= 1;
-        slot[lane] = ent_next;
-        __syncwarp();
-#pragma unroll
-        for (int e = 0; e < kBlockK; e += 2) {  // two entries per shared-memory read: that pipe is the busiest one here
-          const uint4 ent = reinterpret_cast<const uint4*>(slot)[e / 2];
-          v[e] = ldg_if_clear(in_px + (int)ent.x, ent.y, mask);
-          v[e + 1] = ldg_if_clear(in_px + (int)ent.z, ent.w, mask);
-        }
-        return;
-      }
-      if (MODE == kByRun) {
-        const MaskTap* tp = tile_taps + kb * (kBlockK / kRun);
-#pragma unroll
-        for (int r = 0; r < kBlockK / kRun; ++r) {
-          const MaskTap tap = tp[r];
-          const bool ok = (mask & tap.bits) == tap.bits;
-          const float* p = ok ? in_px + tap.off : P.zero;
-          const int stride = ok ? P.run_stride : 0;
-#pragma unroll
-          for (int e = 0; e < kRun; ++e) v[r * kRun + e] = __ldg(p + e * stride);
-        }
-        return;
-      }
-      if (MODE == kInside) {
-        const int4* tp = reinterpret_cast<const int4*>(tile_offsets + kb * kBlockK);
-#pragma unroll
-        for (int e = 0; e < kBlockK; e += 4) {
-          const int4 off = tp[e / 4];
-          v[e] = __ldg(in_px + off.x);
-          v[e + 1] = __ldg(in_px + off.y);
-          v[e + 2] = __ldg(in_px + off.z);
-          v[e + 3] = __ldg(in_px + off.w);
-        }
-        return;
-      }
-      const MaskTap* tp = tile_taps + kb * kBlockK;
-#pragma unroll
-      for (int e = 0; e < kBlockK; ++e) {
-        const MaskTap tap = tp[e];
-        v[e] = ldg_if_bits(in_px + tap.off, mask, tap.bits);
-      }
-    };
-    int tile_local = 0, kb = group;
-    while (kb >= kblocks && tile_local < my_tiles) { kb -= kblocks; ++tile_local; }
-    if (group < my_stages) {
-      setup_tile(tile_local);
-      prefetch_entries(kb);
-      gather(kb);
-    }
-    int ring_sa = group % P.a_stages;  // A slot of the set's current k-block: index % a_stages
-    for (int it = group; it < my_stages; it += SETS) {
-      // a weight gradient's ring is 2 or 4 deep: no counter (its producers have no register to spare)
-      const int sa = MODE == kWeightGrad ? it & (P.a_stages - 1) : ring_sa;
-      const uint32_t st_addr = lane_addr + (uint32_t)(sa * 64);
-      if (MODE != kWeightGrad)
-        for (ring_sa += SETS; ring_sa >= P.a_stages;) ring_sa -= P.a_stages;
-      // The set's next k-block: its tile state and (weight gradient) its table entries, requested now so that
-      // they have arrived when the gather is issued further down.  v[] still holds the current block.
-      const bool has_next = it + SETS < my_stages;
-      if (has_next) {
-        const int before = tile_local;
-        kb += SETS;
-        while (kb >= kblocks) { kb -= kblocks; ++tile_local; }
-        if (tile_local != before) setup_tile(tile_local);
-        prefetch_entries(kb);
-      }
-      // The A slot was last read by the MMAs of k-block it - a_stages.
-      const int prev = it - P.a_stages;
-      if (prev >= 0) mbar_wait(done_bar + 8u * (prev & 3), (uint32_t)(prev >> 2) & 1u, failed, P.status, 0x10);
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < kBlockK / 8; ++c) {
-        uint32_t hi[8], lo[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) split_tf32_trunc(v[c * 8 + e], hi[e], lo[e]);
-        tmem_st8(st_addr + (uint32_t)(c * 8), hi);
-        tmem_st8(st_addr + 32u + (uint32_t)(c * 8), lo);
-      }
-      // With few stages the hand-over of a filled stage is on the critical path: arrive first, then fetch.
-      if (P.a_stages < 4) {
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(ready_bar + 8u * (it & 3));
-      }
-      if (has_next) gather(kb);  // loads in flight across the next wait
-      if (P.a_stages == 4) {
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(ready_bar + 8u * (it & 3));  // one arrival per warp: same-address arrivals serialise
-      }
-    }
-  } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------------ MMA issue (see elect_one)
-    const uint32_t idesc = make_idesc(P.n_pad), tmem = warp_uniform(tmem_base);
-    int tile_iter = 0;
-    Ring ra, rb, rbar;  // A slot, weight slot, barrier pair of the current k-block
-    for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x, ++tile_iter) {
-      const int buf = tile_iter & (P.acc_bufs - 1), ause = tile_iter >> (P.acc_bufs - 1);  // acc_bufs is 1 or 2
-      if (ause > 0) mbar_wait<false>(acc_empty + 8u * buf, (uint32_t)(ause - 1) & 1u, failed, P.status, 0x20);
-      tc_fence_after();
-      const uint32_t d_tmem = tmem + (uint32_t)buf * acc_cols, d_cross = d_tmem + cross;
-      for (int kb = 0; kb < kblocks; ++kb) {
-        mbar_wait<false>(ready_bar + 8u * rbar.idx, (uint32_t)rbar.use & 1u, failed, P.status, 0x40);
-        tc_fence_after();
-        const uint32_t b_hi = base + (uint32_t)rb.idx * L.b_stage_bytes, b_lo = b_hi + (uint32_t)P.n_pad * 128u;
-        const uint64_t dbh = make_desc(b_hi), dbl = make_desc(b_lo);
-        const uint32_t a_hi = tmem + a_col0 + (uint32_t)(ra.idx * 64), a_lo = a_hi + 32u;
-        if (elect_one()) {
-#pragma unroll
-          for (int j = 0; j < kBlockK / 8; ++j) {
-            const uint64_t adv = (uint64_t)(j * 2);
-            const uint32_t add = kb == 0 && j == 0 ? 0u : 1u;
-            umma_tf32_ts(d_cross, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, add);
-            umma_tf32_ts(d_cross, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
-            umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, cross ? add : 1u);
-          }
-          umma_commit(done_bar + 8u * rbar.idx);  // frees the A slot for the producers and the weight slot for the TMA thread
-          if (kb == kblocks - 1) umma_commit(acc_full + 8u * buf);
-        }
-        __syncwarp();
-        ra.advance(P.a_stages);
-        rb.advance(P.b_stages);
-        rbar.advance(4);
-      }
-    }
-  } else if (warp == kTmaWarp) {
-    // ------------------------------------------------------------------ weight tiles by TMA
-    if (lane == 0) {
-      Ring rb;
-      int i = 0;  // running k-block index
-      for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x) {
-        const TileId id = decode_tile<MODE == kWeightGrad>(P, t, kblocks);
-        const int vg = id.vg;
-        for (int kb = 0; kb < kblocks; ++kb, ++i) {
-          const int sb = rb.idx;
-          const int prev = i - P.b_stages;  // the k-block whose MMAs read this weight slot last
-          if (prev >= 0) mbar_wait<false>(done_bar + 8u * (prev & 3), (uint32_t)(prev >> 2) & 1u, failed, P.status, 0x100);
-          const uint32_t b_hi = base + (uint32_t)sb * L.b_stage_bytes, b_lo = b_hi + (uint32_t)P.n_pad * 128u;
-          const uint32_t bar = ready_bar + 8u * (i & 3);
-          mbar_expect_tx(bar, L.b_stage_bytes);
-          tma_load_2d(b_hi, &w_map, (id.kb0 + kb) * kBlockK, vg * P.n_pad, bar);
-          tma_load_2d(b_lo, &w_map, (id.kb0 + kb) * kBlockK, P.lo_row_offset + vg * P.n_pad, bar);
-          rb.advance(P.b_stages);
-        }
-      }
-    }
-  } else if constexpr (!ONE) {
-    // ------------------------------------------------------------------ epilogue
-    const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    int tile_iter = 0;
-    for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x, ++tile_iter) {
-      const TileId id = decode_tile<MODE == kWeightGrad>(P, t, kblocks);
-      const int vg = id.vg, ptile = id.ptile;
-      const int grp = vg / P.tiles_per_group, ntile = vg % P.tiles_per_group;
-      const int buf = tile_iter & (P.acc_bufs - 1), ause = tile_iter >> (P.acc_bufs - 1);
-      if (MODE == kWeightGrad) {
-        // The accumulator is a 128-row slice of this split's partial sums: row-contiguous stores.
-        mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
-        tc_fence_after();
-        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * acc_cols;
-        float* op = P.out + ((size_t)(id.split * P.wg_vgroups + vg) * P.wg_rows_pad + (size_t)ptile * kTileM + row) * P.n_pad;
-        for (int c = 0; c < P.n_pad / 16; ++c) {
-          float v[16];
-          load_acc(acc + (uint32_t)(c * 16), v);
-          if (!failed) {
-            float4* o4 = reinterpret_cast<float4*>(op + c * 16);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) o4[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
-        continue;
-      }
-      const int pix = ptile * kTileM + row;
-      if (P.splits > 1) {
-        // raw sums, lanes along the pixels
-        mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
-        tc_fence_after();
-        const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * acc_cols;
-        float* op = P.partial + (size_t)(id.split * (P.total_tiles / (P.n_pix_tiles * P.splits)) + vg) * P.n_pad * P.pix_pad + pix;
-        for (int c = 0; c < P.n_pad / 16; ++c) {
-          float v[16];
-          load_acc(acc + (uint32_t)(c * 16), v);
-          if (!failed) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) op[(size_t)(c * 16 + j) * P.pix_pad] = v[j];
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
-        continue;
-      }
-      int b = 0, qy = 0, qx = 0;
-      if (pix < P.n_pix) {
-        const int per_img = P.q_h * P.q_w;
-        b = pix / per_img;
-        const int r = pix - b * per_img;
-        qy = r / P.q_w;
-        qx = r - qy * P.q_w;
-      }
-      const int oy0 = qy * P.oy_mul + P.oy_add, ox0 = qx * P.ox_mul + P.ox_add;
-      const int ch0 = grp * P.out_group_channels + ntile * P.out_tile_channels;
-      float* op = P.out + (long long)b * P.out_batch_stride + (long long)ch0 * P.out_plane +
-                  (long long)oy0 * P.out_pitch + ox0;
-      const float* bias = s_bias + (P.n_bias ? ch0 : 0);  // zero padded: readable for every column of the tile
-      // the last channel tile of a group may hold fewer channels than the others
-      const int n_live = min(P.n, (P.out_group_channels - ntile * P.out_tile_channels) * P.cols_per_channel);
-      mbar_wait(acc_full + 8u * buf, (uint32_t)ause & 1u, failed, P.status, 0x200);
-      tc_fence_after();
-      const uint32_t live = (pix < P.n_pix && !failed) ? 1u : 0u;
-      const uint32_t unchecked = P.check_out ? 0u : 1u;
-      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)buf * acc_cols;
-      const int chunks = P.n_pad / 16;
-      for (int c = 0; c < chunks; ++c) {
-        float v[16];
-        load_acc(acc + (uint32_t)(c * 16), v);
-        // Straight-line code: table and bias reads first, then predicated st.global (a generic store could alias
-        // shared memory and would pin every following table read behind it; a branch per column costs more than
-        // the store it guards).
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          ColEnt ce[8];
-          float bv[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int col = c * 16 + h * 8 + j;
-            ce[j] = s_cols[col];
-            bv[j] = bias[col];
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int col = c * 16 + h * 8 + j;
-            const uint32_t in_y = (unsigned)(oy0 + ce[j].cy) < (unsigned)P.out_lim ? 1u : 0u;
-            const uint32_t in_x = (unsigned)(ox0 + ce[j].cx) < (unsigned)P.out_lim ? 1u : 0u;
-            const uint32_t ok = live & (col < n_live ? 1u : 0u) & (unchecked | (in_y & in_x));
-            float y = v[h * 8 + j] + bv[j];
-            y = P.relu ? fmaxf(y, 0.f) : y;
-            stg_if(op + ce[j].off, y, ok);
-          }
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
-    }
-  }
-  if constexpr (ONE) {
-    // The tile's chunks of 16 columns in turn to the epilogue warps and the producers' sets.
-    if (warp < kProducerWarps || warp > kTmaWarp) {
-      const TileId id = decode_tile<false>(P, blockIdx.x, kblocks);
-      const int grp = id.vg / P.tiles_per_group, ntile = id.vg - grp * P.tiles_per_group;
-      const int quarter = warp & 3, pix = id.ptile * kTileM + quarter * 32 + lane, per_img = P.q_h * P.q_w;
-      const int b = pix / per_img, r = pix - b * per_img, qy = r / P.q_w, qx = r - qy * P.q_w;
-      const int oy0 = qy * P.oy_mul + P.oy_add, ox0 = qx * P.ox_mul + P.ox_add;
-      const int ch0 = grp * P.out_group_channels + ntile * P.out_tile_channels;
-      float* op = P.out + (long long)b * P.out_batch_stride + (long long)ch0 * P.out_plane + (long long)oy0 * P.out_pitch + ox0;
-      float* sums = P.partial + (size_t)(id.split * (P.total_tiles / (P.n_pix_tiles * P.splits)) + id.vg) * P.n_pad * P.pix_pad + pix;
-      const float* bias = s_bias + (P.n_bias ? ch0 : 0);
-      const int n_live = min(P.n, (P.out_group_channels - ntile * P.out_tile_channels) * P.cols_per_channel);
-      mbar_wait(acc_full, 0u, failed, P.status, 0x210);
-      tc_fence_after();
-      const bool live = pix < P.n_pix && !failed;
-      const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16);
-      for (int c0 = warp < kProducerWarps ? 16 + (warp >> 2) * 16 : 0; c0 < P.n_pad; c0 += 16 * (1 + SETS)) {
-        float v[16];
-        load_acc(acc + (uint32_t)c0, v);
-        if (P.splits > 1) {
-          if (failed) continue;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) sums[(size_t)(c0 + j) * P.pix_pad] = v[j];  // raw sums, lanes along the pixels
-          continue;
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const ColEnt ce = s_cols[c0 + j];
-          const bool in = !P.check_out || ((unsigned)(oy0 + ce.cy) < (unsigned)P.out_lim && (unsigned)(ox0 + ce.cx) < (unsigned)P.out_lim);
-          const float y = v[j] + bias[c0 + j];
-          stg_if(op + ce.off, P.relu ? fmaxf(y, 0.f) : y, live && c0 + j < n_live && in ? 1u : 0u);
-        }
-      }
-    }
+  } else {
+    constexpr bool half = false;
+#include "gather_roles.inc"
   }
   tc_fence_before();
   __syncthreads();
@@ -1381,7 +1042,17 @@ namespace {
 // conv3's 0.9 M weights 8.0 / 11.6 us for the two operands, bound by neither memory nor launch).
 constexpr int kPackThreads = 128;
 
-__device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, const float* v) {
+// Into the packed operand: pairs of tf32 in two halves, or (PAIRS, scale != 0) pairs of fp16 in the first (half_word).
+template <bool PAIRS>
+__device__ __forceinline__ void store_split4(float* hi, float* lo, size_t at, const float* v, float scale) {
+  if (PAIRS && scale != 0.f) {
+    uint2 h, l;
+    split_half2(v[0] * scale, v[1] * scale, h.x, l.x);
+    split_half2(v[2] * scale, v[3] * scale, h.y, l.y);
+    *reinterpret_cast<uint2*>(hi + half_word(at)) = h;
+    *reinterpret_cast<uint2*>(hi + half_word(at) + kHalfLo) = l;
+    return;
+  }
   float h[4], l[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) split_tf32(v[e], h[e], l[e]);
@@ -1398,7 +1069,15 @@ struct PackDgrad {
   int tiles_per_group, og, Dg, k, s, taps, d_tile, n_real, n_pad, k_real, k_pad, run;
   int parts;   // blocks per row
   int blocks;  // rows * parts
+  const HalfScale* half;  // null: no data gradient by pairs of fp16
 };
+// The scale of weights that are packed as pairs of fp16 for a contraction with operand `other`, or 0.  (PAIRS, here and in the kernels below: a
+// plan without them takes kernels without that code, whose registers the small ones would feel.)
+template <bool PAIRS>
+__device__ __forceinline__ float pack_scale(const HalfScale* half, int other) {
+  return PAIRS && half_route(half, other, kHalfW) ? half[kHalfW].scale : 0.f;
+}
+template <bool PAIRS>
 __device__ __forceinline__ void pack_dgrad_block(const PackDgrad& J, int block) {
   const int r0 = block / J.parts, part = block - r0 * J.parts;
   const int vg = r0 / J.n_pad, j = r0 - vg * J.n_pad;
@@ -1406,6 +1085,7 @@ __device__ __forceinline__ void pack_dgrad_block(const PackDgrad& J, int block) 
   const int py = (j / J.s) % J.s, px = j % J.s, window = J.taps * J.taps;
   const bool live = j < J.n_real && d < J.Dg;
   const float* src = J.W + ((size_t)grp * J.og * J.Dg + d) * J.k * J.k;
+  const float scale = pack_scale<PAIRS>(J.half, kHalfDy);
   const size_t row = (size_t)r0 * J.k_pad;
   for (int kk = (part * (int)blockDim.x + (int)threadIdx.x) * 4; kk < J.k_pad; kk += J.parts * (int)blockDim.x * 4) {
     // reduction index -> (filter / run, jy, jx, filter % run); four in a row are four filters of one tap where run is kRun, and
@@ -1427,12 +1107,12 @@ __device__ __forceinline__ void pack_dgrad_block(const PackDgrad& J, int block) 
         v[e] = (live && kk + e < J.k_real && kr < J.k && kc < J.k) ? __ldg(src + oc * filter + kr * J.k + kc) : 0.f;
       }
     }
-    store_split4(J.hi, J.lo, row + kk, v);
+    store_split4<PAIRS>(J.hi, J.lo, row + kk, v, scale);
   }
 }
 __global__ void __launch_bounds__(kPackThreads) pack_dgrad_kernel(const __grid_constant__ PackDgrad J) {
   pdl_wait();
-  pack_dgrad_block(J, blockIdx.x);
+  pack_dgrad_block<false>(J, blockIdx.x);
 }
 
 // db[c] = sum over the batch of the plane sums (ConvolutionBridge_impl.hxx:575-599), in a fixed order.
@@ -1461,12 +1141,16 @@ struct ReduceExtras {
   PackDgrad pack;
   BiasSum bias;
 };
+struct HalfExtras : ReduceExtras {  // pairs of fp16
+  explicit HalfExtras(const ReduceExtras& e) : ReduceExtras(e) {}
+};
 // True if this block was one of them; `first` of the grid's x are not.
-__device__ __forceinline__ bool extra_block(const ReduceExtras& E, int first) {
+template <bool PAIRS>
+__device__ __forceinline__ bool extra_block_of(const ReduceExtras& E, int first) {
   int block = (int)blockIdx.x - first;
   if (block < 0) return false;
   if (block < E.pack.blocks) {
-    pack_dgrad_block(E.pack, block);
+    pack_dgrad_block<PAIRS>(E.pack, block);
     return true;
   }
   block -= E.pack.blocks;
@@ -1476,6 +1160,8 @@ __device__ __forceinline__ bool extra_block(const ReduceExtras& E, int first) {
 // A reduction with nothing beside it (small layers, whose gradients need neither) is a kernel without that code: with it a network
 // of 10 images, two such reductions of 4 us in its iteration, took 88.0 us instead of 86.2.
 struct NoExtras {};
+__device__ __forceinline__ bool extra_block(const ReduceExtras& E, int first) { return extra_block_of<false>(E, first); }
+__device__ __forceinline__ bool extra_block(const HalfExtras& E, int first) { return extra_block_of<true>(E, first); }
 __device__ __forceinline__ bool extra_block(const NoExtras&, int) { return false; }
 
 // dW[o][kk] and db[o] from the split partial sums, added in split order (deterministic).  One block per 32 x 32
@@ -1570,11 +1256,17 @@ __global__ void __launch_bounds__(32 * SLICES) wgrad_reduce_flat_kernel(const fl
 // dY[b][c][pix] -> hi / lo [row of channel c][b * mm + pix] with row = channel tile * n_pad + channel inside the
 // tile (K-major rows of `row_len` floats, so a TMA box is 32 consecutive pixels x one channel tile), and the plane
 // sum of dY[b][c] for the bias gradient.  One block per plane at a time; every access is a coalesced run.
+// With `half` (and X and dY ok): pairs of fp16 in place of the low parts, and no values.
+// The rows' ends behind the last image are written too then (0): what another form has left there meets zeros, but may read as Inf.
+template <bool PAIRS>
 __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__ dY, float* __restrict__ hi,
                                                        float* __restrict__ lo, float* __restrict__ plane_sums,
                                                        int planes, int channels, int mm, int og, int ch_tile,
-                                                       int tiles_per_group, int n_pad, size_t row_len) {
+                                                       int tiles_per_group, int n_pad, size_t row_len, const HalfScale* half) {
   pdl_wait();
+  const bool pairs = PAIRS && half_route(half, kHalfX, kHalfDy);
+  const float scale = pairs ? half[kHalfDy].scale : 1.f;
+  const int batch = planes / channels;
   // One warp per plane at a time in chunks of 256 elements, the next chunk's loads (of this plane or the warp's next one) in
   // flight while the current one is stored; no block-wide synchronisation.  One chunk at a time left planes of 169 elements at
   // 4.0 TB/s (CaffeNet conv3 at batch 256 50.0 -> 45.6 us, conv5 32.7 -> 30.5, conv2 at batch 32 11.7 -> 10.4; planes of 729 at batch 256
@@ -1588,7 +1280,7 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
   struct Place {
     const float* src;
     size_t at;   // in hi and lo
-    int i0, plane;
+    int i0, plane, end;  // end: mm, or for the last image the end of the row
   };
   auto place = [&](int turn) {
     Place q;
@@ -1599,6 +1291,7 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
     q.src = dY + (size_t)q.plane * mm;
     q.at = ((size_t)(grp * tiles_per_group + tile) * n_pad + within) * row_len + (size_t)b * mm;
     q.i0 = -(int)(((size_t)b * mm) & 31);
+    q.end = PAIRS && b + 1 == batch ? (int)(row_len - (size_t)b * mm) : mm;
     return q;
   };
   float x[8], y[8];
@@ -1614,7 +1307,7 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
   float sum = 0.f;
   for (int turn = warp0;;) {
     Place next = q;
-    const bool plane_ends = q.i0 + 256 >= mm;
+    const bool plane_ends = q.i0 + 256 >= q.end;
     if (plane_ends) {
       turn += nwarps;
       if (turn < planes) next = place(turn);
@@ -1626,10 +1319,14 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
     for (int u = 0; u < 8; ++u) {
       const int i = q.i0 + u * 32 + lane;
       uint32_t h, l;
-      split_tf32_trunc(x[u], h, l);
-      if (i >= 0 && i < mm) {
-        hi[q.at + i] = __uint_as_float(h);
-        lo[q.at + i] = __uint_as_float(l);
+      if (pairs) {
+        store_half_lane(lo + q.at + (i - lane), lane, x[u] * scale, i >= 0 && i < q.end);
+      } else {
+        split_tf32_trunc(x[u], h, l);
+        if (i >= 0 && i < q.end) {
+          hi[q.at + i] = __uint_as_float(h);
+          lo[q.at + i] = __uint_as_float(l);
+        }
       }
       sum += x[u];
     }
@@ -1649,11 +1346,13 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
 }
 
 // Forward B operand: [2 (hi, lo)][vg][n_pad][k_pad] <- W[o][Dg*k*k], zero padded.
+template <bool PAIRS>
 __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                 float* __restrict__ lo, int tiles_per_group, int og,
                                                                 int n_real, int n_pad, int k_real, int k_pad, int run,
-                                                                int window) {
+                                                                int window, const HalfScale* half) {
   pdl_wait();
+  const float scale = pack_scale<PAIRS>(half, kHalfX);
   const int vg = blockIdx.x / n_pad, j = blockIdx.x - vg * n_pad;
   const int ch = (vg % tiles_per_group) * n_real + j;  // inside the group
   const bool live = j < n_real && ch < og;
@@ -1666,9 +1365,13 @@ __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __r
     const int at = run == 1 ? kk : (chunk * kRun + (kk & (kRun - 1))) * window + (r - chunk * window), step = run == 1 ? 1 : window;
 #pragma unroll
     for (int e = 0; e < 4; ++e) v[e] = (live && kk + e < k_real) ? __ldg(src + at + e * step) : 0.f;
-    store_split4(hi, lo, row + kk, v);
+    store_split4<PAIRS>(hi, lo, row + kk, v, scale);
   }
 }
+
+size_t elements_x(const ConvGeom& G) { return (size_t)G.B * G.D * G.n * G.n; }
+size_t elements_y(const ConvGeom& G) { return (size_t)G.B * G.o * G.m * G.m; }
+size_t elements_w(const ConvGeom& G) { return (size_t)G.o * G.Dg * G.k * G.k; }
 
 int round_up(int v, int a) { return (v + a - 1) / a * a; }
 
@@ -1723,12 +1426,15 @@ bool two_ctas_per_sm(int n_pad, int taps_smem, int n_bias, int ptab, int* slots)
 // last round that is nearly empty (CaffeNet conv3 at batch 256: 2 x 338 units on 148 CTAs are five rounds, 3 x 338 half-width
 // ones on 296 are 3.4) asks for narrower tiles, a layer of few pixels (43 tiles at batch 32, 2 at batch 1) for narrower tiles
 // and splits.  A candidate has to win by 1 % and to keep its accumulation chain within `limit` (chain_limit).
+// `half`: the same for operands in pairs of fp16, from 503 measured combinations (layers of 48 to 384 channels, batch 16 to 256; 6 % rms): a
+// k-block of a tile of up to 128 columns is bound by its gather, so wide tiles are the better ones (CaffeNet conv3 at batch 256, 384
+// columns in three tiles 167 us, in two 150).
 struct GatherTiling {
   int tiles = 0, splits = 1, kps = 0;
   double us = 0.0;
 };
 GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, int channels, int cols_per_channel, int kblocks,
-                                  int run, int lane_stride, int n_bias, double limit) {
+                                  int run, int lane_stride, int n_bias, double limit, bool half) {
   GatherTiling best;
   const int t0 = channel_tiles(channels, cols_per_channel);
   for (int t = t0; t > 0 && t <= channels; ++t) {
@@ -1739,21 +1445,39 @@ GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, in
     const bool two = two_ctas_per_sm(n_pad, kblocks * kBlockK / run, n_bias, 0, &slots_unused);
     // a k-block of a CTA that shares its SM, of one that has the SM to itself, of the shape with one CTA per SM
     const double far = lane_stride > 2 ? 1.7 : 1.0;  // lanes 16 bytes and more apart: four wavefronts and more per load
-    const double shared = 2 * std::max(0.11 + 0.0028 * n_pad, (run > 1 ? 0.235 : 0.30) * far);
-    const double alone = std::max(0.19 + 0.0018 * n_pad, 0.27 * far), one = std::max(0.0035 * n_pad, 0.42 * far);
-    const double epilogue = 4.0 + 0.004 * n_pad;
+    const double shared = 2 * (half ? std::max(0.239 + 0.00055 * n_pad, (run > 1 ? 0.24 : 0.318) * far)
+                                    : std::max(0.11 + 0.0028 * n_pad, (run > 1 ? 0.235 : 0.30) * far));
+    const double alone = half ? (run > 1 ? 0.27 : 0.338) * far : std::max(0.19 + 0.0018 * n_pad, 0.27 * far);
+    const double one = half ? std::max(0.00197 * n_pad - 0.051, (run > 1 ? 0.249 : 0.311) * far) : std::max(0.0035 * n_pad, 0.42 * far);
+    const double epilogue = half ? 1.5 + 0.0149 * n_pad : 4.0 + 0.004 * n_pad, overlapped = half ? 0.89 : 0.4, start = half ? 6.8 : 2.6;
     for (int s = 1; s <= std::max(1, std::min(32, kblocks / 2)); ++s) {
       const int kps = (kblocks + s - 1) / s;
       if ((kblocks + kps - 1) / kps != s || kps * (n_pad <= kCrossCols ? 1.0 : 3.0) > limit) continue;
       const long long units = pixel_tiles * groups * t * s, slots = (long long)sms * (two ? 2 : 1), tail = units % slots;
-      double us = (double)(units / slots) * (kps * (two ? shared : one) + 0.4 * epilogue) +
-                  (tail ? kps * (!two ? one : tail > sms ? shared : alone) + epilogue : 0.6 * epilogue) + 2.6;
-      if (s > 1) us += 3.8 + units * 128.0 * n_pad * 4.0 * 0.18e-6;
+      double us = (double)(units / slots) * (kps * (two ? shared : one) + overlapped * epilogue) +
+                  (tail ? kps * (!two ? one : tail > sms ? shared : alone) + epilogue : (1 - overlapped) * epilogue) + start;
+      if (s > 1) us += (half ? 1.4 : 3.8) + units * 128.0 * n_pad * 4.0 * (half ? 0.284e-6 : 0.18e-6);
       if (!best.tiles || us < 0.99 * best.us) best = GatherTiling{t, s, kps, us};
     }
   }
   return best;
 }
+
+// What a launch of operand_scale_kernel over `elements` takes: 5.6 us for CaffeNet conv3's X and W at batch 32 (9 MB), 8.4 for X, dY and W
+// of conv4 (14 MB), 58 for those of conv2 at batch 256 (265 MB).
+// A contraction takes pairs of fp16 from kHalfMinUs on, if by the estimates (6 % rms) they save 1 - kHalfGain of it: operands that do not lie close
+// enough together pay for the look at them and gain nothing.
+constexpr double kHalfMinUs = 25.0, kHalfGain = 0.9;
+int wgrad_columns(const ConvGeom& G) {
+  int chain;
+  const int tiles = weight_grad_tiles(G.og, &chain);
+  return round_up((G.og + tiles - 1) / tiles, 16);
+}
+// The share of the weight gradient's time that pairs of fp16 save (by the gather kernel: at least 512 lowered rows).  More than 128 columns: conv3, conv4 at
+// batch 256 253 -> 165 us, 210 -> 138, at batch 32 44 -> 31; 128 columns, bound by the gather: conv2 425 -> 345, conv5 159 -> 138, at batch
+// 32 65 -> 62, 64 -> 128 channels 56 x 56 50 -> 45.
+double half_weight_gradient(int rows, int columns) { return rows < 512 ? 0.0 : columns > 128 ? 0.3 : columns > 96 ? 0.1 : 0.0; }
+double scales_us(double elements) { return 4.0 + 4.0 * elements / 4e6; }
 
 }  // namespace
 
@@ -1771,6 +1495,8 @@ struct GatherProblem {
   int taps_smem = -1;             // tap-table entries staged in shared memory (-1: k_pad)
   size_t map_k = 0;               // extent of the packed operand along the reduction (0: k_pad)
   size_t smem = 0;
+  bool half = false;              // HALF
+  int a_stages_half = 4, b_stages_half = 4, acc_bufs_half = 1;
   float* zero = nullptr;          // one 0.f, read by taps out of bounds
   bool inside = false;            // kInside
   bool one = false;               // ONE: the tiles of the whole batch are short and have a slot each, if no SMs are kept
@@ -1805,17 +1531,24 @@ struct UmmaPlan {
   MaskTap* wg_pix = nullptr;       // per pixel: offset of the tap origin, taps out of bounds (padded to splits * kps * 32)
   float* wg_plane_sums = nullptr;  // [batch][channel] sums of dY for the bias gradient
   int wg_splits = 1, wg_kps = 1, wg_mtiles = 1;
+  HalfScale* half = nullptr;       // scales of the operands, by kHalfX and so on
+  uint2* half_parts = nullptr;
+  uint32_t* half_ticket = nullptr;
   void* memory = nullptr;          // everything above that lives on the device (PlanMemory)
   size_t bytes = 0;
 };
 
 namespace {
 typedef void (*GatherKernel)(const GatherParams, const CUtensorMap);
-template <int MODE, bool ONE = false>
+template <int FORM, bool ONE = false>
 GatherKernel gather_kernel_of(const GatherProblem& gp) {
-  return gp.sets == 2 ? gather_conv_kernel<2, MODE, ONE> : gather_conv_kernel<4, MODE, ONE>;
+  return gp.sets == 2 ? gather_conv_kernel<2, FORM, ONE> : gather_conv_kernel<4, FORM, ONE>;
 }
-GatherKernel gather_kernel(const GatherProblem& gp, bool weight_grad, bool one) {
+GatherKernel gather_kernel(const GatherProblem& gp, bool weight_grad, bool one, bool half) {
+  if (half) {
+    if (weight_grad) return gather_kernel_of<kHalf + kWeightGrad>(gp);
+    return gp.run == kRun ? gather_kernel_of<kHalf + kByRun>(gp) : gather_kernel_of<kHalf + kByTap>(gp);
+  }
   if (weight_grad) return gather_kernel_of<kWeightGrad>(gp);
   if (gp.run == kRun) return one ? gather_kernel_of<kByRun, true>(gp) : gather_kernel_of<kByRun>(gp);
   if (gp.inside) return gather_kernel_of<kInside>(gp);
@@ -1906,7 +1639,10 @@ void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* d
 void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* db, int splits, int vgroups, int tiles_per_group,
                          int rows_pad, int n_real, int n_pad, int k_real, int og, int accumulate = 0,
                          const ReduceExtras& extras = ReduceExtras()) {
-  if (extras.pack.blocks || extras.bias.db)
+  if (extras.pack.half)
+    launch_wgrad_reduce<HalfExtras>(ctx, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate,
+                                    HalfExtras(extras));
+  else if (extras.pack.blocks || extras.bias.db)
     launch_wgrad_reduce<ReduceExtras>(ctx, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate,
                                       extras);
   else
@@ -1952,6 +1688,10 @@ void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias,
   if (two_ctas_per_sm(gp.n_pad, taps_smem, n_bias, ptab, &b_two)) {
     gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = acc <= 64 && !ptab ? 3 : 2; gp.b_stages = b_two;
   }
+  // As pairs of fp16: A slots of 32 columns, weight slots of half the size.
+  gp.acc_bufs_half = gp.sets == 4 && 2 * acc + 4 * 32 <= 512 ? 2 : 1;
+  gp.a_stages_half = std::min(4, (gp.tmem_cols - gp.acc_bufs_half * acc) / 32);
+  gp.b_stages_half = std::min(4, 2 * gp.b_stages);
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
   const int period = gp.splits == 1 ? gp.n / gp.ch_tile : 1;  // pixels of a stride period, which are columns, where they are stored as such
   gp.one = gp.taps_smem && !gp.inside && gp.split_k <= kOneKblocks * kBlockK && tiles <= (long long)sms * (gp.sets == 2 ? 2 : 1) &&
@@ -2000,8 +1740,15 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     f.run = G.Dg % kRun == 0 ? kRun : 1; f.run_stride = G.n * G.n;
     f.inside = f.run == 1 && G.p == 0;
     const long long pixel_tiles = ((long long)G.B * G.m * G.m + kTileM - 1) / kTileM;
-    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, f.run, G.s,
-                                                 G.bias ? G.o : 0, chain_limit(G.og, 1, f.k_pad / kBlockK));
+    auto tiling = [&](bool half) {
+      return choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, f.run, G.s, G.bias ? G.o : 0,
+                                  chain_limit(G.og, 1, f.k_pad / kBlockK), half);
+    };
+    GatherTiling tl = tiling(false);
+    // Pairs of fp16 where that makes up for a look at the operands.
+    const GatherTiling paired = tiling(true);
+    const bool half = tl.us > kHalfMinUs && !f.inside && paired.us + scales_us(elements_x(G) + elements_w(G)) < kHalfGain * tl.us;
+    if (half) tl = paired;
     f.tiles = tl.tiles;
     f.ch_tile = f.n = (G.og + f.tiles - 1) / f.tiles;
     f.n_pad = round_up(f.n, 16);
@@ -2023,9 +1770,11 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       mem.table(&f.cols, c);
       mem.table(&f.zero, std::vector<float>(1, 0.f));
       finish_problem(mem, f, G.g * f.tiles, G.bias ? G.o : 0, ctx->planning_sms(), pixel_tiles * G.g * f.tiles * f.splits);
+      f.half = half;
       if (f.splits > 1) sums = std::max(sums, (size_t)f.splits * G.g * f.tiles * f.n_pad * f.pix_pad);
     }
   }
+  bool wgrad_half = false;
   // ---- data gradient as a stride-1 gather over dY: one "super pixel" = an s x s block of input pixels; accumulator
   //      columns = (d, py, px), reduction = (oc, jy, jx) with jy, jx < ceil(k/s); depth-to-space in the epilogue.
   {
@@ -2040,8 +1789,19 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     const int ss = G.s * G.s;
     const long long pixel_tiles = ((long long)G.B * p->dgr_q * p->dgr_q + kTileM - 1) / kTileM;
     const int kblocks = round_up(d.k_real, kBlockK) / kBlockK;
-    const GatherTiling tl = choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.Dg, ss, kblocks, d.run, 1, 0,
-                                                 chain_limit(G.Dg, ss, kblocks));
+    auto tiling = [&](bool half) {
+      return choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.Dg, ss, kblocks, d.run, 1, 0, chain_limit(G.Dg, ss, kblocks), half);
+    };
+    GatherTiling tl = tiling(false);
+    // The two gradients share the look at dY: both in pairs of fp16, or one of them, or none.
+    const GatherTiling paired = tiling(true);
+    const double wgrad_us = 2.0 * elements_w(G) * G.B * G.m * G.m / 230e6, wgrad_saves = wgrad_us * half_weight_gradient(p->fwd.k_real, wgrad_columns(G));
+    const double dgrad_saves = tl.us - paired.us, dy = elements_y(G) + elements_w(G), x = elements_x(G);
+    const double best = std::max(dgrad_saves - scales_us(dy), std::max(wgrad_saves - scales_us(dy + x), dgrad_saves + wgrad_saves - scales_us(dy + x)));
+    const bool worth = best > (1 - kHalfGain) * (tl.us + wgrad_us) && tl.us + wgrad_us > kHalfMinUs;
+    const bool half = worth && dgrad_saves > 0;
+    wgrad_half = worth && wgrad_saves - scales_us(dy + x) + (half ? scales_us(dy) : 0) > 0;
+    if (half) tl = paired;
     d.k_pad = round_up(d.k_real, kBlockK);
     d.tiles = tl.tiles;
     d.ch_tile = (G.Dg + d.tiles - 1) / d.tiles;
@@ -2068,6 +1828,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       mem.table(&d.cols, c);
       mem.table(&d.zero, std::vector<float>(1, 0.f));
       finish_problem(mem, d, G.g * d.tiles, 0, ctx->planning_sms(), pixel_tiles * G.g * d.tiles * d.splits);
+      d.half = half;
       if (d.splits > 1) sums = std::max(sums, (size_t)d.splits * G.g * d.tiles * d.n_pad * d.pix_pad);
     }
   }
@@ -2213,8 +1974,14 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       }
     mem.table(&p->wg_pix, t);
     finish_problem(mem, w, vgroups, 0, ctx->planning_sms(), (long long)base_tiles * p->wg_splits);
+    w.half = wgrad_half;
     if (G.bias) mem.room(&p->wg_plane_sums, (size_t)G.B * G.o);
     sums = std::max(sums, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
+  }
+  if (p->fwd.half || p->dgr.half || p->wgp.half) {
+    mem.table(&p->half_ticket, std::vector<uint32_t>(1, 0u));
+    mem.room(&p->half, 3);
+    mem.room(&p->half_parts, (size_t)ctx->sm_count * kScaleBlocksPerSm);
   }
   float* sum_memory = nullptr;
   mem.room(&sum_memory, sums);
@@ -2231,7 +1998,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
   }
   // The kernels that this plan launches, and no others: each is one to load at its first use.
   for (const GatherProblem* gp : {&p->fwd, &p->dgr, &p->wgp})
-    if (rc == CCT_OK && gp->w) rc = set_smem(ctx, gather_kernel(*gp, gp == &p->wgp, gp->one), gather_smem_limit(*gp));
+    if (rc == CCT_OK && gp->w) rc = set_smem(ctx, gather_kernel(*gp, gp == &p->wgp, gp->one, gp->half), gather_smem_limit(*gp));
   if (rc == CCT_OK && !p->w_small && !p->wg_gather) rc = set_smem(ctx, short_wgrad_kernel(p), kSmemLimit);
   if (rc != CCT_OK) {
     umma_plan_destroy(ctx, p);
@@ -2266,13 +2033,15 @@ void fill_common(GatherParams& P, const GatherProblem& gp, cct_ctx* ctx, int vgr
   P.tmem_cols = gp.tmem_cols;
   P.n_bias = P.bias ? n_bias : 0;
   P.lo_row_offset = vgroups * gp.n_pad;
+  P.a_stages_half = gp.a_stages_half; P.b_stages_half = gp.b_stages_half; P.acc_bufs_half = gp.acc_bufs_half;
   P.status = ctx->status_dev;
 }
 
-PackDgrad pack_dgrad_job(const UmmaPlan* p, const float* W) {
+PackDgrad pack_dgrad_job(const UmmaPlan* p, const float* W, bool half) {
   const ConvGeom& G = p->G;
   const GatherProblem& d = p->dgr;
-  PackDgrad J{W, d.w, d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run, 0, 0};
+  PackDgrad J{W, d.w, d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run, 0, 0,
+               half ? p->half : nullptr};
   J.parts = (d.k_pad / 4 + kPackThreads - 1) / kPackThreads;
   J.blocks = G.g * d.tiles * d.n_pad * J.parts;
   return J;
@@ -2332,8 +2101,8 @@ bool small_together(cct_ctx* ctx, const UmmaPlan* p) {
 void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp, bool weight_grad = false) {
   const int slots = (gp.sets == 2 ? 2 : 1) * ctx->launch_sms();
   const bool one = gp.one && P.total_tiles <= slots;
-  const GatherKernel kernel = gather_kernel(gp, weight_grad, one);
-  if (gp.one && !one) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gather_smem_limit(gp));  // (or the launch fails)
+  const GatherKernel kernel = gather_kernel(gp, weight_grad, one, P.half != nullptr);
+  if ((gp.one && !one) || (gp.half && !P.half)) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gather_smem_limit(gp));  // (or the launch fails)
   launch_pdl(kernel, dim3(std::min(P.total_tiles, slots)), dim3(gather_threads(gp.sets)), gp.smem, ctx->stream, P, gp.map);
   if (P.splits > 1) {
     const int vgroups = P.total_tiles / (P.n_pix_tiles * P.splits), cols = P.n_pix_tiles * vgroups * P.n > 32 * ctx->sm_count ? 8 : 1;
@@ -2341,6 +2110,31 @@ void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp,
     launch_pdl(cols == 8 ? gather_reduce_kernel<8> : gather_reduce_kernel<1>, dim3((P.n_pix + 127) / 128, vgroups * col_tiles), dim3(128),
                0, ctx->stream, P, col_tiles);
   }
+}
+
+// The scales of a call's operands (a = null: not needed) in one launch.
+struct ScaleOf {
+  const float *a, *mask;
+  size_t n;
+  int slot, headroom;
+};
+void launch_scales(cct_ctx* ctx, const UmmaPlan* p, std::initializer_list<ScaleOf> operands) {
+  ScaleJobs J{};
+  J.out = p->half; J.parts = p->half_parts; J.ticket = p->half_ticket;
+  size_t total = 0;
+  for (const ScaleOf& o : operands) total += o.a ? o.n : 0;
+  const size_t blocks = (size_t)ctx->sm_count * kScaleBlocksPerSm - 3;  // rounded up for each of three
+  const size_t per_block = (std::max<size_t>(kScaleChunk, (total + blocks - 1) / blocks) + 1023) & ~(size_t)1023;
+  int grid = 0;
+  for (const ScaleOf& o : operands) {
+    if (!o.a) continue;
+    ScaleJob& job = J.job[J.jobs++];
+    job.a = o.a; job.mask = o.mask; job.n = o.n; job.per_block = per_block; job.slot = o.slot; job.headroom = o.headroom;
+    job.first = grid;
+    job.blocks = (int)((o.n + per_block - 1) / per_block);
+    grid += job.blocks;
+  }
+  launch_pdl(operand_scale_kernel, dim3(grid), dim3(kScaleThreads), 0, ctx->stream, J);
 }
 
 }  // namespace
@@ -2360,10 +2154,12 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
     CCT_CHECK_LAUNCH(ctx);
     return CCT_OK;
   }
+  const bool half = f.half && batch == 0;
   if (repack) {
     t->begin(4, ctx->stream);
-    launch_pdl(pack_fwd_kernel, pack_grid(vgroups * f.n_pad, f.k_pad), dim3(kPackThreads), 0, ctx->stream, W, f.w,
-               f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad, f.run, G.k * G.k);
+    if (half) launch_scales(ctx, p, {ScaleOf{X, nullptr, elements_x(G), kHalfX, 0}, ScaleOf{W, nullptr, elements_w(G), kHalfW, 0}});
+    launch_pdl(half ? pack_fwd_kernel<true> : pack_fwd_kernel<false>, pack_grid(vgroups * f.n_pad, f.k_pad), dim3(kPackThreads), 0, ctx->stream, W, f.w,
+               f.w + f.w_half, f.tiles, G.og, f.n, f.n_pad, f.k_real, f.k_pad, f.run, G.k * G.k, half ? p->half : nullptr);
     t->end(4, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   }
@@ -2383,6 +2179,7 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
   P.out_group_channels = G.og;
   P.relu = relu;
   fill_common(P, f, ctx, vgroups, G.o);
+  if (half) { P.half = p->half; P.half_gathered = kHalfX; P.half_packed = kHalfW; }
   t->begin(0, ctx->stream);
   launch_gather(ctx, P, f);
   t->end(0, ctx->stream);
@@ -2392,27 +2189,45 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
 
 bool umma_dy_rows(const UmmaPlan* p, DyRows* rows) {
   if (!p->wg_gather || !p->dgr_row_taps) return false;
-  *rows = DyRows{p->wgp.w, p->wgp.w_half, p->wgp.map_k, p->G.bias ? p->wg_plane_sums : nullptr, p->G.o};
+  *rows = DyRows{p->wgp.w, p->wgp.w_half, p->wgp.map_k, p->G.bias ? p->wg_plane_sums : nullptr, p->G.o, p->G.B,
+                 p->wgp.half ? p->half : nullptr};
   return true;
+}
+
+int umma_rows_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, size_t pooled) {
+  if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
+  if (!p->wgp.half && !p->dgr.half) return CCT_OK;
+  // an element is in up to four windows
+  launch_scales(ctx, p, {ScaleOf{X, nullptr, elements_x(p->G), kHalfX, 0}, ScaleOf{W, nullptr, elements_w(p->G), kHalfW, 0},
+                         ScaleOf{dP, P, pooled, kHalfDy, 2}});
+  CCT_CHECK_LAUNCH(ctx);
+  return CCT_OK;
 }
 
 namespace {
 int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t, const float* pack_W,
-                    SmallConv* with);
+                    SmallConv* with, bool half);
+int data_gradient(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, float* dX, PhaseTimer* t, int batch, bool repack, bool half);
 }
 
 int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dY, float* dX,
                        float* dW, float* db, PhaseTimer* t) {
   const ConvGeom& G = p->G;
-  const size_t nx = (size_t)G.B * G.D * G.n * G.n, ny = (size_t)G.B * G.o * G.m * G.m, nw = (size_t)G.o * G.Dg * G.k * G.k;
+  const size_t nx = elements_x(G), ny = elements_y(G), nw = elements_w(G);
   // Small layers: the data gradient goes with the weight gradient, unless one writes where the other reads.
   if (dX && p->w_small && p->dgr.small_ct && !t->enabled && apart(dX, nx, {{X, nx}, {dY, ny}, {dW, nw}, {db, G.o}}) &&
       apart(dW, nw, {{W, nw}, {dY, ny}}) && (!G.bias || apart(db, G.o, {{W, nw}, {dY, ny}}))) {
     SmallConv d = small_dgrad(G, dY, W, dX, G.B);
-    if (small_together(ctx, p)) return weight_gradient(ctx, p, X, dY, dW, db, t, nullptr, &d);
+    if (small_together(ctx, p)) return weight_gradient(ctx, p, X, dY, dW, db, t, nullptr, &d, false);
   }
-  int rc = umma_conv_wgrad(ctx, p, X, dY, dW, db, t, dX ? W : nullptr);
-  if (rc == CCT_OK && dX) rc = umma_conv_dgrad(ctx, p, W, dY, dX, t, 0, false);
+  if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
+  if (dY && (p->wgp.half || (p->dgr.half && dX))) {  // (else umma_rows_scales)
+    launch_scales(ctx, p, {ScaleOf{p->wgp.half ? X : nullptr, nullptr, nx, kHalfX, 0}, ScaleOf{p->dgr.half && dX ? W : nullptr, nullptr, nw, kHalfW, 0},
+                           ScaleOf{dY, nullptr, ny, kHalfDy, 0}});
+    CCT_CHECK_LAUNCH(ctx);
+  }
+  int rc = weight_gradient(ctx, p, X, dY, dW, db, t, dX ? W : nullptr, nullptr, true);
+  if (rc == CCT_OK && dX) rc = data_gradient(ctx, p, W, dY, dX, t, 0, false, true);
   return rc;
 }
 
@@ -2420,20 +2235,20 @@ int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W
 // gradient of a small layer, in the same launch.
 namespace {
 int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t, const float* pack_W,
-                    SmallConv* with) {
+                    SmallConv* with, bool half) {
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   const ConvGeom& G = p->G;
   ReduceExtras extras{};
-  if (pack_W && !p->dgr.small_ct) extras.pack = pack_dgrad_job(p, pack_W);
+  if (pack_W && !p->dgr.small_ct) extras.pack = pack_dgrad_job(p, pack_W, half && p->dgr.half);
   if (p->wg_gather) {
     struct { int tiles, n, n_pad, k_real; } f = {p->wt_tiles, p->wt_n, p->w_npad, p->fwd.k_real};
     GatherProblem& w = p->wgp;
     const int vgroups = G.g * f.tiles, mm = G.m * G.m;
     t->begin(1, ctx->stream);
     if (dY)  // (else the kernel that made it has written the rows)
-      launch_pdl(split_dy_kernel, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, 
+      launch_pdl(w.half ? split_dy_kernel<true> : split_dy_kernel<false>, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, 
         dY, w.w, w.w + w.w_half, G.bias ? p->wg_plane_sums : nullptr, G.B * G.o, G.o, mm, G.og, f.n, f.tiles,
-        f.n_pad, w.map_k);
+        f.n_pad, w.map_k, half && w.half ? p->half : nullptr);
     CCT_CHECK_LAUNCH(ctx);
     GatherParams P{};
     P.in = X; P.out = p->w_partial; P.bias = nullptr;
@@ -2444,6 +2259,7 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     P.wg_k = G.k; P.wg_kreal = f.k_real;
     fill_common(P, w, ctx, vgroups, 0);
     P.taps = p->wg_pix; P.cols = nullptr;
+    if (half && w.half) { P.half = p->half; P.half_gathered = kHalfX; P.half_packed = kHalfDy; P.half_row_offset = P.lo_row_offset; }
     P.total_tiles = p->wg_splits * vgroups * p->wg_mtiles;
     launch_gather(ctx, P, w, true);
     t->end(1, ctx->stream);
@@ -2505,12 +2321,18 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
 
 }  // namespace
 int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t, const float* pack_W) {
-  return weight_gradient(ctx, p, X, dY, dW, db, t, pack_W, nullptr);
+  return weight_gradient(ctx, p, X, dY, dW, db, t, pack_W, nullptr, false);
 }
 
-// Data gradient of the first `batch` images (0: all of them); `repack` rewrites the packed weights from W first.
+// Data gradient of the first `batch` images (0: all of them); `repack` rewrites the packed weights from W first; `half`: the scales are
+// those of this call's operands.
 int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, float* dX, PhaseTimer* t, int batch,
                     bool repack) {
+  return data_gradient(ctx, p, W, dY, dX, t, batch, repack, false);
+}
+namespace {
+int data_gradient(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, float* dX, PhaseTimer* t, int batch,
+                  bool repack, bool half) {
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   const ConvGeom& G = p->G;
   const int B = batch > 0 ? batch : G.B;
@@ -2526,7 +2348,7 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
       return CCT_OK;
     }
     if (repack) {
-      const PackDgrad J = pack_dgrad_job(p, W);
+      const PackDgrad J = pack_dgrad_job(p, W, half);
       launch_pdl(pack_dgrad_kernel, dim3(J.blocks), dim3(kPackThreads), 0, ctx->stream, J);
       CCT_CHECK_LAUNCH(ctx);
     }
@@ -2555,12 +2377,14 @@ int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, 
       P.taps = p->dgr_row_taps;
       P.run_stride = (int)p->wgp.map_k;
     }
+    if (half && d.half) { P.half = p->half; P.half_gathered = kHalfDy; P.half_packed = kHalfW; }
     launch_gather(ctx, P, d);
     t->end(3, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   }
   return CCT_OK;
 }
+}  // namespace
 
 // ------------------------------------------------------------------ weight gradient without any allocation
 // Scratch for cct_conv_weight_grad_noalloc: the lowered-matrix row table followed by the split partial sums.  It is a

@@ -392,7 +392,9 @@ constexpr size_t kPool32SmemCap = 64 * 1024, kPool32RowsSmem = 28 * 1024;
 // more: CaffeNet conv2 at batch 256 66 + 102 us, this 118; conv5 21 + 31, this 30; at batch 32 10.6 + 11.1, this 17.8.  With two
 // stores per element it pays to turn the planes in shared memory, so that a warp stores whole lines (157 us straight from the 2 x 2
 // blocks), and to keep a block's planes few (28 KB; 36 KB 119 us, 56 KB 123).
-template <bool RELU, bool ROWS>
+// kRowsHalf: rows that are pairs of fp16 where their scales say so, two elements per lane and step.
+enum { kNoRows = 0, kRows = 1, kRowsHalf = 2 };
+template <bool RELU, int ROWS>
 __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
     const float* __restrict__ A, const int32_t* __restrict__ idx, const float* __restrict__ dP, const float* __restrict__ P,
     float* __restrict__ dA, int planes, int n, int m, int half, uint32_t inv_half, int strips, uint32_t inv_strips, int group, int vec_ok,
@@ -404,6 +406,8 @@ __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
   int32_t* s_idx = reinterpret_cast<int32_t*>(pool32_smem);
   float* s_g = pool32_smem + in_pad;
   float* s_out = s_g + in_pad;  // ROWS: the planes, on their way out
+  const bool pairs = ROWS == kRowsHalf && half_route(rows.half, kHalfX, kHalfDy);
+  const float scale = pairs ? rows.half[kHalfDy].scale : 1.f;
   for (int g0 = blockIdx.x * group; g0 < planes; g0 += gridDim.x * group) {
     const int cnt = min(group, planes - g0);
     const size_t in_base = (size_t)g0 * mm;
@@ -498,15 +502,29 @@ __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
         float* hi = rows.rows + (size_t)(plane - b * rows.channels) * rows.row_len + (size_t)b * nn;
         const float* src = s_out + pl * nn;
         float sum = 0.f;
-#pragma unroll 4
-        for (int i = lane - (int)(((size_t)b * nn) & 31); i < nn; i += 32) {
-          const float x = i >= 0 ? src[i] : 0.f;
-          const float l = x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-          if (i >= 0) {
-            hi[i] = x;
-            hi[rows.lo + i] = l;
+        const int end = ROWS == kRowsHalf && (int)b + 1 == rows.batch ? (int)(rows.row_len - (size_t)b * nn) : nn;  // as split_dy_kernel: zeros behind the last image
+        const int i0 = -(int)(((size_t)b * nn) & 31);
+        if (pairs) {
+          const int j0 = -(int)(((size_t)b * nn) & 63);  // (a row's start is 32 floats into a block of 64 or at it: its own is never crossed)
+#pragma unroll 2
+          for (int j = j0; j < end; j += 64) {
+            const int i = j + 2 * lane;
+            const float x0 = i >= 0 && i < nn ? src[i] : 0.f, x1 = i + 1 >= 0 && i + 1 < nn ? src[i + 1] : 0.f;
+            store_half_pair(hi + i, hi + rows.lo + i, x0, x1, scale, i >= 0 && i < end, i + 1 >= 0 && i + 1 < end, (lane & 15) * 2);
+            sum += x0;
+            sum += x1;
           }
-          sum += x;
+        } else {
+#pragma unroll 4
+          for (int i = i0 + lane; i < end; i += 32) {
+            const float x = i >= 0 && i < nn ? src[i] : 0.f;
+            const float l = x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
+            if (i >= 0) {
+              hi[i] = x;
+              hi[rows.lo + i] = l;
+            }
+            sum += x;
+          }
         }
         if (rows.plane_sums) {
 #pragma unroll
@@ -562,7 +580,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_2x2_kernel(const float* __res
 }
 
 // The kernel for windows of 3x3 with stride 2; false if a group of planes does not fit.
-template <bool RELU, bool ROWS>
+template <bool RELU, int ROWS>
 int launch_maxpool_bwd_3x3s2(cct_ctx* ctx, const float* A, const int32_t* idx, const float* dP, const float* P, float* dA, int planes, int n,
                              int m, const DyRows& rows, bool* fits) {
   // Planes per block: a multiple of four, so that every group starts on a 16-byte boundary of the pooled tensors.
@@ -593,7 +611,7 @@ int launch_maxpool_bwd(cct_ctx* ctx, const float* A, const int32_t* idx, const f
   const int half = (n + 1) / 2;
   if (k == 3 && s == 2) {
     bool fits = false;
-    const int rc = launch_maxpool_bwd_3x3s2<RELU, false>(ctx, A, idx, dP, P, dA, planes, n, m, DyRows(), &fits);
+    const int rc = launch_maxpool_bwd_3x3s2<RELU, kNoRows>(ctx, A, idx, dP, P, dA, planes, n, m, DyRows(), &fits);
     if (rc != CCT_OK || fits) return rc;
   }
   const long long items = (long long)planes * half * half;
@@ -653,7 +671,8 @@ int pool_relu_backward_rows(cct_ctx* ctx, const float* P, const int32_t* idx, co
   if (k != 3 || s != 2) return CCT_ERR_UNSUPPORTED;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
   bool fits = false;
-  const int rc = launch_maxpool_bwd_3x3s2<false, true>(ctx, nullptr, idx, dP, P, out.rows, planes, n, (n - k) / s + 1, out, &fits);
+  const int rc = out.half ? launch_maxpool_bwd_3x3s2<false, kRowsHalf>(ctx, nullptr, idx, dP, P, out.rows, planes, n, (n - k) / s + 1, out, &fits)
+                          : launch_maxpool_bwd_3x3s2<false, kRows>(ctx, nullptr, idx, dP, P, out.rows, planes, n, (n - k) / s + 1, out, &fits);
   if (rc != CCT_OK) return rc;
   if (!fits) return CCT_ERR_UNSUPPORTED;
   CCT_CHECK_LAUNCH(ctx);

@@ -1,0 +1,68 @@
+// Operands as pairs of fp16: the scale of one, the split, and the layout of their rows in memory.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+// How one operand of a contraction is split into pairs of fp16, decided on the device at each call (operand_scale.cuh): `scale`, a
+// power of two, brings its largest value to [2^14, 2^15), `inverse` takes it back; `ok`: its values lie close enough together.
+struct alignas(16) HalfScale {
+  float scale, inverse;
+  int ok, pad;
+};
+enum { kHalfX = 0, kHalfW = 1, kHalfDy = 2 };
+
+// Where a row of pairs of fp16 has its elements: of each 32 in a row the hi halves in words 0 - 15, the lo halves in words 16 - 31, so that
+// 32 of the reduction are one 128-byte line.  Element i's word of hi halves; its lo halves are kHalfLo words on.
+constexpr int kHalfLo = 16;
+__host__ __device__ inline size_t half_word(size_t i) { return (i & ~(size_t)31) + ((i & 31) >> 1); }
+
+// Two values as pairs of fp16 (the first in the low half): hi = the value cut to fp16's 11 bits, lo = the rest rounded to 11 bits.
+// The values are scaled so that they lie in fp16's range (operand_scale.cuh); those below 2^-14 lose places of hi to lo.
+__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
+  uint32_t r;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+__device__ __forceinline__ void split_half2(float a, float b, uint32_t& hi, uint32_t& lo) {
+  const float ha = __uint_as_float(__float_as_uint(a) & 0xFFFFE000u), hb = __uint_as_float(__float_as_uint(b) & 0xFFFFE000u);
+  hi = pack_half2(ha, hb);
+  lo = pack_half2(a - ha, b - hb);
+}
+// Whether operands `a` and `b` of a plan's scales (null: none) are both split into pairs of fp16.
+__device__ __forceinline__ bool half_route(const HalfScale* half, int a, int b) { return half && half[a].ok && half[b].ok; }
+
+// A warp writes up to 32 elements of such a row, lane = element of the 32 at `block`: pairs of lanes share a word, except where only one of
+// them is `in` (the ends of an image whose size is odd).
+__device__ __forceinline__ void store_half_lane(float* block, int lane, float v, bool in) {
+  const bool odd = lane & 1;
+  const float other = __shfl_xor_sync(0xffffffffu, v, 1);
+  const bool both = __shfl_xor_sync(0xffffffffu, in ? 1 : 0, 1) && in;
+  uint32_t h, l;
+  split_half2(odd ? other : v, odd ? v : other, h, l);
+  if (both) {
+    reinterpret_cast<uint32_t*>(block)[(lane >> 1) + (odd ? kHalfLo : 0)] = odd ? l : h;
+  } else if (in) {
+    uint16_t* at = reinterpret_cast<uint16_t*>(block) + lane;
+    at[0] = (uint16_t)(odd ? h >> 16 : h);
+    at[2 * kHalfLo] = (uint16_t)(odd ? l >> 16 : l);
+  }
+}
+
+// Two consecutive elements, the first at an even place: the values to `value`, their halves into the row at `low` (both at the first element;
+// `within`: its place in its 32).
+__device__ __forceinline__ void store_half_pair(float* value, float* low, float x0, float x1, float scale, bool in0, bool in1, int within) {
+  uint32_t h, l;
+  split_half2(x0 * scale, x1 * scale, h, l);
+  uint32_t* word = reinterpret_cast<uint32_t*>(low - within) + (within >> 1);
+  if (in0 && in1) {
+    *reinterpret_cast<float2*>(value) = make_float2(x0, x1);
+    word[0] = h;
+    word[kHalfLo] = l;
+  } else if (in0 || in1) {
+    const int which = in0 ? 0 : 1;
+    value[which] = in0 ? x0 : x1;
+    uint16_t* at = reinterpret_cast<uint16_t*>(word) + which;
+    at[0] = (uint16_t)(in0 ? h : h >> 16);
+    at[2 * kHalfLo] = (uint16_t)(in0 ? l : l >> 16);
+  }
+}

@@ -35,7 +35,9 @@ enum {
 enum {
   CCT_ALGO_AUTO = 0,       /* tcgen05 3xTF32 where the shape allows, else SIMT fp32 */
   CCT_ALGO_SIMT_FP32 = 1,  /* direct convolution in fp32 FMA (exact fp32 products) */
-  CCT_ALGO_UMMA_3XTF32 = 2 /* implicit GEMM on tcgen05/TMEM, each operand split hi+lo in TF32, 3 MMAs */
+  CCT_ALGO_UMMA_3XTF32 = 2 /* implicit GEMM on tcgen05/TMEM, each operand split hi+lo, 3 MMAs: in TF32, or in larger
+                            * contractions in FP16 (22 bits as well) after a power of two that each call finds for each
+                            * operand, if its values lie close enough together for that: an error of 2^-40 of the largest */
 };
 
 typedef struct cct_ctx cct_ctx;
@@ -126,7 +128,8 @@ int cct_conv_backward(cct_conv_plan* plan, const float* X, const float* W, const
  *     int32 indices cct_maxpool_forward wrote, dP = gradient of the pooled tensor.  One HBM-bound pass into
  *     plan-owned scratch (cct_conv_plan_reserve_fusion) feeds both gradient kernels.  If P, the pooled tensor
  *     cct_maxpool_forward wrote, is given as well (or instead of A), the sign is taken from it - the element a window
- *     points at holds that window's maximum, so the result is bit-identical - and A, (m / pooled size)^2 times larger,
+ *     points at holds that window's maximum, so the result is the same (bit for bit, where
+ *     the gradients are not split in FP16) - and A, (m / pooled size)^2 times larger,
  *     is not read.
  *   - Input side.  relu_mask_dx != 0 writes dX * [X > 0] instead of dX: the ReLU bridge in front of this layer (whose
  *     output X is), applied by one streaming pass right behind the data-gradient kernel.
