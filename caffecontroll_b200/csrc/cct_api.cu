@@ -565,7 +565,7 @@ int cct_conv_backward_fused(cct_conv_plan* plan, const float* X, const float* W,
     if (f->P && plan->algo == CCT_ALGO_UMMA_3XTF32 && umma_dy_rows(plan->umma, &rows)) {
       // straight into the form the contractions read
       const int pooled = (G.m - f->pool_k) / f->pool_s + 1;
-      int rc = umma_rows_scales(ctx, plan->umma, X, W, f->dP, f->P, (size_t)G.B * G.o * pooled * pooled);
+      int rc = umma_rows_scales(ctx, plan->umma, X, W, f->dP, f->P, f->idx, pooled);
       if (rc == CCT_OK) rc = pool_relu_backward_rows(ctx, f->P, f->idx, f->dP, rows, G.B * G.o, G.m, f->pool_k, f->pool_s);
       if (rc == CCT_OK) rc = umma_conv_backward(ctx, plan->umma, X, W, nullptr, dX, dW, db, &plan->timer);
       if (rc == CCT_OK && f->relu_mask_dx && dX) rc = cct_relu_backward(ctx, X, dX, dX, (size_t)G.B * G.D * G.n * G.n);

@@ -187,7 +187,7 @@ struct DyRows {
   size_t lo = 0, row_len = 0;
   float* plane_sums = nullptr;
   int channels = 0, batch = 0;
-  const HalfScale* half = nullptr;  // set, and X and dY ok: pairs of fp16 of scaled dY in place of the low parts (half_word)
+  const HalfScales* half = nullptr;  // set, and X and dY ok: pairs of fp16 of scaled dY in place of the low parts (half_word)
 };
 struct UmmaPlan;  // opaque: tables, packed weights, split-K scratch
 // `tensor_only`: every pass on the tensor cores, however small the layer (CCT_ALGO_UMMA_3XTF32 by name); otherwise small
@@ -206,7 +206,7 @@ int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W
 // Whether umma_conv_backward takes dY in the form of `rows` (then dY = null), written there by the kernel that makes it;
 // umma_rows_scales comes before that kernel: dY is what a 3x3 / stride 2 pooling of P's windows makes of dP.
 bool umma_dy_rows(const UmmaPlan* p, DyRows* rows);
-int umma_rows_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, size_t pooled);
+int umma_rows_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, const int32_t* idx, int pooled);
 int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t,
                     const float* pack_W = nullptr);
 int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, float* dX, PhaseTimer* t, int batch,

@@ -185,14 +185,22 @@ struct GatherParams {
   int wg_k, wg_kreal;         // kernel size, real rows of the lowered matrix
   // HALF: the scales of the plan's operands, which two of them this contraction has (gathered, packed), the first row of the packed
   // operand in pairs of fp16, and the stages that there is room for then.
-  const HalfScale* half;
-  int half_gathered, half_packed, half_row_offset;
-  int a_stages_half, b_stages_half, acc_bufs_half;
+  const HalfScales* half;
+  int half_row_offset;
+  uint16_t acc_cols_half;
+  uint8_t half_gathered, half_packed, a_stages_half, b_stages_half, acc_bufs_half;
+  uint8_t taps_x;             // taps along a row (taps_per_axis: along a column)
+  // A data gradient by tall blocks of pixels is two launches, of which one returns at once: kOnlyHalf takes the tall blocks in pairs of fp16, kOnlyTf32
+  // the others.  `bad_geom`: the layer, for values that are not finite.
+  uint8_t only;
+  struct { uint8_t kernel, stride; short pad, size; int channels, group_channels; } bad_geom;
   int taps_smem;              // entries of `taps` staged in shared memory (0 in weight-gradient mode)
   const float* zero;          // kByRun: what lanes whose tap is out of bounds read
   int run_stride;             // kByRun: elements between consecutive channels of the gathered tensor
   int* status;
 };
+
+enum { kAny = 0, kOnlyHalf = 1, kOnlyTf32 = 2 };
 
 // Which tile a persistent CTA works on: channel tile, pixel tile (or M-tile), first k-block, split.
 struct TileId {
@@ -240,7 +248,8 @@ __host__ __device__ inline GatherSmem gather_smem(int n_pad, int k_pad, int b_st
 // whose windows lie inside the plane: 5.3 instructions per value instead of 9, AlexNet conv1 at batch 256 320 -> 293 us.  (Entries
 // behind the last real index read the window's first element against a weight of zero; lanes behind the last pixel read the last
 // pixel's window, their columns are not stored.)
-enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3, kHalf = 4 };  // FORM: one of the first four, + kHalf (HALF)
+// FORM: one of these, + kHalf (HALF), + kTall (with it: tall blocks of pixels, GatherProblem::rows)
+enum { kByTap = 0, kByRun = 1, kWeightGrad = 2, kInside = 3, kHalf = 4, kTall = 8 };
 // ONE: every CTA has one tile, a short one (kOneKblocks).  There is no next tile then for the epilogue to overlap with, and the producers,
 // who are through, take their share of its columns (six chunks of 16 took four warps 1.2 us); in front of the first k-block stood three
 // trips to L2 for the tables and the bias, one behind the other, and the allocation of tensor memory (1.3 us in all), now one trip
@@ -262,7 +271,7 @@ template <int SETS, int FORM, bool ONE>
 __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     gather_conv_kernel(const __grid_constant__ GatherParams P, const __grid_constant__ CUtensorMap w_map) {
   constexpr int MODE = FORM % kHalf;
-  constexpr bool HALF = FORM >= kHalf;
+  constexpr bool HALF = FORM >= kHalf, TALL = FORM >= kTall;
   constexpr int kProducerWarps = 4 * SETS, kMmaWarp = kProducerWarps, kTmaWarp = kMmaWarp + 1;
   constexpr int kGatherThreads = gather_threads(SETS);
   extern __shared__ uint8_t smem_raw[];
@@ -282,9 +291,13 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   float* s_bias = reinterpret_cast<float*>(base_ptr + L.bias_off);
   const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
 
-  // HALF: the gathered operand's scale (0: tf32 instead) and what takes both operands' scales back
+  // HALF: the gathered operand's scale (0: tf32 instead), what takes both operands' scales back, how many values are not finite
   float* s_scale = reinterpret_cast<float*>(base_ptr + (tmem_slot + 4 - base));
   int* s_offsets = reinterpret_cast<int*>(s_taps);  // kInside: the offsets alone
+  if (HALF && P.only != kAny) {
+    pdl_wait();
+    if (tall_route(P.half) != (P.only == kOnlyHalf)) return;
+  }
   auto init_barriers = [&]() {
     for (int s = 0; s < kMaxAStages; ++s) { mbar_init(ready_bar + 8u * s, 5); mbar_init(done_bar + 8u * s, 1); }  // 4 producer warps + the TMA thread
     for (int s = 0; s < kMaxAccBufs; ++s) { mbar_init(acc_full + 8u * s, 1); mbar_init(acc_empty + 8u * s, kEpiWarps); }
@@ -320,9 +333,10 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
     pdl_wait();  // so far the plan's tables alone have been read: set-up beside the end of the kernel before (15.6 -> 15.35 us for conv3 of one image)
     for (int i = tid; i < P.n_bias + kBiasPad; i += kGatherThreads) s_bias[i] = i < P.n_bias ? P.bias[i] : 0.f;
     if (HALF && tid == 0) {
-      const HalfScale a = P.half[P.half_gathered], b = P.half[P.half_packed];
-      s_scale[0] = a.ok && b.ok ? a.scale : 0.f;
+      const HalfScale a = P.half->of[P.half_gathered], b = P.half->of[P.half_packed];
+      s_scale[0] = a.ok && b.ok && P.only != kOnlyTf32 ? a.scale : 0.f;
       s_scale[1] = a.inverse * b.inverse;
+      reinterpret_cast<int*>(s_scale)[2] = a.bad;
     }
   }
   tc_fence_before();
@@ -337,8 +351,9 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
   // <2, kWeightGrad> spilled (CaffeNet conv2's weight gradient 332 -> 372 us); as a function or a lambda the kernels of single tiles
   // came out with more registers (37 images of 50 -> 75 channels both ways 35.0 -> 36.4).
   if constexpr (HALF) {
-    if (s_scale[0] != 0.f) {
+    if (TALL || s_scale[0] != 0.f) {
       constexpr bool half = true;
+      const uint32_t acc_cols = (uint32_t)P.acc_cols_half, cross = acc_cols - (uint32_t)P.n_pad;
 #include "gather_roles.inc"
     } else {
       constexpr bool half = false;
@@ -358,9 +373,11 @@ __global__ void __launch_bounds__(gather_threads(SETS), SETS == 2 ? 2 : 1)
 // there are plenty of pixels (one decode of the pixel for eight columns: CaffeNet conv5 at batch 32, 11 MB of L2-resident
 // sums, 14 -> 6 us against one column per thread), one where there are few and the splits' loads have to be in flight
 // together (conv3 of one image, 12 splits: 8 -> 4 us against eight).
-template <int COLS>
+// ONLY: returns at once where the data gradient has gone by tall blocks.
+template <int COLS, bool ONLY>
 __global__ void __launch_bounds__(128) gather_reduce_kernel(const __grid_constant__ GatherParams P, int col_tiles) {
   pdl_wait();
+  if (ONLY && tall_route(P.half)) return;
   const int pix = blockIdx.x * 128 + threadIdx.x;
   const int vg = blockIdx.y / col_tiles, col0 = (blockIdx.y - vg * col_tiles) * COLS, vgroups = gridDim.y / col_tiles;
   const int grp = vg / P.tiles_per_group, ntile = vg - grp * P.tiles_per_group;
@@ -1069,23 +1086,27 @@ struct PackDgrad {
   int tiles_per_group, og, Dg, k, s, taps, d_tile, n_real, n_pad, k_real, k_pad, run;
   int parts;   // blocks per row
   int blocks;  // rows * parts
-  const HalfScale* half;  // null: no data gradient by pairs of fp16
+  const HalfScales* half;  // null: no data gradient by pairs of fp16
+  int rows = 1;            // stride periods of a block of pixels along a column (GatherProblem)
+  int only = kAny;
 };
 // The scale of weights that are packed as pairs of fp16 for a contraction with operand `other`, or 0.  (PAIRS, here and in the kernels below: a
 // plan without them takes kernels without that code, whose registers the small ones would feel.)
 template <bool PAIRS>
-__device__ __forceinline__ float pack_scale(const HalfScale* half, int other) {
-  return PAIRS && half_route(half, other, kHalfW) ? half[kHalfW].scale : 0.f;
+__device__ __forceinline__ float pack_scale(const HalfScales* half, int other) {
+  return PAIRS && half_route(half, other, kHalfW) ? half->of[kHalfW].scale : 0.f;
 }
 template <bool PAIRS>
 __device__ __forceinline__ void pack_dgrad_block(const PackDgrad& J, int block) {
+  if (PAIRS && J.only != kAny && tall_route(J.half) != (J.only == kOnlyHalf)) return;
+  const int periods = PAIRS ? J.rows : 1;
   const int r0 = block / J.parts, part = block - r0 * J.parts;
   const int vg = r0 / J.n_pad, j = r0 - vg * J.n_pad;
-  const int grp = vg / J.tiles_per_group, d = (vg - grp * J.tiles_per_group) * J.d_tile + j / (J.s * J.s);
-  const int py = (j / J.s) % J.s, px = j % J.s, window = J.taps * J.taps;
+  const int grp = vg / J.tiles_per_group, d = (vg - grp * J.tiles_per_group) * J.d_tile + j / (periods * J.s * J.s);
+  const int py = (j / J.s) % (periods * J.s) - (periods - 1) * J.s, px = j % J.s, window = (J.taps + periods - 1) * J.taps;
   const bool live = j < J.n_real && d < J.Dg;
   const float* src = J.W + ((size_t)grp * J.og * J.Dg + d) * J.k * J.k;
-  const float scale = pack_scale<PAIRS>(J.half, kHalfDy);
+  const float scale = PAIRS && J.only == kOnlyTf32 ? 0.f : pack_scale<PAIRS>(J.half, kHalfDy);
   const size_t row = (size_t)r0 * J.k_pad;
   for (int kk = (part * (int)blockDim.x + (int)threadIdx.x) * 4; kk < J.k_pad; kk += J.parts * (int)blockDim.x * 4) {
     // reduction index -> (filter / run, jy, jx, filter % run); four in a row are four filters of one tap where run is kRun, and
@@ -1095,7 +1116,7 @@ __device__ __forceinline__ void pack_dgrad_block(const PackDgrad& J, int block) 
     if (J.run == kRun) {
       const int r = kk / kRun, chunk = r / window, tap = r - chunk * window;
       const int jy = tap / J.taps, kr = py + jy * J.s, kc = px + (tap - jy * J.taps) * J.s;
-      const bool in = live && kk < J.k_real && kr < J.k && kc < J.k;
+      const bool in = live && kk < J.k_real && (!PAIRS || kr >= 0) && kr < J.k && kc < J.k;
       const float* at = src + (size_t)(chunk * kRun + (kk & (kRun - 1))) * filter + kr * J.k + kc;
 #pragma unroll
       for (int e = 0; e < 4; ++e) v[e] = in ? __ldg(at + e * filter) : 0.f;
@@ -1104,7 +1125,7 @@ __device__ __forceinline__ void pack_dgrad_block(const PackDgrad& J, int block) 
       for (int e = 0; e < 4; ++e) {
         const int oc = (kk + e) / window, tap = kk + e - oc * window, jy = tap / J.taps;
         const int kr = py + jy * J.s, kc = px + (tap - jy * J.taps) * J.s;
-        v[e] = (live && kk + e < J.k_real && kr < J.k && kc < J.k) ? __ldg(src + oc * filter + kr * J.k + kc) : 0.f;
+        v[e] = (live && kk + e < J.k_real && (!PAIRS || kr >= 0) && kr < J.k && kc < J.k) ? __ldg(src + oc * filter + kr * J.k + kc) : 0.f;
       }
     }
     store_split4<PAIRS>(J.hi, J.lo, row + kk, v, scale);
@@ -1141,8 +1162,8 @@ struct ReduceExtras {
   PackDgrad pack;
   BiasSum bias;
 };
-struct HalfExtras : ReduceExtras {  // pairs of fp16
-  explicit HalfExtras(const ReduceExtras& e) : ReduceExtras(e) {}
+struct HalfExtras : ReduceExtras {  // pairs of fp16; `tall`: the weights for tall blocks of pixels, if the data gradient has them
+  PackDgrad tall;
 };
 // True if this block was one of them; `first` of the grid's x are not.
 template <bool PAIRS>
@@ -1161,7 +1182,13 @@ __device__ __forceinline__ bool extra_block_of(const ReduceExtras& E, int first)
 // of 10 images, two such reductions of 4 us in its iteration, took 88.0 us instead of 86.2.
 struct NoExtras {};
 __device__ __forceinline__ bool extra_block(const ReduceExtras& E, int first) { return extra_block_of<false>(E, first); }
-__device__ __forceinline__ bool extra_block(const HalfExtras& E, int first) { return extra_block_of<true>(E, first); }
+__device__ __forceinline__ bool extra_block(const HalfExtras& E, int first) {
+  const int block = (int)blockIdx.x - first;
+  if (block < 0) return false;
+  if (block < E.tall.blocks) pack_dgrad_block<true>(E.tall, block);
+  else extra_block_of<true>(E, first + E.tall.blocks);
+  return true;
+}
 __device__ __forceinline__ bool extra_block(const NoExtras&, int) { return false; }
 
 // dW[o][kk] and db[o] from the split partial sums, added in split order (deterministic).  One block per 32 x 32
@@ -1262,10 +1289,10 @@ template <bool PAIRS>
 __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__ dY, float* __restrict__ hi,
                                                        float* __restrict__ lo, float* __restrict__ plane_sums,
                                                        int planes, int channels, int mm, int og, int ch_tile,
-                                                       int tiles_per_group, int n_pad, size_t row_len, const HalfScale* half) {
+                                                       int tiles_per_group, int n_pad, size_t row_len, const HalfScales* half) {
   pdl_wait();
   const bool pairs = PAIRS && half_route(half, kHalfX, kHalfDy);
-  const float scale = pairs ? half[kHalfDy].scale : 1.f;
+  const float scale = pairs ? half->of[kHalfDy].scale : 1.f;
   const int batch = planes / channels;
   // One warp per plane at a time in chunks of 256 elements, the next chunk's loads (of this plane or the warp's next one) in
   // flight while the current one is stored; no block-wide synchronisation.  One chunk at a time left planes of 169 elements at
@@ -1350,7 +1377,7 @@ template <bool PAIRS>
 __global__ void __launch_bounds__(kPackThreads) pack_fwd_kernel(const float* __restrict__ W, float* __restrict__ hi,
                                                                 float* __restrict__ lo, int tiles_per_group, int og,
                                                                 int n_real, int n_pad, int k_real, int k_pad, int run,
-                                                                int window, const HalfScale* half) {
+                                                                int window, const HalfScales* half) {
   pdl_wait();
   const float scale = pack_scale<PAIRS>(half, kHalfX);
   const int vg = blockIdx.x / n_pad, j = blockIdx.x - vg * n_pad;
@@ -1426,15 +1453,18 @@ bool two_ctas_per_sm(int n_pad, int taps_smem, int n_bias, int ptab, int* slots)
 // last round that is nearly empty (CaffeNet conv3 at batch 256: 2 x 338 units on 148 CTAs are five rounds, 3 x 338 half-width
 // ones on 296 are 3.4) asks for narrower tiles, a layer of few pixels (43 tiles at batch 32, 2 at batch 1) for narrower tiles
 // and splits.  A candidate has to win by 1 % and to keep its accumulation chain within `limit` (chain_limit).
-// `half`: the same for operands in pairs of fp16, from 503 measured combinations (layers of 48 to 384 channels, batch 16 to 256; 6 % rms): a
+// `half`: the same for operands in pairs of fp16, from 654 measured combinations (layers of 20 to 384 channels, batch 16 to 256; 6 % rms): a
 // k-block of a tile of up to 128 columns is bound by its gather, so wide tiles are the better ones (CaffeNet conv3 at batch 256, 384
-// columns in three tiles 167 us, in two 150).
+// columns in three tiles 167 us, in two 150); an MMA of more takes the time of the next multiple of 64.
 struct GatherTiling {
   int tiles = 0, splits = 1, kps = 0;
   double us = 0.0;
+  double chain = 0.0;  // additions at full magnitude, a quarter of them: one per eight products or three (chain_limit); pairs of fp16 have half as many
+  bool cross = false;  // pairs of fp16: a second accumulator for the cross terms
 };
 GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, int channels, int cols_per_channel, int kblocks,
-                                  int run, int lane_stride, int n_bias, double limit, bool half) {
+                                  int run, int lane_stride, int n_bias, double limit, bool half, double half_limit = 0.0,
+                                  int most_splits = 32) {
   GatherTiling best;
   const int t0 = channel_tiles(channels, cols_per_channel);
   for (int t = t0; t > 0 && t <= channels; ++t) {
@@ -1445,19 +1475,26 @@ GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, in
     const bool two = two_ctas_per_sm(n_pad, kblocks * kBlockK / run, n_bias, 0, &slots_unused);
     // a k-block of a CTA that shares its SM, of one that has the SM to itself, of the shape with one CTA per SM
     const double far = lane_stride > 2 ? 1.7 : 1.0;  // lanes 16 bytes and more apart: four wavefronts and more per load
-    const double shared = 2 * (half ? std::max(0.239 + 0.00055 * n_pad, (run > 1 ? 0.24 : 0.318) * far)
+    const double shared = 2 * (half ? std::max(0.241 + 0.00053 * n_pad, (run > 1 ? 0.24 : 0.318) * far)
                                     : std::max(0.11 + 0.0028 * n_pad, (run > 1 ? 0.235 : 0.30) * far));
-    const double alone = half ? (run > 1 ? 0.27 : 0.338) * far : std::max(0.19 + 0.0018 * n_pad, 0.27 * far);
-    const double one = half ? std::max(0.00197 * n_pad - 0.051, (run > 1 ? 0.249 : 0.311) * far) : std::max(0.0035 * n_pad, 0.42 * far);
-    const double epilogue = half ? 1.5 + 0.0149 * n_pad : 4.0 + 0.004 * n_pad, overlapped = half ? 0.89 : 0.4, start = half ? 6.8 : 2.6;
-    for (int s = 1; s <= std::max(1, std::min(32, kblocks / 2)); ++s) {
+    const double alone = half ? (run > 1 ? 0.279 : 0.348) * far : std::max(0.19 + 0.0018 * n_pad, 0.27 * far);
+    const double one = half ? std::max(0.00191 * round_up(n_pad, 64) - 0.039, (run > 1 ? 0.25 : 0.312) * far) : std::max(0.0035 * n_pad, 0.42 * far);
+    const double epilogue = half ? 2.1 + 0.0184 * n_pad : 4.0 + 0.004 * n_pad, start = half ? 5.9 : 2.6;
+    for (int s = 1; s <= std::max(1, std::min(most_splits, kblocks / 2)); ++s) {
       const int kps = (kblocks + s - 1) / s;
-      if ((kblocks + kps - 1) / kps != s || kps * (n_pad <= kCrossCols ? 1.0 : 3.0) > limit) continue;
+      const double chain = kps * (n_pad <= kCrossCols ? 1.0 : 3.0);
+      if ((kblocks + kps - 1) / kps != s || (limit && chain > limit)) continue;
+      // Pairs of fp16 are no less accurate than what tf32 would do here: wide tiles take a second accumulator where they have to and there is
+      // room for it beside four A slots (two of a CTA that shares its SM).
+      const bool cross = half && n_pad > kCrossCols && chain / 2 > half_limit;
+      if (half && chain / (cross ? 6 : 2) > half_limit) continue;
+      if (cross && 2 * n_pad > (two ? 256 - 64 : 512 - 128)) continue;
       const long long units = pixel_tiles * groups * t * s, slots = (long long)sms * (two ? 2 : 1), tail = units % slots;
+      const double overlapped = cross ? 1.0 : half ? 0.65 : 0.4;  // of the epilogue that is not (cross: one accumulator buffer)
       double us = (double)(units / slots) * (kps * (two ? shared : one) + overlapped * epilogue) +
                   (tail ? kps * (!two ? one : tail > sms ? shared : alone) + epilogue : (1 - overlapped) * epilogue) + start;
       if (s > 1) us += (half ? 1.4 : 3.8) + units * 128.0 * n_pad * 4.0 * (half ? 0.284e-6 : 0.18e-6);
-      if (!best.tiles || us < 0.99 * best.us) best = GatherTiling{t, s, kps, us};
+      if (!best.tiles || us < 0.99 * best.us) best = GatherTiling{t, s, kps, us, chain, cross};
     }
   }
   return best;
@@ -1467,6 +1504,9 @@ GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, in
 // of conv4 (14 MB), 58 for those of conv2 at batch 256 (265 MB).
 // A contraction takes pairs of fp16 from kHalfMinUs on, if by the estimates (6 % rms) they save 1 - kHalfGain of it: operands that do not lie close
 // enough together pay for the look at them and gain nothing.
+// Blocks of several stride periods: for at least 1 - kTallGain of the data gradient; kTallUs: one launch more, which returns at once.
+constexpr int kMaxTallRows = 4;
+constexpr double kTallUs = 4.0, kTallGain = 0.93;
 constexpr double kHalfMinUs = 25.0, kHalfGain = 0.9;
 int wgrad_columns(const ConvGeom& G) {
   int chain;
@@ -1496,7 +1536,14 @@ struct GatherProblem {
   size_t map_k = 0;               // extent of the packed operand along the reduction (0: k_pad)
   size_t smem = 0;
   bool half = false;              // HALF
-  int a_stages_half = 4, b_stages_half = 4, acc_bufs_half = 1;
+  // Data gradient: stride periods of rows in a block of pixels that share what they gather (their columns stand side by side in the
+  // accumulator).  Taps that one of the pixels does not have are products with zero weights, so blocks of several periods take finite values alone
+  // (tall_route), and only in pairs of fp16, whose MMAs have the time for that.  CaffeNet conv2 (48 columns, three rows 144) at batch 256 502 -> 380 us,
+  // at 128 268 -> 205; 20 -> 50 channels 24 x 24, 256 images, four rows 108 -> 55.  Bound by the MMAs then (tensor pipe 71 % active; 144 columns take
+  // the time of 192, the zero weights 2 / 7 of it) and a last round of units.
+  int rows = 1;
+  bool half_cross = false;        // a second accumulator for the cross terms there too
+  int a_stages_half = 4, b_stages_half = 4, acc_bufs_half = 1, acc_cols_half = 0;
   float* zero = nullptr;          // one 0.f, read by taps out of bounds
   bool inside = false;            // kInside
   bool one = false;               // ONE: the tiles of the whole batch are short and have a slot each, if no SMs are kept
@@ -1504,12 +1551,15 @@ struct GatherProblem {
   int splits = 1, split_k = 0;    // splits of the reduction and the length of one (a multiple of 32; k_pad without splits)
   float* partial = nullptr;       // split sums
   size_t pix_pad = 0;
+  int taps_y = 0, q_h = 0, q0 = 0;  // rows > 1: taps along a column, blocks of pixels along it and the first that holds a pixel
   int small_ct = 0;               // > 0: small_conv_kernel with this many channels per block instead of gather_conv_kernel
 };
 
 struct UmmaPlan {
   ConvGeom G;
   GatherProblem fwd, dgr;
+  GatherProblem tall;  // the data gradient by blocks of several stride periods (rows > 1), where that is faster: dgr is for the calls it does not take
+  MaskTap* tall_row_taps = nullptr;  // as dgr_row_taps
   // data gradient: taps per axis of one stride period; super-pixels of s x s pixels, how many per axis and the first that
   // holds a pixel
   int dgr_taps = 0, dgr_q = 0, dgr_q0 = 0;
@@ -1531,7 +1581,7 @@ struct UmmaPlan {
   MaskTap* wg_pix = nullptr;       // per pixel: offset of the tap origin, taps out of bounds (padded to splits * kps * 32)
   float* wg_plane_sums = nullptr;  // [batch][channel] sums of dY for the bias gradient
   int wg_splits = 1, wg_kps = 1, wg_mtiles = 1;
-  HalfScale* half = nullptr;       // scales of the operands, by kHalfX and so on
+  HalfScales* half = nullptr;      // scales of the operands, by kHalfX and so on
   uint2* half_parts = nullptr;
   uint32_t* half_ticket = nullptr;
   void* memory = nullptr;          // everything above that lives on the device (PlanMemory)
@@ -1547,6 +1597,7 @@ GatherKernel gather_kernel_of(const GatherProblem& gp) {
 GatherKernel gather_kernel(const GatherProblem& gp, bool weight_grad, bool one, bool half) {
   if (half) {
     if (weight_grad) return gather_kernel_of<kHalf + kWeightGrad>(gp);
+    if (gp.rows > 1) return gp.run == kRun ? gather_kernel_of<kTall + kHalf + kByRun>(gp) : gather_kernel_of<kTall + kHalf + kByTap>(gp);
     return gp.run == kRun ? gather_kernel_of<kHalf + kByRun>(gp) : gather_kernel_of<kHalf + kByTap>(gp);
   }
   if (weight_grad) return gather_kernel_of<kWeightGrad>(gp);
@@ -1618,6 +1669,7 @@ int extra_blocks(ReduceExtras& E, int threads) {
   if (E.bias.db) E.bias.blocks = (E.bias.channels + threads / 32 - 1) / (threads / 32);
   return E.pack.blocks + E.bias.blocks;
 }
+int extra_blocks(HalfExtras& E, int threads) { return E.tall.blocks + extra_blocks(static_cast<ReduceExtras&>(E), threads); }
 int extra_blocks(NoExtras&, int) { return 0; }
 
 // Split reduction: tiles when they fill the machine, the flat form otherwise (both add in a fixed order).
@@ -1638,10 +1690,10 @@ void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* d
 }
 void launch_wgrad_reduce(cct_ctx* ctx, const float* partial, float* dW, float* db, int splits, int vgroups, int tiles_per_group,
                          int rows_pad, int n_real, int n_pad, int k_real, int og, int accumulate = 0,
-                         const ReduceExtras& extras = ReduceExtras()) {
+                         const ReduceExtras& extras = ReduceExtras(), const PackDgrad& tall = PackDgrad()) {
   if (extras.pack.half)
     launch_wgrad_reduce<HalfExtras>(ctx, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate,
-                                    HalfExtras(extras));
+                                    HalfExtras{extras, tall});
   else if (extras.pack.blocks || extras.bias.db)
     launch_wgrad_reduce<ReduceExtras>(ctx, partial, dW, db, splits, vgroups, tiles_per_group, rows_pad, n_real, n_pad, k_real, og, accumulate,
                                       extras);
@@ -1673,7 +1725,7 @@ bool use_small_wgrad(long long pixels, int vgroups, int n, int k_real) {
 }
 
 // Tensor-memory and shared-memory budget of a gather problem, room for its packed operand.
-void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias, int sms, long long tiles) {
+void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias, int sms, long long tiles, bool half) {
   // Tensor memory (512 columns) = accumulator buffers + A stages of 64 columns.  Two accumulator buffers let the epilogue
   // overlap the next tile.
   const int acc = acc_columns(gp.n_pad);
@@ -1688,9 +1740,14 @@ void finish_problem(PlanMemory& mem, GatherProblem& gp, int vgroups, int n_bias,
   if (two_ctas_per_sm(gp.n_pad, taps_smem, n_bias, ptab, &b_two)) {
     gp.sets = 2; gp.tmem_cols = 256; gp.acc_bufs = 1; gp.a_stages = acc <= 64 && !ptab ? 3 : 2; gp.b_stages = b_two;
   }
-  // As pairs of fp16: A slots of 32 columns, weight slots of half the size.
-  gp.acc_bufs_half = gp.sets == 4 && 2 * acc + 4 * 32 <= 512 ? 2 : 1;
-  gp.a_stages_half = std::min(4, (gp.tmem_cols - gp.acc_bufs_half * acc) / 32);
+  // As pairs of fp16: A slots of 32 columns, weight slots of half the size.  Four of those are two of tf32: where two CTAs share the SM the rest of
+  // the memory is worth more as L1, from which the producers gather (CaffeNet conv2's weight gradient 341 -> 332 us, conv5's 137 -> 130; one CTA per
+  // SM is slower then, conv3's 162 -> 187).
+  gp.half = half;
+  if (half && gp.sets == 2) gp.b_stages = std::min(gp.b_stages, 2);
+  gp.acc_cols_half = gp.half_cross || gp.n_pad <= kCrossCols ? 2 * gp.n_pad : gp.n_pad;
+  gp.acc_bufs_half = gp.sets == 4 && 2 * gp.acc_cols_half + 4 * 32 <= 512 ? 2 : 1;
+  gp.a_stages_half = std::min(4, (gp.tmem_cols - gp.acc_bufs_half * gp.acc_cols_half) / 32);
   gp.b_stages_half = std::min(4, 2 * gp.b_stages);
   gp.smem = gather_smem(gp.n_pad, taps_smem, gp.b_stages, n_bias, gp.taps_smem == 0 ? 4 * gp.sets : 0).total + 1024;
   const int period = gp.splits == 1 ? gp.n / gp.ch_tile : 1;  // pixels of a stride period, which are columns, where they are stored as such
@@ -1740,15 +1797,16 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     f.run = G.Dg % kRun == 0 ? kRun : 1; f.run_stride = G.n * G.n;
     f.inside = f.run == 1 && G.p == 0;
     const long long pixel_tiles = ((long long)G.B * G.m * G.m + kTileM - 1) / kTileM;
-    auto tiling = [&](bool half) {
+    auto tiling = [&](bool half, double half_limit) {
       return choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.og, 1, f.k_pad / kBlockK, f.run, G.s, G.bias ? G.o : 0,
-                                  chain_limit(G.og, 1, f.k_pad / kBlockK), half);
+                                  chain_limit(G.og, 1, f.k_pad / kBlockK), half, half_limit);
     };
-    GatherTiling tl = tiling(false);
+    GatherTiling tl = tiling(false, 0.0);
     // Pairs of fp16 where that makes up for a look at the operands.
-    const GatherTiling paired = tiling(true);
-    const bool half = tl.us > kHalfMinUs && !f.inside && paired.us + scales_us(elements_x(G) + elements_w(G)) < kHalfGain * tl.us;
+    const GatherTiling paired = tiling(true, tl.chain);
+    const bool half = tl.us > kHalfMinUs && !f.inside && paired.tiles && paired.us + scales_us(elements_x(G) + elements_w(G)) < kHalfGain * tl.us;
     if (half) tl = paired;
+    f.half_cross = tl.cross;
     f.tiles = tl.tiles;
     f.ch_tile = f.n = (G.og + f.tiles - 1) / f.tiles;
     f.n_pad = round_up(f.n, 16);
@@ -1769,8 +1827,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       mem.table(&f.taps, t);
       mem.table(&f.cols, c);
       mem.table(&f.zero, std::vector<float>(1, 0.f));
-      finish_problem(mem, f, G.g * f.tiles, G.bias ? G.o : 0, ctx->planning_sms(), pixel_tiles * G.g * f.tiles * f.splits);
-      f.half = half;
+      finish_problem(mem, f, G.g * f.tiles, G.bias ? G.o : 0, ctx->planning_sms(), pixel_tiles * G.g * f.tiles * f.splits, half);
       if (f.splits > 1) sums = std::max(sums, (size_t)f.splits * G.g * f.tiles * f.n_pad * f.pix_pad);
     }
   }
@@ -1789,19 +1846,38 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     const int ss = G.s * G.s;
     const long long pixel_tiles = ((long long)G.B * p->dgr_q * p->dgr_q + kTileM - 1) / kTileM;
     const int kblocks = round_up(d.k_real, kBlockK) / kBlockK;
-    auto tiling = [&](bool half) {
-      return choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.Dg, ss, kblocks, d.run, 1, 0, chain_limit(G.Dg, ss, kblocks), half);
+    auto tiling = [&](bool half, double half_limit) {
+      return choose_gather_tiling(ctx->planning_sms(), pixel_tiles, G.g, G.Dg, ss, kblocks, d.run, 1, 0, chain_limit(G.Dg, ss, kblocks), half, half_limit);
     };
-    GatherTiling tl = tiling(false);
+    GatherTiling tl = tiling(false, 0.0);
+    // Narrow tiles are bound by what they gather: blocks of `rows` stride periods gather it for more columns at once.
+    struct Tall { int rows, taps_y, q, q0, k_real; long long tiles; };
+    auto tall_of = [&](int rows) {
+      Tall b{rows, J + rows - 1, 0, G.p / (rows * G.s), 0, 0};
+      b.q = (G.n - 1 + G.p) / (rows * G.s) + 1 - b.q0;
+      b.k_real = G.og * J * b.taps_y;
+      b.tiles = ((long long)G.B * b.q * p->dgr_q + kTileM - 1) / kTileM;
+      return b;
+    };
+    GatherTiling paired = tiling(true, tl.chain);
+    if (!paired.tiles) paired.us = tl.us;
+    Tall tall = tall_of(1);
+    for (int rows = 2; rows <= kMaxTallRows; ++rows) {
+      const Tall b = tall_of(rows);
+      if (b.taps_y > kMaxTapsPerAxis || b.k_real > 16384 || rows * ss > 256) break;
+      const GatherTiling t = choose_gather_tiling(ctx->planning_sms(), b.tiles, G.g, G.Dg, rows * ss, round_up(b.k_real, kBlockK) / kBlockK, d.run, 1, 0,
+                                                  0.0, true, tl.chain, 1);
+      if (t.tiles && t.us + kTallUs < kTallGain * paired.us) { paired = t; paired.us += kTallUs; tall = b; }
+    }
     // The two gradients share the look at dY: both in pairs of fp16, or one of them, or none.
-    const GatherTiling paired = tiling(true);
     const double wgrad_us = 2.0 * elements_w(G) * G.B * G.m * G.m / 230e6, wgrad_saves = wgrad_us * half_weight_gradient(p->fwd.k_real, wgrad_columns(G));
     const double dgrad_saves = tl.us - paired.us, dy = elements_y(G) + elements_w(G), x = elements_x(G);
     const double best = std::max(dgrad_saves - scales_us(dy), std::max(wgrad_saves - scales_us(dy + x), dgrad_saves + wgrad_saves - scales_us(dy + x)));
     const bool worth = best > (1 - kHalfGain) * (tl.us + wgrad_us) && tl.us + wgrad_us > kHalfMinUs;
-    const bool half = worth && dgrad_saves > 0;
+    const bool half = worth && paired.tiles && dgrad_saves > 0;
     wgrad_half = worth && wgrad_saves - scales_us(dy + x) + (half ? scales_us(dy) : 0) > 0;
-    if (half) tl = paired;
+    if (half && tall.rows == 1) tl = paired;
+    d.half_cross = tl.cross;
     d.k_pad = round_up(d.k_real, kBlockK);
     d.tiles = tl.tiles;
     d.ch_tile = (G.Dg + d.tiles - 1) / d.tiles;
@@ -1827,8 +1903,32 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       mem.table(&d.taps, t);
       mem.table(&d.cols, c);
       mem.table(&d.zero, std::vector<float>(1, 0.f));
-      finish_problem(mem, d, G.g * d.tiles, 0, ctx->planning_sms(), pixel_tiles * G.g * d.tiles * d.splits);
-      d.half = half;
+      finish_problem(mem, d, G.g * d.tiles, 0, ctx->planning_sms(), pixel_tiles * G.g * d.tiles * d.splits, half);
+      if (half && tall.rows > 1) {
+        GatherProblem& b = p->tall;
+        b.rows = tall.rows; b.run = d.run; b.run_stride = d.run_stride;
+        b.taps_y = tall.taps_y; b.q_h = tall.q; b.q0 = tall.q0;
+        b.k_real = tall.k_real; b.k_pad = round_up(tall.k_real, kBlockK);
+        b.tiles = paired.tiles; b.ch_tile = (G.Dg + b.tiles - 1) / b.tiles;
+        b.n = b.ch_tile * tall.rows * ss; b.n_pad = round_up(b.n, 16);
+        b.half_cross = paired.cross;
+        b.split_k = b.k_pad; b.pix_pad = (size_t)tall.tiles * kTileM;
+        std::vector<MaskTap> bt((size_t)b.k_pad / b.run, MaskTap{0, kPadBit});
+        for (int i = 0; i * b.run < b.k_real; ++i) {
+          const int jx = i % J, jy = (i / J) % b.taps_y, oc = i / (J * b.taps_y) * b.run;
+          bt[i] = MaskTap{oc * G.m * G.m - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
+        }
+        std::vector<ColEnt> bc(b.n_pad);
+        for (int j = 0; j < b.n_pad; ++j) {
+          const int dl = j / (tall.rows * ss), py = (j / G.s) % (tall.rows * G.s), px = j % G.s;
+          bc[j] = ColEnt{dl * G.n * G.n + py * G.n + px, (short)py, (short)px};
+        }
+        mem.table(&b.taps, bt);
+        mem.table(&b.cols, bc);
+        mem.table(&b.zero, std::vector<float>(1, 0.f));
+        finish_problem(mem, b, G.g * b.tiles, 0, ctx->planning_sms(), tall.tiles * G.g * b.tiles, true);
+        b.one = false;
+      }
       if (d.splits > 1) sums = std::max(sums, (size_t)d.splits * G.g * d.tiles * d.n_pad * d.pix_pad);
     }
   }
@@ -1959,6 +2059,15 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
         rt[i] = MaskTap{(int)(oc * w.map_k) - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
       }
       mem.table(&p->dgr_row_taps, rt);
+      const GatherProblem& b = p->tall;
+      if (b.rows > 1) {
+        std::vector<MaskTap> bt((size_t)b.k_pad / b.run, MaskTap{0, kPadBit});
+        for (int i = 0; i * b.run < b.k_real; ++i) {
+          const int jx = i % J, jy = (i / J) % b.taps_y, oc = i / (J * b.taps_y) * b.run;
+          bt[i] = MaskTap{(int)(oc * w.map_k) - jy * G.m - jx, (1u << jy) | (1u << (16 + jx))};
+        }
+        mem.table(&p->tall_row_taps, bt);
+      }
     }
     // Per-pixel table: where the pixel's window starts, and which of its rows and columns lie outside the plane.
     std::vector<uint32_t> outside(G.m);  // the same for rows and columns: bit a = window row a of output row r is outside
@@ -1973,14 +2082,13 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
         for (int q = 0; q < G.m; ++q, ++i) t[i] = MaskTap{row + q * G.s, outside[r] | (outside[q] << 16) | 0x80008000u};
       }
     mem.table(&p->wg_pix, t);
-    finish_problem(mem, w, vgroups, 0, ctx->planning_sms(), (long long)base_tiles * p->wg_splits);
-    w.half = wgrad_half;
+    finish_problem(mem, w, vgroups, 0, ctx->planning_sms(), (long long)base_tiles * p->wg_splits, wgrad_half);
     if (G.bias) mem.room(&p->wg_plane_sums, (size_t)G.B * G.o);
     sums = std::max(sums, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
   }
   if (p->fwd.half || p->dgr.half || p->wgp.half) {
-    mem.table(&p->half_ticket, std::vector<uint32_t>(1, 0u));
-    mem.room(&p->half, 3);
+    mem.table(&p->half_ticket, std::vector<uint32_t>(2, 0u));
+    mem.room(&p->half, 1);
     mem.room(&p->half_parts, (size_t)ctx->sm_count * kScaleBlocksPerSm);
   }
   float* sum_memory = nullptr;
@@ -1989,6 +2097,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
   p->fwd.partial = p->dgr.partial = p->w_partial = sum_memory;
   if (rc == CCT_OK && p->fwd.w) rc = encode_problem(ctx, p->fwd, G.g * p->fwd.tiles);
   if (rc == CCT_OK && p->dgr.w) rc = encode_problem(ctx, p->dgr, G.g * p->dgr.tiles);
+  if (rc == CCT_OK && p->tall.w) rc = encode_problem(ctx, p->tall, G.g * p->tall.tiles);
   if (rc == CCT_OK && p->wg_gather) {
     rc = encode_problem(ctx, p->wgp, G.g * p->wt_tiles);
     if (rc == CCT_OK && cudaMemsetAsync(p->wgp.w, 0, 2 * p->wgp.w_half * sizeof(float), ctx->stream) != cudaSuccess) {  // padded channel rows stay zero
@@ -1997,7 +2106,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     }
   }
   // The kernels that this plan launches, and no others: each is one to load at its first use.
-  for (const GatherProblem* gp : {&p->fwd, &p->dgr, &p->wgp})
+  for (const GatherProblem* gp : {&p->fwd, &p->dgr, &p->wgp, &p->tall})
     if (rc == CCT_OK && gp->w) rc = set_smem(ctx, gather_kernel(*gp, gp == &p->wgp, gp->one, gp->half), gather_smem_limit(*gp));
   if (rc == CCT_OK && !p->w_small && !p->wg_gather) rc = set_smem(ctx, short_wgrad_kernel(p), kSmemLimit);
   if (rc != CCT_OK) {
@@ -2033,15 +2142,14 @@ void fill_common(GatherParams& P, const GatherProblem& gp, cct_ctx* ctx, int vgr
   P.tmem_cols = gp.tmem_cols;
   P.n_bias = P.bias ? n_bias : 0;
   P.lo_row_offset = vgroups * gp.n_pad;
-  P.a_stages_half = gp.a_stages_half; P.b_stages_half = gp.b_stages_half; P.acc_bufs_half = gp.acc_bufs_half;
+  P.a_stages_half = (uint8_t)gp.a_stages_half; P.b_stages_half = (uint8_t)gp.b_stages_half; P.acc_bufs_half = (uint8_t)gp.acc_bufs_half; P.acc_cols_half = (uint16_t)gp.acc_cols_half;
   P.status = ctx->status_dev;
 }
 
-PackDgrad pack_dgrad_job(const UmmaPlan* p, const float* W, bool half) {
+PackDgrad pack_dgrad_job(const UmmaPlan* p, const GatherProblem& d, const float* W, bool half) {
   const ConvGeom& G = p->G;
-  const GatherProblem& d = p->dgr;
   PackDgrad J{W, d.w, d.w + d.w_half, d.tiles, G.og, G.Dg, G.k, G.s, p->dgr_taps, d.ch_tile, d.n, d.n_pad, d.k_real, d.k_pad, d.run, 0, 0,
-               half ? p->half : nullptr};
+               half ? p->half : nullptr, d.rows, half && p->tall.rows > 1 ? (d.rows > 1 ? kOnlyHalf : kOnlyTf32) : kAny};
   J.parts = (d.k_pad / 4 + kPackThreads - 1) / kPackThreads;
   J.blocks = G.g * d.tiles * d.n_pad * J.parts;
   return J;
@@ -2107,7 +2215,9 @@ void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp,
   if (P.splits > 1) {
     const int vgroups = P.total_tiles / (P.n_pix_tiles * P.splits), cols = P.n_pix_tiles * vgroups * P.n > 32 * ctx->sm_count ? 8 : 1;
     const int col_tiles = (P.n + cols - 1) / cols;
-    launch_pdl(cols == 8 ? gather_reduce_kernel<8> : gather_reduce_kernel<1>, dim3((P.n_pix + 127) / 128, vgroups * col_tiles), dim3(128),
+    auto kernel = P.only == kOnlyTf32 ? (cols == 8 ? gather_reduce_kernel<8, true> : gather_reduce_kernel<1, true>)
+                                      : (cols == 8 ? gather_reduce_kernel<8, false> : gather_reduce_kernel<1, false>);
+    launch_pdl(kernel, dim3((P.n_pix + 127) / 128, vgroups * col_tiles), dim3(128),
                0, ctx->stream, P, col_tiles);
   }
 }
@@ -2117,6 +2227,8 @@ struct ScaleOf {
   const float *a, *mask;
   size_t n;
   int slot, headroom;
+  const int32_t* where = nullptr;
+  int pooled = 1, plane = 1;
 };
 void launch_scales(cct_ctx* ctx, const UmmaPlan* p, std::initializer_list<ScaleOf> operands) {
   ScaleJobs J{};
@@ -2130,6 +2242,7 @@ void launch_scales(cct_ctx* ctx, const UmmaPlan* p, std::initializer_list<ScaleO
     if (!o.a) continue;
     ScaleJob& job = J.job[J.jobs++];
     job.a = o.a; job.mask = o.mask; job.n = o.n; job.per_block = per_block; job.slot = o.slot; job.headroom = o.headroom;
+    job.where = o.where; job.pooled = o.pooled; job.plane = o.plane;
     job.first = grid;
     job.blocks = (int)((o.n + per_block - 1) / per_block);
     grid += job.blocks;
@@ -2179,7 +2292,7 @@ int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W,
   P.out_group_channels = G.og;
   P.relu = relu;
   fill_common(P, f, ctx, vgroups, G.o);
-  if (half) { P.half = p->half; P.half_gathered = kHalfX; P.half_packed = kHalfW; }
+  if (half) { P.half = p->half; P.half_gathered = kHalfX; P.half_packed = kHalfW; P.taps_x = (uint8_t)G.k; }
   t->begin(0, ctx->stream);
   launch_gather(ctx, P, f);
   t->end(0, ctx->stream);
@@ -2194,12 +2307,13 @@ bool umma_dy_rows(const UmmaPlan* p, DyRows* rows) {
   return true;
 }
 
-int umma_rows_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, size_t pooled) {
+int umma_rows_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, const int32_t* idx, int pooled) {
+  const ConvGeom& G = p->G;
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   if (!p->wgp.half && !p->dgr.half) return CCT_OK;
   // an element is in up to four windows
-  launch_scales(ctx, p, {ScaleOf{X, nullptr, elements_x(p->G), kHalfX, 0}, ScaleOf{W, nullptr, elements_w(p->G), kHalfW, 0},
-                         ScaleOf{dP, P, pooled, kHalfDy, 2}});
+  launch_scales(ctx, p, {ScaleOf{p->wgp.half ? X : nullptr, nullptr, elements_x(G), kHalfX, 0}, ScaleOf{p->dgr.half ? W : nullptr, nullptr, elements_w(G), kHalfW, 0},
+                         ScaleOf{dP, P, (size_t)G.B * G.o * pooled * pooled, kHalfDy, 2, idx, pooled * pooled, G.m * G.m}});
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
@@ -2239,7 +2353,11 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
   const ConvGeom& G = p->G;
   ReduceExtras extras{};
-  if (pack_W && !p->dgr.small_ct) extras.pack = pack_dgrad_job(p, pack_W, half && p->dgr.half);
+  PackDgrad tall{};
+  if (pack_W && !p->dgr.small_ct) {
+    extras.pack = pack_dgrad_job(p, p->dgr, pack_W, half && p->dgr.half);
+    if (half && p->tall.rows > 1) tall = pack_dgrad_job(p, p->tall, pack_W, true);
+  }
   if (p->wg_gather) {
     struct { int tiles, n, n_pad, k_real; } f = {p->wt_tiles, p->wt_n, p->w_npad, p->fwd.k_real};
     GatherProblem& w = p->wgp;
@@ -2267,7 +2385,7 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     if (G.bias) extras.bias = BiasSum{p->wg_plane_sums, db, G.B, G.o, 0};
     t->begin(2, ctx->stream);
     launch_wgrad_reduce(ctx, p->w_partial, dW, nullptr, p->wg_splits, vgroups, f.tiles, p->wg_mtiles * kTileM, f.n,
-                        f.n_pad, f.k_real, G.og, 0, extras);
+                        f.n_pad, f.k_real, G.og, 0, extras, tall);
     t->end(2, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   } else {
@@ -2312,7 +2430,7 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     CCT_CHECK_LAUNCH(ctx);
     t->begin(2, ctx->stream);
     launch_wgrad_reduce(ctx, p->w_partial, dW, G.bias ? db : nullptr, p->w_splits, vgroups, f.tiles, rows_pad, f.n, P.n_pad,
-                        f.k_real, G.og, 0, extras);
+                        f.k_real, G.og, 0, extras, tall);
     t->end(2, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
   }
@@ -2348,7 +2466,7 @@ int data_gradient(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, fl
       return CCT_OK;
     }
     if (repack) {
-      const PackDgrad J = pack_dgrad_job(p, W, half);
+      const PackDgrad J = pack_dgrad_job(p, d, W, half);
       launch_pdl(pack_dgrad_kernel, dim3(J.blocks), dim3(kPackThreads), 0, ctx->stream, J);
       CCT_CHECK_LAUNCH(ctx);
     }
@@ -2377,7 +2495,24 @@ int data_gradient(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, fl
       P.taps = p->dgr_row_taps;
       P.run_stride = (int)p->wgp.map_k;
     }
-    if (half && d.half) { P.half = p->half; P.half_gathered = kHalfDy; P.half_packed = kHalfW; }
+    if (half && d.half) { P.half = p->half; P.half_gathered = kHalfDy; P.half_packed = kHalfW; P.taps_x = (uint8_t)p->dgr_taps; }
+    if (half && p->tall.rows > 1) {
+      const GatherProblem& b = p->tall;
+      GatherParams Q = P;
+      Q.n_pix = B * b.q_h * p->dgr_q; Q.q_h = b.q_h;
+      Q.iy_mul = b.rows; Q.iy_add = b.q0 * b.rows + b.rows - 1;
+      Q.taps_per_axis = b.taps_y;
+      Q.oy_mul = b.rows * G.s; Q.oy_add = b.q0 * b.rows * G.s - G.p;
+      fill_common(Q, b, ctx, G.g * b.tiles, 0);
+      if (rows) {
+        Q.taps = p->tall_row_taps;
+        Q.run_stride = (int)p->wgp.map_k;
+      }
+      Q.only = kOnlyHalf;
+      Q.bad_geom = {(uint8_t)G.k, (uint8_t)G.s, (short)G.p, (short)G.m, G.o, G.og};
+      P.only = kOnlyTf32;
+      launch_gather(ctx, Q, b);
+    }
     launch_gather(ctx, P, d);
     t->end(3, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);

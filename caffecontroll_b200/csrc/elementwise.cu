@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(kPool32Threads) maxpool_bwd_3x3s2_kernel(
   float* s_g = pool32_smem + in_pad;
   float* s_out = s_g + in_pad;  // ROWS: the planes, on their way out
   const bool pairs = ROWS == kRowsHalf && half_route(rows.half, kHalfX, kHalfDy);
-  const float scale = pairs ? rows.half[kHalfDy].scale : 1.f;
+  const float scale = pairs ? rows.half->of[kHalfDy].scale : 1.f;
   for (int g0 = blockIdx.x * group; g0 < planes; g0 += gridDim.x * group) {
     const int cnt = min(group, planes - g0);
     const size_t in_base = (size_t)g0 * mm;

@@ -7,9 +7,15 @@
 // power of two, brings its largest value to [2^14, 2^15), `inverse` takes it back; `ok`: its values lie close enough together.
 struct alignas(16) HalfScale {
   float scale, inverse;
-  int ok, pad;
+  int ok;
+  int bad;  // dY: values that are not finite, the first kMaxBad of them listed behind the scales (HalfScales)
 };
 enum { kHalfX = 0, kHalfW = 1, kHalfDy = 2 };
+constexpr int kMaxBad = 16;
+struct HalfScales {
+  HalfScale of[3];
+  int bad[kMaxBad];  // elements of dY, in no order
+};
 
 // Where a row of pairs of fp16 has its elements: of each 32 in a row the hi halves in words 0 - 15, the lo halves in words 16 - 31, so that
 // 32 of the reduction are one 128-byte line.  Element i's word of hi halves; its lo halves are kHalfLo words on.
@@ -29,7 +35,9 @@ __device__ __forceinline__ void split_half2(float a, float b, uint32_t& hi, uint
   lo = pack_half2(a - ha, b - hb);
 }
 // Whether operands `a` and `b` of a plan's scales (null: none) are both split into pairs of fp16.
-__device__ __forceinline__ bool half_route(const HalfScale* half, int a, int b) { return half && half[a].ok && half[b].ok; }
+__device__ __forceinline__ bool half_route(const HalfScales* half, int a, int b) { return half && half->of[a].ok && half->of[b].ok; }
+// Whether a data gradient by tall blocks of pixels (GatherProblem::rows) takes them.
+__device__ __forceinline__ bool tall_route(const HalfScales* half) { return half_route(half, kHalfDy, kHalfW) && half->of[kHalfDy].bad <= kMaxBad; }
 
 // A warp writes up to 32 elements of such a row, lane = element of the 32 at `block`: pairs of lanes share a word, except where only one of
 // them is `in` (the ends of an image whose size is odd).

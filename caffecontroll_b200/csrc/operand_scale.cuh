@@ -25,21 +25,24 @@ struct ScaleJob {
   int first = 0, blocks = 0;    // of the grid
   int slot = 0;
   int headroom = 0;             // octaves that the operand may be larger than `a` (sums of up to four windows' gradients: 2)
+  // Of a pooled gradient: which element of its plane of `plane` each is added to, and the pooled planes' size.
+  const int32_t* where = nullptr;
+  int pooled = 1, plane = 1;
 };
 struct ScaleJobs {
   ScaleJob job[3];
   int jobs;
-  HalfScale* out;
+  HalfScales* out;
   uint2* parts;       // per block: the largest value's bits, the mean exponent of those that are not 0 (each rounded down to even)
-  uint32_t* ticket;   // 0 before and after every launch
+  uint32_t* ticket;   // two words, 0 before and after every launch: blocks that are through, values that are not finite
 };
 
 // The largest finite value, the number of those that are not 0 and the sum of their exponents, halved (the top byte: one instruction).
 struct ScaleStats {
   uint32_t top = 0, count = 0, halves = 0;
-  // 4 * N values; all finite, as nearly always: four instructions each
+  // 4 * N values; all finite, as nearly always (and said so): four instructions each
   template <int N>
-  __device__ __forceinline__ void add(const float4 (&v)[N]) {
+  __device__ __forceinline__ bool add(const float4 (&v)[N]) {
     uint32_t u[4 * N], most = 0;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -48,7 +51,8 @@ struct ScaleStats {
     }
 #pragma unroll
     for (int i = 0; i < 4 * N; ++i) most = max(most, u[i]);
-    if (most >= 0x7f800000u) {
+    const bool finite = most < 0x7f800000u;
+    if (!finite) {
       most = 0;
 #pragma unroll
       for (int i = 0; i < 4 * N; ++i) {
@@ -62,8 +66,19 @@ struct ScaleStats {
       count += min(u[i], 1u);
       halves = __dp4a(u[i], 0x01000000u, halves);
     }
+    return finite;
   }
 };
+
+// Lists what is not finite of four elements of dY from `i` on.
+__device__ __noinline__ void list_bad(const ScaleJobs& J, const ScaleJob& job, size_t i, float4 v) {
+  const float x[4] = {v.x, v.y, v.z, v.w};
+  for (int e = 0; e < 4; ++e)
+    if ((__float_as_uint(x[e]) & 0x7f800000u) == 0x7f800000u) {
+      const uint32_t at = atomicAdd(J.ticket + 1, 1u);
+      if (at < (uint32_t)kMaxBad) J.out->bad[at] = (int)(job.where ? (i + e) / job.pooled * job.plane + __ldg(job.where + i + e) : i + e);
+    }
+}
 
 __global__ void __launch_bounds__(kScaleThreads, kScaleBlocksPerSm) operand_scale_kernel(const __grid_constant__ ScaleJobs J) {
   __shared__ uint32_t part[3][kScaleThreads / 32];
@@ -91,7 +106,8 @@ __global__ void __launch_bounds__(kScaleThreads, kScaleBlocksPerSm) operand_scal
           v[u] = make_float4(m.x > 0.f ? v[u].x : 0.f, m.y > 0.f ? v[u].y : 0.f, m.z > 0.f ? v[u].z : 0.f, m.w > 0.f ? v[u].w : 0.f);
         }
       }
-      s.add(v);
+      if (!s.add(v) && job.slot == kHalfDy)
+        for (int u = 0; u < kAhead; ++u) list_bad(J, job, i + u * kScaleThreads * 4, v[u]);
     }
   }
   for (; i < end; i += kScaleThreads * 4) {
@@ -99,7 +115,7 @@ __global__ void __launch_bounds__(kScaleThreads, kScaleBlocksPerSm) operand_scal
 #pragma unroll
     for (int e = 0; e < 4; ++e) t[e] = i + e < end && (!job.mask || __ldg(job.mask + i + e) > 0.f) ? __ldg(job.a + i + e) : 0.f;
     const float4 v[1] = {make_float4(t[0], t[1], t[2], t[3])};
-    s.add(v);
+    if (!s.add(v) && job.slot == kHalfDy) list_bad(J, job, i, v[0]);
   }
   s.top = __reduce_max_sync(0xffffffffu, s.top);
   s.count = __reduce_add_sync(0xffffffffu, s.count);
@@ -132,8 +148,9 @@ __global__ void __launch_bounds__(kScaleThreads, kScaleBlocksPerSm) operand_scal
       const int e = (int)(top >> 23), up = 14 - mine.headroom - (e - 127);  // the scale is 2^up
       const bool ok = top == 0 || (e >= 127 - 45 && e <= 127 + 45 && (int)low >= e - kHalfOctaves);
       const bool scaled = ok && top != 0;
-      J.out[mine.slot] = HalfScale{scaled ? __uint_as_float((uint32_t)(127 + up) << 23) : 1.f,
-                                   scaled ? __uint_as_float((uint32_t)(127 - up) << 23) : 1.f, ok ? 1 : 0, 0};
+      J.out->of[mine.slot] = HalfScale{scaled ? __uint_as_float((uint32_t)(127 + up) << 23) : 1.f,
+                                   scaled ? __uint_as_float((uint32_t)(127 - up) << 23) : 1.f, ok ? 1 : 0,
+                                       mine.slot == kHalfDy ? (int)min(atomicExch(J.ticket + 1, 0u), (uint32_t)kMaxBad + 1u) : 0};
     }
   }
 }

@@ -89,9 +89,12 @@ def launches(ctx, call):
 # a block of 32); reductions that are no multiple of 32; split reductions.  Launches: the look at the operands, packing, contraction and the sum of
 # its splits; the look, the split of dY, contraction, sums and packing, contraction and the sum of its splits.
 @pytest.mark.parametrize("shape,forward,backward", [
-    ((67, 256, 13, 384, 3, 1, 1, 1), (3, 4), (5, 6)), ((67, 250, 17, 300, 3, 1, 1, 1), (3, 4), (5, 6)), ((64, 96, 27, 256, 5, 1, 2, 2), (3,), (4, 5)),
-    ((50, 192, 31, 320, 3, 2, 1, 1), (3, 4), (5,)), ((64, 384, 13, 384, 3, 1, 1, 2), (3,), (5,)), ((25, 120, 41, 160, 5, 1, 2, 1), (3, 4), (5, 6)),
-    ((64, 1024, 27, 600, 1, 1, 0, 1), (3,), (5,)),
+    ((67, 256, 13, 384, 3, 1, 1, 1), (3, 4), (5, 6)), ((67, 250, 17, 300, 3, 1, 1, 1), (3, 4), (5, 6)), ((64, 96, 27, 256, 5, 1, 2, 2), (3,), (4, 5, 6, 7)),
+    ((50, 192, 31, 320, 3, 2, 1, 1), (2, 3, 4), (5,)), ((64, 384, 13, 384, 3, 1, 1, 2), (3,), (5,)), ((25, 120, 41, 160, 5, 1, 2, 1), (3, 4), (5, 6)),
+    ((64, 1024, 27, 600, 1, 1, 0, 1), (2, 3), (5,)),
+    # data gradients by tall blocks of pixels, two launches: by eight and single channels, strides, groups, one and two CTAs per SM
+    ((128, 96, 27, 256, 5, 1, 2, 2), (3,), (6, 7)), ((64, 24, 60, 256, 5, 2, 2, 1), (2, 3, 4), (6, 7)), ((256, 20, 24, 50, 5, 1, 0, 1), (2,), (5, 6)),
+    ((50, 31, 43, 250, 5, 1, 2, 1), (3, 4), (6, 7)),
 ])
 def test_pairs_of_fp16(ctx, layer, shape, forward, backward):
     B, D, n, o, k, s, p, g = shape
@@ -153,28 +156,52 @@ def test_operands_far_apart(layer, what):
     assert off(dW, dWr) <= 2 * bound(176 * 32)
 
 
+TALL = [(128, 96, 27, 256, 5, 1, 2, 2), (64, 24, 60, 256, 5, 2, 2, 1), (256, 20, 24, 50, 5, 1, 0, 1), (50, 31, 43, 250, 5, 1, 2, 1)]
+
+
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
-def test_values_that_are_not_finite(layer, value):
+@pytest.mark.parametrize("shape", [SHAPE] + TALL)
+def test_values_that_are_not_finite(layer, shape, value):
     """They reach their windows, and nothing else changes by a bit; the calls after them are what those before them were."""
-    at = layer(SHAPE)
-    B, D, n, o, k, s, p, g = SHAPE
+    at = layer(shape)
+    B, D, n, o, k, s, p, g = shape
     X, W, b, dY = at.operands(3)
     W = torch.where(W == 0, torch.full_like(W, 0.01), W)
-    X[B - 1, 5, 6, 7] = dY[B - 1, 9, 12, 12] = 0
+    where = [(B - 1, 9, at.m - 1, at.m // 2), (0, o - 1, 0, 0), (B // 2, 3, at.m // 2, at.m // 2)]
+    X[B - 1, D - 1, 6, 7] = 0
+    for w in where:
+        dY[w] = 0
     Y, (dX, dW, db) = at.forward(X, W, b), at.backward(X, W, dY)
     Xn, dYn = X.clone(), dY.clone()
-    Xn[B - 1, 5, 6, 7] = dYn[B - 1, 9, 12, 12] = value
-    inside = torch.zeros_like(Y, dtype=torch.bool)
-    inside[B - 1, :, 5:8, 6:9] = True
+    Xn[B - 1, D - 1, 6, 7] = value
+    for w in where:
+        dYn[w] = value
+    ones = torch.ones_like(W)
+    inside = torch.nn.functional.conv2d((Xn != X).float(), ones, None, s, p, 1, g) != 0
     Yn = at.forward(Xn, W, b)
     assert not torch.isfinite(Yn[inside]).any() and torch.equal(Yn[~inside], Y[~inside])
-    inside = torch.zeros_like(X, dtype=torch.bool)
-    inside[B - 1, :, 11:13, 11:13] = True
+    inside = torch.nn.grad.conv2d_input(X.shape, ones, (dYn != dY).float(), s, p, 1, g) != 0
     dXn, dWn, dbn = at.backward(X, W, dYn)
     assert not torch.isfinite(dXn[inside]).any() and torch.equal(dXn[~inside], dX[~inside])
-    others = torch.arange(o, device="cuda") != 9
-    assert torch.equal(dWn[others], dW[others]) and not torch.isfinite(dbn[9]) and torch.equal(dbn[others], db[others])
+    others = torch.ones(o, dtype=torch.bool, device="cuda")
+    others[[w[1] for w in where]] = False
+    assert torch.equal(dWn[others], dW[others]) and not torch.isfinite(dbn[~others]).any() and torch.equal(dbn[others], db[others])
     assert torch.equal(at.forward(X, W, b), Y) and all(torch.equal(u, v) for u, v in zip(at.backward(X, W, dY), (dX, dW, db)))
+
+
+@pytest.mark.parametrize("shape", [t for t in TALL if t[5] == 1])  # (with a stride a block of one period has zero weights for some pixels as well)
+def test_many_values_that_are_not_finite(layer, shape):
+    """More than a data gradient by tall blocks keeps a list of: it takes the others, and back."""
+    at = layer(shape)
+    _, _, _, _, _, s, p, g = shape
+    X, W, b, dY = at.operands(8)
+    clean = at.backward(X, W, dY)[0]
+    wild = dY.clone()
+    wild[1, 2, :, 3] = float("nan")
+    inside = torch.nn.grad.conv2d_input(X.shape, torch.ones_like(W), torch.isnan(wild).float(), s, p, 1, g) != 0
+    dX = at.backward(X, W, wild)[0]
+    assert torch.isnan(dX[inside]).all() and off(dX[~inside], clean[~inside].double()) <= 4 * bound(shape[3] // g * shape[4] ** 2)
+    assert torch.equal(at.backward(X, W, dY)[0], clean)
 
 
 def test_one_way_after_the_other(layer):
@@ -192,7 +219,7 @@ def test_one_way_after_the_other(layer):
     assert all(torch.equal(u, v) for u, v in zip(at.backward(X, W, dY), first))
 
 
-@pytest.mark.parametrize("shape", [(37, 384, 13, 256, 3, 1, 1, 1), (64, 384, 14, 512, 3, 1, 1, 2), (65, 256, 13, 384, 3, 1, 1, 1)])
+@pytest.mark.parametrize("shape", [(37, 384, 13, 256, 3, 1, 1, 1), (64, 384, 14, 512, 3, 1, 1, 2), (65, 256, 13, 384, 3, 1, 1, 1), TALL[0]])
 def test_pooled_gradients_in_rows(ctx, layer, shape):
     """The pooling kernel writes the rows of dY itself: the gradients of the chain pool -> ReLU -> convolution against 64 bits, and twice the same."""
     B, D, n, o, k, s, p, g = shape
@@ -219,3 +246,15 @@ def test_pooled_gradients_in_rows(ctx, layer, shape):
     for got, ref, products, name in zip(runs[0], (dXr, dWr, dbr), (o // g * k * k, 176 * 32, 1), ("dX", "dW", "db")):
         assert off(got, ref) <= bound(products), name
     assert all(torch.equal(u, v) for u, v in zip(*runs))
+    # one that is not finite: the pixels of the window of the element that it goes to
+    at_most = (P[1, 2] > 0).nonzero()[0].tolist()
+    dP[1, 2, at_most[0], at_most[1]] = float("nan")
+    dX = torch.full_like(X, 7)
+    torch.cuda.synchronize()
+    capi.check(ctx.lib.cct_conv_backward_fused(at.plan, X.data_ptr(), W.data_ptr(), None, C.byref(f), dX.data_ptr(), dW.data_ptr(), db.data_ptr()),
+               "backward", ctx.h)
+    ctx.sync()
+    hit = torch.zeros(B, o, m * m, device="cuda")
+    hit[1, 2, index[1, 2, at_most[0], at_most[1]]] = 1
+    inside = torch.nn.grad.conv2d_input(X.shape, torch.ones_like(W), hit.view(B, o, m, m), s, p, 1, g) != 0
+    assert torch.isnan(dX[inside]).all() and torch.equal(dX[~inside], runs[0][0][~inside])
