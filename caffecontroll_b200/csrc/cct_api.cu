@@ -554,6 +554,7 @@ int cct_conv_backward_fused(cct_conv_plan* plan, const float* X, const float* W,
   const ConvGeom& G = plan->G;
   if (G.bias && !db) return CCT_ERR_INVALID;
   CCT_CUDA(ctx, cudaSetDevice(ctx->device));
+  bool scaled = false;
   if (f->dP) {
     // conv -> ReLU -> max-pool behind this layer: one pass builds the output gradient both kernels read.
     if ((!f->A && !f->P) || !f->idx || f->pool_k <= 0 || f->pool_s <= 0 || f->pool_k > G.m) return CCT_ERR_INVALID;
@@ -561,13 +562,16 @@ int cct_conv_backward_fused(cct_conv_plan* plan, const float* X, const float* W,
       ctx->last_error = "cct_conv_backward_fused with a pooled gradient needs cct_conv_plan_reserve_fusion(plan) first";
       return CCT_ERR_INVALID;
     }
+    if (f->P && plan->algo == CCT_ALGO_UMMA_3XTF32) {
+      const int rc = umma_pooled_scales(ctx, plan->umma, X, W, f->dP, f->P, f->idx, f->pool_k, f->pool_s, dX != nullptr);
+      if (rc != CCT_OK) return rc;
+      scaled = true;
+    }
     DyRows rows;
-    if (f->P && plan->algo == CCT_ALGO_UMMA_3XTF32 && umma_dy_rows(plan->umma, &rows)) {
+    if (scaled && umma_dy_rows(plan->umma, &rows)) {
       // straight into the form the contractions read
-      const int pooled = (G.m - f->pool_k) / f->pool_s + 1;
-      int rc = umma_rows_scales(ctx, plan->umma, X, W, f->dP, f->P, f->idx, pooled);
-      if (rc == CCT_OK) rc = pool_relu_backward_rows(ctx, f->P, f->idx, f->dP, rows, G.B * G.o, G.m, f->pool_k, f->pool_s);
-      if (rc == CCT_OK) rc = umma_conv_backward(ctx, plan->umma, X, W, nullptr, dX, dW, db, &plan->timer);
+      int rc = pool_relu_backward_rows(ctx, f->P, f->idx, f->dP, rows, G.B * G.o, G.m, f->pool_k, f->pool_s);
+      if (rc == CCT_OK) rc = umma_conv_backward(ctx, plan->umma, X, W, nullptr, dX, dW, db, &plan->timer, true);
       if (rc == CCT_OK && f->relu_mask_dx && dX) rc = cct_relu_backward(ctx, X, dX, dX, (size_t)G.B * G.D * G.n * G.n);
       if (rc != CCT_ERR_UNSUPPORTED) return rc;
     }
@@ -580,7 +584,7 @@ int cct_conv_backward_fused(cct_conv_plan* plan, const float* X, const float* W,
   // The ReLU bridge in front of the layer: dX *= [X > 0] as one HBM-bound pass behind the data-gradient kernel.
   // (Folded into that kernel's epilogue it cost more than the pass: one extra load per accumulator column in the four
   // epilogue warps made the epilogue the bottleneck of wide data gradients.)
-  int rc = plan->algo == CCT_ALGO_UMMA_3XTF32 ? umma_conv_backward(ctx, plan->umma, X, W, dY, dX, dW, db, &plan->timer)
+  int rc = plan->algo == CCT_ALGO_UMMA_3XTF32 ? umma_conv_backward(ctx, plan->umma, X, W, dY, dX, dW, db, &plan->timer, scaled)
                                               : simt_conv_backward(ctx, G, X, W, dY, dX, dW, db, &plan->timer);
   if (rc == CCT_OK && f->relu_mask_dx && dX) rc = cct_relu_backward(ctx, X, dX, dX, (size_t)G.B * G.D * G.n * G.n);
   return rc;

@@ -202,11 +202,13 @@ bool umma_supported(const ConvGeom& G);
 int umma_conv_forward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* bias, float* Y,
                       int relu, PhaseTimer* t, int batch = 0, bool repack = true);
 int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dY, float* dX,
-                       float* dW, float* db, PhaseTimer* t);
-// Whether umma_conv_backward takes dY in the form of `rows` (then dY = null), written there by the kernel that makes it;
-// umma_rows_scales comes before that kernel: dY is what a 3x3 / stride 2 pooling of P's windows makes of dP.
+                       float* dW, float* db, PhaseTimer* t, bool scaled = false);
+// Whether umma_conv_backward takes dY in the form of `rows` (then dY = null), written there by the kernel that makes it.
 bool umma_dy_rows(const UmmaPlan* p, DyRows* rows);
-int umma_rows_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, const int32_t* idx, int pooled);
+// Where dY is what pooling P's windows (k x k, stride s) makes of dP, the scales come from dP, which is smaller; before that kernel (whose rows need
+// them); umma_conv_backward is `scaled` then.
+int umma_pooled_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, const int32_t* idx, int k, int s,
+                       bool dgrad);
 int umma_conv_wgrad(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, float* dW, float* db, PhaseTimer* t,
                     const float* pack_W = nullptr);
 int umma_conv_dgrad(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, float* dX, PhaseTimer* t, int batch,

@@ -452,6 +452,7 @@ struct WgradParams {
   int kblocks_total, kblocks_per_split;  // end of this launch's k-block range, k-blocks per split
   int kb_first;                          // first k-block of this launch (a later round of a launch sequence starts further in)
   int* status;
+  const HalfScales* half = nullptr;      // wgrad_ts_kernel<true>: returns at once where wgrad_half_kernel takes the call
 };
 
 struct WgSmem {
@@ -751,6 +752,10 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
   const int grp = vg / P.tiles_per_group, ntile = vg % P.tiles_per_group;
   constexpr uint32_t kACol0 = 2 * kTsNTile;  // tensor memory: two accumulators of 192 columns, then 2 x 64 columns of A
 
+  if (WIDE && P.half) {
+    pdl_wait();
+    if (half_route(P.half, kHalfX, kHalfDy)) return;
+  }
   if (WIDE) {  // lowered rows that no warp stages: zeros
     const int words = (kTsRows - P.ones_row - 1) * 32;
     for (int i = tid; i < words * 2 * kTsStages; i += kTsThreads) {
@@ -1017,6 +1022,283 @@ __global__ void __launch_bounds__(ts_threads(WIDE), 1) wgrad_ts_kernel(const __g
             umma_tf32_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
             umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
             umma_tf32_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, 1u);
+          }
+        }
+        umma_commit(empty + 8u * s);
+        if (kbl == kblocks - 1) umma_commit(acc_full);
+      }
+      __syncwarp();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem_base, 512);
+}
+
+// The same in pairs of fp16, for stride 4 (AlexNet / CaffeNet conv1).  A stage is 64 pixels: one row of 128 bytes per lowered row for the hi
+// halves and one for the lo halves, so that a lane stores a whole word: it owns two neighbouring pixels, whose windows overlap - 15 of 22 elements
+// of a window row, at most five aligned 16-byte loads for both where each alone took three or four.  24 MMAs of 96 cycles per 64 pixels instead of per
+// 32, and half the stores.  Rows of an odd number of pixels have one more, so that neighbours are neighbours in memory: the last pair is the last two
+// pixels, the first of them a second time with a dY of 0 (its window is that of a real pixel: a value that is not finite in it stays in its
+// rows).  AlexNet conv1 at batch 256 358 -> 245 us (and 98 for the scales, which the data gradient shares).  The load-store pipe is 68 % busy then, a third
+// of it the MMAs' reads, issue 58 %: with the kernel size known at run time there were twice the instructions for a tap (285 us); stages of 32 pixels,
+// four of them, with half a warp to a window row, were slower (270: bank conflicts, registers).  The row of ones is not scaled.
+constexpr int kThTapWarps = 18, kThDyWarps = 8, kThThreads = (kThTapWarps + kThDyWarps + 1) * 32, kThPixels = 64;  // 864
+constexpr int kThWords = 20;  // five blocks: 13 taps and the neighbour's 4 more, at any alignment
+
+// Taps 0 .. K - 1 of two pixels, which start at w[SHIFT] and four words on, to lowered rows `row`, `row` + 1 ..; at[x]: the lane's word in a row whose
+// swizzle phase is x past that of the warp's first row, with `row`'s 128 bytes left to add.
+template <int K, int SHIFT, int PHASE>
+__device__ __forceinline__ void store_pairs(const float* w, uint8_t* row, const uint32_t* at, float scale) {
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    uint32_t h, l;
+    split_half2(w[SHIFT + r] * scale, w[SHIFT + 4 + r] * scale, h, l);
+    uint8_t* dst = row + at[(PHASE + r) & 7] + r * 128;
+    *reinterpret_cast<uint32_t*>(dst) = h;
+    *reinterpret_cast<uint32_t*>(dst + kTsTile) = l;
+  }
+}
+template <int K, int PHASE>
+__device__ __forceinline__ void store_shifted(const float* w, int shift, uint8_t* row, const uint32_t* at, float scale) {
+  switch ((int)warp_uniform((uint32_t)shift)) {
+    case 0: store_pairs<K, 0, PHASE>(w, row, at, scale); break;
+    case 1: store_pairs<K, 1, PHASE>(w, row, at, scale); break;
+    case 2: store_pairs<K, 2, PHASE>(w, row, at, scale); break;
+    default: store_pairs<K, 3, PHASE>(w, row, at, scale); break;
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(kThThreads, 1) wgrad_half_kernel(const __grid_constant__ WgradParams P) {
+  constexpr int kMmaWarp = kThTapWarps + kThDyWarps;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  const uint32_t full = base + kTsBarsOff, empty = full + 8u * kTsStages, acc_full = empty + 8u * kTsStages, tmem_slot = acc_full + 8u;
+  const int tid = threadIdx.x, warp = (int)warp_uniform(tid >> 5), lane = tid & 31;
+  const int split = blockIdx.y, vg = blockIdx.z;
+  const int grp = vg / P.tiles_per_group, ntile = vg % P.tiles_per_group;
+  constexpr uint32_t kACol0 = 2 * kTsNTile;  // tensor memory: two accumulators of 192 columns, then 2 x 64 columns of A
+
+  pdl_wait();
+  if (!half_route(P.half, kHalfX, kHalfDy)) return;
+  const HalfScale sx = P.half->of[kHalfX], sy = P.half->of[kHalfDy];
+  for (int i = tid; i < (kTsRows - P.ones_row - 1) * 32 * 2 * kTsStages; i += kThThreads) {  // lowered rows that no warp stages: zeros
+    const int words = (kTsRows - P.ones_row - 1) * 32, part = i / words;
+    reinterpret_cast<uint32_t*>(base_ptr + (size_t)part * kTsTile + (size_t)(P.ones_row + 1) * 128)[i - part * words] = 0u;
+  }
+  for (int i = tid; i < 32 * kTsStages; i += kThThreads) {  // the row of ones (in pairs of fp16), which needs no swizzle
+    uint8_t* at = base_ptr + (size_t)(i >> 5) * kTsStage + P.ones_row * 128 + (i & 31) * 4;
+    *reinterpret_cast<uint32_t*>(at) = 0x3c003c00u;
+    *reinterpret_cast<uint32_t*>(at + kTsTile) = 0u;
+  }
+  fence_proxy_async_smem();
+  if (tid == 0) {
+    for (int s = 0; s < kTsStages; ++s) { mbar_init(full + 8u * s, kThTapWarps + kThDyWarps); mbar_init(empty + 8u * s, 1); }
+    mbar_init(acc_full, 1);
+    fence_mbar_init();
+  }
+  if (warp == 0) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t tmem_base;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  // k-blocks of 64 pixels over rows of `pitch`
+  const int pitch = P.m + (P.m & 1), per_image = P.m * pitch, images = P.n_pix / P.mm;
+  const int total = (images * per_image + kThPixels - 1) / kThPixels, per_split = (total + (int)gridDim.y - 1) / (int)gridDim.y;
+  const int kb_begin = split * per_split, kblocks = max(0, min(total, kb_begin + per_split) - kb_begin);
+  bool failed = false;
+
+  if (warp < kMmaWarp) {
+    // this lane's pixel (tap warps: the first of two), advanced by `step`
+    int pb, pr, pc;
+    auto set_pixel = [&](int pix) {
+      pb = pix / per_image;
+      const int in = pix - pb * per_image;
+      pr = in / pitch;
+      pc = in - pr * pitch;
+    };
+    auto next_pixel = [&](int step) {
+      pc += step;
+      while (pc >= pitch) { pc -= pitch; ++pr; }
+      while (pr >= P.m) { pr -= P.m; ++pb; }
+    };
+    if (warp < kThTapWarps) {
+      // ---- window rows u = 2 warp and 2 warp + 1: lowered rows u * K + kc
+      set_pixel(kb_begin * kThPixels + 2 * lane);
+      const int units = P.ones_row / K, mine = min(kTsWideRows, max(0, units - kTsWideRows * warp));
+      const float* x = P.x + (long long)grp * P.x_group_stride;
+      int unit_at[kTsWideRows];
+#pragma unroll
+      for (int i = 0; i < kTsWideRows; ++i) {
+        const int u = kTsWideRows * warp + i, d = u / K;
+        unit_at[i] = d * P.n * P.n + (u - d * K) * P.n;
+      }
+      uint32_t at[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) at[r] = (uint32_t)lane * 4u ^ (uint32_t)(((kTsWideRows * warp * K + r) & 7) << 4);
+      uint8_t* row0 = base_ptr + kTsWideRows * warp * K * 128;
+      const float scale = __uint_as_float(warp_uniform(__float_as_uint(sx.scale)));
+      const int misaligned = (int)((reinterpret_cast<uintptr_t>(x) >> 2) & 3);  // words between x and its 16-byte block
+      float w[kTsWideRows][kThWords];
+      int shift[kTsWideRows] = {0, 0};
+      auto load_rows = [&]() {
+        const bool ok = pb < images;
+        const int col = pc + 1 < P.m ? pc : pc - 1;  // the last pair of an odd row
+        const int at0 = pb * (int)P.x_batch_stride + pr * 4 * P.n + col * 4;
+        const int pb0 = __shfl_sync(0xffffffffu, pb, 0);
+        const bool one_image = __all_sync(0xffffffffu, ok && pb == pb0);
+        int far_r = pr, far_c = pc + 2 * kThPixels;  // the lines of the k-block after the next one, if it lies in the same image
+        while (far_c >= pitch) { far_c -= pitch; ++far_r; }
+        const bool far_in = ok && far_r < P.m && (lane & 3) == 0;
+        const int far0 = pb * (int)P.x_batch_stride + far_r * 4 * P.n + far_c * 4;
+#pragma unroll
+        for (int i = 0; i < kTsWideRows; ++i) {
+          if (i >= mine) break;
+          const int from = at0 + unit_at[i];
+          if (far_in) prefetch_l2(x + far0 + unit_at[i]);
+          shift[i] = (from + misaligned) & 3;  // of this lane; of every lane where the pixels are one image's
+          const int first = from - shift[i];
+          if (__all_sync(0xffffffffu, one_image && first >= 0 && first + kThWords <= P.x_count)) {
+            const float4* block = reinterpret_cast<const float4*>(x + first);
+#pragma unroll
+            for (int j = 0; j < (K + 4 + 3 + 3) / 4; ++j) {
+              if (4 * j >= K + 4 && 4 * j >= K + 4 + shift[i]) break;
+              const float4 v = __ldg(block + j);
+              w[i][4 * j] = v.x; w[i][4 * j + 1] = v.y; w[i][4 * j + 2] = v.z; w[i][4 * j + 3] = v.w;
+            }
+          } else {
+            shift[i] = 0;
+#pragma unroll
+            for (int r = 0; r < K + 4; ++r) w[i][r] = ok && from + r < P.x_count ? __ldg(x + from + r) : 0.f;
+          }
+        }
+      };
+      if (kblocks > 0) load_rows();
+      Ring ring;
+      for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(kTsStages)) {
+        const int s = ring.idx, use = ring.use;
+        if (use > 0) mbar_wait(empty + 8u * s, (uint32_t)(use - 1) & 1u, failed, P.status, 0x3110);
+        uint8_t* row = row0 + (size_t)s * kTsStage;
+        if (mine > 0) store_shifted<K, 0>(w[0], shift[0], row, at, scale);
+        if (mine > 1) store_shifted<K, K>(w[1], shift[1], row + K * 128, at, scale);
+        if (kbl + 1 < kblocks) {  // the next k-block's loads go in flight before the barrier work
+          next_pixel(kThPixels);
+          load_rows();
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + 8u * s);
+      }
+    } else {
+      // ---- dY: two warps per quadrant of channels (= the tensor-memory lanes a warp reaches, its number mod 4); each loads half of the channels and
+      // stores half of the pixels, 32 pixels at a time.
+      constexpr int kChannels = 16;
+      const int q = warp & 3, half = (warp - kThTapWarps) >> 2;
+      set_pixel(kb_begin * kThPixels + lane);
+      const int ch0 = q * 32 + half * kChannels;
+      const float* dyg = P.dy + (long long)(grp * P.dy_group_channels + ntile * P.n_real + ch0) * P.mm;
+      const int n_live = min(P.n_real, P.dy_group_channels - ntile * P.n_real);  // the last tile of a group may be shorter
+      const int live = min(kChannels, max(0, n_live - ch0));  // real channels of this warp
+      const bool any = n_live > q * 32;                       // of the quadrant
+      float* turn = reinterpret_cast<float*>(base_ptr + kTsTurnOff) + q * (32 * 33);
+      const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + kACol0 + (uint32_t)(half * 8);
+      if (!any) {  // zeros, once
+        const uint32_t zeros[8] = {};
+        for (int c = 0; c < kTsStages * 4; ++c) tmem_st8(lane_addr + (uint32_t)(c * 16), zeros);
+        tmem_wait_st();
+      }
+      auto quadrant_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory"); };
+      float vb[kChannels];
+      auto load_rows = [&]() {
+        // of the last pair of an odd row the second is the last pixel
+        const bool ok = pb < images && !(pc + 1 == P.m && pitch > P.m);
+        const int col = pc == P.m ? pc - 1 : pc;
+        const float* dsrc = dyg + (long long)pb * P.dy_batch_stride + pr * P.m + col;
+        // one lane per channel: the line four blocks of 32 on
+        if (lane < live && pr * P.m + col + 4 * kBlockK < P.mm && ok) prefetch_l2(dsrc + (long long)lane * P.mm + 4 * kBlockK - lane);
+#pragma unroll
+        for (int i = 0; i < kChannels; ++i) vb[i] = 0.f;
+        if (ok && live == kChannels) {
+#pragma unroll
+          for (int i = 0; i < kChannels; ++i) vb[i] = __ldg(dsrc + (size_t)i * P.mm);
+        } else if (ok) {
+#pragma unroll
+          for (int i = 0; i < kChannels; ++i)
+            if (i < live) vb[i] = __ldg(dsrc + (size_t)i * P.mm);
+        }
+      };
+      if (kblocks > 0 && any) load_rows();
+      Ring ring;
+      for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(kTsStages)) {
+        const int s = ring.idx, use = ring.use;
+#pragma unroll 1
+        for (int part = 0; any && part < 2; ++part) {  // 32 of the 64 pixels
+#pragma unroll
+          for (int i = 0; i < kChannels; ++i) turn[(half * kChannels + i) * 33 + lane] = vb[i];  // row = channel, column = pixel
+          quadrant_sync();
+          if (part == 0 || kbl + 1 < kblocks) {
+            next_pixel(kBlockK);
+            load_rows();
+          }
+          // The stage's 64 tensor-memory columns were last read by the MMAs of k-block kbl - 2.
+          if (part == 0 && use > 0) mbar_wait(empty + 8u * s, (uint32_t)(use - 1) & 1u, failed, P.status, 0x3111);
+          tc_fence_after();
+          uint32_t hi[8], lo[8];  // lane = channel now: sixteen of its pixels
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float* t = turn + lane * 33 + half * 16 + 2 * e;
+            split_half2(t[0] * sy.scale, t[1] * sy.scale, hi[e], lo[e]);
+          }
+          const uint32_t st_addr = lane_addr + (uint32_t)(s * 64 + part * 16);
+          tmem_st8(st_addr, hi);
+          tmem_st8(st_addr + 32u, lo);
+          quadrant_sync();  // every lane has read the tile before the next 32 pixels overwrite it
+        }
+        if (!any && use > 0) mbar_wait(empty + 8u * s, (uint32_t)(use - 1) & 1u, failed, P.status, 0x3112);  // (or the barrier would run ahead)
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + 8u * s);
+      }
+      // ---- epilogue: lane = channel, one accumulator column = one lowered row
+      if (kblocks > 0) mbar_wait(acc_full, 0u, failed, P.status, 0x3120);
+      tc_fence_after();
+      const int ch = q * 32 + lane;
+      float* op = P.partial + ((size_t)split * gridDim.z + vg) * kTsRows * P.n_pad + ch;
+      for (int c = half; c < kTsRows / 16; c += 2) {
+        float acc[16];
+        tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 16), acc);
+        if (!failed && ch < P.n_pad) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            op[(size_t)(c * 16 + j) * P.n_pad] = kblocks > 0 ? acc[j] * (c * 16 + j == P.ones_row ? sy.inverse : sx.inverse * sy.inverse) : 0.f;
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ MMA issue (see elect_one)
+    const uint32_t idesc = make_idesc_f16(kTsNTile), tmem = warp_uniform(tmem_base);
+    Ring ring;
+    for (int kbl = 0; kbl < kblocks; ++kbl, ring.advance(kTsStages)) {
+      const int s = ring.idx;
+      mbar_wait(full + 8u * s, (uint32_t)ring.use & 1u, failed, P.status, 0x3140);
+      tc_fence_after();
+      const uint32_t st = base + (uint32_t)s * kTsStage;
+      const uint32_t a_hi = tmem + kACol0 + (uint32_t)(s * 64), a_lo = a_hi + 32u;
+      if (elect_one()) {
+#pragma unroll
+        for (int u = 0; u < kTsRows / kTsNTile; ++u) {
+          const uint32_t d_tmem = tmem + (uint32_t)(u * kTsNTile);
+          const uint64_t dbh = make_desc(st + (uint32_t)u * kTsNTile * 128u), dbl = make_desc(st + kTsTile + (uint32_t)u * kTsNTile * 128u);
+#pragma unroll
+          for (int j = 0; j < kThPixels / 16; ++j) {
+            const uint64_t adv = (uint64_t)(j * 2);
+            umma_f16_ts(d_tmem, a_lo + (uint32_t)(j * 8), dbh + adv, idesc, (kbl == 0 && j == 0) ? 0u : 1u);
+            umma_f16_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbl + adv, idesc, 1u);
+            umma_f16_ts(d_tmem, a_hi + (uint32_t)(j * 8), dbh + adv, idesc, 1u);
           }
         }
         umma_commit(empty + 8u * s);
@@ -1502,12 +1784,26 @@ GatherTiling choose_gather_tiling(int sms, long long pixel_tiles, int groups, in
 
 // What a launch of operand_scale_kernel over `elements` takes: 5.6 us for CaffeNet conv3's X and W at batch 32 (9 MB), 8.4 for X, dY and W
 // of conv4 (14 MB), 58 for those of conv2 at batch 256 (265 MB).
-// A contraction takes pairs of fp16 from kHalfMinUs on, if by the estimates (6 % rms) they save 1 - kHalfGain of it: operands that do not lie close
-// enough together pay for the look at them and gain nothing.
+// A contraction takes pairs of fp16 from kHalfMinUs on, if by the estimates (6 % rms) they save 1 - kHalfGain of it and kHalfLeastUs: operands that do not
+// lie close enough together pay for the look at them and gain nothing.
 // Blocks of several stride periods: for at least 1 - kTallGain of the data gradient; kTallUs: one launch more, which returns at once.
 constexpr int kMaxTallRows = 4;
 constexpr double kTallUs = 4.0, kTallGain = 0.93;
-constexpr double kHalfMinUs = 25.0, kHalfGain = 0.9;
+constexpr double kHalfMinUs = 25.0, kHalfGain = 0.95, kHalfLeastUs = 5.0;
+bool half_pays(double us, double saves) { return us > kHalfMinUs && saves > (1 - kHalfGain) * us && saves > kHalfLeastUs; }
+// Lowered matrices of 257 .. 384 rows (with the row of ones) and tiles of at most 128 filters: wgrad_ts_kernel; its wide loads: see there.  Below
+// eight taps a window row has fewer than three blocks' worth.  With stride 4 wgrad_half_kernel.
+bool ts_rows(int rows, int columns) { return round_up(rows + 1, kTileM) == kTsRows && columns <= kTileM; }
+bool ts_wide(const ConvGeom& G) {
+  return G.s % 4 == 0 && G.p == 0 && G.k >= 8 && G.k <= kTsWideTaps && G.Dg * G.k <= kTsWideRows * ts_tap_warps(true);
+}
+WgradKernel half_ts_kernel(int k) {
+  switch (k) {
+    case 8: return wgrad_half_kernel<8>;    case 9: return wgrad_half_kernel<9>;    case 10: return wgrad_half_kernel<10>;
+    case 11: return wgrad_half_kernel<11>;  case 12: return wgrad_half_kernel<12>;  default: return wgrad_half_kernel<13>;
+  }
+}
+bool half_ts(const ConvGeom& G, int rows, int columns) { return ts_rows(rows, columns) && ts_wide(G) && G.s == 4 && G.m > 1; }
 int wgrad_columns(const ConvGeom& G) {
   int chain;
   const int tiles = weight_grad_tiles(G.og, &chain);
@@ -1516,8 +1812,12 @@ int wgrad_columns(const ConvGeom& G) {
 // The share of the weight gradient's time that pairs of fp16 save (by the gather kernel: at least 512 lowered rows).  More than 128 columns: conv3, conv4 at
 // batch 256 253 -> 165 us, 210 -> 138, at batch 32 44 -> 31; 128 columns, bound by the gather: conv2 425 -> 345, conv5 159 -> 138, at batch
 // 32 65 -> 62, 64 -> 128 channels 56 x 56 50 -> 45.
-double half_weight_gradient(int rows, int columns) { return rows < 512 ? 0.0 : columns > 128 ? 0.3 : columns > 96 ? 0.1 : 0.0; }
-double scales_us(double elements) { return 4.0 + 4.0 * elements / 4e6; }
+// wgrad_half_kernel: AlexNet conv1 at batch 256 358 us -> 245.
+double half_weight_gradient(const ConvGeom& G, int rows, int columns) {
+  if (half_ts(G, rows, columns)) return 0.31;
+  return rows < 512 ? 0.0 : columns > 128 ? 0.3 : columns > 96 ? 0.1 : 0.0;
+}
+double scales_us(double elements) { return 4.0 + 4.0 * elements / 4.8e6; }
 
 }  // namespace
 
@@ -1570,6 +1870,7 @@ struct UmmaPlan {
   size_t w_smem = 0;
   bool w_small = false;             // weight gradient by small_wgrad_kernel
   int ws_rows = 0, ws_cols = 0, ws_pix = 0;  // its row tiles, channel tiles and pixels per split
+  bool w_half = false;              // weight gradient in pairs of fp16 (wgp.half, or wgrad_half_kernel in place of wgrad_ts_kernel)
   bool w_ts = false;  // weight gradient by wgrad_ts_kernel (dY through tensor memory) instead of wgrad_kernel
   MaskTap* w_taps = nullptr;
   float* w_partial = nullptr;
@@ -1606,10 +1907,6 @@ GatherKernel gather_kernel(const GatherProblem& gp, bool weight_grad, bool one, 
   return one ? gather_kernel_of<kByTap, true>(gp) : gather_kernel_of<kByTap>(gp);
 }
 int gather_smem_limit(const GatherProblem& gp) { return gp.sets == 2 ? 113 * 1024 : kSmemLimit; }
-// wgrad_ts_kernel's wide loads: see there.  Below eight taps a window row has fewer than three blocks' worth.
-bool ts_wide(const ConvGeom& G) {
-  return G.s % 4 == 0 && G.p == 0 && G.k >= 8 && G.k <= kTsWideTaps && G.Dg * G.k <= kTsWideRows * ts_tap_warps(true);
-}
 WgradKernel short_wgrad_kernel(const UmmaPlan* p) {
   if (!p->w_ts) return wgrad_pick(p->w_subs, p->w_npad);
   return ts_wide(p->G) ? wgrad_ts_kernel<true> : wgrad_ts_kernel<false>;
@@ -1804,7 +2101,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     GatherTiling tl = tiling(false, 0.0);
     // Pairs of fp16 where that makes up for a look at the operands.
     const GatherTiling paired = tiling(true, tl.chain);
-    const bool half = tl.us > kHalfMinUs && !f.inside && paired.tiles && paired.us + scales_us(elements_x(G) + elements_w(G)) < kHalfGain * tl.us;
+    const bool half = !f.inside && paired.tiles && half_pays(tl.us, tl.us - paired.us - scales_us(elements_x(G) + elements_w(G)));
     if (half) tl = paired;
     f.half_cross = tl.cross;
     f.tiles = tl.tiles;
@@ -1870,10 +2167,10 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       if (t.tiles && t.us + kTallUs < kTallGain * paired.us) { paired = t; paired.us += kTallUs; tall = b; }
     }
     // The two gradients share the look at dY: both in pairs of fp16, or one of them, or none.
-    const double wgrad_us = 2.0 * elements_w(G) * G.B * G.m * G.m / 230e6, wgrad_saves = wgrad_us * half_weight_gradient(p->fwd.k_real, wgrad_columns(G));
+    const double wgrad_us = 2.0 * elements_w(G) * G.B * G.m * G.m / (half_ts(G, p->fwd.k_real, wgrad_columns(G)) ? 152e6 : 230e6), wgrad_saves = wgrad_us * half_weight_gradient(G, p->fwd.k_real, wgrad_columns(G));
     const double dgrad_saves = tl.us - paired.us, dy = elements_y(G) + elements_w(G), x = elements_x(G);
     const double best = std::max(dgrad_saves - scales_us(dy), std::max(wgrad_saves - scales_us(dy + x), dgrad_saves + wgrad_saves - scales_us(dy + x)));
-    const bool worth = best > (1 - kHalfGain) * (tl.us + wgrad_us) && tl.us + wgrad_us > kHalfMinUs;
+    const bool worth = half_pays(tl.us + wgrad_us, best);
     const bool half = worth && paired.tiles && dgrad_saves > 0;
     wgrad_half = worth && wgrad_saves - scales_us(dy + x) + (half ? scales_us(dy) : 0) > 0;
     if (half && tall.rows == 1) tl = paired;
@@ -1947,7 +2244,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       if (u <= p->w_mtiles && u * (f.n_pad <= 64 ? 2 : 1) * f.n_pad <= 512 && 2 * wg_smem(f.n_pad, u, 2).stage_bytes + 8192 <= (uint32_t)kSmemLimit)
         subs = u;
     // 257 .. 384 rows and one channel tile of at most 128: the role-exchanged kernel, one CTA for all rows
-    p->w_ts = p->w_mtiles * kTileM == kTsRows && f.n_pad <= kTileM;
+    p->w_ts = ts_rows(f.k_real, f.n_pad);
     const int n_pix = G.B * G.m * G.m;
     p->w_kblocks_total = (n_pix + kBlockK - 1) / kBlockK;
     for (;; subs = 1) {
@@ -1984,6 +2281,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       sums = std::max(sums, (size_t)p->w_splits * G.g * f.tiles * p->ws_rows * kSwTile * p->ws_cols * kSwTile);
     }
     p->wg_gather = !p->w_small && f.k_real >= 512;  // see below
+    p->w_half = wgrad_half && !p->w_small && (p->wg_gather || half_ts(G, f.k_real, f.n_pad));
     if (!p->w_small && !p->wg_gather)
       sums = std::max(sums, (size_t)p->w_splits * G.g * f.tiles * p->w_mtiles * kTileM * f.n_pad);
     if (!p->wg_gather) {
@@ -2086,7 +2384,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
     if (G.bias) mem.room(&p->wg_plane_sums, (size_t)G.B * G.o);
     sums = std::max(sums, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
   }
-  if (p->fwd.half || p->dgr.half || p->wgp.half) {
+  if (p->fwd.half || p->dgr.half || p->w_half) {
     mem.table(&p->half_ticket, std::vector<uint32_t>(2, 0u));
     mem.room(&p->half, 1);
     mem.room(&p->half_parts, (size_t)ctx->sm_count * kScaleBlocksPerSm);
@@ -2109,6 +2407,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
   for (const GatherProblem* gp : {&p->fwd, &p->dgr, &p->wgp, &p->tall})
     if (rc == CCT_OK && gp->w) rc = set_smem(ctx, gather_kernel(*gp, gp == &p->wgp, gp->one, gp->half), gather_smem_limit(*gp));
   if (rc == CCT_OK && !p->w_small && !p->wg_gather) rc = set_smem(ctx, short_wgrad_kernel(p), kSmemLimit);
+  if (rc == CCT_OK && p->w_half && !p->wg_gather) rc = set_smem(ctx, half_ts_kernel(G.k), kSmemLimit);
   if (rc != CCT_OK) {
     umma_plan_destroy(ctx, p);
     return rc;
@@ -2307,13 +2606,17 @@ bool umma_dy_rows(const UmmaPlan* p, DyRows* rows) {
   return true;
 }
 
-int umma_rows_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, const int32_t* idx, int pooled) {
+int umma_pooled_scales(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dP, const float* P, const int32_t* idx, int k, int s,
+                       bool dgrad) {
   const ConvGeom& G = p->G;
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
-  if (!p->wgp.half && !p->dgr.half) return CCT_OK;
-  // an element is in up to four windows
-  launch_scales(ctx, p, {ScaleOf{p->wgp.half ? X : nullptr, nullptr, elements_x(G), kHalfX, 0}, ScaleOf{p->dgr.half ? W : nullptr, nullptr, elements_w(G), kHalfW, 0},
-                         ScaleOf{dP, P, (size_t)G.B * G.o * pooled * pooled, kHalfDy, 2, idx, pooled * pooled, G.m * G.m}});
+  if (!p->w_half && !(p->dgr.half && dgrad)) return CCT_OK;
+  const int pooled = (G.m - k) / s + 1, windows = (k + s - 1) / s;
+  int headroom = 0;  // an element is in up to windows^2 of them
+  while ((1 << headroom) < windows * windows) ++headroom;
+  launch_scales(ctx, p, {ScaleOf{p->w_half ? X : nullptr, nullptr, elements_x(G), kHalfX, 0},
+                         ScaleOf{p->dgr.half && dgrad ? W : nullptr, nullptr, elements_w(G), kHalfW, 0},
+                         ScaleOf{dP, P, (size_t)G.B * G.o * pooled * pooled, kHalfDy, headroom, idx, pooled * pooled, G.m * G.m}});
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
@@ -2325,7 +2628,7 @@ int data_gradient(cct_ctx* ctx, UmmaPlan* p, const float* W, const float* dY, fl
 }
 
 int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W, const float* dY, float* dX,
-                       float* dW, float* db, PhaseTimer* t) {
+                       float* dW, float* db, PhaseTimer* t, bool scaled) {
   const ConvGeom& G = p->G;
   const size_t nx = elements_x(G), ny = elements_y(G), nw = elements_w(G);
   // Small layers: the data gradient goes with the weight gradient, unless one writes where the other reads.
@@ -2335,8 +2638,8 @@ int umma_conv_backward(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* W
     if (small_together(ctx, p)) return weight_gradient(ctx, p, X, dY, dW, db, t, nullptr, &d, false);
   }
   if (*ctx->status_host != 0) return CCT_ERR_TIMEOUT;
-  if (dY && (p->wgp.half || (p->dgr.half && dX))) {  // (else umma_rows_scales)
-    launch_scales(ctx, p, {ScaleOf{p->wgp.half ? X : nullptr, nullptr, nx, kHalfX, 0}, ScaleOf{p->dgr.half && dX ? W : nullptr, nullptr, nw, kHalfW, 0},
+  if (!scaled && (p->w_half || (p->dgr.half && dX))) {
+    launch_scales(ctx, p, {ScaleOf{p->w_half ? X : nullptr, nullptr, nx, kHalfX, 0}, ScaleOf{p->dgr.half && dX ? W : nullptr, nullptr, nw, kHalfW, 0},
                            ScaleOf{dY, nullptr, ny, kHalfDy, 0}});
     CCT_CHECK_LAUNCH(ctx);
   }
@@ -2424,6 +2727,10 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
       }
     } else {
       if (p->w_ts) P.x_count = (int)((long long)G.B * G.D * G.n * G.n - (G.g - 1) * P.x_group_stride);
+      if (half && p->w_half) {
+        P.half = p->half;
+        launch_pdl(half_ts_kernel(G.k), dim3(grid), dim3(kThThreads), p->w_smem, ctx->stream, P);
+      }
       launch_pdl(short_wgrad_kernel(p), dim3(grid), dim3(p->w_ts ? ts_threads(ts_wide(G)) : kWgThreads), p->w_smem, ctx->stream, P);
     }
     t->end(1, ctx->stream);

@@ -95,6 +95,10 @@ def launches(ctx, call):
     # data gradients by tall blocks of pixels, two launches: by eight and single channels, strides, groups, one and two CTAs per SM
     ((128, 96, 27, 256, 5, 1, 2, 2), (3,), (6, 7)), ((64, 24, 60, 256, 5, 2, 2, 1), (2, 3, 4), (6, 7)), ((256, 20, 24, 50, 5, 1, 0, 1), (2,), (5, 6)),
     ((50, 31, 43, 250, 5, 1, 2, 1), (3, 4), (6, 7)),
+    # weight gradients of 257 - 384 lowered rows with stride 4, two launches as well: odd and even rows of pixels, window rows at every place of their
+    # 16-byte blocks, tiles of filters that end inside a quadrant, groups
+    ((90, 2, 200, 128, 12, 4, 0, 1), (2,), (6, 7)), ((90, 3, 190, 128, 10, 4, 0, 1), (2,), (6, 7)), ((90, 2, 201, 128, 13, 4, 0, 1), (2,), (6, 7)),
+    ((64, 4, 199, 256, 12, 4, 0, 2), (2, 3), (6, 7)), ((128, 3, 150, 120, 11, 4, 0, 1), (2,), (6, 7)),
 ])
 def test_pairs_of_fp16(ctx, layer, shape, forward, backward):
     B, D, n, o, k, s, p, g = shape
@@ -102,7 +106,9 @@ def test_pairs_of_fp16(ctx, layer, shape, forward, backward):
     X, W, b, dY = at.operands(D)
     assert launches(ctx, lambda: at.forward(X, W, b)) in forward and launches(ctx, lambda: at.backward(X, W, dY)) in backward
     Y, (dX, dW, db) = at.forward(X, W, b), at.backward(X, W, dY)
-    for got, ref, products, name in zip((Y, dX, dW, db), at.exact(X, W, b, dY), (D // g * k * k, o // g * k * k, 176 * 32, 1), ("Y", "dX", "dW", "db")):
+    # with stride 4 db is a row of the weight gradient (the row of ones), a chain of up to 176 blocks as the others; otherwise fp32 sums
+    chains = (D // g * k * k, o // g * k * k, 176 * 32, 176 * 32 if s == 4 else 1)
+    for got, ref, products, name in zip((Y, dX, dW, db), at.exact(X, W, b, dY), chains, ("Y", "dX", "dW", "db")):
         assert off(got, ref) <= bound(products), name
 
 
@@ -156,11 +162,12 @@ def test_operands_far_apart(layer, what):
     assert off(dW, dWr) <= 2 * bound(176 * 32)
 
 
+STRIDE_4 = [(90, 2, 201, 128, 13, 4, 0, 1), (128, 3, 150, 120, 11, 4, 0, 1)]
 TALL = [(128, 96, 27, 256, 5, 1, 2, 2), (64, 24, 60, 256, 5, 2, 2, 1), (256, 20, 24, 50, 5, 1, 0, 1), (50, 31, 43, 250, 5, 1, 2, 1)]
 
 
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
-@pytest.mark.parametrize("shape", [SHAPE] + TALL)
+@pytest.mark.parametrize("shape", [SHAPE] + TALL + STRIDE_4)
 def test_values_that_are_not_finite(layer, shape, value):
     """They reach their windows, and nothing else changes by a bit; the calls after them are what those before them were."""
     at = layer(shape)
@@ -186,6 +193,9 @@ def test_values_that_are_not_finite(layer, shape, value):
     others = torch.ones(o, dtype=torch.bool, device="cuda")
     others[[w[1] for w in where]] = False
     assert torch.equal(dWn[others], dW[others]) and not torch.isfinite(dbn[~others]).any() and torch.equal(dbn[others], db[others])
+    taps = torch.nn.grad.conv2d_weight((Xn != X).float(), W.shape, torch.ones_like(dY), s, p, 1, g) != 0
+    dWn = at.backward(Xn, W, dY)[1]
+    assert not torch.isfinite(dWn[taps]).any() and torch.equal(dWn[~taps], dW[~taps])
     assert torch.equal(at.forward(X, W, b), Y) and all(torch.equal(u, v) for u, v in zip(at.backward(X, W, dY), (dX, dW, db)))
 
 
