@@ -1565,17 +1565,11 @@ __global__ void __launch_bounds__(32 * SLICES) wgrad_reduce_flat_kernel(const fl
 // dY[b][c][pix] -> hi / lo [row of channel c][b * mm + pix] with row = channel tile * n_pad + channel inside the
 // tile (K-major rows of `row_len` floats, so a TMA box is 32 consecutive pixels x one channel tile), and the plane
 // sum of dY[b][c] for the bias gradient.  One block per plane at a time; every access is a coalesced run.
-// With `half` (and X and dY ok): pairs of fp16 in place of the low parts, and no values.
-// The rows' ends behind the last image are written too then (0): what another form has left there meets zeros, but may read as Inf.
-template <bool PAIRS>
 __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__ dY, float* __restrict__ hi,
                                                        float* __restrict__ lo, float* __restrict__ plane_sums,
                                                        int planes, int channels, int mm, int og, int ch_tile,
-                                                       int tiles_per_group, int n_pad, size_t row_len, const HalfScales* half) {
+                                                       int tiles_per_group, int n_pad, size_t row_len) {
   pdl_wait();
-  const bool pairs = PAIRS && half_route(half, kHalfX, kHalfDy);
-  const float scale = pairs ? half->of[kHalfDy].scale : 1.f;
-  const int batch = planes / channels;
   // One warp per plane at a time in chunks of 256 elements, the next chunk's loads (of this plane or the warp's next one) in
   // flight while the current one is stored; no block-wide synchronisation.  One chunk at a time left planes of 169 elements at
   // 4.0 TB/s (CaffeNet conv3 at batch 256 50.0 -> 45.6 us, conv5 32.7 -> 30.5, conv2 at batch 32 11.7 -> 10.4; planes of 729 at batch 256
@@ -1589,7 +1583,7 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
   struct Place {
     const float* src;
     size_t at;   // in hi and lo
-    int i0, plane, end;  // end: mm, or for the last image the end of the row
+    int i0, plane;
   };
   auto place = [&](int turn) {
     Place q;
@@ -1600,7 +1594,6 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
     q.src = dY + (size_t)q.plane * mm;
     q.at = ((size_t)(grp * tiles_per_group + tile) * n_pad + within) * row_len + (size_t)b * mm;
     q.i0 = -(int)(((size_t)b * mm) & 31);
-    q.end = PAIRS && b + 1 == batch ? (int)(row_len - (size_t)b * mm) : mm;
     return q;
   };
   float x[8], y[8];
@@ -1616,7 +1609,7 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
   float sum = 0.f;
   for (int turn = warp0;;) {
     Place next = q;
-    const bool plane_ends = q.i0 + 256 >= q.end;
+    const bool plane_ends = q.i0 + 256 >= mm;
     if (plane_ends) {
       turn += nwarps;
       if (turn < planes) next = place(turn);
@@ -1628,14 +1621,10 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
     for (int u = 0; u < 8; ++u) {
       const int i = q.i0 + u * 32 + lane;
       uint32_t h, l;
-      if (pairs) {
-        store_half_lane(lo + q.at + (i - lane), lane, x[u] * scale, i >= 0 && i < q.end);
-      } else {
-        split_tf32_trunc(x[u], h, l);
-        if (i >= 0 && i < q.end) {
-          hi[q.at + i] = __uint_as_float(h);
-          lo[q.at + i] = __uint_as_float(l);
-        }
+      split_tf32_trunc(x[u], h, l);
+      if (i >= 0 && i < mm) {
+        hi[q.at + i] = __uint_as_float(h);
+        lo[q.at + i] = __uint_as_float(l);
       }
       sum += x[u];
     }
@@ -1651,6 +1640,67 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
     q = next;
 #pragma unroll
     for (int u = 0; u < 8; ++u) x[u] = y[u];
+  }
+}
+
+// The same for a weight gradient that may take pairs of fp16 (`half`, and X and dY ok: pairs in place of the low parts, and no values).  A warp
+// writes kSplitRun consecutive elements of a row, two to a lane, whatever images they are of: whole lines of the rows and no lane without work (by planes of
+// 169 elements a third had none: CaffeNet conv3, batch 256, 48.5 -> 30 us).  The sums for the bias gradient are those of the runs, `plane_sums`
+// [run][channel].  The rows' ends behind the last image are written too (0): what another form has left there meets zeros, but may read as Inf.
+constexpr int kSplitRun = 1024, kSplitAhead = 4;
+__global__ void __launch_bounds__(256) split_dy_runs_kernel(const float* __restrict__ dY, float* __restrict__ hi, float* __restrict__ lo,
+                                                            float* __restrict__ run_sums, int batch, int channels, int mm, int og,
+                                                            int ch_tile, int tiles_per_group, int n_pad, size_t row_len, int runs,
+                                                            const HalfScales* half) {
+  pdl_wait();
+  const bool pairs = half_route(half, kHalfX, kHalfDy);
+  const float scale = pairs ? half->of[kHalfDy].scale : 1.f;
+  const int lane = threadIdx.x & 31, item = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (item >= channels * runs) return;
+  const int c = item / runs, run = item - c * runs;
+  const int grp = c / og, j = c - grp * og, tile = j / ch_tile;
+  const size_t row = ((size_t)(grp * tiles_per_group + tile) * n_pad + (j - tile * ch_tile)) * row_len;
+  const unsigned first = (unsigned)run * kSplitRun + 2u * lane, end = (unsigned)min((size_t)(run + 1) * kSplitRun, row_len);
+  // this lane's first element: image, place in the plane
+  int b = (int)(first / (unsigned)mm), r = (int)(first - (unsigned)b * mm);
+  const size_t image = (size_t)channels * mm;
+  const float* src = dY + (size_t)b * image + (size_t)c * mm;
+  float sum = 0.f;
+  for (unsigned q = first; q - 2u * lane < end; q += 64 * kSplitAhead) {
+    float x[kSplitAhead][2];
+#pragma unroll
+    for (int u = 0; u < kSplitAhead; ++u) {
+      const bool wraps = r + 1 == mm;  // the second element is the next image's first
+      x[u][0] = b < batch ? __ldg(src + r) : 0.f;
+      x[u][1] = b + (wraps ? 1 : 0) < batch ? __ldg(wraps ? src + image : src + r + 1) : 0.f;
+      r += 64;
+      while (r >= mm) { r -= mm; ++b; src += image; }
+    }
+#pragma unroll
+    for (int u = 0; u < kSplitAhead; ++u) {
+      const unsigned at = q + 64u * u;
+      if (at >= end) continue;  // (whole rows of 32: both elements, half a warp)
+      if (pairs) {
+        uint32_t h, l;
+        split_half2(x[u][0] * scale, x[u][1] * scale, h, l);
+        uint32_t* word = reinterpret_cast<uint32_t*>(lo + row + half_word(at));
+        word[0] = h;
+        word[kHalfLo] = l;
+      } else {
+        uint32_t h[2], l[2];
+        split_tf32_trunc(x[u][0], h[0], l[0]);
+        split_tf32_trunc(x[u][1], h[1], l[1]);
+        *reinterpret_cast<uint2*>(hi + row + at) = make_uint2(h[0], h[1]);
+        *reinterpret_cast<uint2*>(lo + row + at) = make_uint2(l[0], l[1]);
+      }
+      sum += x[u][0];
+      sum += x[u][1];
+    }
+  }
+  if (run_sums) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) run_sums[(size_t)run * channels + c] = sum;
   }
 }
 
@@ -2381,7 +2431,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       }
     mem.table(&p->wg_pix, t);
     finish_problem(mem, w, vgroups, 0, ctx->planning_sms(), (long long)base_tiles * p->wg_splits, wgrad_half);
-    if (G.bias) mem.room(&p->wg_plane_sums, (size_t)G.B * G.o);
+    if (G.bias) mem.room(&p->wg_plane_sums, std::max<size_t>(G.B, (w.map_k + kSplitRun - 1) / kSplitRun) * G.o);
     sums = std::max(sums, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
   }
   if (p->fwd.half || p->dgr.half || p->w_half) {
@@ -2666,10 +2716,14 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     GatherProblem& w = p->wgp;
     const int vgroups = G.g * f.tiles, mm = G.m * G.m;
     t->begin(1, ctx->stream);
-    if (dY)  // (else the kernel that made it has written the rows)
-      launch_pdl(w.half ? split_dy_kernel<true> : split_dy_kernel<false>, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, 
-        dY, w.w, w.w + w.w_half, G.bias ? p->wg_plane_sums : nullptr, G.B * G.o, G.o, mm, G.og, f.n, f.tiles,
-        f.n_pad, w.map_k, half && w.half ? p->half : nullptr);
+    float* sums = G.bias ? p->wg_plane_sums : nullptr;
+    const int runs = w.half ? (int)((w.map_k + kSplitRun - 1) / kSplitRun) : 0;
+    if (dY && w.half)  // (without dY the kernel that made it has written the rows)
+      launch_pdl(split_dy_runs_kernel, dim3((G.o * runs + 7) / 8), dim3(256), 0, ctx->stream, dY, w.w, w.w + w.w_half, sums, G.B, G.o, mm, G.og, f.n,
+                 f.tiles, f.n_pad, w.map_k, runs, half ? p->half : nullptr);
+    else if (dY)
+      launch_pdl(split_dy_kernel, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, dY, w.w, w.w + w.w_half, sums,
+                 G.B * G.o, G.o, mm, G.og, f.n, f.tiles, f.n_pad, w.map_k);
     CCT_CHECK_LAUNCH(ctx);
     GatherParams P{};
     P.in = X; P.out = p->w_partial; P.bias = nullptr;
@@ -2685,7 +2739,7 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     launch_gather(ctx, P, w, true);
     t->end(1, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
-    if (G.bias) extras.bias = BiasSum{p->wg_plane_sums, db, G.B, G.o, 0};
+    if (G.bias) extras.bias = BiasSum{p->wg_plane_sums, db, dY && w.half ? runs : G.B, G.o, 0};
     t->begin(2, ctx->stream);
     launch_wgrad_reduce(ctx, p->w_partial, dW, nullptr, p->wg_splits, vgroups, f.tiles, p->wg_mtiles * kTileM, f.n,
                         f.n_pad, f.k_real, G.og, 0, extras, tall);

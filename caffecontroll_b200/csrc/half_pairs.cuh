@@ -39,23 +39,6 @@ __device__ __forceinline__ bool half_route(const HalfScales* half, int a, int b)
 // Whether a data gradient by tall blocks of pixels (GatherProblem::rows) takes them.
 __device__ __forceinline__ bool tall_route(const HalfScales* half) { return half_route(half, kHalfDy, kHalfW) && half->of[kHalfDy].bad <= kMaxBad; }
 
-// A warp writes up to 32 elements of such a row, lane = element of the 32 at `block`: pairs of lanes share a word, except where only one of
-// them is `in` (the ends of an image whose size is odd).
-__device__ __forceinline__ void store_half_lane(float* block, int lane, float v, bool in) {
-  const bool odd = lane & 1;
-  const float other = __shfl_xor_sync(0xffffffffu, v, 1);
-  const bool both = __shfl_xor_sync(0xffffffffu, in ? 1 : 0, 1) && in;
-  uint32_t h, l;
-  split_half2(odd ? other : v, odd ? v : other, h, l);
-  if (both) {
-    reinterpret_cast<uint32_t*>(block)[(lane >> 1) + (odd ? kHalfLo : 0)] = odd ? l : h;
-  } else if (in) {
-    uint16_t* at = reinterpret_cast<uint16_t*>(block) + lane;
-    at[0] = (uint16_t)(odd ? h >> 16 : h);
-    at[2 * kHalfLo] = (uint16_t)(odd ? l >> 16 : l);
-  }
-}
-
 // Two consecutive elements, the first at an even place: the values to `value`, their halves into the row at `low` (both at the first element;
 // `within`: its place in its 32).
 __device__ __forceinline__ void store_half_pair(float* value, float* low, float x0, float x1, float scale, bool in0, bool in1, int within) {
