@@ -1643,14 +1643,23 @@ __global__ void __launch_bounds__(256) split_dy_kernel(const float* __restrict__
   }
 }
 
-// The same for a weight gradient that may take pairs of fp16 (`half`, and X and dY ok: pairs in place of the low parts, and no values).  A warp
-// writes kSplitRun consecutive elements of a row, two to a lane, whatever images they are of: whole lines of the rows and no lane without work (by planes of
-// 169 elements a third had none: CaffeNet conv3, batch 256, 48.5 -> 30 us).  The sums for the bias gradient are those of the runs, `plane_sums`
-// [run][channel].  The rows' ends behind the last image are written too (0): what another form has left there meets zeros, but may read as Inf.
-constexpr int kSplitRun = 1024, kSplitAhead = 4;
+// The same by runs of a channel's row, whatever images they are of: a warp writes `len` consecutive elements, two to a lane - whole lines of the rows and no
+// lane without work (by planes of 169 elements a third had none: CaffeNet conv3, batch 256, in pairs of fp16 48 -> 25 us), and as many warps as there
+// are runs (2 images, 64 channels 112 x 112: 128 planes 29.1 us, runs 5.3).  With `half`, and X and dY ok, pairs of fp16 in place of the low parts, and no
+// values.  The sums for the bias gradient are those of the runs, [run][channel].  The rows' ends behind the last image are written too (0): what another
+// form has left there meets zeros, but may read as Inf.
+// Many large planes stay with the other kernel where there are no pairs: 32 images, 256 channels 27 x 27 13.0 us, here 13.8; and so do layers whose gradient a
+// pooling layer could write (tiles of channels without padding).
+constexpr int kSplitRun = 1024, kSplitAhead = 4, kSplitRunLeast = 64 * kSplitAhead;
+bool split_by_planes(int planes, int mm) { return planes >= 4096 && mm >= 512; }
+int split_run(int channels, size_t row_len, int sms) {
+  int len = kSplitRun;  // shorter ones until every SM has sixteen warps
+  while (len > kSplitRunLeast && channels * (double)row_len < 16.0 * sms * len) len /= 2;
+  return len;
+}
 __global__ void __launch_bounds__(256) split_dy_runs_kernel(const float* __restrict__ dY, float* __restrict__ hi, float* __restrict__ lo,
                                                             float* __restrict__ run_sums, int batch, int channels, int mm, int og,
-                                                            int ch_tile, int tiles_per_group, int n_pad, size_t row_len, int runs,
+                                                            int ch_tile, int tiles_per_group, int n_pad, size_t row_len, int runs, int len,
                                                             const HalfScales* half) {
   pdl_wait();
   const bool pairs = half_route(half, kHalfX, kHalfDy);
@@ -1660,7 +1669,7 @@ __global__ void __launch_bounds__(256) split_dy_runs_kernel(const float* __restr
   const int c = item / runs, run = item - c * runs;
   const int grp = c / og, j = c - grp * og, tile = j / ch_tile;
   const size_t row = ((size_t)(grp * tiles_per_group + tile) * n_pad + (j - tile * ch_tile)) * row_len;
-  const unsigned first = (unsigned)run * kSplitRun + 2u * lane, end = (unsigned)min((size_t)(run + 1) * kSplitRun, row_len);
+  const unsigned first = (unsigned)run * len + 2u * lane, end = (unsigned)min((size_t)(run + 1) * len, row_len);
   // this lane's first element: image, place in the plane
   int b = (int)(first / (unsigned)mm), r = (int)(first - (unsigned)b * mm);
   const size_t image = (size_t)channels * mm;
@@ -2431,7 +2440,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       }
     mem.table(&p->wg_pix, t);
     finish_problem(mem, w, vgroups, 0, ctx->planning_sms(), (long long)base_tiles * p->wg_splits, wgrad_half);
-    if (G.bias) mem.room(&p->wg_plane_sums, std::max<size_t>(G.B, (w.map_k + kSplitRun - 1) / kSplitRun) * G.o);
+    if (G.bias) mem.room(&p->wg_plane_sums, std::max<size_t>(G.B, (w.map_k + kSplitRunLeast - 1) / kSplitRunLeast) * G.o);
     sums = std::max(sums, (size_t)p->wg_splits * vgroups * p->wg_mtiles * kTileM * f.n_pad);
   }
   if (p->fwd.half || p->dgr.half || p->w_half) {
@@ -2717,10 +2726,13 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     const int vgroups = G.g * f.tiles, mm = G.m * G.m;
     t->begin(1, ctx->stream);
     float* sums = G.bias ? p->wg_plane_sums : nullptr;
-    const int runs = w.half ? (int)((w.map_k + kSplitRun - 1) / kSplitRun) : 0;
-    if (dY && w.half)  // (without dY the kernel that made it has written the rows)
+    // Without dY the kernel that made it has written the rows, whose sums are those of planes: where it could, a dY of its own gives the same sums.
+    const bool planes = !dY || (!w.half && (p->dgr_row_taps || split_by_planes(G.B * G.o, mm)));
+    const int len = split_run(G.o, w.map_k, ctx->sm_count), runs = (int)((w.map_k + len - 1) / len);
+    if (!planes)
       launch_pdl(split_dy_runs_kernel, dim3((G.o * runs + 7) / 8), dim3(256), 0, ctx->stream, dY, w.w, w.w + w.w_half, sums, G.B, G.o, mm, G.og, f.n,
-                 f.tiles, f.n_pad, w.map_k, runs, half ? p->half : nullptr);
+                 f.tiles, f.n_pad, w.map_k, runs, len,
+                 half && w.half ? p->half : nullptr);
     else if (dY)
       launch_pdl(split_dy_kernel, dim3(std::min((G.B * G.o + 7) / 8, ctx->sm_count * 8)), dim3(256), 0, ctx->stream, dY, w.w, w.w + w.w_half, sums,
                  G.B * G.o, G.o, mm, G.og, f.n, f.tiles, f.n_pad, w.map_k);
@@ -2739,7 +2751,7 @@ int weight_gradient(cct_ctx* ctx, UmmaPlan* p, const float* X, const float* dY, 
     launch_gather(ctx, P, w, true);
     t->end(1, ctx->stream);
     CCT_CHECK_LAUNCH(ctx);
-    if (G.bias) extras.bias = BiasSum{p->wg_plane_sums, db, dY && w.half ? runs : G.B, G.o, 0};
+    if (G.bias) extras.bias = BiasSum{p->wg_plane_sums, db, planes ? G.B : runs, G.o, 0};
     t->begin(2, ctx->stream);
     launch_wgrad_reduce(ctx, p->w_partial, dW, nullptr, p->wg_splits, vgroups, f.tiles, p->wg_mtiles * kTileM, f.n,
                         f.n_pad, f.k_real, G.og, 0, extras, tall);
