@@ -1868,13 +1868,24 @@ int wgrad_columns(const ConvGeom& G) {
   const int tiles = weight_grad_tiles(G.og, &chain);
   return round_up((G.og + tiles - 1) / tiles, 16);
 }
-// The share of the weight gradient's time that pairs of fp16 save (by the gather kernel: at least 512 lowered rows).  More than 128 columns: conv3, conv4 at
-// batch 256 253 -> 165 us, 210 -> 138, at batch 32 44 -> 31; 128 columns, bound by the gather: conv2 425 -> 345, conv5 159 -> 138, at batch
-// 32 65 -> 62, 64 -> 128 channels 56 x 56 50 -> 45.
-// wgrad_half_kernel: AlexNet conv1 at batch 256 358 us -> 245.
-double half_weight_gradient(const ConvGeom& G, int rows, int columns) {
-  if (half_ts(G, rows, columns)) return 0.31;
-  return rows < 512 ? 0.0 : columns > 128 ? 0.3 : columns > 96 ? 0.1 : 0.0;
+// From how many lowered rows on the weight gradient goes through the gather kernel, which needs dY in rows: see umma_plan_create; and in pairs of
+// fp16, whose MMAs the short kernels' staging from shared memory would not keep up with.
+constexpr int kGatherRows = 512, kGatherHalfRows = 320;
+bool half_gather(const ConvGeom& G, int rows, int columns) { return rows >= kGatherRows || (rows >= kGatherHalfRows && !ts_rows(rows, columns) && columns > 96); }
+// What the weight gradient takes (us), and what pairs of fp16 save of it.  By the gather kernel, more than 128 columns: conv3, conv4 at batch 256 253 -> 165
+// us, 210 -> 138, at batch 32 44 -> 31; 128 columns, bound by the gather: conv2 425 -> 345, conv5 159 -> 138, at batch 32 65 -> 62, 64 -> 128
+// channels 56 x 56 50 -> 45.  With fewer rows than kGatherRows dY is turned into rows for it: 48 -> 192 channels 28 x 28, 64 images (432 rows) 73 -> 34 + 16,
+// 40 -> 370 30 x 30, 50 images (360) 97 -> 44 + 24, 16 -> 128 40 x 40 5 x 5, 100 images (400) 127 -> 69 + 28; 24 -> 296, 72 x 72 by 2, 30 images (216)
+// 51 -> 34 + 17: no.  wgrad_half_kernel: AlexNet conv1 at batch 256 358 -> 245.
+struct WgradTime {
+  double us, saves;
+};
+WgradTime weight_gradient_time(const ConvGeom& G, int rows, int columns) {
+  const double flops = 2.0 * elements_w(G) * G.B * G.m * G.m;
+  if (half_ts(G, rows, columns)) return {flops / 152e6, 0.31 * flops / 152e6};
+  if (rows >= kGatherRows) return {flops / 230e6, (columns > 128 ? 0.3 : columns > 96 ? 0.1 : 0.0) * flops / 230e6};
+  const double us = flops / 125e6;
+  return {us, half_gather(G, rows, columns) ? 0.45 * us - 3.0 - elements_y(G) * 8.0 / 5e6 : 0.0};
 }
 double scales_us(double elements) { return 4.0 + 4.0 * elements / 4.8e6; }
 
@@ -2226,7 +2237,8 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       if (t.tiles && t.us + kTallUs < kTallGain * paired.us) { paired = t; paired.us += kTallUs; tall = b; }
     }
     // The two gradients share the look at dY: both in pairs of fp16, or one of them, or none.
-    const double wgrad_us = 2.0 * elements_w(G) * G.B * G.m * G.m / (half_ts(G, p->fwd.k_real, wgrad_columns(G)) ? 152e6 : 230e6), wgrad_saves = wgrad_us * half_weight_gradient(G, p->fwd.k_real, wgrad_columns(G));
+    const WgradTime wgrad = weight_gradient_time(G, p->fwd.k_real, wgrad_columns(G));
+    const double wgrad_us = wgrad.us, wgrad_saves = wgrad.saves;
     const double dgrad_saves = tl.us - paired.us, dy = elements_y(G) + elements_w(G), x = elements_x(G);
     const double best = std::max(dgrad_saves - scales_us(dy), std::max(wgrad_saves - scales_us(dy + x), dgrad_saves + wgrad_saves - scales_us(dy + x)));
     const bool worth = half_pays(tl.us + wgrad_us, best);
@@ -2339,7 +2351,7 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       p->w_splits = (n_pix + p->ws_pix - 1) / p->ws_pix;
       sums = std::max(sums, (size_t)p->w_splits * G.g * f.tiles * p->ws_rows * kSwTile * p->ws_cols * kSwTile);
     }
-    p->wg_gather = !p->w_small && f.k_real >= 512;  // see below
+    p->wg_gather = !p->w_small && (f.k_real >= kGatherRows || (wgrad_half && half_gather(G, f.k_real, f.n_pad)));  // see below
     p->w_half = wgrad_half && !p->w_small && (p->wg_gather || half_ts(G, f.k_real, f.n_pad));
     if (!p->w_small && !p->wg_gather)
       sums = std::max(sums, (size_t)p->w_splits * G.g * f.tiles * p->w_mtiles * kTileM * f.n_pad);
@@ -2381,7 +2393,9 @@ int umma_plan_create(cct_ctx* ctx, const ConvGeom& G, bool tensor_only, UmmaPlan
       const bool two_per_sm = f.n_pad <= 128;  // the shape finish_problem() will pick for this accumulator width
       const int slots = ctx->planning_sms() * (two_per_sm ? 2 : 1);
       const double us_per_kblock = 12.0 * (f.n_pad / 2.0) / 1900.0 * (two_per_sm ? 2.0 : 1.0);
-      const int s_min = std::max(1, (kb_total + p->w_chain - 1) / p->w_chain);
+      // (half the additions per k-block in pairs of fp16: no less accurate than the short kernels that would have taken the layer)
+      const int chain = f.k_real >= kGatherRows ? p->w_chain : std::min(p->w_chain, 2 * p->w_kblocks_per_split);
+      const int s_min = std::max(1, (kb_total + chain - 1) / chain);
       // First without the set-up, among units of at least sixteen k-blocks; then with it, among units no longer than that:
       // a set-up would rather have fewer splits, whose longer chains are less accurate.
       for (const int setup : {0, 5}) {

@@ -95,6 +95,8 @@ def launches(ctx, call):
     # data gradients by tall blocks of pixels, two launches: by eight and single channels, strides, groups, one and two CTAs per SM
     ((128, 96, 27, 256, 5, 1, 2, 2), (3,), (6, 7)), ((64, 24, 60, 256, 5, 2, 2, 1), (2, 3, 4), (6, 7)), ((256, 20, 24, 50, 5, 1, 0, 1), (2,), (5, 6)),
     ((50, 31, 43, 250, 5, 1, 2, 1), (3, 4), (6, 7)),
+    # weight gradients of 320 - 511 lowered rows, by the gather kernel
+    ((100, 16, 40, 128, 5, 1, 2, 1), (2, 3), (6, 7)), ((100, 45, 41, 333, 3, 1, 1, 1), (3, 4), (6, 7)),
     # weight gradients of 257 - 384 lowered rows with stride 4, two launches as well: odd and even rows of pixels, window rows at every place of their
     # 16-byte blocks, tiles of filters that end inside a quadrant, groups
     ((90, 2, 200, 128, 12, 4, 0, 1), (2,), (6, 7)), ((90, 3, 190, 128, 10, 4, 0, 1), (2,), (6, 7)), ((90, 2, 201, 128, 13, 4, 0, 1), (2,), (6, 7)),
