@@ -9,7 +9,7 @@ one process per GPU.
 Prints ONE JSON line (rank 0).  `value` is whole-job images/s with inputs resident in HBM, device-timed, maximum over
 ranks; `e2e` is the same metric with every step's inputs uploaded from pinned host memory and the loss (or the host-buffer
 calls' outputs) read back inside the timed region; `roofline` describes the slowest contraction kernel group against
-the 3xTF32 tensor roofline measured in the same run; `cpu_baseline` is the reference CPU path timed on this box's host
+the tensor roofline of three 16-bit products per multiply-add; `cpu_baseline` is the reference CPU path timed on this box's host
 cores in the same run.
 """
 import argparse
@@ -140,18 +140,18 @@ def measure_tf32_peak(seconds=2.0):
 
 
 def tensor_roofline(peaks, measure=True):
-    """fp32-equivalent 3xTF32 roofline in TFLOP/s: the measured TF32 matmul rate / 3 (three MMAs per product)."""
+    """fp32-equivalent roofline in TFLOP/s: the measured rate of 16-bit matmuls / 3 (the larger contractions' three products of fp16 pairs; the
+    others' are three of TF32, whose measured rate stands beside it)."""
     out = {"bf16_burst": peaks["bf16_tflops"], "bf16_sustained": peaks.get("bf16_tflops_sustained")}
     if measure:
         burst, sustained = measure_tf32_peak()
-        out.update(tf32_burst=burst, tf32_sustained=sustained, peak=burst / 3.0, peak_sustained=sustained / 3.0,
-                   source="TF32 8192^3 library matmul measured in this run: burst %.1f, sustained %.1f TFLOP/s; / 3 for "
-                          "3xTF32 - of measured (bf16 in MEASURED_PEAKS.json: %.1f burst)" %
-                          (burst, sustained, peaks["bf16_tflops"]))
+        out.update(tf32_burst=burst, tf32_sustained=sustained)
     else:
-        out.update(tf32_burst=None, tf32_sustained=None, peak=peaks["bf16_tflops"] / 6.0,
-                   peak_sustained=(peaks.get("bf16_tflops_sustained") or 0) / 6.0,
-                   source="%s: bf16 burst %.1f TFLOP/s / 2 (assumed TF32 rate) / 3" % (peaks["source"], peaks["bf16_tflops"]))
+        out.update(tf32_burst=None, tf32_sustained=None)
+    out.update(peak=peaks["bf16_tflops"] / 3.0, peak_sustained=(peaks.get("bf16_tflops_sustained") or 0) / 3.0,
+               source="%s: 16-bit matmul burst %.1f, sustained %.1f TFLOP/s, / 3 - of measured%s" %
+                      (peaks["source"], peaks["bf16_tflops"], peaks.get("bf16_tflops_sustained") or 0,
+                       "; TF32 8192^3 library matmul in this run: burst %.1f, sustained %.1f" % (burst, sustained) if measure else ""))
     return out
 
 
@@ -438,7 +438,7 @@ def run_conv_stack(args, rank, world, local_rank):
                            "dgrad_tflops": F / (k_ms[3] * 1e-3) / 1e12 if needs_dx and k_ms[3] > 0 else None}
     if rank == 0:
         peaks = load_peaks()
-        peak = peaks["bf16_tflops"] / 6.0
+        peak = peaks["bf16_tflops"] / 3.0
         tf = world * flops / (ms_step * 1e-3) / 1e12
         line = {
             "metric": METRIC, "value": world * B / (ms_step * 1e-3), "unit": "images/s", "n_gpus": world,
@@ -451,8 +451,8 @@ def run_conv_stack(args, rank, world, local_rank):
             "tflops": tf,
             "roofline": {"bound": "tensor", "kernel": "all contraction kernels of the five layers", "achieved": tf / world,
                          "peak": peak, "unit": "TFLOP/s", "frac": tf / world / peak, "traffic": None,
-                         "peak_source": "%s: bf16 burst %.1f TFLOP/s / 2 / 3 - of measured; sustained figure %.1f" %
-                                        (peaks["source"], peaks["bf16_tflops"], (peaks.get("bf16_tflops_sustained") or 0) / 6.0),
+                         "peak_source": "%s: 16-bit matmul burst %.1f TFLOP/s / 3 - of measured; sustained figure %.1f" %
+                                        (peaks["source"], peaks["bf16_tflops"], (peaks.get("bf16_tflops_sustained") or 0) / 3.0),
                          "flops_per_step": flops, "layers": per_layer},
             "cpu_baseline": None, "e2e": None, "clocks": clocks, "gpu_launches": timed_launches,
         }
