@@ -2594,8 +2594,32 @@ void launch_gather(cct_ctx* ctx, const GatherParams& P, const GatherProblem& gp,
   }
 }
 
+// The scales of a call's operands (a = null: not needed) in one launch.
+struct ScaleOf {
+  const float *a, *mask;
+  size_t n;
+  int slot, headroom;
+  const int32_t* where = nullptr;
+  int pooled = 1, plane = 1;
+};
 void launch_scales(cct_ctx* ctx, const UmmaPlan* p, std::initializer_list<ScaleOf> operands) {
-  launch_scales(ctx, p->half, p->half_parts, p->half_ticket, operands);
+  ScaleJobs J{};
+  J.out = p->half; J.parts = p->half_parts; J.ticket = p->half_ticket;
+  size_t total = 0;
+  for (const ScaleOf& o : operands) total += o.a ? o.n : 0;
+  const size_t blocks = (size_t)ctx->sm_count * kScaleBlocksPerSm - 3;  // rounded up for each of three
+  const size_t per_block = (std::max<size_t>(kScaleChunk, (total + blocks - 1) / blocks) + 1023) & ~(size_t)1023;
+  int grid = 0;
+  for (const ScaleOf& o : operands) {
+    if (!o.a) continue;
+    ScaleJob& job = J.job[J.jobs++];
+    job.a = o.a; job.mask = o.mask; job.n = o.n; job.per_block = per_block; job.slot = o.slot; job.headroom = o.headroom;
+    job.where = o.where; job.pooled = o.pooled; job.plane = o.plane;
+    job.first = grid;
+    job.blocks = (int)((o.n + per_block - 1) / per_block);
+    grid += job.blocks;
+  }
+  launch_pdl(operand_scale_kernel, dim3(grid), dim3(kScaleThreads), 0, ctx->stream, J);
 }
 
 }  // namespace

@@ -18,19 +18,11 @@
 // fp32 in tensor memory.  Long reductions are split over CTAs (bounded accumulation chains, as in the convolution
 // kernels); a small kernel adds the partial sums in split order and applies bias / ReLU / dropout (forward) or the
 // masks of the bridges in front of the layer (data gradient).
-//
-// Large layers of more than 128 images contract pairs of fp16 instead (half_pairs.cuh; operand_scale.cuh has what an operand has to be like): B, small,
-// is looked at and split once per call, A is split by the transform warps.  The weights are too many to be read beforehand (151 MB in fc6: 25 us of
-// the 34 that are saved): their scale comes from a sample, a thirty-second of them, with four octaves to spare, and the transform warps look
-// whether a value is too large for it or a row too small; then a launch behind, which otherwise returns at once (3 us), does the contraction on tf32.
-// fc6, batch 256, both ways 289 -> 227 us.
 #include <algorithm>
 #include <cstdio>
 #include <new>
 
 #include "cct_internal.h"
-#include "half_pairs.cuh"
-#include "operand_scale.cuh"
 #include "umma_ptx.cuh"
 
 namespace {
@@ -82,95 +74,9 @@ __device__ __forceinline__ void fc_store_3d(const void* tmap, uint32_t src, int 
                : "memory");
 }
 
-// A contraction in pairs of fp16: the operands' scales, what takes the sum back, and where to say that a value of A lay outside.
-struct FcHalf {
-  float scale_a, back;
-  int* outside;
-};
-constexpr float kFcHalfMost = 65504.f, kFcHalfLeast = 0.0625f;  // scaled: fp16's largest; 2^-4, which keeps 21 bits (lo's last place is 2^-24)
-constexpr int kFcSampleHeadroom = 4;  // octaves between the largest of a sample and 2^15
-
-// What the contractions in pairs of fp16 read by TMA as their operand B: rows of 32 hi and 32 lo (half_pairs.cuh), zeros behind the last of the
-// reduction.  Split once here instead of by every tile of the other operand: with that in the transform warps the contraction was no faster than
-// on tf32 (fc6, batch 256: 82 us, twice as many values to split as of the other operand).
-struct FcSplit {
-  const float* src;  // [rows][cols], rows `pitch` apart
-  int rows, cols, pitch, slot;
-  float* out;        // [rows][out_pitch]: the reduction along a row
-  int out_pitch;
-  float* flipped;    // [cols][flipped_pitch]: the reduction over the rows (null: not needed)
-  int flipped_pitch;
-  unsigned flip_blocks, per_strip;  // of the grid; tiles of a strip of 32 rows
-  const HalfScales* half;
-};
-constexpr int kFlipCols = 64;
-__global__ void __launch_bounds__(256) fc_split_kernel(const __grid_constant__ FcSplit S) {
-  __shared__ float tile[32][kFlipCols + 1];
-  pdl_wait();
-  const HalfScale scale = S.half->of[S.slot];
-  if (!scale.ok) return;
-  float x[8];
-  uint32_t hi[4], lo[4];
-  float* to;
-  if (blockIdx.x < S.flip_blocks) {  // 32 rows x 64 columns: a line of each column
-    const int r0 = (int)(blockIdx.x / S.per_strip) * 32, c0 = (int)(blockIdx.x % S.per_strip) * kFlipCols;
-    for (int e = threadIdx.x; e < 32 * kFlipCols; e += 256) {
-      const int r = e / kFlipCols, c = e % kFlipCols;
-      tile[r][c] = r0 + r < S.rows && c0 + c < S.cols ? __ldg(S.src + (size_t)(r0 + r) * S.pitch + c0 + c) : 0.f;
-    }
-    __syncthreads();
-    const int c = threadIdx.x >> 2, part = threadIdx.x & 3;
-    if (c0 + c >= S.cols) return;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = tile[part * 8 + e][c];
-    to = S.flipped + (size_t)(c0 + c) * S.flipped_pitch + r0 + part * 4;
-  } else {  // eight of a row
-    const int per_row = S.out_pitch / 8;
-    const size_t t = (size_t)(blockIdx.x - S.flip_blocks) * 256 + threadIdx.x;
-    const int r = (int)(t / per_row), c = (int)(t - (size_t)r * per_row) * 8;
-    if (r >= S.rows) return;
-    const float* from = S.src + (size_t)r * S.pitch + c;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {  // pitches are multiples of four floats
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c + 4 * q < S.pitch) v = __ldg(reinterpret_cast<const float4*>(from + 4 * q));
-      x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
-    }
-    to = S.out + (size_t)r * S.out_pitch + (c & ~31) + (c & 31) / 2;
-  }
-#pragma unroll
-  for (int e = 0; e < 4; ++e) split_half2(x[2 * e] * scale.scale, x[2 * e + 1] * scale.scale, hi[e], lo[e]);
-  *reinterpret_cast<uint4*>(to) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-  *reinterpret_cast<uint4*>(to + kHalfLo) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-}
-
-// Half `h` of row m's 32 reduction indices of A's raw tile.  MN-major: 32 x 32 boxes, row = reduction index (128 bytes), 32-byte chunks XORed
-// with the row index mod 4; K-major: rows of 128 bytes, 16-byte chunks XORed with the row index mod 8.
-__device__ __forceinline__ void fc_load_a(const uint8_t* st, int mn, int m, int h, float (&x)[16]) {
-  if (mn) {
-    const uint8_t* box = st + (size_t)(m >> 5) * 4096u;
-#pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      const uint32_t k = (uint32_t)(h * 16 + e);
-      const uint32_t off = k * 128u + (uint32_t)(m & 31) * 4u;
-      x[e] = *reinterpret_cast<const float*>(box + (off ^ ((k & 3u) << 5)));
-    }
-  } else {
-    const uint8_t* rowp = st + (size_t)m * 128u;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const uint32_t c = (uint32_t)(h * 4 + e);
-      const float4 v4 = *reinterpret_cast<const float4*>(rowp + ((c ^ (uint32_t)(m & 7)) << 4));
-      x[4 * e] = v4.x; x[4 * e + 1] = v4.y; x[4 * e + 2] = v4.z; x[4 * e + 3] = v4.w;
-    }
-  }
-}
-
 // What bounds it: at batch 256 the tensor pipe (12 MMAs of N / 2 cycles per k-block; fc6's forward pass 84 us, data gradient 76, pipe
 // 83 % active on the 128 and 144 SMs with a block, banks of shared memory 40 - 45 % busy), at small batches the stream of W (or,
 // for the weight gradient, of dW) - so the same roles in two shapes.
-// In pairs of fp16: the way from L2 to the SM (48 KB a k-block of 256 columns in 0.62 us on each of 128 SMs: 9.9 TB/s; MMAs 0.44 us): fc6 52 us forward,
-// 72 weight gradient, 52 data gradient, instead of 86, 97 and 79.
 //   N > 128 columns: one CTA per SM, the whole batch in one accumulator, so that a weight tile is split into tensor memory
 //   once (two CTAs with half the batch each split it twice and waited for it: 61 % of the tensor pipe).
 //   N <= 128: two CTAs per SM, 256 tensor-memory columns each.
@@ -183,9 +89,9 @@ __device__ __forceinline__ void fc_load_a(const uint8_t* st, int mn, int m, int 
 // about ten instructions each and made the weight gradient of small batches instruction-bound (fc6, batch 32: 70 us, 2.1 TB/s).
 // TWO: block `block0` of `blocks` that share the tiles (else the grid's: said of the loops as such, since with variables in their place fc6
 // at batch 256 took 308 us both ways instead of 300).
-template <bool TWO, bool HALF>
+template <bool TWO>
 __device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtensorMap& a_map, const CUtensorMap& b_map, const CUtensorMap& out_map,
-                                             unsigned block0, unsigned blocks, const FcHalf& H) {
+                                             unsigned block0, unsigned blocks) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
@@ -199,7 +105,7 @@ __device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtens
   if (tid == 0) {
     for (int s = 0; s < kFcRing; ++s) {
       mbar_init(raw_bar + 8u * s, 1);
-      mbar_init(lo_bar + 8u * s, HALF ? kFcXformWarps / 2 : kFcXformWarps);
+      mbar_init(lo_bar + 8u * s, kFcXformWarps);
       mbar_init(done_bar + 8u * s, 1);
     }
     for (int b = 0; b < 2; ++b) { mbar_init(acc_full + 8u * b, 1); mbar_init(acc_empty + 8u * b, kFcEpiWarps); }
@@ -213,8 +119,7 @@ __device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtens
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-  constexpr int kACols = HALF ? 32 : 64;  // of an A slot: hi, lo; two halves to a column
-  const uint32_t a_col0 = (uint32_t)(P.acc_bufs * P.n_pad);  // A slots behind the accumulators
+  const uint32_t a_col0 = (uint32_t)(P.acc_bufs * P.n_pad);  // A slots (64 columns: 32 hi + 32 lo) behind the accumulators
   const int total_tiles = P.m_tiles * P.n_tiles * P.splits;
   bool failed = false;
   // tile t -> (split, n-tile, m-tile), m-tile fastest; k-blocks [kb0, kb1)
@@ -260,7 +165,7 @@ __device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtens
       }
     }
   } else if (warp == kFcMmaWarp) {  // see elect_one
-    const uint32_t idesc = HALF ? make_idesc_f16(P.n_pad) : make_idesc(P.n_pad) | (P.b_mn ? 1u << 16 : 0u);  // A from tensor memory: lanes x K
+    const uint32_t idesc = make_idesc(P.n_pad) | (P.b_mn ? 1u << 16 : 0u);  // A from tensor memory: lanes x K
     const uint32_t tmem = warp_uniform(tmem_base);
     Ring raw, lo, ta;
     int i = 0, tile_iter = 0;
@@ -277,18 +182,8 @@ __device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtens
         tc_fence_after();
         const uint32_t b_raw = base + (uint32_t)raw.idx * L.raw_bytes + kFcATile;
         const uint32_t b_lo = base + L.lo_off + (uint32_t)lo.idx * L.b_tile_bytes;
-        const uint32_t t_hi = tmem + a_col0 + (uint32_t)(ta.idx * kACols), t_lo = t_hi + 32u;
-        if (HALF && elect_one()) {
-          const uint64_t bh = make_desc(b_raw), bl = bh + 4;  // a row: 64 bytes of hi, 64 of lo
-#pragma unroll
-          for (int j = 0; j < kBlockK / 16; ++j) {
-            umma_f16_ts(d_tmem, t_hi + (uint32_t)(16 + j * 8), bh + (uint64_t)(j * 2), idesc, (kb == kb0 && j == 0) ? 0u : 1u);
-            umma_f16_ts(d_tmem, t_hi + (uint32_t)(j * 8), bl + (uint64_t)(j * 2), idesc, 1u);
-            umma_f16_ts(d_tmem, t_hi + (uint32_t)(j * 8), bh + (uint64_t)(j * 2), idesc, 1u);
-          }
-          umma_commit(done_bar + 8u * (i & 3));
-          if (kb == kb1 - 1) umma_commit(acc_full + 8u * buf);
-        } else if (!HALF && elect_one()) {
+        const uint32_t t_hi = tmem + a_col0 + (uint32_t)(ta.idx * 64), t_lo = t_hi + 32u;
+        if (elect_one()) {
 #pragma unroll
           for (int j = 0; j < kBlockK / 8; ++j) {
             // K-major: 8 reduction indices = 32 bytes along the swizzled row; MN-major: 8 rows of 128 bytes
@@ -314,46 +209,38 @@ __device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtens
     const int b_vec = (int)(L.b_tile_bytes / 16);
     const int q = warp & 3, half = (warp - kFcXformWarp0) >> 2;
     const int m = q * 32 + lane;  // row of the tile = tensor-memory lane; this thread takes half of the k-block's 32 indices
-    const int back = HALF ? P.a_slots : min(P.lo_slots, P.a_slots);
+    const int back = min(P.lo_slots, P.a_slots);
     Ring raw, lo, ta;
     int i = 0;
-    float most = 0.f, least = __int_as_float(0x7f800000);  // HALF: of the largest values of A's rows, unless that is 0
     for (int t = TWO ? block0 : blockIdx.x; t < total_tiles; t += TWO ? blocks : gridDim.x) {
       int mt, nt, split, kb0, kb1;
       tile_of(t, mt, nt, split, kb0, kb1);
-      float top = 0.f;
       for (int kb = kb0; kb < kb1; ++kb, ++i) {
-        if (HALF && (i & 1) != half) {
-          raw.advance(P.raw_slots);
-          ta.advance(P.a_slots);
-          continue;
-        }
         mbar_wait(raw_bar + 8u * raw.idx, (uint32_t)raw.use & 1u, failed, P.status, 0x1500);
         if (i >= back) mbar_wait(done_bar + 8u * ((i - back) & 3), (uint32_t)((i - back) >> 2) & 1u, failed, P.status, 0x1510);
         tc_fence_after();
         const uint8_t* st = base_ptr + (size_t)raw.idx * L.raw_bytes;
-        if constexpr (HALF) {  // four warps take a k-block, the other four the next
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              float x[16];
-              fc_load_a(st, P.a_mn, m, h, x);
-#pragma unroll
-              for (int e = 0; e < 16; ++e) top = fmaxf(top, fabsf(x[e]));
-              uint32_t hi[8], l8[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) split_half2(x[2 * e] * H.scale_a, x[2 * e + 1] * H.scale_a, hi[e], l8[e]);
-              const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + a_col0 + (uint32_t)(ta.idx * kACols + h * 8);
-              tmem_st8(at, hi);
-              tmem_st8(at + 16u, l8);
-            }
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(lo_bar + 8u * (i & 3));
-        } else {
         float x[16];
-        fc_load_a(st, P.a_mn, m, half, x);
-        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + a_col0 + (uint32_t)(ta.idx * kACols + half * 16);
+        if (P.a_mn) {
+          // 32 x 32 boxes, row = reduction index (128 bytes), 32-byte chunks XORed with the row index mod 4
+          const uint8_t* box = st + (size_t)(m >> 5) * 4096u;
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const uint32_t k = (uint32_t)(half * 16 + e);
+            const uint32_t off = k * 128u + (uint32_t)(m & 31) * 4u;
+            x[e] = *reinterpret_cast<const float*>(box + (off ^ ((k & 3u) << 5)));
+          }
+        } else {
+          // rows of 128 bytes, 16-byte chunks XORed with the row index mod 8
+          const uint8_t* rowp = st + (size_t)m * 128u;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint32_t c = (uint32_t)(half * 4 + e);
+            const float4 v4 = *reinterpret_cast<const float4*>(rowp + ((c ^ (uint32_t)(m & 7)) << 4));
+            x[4 * e] = v4.x; x[4 * e + 1] = v4.y; x[4 * e + 2] = v4.z; x[4 * e + 3] = v4.w;
+          }
+        }
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + a_col0 + (uint32_t)(ta.idx * 64 + half * 16);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t hi[8], l8[8];
@@ -379,19 +266,11 @@ __device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtens
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(lo_bar + 8u * (i & 3));
-        }
         raw.advance(P.raw_slots);
         lo.advance(P.lo_slots);
         ta.advance(P.a_slots);
       }
-      if (HALF) {
-        most = fmaxf(most, top);
-        if (top > 0.f) least = fminf(least, top);
-      }
     }
-    // A value that does not fit into fp16, or a row (its part of one sum) that loses places there, by its largest value: the launch behind this one takes over.
-    if constexpr (HALF)
-      if (H.outside && (!(most * H.scale_a < kFcHalfMost) || least * H.scale_a < kFcHalfLeast)) *H.outside = 1;
   } else {
     // ---- epilogue: lane = m (contiguous in the output), one column = one n
     const int quarter = warp;  // warps 0-3 own tensor-memory lanes 32 * warp ...
@@ -413,12 +292,6 @@ __device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtens
         tmem_ld16(acc + (uint32_t)(c * 16), v[0]);
         if (two) tmem_ld16(acc + (uint32_t)(c * 16 + 16), v[1]);
         if (failed || m0 >= P.M) continue;
-        if constexpr (HALF) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[h][j] *= H.back;
-        }
         if (P.direct) {
 #pragma unroll
           for (int h = 0; h < 2; ++h)
@@ -460,18 +333,7 @@ __device__ __forceinline__ void fc_gemm_body(const FcGemmParams& P, const CUtens
 __global__ void __launch_bounds__(kFcThreads, 2)
     fc_gemm_kernel(const __grid_constant__ FcGemmParams P, const __grid_constant__ CUtensorMap a_map,
                    const __grid_constant__ CUtensorMap b_map, const __grid_constant__ CUtensorMap out_map) {
-  fc_gemm_body<false, false>(P, a_map, b_map, out_map, 0, 0, FcHalf{});
-}
-// In pairs of fp16, where the operands' scales say so (22 bits of each operand as with tf32, half the truncated additions: errors halve): a k-block is 6 MMAs of N / 2 cycles instead of 12, and
-// B comes split (fc_split_kernel), so that the transform warps have A alone.
-// `outside`: A's scale comes from a sample, so the kernel looks at all its values itself (null: the scale's launch has).
-__global__ void __launch_bounds__(kFcThreads, 2)
-    fc_gemm_half_kernel(const __grid_constant__ FcGemmParams P, const __grid_constant__ CUtensorMap a_map, const __grid_constant__ CUtensorMap b_map,
-                        const __grid_constant__ CUtensorMap out_map, HalfScales* half, int a, int b) {
-  pdl_wait();
-  if (!half_route(half, a, b)) return;
-  const HalfScale A = half->of[a], B = half->of[b];
-  fc_gemm_body<false, true>(P, a_map, b_map, out_map, 0, 0, FcHalf{A.scale, A.inverse * B.inverse, a == kHalfW ? &half->of[kHalfW].bad : nullptr});
+  fc_gemm_body<false>(P, a_map, b_map, out_map, 0, 0);
 }
 // The two contractions of a backward pass of few tiles in one launch: blocks [0, first) work on the weight gradient, those behind them on
 // the data gradient.  Each of such a layer's launches is five microseconds of set-up and hand-overs however little it does: 800 -> 500,
@@ -484,18 +346,7 @@ __global__ void __launch_bounds__(kFcThreads, 2) fc_gemm_two_kernel(const __grid
   const bool second = blockIdx.x >= first;
   const FcGemmParams P = second ? d.P : w.P;
   const FcJob& J = second ? d : w;
-  fc_gemm_body<true, false>(P, J.a, J.b, J.out, blockIdx.x - (second ? first : 0u), second ? gridDim.x - first : first, FcHalf{});
-}
-// What fc_gemm_half_kernel left: `w` (blocks [0, first)) where X or dY is not for pairs of fp16, `d`, weights by operand `b`, where W or that one is
-// not or a value of W lay outside.  Nearly always neither, and all blocks return.
-__global__ void __launch_bounds__(kFcThreads, 2)
-    fc_gemm_rest_kernel(const __grid_constant__ FcJob w, const __grid_constant__ FcJob d, unsigned first, const HalfScales* half, int b) {
-  pdl_wait();
-  const bool second = blockIdx.x >= first;
-  if (second ? half_route(half, kHalfW, b) && !half->of[kHalfW].bad : half_route(half, kHalfX, kHalfDy)) return;
-  const FcGemmParams P = second ? d.P : w.P;
-  const FcJob& J = second ? d : w;
-  fc_gemm_body<true, false>(P, J.a, J.b, J.out, blockIdx.x - (second ? first : 0u), second ? gridDim.x - first : first, FcHalf{});
+  fc_gemm_body<true>(P, J.a, J.b, J.out, blockIdx.x - (second ? first : 0u), second ? gridDim.x - first : first);
 }
 
 // db[o] = sum_b dY[b][o] (FullyConnectedBridge_impl.hxx:298: backward_bias_fc).  A block of 32 x 8 threads owns 32
@@ -677,14 +528,14 @@ struct FcShape {
 };
 
 // Rings that fit: the raw ring first (it holds a slot for TMA + transform + MMA), then the second tile on its way out.
-bool fc_fit_rings(FcShape& s, bool half = false) {
+bool fc_fit_rings(FcShape& s) {
   FcGemmParams& P = s.P;
   const size_t budget = s.pair ? 113 * 1024 : kSmemLimit;
   P.tmem_cols = s.pair ? 256 : 512;
-  P.a_slots = std::min(kFcRing, (P.tmem_cols - P.acc_bufs * P.n_pad) / (half ? 32 : 64));
+  P.a_slots = std::min(kFcRing, (P.tmem_cols - P.acc_bufs * P.n_pad) / 64);
   for (int raw = kFcRing; raw >= 2; --raw)
     for (int st = 2; st >= 1; --st) {
-      const int lo = half ? 0 : std::min(raw, P.n_pad <= 64 ? 3 : 2);
+      const int lo = std::min(raw, P.n_pad <= 64 ? 3 : 2);
       const size_t need = fc_smem(P.n_pad, raw, lo, st).total + 1024;
       if (need <= budget) {
         P.raw_slots = raw; P.lo_slots = lo; P.store_bufs = st;
@@ -785,30 +636,6 @@ bool fc_pair_faster(int sms, const FcShape& w, const FcShape& d, const FcShape& 
   return 20 * (tw + td) <= 21 * slots || td > sms || (w.P.kblocks_total <= 2 && d.P.kblocks_per_split < 8) || second_round_empty;
 }
 
-// Microseconds that a contraction in pairs of fp16 saves.  A k-block of its tiles takes half of tf32's MMA time or, mostly, as long as the way of its
-// 16 KB of A and 128 bytes a column of B from L2 to the SM at some 77 KB / us with all SMs at it (256 columns: 0.62 us, 72 k-blocks of fc6 52 us; tf32's
-// MMAs 0.88, measured 1.1 with what surrounds them).  Two CTAs per SM, up to 128 columns, wait for the weights as it is.
-double fc_half_saves(int sms, const FcShape& s) {
-  if (s.pair) return -1e9;
-  const double mma = 12 * (s.P.n_pad / 2.0) / 1750.0, half = std::max(0.6 * mma, (16 + s.P.n_pad / 8.0) / 77.0);
-  const long long tiles = (long long)s.P.m_tiles * s.P.n_tiles * s.P.splits;
-  return (double)((tiles + sms - 1) / sms * s.P.kblocks_per_split) * (1.2 * mma - half);
-}
-// Whether a pass of them takes it: launches for the scales, the split and the rest, and their reads and writes.  Forward, 256 images: 9216 -> 4096
-// 86 -> 69 us, 4096 -> 4096 45 -> 41, 9080 -> 2108 51 -> 47, but 4096 -> 1000 20 -> 25; 160 images, 8924 -> 3188 49 -> 52.  Backward: 173 -> 144, 90 -> 84,
-// 113 -> 104, 37 -> 41, 109 -> 104; 512 images, 9680 -> 2964, 286 -> 207.  The estimate is on the safe side by up to 20 us.
-bool fc_half_forward_pays(int sms, const FcShape& f, size_t x) { return fc_half_saves(sms, f) > 8 + 12.0 * x / 6.5e6 + 3; }
-bool fc_half_backward_pays(int sms, const FcShape& d, const FcShape& w, size_t x, size_t dy) {
-  return fc_half_saves(sms, d) + fc_half_saves(sms, w) > 16 + (4.0 * x + 20.0 * dy) / 6.5e6 + 3;
-}
-
-ScaleOf fc_scale(const float* a, size_t n, int slot) {
-  ScaleOf o{a, nullptr, n, slot, 0};
-  o.sample = slot == kHalfW;
-  o.headroom = o.sample ? kFcSampleHeadroom : 0;
-  return o;
-}
-
 }  // namespace
 
 struct cct_fc_plan {
@@ -816,13 +643,6 @@ struct cct_fc_plan {
   int B = 0, K = 0, O = 0, bias = 0;
   int K4 = 0, O4 = 0;        // row pitches: multiples of four floats
   FcShape fwd, dgr, wgr, wgr_pair;  // wgr_pair: the weight gradient's, beside the data gradient in one launch
-  bool half_forward = false, half_backward = false;  // in pairs of fp16, where the values allow it
-  FcShape fwd_half, dgr_half, wgr_half;
-  float *split = nullptr, *flipped = nullptr;  // X (forward) or dY in pairs of fp16, dY the other way round
-  FcMap x_half, dy_half, dy_flipped;
-  HalfScales* half = nullptr;  // of the present call, with what finds them
-  uint2* half_parts = nullptr;
-  uint32_t* half_ticket = nullptr;
   bool pair = false;         // both gradients in one launch, where the SMs that a call has can take their tiles
   bool dot = false, dot_narrow = false;  // forward pass by fc_dot_kernel: rows on 16-byte boundaries, and off them
   bool small_forward = false, small = false;  // else the forward pass, and the backward pass, by fc_small_kernel, with these splits (where an
@@ -844,36 +664,6 @@ int fc_launch(cct_ctx* ctx, const FcShape& s, const FcMap& a, const FcMap& b, co
   const int tiles = P.m_tiles * P.n_tiles * P.splits;
   launch_pdl(fc_gemm_kernel, dim3(std::min(tiles, (s.pair ? 2 : 1) * ctx->launch_sms())), dim3(kFcThreads), s.smem, ctx->stream, P,
              a.map, b.map, out.map);
-  CCT_CHECK_LAUNCH(ctx);
-  return CCT_OK;
-}
-
-int fc_launch_half(cct_ctx* ctx, const cct_fc_plan* plan, const FcShape& s, const FcMap& a, const FcMap& b, const FcMap& out, int a_slot, int b_slot,
-                   float* direct = nullptr, long long ld_direct = 0) {
-  FcGemmParams P = s.P;
-  P.direct = direct; P.ld_direct = ld_direct;
-  P.status = ctx->status_dev;
-  launch_pdl(fc_gemm_half_kernel, dim3(std::min<long long>(fc_tiles(s), (s.pair ? 2 : 1) * ctx->launch_sms())), dim3(kFcThreads), s.smem, ctx->stream, P,
-             a.map, b.map, out.map, plan->half, a_slot, b_slot);
-  CCT_CHECK_LAUNCH(ctx);
-  return CCT_OK;
-}
-int fc_split(cct_ctx* ctx, const cct_fc_plan* plan, const float* src, int rows, int cols, int pitch, int slot, bool flip) {
-  FcSplit S{src, rows, cols, pitch, slot, plan->split, fc_round_up(cols, 32), flip ? plan->flipped : nullptr, fc_round_up(rows, 32),
-            0, (unsigned)((cols + kFlipCols - 1) / kFlipCols), plan->half};
-  if (flip) S.flip_blocks = S.per_strip * (unsigned)((rows + 31) / 32);
-  const size_t threads = (size_t)rows * (S.out_pitch / 8);
-  launch_pdl(fc_split_kernel, dim3(S.flip_blocks + (unsigned)((threads + 255) / 256)), dim3(256), 0, ctx->stream, S);
-  CCT_CHECK_LAUNCH(ctx);
-  return CCT_OK;
-}
-// What the launches in pairs of fp16 left (see fc_gemm_rest_kernel): the weights' contraction `d` with operand `b`, in a backward pass also the weight
-// gradient (`w`, null: none).
-int fc_launch_rest(cct_ctx* ctx, const cct_fc_plan* plan, const FcJob* w, const FcShape* ws, const FcJob& d, const FcShape& ds, int b) {
-  auto grid = [&](const FcShape& s) { return (int)std::min<long long>(fc_tiles(s), (s.pair ? 2 : 1) * ctx->launch_sms()); };
-  const int first = w ? grid(*ws) : 0;
-  launch_pdl(fc_gemm_rest_kernel, dim3(first + grid(ds)), dim3(kFcThreads), std::max(w ? ws->smem : 0, ds.smem), ctx->stream, w ? *w : d, d,
-             (unsigned)first, plan->half, b);
   CCT_CHECK_LAUNCH(ctx);
   return CCT_OK;
 }
@@ -1002,21 +792,7 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   auto room = [](size_t n) { return (n + 63) & ~(size_t)63; };
   const size_t x = pad_k ? room((size_t)batch * p->K4) : 0, w = pad_k ? room((size_t)out_features * p->K4) : 0,
                dy = pad_o ? room((size_t)batch * p->O4) : 0;
-  p->half_forward = !few && fc_half_forward_pays(ctx->sm_count, p->fwd, (size_t)batch * in_features);
-  p->half_backward = !p->small && !p->pair &&
-                     fc_half_backward_pays(ctx->sm_count, p->dgr, p->wgr, (size_t)batch * in_features, (size_t)batch * out_features);
-  auto in_half = [](FcShape s) {
-    s.P.b_mn = 0;
-    return s;
-  };
-  p->fwd_half = in_half(p->fwd); p->dgr_half = in_half(p->dgr); p->wgr_half = in_half(p->wgr);
-  p->half_forward = p->half_forward && fc_fit_rings(p->fwd_half, true);
-  p->half_backward = p->half_backward && fc_fit_rings(p->dgr_half, true) && fc_fit_rings(p->wgr_half, true);
-  const size_t split = std::max(p->half_forward ? (size_t)batch * fc_round_up(in_features, 32) : 0, p->half_backward ? (size_t)batch * fc_round_up(out_features, 32) : 0),
-               flipped = p->half_backward ? (size_t)out_features * fc_round_up(batch, 32) : 0;
-  const size_t parts = 2ull * ctx->sm_count * kScaleBlocksPerSm;
-  const size_t scales = p->half_forward || p->half_backward ? room(sizeof(HalfScales) / sizeof(float) + 64) + room(2 * parts) + room(split) + room(flipped) : 0;
-  p->bytes = (room(sums) + x + w + dy + scales) * sizeof(float);
+  p->bytes = (room(sums) + x + w + dy) * sizeof(float);
   if (cudaMalloc((void**)&p->partial, p->bytes) != cudaSuccess) {
     cudaGetLastError();
     ctx->last_error = "cudaMalloc of the fully connected layer's scratch failed";
@@ -1026,22 +802,7 @@ int cct_fc_plan_create(cct_ctx* ctx, int batch, int in_features, int out_feature
   float* at = p->partial + room(sums);
   if (pad_k) { p->Xp = at; p->Wp = at + x; }
   if (pad_o) p->dYp = at + x + w;
-  if (scales) {
-    at += x + w + dy;
-    p->half = reinterpret_cast<HalfScales*>(at);
-    p->half_ticket = reinterpret_cast<uint32_t*>(at + room(sizeof(HalfScales) / sizeof(float) + 2) - 2);
-    at += room(sizeof(HalfScales) / sizeof(float) + 64);
-    p->half_parts = reinterpret_cast<uint2*>(at);
-    p->split = at + room(2 * parts);
-    p->flipped = p->split + room(split);
-  }
   cudaError_t e = cudaFuncSetAttribute(fc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-  if (scales) {
-    const uint32_t none[2] = {0, 0};
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_gemm_half_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fc_gemm_rest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-    if (e == cudaSuccess) e = cudaMemcpy(p->half_ticket, none, sizeof(none), cudaMemcpyHostToDevice);
-  }
   if (e == cudaSuccess && p->pair && !p->small) e = cudaFuncSetAttribute(fc_gemm_two_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024);
   if (e != cudaSuccess) {
     ctx->last_error = std::string("cudaFuncSetAttribute(fc_gemm_kernel): ") + cudaGetErrorString(e);
@@ -1107,17 +868,7 @@ int cct_fc_forward(cct_fc_plan* plan, const float* X, const float* W, const floa
   int rc = fc_operand_map(ctx, &plan->w_fwd, W, O, K, K4, kTileM, false);
   if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->x_fwd, X, B, K, K4, plan->fwd.P.n_pad, false);
   if (rc == CCT_OK) rc = fc_output_map(ctx, &plan->out_fwd, plan->partial, O, B, plan->fwd.P.splits, O4);
-  if (rc == CCT_OK && plan->half_forward) {
-    launch_scales(ctx, plan->half, plan->half_parts, plan->half_ticket, {fc_scale(X, (size_t)B * K4, kHalfX), fc_scale(W, (size_t)O * K4, kHalfW)});
-    rc = fc_split(ctx, plan, X, B, K, K4, kHalfX, false);
-    if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->x_half, plan->split, B, fc_round_up(K, 32), fc_round_up(K, 32), plan->fwd_half.P.n_pad, false);
-    if (rc == CCT_OK) rc = fc_launch_half(ctx, plan, plan->fwd_half, plan->w_fwd, plan->x_half, plan->out_fwd, kHalfW, kHalfX);
-    FcJob d{plan->fwd.P, plan->w_fwd.map, plan->x_fwd.map, plan->out_fwd.map};
-    d.P.status = ctx->status_dev;
-    if (rc == CCT_OK) rc = fc_launch_rest(ctx, plan, nullptr, nullptr, d, plan->fwd, kHalfX);
-  } else if (rc == CCT_OK) {
-    rc = fc_launch(ctx, plan->fwd, plan->w_fwd, plan->x_fwd, plan->out_fwd);
-  }
+  if (rc == CCT_OK) rc = fc_launch(ctx, plan->fwd, plan->w_fwd, plan->x_fwd, plan->out_fwd);
   if (rc == CCT_OK)
     rc = fc_reduce(ctx, FcReduceParams{plan->partial, Y, plan->bias ? bias : nullptr, nullptr, drop_mask, drop_scale, B, O, O4,
                                        plan->fwd.P.splits, relu});
@@ -1151,10 +902,6 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
   const bool together = clear && w_small && d_small;
   const int two = clear && plan->pair && !w_small && !d_small ? share_slots(2ll * ctx->launch_sms(), fc_tiles(plan->wgr_pair), fc_tiles(plan->dgr)) : 0;
   const bool direct = K4 != K || !fc_aligned({dW});  // dW: an output no tensor map describes
-  // In pairs of fp16: the weight gradient's other form runs behind the data gradient, so neither may write what the other reads.
-  const bool half = plan->half_backward && !w_small && !d_small && dX && apart(dW, nw, {{W, nw}, {dY, ny}, {X, nx}}) &&
-                    apart(db, nb, {{W, nw}, {dY, ny}, {X, nx}});
-  FcJob w_rest{};
   if (w_small) {
     if (!together) rc = fc_small(ctx, W_job);
     if (rc != CCT_OK) return rc;
@@ -1163,17 +910,7 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     rc = fc_operand_map(ctx, &plan->x_wgr, Xm, B, K, K4, 32, true);
     if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_wgr, dYm, B, O, O4, 32, true);
     if (rc == CCT_OK && !direct) rc = fc_output_map(ctx, &plan->out_wgr, dW, K, O, 1, K);
-    if (rc == CCT_OK && half) {
-      if (plan->Wp) { fc_pad(ctx, W, plan->Wp, O, K, K4); W = plan->Wp; }
-      launch_scales(ctx, plan->half, plan->half_parts, plan->half_ticket,
-                    {fc_scale(Xm, (size_t)B * K4, kHalfX), fc_scale(W, (size_t)O * K4, kHalfW), fc_scale(dYm, (size_t)B * O4, kHalfDy)});
-      w_rest = FcJob{plan->wgr.P, plan->x_wgr.map, plan->dy_wgr.map, (direct ? plan->x_wgr : plan->out_wgr).map};
-      w_rest.P.direct = direct ? dW : nullptr; w_rest.P.ld_direct = K; w_rest.P.status = ctx->status_dev;
-      rc = fc_split(ctx, plan, dYm, B, O, O4, kHalfDy, true);
-      if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_flipped, plan->flipped, O, fc_round_up(B, 32), fc_round_up(B, 32), plan->wgr_half.P.n_pad, false);
-      if (rc == CCT_OK)
-        rc = fc_launch_half(ctx, plan, plan->wgr_half, plan->x_wgr, plan->dy_flipped, direct ? plan->x_wgr : plan->out_wgr, kHalfX, kHalfDy, direct ? dW : nullptr, K);
-    } else if (rc == CCT_OK && !two)
+    if (rc == CCT_OK && !two)
       rc = fc_launch(ctx, plan->wgr, plan->x_wgr, plan->dy_wgr, direct ? plan->x_wgr : plan->out_wgr, direct ? dW : nullptr, K);
     if (rc != CCT_OK) return rc;
     if (plan->bias) {
@@ -1198,17 +935,11 @@ int cct_fc_backward(cct_fc_plan* plan, const float* X, const float* W, const flo
     plan->timer.end(3, ctx->stream);
   } else if (dX) {
     plan->timer.begin(3, ctx->stream);
-    if (plan->Wp && !half) { fc_pad(ctx, W, plan->Wp, O, K, K4); W = plan->Wp; }
+    if (plan->Wp) { fc_pad(ctx, W, plan->Wp, O, K, K4); W = plan->Wp; }
     rc = fc_operand_map(ctx, &plan->w_dgr, W, O, K, K4, 32, true);
     if (rc == CCT_OK) rc = fc_operand_map(ctx, &plan->dy_dgr, dYm, B, O, O4, plan->dgr.P.n_pad, false);
     if (rc == CCT_OK) rc = fc_output_map(ctx, &plan->out_dgr, plan->partial, K, B, plan->dgr.P.splits, K4);
-    if (rc == CCT_OK && half) {
-      rc = fc_operand_map(ctx, &plan->dy_half, plan->split, B, fc_round_up(O, 32), fc_round_up(O, 32), plan->dgr_half.P.n_pad, false);
-      if (rc == CCT_OK) rc = fc_launch_half(ctx, plan, plan->dgr_half, plan->w_dgr, plan->dy_half, plan->out_dgr, kHalfW, kHalfDy);
-      FcJob d{plan->dgr.P, plan->w_dgr.map, plan->dy_dgr.map, plan->out_dgr.map};
-      d.P.status = ctx->status_dev;
-      if (rc == CCT_OK) rc = fc_launch_rest(ctx, plan, &w_rest, &plan->wgr, d, plan->dgr, kHalfDy);
-    } else if (rc == CCT_OK) rc = two ? fc_launch_two(ctx, plan, two, direct ? dW : nullptr, K) : fc_launch(ctx, plan->dgr, plan->w_dgr, plan->dy_dgr, plan->out_dgr);
+    if (rc == CCT_OK) rc = two ? fc_launch_two(ctx, plan, two, direct ? dW : nullptr, K) : fc_launch(ctx, plan->dgr, plan->w_dgr, plan->dy_dgr, plan->out_dgr);
     if (rc == CCT_OK)
       rc = fc_reduce(ctx, FcReduceParams{plan->partial, dX, nullptr, in_relu ? X : nullptr, in_drop_mask, in_drop_scale, B, K, K4,
                                          plan->dgr.P.splits, 0, 0, bias_sum});

@@ -21,7 +21,7 @@ constexpr int kScaleChunk = 8192;  // elements of a block at least
 struct ScaleJob {
   const float* a = nullptr;
   const float* mask = nullptr;  // set: elements whose mask is not positive count as 0
-  size_t n = 0, per_block = 0, read = 0;  // a block reads the first `read` of its `per_block` elements
+  size_t n = 0, per_block = 0;
   int first = 0, blocks = 0;    // of the grid
   int slot = 0;
   int headroom = 0;             // octaves that the operand may be larger than `a` (sums of up to four windows' gradients: 2)
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kScaleThreads, kScaleBlocksPerSm) operand_scal
   int which = 0;
   while (which + 1 < J.jobs && (int)blockIdx.x >= J.job[which + 1].first) ++which;
   const ScaleJob& job = J.job[which];
-  const size_t begin = (size_t)(blockIdx.x - job.first) * job.per_block, end = min(job.n, begin + job.read);
+  const size_t begin = (size_t)(blockIdx.x - job.first) * job.per_block, end = min(job.n, begin + job.per_block);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   ScaleStats s;
   // per_block is a multiple of 1024 floats: a block's part starts on a 16-byte boundary if the tensor does
@@ -165,40 +165,6 @@ __global__ void __launch_bounds__(kScaleThreads, kScaleBlocksPerSm) operand_scal
                                      scaled ? __uint_as_float((uint32_t)(127 - up) << 23) : 1.f, ok ? 1 : 0,
                                      mine.slot == kHalfDy ? (int)min(atomicExch(J.ticket + 1, 0u), (uint32_t)kMaxBad + 1u) : 0};
   }
-}
-
-// The scales of a call's operands (a = null: not needed) in one launch.
-struct ScaleOf {
-  const float *a, *mask;
-  size_t n;
-  int slot, headroom;
-  const int32_t* where = nullptr;
-  int pooled = 1, plane = 1;
-  bool sample = false;  // read kSampleChunk of every kSampleEvery elements (the contraction itself looks at the others)
-};
-constexpr int kSampleChunk = 2048, kSampleEvery = 32 * kSampleChunk;
-void launch_scales(cct_ctx* ctx, HalfScales* out, uint2* parts, uint32_t* ticket, std::initializer_list<ScaleOf> operands) {
-  ScaleJobs J{};
-  J.out = out; J.parts = parts; J.ticket = ticket;
-  size_t total = 0;
-  for (const ScaleOf& o : operands) total += !o.a ? 0 : o.sample ? o.n / (kSampleEvery / kSampleChunk) : o.n;
-  const size_t blocks = (size_t)ctx->sm_count * kScaleBlocksPerSm - 3;  // rounded up for each of three
-  const size_t per_block = (std::max<size_t>(kScaleChunk, (total + blocks - 1) / blocks) + 1023) & ~(size_t)1023;
-  int grid = 0;
-  for (const ScaleOf& o : operands) {
-    if (!o.a) continue;
-    ScaleJob& job = J.job[J.jobs++];
-    job.a = o.a; job.mask = o.mask; job.n = o.n; job.slot = o.slot; job.headroom = o.headroom;
-    job.where = o.where; job.pooled = o.pooled; job.plane = o.plane;
-    // a sample's blocks: as many as a whole operand of its size would have, each with its part of the places
-    const size_t sampled = (o.n + kSampleEvery - 1) / kSampleEvery, most = blocks / 2;
-    job.per_block = !o.sample ? per_block : kSampleEvery * ((sampled + most - 1) / most);
-    job.read = !o.sample ? per_block : kSampleChunk;
-    job.first = grid;
-    job.blocks = (int)((o.n + job.per_block - 1) / job.per_block);
-    grid += job.blocks;
-  }
-  launch_pdl(operand_scale_kernel, dim3(grid), dim3(kScaleThreads), 0, ctx->stream, J);
 }
 
 }  // namespace

@@ -270,98 +270,3 @@ def test_pooled_gradients_in_rows(ctx, layer, shape):
     hit[1, 2, index[1, 2, at_most[0], at_most[1]]] = 1
     inside = torch.nn.grad.conv2d_input(X.shape, torch.ones_like(W), hit.view(B, o, m, m), s, p, 1, g) != 0
     assert torch.isnan(dX[inside]).all() and torch.equal(dX[~inside], runs[0][0][~inside])
-
-
-class Full:
-    """A fully connected layer on torch's memory."""
-
-    def __init__(self, ctx, B, K, o):
-        self.ctx, self.plan = ctx, C.c_void_p()
-        capi.check(ctx.lib.cct_fc_plan_create(ctx.h, B, K, o, 1, C.byref(self.plan)), "plan", ctx.h)
-        gen = torch.Generator(device="cuda").manual_seed(B + K)
-        self.X, self.dY = torch.randn((B, K), device="cuda", generator=gen).clamp(min=0), torch.randn((B, o), device="cuda", generator=gen)
-        self.W, self.b = 0.02 * torch.randn((o, K), device="cuda", generator=gen), torch.randn(o, device="cuda", generator=gen)
-        self.Y, self.dX, self.dW, self.db = (torch.full_like(t, 7) for t in (self.dY, self.X, self.W, self.b))
-
-    def run(self):
-        torch.cuda.synchronize()
-        n = [launches(self.ctx, lambda: capi.check(self.ctx.lib.cct_fc_forward(
-                 self.plan, self.X.data_ptr(), self.W.data_ptr(), self.b.data_ptr(), self.Y.data_ptr(), 0, None, 1.0), "forward", self.ctx.h)),
-             launches(self.ctx, lambda: capi.check(self.ctx.lib.cct_fc_backward(
-                 self.plan, self.X.data_ptr(), self.W.data_ptr(), self.dY.data_ptr(), self.dX.data_ptr(), self.dW.data_ptr(), self.db.data_ptr(),
-                 0, None, 1.0), "backward", self.ctx.h))]
-        self.ctx.sync()
-        return n
-
-    def exact(self):
-        X, W, dY = self.X.double(), self.W.double(), self.dY.double()
-        return X @ W.t() + self.b.double(), dY @ W, dY.t() @ X, dY.sum(0)
-
-    def close(self):
-        self.ctx.lib.cct_fc_plan_destroy(self.plan)
-
-
-# The three products in tf32: twice the instructions, and both of an operand's parts cut.
-def full_bounds(B, K, o):
-    return 2 * bound(K), 2 * bound(o), 2 * bound(B), 2.0 ** -18
-
-
-# A whole tile of 256 columns; a ragged last one, with rows that are no multiple of 16 bytes; 208 columns, reductions with a part of a k-block.
-@pytest.mark.parametrize("shape", [(256, 9216, 4096), (500, 9001, 3003), (200, 9988, 5000)])
-def test_full_layers_in_pairs(ctx, shape):
-    """Each contraction, values that a sample of the weights does not show, operands that are not for pairs, and the same bits after those."""
-    f = Full(ctx, *shape)
-    try:
-        outputs, limits = (f.Y, f.dX, f.dW, f.db), full_bounds(*shape)
-
-        def check(factor):
-            for got, want, limit in zip(outputs, f.exact(), limits):
-                assert off(got, want) < factor * limit
-        pads = [0, 0] if shape[1] % 4 == 0 else [2, 3]
-        assert f.run() == [5 + pads[0], 6 + pads[1]]  # scales, split, contraction, what that left, reduction; two contractions in a backward pass
-        check(0.5)
-        first = [t.clone() for t in outputs]
-        W, X, dY, b = f.W.clone(), f.X.clone(), f.dY.clone(), f.b.clone()
-        f.W.view(-1)[50001] = 600.0  # between the places that are looked at beforehand: no fp16
-        f.run()
-        check(1)
-        f.W.copy_(W)
-        f.W[7] *= 2.0 ** -40  # a row of small weights keeps its places
-        f.b.zero_()
-        f.run()
-        check(1)
-        assert off(f.Y[:, 7], f.exact()[0][:, 7]) < limits[0]
-        f.W.copy_(W)
-        f.X[3] *= 2.0 ** -40
-        f.dY[:, 5] *= 2.0 ** 40
-        f.run()
-        for got, want, limit in zip(outputs[:1], f.exact()[:1], limits):
-            assert off(got[3], want[3]) < limit
-        assert off(f.dW[4], f.exact()[2][4]) < limits[2]
-        f.X.copy_(X); f.dY.copy_(dY)
-        for t, at in ((f.X, (3, 17)), (f.W, (11, 33)), (f.dY, (5, 4))):
-            keep = t[at].item()
-            for value in (float("inf"), float("nan")):
-                t[at] = value
-                f.run()
-                for got, want in zip(outputs, f.exact()):
-                    assert torch.equal(torch.isfinite(got), torch.isfinite(want))
-            t[at] = keep
-        f.b.copy_(b)
-        f.run()
-        assert all(torch.equal(a, b) for a, b in zip(first, outputs))
-    finally:
-        f.close()
-
-
-def test_full_layers_in_pairs_off_the_boundaries(ctx):
-    """A weight gradient that no tensor map describes is written by the threads."""
-    f = Full(ctx, 256, 9216, 4096)
-    try:
-        f.run()
-        want = f.dW.clone()
-        f.dW = torch.full((f.W.numel() + 1,), 7.0, device="cuda")[1:].view_as(f.W)
-        f.run()
-        assert torch.equal(f.dW, want)
-    finally:
-        f.close()
